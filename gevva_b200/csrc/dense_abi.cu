@@ -30,7 +30,21 @@ struct gevva_dense {
   float* ones = nullptr;          // [128]
   float* down_scale = nullptr;    // [1]: weights.down_scale on the device, for gevva_ff_finalize
   int* ints = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;  // gevva_ff_layer_launch: to the second stream and back
 };
+
+int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
+                        int sm_count) {
+  gv::launch_dense_plan(tokens, d->plan, stream);
+  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, stream);
+  gv::launch_grouped_gemm(d->gate_up, d->plan, sm_count, stream);
+  gv::launch_gelu_quantize_fp8(d->gate_up_out, d->act_scales, d->weights.gate_scale, d->weights.up_scale,
+                               d->prod_fp8, d->prod_scales, tokens, stream);
+  gv::GemmOperands down = d->down;
+  down.out = out_unscaled;
+  gv::launch_grouped_gemm(down, d->plan, sm_count, stream);
+  return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
+}
 
 extern "C" {
 
@@ -44,6 +58,8 @@ void gevva_dense_destroy(gevva_dense* d) {
   cudaFree(d->ones);
   cudaFree(d->down_scale);
   cudaFree(d->ints);
+  if (d->fork) cudaEventDestroy(d->fork);
+  if (d->join) cudaEventDestroy(d->join);
   delete d;
 }
 
@@ -75,6 +91,8 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
     e = cudaMemcpy(d->down_scale, &weights->down_scale, sizeof(float), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->ints), int_count * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(d->ints, 0, int_count * sizeof(int));
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d->fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d->join, cudaEventDisableTiming);
   if (e == cudaSuccess) {
     float host_ones[gv::kExperts];
     for (float& v : host_ones) v = 1.0f;
@@ -118,15 +136,7 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
 int gevva_dense_launch(gevva_dense* d, const void* in, void* out_unscaled, int tokens,
                        gevva_stream_t stream) {
   if (!d || !in || !out_unscaled || tokens < 1 || tokens > d->max_tokens) return GEVVA_MOE_BAD_ARGUMENT;
-  gv::launch_dense_plan(tokens, d->plan, stream);
-  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, stream);
-  gv::launch_grouped_gemm(d->gate_up, d->plan, d->sm_count, stream);
-  gv::launch_gelu_quantize_fp8(d->gate_up_out, d->act_scales, d->weights.gate_scale, d->weights.up_scale,
-                               d->prod_fp8, d->prod_scales, tokens, stream);
-  gv::GemmOperands down = d->down;
-  down.out = out_unscaled;
-  gv::launch_grouped_gemm(down, d->plan, d->sm_count, stream);
-  return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
+  return gv::dense_launch_on(d, in, out_unscaled, tokens, stream, d->sm_count);
 }
 
 const float* gevva_dense_output_scales(const gevva_dense* d) { return d ? d->prod_scales : nullptr; }
@@ -172,6 +182,84 @@ int gevva_ff_finalize(const void* dense, const void* dense_weight, const void* e
   gv::launch_ff_finalize(dense, dense_weight, expert_routes, route_weights, inverse_routes, expert_weight,
                          combined_weight, residual, layer_scalar, output, rows, dense_activation_scales,
                          dense_projection_scale, stream);
+  return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
+}
+
+// The intermediates of one layer call, carved from the caller's workspace.
+namespace {
+struct LayerWorkspace {
+  uint8_t* dense_in;
+  uint8_t* expert_in;
+  uint8_t* router_in;
+  uint8_t* dense_out;
+  float* route_weights;
+  int* ids;
+  size_t bytes;
+  LayerWorkspace(void* base, int tokens) {
+    uint8_t* cursor = static_cast<uint8_t*>(base);
+    size_t used = 0;
+    auto carve = [&](size_t n) {
+      uint8_t* p = cursor ? cursor + used : nullptr;
+      used += (n + 255) & ~static_cast<size_t>(255);
+      return p;
+    };
+    const size_t t = static_cast<size_t>(tokens);
+    const size_t rows = t * gv::kHidden * 2;
+    dense_in = carve(rows);
+    expert_in = carve(rows);
+    router_in = carve(rows);
+    dense_out = carve(rows);
+    route_weights = reinterpret_cast<float*>(carve(t * gv::kTopK * sizeof(float)));
+    ids = reinterpret_cast<int*>(carve(t * gv::kTopK * sizeof(int)));
+    bytes = used;
+  }
+};
+// SMs that the dense MLP of a decode-sized layer gets beside the experts (see gevva_ff_layer_launch).
+constexpr int kDenseSmsBesideDecode = 16;
+}  // namespace
+
+size_t gevva_ff_layer_workspace_bytes(int tokens) { return tokens < 1 ? 0 : LayerWorkspace(nullptr, tokens).bytes; }
+
+int gevva_ff_layer_launch(const gevva_ff_layer* layer, const void* hidden, void* out, void* workspace, int tokens,
+                          gevva_stream_t stream, gevva_stream_t aux_stream) {
+  if (!layer || !layer->dense_pre || !layer->expert_pre || !layer->router_scale || !layer->router_weight ||
+      !layer->expert_scale || !layer->dense_post || !layer->expert_post || !layer->combined_post ||
+      !layer->layer_scalar || !layer->experts || !layer->dense || !hidden || !out || !workspace ||
+      (reinterpret_cast<uintptr_t>(workspace) & 255) || tokens < 1 || tokens > layer->dense->max_tokens)
+    return GEVVA_MOE_BAD_ARGUMENT;
+  const LayerWorkspace w(workspace, tokens);
+  gevva_dense* dense = layer->dense;
+  const bool beside = aux_stream != stream;
+  // The dense MLP starts as soon as its input exists, on SMs that the router leaves idle.  A
+  // decode-sized expert launch holds its SMs from the router to its end, so it leaves a few to the
+  // dense side: the experts' time is that of their weights' way through HBM, which 132 SMs fill as
+  // well as 148, and the dense weights (18 MB) pass meanwhile instead of afterwards.
+  const int sms = gv::moe_sm_count(layer->experts);
+  const bool split = beside && tokens <= gv::kFusedSortQuantizeMaxTokens && sms > 2 * kDenseSmsBesideDecode;
+  const int dense_sms = split ? kDenseSmsBesideDecode : sms;
+  const int expert_sms = split ? sms - kDenseSmsBesideDecode : sms;
+  gv::launch_ff_prepare(hidden, layer->dense_pre, layer->expert_pre, layer->router_scale, w.dense_in, w.expert_in,
+                        w.router_in, tokens, stream);
+  if (beside) {
+    if (cudaEventRecord(dense->fork, stream) != cudaSuccess ||
+        cudaStreamWaitEvent(aux_stream, dense->fork, 0) != cudaSuccess)
+      return GEVVA_MOE_CUDA_ERROR;
+  }
+  int status = gv::dense_launch_on(dense, w.dense_in, w.dense_out, tokens, beside ? aux_stream : stream, dense_sms);
+  if (beside && cudaEventRecord(dense->join, aux_stream) != cudaSuccess) return GEVVA_MOE_CUDA_ERROR;
+  if (status == GEVVA_MOE_OK)
+    status = gevva_moe_route_project(w.router_in, layer->router_weight, nullptr, layer->expert_scale, w.route_weights,
+                                     w.ids, nullptr, tokens, gevva_moe_status_word(layer->experts), stream);
+  if (status == GEVVA_MOE_OK)
+    status = gv::moe_launch_stages_on(layer->experts, w.expert_in, w.ids, nullptr, nullptr, tokens,
+                                      GEVVA_MOE_STAGE_ALL & ~static_cast<unsigned>(GEVVA_MOE_STAGE_REDUCE), stream,
+                                      expert_sms);
+  // joined in every case: a caller that captures `stream` must get its second stream back
+  if (beside && cudaStreamWaitEvent(stream, dense->join, 0) != cudaSuccess) return GEVVA_MOE_CUDA_ERROR;
+  if (status != GEVVA_MOE_OK) return status;
+  gv::launch_ff_finalize(w.dense_out, layer->dense_post, gevva_moe_routed_output(layer->experts), w.route_weights,
+                         gevva_moe_inverse_routes(layer->experts), layer->expert_post, layer->combined_post, hidden,
+                         layer->layer_scalar, out, tokens, dense->prod_scales, dense->down_scale, stream);
   return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
 }
 

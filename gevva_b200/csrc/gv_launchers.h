@@ -6,7 +6,18 @@
 #include <stddef.h>
 #include <stdint.h>
 
+struct gevva_moe;
+struct gevva_dense;
+
 namespace gv {
+
+// gevva_moe_launch_stages and gevva_dense_launch on at most `sm_count` SMs (their persistent kernels
+// take one CTA per SM): what lets the two sides of a feed-forward layer run beside each other.
+int moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, const float* route_weights, void* out,
+                         int tokens, unsigned stages, cudaStream_t stream, int sm_count);
+int dense_launch_on(gevva_dense* dense, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
+                    int sm_count);
+int moe_sm_count(const gevva_moe* runner);
 
 // Device-resident description of one launch's routing, written by the route sort
 // and read by every later stage without a host round trip.

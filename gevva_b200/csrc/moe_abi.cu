@@ -252,6 +252,87 @@ struct StageRange {
 };
 }  // namespace
 
+int gv::moe_sm_count(const gevva_moe* runner) { return runner->sm_count; }
+
+int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, const float* route_weights, void* out,
+                             int tokens, unsigned stages, cudaStream_t stream, int sm_count) {
+  Scratch* s = runner->scratch;
+  // "expert runner token count exceeds its plan", src/nvfp4_cutlass.cu:1830-1832
+  if (tokens < 1 || tokens > s->max_tokens) return GEVVA_MOE_BAD_ARGUMENT;
+  if ((stages & (GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE)) && !ids) return GEVVA_MOE_BAD_ARGUMENT;
+  if ((stages & GEVVA_MOE_STAGE_QUANTIZE) && !in) return GEVVA_MOE_BAD_ARGUMENT;
+  if ((stages & GEVVA_MOE_STAGE_REDUCE) && (!out || !route_weights)) return GEVVA_MOE_BAD_ARGUMENT;
+  const int routes = tokens * kTopK;
+  // Decode-sized batches (at most a few rows per expert) stream weights and gain nothing from
+  // pairing two row tiles of an expert; they keep the one-CTA-per-tile kernel.
+  const bool use_pairs = runner->pairs && tokens > gv::kFusedSortQuantizeMaxTokens;
+  const unsigned front = GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE;
+  const unsigned layer_body = front | GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU | GEVVA_MOE_STAGE_W2;
+  if ((stages & layer_body) == layer_body && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode &&
+      runner->decode_front && tokens <= gv::kFusedSortQuantizeMaxTokens && tokens <= sm_count) {
+    // decode-sized batch: sort, quantiser and both GEMMs in one persistent launch; the weights start
+    // streaming while the input is still being quantised
+    StageRange range(runner->nvtx, "gevva_moe.sort+quantize+w13+geglu+w2");
+    gv::launch_decode_layer(in, ids, runner->weights.in_scale_q1, tokens, s->input_codes, s->input_sf,
+                            runner->w13_fused, runner->w2, s->plan, sm_count, stream);
+    stages &= ~layer_body;
+  }
+  if ((stages & front) == front && tokens <= gv::kFusedSortQuantizeMaxTokens) {
+    // decode-sized batch: one launch does both
+    StageRange range(runner->nvtx, "gevva_moe.sort+quantize");
+    gv::launch_route_sort_quantize_small(in, ids, runner->weights.in_scale_q1, s->plan, tokens, s->input_codes,
+                                         s->input_sf, stream);
+  } else {
+    if (stages & GEVVA_MOE_STAGE_SORT) {
+      StageRange range(runner->nvtx, "gevva_moe.sort");
+      gv::launch_route_sort(ids, routes, s->plan, stream);
+    }
+    StageRange range(runner->nvtx && (stages & GEVVA_MOE_STAGE_QUANTIZE), "gevva_moe.quantize");
+    if (stages & GEVVA_MOE_STAGE_QUANTIZE)
+      gv::launch_quantize_input(in, ids, runner->weights.in_scale_q1, s->plan, tokens, s->input_codes,
+                                s->input_sf, stream);
+  }
+  const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
+  const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
+  if ((stages & gemms) == gemms && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode &&
+      tokens <= gv::kFusedSortQuantizeMaxTokens && (stages & front) == front) {
+    // decode-sized batch: both GEMMs in one persistent launch, weights streaming across the boundary
+    // (the readiness counters it needs are zeroed by the fused sort + quantise launch above)
+    StageRange range(runner->nvtx, "gevva_moe.w13+geglu+w2");
+    gv::launch_decode_experts(runner->w13_fused, runner->w2, s->plan, sm_count, stream);
+    stages &= ~gemms;
+  }
+  if ((stages & both) == both && !(stages & GEVVA_MOE_STAGE_UNFUSED)) {
+    // production path: GeGLU + requantise inside the w13 epilogue, no bf16 w13 output
+    StageRange range(runner->nvtx, "gevva_moe.w13+geglu");
+    if (runner->w13_pair_form && tokens > gv::kFusedSortQuantizeMaxTokens && s->plan.pair_tile &&
+        sm_count >= 2) {
+      gv::launch_w13_pairs(runner->w13_pairs, s->plan, sm_count, stream);
+    } else {
+      gv::GemmOperands w13 = runner->w13_fused;
+      w13.use_pairs = use_pairs;
+      gv::launch_grouped_gemm(w13, s->plan, sm_count, stream);
+    }
+  } else {
+    if (stages & GEVVA_MOE_STAGE_W13)
+      gv::launch_grouped_gemm(runner->w13, s->plan, sm_count, stream);
+    if (stages & GEVVA_MOE_STAGE_GEGLU)
+      gv::launch_geglu_quantize(s->w13_out, runner->weights.in_scale_q2, s->plan, routes,
+                                s->inter_codes, s->inter_sf, stream);
+  }
+  if (stages & GEVVA_MOE_STAGE_W2) {
+    StageRange range(runner->nvtx, "gevva_moe.w2");
+    gv::GemmOperands w2 = runner->w2;
+    w2.use_pairs = use_pairs;
+    gv::launch_grouped_gemm(w2, s->plan, sm_count, stream);
+  }
+  StageRange reduce_range(runner->nvtx && (stages & GEVVA_MOE_STAGE_REDUCE), "gevva_moe.reduce");
+  if (stages & GEVVA_MOE_STAGE_REDUCE)
+    gv::launch_reduce_routes(s->w2_out, route_weights, s->plan.inverse_routes, tokens, out, stream);
+  GV_CUDA(cudaGetLastError(), "moe launch");
+  return GEVVA_MOE_OK;
+}
+
 extern "C" {
 
 const char* gevva_moe_strerror(int status) {
@@ -470,81 +551,7 @@ int gevva_moe_launch_stages(gevva_moe* runner, const void* in, const int* ids,
                             const float* route_weights, void* out, int tokens, unsigned stages,
                             gevva_stream_t stream) {
   if (!runner) return GEVVA_MOE_BAD_ARGUMENT;
-  Scratch* s = runner->scratch;
-  // "expert runner token count exceeds its plan", src/nvfp4_cutlass.cu:1830-1832
-  if (tokens < 1 || tokens > s->max_tokens) return GEVVA_MOE_BAD_ARGUMENT;
-  if ((stages & (GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE)) && !ids) return GEVVA_MOE_BAD_ARGUMENT;
-  if ((stages & GEVVA_MOE_STAGE_QUANTIZE) && !in) return GEVVA_MOE_BAD_ARGUMENT;
-  if ((stages & GEVVA_MOE_STAGE_REDUCE) && (!out || !route_weights)) return GEVVA_MOE_BAD_ARGUMENT;
-  const int routes = tokens * kTopK;
-  // Decode-sized batches (at most a few rows per expert) stream weights and gain nothing from
-  // pairing two row tiles of an expert; they keep the one-CTA-per-tile kernel.
-  const bool use_pairs = runner->pairs && tokens > gv::kFusedSortQuantizeMaxTokens;
-  const unsigned front = GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE;
-  const unsigned layer_body = front | GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU | GEVVA_MOE_STAGE_W2;
-  if ((stages & layer_body) == layer_body && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode &&
-      runner->decode_front && tokens <= gv::kFusedSortQuantizeMaxTokens && tokens <= runner->sm_count) {
-    // decode-sized batch: sort, quantiser and both GEMMs in one persistent launch; the weights start
-    // streaming while the input is still being quantised
-    StageRange range(runner->nvtx, "gevva_moe.sort+quantize+w13+geglu+w2");
-    gv::launch_decode_layer(in, ids, runner->weights.in_scale_q1, tokens, s->input_codes, s->input_sf,
-                            runner->w13_fused, runner->w2, s->plan, runner->sm_count, stream);
-    stages &= ~layer_body;
-  }
-  if ((stages & front) == front && tokens <= gv::kFusedSortQuantizeMaxTokens) {
-    // decode-sized batch: one launch does both
-    StageRange range(runner->nvtx, "gevva_moe.sort+quantize");
-    gv::launch_route_sort_quantize_small(in, ids, runner->weights.in_scale_q1, s->plan, tokens, s->input_codes,
-                                         s->input_sf, stream);
-  } else {
-    if (stages & GEVVA_MOE_STAGE_SORT) {
-      StageRange range(runner->nvtx, "gevva_moe.sort");
-      gv::launch_route_sort(ids, routes, s->plan, stream);
-    }
-    StageRange range(runner->nvtx && (stages & GEVVA_MOE_STAGE_QUANTIZE), "gevva_moe.quantize");
-    if (stages & GEVVA_MOE_STAGE_QUANTIZE)
-      gv::launch_quantize_input(in, ids, runner->weights.in_scale_q1, s->plan, tokens, s->input_codes,
-                                s->input_sf, stream);
-  }
-  const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
-  const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
-  if ((stages & gemms) == gemms && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode &&
-      tokens <= gv::kFusedSortQuantizeMaxTokens && (stages & front) == front) {
-    // decode-sized batch: both GEMMs in one persistent launch, weights streaming across the boundary
-    // (the readiness counters it needs are zeroed by the fused sort + quantise launch above)
-    StageRange range(runner->nvtx, "gevva_moe.w13+geglu+w2");
-    gv::launch_decode_experts(runner->w13_fused, runner->w2, s->plan, runner->sm_count, stream);
-    stages &= ~gemms;
-  }
-  if ((stages & both) == both && !(stages & GEVVA_MOE_STAGE_UNFUSED)) {
-    // production path: GeGLU + requantise inside the w13 epilogue, no bf16 w13 output
-    StageRange range(runner->nvtx, "gevva_moe.w13+geglu");
-    if (runner->w13_pair_form && tokens > gv::kFusedSortQuantizeMaxTokens && s->plan.pair_tile &&
-        runner->sm_count >= 2) {
-      gv::launch_w13_pairs(runner->w13_pairs, s->plan, runner->sm_count, stream);
-    } else {
-      gv::GemmOperands w13 = runner->w13_fused;
-      w13.use_pairs = use_pairs;
-      gv::launch_grouped_gemm(w13, s->plan, runner->sm_count, stream);
-    }
-  } else {
-    if (stages & GEVVA_MOE_STAGE_W13)
-      gv::launch_grouped_gemm(runner->w13, s->plan, runner->sm_count, stream);
-    if (stages & GEVVA_MOE_STAGE_GEGLU)
-      gv::launch_geglu_quantize(s->w13_out, runner->weights.in_scale_q2, s->plan, routes,
-                                s->inter_codes, s->inter_sf, stream);
-  }
-  if (stages & GEVVA_MOE_STAGE_W2) {
-    StageRange range(runner->nvtx, "gevva_moe.w2");
-    gv::GemmOperands w2 = runner->w2;
-    w2.use_pairs = use_pairs;
-    gv::launch_grouped_gemm(w2, s->plan, runner->sm_count, stream);
-  }
-  StageRange reduce_range(runner->nvtx && (stages & GEVVA_MOE_STAGE_REDUCE), "gevva_moe.reduce");
-  if (stages & GEVVA_MOE_STAGE_REDUCE)
-    gv::launch_reduce_routes(s->w2_out, route_weights, s->plan.inverse_routes, tokens, out, stream);
-  GV_CUDA(cudaGetLastError(), "moe launch");
-  return GEVVA_MOE_OK;
+  return gv::moe_launch_stages_on(runner, in, ids, route_weights, out, tokens, stages, stream, runner->sm_count);
 }
 
 int gevva_moe_launch(gevva_moe* runner, const void* in, const int* ids, const float* route_weights,

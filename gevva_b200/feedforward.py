@@ -6,8 +6,8 @@ from dataclasses import dataclass
 
 import torch
 
-from .runtime import (EXPERTS, HIDDEN, TOP_K, GevvaMoeError, Nvfp4ExpertRunner, _check, _ptr,
-                      _stream_handle, _view, library, route_project)
+from .runtime import (HIDDEN, GevvaMoeError, Nvfp4ExpertRunner, _address, _check, _enqueue, _ptr, _stream_handle,
+                      _view, library)
 
 DENSE = 2112
 
@@ -15,6 +15,12 @@ DENSE = 2112
 class _DenseWeights(ctypes.Structure):
     _fields_ = [("gate_up", ctypes.c_void_p), ("down", ctypes.c_void_p), ("gate_scale", ctypes.c_float),
                 ("up_scale", ctypes.c_float), ("down_scale", ctypes.c_float)]
+
+
+class _Layer(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in
+                ("dense_pre", "expert_pre", "router_scale", "router_weight", "expert_scale", "dense_post",
+                 "expert_post", "combined_post", "layer_scalar", "experts", "dense")]
 
 
 def _lib():
@@ -34,6 +40,9 @@ def _lib():
     lib.gevva_dense_projection_scale.restype = vp
     lib.gevva_dense_buffer.argtypes = [vp, i32, ctypes.POINTER(vp), ctypes.POINTER(ctypes.c_size_t)]
     lib.gevva_pack_fp8.argtypes = [vp, ctypes.c_size_t, vp, vp, vp]
+    lib.gevva_ff_layer_workspace_bytes.argtypes = [i32]
+    lib.gevva_ff_layer_workspace_bytes.restype = ctypes.c_size_t
+    lib.gevva_ff_layer_launch.argtypes = [ctypes.POINTER(_Layer), vp, vp, vp, i32, vp, vp]
     lib._gv_ff_ready = True
     return lib
 
@@ -58,10 +67,9 @@ def ff_prepare(x, dense_weight, expert_weight, router_scale):
     rows = x.shape[0]
     _check(x, torch.bfloat16, (rows, HIDDEN), "input")
     outs = [torch.empty_like(x) for _ in range(3)]
-    with torch.cuda.device(x.device):
-        _status(_lib().gevva_ff_prepare(_ptr(x), _ptr(dense_weight), _ptr(expert_weight), _ptr(router_scale),
-                                        _ptr(outs[0]), _ptr(outs[1]), _ptr(outs[2]), rows,
-                                        _stream_handle(None)), "ff_prepare")
+    _status(_enqueue(_lib().gevva_ff_prepare, x.device, None, x.data_ptr(), _address(dense_weight),
+                     _address(expert_weight), _address(router_scale), outs[0].data_ptr(), outs[1].data_ptr(),
+                     outs[2].data_ptr(), rows), "ff_prepare")
     return outs  # dense_pre, expert_pre, router_input
 
 
@@ -72,11 +80,11 @@ def ff_finalize(dense, dense_weight, expert_routes, route_weights, inverse_route
     None), as the reference kernel takes them."""
     rows = dense.shape[0]
     out = torch.empty_like(residual)
-    with torch.cuda.device(dense.device):
-        _status(_lib().gevva_ff_finalize(
-            _ptr(dense), _ptr(dense_weight), _ptr(expert_routes), _ptr(route_weights), _ptr(inverse_routes),
-            _ptr(expert_weight), _ptr(combined_weight), _ptr(residual), _ptr(layer_scalar), _ptr(out), rows,
-            _ptr(dense_activation_scales), _ptr(dense_projection_scale), _stream_handle(None)), "ff_finalize")
+    _status(_enqueue(
+        _lib().gevva_ff_finalize, dense.device, None, _address(dense), _address(dense_weight), _address(expert_routes),
+        _address(route_weights), _address(inverse_routes), _address(expert_weight), _address(combined_weight),
+        _address(residual), _address(layer_scalar), _address(out), rows, _address(dense_activation_scales),
+        _address(dense_projection_scale)), "ff_finalize")
     return out
 
 
@@ -109,9 +117,8 @@ class DenseMlp:
         _check(x, torch.bfloat16, (tokens, HIDDEN), "input")
         if out is None:
             out = torch.empty_like(x)
-        with torch.cuda.device(self.device):
-            _status(_lib().gevva_dense_launch(self._handle, _ptr(x), _ptr(out), tokens, _stream_handle(stream)),
-                    "dense launch")
+        _status(_enqueue(_lib().gevva_dense_launch, self.device, stream, self._handle, x.data_ptr(), _address(out),
+                         tokens), "dense launch")
         scales = _view(_lib().gevva_dense_output_scales(self._handle), (tokens,), torch.int32,
                        self.device).view(torch.float32)
         return out, scales
@@ -142,19 +149,24 @@ class FeedForwardLayer:
     dense: DenseMlp
 
     def forward(self, hidden, aux_stream=None):
+        """The layer's output, a new tensor; with `aux_stream` the dense MLP runs there, beside the
+        experts.  One native call (gevva_ff_layer_launch) does all launches: called one by one from
+        Python they took 137 us of host time a layer, four times what the GPU needs for one token."""
         tokens = hidden.shape[0]
-        dense_in, expert_in, router_in = ff_prepare(hidden, self.dense_pre, self.expert_pre, self.router_scale)
-        weights, ids = route_project(router_in, self.router_w, self.expert_scale, status_of=self.experts)
-        main = torch.cuda.current_stream()
-        if aux_stream is not None:
-            aux_stream.wait_stream(main)
-            with torch.cuda.stream(aux_stream):
-                dense_out, dense_scales = self.dense.launch(dense_in)
-        else:
-            dense_out, dense_scales = self.dense.launch(dense_in)
-        self.experts.launch_batch_unreduced(expert_in, ids, tokens)
-        if aux_stream is not None:
-            main.wait_stream(aux_stream)
-        return ff_finalize(dense_out, self.dense_post, self.experts.routed_output(), weights,
-                           self.experts.inverse_routes(), self.expert_post, self.combined_post, hidden,
-                           self.layer_scalar, dense_scales, self.dense.projection_scale)
+        _check(hidden, torch.bfloat16, (tokens, HIDDEN), "input")
+        lib = _lib()
+        out = torch.empty_like(hidden)
+        workspace = torch.empty(lib.gevva_ff_layer_workspace_bytes(tokens), dtype=torch.uint8, device=hidden.device)
+        layer = _Layer(self.dense_pre.data_ptr(), self.expert_pre.data_ptr(), self.router_scale.data_ptr(),
+                       self.router_w.data_ptr(), self.expert_scale.data_ptr(), self.dense_post.data_ptr(),
+                       self.expert_post.data_ptr(), self.combined_post.data_ptr(), self.layer_scalar.data_ptr(),
+                       self.experts._handle, self.dense._handle)
+
+        def launch(main):
+            return lib.gevva_ff_layer_launch(ctypes.byref(layer), hidden.data_ptr(), out.data_ptr(),
+                                             workspace.data_ptr(), tokens, main,
+                                             main if aux_stream is None else aux_stream.cuda_stream)
+
+        _status(_enqueue(launch, hidden.device, None), "feed-forward layer")
+        self.experts._tokens = tokens
+        return out

@@ -88,6 +88,12 @@ def library():
     lib.gevva_moe_buffer.restype = i32
     lib.gevva_moe_pack_experts.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp]
     lib.gevva_moe_pack_experts.restype = i32
+    lib.gevva_moe_route_project.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, vp, vp]
+    lib.gevva_moe_route_project_fp8.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, vp]
+    lib.gevva_moe_status_word.argtypes = [vp]
+    lib.gevva_moe_status_word.restype = vp
+    lib.gevva_moe_route_sort_noalloc.argtypes = [vp, i32, vp, vp, vp, vp, vp, vp, vp]
+    lib.gevva_moe_route_sort_noalloc.restype = i32
     _lib = lib
     return lib
 
@@ -104,9 +110,34 @@ def _ptr(tensor):
     return ctypes.c_void_p(tensor.data_ptr()) if tensor is not None else ctypes.c_void_p(0)
 
 
+# The launch path of an eager decode step is host work (three launches take the GPU about 20 us), so
+# the helpers below do no more than they must: addresses travel as integers (the argtypes convert
+# them), the current stream is read as its handle instead of as a Stream object, and the current
+# device is switched only when it is another one.
+_current_device = torch._C._cuda_getDevice
+_current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
+def _address(tensor):
+    return tensor.data_ptr() if tensor is not None else None
+
+
+def _enqueue(function, device, stream, *args):
+    """function(*args, stream handle) with `device` current; stream None is the device's current one."""
+    index = device.index
+    if stream is None:
+        handle = _current_raw_stream(index)
+    else:
+        handle = stream if isinstance(stream, int) else stream.cuda_stream
+    if _current_device() == index:
+        return function(*args, handle)
+    with torch.cuda.device(device):
+        return function(*args, handle)
+
+
 def _check(tensor, dtype, shape, name):
-    if tensor.dtype != dtype or tuple(tensor.shape) != tuple(shape) or not tensor.is_contiguous() \
-            or not tensor.is_cuda:
+    if tensor.dtype is not dtype or tensor.shape != shape or not tensor.is_contiguous() or not tensor.is_cuda:
         raise ValueError(f"{name}: expected contiguous CUDA {dtype} {tuple(shape)}, got "
                          f"{tensor.dtype} {tuple(tensor.shape)} on {tensor.device}")
 
@@ -212,10 +243,8 @@ class Nvfp4ExpertRunner:
 
     # -- additions of this build ------------------------------------------------------
     def _launch(self, input, expert_ids, route_weights, output, tokens, stages, stream):
-        with torch.cuda.device(self._device):
-            status = library().gevva_moe_launch_stages(
-                self._handle, _ptr(input), _ptr(expert_ids), _ptr(route_weights), _ptr(output),
-                int(tokens), stages, _stream_handle(stream))
+        status = _enqueue(library().gevva_moe_launch_stages, self._device, stream, self._handle, _address(input),
+                          _address(expert_ids), _address(route_weights), _address(output), int(tokens), stages)
         if status != 0:
             raise GevvaMoeError(status, "launch")
         self._tokens = int(tokens)
@@ -260,11 +289,10 @@ def route_128_top8(logits, expert_scale, activation_scales=None, projection_weig
         weights = torch.empty((rows, TOP_K), dtype=torch.float32, device=logits.device)
     if ids is None:
         ids = torch.empty((rows, TOP_K), dtype=torch.int32, device=logits.device)
-    with torch.cuda.device(logits.device):
-        status = library().gevva_moe_route(
-            _ptr(logits), int(logits.stride(0)) if rows > 1 else max(int(logits.stride(0)), EXPERTS),
-            _ptr(expert_scale), _ptr(weights), _ptr(ids), rows, _ptr(activation_scales),
-            _ptr(projection_weight_scale), _stream_handle(stream))
+    ld = logits.stride(0)
+    status = _enqueue(library().gevva_moe_route, logits.device, stream, logits.data_ptr(),
+                      ld if rows > 1 else max(ld, EXPERTS), expert_scale.data_ptr(), weights.data_ptr(),
+                      ids.data_ptr(), rows, _address(activation_scales), _address(projection_weight_scale))
     if status != 0:
         raise GevvaMoeError(status, "route_128_top8")
     return weights, ids
@@ -292,22 +320,16 @@ def route_project(router_input, router_weight, expert_scale, bias=None, want_log
         ids = torch.empty((rows, TOP_K), dtype=torch.int32, device=device)
     logits = torch.empty((rows, EXPERTS), dtype=torch.bfloat16, device=device) if want_logits else None
     lib = library()
-    vp, i32 = ctypes.c_void_p, ctypes.c_int
-    lib.gevva_moe_route_project.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, vp, vp]
-    lib.gevva_moe_route_project_fp8.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, vp]
-    lib.gevva_moe_status_word.argtypes = [vp]
-    lib.gevva_moe_status_word.restype = vp
-    status_word = vp(lib.gevva_moe_status_word(status_of._handle)) if status_of is not None else vp(0)
-    with torch.cuda.device(device):
-        if fp8:
-            status = lib.gevva_moe_route_project_fp8(
-                _ptr(router_input), _ptr(activation_scales), _ptr(router_weight), _ptr(weight_scale),
-                _ptr(expert_scale), _ptr(weights), _ptr(ids), _ptr(logits), rows, status_word,
-                _stream_handle(stream))
-        else:
-            status = lib.gevva_moe_route_project(
-                _ptr(router_input), _ptr(router_weight), _ptr(bias), _ptr(expert_scale), _ptr(weights),
-                _ptr(ids), _ptr(logits), rows, status_word, _stream_handle(stream))
+    status_word = lib.gevva_moe_status_word(status_of._handle) if status_of is not None else None
+    if fp8:
+        status = _enqueue(lib.gevva_moe_route_project_fp8, device, stream, router_input.data_ptr(),
+                          activation_scales.data_ptr(), router_weight.data_ptr(), _address(weight_scale),
+                          expert_scale.data_ptr(), weights.data_ptr(), ids.data_ptr(), _address(logits), rows,
+                          status_word)
+    else:
+        status = _enqueue(lib.gevva_moe_route_project, device, stream, router_input.data_ptr(),
+                          router_weight.data_ptr(), _address(bias), expert_scale.data_ptr(), weights.data_ptr(),
+                          ids.data_ptr(), _address(logits), rows, status_word)
     if status != 0:
         raise GevvaMoeError(status, "route_project")
     return (weights, ids, logits) if want_logits else (weights, ids)
@@ -340,9 +362,6 @@ def route_sort_noalloc(expert_ids, stream=None):
     sorted_experts, sorted_routes, inverse_routes [8*tokens]; expert_offsets,
     scale_row_offsets [129]; status [1] (1 if an id was outside [0,128))."""
     lib = library()
-    vp = ctypes.c_void_p
-    lib.gevva_moe_route_sort_noalloc.argtypes = [vp, ctypes.c_int, vp, vp, vp, vp, vp, vp, vp]
-    lib.gevva_moe_route_sort_noalloc.restype = ctypes.c_int
     tokens = expert_ids.shape[0]
     _check(expert_ids, torch.int32, (tokens, TOP_K), "expert_ids")
     device = expert_ids.device

@@ -325,6 +325,30 @@ const float* gevva_dense_projection_scale(const gevva_dense* dense);
 /* stage buffers for parity tests: 0 input e4m3, 1 input scales, 2 gate|up bf16 unscaled,
  * 3 product e4m3, 4 product scales */
 int gevva_dense_buffer(const gevva_dense* dense, int which, void** device_ptr, size_t* bytes);
+/* One whole feed-forward layer (the wiring of src/cuda/runtime/prefill.cuh:1200-1250) in one call:
+ * gevva_ff_prepare, gevva_moe_route_project, the experts unreduced, the dense MLP and
+ * gevva_ff_finalize.  The dense MLP runs on `aux_stream`, forked from and joined to `stream` by
+ * events, and shares the SMs with the expert kernels; aux_stream == stream runs everything in
+ * order on one stream.  Same bits as the five calls.  `workspace` is device memory of at least
+ * gevva_ff_layer_workspace_bytes(tokens) bytes, 256-byte aligned, used until `stream` has passed the
+ * call; every weight pointer is bf16 as in the calls above. */
+typedef struct {
+  const void* dense_pre;
+  const void* expert_pre;
+  const void* router_scale;
+  const void* router_weight;
+  const void* expert_scale;
+  const void* dense_post;
+  const void* expert_post;
+  const void* combined_post;
+  const void* layer_scalar;
+  gevva_moe* experts;
+  gevva_dense* dense;
+} gevva_ff_layer;
+size_t gevva_ff_layer_workspace_bytes(int tokens);
+int gevva_ff_layer_launch(const gevva_ff_layer* layer, const void* hidden, void* out, void* workspace,
+                          int tokens, gevva_stream_t stream, gevva_stream_t aux_stream);
+
 /* Per-tensor FP8 quantiser (tools/pack_fp8_dense.py:64-70): scale = amax/448, q = e4m3(w/scale). */
 int gevva_pack_fp8(const float* weights, size_t count, void* out, float* scale, gevva_stream_t stream);
 

@@ -196,3 +196,29 @@ def test_thirty_layers_captured_into_one_graph_at_verifier_size(cuda_device):
     assert torch.equal(static_out, want_second)
     for layer in stack.layers:
         layer.experts.check()
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 128, 129, 301])
+def test_layer_call_equals_its_parts(cuda_device, tokens):
+    """gevva_ff_layer_launch against the calls it stands for, made one by one: the same bits, on one
+    stream and with the dense MLP on a second one, on both sides of the size (128 tokens) up to which
+    the dense MLP and the experts share the SMs."""
+    from gevva_b200 import feedforward as ff
+    from gevva_b200.runtime import route_project
+    from gevva_b200.synthetic import SyntheticStack
+    stack = SyntheticStack(1, 512, cuda_device, seed=5)
+    layer = stack.layers[0]
+    hidden = hashgen.activations(tokens, HIDDEN, 21 + tokens, cuda_device)
+    dense_in, expert_in, router_in = ff.ff_prepare(hidden, layer.dense_pre, layer.expert_pre, layer.router_scale)
+    weights, ids = route_project(router_in, layer.router_w, layer.expert_scale, status_of=layer.experts)
+    dense_out, dense_scales = layer.dense.launch(dense_in)
+    layer.experts.launch_batch_unreduced(expert_in, ids, tokens)
+    want = ff.ff_finalize(dense_out, layer.dense_post, layer.experts.routed_output(), weights,
+                          layer.experts.inverse_routes(), layer.expert_post, layer.combined_post, hidden,
+                          layer.layer_scalar, dense_scales, layer.dense.projection_scale)
+    for aux in (None, torch.cuda.Stream(device=cuda_device)):
+        for _ in range(2):
+            got = layer.forward(hidden, aux)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    layer.experts.check()
