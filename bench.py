@@ -155,6 +155,8 @@ def launches_per_step(world, tokens, sm_count=148, ep_chunks=2, ep_parts=1):
     if world == 1:
         if tokens <= 128:
             return 1 + 1 + 1          # fused router; sort, quantiser and both expert GEMMs in one launch; reduce
+        if tokens <= 640:
+            return 1 + sort + 1 + 2   # fused router; sort; quantise; both expert GEMMs in one launch; reduce
         return 1 + sort + 1 + 3       # fused router; sort; quantise; w13, w2, reduce
     # fused router; sort + count exchange (with the first barrier inside); dispatch, row destinations;
     # scale re-tiling (waits for every rank's rows) + (w13, w2) per compute part; reduce; one flag barrier

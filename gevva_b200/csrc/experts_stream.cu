@@ -1,0 +1,791 @@
+// Both expert GEMMs of a batch with few rows an expert, in one persistent launch that streams weights.
+//
+// What bounds it.  Every routed expert's 3.3 MB come from HBM once: 65 us of it when all 128 experts are
+// hit, whatever the batch; with a handful of tokens the time is the chain sort -> quantise -> w13 ->
+// GeGLU -> w2.  So the weights sit on MMA-M (128 rows a tile, all of them real) and the rows of an
+// expert on MMA-N, in multiples of 16: an MMA of 16 rows takes a sixteenth of the tensor time of the
+// 128 x 256 form with its padded row tile, a pipeline stage carries 18 KB of weights instead of 34 and is
+// held for that much shorter, and a w13 item is 64 intermediate columns (11 an expert, 180 KB), so one
+// token's eight experts keep 88 SMs busy instead of 48.
+//
+//   w13 item   (chunk of at most 64 rows of an expert) x (unit of 64 intermediate columns): MMA rows 0..63
+//              are the unit's up rows, 64..127 its gate rows (one 3-D box brings both; their scales come
+//              from a copy re-tiled by unit, made at runner creation)
+//   w2 item    (chunk) x (128 output columns)
+// One list per launch, all w13 items chunk by chunk, then all w2 items; dealt round-robin, the w2 part
+// so that the CTAs that are one w13 item short (180 KB) get four w2 items (48 KB each) first.
+//
+// Roles (13 warps): 0 fetches weights, 1 issues MMAs, 2 fetches activations, 3 copies scale factors to
+// tensor memory one stage ahead, 4..11 are the epilogue (two warps per 32-lane quarter, alternating
+// groups of eight rows), 12 publishes finished w13 items.  Seven stages of one K block (256 elements); four accumulators of 64 columns,
+// so nothing waits for a drain.  In the w13 epilogue a thread holds one weight row for eight tokens, so
+// bf16(alpha * acc), which is what the reference's GEMM stores, changes hands through shared memory and a
+// thread then owns one column of a token: GeGLU, block maximum over sixteen lanes, codes.  The w2
+// epilogue pairs two columns by one shuffle per two tokens and stores 64-byte pieces of a row.
+//
+// A w2 item needs the w2 operand rows of its expert: when the epilogue warps have stored an item, a
+// publisher warp adds one to the expert's counter (release); the activation side of a w2 item waits for
+// 11 x chunks of them (bounded acquire spin), crosses to the async proxy and loads.  The weight side
+// waits for nothing, so weight bytes keep arriving across the boundary.  All CTAs are co-resident (one per
+// SM) and no wait can form a cycle.
+//
+// In its kFront form (at most 128 tokens) the kernel also sorts the routes and quantises the input: every
+// CTA counts the batch's at most 1024 routes and derives the group geometry for itself; CTA t < tokens
+// ranks the routes of token t and quantises it with eleven warps, eight columns a thread (88 threads of
+// 32 columns took 4.3 us of the chain, this takes about one), then adds one to a counter that the
+// activation side waits for.  Meanwhile the weight side has filled its stages.  The CTA that finishes last
+// puts all counters back to zero.
+#include "gv_common.cuh"
+#include "gv_gemm_parts.cuh"
+#include "gv_launchers.h"
+#include "gv_quantize.cuh"
+
+namespace gv {
+
+namespace {
+
+constexpr int kStStages = 7;
+constexpr int kStRows = 64;                               // rows of a chunk at most (MMA-N)
+constexpr int kStAccStages = 4;
+constexpr int kStWeightWarp = 0, kStMmaWarp = 1, kStTokenWarp = 2, kStScaleWarp = 3, kStEpilogueWarp = 4;
+constexpr int kStEpilogueWarps = 8;
+constexpr int kStPublishWarp = kStEpilogueWarp + kStEpilogueWarps;     // 12
+constexpr int kStThreads = (kStPublishWarp + 1) * 32;                  // 416
+constexpr int kStQuantiseThreads = kStThreads - 64;       // warps 1..11: 352 = 2816 / 8
+static_assert(kStQuantiseThreads * 8 == kHidden, "eight columns a thread");
+constexpr uint32_t kStTmemColumns = 512;
+constexpr uint32_t kStSfColumn = kStAccStages * kStRows;  // 256
+constexpr uint32_t kStSfColumnsPerStage = 32;             // 16 for the weights, 16 for the rows
+static_assert(kStSfColumn + kStSfColumnsPerStage * kStStages <= kStTmemColumns, "tensor memory budget");
+constexpr int kStWeightBytes = kTileM * kTileKBytes;      // 16 KiB
+constexpr int kStTokenBytes = kStRows * kTileKBytes;      // 8 KiB
+constexpr int kStUnits = kInter / 64;                     // 11 w13 items a chunk
+constexpr int kStUnitSlots = kStUnits + 1;                // the re-tiled scales keep 12 per expert
+constexpr int kStDownTiles = kHidden / 128;               // 22 w2 items a chunk
+constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
+constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192
+constexpr int kStDownLastMmas = 3;
+constexpr int kStMaxChunks = 384;
+constexpr int kStExchangeRows = 32;
+
+struct alignas(1024) StreamSmem {
+  uint8_t a[kStStages][kStWeightBytes];
+  uint8_t b[kStStages][kStTokenBytes];
+  uint8_t sfa[kStStages][kSfStageBytes];
+  uint8_t sfb[kStStages][kSfStageBytes];
+  __nv_bfloat16 exchange[2][kStExchangeRows][128];  // [token][MMA row]
+  uint64_t full[kStStages], empty[kStStages], sf_full[kStStages];
+  uint64_t acc_full[kStAccStages], acc_empty[kStAccStages];
+  volatile int progress[kStEpilogueWarps];  // w13 items whose rows each epilogue warp has stored
+  uint32_t tmem_base;
+  volatile int abort;
+  volatile int left;  // an epilogue warp gave up waiting
+  int last;           // this CTA is the last one to finish
+  int chunks;
+  int offsets[kExperts + 1];
+  int scale_rows[kExperts + 1];
+  int chunks_of[kExperts];
+  short chunk_expert[kStMaxChunks];
+  short chunk_index[kStMaxChunks];  // which chunk of its expert
+  int histogram[kExperts];
+  int own_expert[kTopK];
+  int own_rank[kTopK];
+  alignas(16) int route_row[kTopK];
+  alignas(16) float route_multiplier[kTopK];
+  unsigned long long route_scale_base[kTopK];
+  float scale_q1[kExperts];
+  alignas(16) float erf_table[GV_ERF_TABLE_FLOATS];
+};
+constexpr size_t kStSmemBytes = sizeof(StreamSmem) + 1024;
+static_assert(kStSmemBytes <= 232448, "shared memory budget of one sm_100 CTA");
+
+struct StreamMaps {
+  CUtensorMap w13;                 // [256 halves, 704 rows, 1408 bytes], box 2 x 64 rows x 128 bytes
+  CUtensorMap w2;                  // [128 * 2816 rows, 352 bytes], box 128 rows x 128 bytes
+  CUtensorMap up[kStRows / 8];     // input codes through boxes of 8, 16, ... 64 rows x 128 bytes
+  CUtensorMap down[kStRows / 8];   // w2 operand codes likewise
+};
+
+struct StreamParams {
+  RoutePlan plan;
+  const uint8_t* w13_scales;  // re-tiled by unit
+  const uint8_t* w2_scales;   // sidecar layout
+  const uint8_t* input_scales;
+  uint8_t* inter_codes;
+  uint8_t* inter_scales;
+  __nv_bfloat16* routed;
+  const float *alpha1, *alpha2, *in_scale_q2;
+  // kFront only
+  const __nv_bfloat16* input;
+  const int* expert_ids;
+  const float* in_scale_q1;
+  uint8_t* packed;
+  uint8_t* scales;
+  int tokens;
+};
+
+struct StreamItem {
+  bool down;
+  int expert;
+  int chunk;   // of the expert
+  int n_tile;  // unit of 64 intermediate columns, or tile of 128 output columns
+};
+
+// This CTA's items in order.
+struct StreamSchedule {
+  int up_count, count;
+  int first_extra, lacking, pre;  // w2: CTAs >= first_extra are one w13 item short and take `pre` items first
+  __device__ StreamSchedule(int chunks) {
+    const int ctas = gridDim.x, cta = blockIdx.x;
+    const int up = chunks * kStUnits, down = chunks * kStDownTiles;
+    up_count = up > cta ? (up - 1 - cta) / ctas + 1 : 0;
+    first_extra = up % ctas;
+    lacking = first_extra == 0 ? 0 : ctas - first_extra;
+    pre = lacking > 0 && down >= 4 * lacking + 4 * ctas ? 4 : 0;  // a short list is spread evenly instead
+    const int rest = down - pre * lacking;
+    const int turn = cta >= first_extra ? cta - first_extra : cta - first_extra + ctas;  // lacking CTAs come first
+    const int mine = (cta >= first_extra ? pre : 0) + (rest > turn ? (rest - 1 - turn) / ctas + 1 : 0);
+    count = up_count + mine;
+  }
+  __device__ __forceinline__ StreamItem item(int i, const StreamSmem* smem) const {
+    const int ctas = gridDim.x, cta = blockIdx.x;
+    StreamItem it;
+    int index, per_chunk;
+    it.down = i >= up_count;
+    if (!it.down) {
+      index = cta + i * ctas;
+      per_chunk = kStUnits;
+    } else {
+      int k = i - up_count;
+      const bool is_short = cta >= first_extra;
+      const int turn = is_short ? cta - first_extra : cta - first_extra + ctas;
+      if (is_short && k < pre) {
+        index = turn + k * lacking;
+      } else {
+        if (is_short) k -= pre;
+        index = pre * lacking + turn + k * ctas;
+      }
+      per_chunk = kStDownTiles;
+    }
+    const int chunk = index / per_chunk;
+    it.n_tile = index - chunk * per_chunk;
+    it.expert = smem->chunk_expert[chunk];
+    it.chunk = smem->chunk_index[chunk];
+    return it;
+  }
+};
+
+__device__ __forceinline__ void stream_load_3d(void* smem_dst, const void* tensor_map, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(tensor_map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_load_32x8(uint32_t tmem_address, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(tmem_address)
+               : "memory");
+}
+
+// The MMAs of one K block (K = 64 each) with a runtime instruction descriptor (its N field).  Scale
+// columns of the stage: weights of MMA j at +4j; rows at +16 + 4j, plus two where the chunk is the second
+// half of its 128-row scale atom.
+template <int kMmas>
+__device__ __forceinline__ void stream_mmas(uint32_t tmem_acc, uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t a_lo,
+                                            uint32_t b_lo, uint32_t descriptor, uint32_t accumulate) {
+  constexpr uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // 8 rows x 128 B groups, 128B swizzle
+#pragma unroll
+  for (int j = 0; j < kMmas; ++j) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 d0, d1;\n\t"
+        "setp.ne.b32 p, %7, 0;\n\t"
+        "mov.b64 d0, {%1, %3};\n\t"
+        "mov.b64 d1, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], d0, d1, %4, [%5], [%6], p;\n\t}" ::"r"(tmem_acc),
+        "r"(a_lo + 2 * j), "r"(b_lo + 2 * j), "r"(hi), "r"(descriptor), "r"(tmem_sfa + 4 * j), "r"(tmem_sfb + 4 * j),
+        "r"(j == 0 ? accumulate : 1u)
+        : "memory");
+  }
+}
+
+__device__ __forceinline__ int stream_load_acquire(const int* address) {
+  int value;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(value) : "l"(address) : "memory");
+  return value;
+}
+
+// Bounded acquire spin of a whole warp on a counter in global memory.
+__device__ __forceinline__ bool stream_wait_counter(const int* counter, int target, StreamSmem* smem, int* status) {
+  const long long start = clock64();
+  bool ready = false;
+  for (uint32_t spin = 1; !ready; ++spin) {
+    ready = stream_load_acquire(counter) >= target;
+    if (!ready && (spin & 63u) == 0) {
+      if (smem->abort) break;
+      if (clock64() - start > kWaitLimitCycles) {
+        smem->abort = 1;
+        atomicExch(status, static_cast<int>(kWaitTimeout));
+        break;
+      }
+    }
+  }
+  return __all_sync(0xffffffffu, ready);
+}
+
+// This CTA's token by 352 threads, eight columns each (`raw`; two threads a 16-value block): the codes and
+// scale bytes of its eight routes go to their sorted rows.  The arithmetic of quantize_routes_of_token.
+__device__ __forceinline__ void stream_quantise_token(const StreamParams& p, const StreamSmem* smem, int q, const uint4& raw) {
+  float values[8];
+  unpack_bf16x8(raw, values);
+  float maximum = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) maximum = fmaxf(maximum, fabsf(values[i]));
+  maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, 1));
+  // scale groups q/2 of a row, four to an aligned word of the swizzled layout: eight threads a word
+  const uint32_t scale_offset = static_cast<uint32_t>(q >> 3) * kSfAtomBytes;
+  uint32_t codes = 0, scale_word = 0, previous = 0;
+  bool have = false;
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k) {
+    const int row = smem->route_row[k];
+    if (row < 0) continue;
+    const float multiplier = smem->route_multiplier[k];
+    if (!have || __float_as_uint(multiplier) != previous) {  // routes of equal static scale share the result
+      have = true;
+      previous = __float_as_uint(multiplier);
+      const uint32_t scale = encode_e4m3(__fdiv_rn(__fmul_rn(multiplier, maximum), 6.0f));
+      const float rounded = decode_e4m3(scale);
+      const float inverse = rounded == 0.0f ? 0.0f : __fdiv_rn(multiplier, rounded);
+      codes = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        codes |= encode_e2m1x2(__fmul_rn(values[2 * i], inverse), __fmul_rn(values[2 * i + 1], inverse)) << (8 * i);
+      scale_word = scale | (__shfl_down_sync(0xffffffffu, scale, 2) << 8) | (__shfl_down_sync(0xffffffffu, scale, 4) << 16) |
+                   (__shfl_down_sync(0xffffffffu, scale, 6) << 24);
+    }
+    *reinterpret_cast<uint32_t*>(p.packed + static_cast<size_t>(row) * (kHidden / 2) + 4 * q) = codes;
+    if ((q & 7) == 0) *reinterpret_cast<uint32_t*>(p.scales + smem->route_scale_base[k] + scale_offset) = scale_word;
+  }
+}
+
+template <bool kFront>
+__global__ void __launch_bounds__(kStThreads, 1)
+stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  StreamSmem* smem =
+      reinterpret_cast<StreamSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5;
+  const int lane = tid & 31;
+  const int cta = blockIdx.x;
+  int* const status = p.plan.status;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStStages; ++s) {
+      mbar_init(&smem->full[s], 2);  // one arrival (with its byte count) per producer warp
+      mbar_init(&smem->empty[s], 1);
+      mbar_init(&smem->sf_full[s], 1);
+    }
+    for (int s = 0; s < kStAccStages; ++s) {
+      mbar_init(&smem->acc_full[s], 1);
+      mbar_init(&smem->acc_empty[s], kStEpilogueWarps);
+    }
+    for (int w = 0; w < kStEpilogueWarps; ++w) smem->progress[w] = 0;
+    smem->abort = 0;
+    smem->left = 0;
+    fence_barrier_init();
+    prefetch_tensor_map(&maps.w13);
+    prefetch_tensor_map(&maps.w2);
+    prefetch_tensor_map(&maps.up[0]);
+    prefetch_tensor_map(&maps.down[0]);
+  }
+  if (warp == kStMmaWarp) {
+    tmem_alloc(&smem->tmem_base, kStTmemColumns);
+    tmem_relinquish();
+  }
+  load_erf_table(smem->erf_table);
+  if (kFront && tid < kExperts) smem->histogram[tid] = 0;
+  if (kFront && tid < kTopK) smem->own_rank[tid] = 0;
+  grid_launch_dependents();
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = smem->tmem_base;
+  grid_dependency_wait();  // what earlier kernels of the stream wrote is visible from here on
+
+  // ---------------- group geometry ----------------
+  const bool has_token = kFront && cta < p.tokens;
+  uint4 raw = make_uint4(0, 0, 0, 0);
+  if constexpr (kFront) {
+    const int routes = p.tokens * kTopK;
+    int mine[kTopK];
+    // the token itself and the static scales are on their way while the geometry is worked out
+    if (has_token && tid >= 32 && tid < 32 + kStQuantiseThreads)
+      raw = __ldg(reinterpret_cast<const uint4*>(p.input + static_cast<size_t>(cta) * kHidden) + (tid - 32));
+    if (has_token && tid < kExperts) smem->scale_q1[tid] = p.in_scale_q1[tid];
+    if (has_token) {
+#pragma unroll
+      for (int k = 0; k < kTopK; ++k) mine[k] = p.expert_ids[cta * kTopK + k];
+      if (tid < kTopK) smem->own_expert[tid] = p.expert_ids[cta * kTopK + tid];
+    }
+    for (int route = tid; route < routes; route += kStThreads) {
+      const int expert = p.expert_ids[route];
+      if (expert < 0 || expert >= kExperts) {
+        if (cta == 0) atomicExch(status, static_cast<int>(kBadExpertId));
+        continue;
+      }
+      atomicAdd(&smem->histogram[expert], 1);
+      if (has_token) {
+#pragma unroll
+        for (int k = 0; k < kTopK; ++k)
+          if (expert == mine[k] && route < cta * kTopK + k) atomicAdd(&smem->own_rank[k], 1);
+      }
+    }
+  } else {
+    if (tid < kExperts) smem->histogram[tid] = p.plan.expert_offsets[tid + 1] - p.plan.expert_offsets[tid];
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // lane l scans experts 4l..4l+3: rows, 128-row scale tiles, chunks
+    int counts[4], rows = 0, tiles = 0, chunks = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      counts[i] = smem->histogram[4 * lane + i];
+      rows += counts[i];
+      tiles += (counts[i] + kTileM - 1) / kTileM;
+      chunks += (counts[i] + kStRows - 1) / kStRows;
+    }
+    int rows_inclusive = rows, tiles_inclusive = tiles, chunks_inclusive = chunks;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const int r = __shfl_up_sync(0xffffffffu, rows_inclusive, offset);
+      const int t = __shfl_up_sync(0xffffffffu, tiles_inclusive, offset);
+      const int c = __shfl_up_sync(0xffffffffu, chunks_inclusive, offset);
+      if (lane >= offset) {
+        rows_inclusive += r;
+        tiles_inclusive += t;
+        chunks_inclusive += c;
+      }
+    }
+    int row = rows_inclusive - rows, tile = tiles_inclusive - tiles, chunk = chunks_inclusive - chunks;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int expert = 4 * lane + i;
+      const int expert_tiles = (counts[i] + kTileM - 1) / kTileM;
+      const int expert_chunks = (counts[i] + kStRows - 1) / kStRows;
+      smem->offsets[expert] = row;
+      smem->scale_rows[expert] = tile * kTileM;
+      smem->chunks_of[expert] = expert_chunks;
+      for (int c = 0; c < expert_chunks; ++c) {
+        smem->chunk_expert[chunk + c] = static_cast<short>(expert);
+        smem->chunk_index[chunk + c] = static_cast<short>(c);
+      }
+      if (kFront && cta == 0) {
+        p.plan.expert_offsets[expert] = row;
+        p.plan.scale_row_offsets[expert] = tile * kTileM;
+        for (int t = 0; t < expert_tiles; ++t) p.plan.tile_expert[tile + t] = expert;
+      }
+      row += counts[i];
+      tile += expert_tiles;
+      chunk += expert_chunks;
+    }
+    if (lane == 31) {
+      smem->offsets[kExperts] = row;
+      smem->scale_rows[kExperts] = tile * kTileM;
+      smem->chunks = chunk;
+      if (kFront && cta == 0) {
+        p.plan.expert_offsets[kExperts] = row;
+        p.plan.scale_row_offsets[kExperts] = tile * kTileM;
+        p.plan.num_m_tiles[0] = tile;
+      }
+    }
+  }
+  __syncthreads();
+  const StreamSchedule schedule(smem->chunks);
+  bool ok = true;
+
+  if (has_token && warp != kStWeightWarp && warp != kStPublishWarp) {
+    // ---------------- this CTA's token: its routes' rows, then its codes ----------------
+    const int q = tid - 32;
+    if (q < kTopK) {
+      const int route = cta * kTopK + q;
+      const int expert = smem->own_expert[q];
+      int dst = -1;
+      if (expert >= 0 && expert < kExperts) {  // others are flagged above
+        dst = smem->offsets[expert] + smem->own_rank[q];
+        p.plan.sorted_experts[dst] = expert;
+        p.plan.sorted_routes[dst] = route;
+        p.plan.inverse_routes[route] = dst;
+        smem->route_multiplier[q] = smem->scale_q1[expert];
+        smem->route_scale_base[q] = static_cast<unsigned long long>(smem->scale_rows[expert]) * (kHidden / 16) +
+                                    sf_offset(smem->own_rank[q], 0, kHidden / 16);
+      }
+      smem->route_row[q] = dst;
+    }
+    named_barrier(1, kStQuantiseThreads);
+    stream_quantise_token(p, smem, q, raw);
+    named_barrier(1, kStQuantiseThreads);
+    if (q == 0) {
+      __threadfence();
+      atomicAdd(p.plan.front_sync, 1);
+    }
+  }
+
+  if (warp == kStWeightWarp || warp == kStTokenWarp) {
+    // ---------------- producers ----------------
+    const bool weight_side = warp == kStWeightWarp;
+    int stage = 0, issued = 0;
+    uint32_t phase = 0;
+    if (kFront && !weight_side) {
+      // the w13 operand exists once every token's CTA has quantised its token and counted itself
+      ok = stream_wait_counter(p.plan.front_sync, p.tokens, smem, status);
+      asm volatile("fence.proxy.async.global;" ::: "memory");
+    }
+    for (int i = 0; ok && i < schedule.count; ++i) {
+      const StreamItem it = schedule.item(i, smem);
+      const int k_blocks = it.down ? kStDownKBlocks : kStUpKBlocks;
+      const int first = it.chunk * kStRows;
+      const int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
+      const int boxes = rows >= kStRows ? kStRows / 8 : (rows + 7) / 8;
+      const int row = smem->offsets[it.expert] + first;
+      const uint8_t* sf;
+      if (weight_side) {
+        sf = it.down ? p.w2_scales + static_cast<size_t>(it.expert * kHidden + it.n_tile * 128) * (kInter / 16)
+                     : p.w13_scales + static_cast<size_t>(it.expert * kStUnitSlots + it.n_tile) * kStUpKBlocks * kSfStageBytes;
+      } else {
+        const size_t scale_row = smem->scale_rows[it.expert] + first / kTileM * kTileM;
+        sf = it.down ? p.inter_scales + scale_row * (kInter / 16) : p.input_scales + scale_row * (kHidden / 16);
+        if (it.down) {
+          // the rows exist once every w13 item of the expert has been counted; they were written by ordinary stores of other SMs and are read through the async proxy
+          ok = stream_wait_counter(p.plan.tile_ready + it.expert, kStUnits * smem->chunks_of[it.expert], smem, status);
+          if (!ok) break;
+          asm volatile("fence.proxy.async.global;" ::: "memory");
+        }
+      }
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, status));
+        if (!ok) break;
+        if (elect_one()) {
+          const uint32_t sf_bytes = static_cast<uint32_t>(it.down && kb + 1 == k_blocks ? kStDownLastMmas : 4) * kSfAtomBytes;
+          const int x = kb * kTileKBytes;
+          uint64_t* bar = &smem->full[stage];
+          if (weight_side) {
+            mbar_arrive_expect_tx(bar, kStWeightBytes + sf_bytes);
+            if (it.down) tma_load_2d(smem->a[stage], &maps.w2, bar, x, it.expert * kHidden + it.n_tile * 128);
+            else stream_load_3d(smem->a[stage], &maps.w13, bar, x, it.n_tile * 64, 2 * it.expert);
+            bulk_load_1d(smem->sfa[stage], sf + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes, bar);
+          } else {
+            mbar_arrive_expect_tx(bar, static_cast<uint32_t>(boxes * 8 * kTileKBytes) + sf_bytes);
+            tma_load_2d(smem->b[stage], it.down ? &maps.down[boxes - 1] : &maps.up[boxes - 1], bar, x, row);
+            bulk_load_1d(smem->sfb[stage], sf + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes, bar);
+          }
+        }
+        __syncwarp();
+        ++issued;
+        if (++stage == kStStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    if (!ok && lane == 0) {
+      // unwinding: the copies already issued land before shared memory is given up
+      const int pending = issued < kStStages ? issued : kStStages;
+      for (int i = 0; i < pending; ++i) {
+        if (--stage < 0) {
+          stage = kStStages - 1;
+          phase ^= 1u;
+        }
+        mbar_wait_bounded(&smem->full[stage], phase, 40000000ll);
+      }
+    }
+  } else if (warp == kStMmaWarp) {
+    // ---------------- MMA issuer ----------------
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    const uint32_t a_lo0 = (smem_u32(smem->a[0]) & 0x3ffffu) >> 4;
+    const uint32_t b_lo0 = (smem_u32(smem->b[0]) & 0x3ffffu) >> 4;
+    const bool leader = elect_one();
+    for (int i = 0; ok && i < schedule.count; ++i) {
+      const StreamItem it = schedule.item(i, smem);
+      const int k_blocks = it.down ? kStDownKBlocks : kStUpKBlocks;
+      const int first = it.chunk * kStRows;
+      int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
+      rows = rows > kStRows ? kStRows : rows;
+      // E2M1 x E2M1, both K-major, UE4M3 scales, M = 128; N = the rows in multiples of 16
+      const uint32_t descriptor = (1u << 7) | (1u << 10) | (static_cast<uint32_t>((rows + 15) / 16 * 2) << 17) |
+                                  (static_cast<uint32_t>(kTileM >> 4) << 24);
+      const uint32_t half = (first % kTileM) / 32;
+      if (!__all_sync(0xffffffffu, wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, status))) break;
+      tc_fence_after_sync();
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        ok = wait_or_abort<false>(&smem->sf_full[stage], phase, smem, status);
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (leader) {
+          const uint32_t sf = tmem_base + kStSfColumn + kStSfColumnsPerStage * stage;
+          const uint32_t a_lo = a_lo0 + static_cast<uint32_t>(stage) * (kStWeightBytes >> 4);
+          const uint32_t b_lo = b_lo0 + static_cast<uint32_t>(stage) * (kStTokenBytes >> 4);
+          const uint32_t d = tmem_base + static_cast<uint32_t>(acc) * kStRows;
+          if (it.down && kb + 1 == k_blocks) stream_mmas<kStDownLastMmas>(d, sf, sf + 16 + half, a_lo, b_lo, descriptor, kb != 0);
+          else stream_mmas<4>(d, sf, sf + 16 + half, a_lo, b_lo, descriptor, kb != 0);
+          tc_commit(&smem->empty[stage]);
+          if (kb + 1 == k_blocks) tc_commit(&smem->acc_full[acc]);
+        }
+        if (++stage == kStStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      if (++acc == kStAccStages) {
+        acc = 0;
+        acc_phase ^= 1u;
+      }
+    }
+  } else if (warp == kStScaleWarp) {
+    // ---------------- scale-factor copier ----------------
+    int stage = 0;
+    uint32_t phase = 0;
+    const uint32_t sfa_lo0 = (smem_u32(smem->sfa[0]) & 0x3ffffu) >> 4;
+    const uint32_t sfb_lo0 = (smem_u32(smem->sfb[0]) & 0x3ffffu) >> 4;
+    constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);  // 8 rows x 16 B, no swizzle
+    const bool leader = elect_one();
+    for (int i = 0; ok && i < schedule.count; ++i) {
+      const bool down = i >= schedule.up_count;
+      const int k_blocks = down ? kStDownKBlocks : kStUpKBlocks;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        ok = wait_or_abort<false>(&smem->full[stage], phase, smem, status);
+        if (!ok) break;
+        if (leader) {
+          const uint32_t sfa = sfa_lo0 + static_cast<uint32_t>(stage) * (kSfStageBytes >> 4);
+          const uint32_t sfb = sfb_lo0 + static_cast<uint32_t>(stage) * (kSfStageBytes >> 4);
+          const uint32_t sf = tmem_base + kStSfColumn + kStSfColumnsPerStage * stage;
+          if (down && kb + 1 == k_blocks) issue_sf_copies<kStDownLastMmas, 128>(sf, sfa, sfb, hi_sf);
+          else issue_sf_copies<4, 128>(sf, sfa, sfb, hi_sf);
+          tc_commit(&smem->sf_full[stage]);
+        }
+        if (++stage == kStStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  } else if (warp == kStPublishWarp) {
+    // ---------------- publisher ----------------
+    // Making an item's stores visible to the grid takes one to two microseconds under load.  The epilogue
+    // warps leave that to this warp (their progress is a release to the CTA, the fence here extends it to
+    // the GPU) and go on; several items that finish meanwhile share one fence.
+    int published = 0;
+    const long long start = clock64();
+    while (published < schedule.up_count) {
+      int done = lane < kStEpilogueWarps ? smem->progress[lane] : schedule.up_count;
+      done = __reduce_min_sync(0xffffffffu, done);
+      if (done == published) {
+        if (smem->abort || clock64() - start > 2 * kWaitLimitCycles) break;
+        __nanosleep(64);
+        continue;
+      }
+      if (lane == 0) __threadfence();
+      __syncwarp();
+      for (int i = published + lane; i < done; i += 32) atomicAdd(p.plan.tile_ready + schedule.item(i, smem).expert, 1);
+      published = done;
+    }
+  } else {
+    // ---------------- epilogue ----------------
+    const int quarter = warp & 3;                        // the tensor-memory lanes this warp may read
+    const int side = (warp - kStEpilogueWarp) >> 2;      // groups side, side + 2, ... of eight rows
+    const int et = tid - kStEpilogueWarp * 32;
+    int acc = 0, buffer = 0;
+    uint32_t acc_phase = 0;
+    for (int i = 0; i < schedule.count; ++i) {
+      const StreamItem it = schedule.item(i, smem);
+      const int first = it.chunk * kStRows;
+      const int row0 = smem->offsets[it.expert] + first;
+      int rows = smem->offsets[it.expert + 1] - row0;
+      rows = rows > kStRows ? kStRows : rows;
+      const float alpha = it.down ? p.alpha2[it.expert] : p.alpha1[it.expert];
+      const float multiplier = it.down ? 0.0f : p.in_scale_q2[it.expert];
+      const bool ready = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, status));
+      uint32_t r[4][8];
+      if (ready) {
+        tc_fence_after_sync();
+        const uint32_t source = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * kStRows;
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          if ((side + 2 * g) * 8 < rows) tmem_load_32x8(source + (side + 2 * g) * 8, r[g]);
+        tmem_load_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&smem->acc_empty[acc]);
+      }
+      if (++acc == kStAccStages) {
+        acc = 0;
+        acc_phase ^= 1u;
+      }
+      if (it.down) {
+        if (!ready) break;
+        __nv_bfloat16* out = p.routed + static_cast<size_t>(row0) * kHidden + it.n_tile * 128 + quarter * 32 + (lane & ~1);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const int token0 = (side + 2 * g) * 8;
+          if (token0 >= rows) break;
+#pragma unroll
+          for (int pair = 0; pair < 4; ++pair) {
+            // even lanes finish token 2*pair, odd lanes token 2*pair + 1, two columns each
+            const uint32_t keep = (lane & 1) ? r[g][2 * pair + 1] : r[g][2 * pair];
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? r[g][2 * pair] : r[g][2 * pair + 1], 1);
+            const float lo = __fmul_rn(alpha, __uint_as_float((lane & 1) ? other : keep));
+            const float hi = __fmul_rn(alpha, __uint_as_float((lane & 1) ? keep : other));
+            const int token = token0 + 2 * pair + (lane & 1);
+            if (token < rows) *reinterpret_cast<uint32_t*>(out + static_cast<size_t>(token) * kHidden) = pack_bf16x2(lo, hi);
+          }
+        }
+        continue;
+      }
+      // w13: 32 tokens at a time through the exchange tile
+      const int column = et & 63;
+      bool stop = false;
+#pragma unroll
+      for (int part = 0; part < kStRows / kStExchangeRows; ++part) {
+        const int base = part * kStExchangeRows;
+        if (base >= rows) break;
+        if (ready) {
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            const int token0 = (side + 2 * g) * 8;  // within the part
+            if (base + token0 < rows) {
+#pragma unroll
+              for (int t = 0; t < 8; ++t)
+                smem->exchange[buffer][token0 + t][quarter * 32 + lane] =
+                    __float2bfloat16_rn(__fmul_rn(alpha, __uint_as_float(r[2 * part + g][t])));
+            }
+          }
+        } else {
+          smem->left = 1;
+        }
+        // All eight warps meet here also when one of them gave up, and then leave together.
+        named_barrier(2, kStEpilogueWarps * 32);
+        if (smem->left) {
+          stop = true;
+          break;
+        }
+        for (int token = et >> 6; token < kStExchangeRows; token += 4) {
+          if (base + token >= rows) break;
+          const float up = __bfloat162float(smem->exchange[buffer][token][column]);
+          const float gate = __bfloat162float(smem->exchange[buffer][token][64 + column]);
+          const float v = __fmul_rn(gv_gelu_erf(gate, smem->erf_table), up);
+          float maximum = fabsf(v);
+#pragma unroll
+          for (int offset = 8; offset; offset >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
+          const uint32_t scale = encode_e4m3(__fdiv_rn(__fmul_rn(multiplier, maximum), 6.0f));
+          const float rounded = decode_e4m3(scale);
+          const float inverse = rounded == 0.0f ? 0.0f : __fdiv_rn(multiplier, rounded);
+          const float scaled = __fmul_rn(v, inverse);
+          // columns 2c and 2c + 1 make byte c of the block's eight code bytes
+          const float other = __shfl_xor_sync(0xffffffffu, scaled, 1);
+          uint32_t word = encode_e2m1x2(scaled, other) << (8 * ((column >> 1) & 3));  // meaningful in even lanes
+          if (column & 1) word = 0;
+          word |= __shfl_xor_sync(0xffffffffu, word, 2);
+          word |= __shfl_xor_sync(0xffffffffu, word, 4);
+          const uint32_t high = __shfl_down_sync(0xffffffffu, word, 8);
+          if ((column & 15) == 0) {
+            const int block = it.n_tile * 4 + (column >> 4);
+            *reinterpret_cast<uint2*>(p.inter_codes + static_cast<size_t>(row0 + base + token) * (kInter / 2) + block * 8) =
+                make_uint2(word, high);
+            p.inter_scales[static_cast<size_t>(smem->scale_rows[it.expert]) * (kInter / 16) +
+                           sf_offset(first + base + token, block, kInter / 16)] = static_cast<uint8_t>(scale);
+          }
+        }
+        buffer ^= 1;
+      }
+      if (stop) break;
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence_block();
+        smem->progress[warp - kStEpilogueWarp] = i + 1;
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == kStMmaWarp) {
+    tc_fence_after_sync();
+    __syncwarp();
+    tmem_dealloc(tmem_base, kStTmemColumns);
+  }
+  // The CTA that finishes last puts the counters back for the next launch: every wait on them lies
+  // before a CTA's end.
+  if (tid == 0) {
+    __threadfence();
+    smem->last = atomicAdd(p.plan.front_sync + 1, 1) == static_cast<int>(gridDim.x) - 1;
+  }
+  __syncthreads();
+  if (smem->last) {
+    if (tid < kExperts) p.plan.tile_ready[tid] = 0;
+    if (tid < 2) p.plan.front_sync[tid] = 0;
+  }
+}
+
+StreamParams make_params(const StreamOperands& op, const RoutePlan& plan) {
+  StreamParams p{};
+  p.plan = plan;
+  p.w13_scales = op.w13_scales;
+  p.w2_scales = op.w2_scales;
+  p.input_scales = op.input_scales;
+  p.inter_codes = op.inter_codes;
+  p.inter_scales = op.inter_scales;
+  p.routed = static_cast<__nv_bfloat16*>(op.routed);
+  p.alpha1 = op.alpha1;
+  p.alpha2 = op.alpha2;
+  p.in_scale_q2 = op.in_scale_q2;
+  return p;
+}
+
+StreamMaps make_maps(const StreamOperands& op) {
+  StreamMaps maps;
+  maps.w13 = op.map_w13;
+  maps.w2 = op.map_w2;
+  for (int i = 0; i < kStRows / 8; ++i) {
+    maps.up[i] = op.map_up[i];
+    maps.down[i] = op.map_down[i];
+  }
+  return maps;
+}
+
+}  // namespace
+
+static_assert(kStRows / 8 == kStreamBoxes, "one map per box height");
+static_assert(kExperts + kStreamMaxTokens * kTopK / kStRows <= kStMaxChunks, "chunk list");
+
+int prepare_stream_experts() {
+  cudaError_t e = cudaFuncSetAttribute(stream_experts_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(kStSmemBytes));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(stream_experts_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kStSmemBytes));
+  return static_cast<int>(e);
+}
+
+void launch_stream_experts(const StreamOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream) {
+  launch_chained(stream_experts_kernel<false>, dim3(sm_count), dim3(kStThreads), kStSmemBytes, stream, make_maps(op),
+                 make_params(op, plan));
+}
+
+void launch_stream_layer(const StreamOperands& op, const RoutePlan& plan, const void* input_bf16, const int* expert_ids,
+                         const float* in_scale_q1, uint8_t* packed, uint8_t* scales, int tokens, int sm_count,
+                         cudaStream_t stream) {
+  StreamParams p = make_params(op, plan);
+  p.input = static_cast<const __nv_bfloat16*>(input_bf16);
+  p.expert_ids = expert_ids;
+  p.in_scale_q1 = in_scale_q1;
+  p.packed = packed;
+  p.scales = scales;
+  p.tokens = tokens;
+  launch_chained(stream_experts_kernel<true>, dim3(sm_count), dim3(kStThreads), kStSmemBytes, stream, make_maps(op), p);
+}
+
+}  // namespace gv

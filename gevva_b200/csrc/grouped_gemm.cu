@@ -632,7 +632,7 @@ int prepare_grouped_gemm() {
   if (e == cudaSuccess) e = raise_smem_limit<kPlain, 1, 256>();
   if (e == cudaSuccess) e = raise_smem_limit<kGeglu, 1, 256>();
   if (e == cudaSuccess) e = raise_smem_limit<kFp8, 1, 128>();
-  if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_decode_experts());
+  if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_stream_experts());
   if (e == cudaSuccess) return prepare_grouped_gemm_pairs();
   return static_cast<int>(e);
 }

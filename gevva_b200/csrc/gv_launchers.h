@@ -32,15 +32,15 @@ struct RoutePlan {
   int* pair_tile;          // optional [R/128 + 128]: 2 * (first tile of a pair) + (1 if the pair has two
                            // tiles); a pair = two consecutive 128-row tiles of one expert, or its last odd one
   int* num_pairs;          // optional [1]
-  int* tile_ready;         // optional [R/128 + 128]: per row tile, epilogue warps of its w13 items that have
-                           // stored their share of the w2 operand (merged decode kernel); zeroed by the sort
+  int* tile_ready;         // optional [R/128 + 128], zero on entry and on exit: per expert, w13 items that have
+                           // stored their share of the w2 operand (streaming kernel)
   const int* tile_first;   // optional [1]: a GEMM launch covers tiles [tile_first, tile_first + num_m_tiles)
   int* chunk_hist;         // [ceil(R/1024) * 128] scratch of the multi-block sort
   int* status;             // [1]   device status word (gv::Status)
   const int* remap;        // optional [128]: sort key = remap[expert id] (expert-parallel placement)
   int* sync;               // optional [2], zero on entry: arrival/departure counters of the one-launch sort
   int* front_sync;         // optional [2], zero on entry and on exit: tokens quantised / CTAs finished, of the
-                           // decode kernel that sorts and quantises by itself
+                           // streaming kernel
 };
 
 void launch_route(const void* logits_bf16, int ld, const void* expert_scale_bf16, float* weights,
@@ -144,16 +144,31 @@ void launch_retile_w13_unit_scales(const uint8_t* sidecar_scales, uint8_t* tiled
 void launch_w13_pairs(const W13PairOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
 int prepare_w13_pairs();
 
-// Both expert GEMMs of a batch of at most 128 tokens in one persistent launch (grouped_gemm_decode.cu):
-// the fused w13 form, then w2, with per-tile readiness counters (plan.tile_ready) in between.
-void launch_decode_experts(const GemmOperands& w13_fused, const GemmOperands& w2, const RoutePlan& plan,
-                           int sm_count, cudaStream_t stream);
-// The same with the route sort and the input quantiser inside (needs plan.front_sync and
-// tokens <= min(128, sm_count)): a decode layer step without the router and the reduce.
-void launch_decode_layer(const void* input_bf16, const int* expert_ids, const float* in_scale_q, int tokens,
-                         uint8_t* packed, uint8_t* scales, const GemmOperands& w13_fused, const GemmOperands& w2,
-                         const RoutePlan& plan, int sm_count, cudaStream_t stream);
-int prepare_decode_experts();
+// Both expert GEMMs of a batch with few rows an expert in one persistent launch with the weights on the
+// MMA's M side (experts_stream.cu).
+constexpr int kStreamBoxes = 8;         // activation boxes of 8, 16, ... 64 rows
+constexpr int kStreamMaxTokens = 2048;  // the kernel's chunk list; where the launch pays is the caller's rule
+struct StreamOperands {
+  CUtensorMap map_w13;                 // as W13PairOperands::map_w
+  CUtensorMap map_w2;                  // [128 * 2816, 352] bytes, box 128 x 128 B
+  CUtensorMap map_up[kStreamBoxes];    // input codes [row capacity, 1408] through boxes of 8(i+1) rows x 128 B
+  CUtensorMap map_down[kStreamBoxes];  // w2 operand codes [row capacity, 352] likewise
+  const uint8_t* w13_scales;           // launch_retile_w13_unit_scales
+  const uint8_t* w2_scales;            // sidecar layout
+  const uint8_t* input_scales;
+  uint8_t* inter_codes;
+  uint8_t* inter_scales;
+  void* routed;                        // bf16 [row capacity, 2816]
+  const float *alpha1, *alpha2, *in_scale_q2;
+};
+// On a sorted plan and a quantised input; plan.tile_ready (by expert here) and plan.front_sync zero on
+// entry and on exit.
+void launch_stream_experts(const StreamOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
+// With the route sort and the input quantiser inside; tokens <= min(128, sm_count).
+void launch_stream_layer(const StreamOperands& op, const RoutePlan& plan, const void* input_bf16, const int* expert_ids,
+                         const float* in_scale_q1, uint8_t* packed, uint8_t* scales, int tokens, int sm_count,
+                         cudaStream_t stream);
+int prepare_stream_experts();
 
 // Must be called once per device before launch_grouped_gemm (sets the dynamic
 // shared-memory limit).  Returns a cudaError_t value.

@@ -1,5 +1,4 @@
-// Device side of the input quantiser, shared by its own launches (moe_kernels.cu) and by the
-// decode kernel that quantises its token itself (grouped_gemm_decode.cu).
+// Device side of the input quantiser, shared by its two launches (moe_kernels.cu).
 #pragma once
 
 #include "gv_common.cuh"

@@ -24,6 +24,8 @@ namespace {
 using namespace gv;
 
 constexpr int kMaxTokens = 131072;
+constexpr int kStreamTokens = 640;  // see moe_launch_stages_on
+static_assert(kStreamTokens <= gv::kStreamMaxTokens, "the streaming kernel's chunk list");
 
 // The CUDA face of the allocator that gv_scratch.h takes as a parameter.
 struct CudaScratchRuntime {
@@ -229,12 +231,13 @@ struct gevva_moe {
   gv::GemmOperands w2{};
   uint8_t* w13_sf_tiled = nullptr;  // runner-owned re-tiling of weights.w13_sf
   gv::W13PairOperands w13_pairs{};  // the CTA-pair form of the fused w13 stage
-  uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf for it
+  uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf for it and for the streaming form
+  gv::StreamOperands stream_experts{};  // few rows an expert: both GEMMs in one launch, weights on the MMA's M side
   bool w13_pair_form = false;       // GEVVA_MOE_OPTION_W13_PAIRS, or GEVVA_MOE_W13_PAIRS=1 for a whole process
   int sm_count = 0;
   bool pairs = false;               // GEVVA_MOE_OPTION_PAIRS: prefill-sized launches run the expert GEMMs as CTA pairs
-  bool decode_front = true;         // ... and the route sort and the input quantiser in the same launch (GEVVA_MOE_DECODE_FRONT=0: a launch of their own)
-  bool merged_decode = true;        // batches of at most 128 tokens: w13 and w2 in one launch (GEVVA_MOE_DECODE_MERGED=0: two)
+  bool decode_front = true;         // batches of at most 128 tokens: ... and the route sort and the input quantiser in the same launch (GEVVA_MOE_DECODE_FRONT=0: a launch of their own)
+  bool merged_decode = true;        // batches of at most kStreamTokens: w13 and w2 in one launch (GEVVA_MOE_DECODE_MERGED=0: two)
   bool nvtx = false;                // GEVVA_MOE_OPTION_NVTX: one range per stage around its launches
 };
 
@@ -273,8 +276,8 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
     // decode-sized batch: sort, quantiser and both GEMMs in one persistent launch; the weights start
     // streaming while the input is still being quantised
     StageRange range(runner->nvtx, "gevva_moe.sort+quantize+w13+geglu+w2");
-    gv::launch_decode_layer(in, ids, runner->weights.in_scale_q1, tokens, s->input_codes, s->input_sf,
-                            runner->w13_fused, runner->w2, s->plan, sm_count, stream);
+    gv::launch_stream_layer(runner->stream_experts, s->plan, in, ids, runner->weights.in_scale_q1, s->input_codes,
+                            s->input_sf, tokens, sm_count, stream);
     stages &= ~layer_body;
   }
   if ((stages & front) == front && tokens <= gv::kFusedSortQuantizeMaxTokens) {
@@ -294,12 +297,15 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   }
   const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
   const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
-  if ((stages & gemms) == gemms && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode &&
-      tokens <= gv::kFusedSortQuantizeMaxTokens && (stages & front) == front) {
-    // decode-sized batch: both GEMMs in one persistent launch, weights streaming across the boundary
-    // (the readiness counters it needs are zeroed by the fused sort + quantise launch above)
+  // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side
+  // does both GEMMs.  Up to about 40 rows an expert that is faster than the two 128-row-tile launches
+  // (per layer of two distinct ones, us, one B200: 129 tokens 101.9 against 111.4, 200 103.4 / 112.5,
+  // 450 108.0 / 116.8, 613 118.4 / 121.3, 800 137.7 / 126.9): above, its GeGLU epilogue, which handles
+  // a column of a token per thread through shared memory, outweighs the weights.
+  if ((stages & gemms) == gemms && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !runner->pairs &&
+      !runner->w13_pair_form && tokens <= kStreamTokens) {
     StageRange range(runner->nvtx, "gevva_moe.w13+geglu+w2");
-    gv::launch_decode_experts(runner->w13_fused, runner->w2, s->plan, sm_count, stream);
+    gv::launch_stream_experts(runner->stream_experts, s->plan, sm_count, stream);
     stages &= ~gemms;
   }
   if ((stages & both) == both && !(stages & GEVVA_MOE_STAGE_UNFUSED)) {
@@ -431,23 +437,45 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
     std::snprintf(g_error_text, sizeof(g_error_text), "cuTensorMapEncodeTiled failed (scale maps)");
     return GEVVA_MOE_CUDA_ERROR;
   }
-  const char* w13_pairs_env = std::getenv("GEVVA_MOE_W13_PAIRS");
-  m->w13_pair_form = (options && (options->flags & GEVVA_MOE_OPTION_W13_PAIRS)) || (w13_pairs_env && w13_pairs_env[0] == '1');
-  if (m->w13_pair_form) {
-    // opt-in (measured slower than the one-CTA kernel on this part): its 35 MB re-tiled scale copy
-    // and its tensor maps exist only when asked for
-    cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
-    if (e == cudaSuccess)
-      e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_units), gv::w13_unit_scale_bytes(kExperts));
+  {
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_units), gv::w13_unit_scale_bytes(kExperts));
     if (e == cudaSuccess) {
-      gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_units, kExperts,
-                                        nullptr);
+      gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_units, kExperts, nullptr);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
       gevva_moe_destroy(m);
       return cuda_failure(e, "w13 unit scale re-tiling");
+    }
+    gv::StreamOperands& st = m->stream_experts;
+    ok = make_w13_unit_map(&st.map_w13, weights->w13, kExperts);
+    for (int i = 0; i < gv::kStreamBoxes; ++i)
+      ok = ok && make_operand_map(&st.map_up[i], s->input_codes, rows, kHidden / 2, 8 * (i + 1)) &&
+           make_operand_map(&st.map_down[i], s->inter_codes, rows, kInter / 2, 8 * (i + 1));
+    if (!ok) {
+      gevva_moe_destroy(m);
+      std::snprintf(g_error_text, sizeof(g_error_text), "cuTensorMapEncodeTiled failed (streaming form)");
+      return GEVVA_MOE_CUDA_ERROR;
+    }
+    st.map_w2 = m->w2.map_b;
+    st.w13_scales = m->w13_sf_units;
+    st.w2_scales = static_cast<const uint8_t*>(weights->w2_sf);
+    st.input_scales = s->input_sf;
+    st.inter_codes = s->inter_codes;
+    st.inter_scales = s->inter_sf;
+    st.routed = s->w2_out;
+    st.alpha1 = weights->alpha1;
+    st.alpha2 = weights->alpha2;
+    st.in_scale_q2 = weights->in_scale_q2;
+  }
+  const char* w13_pairs_env = std::getenv("GEVVA_MOE_W13_PAIRS");
+  m->w13_pair_form = (options && (options->flags & GEVVA_MOE_OPTION_W13_PAIRS)) || (w13_pairs_env && w13_pairs_env[0] == '1');
+  if (m->w13_pair_form) {
+    const cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
+    if (e != cudaSuccess) {
+      gevva_moe_destroy(m);
+      return cuda_failure(e, "w13 pair form");
     }
     gv::W13PairOperands& wp = m->w13_pairs;
     ok = true;

@@ -649,6 +649,41 @@ def test_decode_kernel_that_sorts_and_quantises_itself(gm, weights, cuda_device,
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("tokens", [2, 65, 128, 129, 300, 640])
+def test_streaming_experts_equal_the_two_launches(gm, weights, cuda_device, tokens, monkeypatch):
+    """The launch that does both GEMMs with the weights on the MMA's M side (up to 640 tokens) against
+    the two launches with 128-row tiles: the same w2 operand bytes, routed rows and output, with groups
+    at the edges of its 16-row MMAs, 64-row chunks and 128-row scale tiles, run twice on one scratch
+    (its counters go back to zero)."""
+    from gevva_b200 import runtime as rt
+    edges = [c for c in (1, 15, 16, 17, 63, 64, 65, 129) if c <= tokens]
+    rng = np.random.default_rng(tokens)
+    ids = np.empty((tokens, TOP_K), dtype=np.int32)
+    for t in range(tokens):
+        mine = [e for e, count in enumerate(edges) if t < count]
+        rest = rng.choice(np.arange(16, EXPERTS), TOP_K - len(mine), replace=False)
+        ids[t] = rng.permutation(np.concatenate([np.array(mine, dtype=np.int64), rest]))
+    x = hashgen.activations(tokens, HIDDEN, 75, cuda_device)
+    dev_ids = torch.from_numpy(ids).to(cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    routes = tokens * TOP_K
+    results = []
+    for merged in ("0", "1"):
+        monkeypatch.setenv("GEVVA_MOE_DECODE_MERGED", merged)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        out = torch.empty_like(x)
+        for _ in range(2):
+            out.zero_()
+            runner.launch_batch(x, dev_ids, rw, out, tokens)
+        runner.check()
+        results.append((out, runner.buffer(rt.BUF_INTER_CODES)[: routes * INTER // 2].clone(),
+                        runner.buffer(rt.BUF_INTER_SF).clone(),
+                        runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: routes * HIDDEN].clone()))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert results[0][0].float().abs().max() > 0
+
+
 def test_nvtx_ranges_do_not_change_results(gm, weights, cuda_device):
     """A runner created with the NVTX option marks its stages and computes the same bits; unknown
     option flags are refused."""
