@@ -485,7 +485,7 @@ struct gevva_moe_ep {
   uint8_t* inter_sf = nullptr;
   unsigned long long* row_dest = nullptr;
   unsigned long long* row_dest_local = nullptr;  // measurement aid, allocated on first use
-  uint8_t* w13_sf_tiled = nullptr;
+  uint8_t* w13_sf_units = nullptr;
   // the compute phase runs the local experts in two halves so that the NVLink-bound w2 of the
   // first half overlaps the w13 of the second: a side stream and two events order them
   int* split = nullptr;  // device [2 * chunks]: first tile and tile count of each part
@@ -505,7 +505,7 @@ void gevva_moe_ep_destroy(gevva_moe_ep* ep) {
   cudaFree(ep->inter_sf);
   cudaFree(ep->row_dest);
   cudaFree(ep->row_dest_local);
-  cudaFree(ep->w13_sf_tiled);
+  cudaFree(ep->w13_sf_units);
   if (ep->side) cudaStreamDestroy(ep->side);
   if (ep->fork) cudaEventDestroy(ep->fork);
   if (ep->join) cudaEventDestroy(ep->join);
@@ -588,7 +588,7 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
   if (e == cudaSuccess) e = cudaMemset(ep->inter_sf, 0, padded * (kInter / 16));
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&ep->row_dest), cap * sizeof(unsigned long long));
   if (e == cudaSuccess)
-    e = cudaMalloc(reinterpret_cast<void**>(&ep->w13_sf_tiled), gv::retiled_w13_scale_bytes(el));
+    e = cudaMalloc(reinterpret_cast<void**>(&ep->w13_sf_units), gv::w13_unit_scale_bytes(el));
   if (e != cudaSuccess) {
     gevva_moe_ep_destroy(ep);
     return GEVVA_MOE_CUDA_ERROR;
@@ -638,8 +638,8 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
   ep->dev.remap = remap;
   sp.remap = remap;
 
-  gv::launch_retile_w13_scales(static_cast<const uint8_t*>(local_weights->w13_sf), ep->w13_sf_tiled, el,
-                               nullptr);
+  gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(local_weights->w13_sf), ep->w13_sf_units, el,
+                                    nullptr);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   bool ok = e == cudaSuccess;
@@ -648,8 +648,7 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
   ok = ok && make_map(&ep->w2.map_a32, ep->inter_codes, cap, kInter / 2, 32);
   ok = ok && make_map(&ep->w13.map_b, local_weights->w13, static_cast<uint64_t>(el) * kW13Out,
                       kHidden / 2, kTileM);
-  ok = ok && make_map(&ep->w13.map_b64, local_weights->w13, static_cast<uint64_t>(el) * kW13Out,
-                      kHidden / 2, 64);
+  ok = ok && gv::make_w13_unit_tensor_map(&ep->w13.map_b_units, local_weights->w13, static_cast<uint64_t>(el));
   ok = ok && make_map(&ep->w2.map_a, ep->inter_codes, cap, kInter / 2, kTileM);
   ok = ok && make_map(&ep->w2.map_b, local_weights->w2, static_cast<uint64_t>(el) * kHidden, kInter / 2,
                       kTileM);
@@ -658,7 +657,7 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
     return GEVVA_MOE_CUDA_ERROR;
   }
   ep->w13.a_scales = ep->input_sf;
-  ep->w13.b_scales = ep->w13_sf_tiled;
+  ep->w13.unit_scales = ep->w13_sf_units;
   ep->w13.alpha = local_weights->alpha1;
   ep->w13.out = nullptr;
   ep->w13.n_out = kW13Out;

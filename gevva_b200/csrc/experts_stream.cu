@@ -59,8 +59,6 @@ constexpr uint32_t kStSfColumnsPerStage = 32;             // 16 for the weights,
 static_assert(kStSfColumn + kStSfColumnsPerStage * kStStages <= kStTmemColumns, "tensor memory budget");
 constexpr int kStWeightBytes = kTileM * kTileKBytes;      // 16 KiB
 constexpr int kStTokenBytes = kStRows * kTileKBytes;      // 8 KiB
-constexpr int kStUnits = kInter / 64;                     // 11 w13 items a chunk
-constexpr int kStUnitSlots = kStUnits + 1;                // the re-tiled scales keep 12 per expert
 constexpr int kStDownTiles = kHidden / 128;               // 22 w2 items a chunk
 constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
 constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192
@@ -94,7 +92,7 @@ struct alignas(1024) StreamSmem {
   alignas(16) float route_multiplier[kTopK];
   unsigned long long route_scale_base[kTopK];
   float scale_q1[kExperts];
-  alignas(16) float erf_table[GV_ERF_TABLE_FLOATS];
+  GegluTables tables;
 };
 constexpr size_t kStSmemBytes = sizeof(StreamSmem) + 1024;
 static_assert(kStSmemBytes <= 232448, "shared memory budget of one sm_100 CTA");
@@ -137,7 +135,7 @@ struct StreamSchedule {
   int first_extra, lacking, pre;  // w2: CTAs >= first_extra are one w13 item short and take `pre` items first
   __device__ StreamSchedule(int chunks) {
     const int ctas = gridDim.x, cta = blockIdx.x;
-    const int up = chunks * kStUnits, down = chunks * kStDownTiles;
+    const int up = chunks * kUnits, down = chunks * kStDownTiles;
     up_count = up > cta ? (up - 1 - cta) / ctas + 1 : 0;
     first_extra = up % ctas;
     lacking = first_extra == 0 ? 0 : ctas - first_extra;
@@ -154,7 +152,7 @@ struct StreamSchedule {
     it.down = i >= up_count;
     if (!it.down) {
       index = cta + i * ctas;
-      per_chunk = kStUnits;
+      per_chunk = kUnits;
     } else {
       int k = i - up_count;
       const bool is_short = cta >= first_extra;
@@ -174,14 +172,6 @@ struct StreamSchedule {
     return it;
   }
 };
-
-__device__ __forceinline__ void stream_load_3d(void* smem_dst, const void* tensor_map, uint64_t* bar, int x, int y, int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
-      "l"(tensor_map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
 
 __device__ __forceinline__ void tmem_load_32x8(uint32_t tmem_address, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -256,9 +246,9 @@ __device__ __forceinline__ void stream_quantise_token(const StreamParams& p, con
     if (!have || __float_as_uint(multiplier) != previous) {  // routes of equal static scale share the result
       have = true;
       previous = __float_as_uint(multiplier);
-      const uint32_t scale = encode_e4m3(__fdiv_rn(__fmul_rn(multiplier, maximum), 6.0f));
-      const float rounded = decode_e4m3(scale);
-      const float inverse = rounded == 0.0f ? 0.0f : __fdiv_rn(multiplier, rounded);
+      const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
+      const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, smem->tables.reciprocals)
+                                                               : scale_inverse_divided(multiplier, scale);
       codes = 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -306,7 +296,9 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     tmem_alloc(&smem->tmem_base, kStTmemColumns);
     tmem_relinquish();
   }
-  load_erf_table(smem->erf_table);
+  load_geglu_tables(&smem->tables);
+  __syncthreads();
+  fill_geglu_tables(&smem->tables);
   if (kFront && tid < kExperts) smem->histogram[tid] = 0;
   if (kFront && tid < kTopK) smem->own_rank[tid] = 0;
   grid_launch_dependents();
@@ -454,13 +446,13 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
       const uint8_t* sf;
       if (weight_side) {
         sf = it.down ? p.w2_scales + static_cast<size_t>(it.expert * kHidden + it.n_tile * 128) * (kInter / 16)
-                     : p.w13_scales + static_cast<size_t>(it.expert * kStUnitSlots + it.n_tile) * kStUpKBlocks * kSfStageBytes;
+                     : p.w13_scales + static_cast<size_t>(it.expert * kUnitSlots + it.n_tile) * kStUpKBlocks * kSfStageBytes;
       } else {
         const size_t scale_row = smem->scale_rows[it.expert] + first / kTileM * kTileM;
         sf = it.down ? p.inter_scales + scale_row * (kInter / 16) : p.input_scales + scale_row * (kHidden / 16);
         if (it.down) {
           // the rows exist once every w13 item of the expert has been counted; they were written by ordinary stores of other SMs and are read through the async proxy
-          ok = stream_wait_counter(p.plan.tile_ready + it.expert, kStUnits * smem->chunks_of[it.expert], smem, status);
+          ok = stream_wait_counter(p.plan.tile_ready + it.expert, kUnits * smem->chunks_of[it.expert], smem, status);
           if (!ok) break;
           asm volatile("fence.proxy.async.global;" ::: "memory");
         }
@@ -475,7 +467,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
           if (weight_side) {
             mbar_arrive_expect_tx(bar, kStWeightBytes + sf_bytes);
             if (it.down) tma_load_2d(smem->a[stage], &maps.w2, bar, x, it.expert * kHidden + it.n_tile * 128);
-            else stream_load_3d(smem->a[stage], &maps.w13, bar, x, it.n_tile * 64, 2 * it.expert);
+            else tma_load_3d(smem->a[stage], &maps.w13, bar, x, it.n_tile * 64, 2 * it.expert);
             bulk_load_1d(smem->sfa[stage], sf + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes, bar);
           } else {
             mbar_arrive_expect_tx(bar, static_cast<uint32_t>(boxes * 8 * kTileKBytes) + sf_bytes);
@@ -676,13 +668,13 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
           if (base + token >= rows) break;
           const float up = __bfloat162float(smem->exchange[buffer][token][column]);
           const float gate = __bfloat162float(smem->exchange[buffer][token][64 + column]);
-          const float v = __fmul_rn(gv_gelu_erf(gate, smem->erf_table), up);
+          const float v = __fmul_rn(gelu_of_bf16(gate, &smem->tables), up);
           float maximum = fabsf(v);
 #pragma unroll
           for (int offset = 8; offset; offset >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
-          const uint32_t scale = encode_e4m3(__fdiv_rn(__fmul_rn(multiplier, maximum), 6.0f));
-          const float rounded = decode_e4m3(scale);
-          const float inverse = rounded == 0.0f ? 0.0f : __fdiv_rn(multiplier, rounded);
+          const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
+          const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, smem->tables.reciprocals)
+                                                                   : scale_inverse_divided(multiplier, scale);
           const float scaled = __fmul_rn(v, inverse);
           // columns 2c and 2c + 1 make byte c of the block's eight code bytes
           const float other = __shfl_xor_sync(0xffffffffu, scaled, 1);

@@ -26,9 +26,9 @@
 // Two epilogues:
 //   kPlain  bf16(alpha*acc), staged through shared memory so that every global
 //           store instruction writes two full 256-byte row segments;
-//   kGeglu  the 256 weight rows of an item are up rows [128j,128j+128) and gate rows
-//           [704+128j, 704+128j+128) of w13 (the sixth item of a row tile is half empty),
-//           so a thread holds up and gate of the same columns: v = gelu_erf(bf16(gate)) *
+//   kGeglu  the 256 weight rows of an item are two units of 64 up rows and 64 gate rows of the same
+//           intermediate columns (eleven units, so the sixth item of a row tile has one and runs
+//           at N = 128), so a thread holds up and gate of the same columns: v = gelu_erf(bf16(gate)) *
 //           bf16(up), two 16-value blocks per thread -> 16 code bytes and two scale bytes,
 //           written straight into the w2 operand buffers.  The bf16 w13 output never
 //           exists in memory.
@@ -38,8 +38,8 @@
 // (src/nvfp4_cutlass.cu:321-323); one atom is exactly what one MMA (K = 64)
 // consumes and what tcgen05.cp 32x128b.warpx4 moves, so a K block of 256 needs a
 // contiguous 2 KiB per operand, fetched with one untiled bulk copy.  For kGeglu the
-// weight scales come from a copy re-tiled once at runner creation so that the
-// [128 up | 128 gate] rows of an item form such atoms (retile_w13_scales_kernel below).
+// weight scales come from a copy re-tiled once at runner creation so that the [64 up | 64 gate]
+// rows of a unit form such atoms (retile_w13_unit_scales_kernel, grouped_gemm_w13_pair.cu).
 //
 // Every wait is bounded: on expiry the kernel records kWaitTimeout in the status
 // word, all roles leave their loops, tensor memory is released and the CTA exits.
@@ -103,7 +103,7 @@ struct alignas(1024) GemmSmem {
   uint32_t tmem_base;
   volatile int abort;
   int quarter_left[4];  // plain epilogue: a warp of this quarter gave up waiting
-  alignas(16) float erf_table[GV_ERF_TABLE_FLOATS];
+  GegluTables tables[kMode == kGeglu ? 1 : 0];
 };
 
 template <int kMode, int kAtoms, int kN> constexpr size_t gemm_smem_bytes() {
@@ -182,8 +182,7 @@ template <int kMode, int kAtomsPerStage, int kN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                           const __grid_constant__ CUtensorMap map_a32,
-                          const __grid_constant__ CUtensorMap map_b,
-                          const __grid_constant__ CUtensorMap map_b64, const GemmParams p) {
+                          const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   using Smem = GemmSmem<kMode, kAtomsPerStage, kN>;
   using Shape = typename Smem::Shape;
   constexpr int kStages = Smem::kStages;
@@ -214,13 +213,16 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     prefetch_tensor_map(&map_a);
     prefetch_tensor_map(&map_a32);
     prefetch_tensor_map(&map_b);
-    if (kMode == kGeglu) prefetch_tensor_map(&map_b64);
   }
   if (warp == 1) {
     tmem_alloc(&smem->tmem_base, kTmemColumns);
     tmem_relinquish();
   }
-  if (kMode == kGeglu) load_erf_table(smem->erf_table);
+  if constexpr (kMode == kGeglu) {
+    load_geglu_tables(smem->tables);
+    __syncthreads();
+    fill_geglu_tables(smem->tables);
+  }
   grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
@@ -250,22 +252,19 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const int expert = p.tile_expert[m_tile];
       int row = 0, row2 = 0;
       const uint8_t* sf_src;
-      const uint8_t* sf_src2 = nullptr;  // wide plain tiles: scales of weight rows 128..255
+      const uint8_t* sf_src2 = nullptr;  // wide tiles: scales of weight rows 128..255
       bool short_tile = false;  // decode-sized groups: fetch 32 activation rows instead of 128
-      bool half_item = false;   // fused wide tiles: the last item of a row tile has 64 up and 64 gate rows
+      bool half_item = false;   // fused form: the last item of a row tile has one unit
       if (!weight_side) {
         row = p.expert_offsets[expert] + (m_tile * kTileM - p.scale_row_offsets[expert]);
         short_tile = p.expert_offsets[expert + 1] - row <= 32;
         sf_src = p.a_scales + static_cast<size_t>(m_tile) * kTileM * p.groups;
       } else if (kMode == kGeglu) {
-        // up rows; the gate rows lie kInter further on.  The last item of a row tile has only
-        // 64 up and 64 gate rows left: only those are fetched (64-row boxes); the rest of each
-        // 128-row half keeps whatever the stage held, its scales are zero in the re-tiled copy
-        // and its columns are dropped by the epilogue.
-        row = expert * kW13Out + n_tile * (kN / 2);
-        row2 = row + kInter;
+        // units 2 * n_tile and the next one; the last item of a row tile has one unit left
+        row = n_tile * kN / 2;
         half_item = kWide && (n_tile + 1) * (kN / 2) > kInter;
-        sf_src = p.b_scales + (static_cast<size_t>(expert) * p.n_tiles + n_tile) * kN * p.groups;
+        sf_src = p.b_scales + (static_cast<size_t>(expert) * kUnitSlots + 2 * n_tile) * p.k_blocks * kSfStageBytes;
+        sf_src2 = sf_src + static_cast<size_t>(p.k_blocks) * kSfStageBytes;
       } else {
         row = expert * p.n_out + n_tile * kN;
         row2 = row + 128;
@@ -285,7 +284,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           if (!weight_side)
             expected = atoms * (short_tile ? kOperandStageBytes / 4 : kOperandStageBytes) + sf_bytes;
           else if (kWide && kMode == kGeglu)
-            expected = (half_item ? Shape::kWeightBytes / 2 : Shape::kWeightBytes) + Shape::kWeightSfBytes;
+            expected = (half_item ? 1u : 2u) * (Shape::kWeightBytes / 2 + kSfStageBytes);
           else
             expected = atoms * Shape::kWeightBytes + (kWide ? 2u : 1u) * sf_bytes;
           mbar_arrive_expect_tx(&smem->full[stage], expected);
@@ -296,10 +295,14 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
             if (!weight_side) {
               tma_load_2d(smem->a[stage] + atom * kOperandStageBytes, short_tile ? &map_a32 : &map_a,
                           &smem->full[stage], x, row);
+            } else if (kMode == kGeglu) {
+              // a unit's up rows and gate rows in one box
+              tma_load_3d(smem->b[stage], &map_b, &smem->full[stage], x, row, 2 * expert);
+              if (!half_item)
+                tma_load_3d(smem->b[stage] + kOperandStageBytes, &map_b, &smem->full[stage], x, row + 64, 2 * expert);
             } else if (kWide) {
-              const CUtensorMap* map = half_item ? &map_b64 : &map_b;
-              tma_load_2d(smem->b[stage], map, &smem->full[stage], x, row);
-              tma_load_2d(smem->b[stage] + kOperandStageBytes, map, &smem->full[stage], x, row2);
+              tma_load_2d(smem->b[stage], &map_b, &smem->full[stage], x, row);
+              tma_load_2d(smem->b[stage] + kOperandStageBytes, &map_b, &smem->full[stage], x, row2);
             } else {
               tma_load_2d(smem->b[stage] + atom * kOperandStageBytes, &map_b, &smem->full[stage], x, row);
             }
@@ -309,9 +312,11 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               bulk_load_1d(smem->sfa[stage], sf_src + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes,
                            &smem->full[stage]);
             } else if (kWide && kMode == kGeglu) {
-              // re-tiled scales: [rows 0..127 | rows 128..255] x four MMAs, 4 KiB per K block
-              bulk_load_1d(smem->sfb[stage], sf_src + static_cast<size_t>(kb) * Shape::kWeightSfBytes,
-                           Shape::kWeightSfBytes, &smem->full[stage]);
+              bulk_load_1d(smem->sfb[stage], sf_src + static_cast<size_t>(kb) * kSfStageBytes, kSfStageBytes,
+                           &smem->full[stage]);
+              if (!half_item)
+                bulk_load_1d(smem->sfb[stage] + kSfStageBytes, sf_src2 + static_cast<size_t>(kb) * kSfStageBytes,
+                             kSfStageBytes, &smem->full[stage]);
             } else {
               bulk_load_1d(smem->sfb[stage], sf_src + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes,
                            &smem->full[stage]);
@@ -365,6 +370,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                       wait_or_abort<false>(&smem->acc_empty[acc_stage], acc_phase ^ 1u, smem, p.status)))
         break;
       const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc_stage * kTileN);
+      const bool half_item = kMode == kGeglu && item.n_tile == p.n_tiles - 1;
       bool ok = true;
       tc_fence_after_sync();  // the epilogue's tensor-memory loads of this accumulator are done
       for (int kb = 0; kb < p.k_blocks; kb += kAtoms) {
@@ -395,6 +401,8 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               else if (p.last_mmas == 3) issue_k_block_fp8<3>(tmem_acc, aa, bb, hi_ab, accumulate);
               else if (p.last_mmas == 2) issue_k_block_fp8<2>(tmem_acc, aa, bb, hi_ab, accumulate);
               else issue_k_block_fp8<1>(tmem_acc, aa, bb, hi_ab, accumulate);
+            } else if (kMode == kGeglu && half_item) {
+              issue_mmas<4, kN, kMode == kGeglu>(tmem_acc, ts, aa, bb, hi_ab, accumulate);
             } else if (k != p.k_blocks - 1 || full_last) {
               issue_mmas<4, kN>(tmem_acc, ts, aa, bb, hi_ab, accumulate);
             } else if (p.last_mmas == 3) {
@@ -438,6 +446,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       for (int round = 0; ok && round < rounds; ++round) {
         WorkItem item;
         if (!work_item<kMode, kN>(round, total_items, m_tiles, p.n_tiles, tile_first, item)) continue;
+        const bool half_item = kMode == kGeglu && item.n_tile == p.n_tiles - 1;
         for (int kb = 0; kb < p.k_blocks; kb += kAtoms) {
           ok = wait_or_abort<false>(&smem->full[stage], phase, smem, p.status);
           if (!ok) break;
@@ -452,7 +461,8 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               const uint32_t sa = sfa_lo + atom * (kSfStageBytes >> 4);
               const uint32_t sb = sfb_lo + atom * (Shape::kWeightSfBytes >> 4);
               const uint32_t ts = tmem_sf + atom * Shape::kSfColumns;
-              if (k != p.k_blocks - 1 || full_last) issue_sf_copies<4, kN>(ts, sa, sb, hi_sf);
+              if (kMode == kGeglu && half_item) issue_sf_copies<4, kN, kMode == kGeglu>(ts, sa, sb, hi_sf);
+              else if (k != p.k_blocks - 1 || full_last) issue_sf_copies<4, kN>(ts, sa, sb, hi_sf);
               else if (p.last_mmas == 3) issue_sf_copies<3, kN>(ts, sa, sb, hi_sf);
               else if (p.last_mmas == 2) issue_sf_copies<2, kN>(ts, sa, sb, hi_sf);
               else issue_sf_copies<1, kN>(ts, sa, sb, hi_sf);
@@ -523,23 +533,24 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                           n_tile * kN + kStoreColumns, p);
         }
       } else {
-        // Fused GeGLU + NVFP4 requantise, wide tile.  Accumulator columns [0,128) are up and
-        // [128,256) gate of intermediate columns [128*n_tile, 128*n_tile+128); this warp owns
-        // the two 16-column blocks 2*sub and 2*sub+1 of them.
+        // Fused GeGLU + NVFP4 requantise, wide tile.  Accumulator columns are [64 up | 64 gate] of unit
+        // 2*n_tile, then of the next one; this warp owns the two 16-column blocks 2*sub and 2*sub+1 of
+        // the item's 128 intermediate columns.
+        const uint32_t tmem_up = tmem_row + (sub >> 1) * 128 + (sub & 1) * 32;
         const float multiplier = p.next_scale_q[expert];
         uint32_t up0[16], gate0[16], up1[16], gate1[16];
-        tmem_load_32x16(tmem_row + sub * 32, up0);
-        tmem_load_32x16(tmem_row + 128 + sub * 32, gate0);
-        tmem_load_32x16(tmem_row + sub * 32 + 16, up1);
-        tmem_load_32x16(tmem_row + 128 + sub * 32 + 16, gate1);
+        tmem_load_32x16(tmem_up, up0);
+        tmem_load_32x16(tmem_up + 64, gate0);
+        tmem_load_32x16(tmem_up + 16, up1);
+        tmem_load_32x16(tmem_up + 80, gate1);
         tmem_load_wait();
         tc_fence_before_sync();
         mbar_arrive(&smem->acc_empty[acc_stage]);
         const bool columns_exist = n_tile * 128 + sub * 32 < kInter;  // the last item is half empty
         if (row_local < rows_valid && columns_exist) {
           uint4 codes;
-          const uint32_t scale0 = geglu_block(up0, gate0, alpha, multiplier, smem->erf_table, codes.x, codes.y);
-          const uint32_t scale1 = geglu_block(up1, gate1, alpha, multiplier, smem->erf_table, codes.z, codes.w);
+          const uint32_t scale0 = geglu_block_fast(up0, gate0, alpha, multiplier, smem->tables, codes.x, codes.y);
+          const uint32_t scale1 = geglu_block_fast(up1, gate1, alpha, multiplier, smem->tables, codes.z, codes.w);
           // the w2 operand: read eleven times by the next launch, so L2 is asked to keep it
           unsigned long long keep_in_l2;
           asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep_in_l2));
@@ -619,11 +630,11 @@ template <int kMode, int kN>
 void launch_variant(const GemmOperands& op, const GemmParams& p, int sm_count, cudaStream_t stream) {
   if (op.serial_launch) {
     grouped_nvfp4_gemm_kernel<kMode, 1, kN><<<sm_count, kGemmThreads, gemm_smem_bytes<kMode, 1, kN>(), stream>>>(
-        op.map_a, op.map_a32, op.map_b, op.map_b64, p);
+        op.map_a, op.map_a32, op.map_b, p);
     return;
   }
   launch_chained(grouped_nvfp4_gemm_kernel<kMode, 1, kN>, dim3(sm_count), dim3(kGemmThreads),
-                 gemm_smem_bytes<kMode, 1, kN>(), stream, op.map_a, op.map_a32, op.map_b, op.map_b64, p);
+                 gemm_smem_bytes<kMode, 1, kN>(), stream, op.map_a, op.map_a32, op.map_b, p);
 }
 }  // namespace
 
@@ -679,7 +690,10 @@ void launch_grouped_gemm(const GemmOperands& op, const RoutePlan& plan, int sm_c
     launch_variant<kFp8, 128>(op, p, sm_count, stream);
   } else if (op.fused_geglu) {
     p.n_tiles = kFusedItems;
-    launch_variant<kGeglu, 256>(op, p, sm_count, stream);
+    p.b_scales = op.unit_scales;
+    GemmOperands fused = op;
+    fused.map_b = op.map_b_units;
+    launch_variant<kGeglu, 256>(fused, p, sm_count, stream);
   } else if (op.n_out % 256 == 0) {
     p.n_tiles = op.n_out / 256;
     launch_variant<kPlain, 256>(op, p, sm_count, stream);

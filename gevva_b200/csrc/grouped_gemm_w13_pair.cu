@@ -33,7 +33,7 @@ namespace gv {
 
 namespace {
 
-constexpr int kWpStages = 5;
+constexpr int kWpStages = 4;
 constexpr int kWpThreads = (2 + 4 * kEpilogueWarpsPerQuarter) * 32;     // 576: leaves 112 registers per thread
 constexpr uint32_t kWpTmemColumns = 512;
 constexpr uint32_t kWpSfColumn = 256;          // accumulator: columns [0, 256)
@@ -58,7 +58,7 @@ struct alignas(1024) WpSmem {
   uint32_t tmem_base;
   volatile int abort;
   int group_left[4];
-  alignas(16) float erf_table[GV_ERF_TABLE_FLOATS];
+  GegluTables tables;
 };
 
 constexpr size_t kWpSmemBytes = sizeof(WpSmem) + 1024;
@@ -203,25 +203,6 @@ __device__ __forceinline__ int wp_lower_bound(const int* __restrict__ pair_tile,
   return lo;
 }
 
-__device__ __forceinline__ float wp_bf16_lo(uint32_t pair) { return __uint_as_float(pair << 16); }
-__device__ __forceinline__ float wp_bf16_hi(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
-
-// GeGLU and block quantisation of 16 columns of one token from values already rounded to bf16
-// (what the reference's GEMM stores and its GeGLU kernel reads back, src/nvfp4_cutlass.cu:582-583).
-__device__ __forceinline__ uint32_t wp_geglu_block(const uint4& u0, const uint4& u1, const uint4& g0, const uint4& g1,
-                                                   float multiplier, const float* erf_table, uint32_t& codes_lo,
-                                                   uint32_t& codes_hi) {
-  const uint32_t up[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-  const uint32_t gate[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-  float values[16];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    values[2 * i] = __fmul_rn(gv_gelu_erf(wp_bf16_lo(gate[i]), erf_table), wp_bf16_lo(up[i]));
-    values[2 * i + 1] = __fmul_rn(gv_gelu_erf(wp_bf16_hi(gate[i]), erf_table), wp_bf16_hi(up[i]));
-  }
-  return quantize_block16(values, multiplier, codes_lo, codes_hi);
-}
-
 struct WpTokenMaps {
   CUtensorMap rows[16];   // boxes of 8, 16, ... 128 token rows x 128 bytes
 };
@@ -270,7 +251,9 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
     tmem_alloc(&smem->tmem_base, kWpTmemColumns);  // the whole tensor memory: both CTAs get address 0
     tmem_relinquish();
   }
-  load_erf_table(smem->erf_table);
+  load_geglu_tables(&smem->tables);
+  __syncthreads();
+  fill_geglu_tables(&smem->tables);
   grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
@@ -489,7 +472,9 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
         const uint4 g0 = *reinterpret_cast<const uint4*>(row + (((8 + 2 * b) ^ swz) << 4));
         const uint4 g1 = *reinterpret_cast<const uint4*>(row + (((8 + 2 * b + 1) ^ swz) << 4));
         uint2 codes;
-        uint32_t scale = wp_geglu_block(u0, u1, g0, g1, multiplier, smem->erf_table, codes.x, codes.y);
+        const uint32_t ups[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+        const uint32_t gates[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+        uint32_t scale = geglu_block_of_bf16(ups, gates, multiplier, &smem->tables, codes.x, codes.y);
         const int token = 128 * pass + 32 * group + t;
         const bool valid = token < item.valid;
         if (valid)

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gv_exact.h"
 #include "gv_transcendentals.h"
 
 namespace gv {
@@ -66,6 +67,13 @@ __device__ __forceinline__ uint32_t encode_e4m3(float value) {
 __device__ __forceinline__ uint32_t encode_e2m1x2(float first, float second) {
   return static_cast<uint32_t>(
       __nv_cvt_float2_to_fp4x2(float2{first, second}, __NV_E2M1, cudaRoundNearest));
+}
+
+// multiplier / (value of an E4M3 scale), 0 for scale 0, by division: for multipliers outside the range
+// of gv_scale_inverse (gv_exact.h).
+__device__ __forceinline__ float scale_inverse_divided(float multiplier, uint32_t scale) {
+  const float rounded = decode_e4m3(scale);
+  return rounded == 0.0f ? 0.0f : __fdiv_rn(multiplier, rounded);
 }
 
 // NVFP4 block quantiser for 16 values held in registers
@@ -247,6 +255,15 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tensor_m
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"(tensor_map), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      : "memory");
+}
+
+// The same with three coordinates.
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tensor_map, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tensor_map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 

@@ -114,7 +114,130 @@ __device__ __forceinline__ uint32_t geglu_block(const uint32_t (&up)[16], const 
   return quantize_block16(values, multiplier, codes_lo, codes_hi);
 }
 
+// The same arithmetic in a third of the instructions, for the kernels that keep its tables.
+//
+// At FP4 rates the GELU and quantisation of one output value cost as many issue slots as its 5632
+// multiply-adds cost tensor cycles, so what a value costs matters: 24 instructions of erf (two of
+// them conversions at a quarter of the rate, two 16-byte table loads that take seven shared-memory
+// wavefronts each) become one 4-byte load.  That works because the gate has been rounded to bf16: erf's
+// argument takes a few thousand values, and `erf_of` holds gv_erff for every bf16 magnitude from 2^-14 up
+// to where it is 1.  Smaller magnitudes (one gate in 20000 of unit variance) send the whole block
+// through the polynomial.  The results are gv_gelu_erf's and quantize_block16's, bit for bit.
+constexpr int kErfFirst = (127 - 14) << 7;                    // bf16 bits of 2^-14
+constexpr int kErfEntries = 16 * 128 + 54 + 2;                // up to 4 * sqrt(2), where |x| / sqrt(2) >= 4 and erf is 1
+
+struct GegluTables {
+  float erf_of[kErfEntries];
+  alignas(16) float reciprocals[GV_RECIPROCAL_FLOATS];
+  alignas(16) float erf_table[GV_ERF_TABLE_FLOATS];
+};
+static __constant__ float g_reciprocals[GV_RECIPROCAL_FLOATS] = GV_RECIPROCALS_INIT;
+
+// Two steps with a block barrier after each (the second reads what the first wrote).
+__device__ __forceinline__ void load_geglu_tables(GegluTables* tables) {
+  load_erf_table(tables->erf_table);
+  if (threadIdx.x < GV_RECIPROCAL_FLOATS) tables->reciprocals[threadIdx.x] = g_reciprocals[threadIdx.x];
+}
+__device__ __forceinline__ void fill_geglu_tables(GegluTables* tables) {
+  for (int i = threadIdx.x; i < kErfEntries; i += blockDim.x)
+    tables->erf_of[i] = gv_erff(__fmul_rn(__uint_as_float(static_cast<uint32_t>(kErfFirst + i) << 16), 0.7071067811865475f),
+                                tables->erf_table);
+}
+
+// erf-GELU of a bf16 value from erf of its magnitude (gv_gelu_erf's last three operations).
+__device__ __forceinline__ float gelu_from_erf(float value, float erf_of_magnitude) {
+  return __fmul_rn(__fmul_rn(0.5f, value), __fadd_rn(1.0f, copysignf(erf_of_magnitude, value)));
+}
+
+// Index of a bf16 magnitude (15 bits) in erf_of; negative where the table does not reach.
+__device__ __forceinline__ int erf_index(uint32_t magnitude) {
+  return min(static_cast<int>(magnitude) - kErfFirst, kErfEntries - 1);
+}
+
+__device__ __forceinline__ float gelu_of_bf16(float value, const GegluTables* tables) {
+  const int index = erf_index((__float_as_uint(value) >> 16) & 0x7fffu);
+  return index >= 0 ? gelu_from_erf(value, tables->erf_of[index]) : gv_gelu_erf(value, tables->erf_table);
+}
+
+// quantize_block16 with the divisions of gv_exact.h.
+__device__ __forceinline__ uint32_t quantize_block16_fast(const float (&values)[16], float multiplier,
+                                                          const float* reciprocals, uint32_t& codes_lo,
+                                                          uint32_t& codes_hi) {
+  float maximum = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) maximum = fmaxf(maximum, fabsf(values[i]));
+  const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
+  const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, reciprocals)
+                                                           : scale_inverse_divided(multiplier, scale);
+  uint32_t words[2];
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const float* v = values + 8 * half;
+    asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+        "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+        : "=r"(words[half])
+        : "f"(__fmul_rn(v[0], inverse)), "f"(__fmul_rn(v[1], inverse)), "f"(__fmul_rn(v[2], inverse)),
+          "f"(__fmul_rn(v[3], inverse)), "f"(__fmul_rn(v[4], inverse)), "f"(__fmul_rn(v[5], inverse)),
+          "f"(__fmul_rn(v[6], inverse)), "f"(__fmul_rn(v[7], inverse)));
+  }
+  codes_lo = words[0];
+  codes_hi = words[1];
+  return scale;
+}
+
+// One 16-value block from up and gate values already rounded to bf16, two to a word.
+__device__ __forceinline__ uint32_t geglu_block_of_bf16(const uint32_t (&ups)[8], const uint32_t (&gates)[8],
+                                                        float multiplier, const GegluTables* tables,
+                                                        uint32_t& codes_lo, uint32_t& codes_hi) {
+  int smallest = 0;  // its sign bit: some magnitude lies below the table
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    smallest |= (static_cast<int>(gates[i] & 0x7fffu) - kErfFirst) | (static_cast<int>((gates[i] >> 16) & 0x7fffu) - kErfFirst);
+  float values[16];
+  if (smallest >= 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      values[2 * i] = gelu_from_erf(__uint_as_float(gates[i] << 16), tables->erf_of[erf_index(gates[i] & 0x7fffu)]);
+      values[2 * i + 1] =
+          gelu_from_erf(__uint_as_float(gates[i] & 0xffff0000u), tables->erf_of[erf_index((gates[i] >> 16) & 0x7fffu)]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      values[2 * i] = gv_gelu_erf(__uint_as_float(gates[i] << 16), tables->erf_table);
+      values[2 * i + 1] = gv_gelu_erf(__uint_as_float(gates[i] & 0xffff0000u), tables->erf_table);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    values[2 * i] = __fmul_rn(values[2 * i], __uint_as_float(ups[i] << 16));
+    values[2 * i + 1] = __fmul_rn(values[2 * i + 1], __uint_as_float(ups[i] & 0xffff0000u));
+  }
+  return quantize_block16_fast(values, multiplier, tables->reciprocals, codes_lo, codes_hi);
+}
+
+// One 16-value block of one row from the accumulators.
+__device__ __forceinline__ uint32_t geglu_block_fast(const uint32_t (&up)[16], const uint32_t (&gate)[16], float alpha,
+                                                     float multiplier, const GegluTables* tables, uint32_t& codes_lo,
+                                                     uint32_t& codes_hi) {
+  uint32_t gates[8], ups[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    gates[i] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(gate[2 * i])), __fmul_rn(alpha, __uint_as_float(gate[2 * i + 1])));
+    ups[i] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(up[2 * i])), __fmul_rn(alpha, __uint_as_float(up[2 * i + 1])));
+  }
+  return geglu_block_of_bf16(ups, gates, multiplier, tables, codes_lo, codes_hi);
+}
+
 constexpr int kFusedItems = (kInter + 127) / 128;  // 6
+// w13 scales re-tiled by unit of 64 intermediate columns (64 up rows, 64 gate rows): [expert][unit][K block
+// of 256][2 KiB]; the twelfth unit of an expert pads it to pairs.
+constexpr int kUnits = kInter / 64;                // 11
+constexpr int kUnitSlots = kUnits + 1;
 
 
 // Instruction descriptor: E2M1 x E2M1 (format 1 in the mxf4 kinds), both K-major,
@@ -134,8 +257,9 @@ constexpr uint32_t kInstrDesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(
 //   hi_ab / hi_sf   high words (stride, version, swizzle) shared by all stages
 // Scale columns of a K block in tensor memory: at N = 128, A of MMA j at +4j and B at +16+4j;
 // at N = 256, A at +16j, B rows 0..127 at +16j+4, B rows 128..255 at +16j+8 (the second half of
-// the weight scales lies 2 KiB = 128 descriptor units after the first in shared memory).
-template <int kMmas, int kN>
+// the weight scales lies 2 KiB = 128 descriptor units after the first in shared memory).  kHalf: the
+// N = 256 layout with only its first 128 weight rows present, for half the tensor time.
+template <int kMmas, int kN, bool kHalf = false>
 __device__ __forceinline__ void issue_sf_copies(uint32_t tmem_sf, uint32_t sfa_lo, uint32_t sfb_lo, uint32_t hi_sf) {
   static_assert(kMmas >= 1 && kMmas <= 4, "a K block holds one to four MMAs");
 #define GV_SF_OPERANDS ::"r"(tmem_sf), "r"(sfa_lo), "r"(sfb_lo), "r"(hi_sf) : "memory"
@@ -153,26 +277,32 @@ __device__ __forceinline__ void issue_sf_copies(uint32_t tmem_sf, uint32_t sfa_l
     if constexpr (kMmas >= 4) asm volatile(GV_SF_PROLOGUE GV_SF_COPY(3) "}" GV_SF_OPERANDS);
 #undef GV_SF_COPY
   } else {
-#define GV_SF_COPY(j)                                                        \
-  GV_SF_ONE("%1", #j "*32", #j "*16") GV_SF_ONE("%2", #j "*32", "4+" #j "*16") \
-  GV_SF_ONE("%2", "128+" #j "*32", "8+" #j "*16")
+#define GV_SF_COPY(j) GV_SF_ONE("%1", #j "*32", #j "*16") GV_SF_ONE("%2", #j "*32", "4+" #j "*16")
     asm volatile(GV_SF_PROLOGUE GV_SF_COPY(0) "}" GV_SF_OPERANDS);
     if constexpr (kMmas >= 2) asm volatile(GV_SF_PROLOGUE GV_SF_COPY(1) "}" GV_SF_OPERANDS);
     if constexpr (kMmas >= 3) asm volatile(GV_SF_PROLOGUE GV_SF_COPY(2) "}" GV_SF_OPERANDS);
     if constexpr (kMmas >= 4) asm volatile(GV_SF_PROLOGUE GV_SF_COPY(3) "}" GV_SF_OPERANDS);
 #undef GV_SF_COPY
+    if constexpr (!kHalf) {
+#define GV_SF_COPY(j) GV_SF_ONE("%2", "128+" #j "*32", "8+" #j "*16")
+      asm volatile(GV_SF_PROLOGUE GV_SF_COPY(0) "}" GV_SF_OPERANDS);
+      if constexpr (kMmas >= 2) asm volatile(GV_SF_PROLOGUE GV_SF_COPY(1) "}" GV_SF_OPERANDS);
+      if constexpr (kMmas >= 3) asm volatile(GV_SF_PROLOGUE GV_SF_COPY(2) "}" GV_SF_OPERANDS);
+      if constexpr (kMmas >= 4) asm volatile(GV_SF_PROLOGUE GV_SF_COPY(3) "}" GV_SF_OPERANDS);
+#undef GV_SF_COPY
+    }
   }
 #undef GV_SF_ONE
 #undef GV_SF_PROLOGUE
 #undef GV_SF_OPERANDS
 }
 
-template <int kMmas, int kN>
+template <int kMmas, int kN, bool kHalf = false>
 __device__ __forceinline__ void issue_mmas(uint32_t tmem_acc, uint32_t tmem_sf, uint32_t a_lo, uint32_t b_lo,
                                            uint32_t hi_ab, uint32_t accumulate) {
   static_assert(kMmas >= 1 && kMmas <= 4, "a K block holds one to four MMAs");
 #define GV_OPERANDS                                                                                  \
-  ::"r"(tmem_acc), "r"(tmem_sf), "r"(a_lo), "r"(b_lo), "r"(hi_ab), "r"(kInstrDesc<kN>), "r"(accumulate) \
+  ::"r"(tmem_acc), "r"(tmem_sf), "r"(a_lo), "r"(b_lo), "r"(hi_ab), "r"(kInstrDesc<kHalf ? kN / 2 : kN>), "r"(accumulate) \
   : "memory"
 #define GV_PROLOGUE "{\n\t.reg .pred p, pt;\n\t.reg .b32 lo, ta, tb;\n\t.reg .b64 d0, d1;\n\t" \
                     "setp.ne.b32 p, %6, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"

@@ -81,7 +81,8 @@ struct GemmOperands {
   CUtensorMap map_a;        // [row capacity, K/2] bytes, box 128 x 128 B, 128B swizzle
   CUtensorMap map_a32;      // same matrix through a 32-row box (groups of at most 32 rows)
   CUtensorMap map_b;        // [128*N, K/2] bytes, same box
-  CUtensorMap map_b64;      // fused w13 form only: the same matrix through a 64-row box
+  CUtensorMap map_b64;      // CTA-pair fused w13 form: the same matrix through a 64-row box
+  CUtensorMap map_b_units;  // fused w13 form: [experts * 2 halves, 704 rows, 1408 bytes], box 2 x 64 rows x 128 B
   CUtensorMap map_a_sf;     // CTA-pair form: a_scales as [atoms of 512 B][128 x u32], box of four atoms
   CUtensorMap map_b_sf;     // CTA-pair form: b_scales likewise; box of eight atoms (fused w13) or four (w2)
   const uint8_t* a_scales;  // activation scale regions
@@ -91,10 +92,11 @@ struct GemmOperands {
   const unsigned long long* row_dest;  // optional: per-row output address instead of `out`
   int n_out;                // N: 1408 or 2816
   int k_in;                 // K: 2816 or 704
-  // Fused w13 form (GeGLU + requantise in the epilogue, no bf16 output): b_scales is the
-  // re-tiled copy made by launch_retile_w13_scales, map_b64 serves the last, half-filled item
-  // of each row tile, and the results go to the w2 operand buffers below.
+  // Fused w13 form (GeGLU + requantise in the epilogue, no bf16 output): weights through map_b_units
+  // with unit_scales, results to the w2 operand buffers below.  (As CTA pairs: map_b, map_b64 and
+  // the copy made by launch_retile_w13_scales in b_scales.)
   bool fused_geglu;
+  const uint8_t* unit_scales;  // launch_retile_w13_unit_scales
   bool serial_launch;         // launch the ordinary way: no start before the stream's previous kernel ends
   bool use_pairs;             // NVFP4 forms with 256 weight rows per item: run as CTA pairs (tcgen05 cta_group::2)
                               // when the plan carries a pair list
@@ -116,6 +118,9 @@ void launch_retile_w13_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int
 // swizzle; bytes out of range read as zero.  False if the driver entry point is missing.
 bool make_operand_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
                              int box_rows);
+
+// w13 codes [experts, 2 halves, 704 rows, 1408 bytes] through a box of both halves x 64 rows x 128 bytes.
+bool make_w13_unit_tensor_map(CUtensorMap* map, const void* base, uint64_t experts);
 
 // Scale-factor bytes seen as rows of one 512-byte atom each (128 x u32), through a box of
 // `box_atoms` consecutive atoms; no swizzle.

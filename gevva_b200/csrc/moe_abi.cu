@@ -199,6 +199,9 @@ int make_scratch(int tokens, Scratch** out) {
 }  // namespace
 
 namespace gv {
+bool make_w13_unit_tensor_map(CUtensorMap* map, const void* base, uint64_t experts) {
+  return make_w13_unit_map(map, base, experts);
+}
 bool make_operand_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
                              int box_rows) {
   return make_operand_map(map, base, rows, row_bytes, box_rows);
@@ -229,9 +232,9 @@ struct gevva_moe {
   gv::GemmOperands w13{};        // bf16 output (stage access, debugging)
   gv::GemmOperands w13_fused{};  // GeGLU + requantise in the epilogue (the production path)
   gv::GemmOperands w2{};
-  uint8_t* w13_sf_tiled = nullptr;  // runner-owned re-tiling of weights.w13_sf
+  uint8_t* w13_sf_tiled = nullptr;  // runner-owned re-tiling of weights.w13_sf for the CTA-pair tile kernels
   gv::W13PairOperands w13_pairs{};  // the CTA-pair form of the fused w13 stage
-  uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf for it and for the streaming form
+  uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf by unit of 64 columns
   gv::StreamOperands stream_experts{};  // few rows an expert: both GEMMs in one launch, weights on the MMA's M side
   bool w13_pair_form = false;       // GEVVA_MOE_OPTION_W13_PAIRS, or GEVVA_MOE_W13_PAIRS=1 for a whole process
   int sm_count = 0;
@@ -407,46 +410,43 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   ok = ok && make_operand_map(&m->w2.map_a, s->inter_codes, rows, kInter / 2);
   ok = ok && make_operand_map(&m->w2.map_b, weights->w2, static_cast<uint64_t>(kExperts) * kHidden,
                               kInter / 2);
-  ok = ok && make_operand_map(&m->w13.map_b64, weights->w13, static_cast<uint64_t>(kExperts) * kW13Out,
-                              kHidden / 2, 64);
   if (!ok) {
     gevva_moe_destroy(m);
     std::snprintf(g_error_text, sizeof(g_error_text), "cuTensorMapEncodeTiled failed");
     return GEVVA_MOE_CUDA_ERROR;
   }
-  // The fused w13 epilogue pairs up rows with gate rows inside one MMA tile; its weight
-  // scales are a one-off re-tiling of the caller's tensor (the caller's memory is not touched).
-  cudaError_t tiled_error =
-      cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_tiled), gv::retiled_w13_scale_bytes(kExperts));
-  if (tiled_error == cudaSuccess) {
-    gv::launch_retile_w13_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_tiled, kExperts,
-                                 nullptr);
-    tiled_error = cudaGetLastError();
-  }
-  if (tiled_error == cudaSuccess) tiled_error = cudaStreamSynchronize(nullptr);
-  if (tiled_error != cudaSuccess) {
-    gevva_moe_destroy(m);
-    return cuda_failure(tiled_error, "w13 scale re-tiling");
-  }
-  ok = make_scale_map(&m->w13.map_a_sf, s->input_sf, s->input_sf_bytes, 4) &&
-       make_scale_map(&m->w13.map_b_sf, m->w13_sf_tiled, gv::retiled_w13_scale_bytes(kExperts), 8) &&
-       make_scale_map(&m->w2.map_a_sf, s->inter_sf, s->inter_sf_bytes, 4) &&
-       make_scale_map(&m->w2.map_b_sf, weights->w2_sf, static_cast<uint64_t>(kExperts) * kHidden * (kInter / 16), 4);
-  if (!ok) {
-    gevva_moe_destroy(m);
-    std::snprintf(g_error_text, sizeof(g_error_text), "cuTensorMapEncodeTiled failed (scale maps)");
-    return GEVVA_MOE_CUDA_ERROR;
-  }
+  // The fused w13 epilogues pair up rows with gate rows inside one MMA tile; their weight scales are a
+  // one-off re-tiling of the caller's tensor (the caller's memory is not touched).
   {
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_units), gv::w13_unit_scale_bytes(kExperts));
     if (e == cudaSuccess) {
       gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_units, kExperts, nullptr);
       e = cudaGetLastError();
     }
+    if (e == cudaSuccess && m->pairs) {
+      // the opt-in CTA-pair form of the tile kernels has a tiling of its own
+      e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_tiled), gv::retiled_w13_scale_bytes(kExperts));
+      if (e == cudaSuccess) {
+        gv::launch_retile_w13_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_tiled, kExperts, nullptr);
+        e = cudaGetLastError();
+      }
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
       gevva_moe_destroy(m);
-      return cuda_failure(e, "w13 unit scale re-tiling");
+      return cuda_failure(e, "w13 scale re-tiling");
+    }
+    if (m->pairs) {
+      ok = make_scale_map(&m->w13.map_a_sf, s->input_sf, s->input_sf_bytes, 4) &&
+           make_scale_map(&m->w13.map_b_sf, m->w13_sf_tiled, gv::retiled_w13_scale_bytes(kExperts), 8) &&
+           make_scale_map(&m->w2.map_a_sf, s->inter_sf, s->inter_sf_bytes, 4) &&
+           make_scale_map(&m->w2.map_b_sf, weights->w2_sf, static_cast<uint64_t>(kExperts) * kHidden * (kInter / 16), 4) &&
+           make_operand_map(&m->w13.map_b64, weights->w13, static_cast<uint64_t>(kExperts) * kW13Out, kHidden / 2, 64);
+      if (!ok) {
+        gevva_moe_destroy(m);
+        std::snprintf(g_error_text, sizeof(g_error_text), "cuTensorMapEncodeTiled failed (pair maps)");
+        return GEVVA_MOE_CUDA_ERROR;
+      }
     }
     gv::StreamOperands& st = m->stream_experts;
     ok = make_w13_unit_map(&st.map_w13, weights->w13, kExperts);
@@ -502,7 +502,9 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   m->w13.n_out = kW13Out;
   m->w13.k_in = kHidden;
   m->w13_fused = m->w13;
-  m->w13_fused.b_scales = m->w13_sf_tiled;
+  m->w13_fused.b_scales = m->w13_sf_tiled;  // pairs only
+  m->w13_fused.map_b_units = m->stream_experts.map_w13;
+  m->w13_fused.unit_scales = m->w13_sf_units;
   m->w13_fused.out = nullptr;
   m->w13_fused.fused_geglu = true;
   m->w13_fused.next_codes = s->inter_codes;
