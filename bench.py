@@ -153,7 +153,7 @@ def launches_per_step(world, tokens, sm_count=148, ep_chunks=2, ep_parts=1):
     (gevva_moe_launch_stages in csrc/moe_abi.cu, the four gevva_moe_ep_* calls in csrc/ep.cu)."""
     sort = 1 if tokens * TOP_K <= 1024 or (tokens * TOP_K + 1023) // 1024 <= sm_count else 3
     if world == 1:
-        if tokens <= 128:
+        if tokens <= 2 * sm_count:
             return 1 + 1 + 1          # fused router; sort, quantiser and both expert GEMMs in one launch; reduce
         if tokens <= 640:
             return 1 + sort + 1 + 2   # fused router; sort; quantise; both expert GEMMs in one launch; reduce

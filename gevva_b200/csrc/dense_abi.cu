@@ -35,8 +35,7 @@ struct gevva_dense {
 
 int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
                         int sm_count) {
-  gv::launch_dense_plan(tokens, d->plan, stream);
-  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, stream);
+  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, d->plan, stream);
   gv::launch_grouped_gemm(d->gate_up, d->plan, sm_count, stream);
   gv::launch_gelu_quantize_fp8(d->gate_up_out, d->act_scales, d->weights.gate_scale, d->weights.up_scale,
                                d->prod_fp8, d->prod_scales, tokens, stream);
@@ -214,8 +213,16 @@ struct LayerWorkspace {
     bytes = used;
   }
 };
-// SMs that the dense MLP of a decode-sized layer gets beside the experts (see gevva_ff_layer_launch).
-constexpr int kDenseSmsBesideDecode = 16;
+// SMs that the dense MLP of a decode-sized layer gets beside the experts.  An expert launch of this size
+// holds its SMs from the router to its end, and its time is that of its weights' way through HBM, which 132
+// SMs fill as well as 148; the 18 MB of dense weights pass meanwhile.  With a few tokens the experts are
+// few and the dense side is the longer chain, so it gets more (whole layers in a graph, us, at 16 / 24 /
+// 32 / 48 SMs: 1 token 51.8 / 43.1 / 43.0 / 33.6, 4 tokens 58.4 / 49.5 / 48.8 / 46.5, 8 tokens 65.5 / 57.9 /
+// 57.5 / 61.9, 16 tokens 74.8 / 76.4 / 77.7 / 82.3, 40 tokens 97.1 / 98.8 / 101.4 / 108.0).
+int dense_sms_beside(int tokens, int sms) {
+  const int wanted = tokens <= 4 ? 48 : tokens <= 8 ? 32 : 16;
+  return wanted * 2 < sms ? wanted : sms / 2;
+}
 }  // namespace
 
 size_t gevva_ff_layer_workspace_bytes(int tokens) { return tokens < 1 ? 0 : LayerWorkspace(nullptr, tokens).bytes; }
@@ -230,14 +237,12 @@ int gevva_ff_layer_launch(const gevva_ff_layer* layer, const void* hidden, void*
   const LayerWorkspace w(workspace, tokens);
   gevva_dense* dense = layer->dense;
   const bool beside = aux_stream != stream;
-  // The dense MLP starts as soon as its input exists, on SMs that the router leaves idle.  A
-  // decode-sized expert launch holds its SMs from the router to its end, so it leaves a few to the
-  // dense side: the experts' time is that of their weights' way through HBM, which 132 SMs fill as
-  // well as 148, and the dense weights (18 MB) pass meanwhile instead of afterwards.
+  // The dense MLP starts as soon as its input exists, on SMs that the router leaves idle; beside a
+  // decode-sized expert launch on SMs of its own.
   const int sms = gv::moe_sm_count(layer->experts);
-  const bool split = beside && tokens <= gv::kFusedSortQuantizeMaxTokens && sms > 2 * kDenseSmsBesideDecode;
-  const int dense_sms = split ? kDenseSmsBesideDecode : sms;
-  const int expert_sms = split ? sms - kDenseSmsBesideDecode : sms;
+  const bool split = beside && tokens <= gv::kFusedSortQuantizeMaxTokens && sms > 1;
+  const int dense_sms = split ? dense_sms_beside(tokens, sms) : sms;
+  const int expert_sms = split ? sms - dense_sms : sms;
   gv::launch_ff_prepare(hidden, layer->dense_pre, layer->expert_pre, layer->router_scale, w.dense_in, w.expert_in,
                         w.router_in, tokens, stream);
   if (beside) {

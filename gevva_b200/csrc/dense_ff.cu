@@ -81,6 +81,8 @@ ff_prepare_kernel(const __nv_bfloat16* __restrict__ input, const __nv_bfloat16* 
                   const __nv_bfloat16* __restrict__ router_scale, __nv_bfloat16* __restrict__ dense_out,
                   __nv_bfloat16* __restrict__ expert_out, __nv_bfloat16* __restrict__ router_out) {
   __shared__ float scratch[kRowThreads / 32 + 1];
+  grid_launch_dependents();
+  grid_dependency_wait();
   const size_t base = static_cast<size_t>(blockIdx.x) * kHidden;
   float x[8], dw[8], ew[8], rs[8];
   unpack8(__ldg(reinterpret_cast<const uint4*>(input + base) + threadIdx.x), x);
@@ -128,8 +130,13 @@ __device__ __forceinline__ uint2 encode_e4m3x8(const float* v, float inverse) {
 
 __global__ void __launch_bounds__(kRowThreads)
 fp8_quantize_rows_kernel(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ out,
-                         float* __restrict__ scales) {
+                         float* __restrict__ scales, int rows, RoutePlan plan) {
   __shared__ float scratch[kRowThreads / 32 + 1];
+  __shared__ int scan_scratch[16];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  // the projections are grouped GEMMs with a single "expert" that owns every row: their plan
+  if (blockIdx.x == 0 && threadIdx.x < kExperts) publish_groups(threadIdx.x == 0 ? rows : 0, rows, plan, scan_scratch);
   const size_t base = static_cast<size_t>(blockIdx.x) * kHidden;
   float x[8];
   unpack8(__ldg(reinterpret_cast<const uint4*>(input + base) + threadIdx.x), x);
@@ -148,6 +155,8 @@ gelu_quantize_fp8_kernel(const __nv_bfloat16* __restrict__ gate_up,
                          const float* __restrict__ activation_scales, float gate_w_scale,
                          float up_w_scale, uint8_t* __restrict__ out, float* __restrict__ scales) {
   __shared__ float scratch[kDenseThreads / 32 + 1];
+  grid_launch_dependents();
+  grid_dependency_wait();
   const int row = blockIdx.x;
   const bool active = threadIdx.x < kDense / 8;
   const float gate_scale = __fmul_rn(activation_scales[row], gate_w_scale);
@@ -187,6 +196,8 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
                    const float* __restrict__ dense_activation_scales,
                    const float* __restrict__ dense_projection_scale) {
   __shared__ float scratch[kRowThreads / 32 + 1];
+  grid_launch_dependents();
+  grid_dependency_wait();
   const int row = blockIdx.x;
   const size_t base = static_cast<size_t>(row) * kHidden;
   float d[8], e[8], w[8];
@@ -238,12 +249,6 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
   reinterpret_cast<uint4*>(output + base)[threadIdx.x] = pack8(out);
 }
 
-// Plan of a dense GEMM seen as a grouped one with a single "expert" that owns every row.
-__global__ void __launch_bounds__(kExperts) dense_plan_kernel(int rows, RoutePlan plan) {
-  __shared__ int scan_scratch[16];
-  publish_groups(threadIdx.x == 0 ? rows : 0, rows, plan, scan_scratch);
-}
-
 __global__ void fp8_amax_kernel(const float* __restrict__ w, size_t count, unsigned int* amax_bits) {
   float maximum = 0.0f;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
@@ -269,23 +274,23 @@ void launch_ff_prepare(const void* input, const void* dense_weight, const void* 
                        const void* router_scale, void* dense_out, void* expert_out, void* router_out,
                        int rows, cudaStream_t stream) {
   using B = __nv_bfloat16;
-  ff_prepare_kernel<<<rows, kRowThreads, 0, stream>>>(
-      static_cast<const B*>(input), static_cast<const B*>(dense_weight), static_cast<const B*>(expert_weight),
-      static_cast<const B*>(router_scale), static_cast<B*>(dense_out), static_cast<B*>(expert_out),
-      static_cast<B*>(router_out));
+  launch_chained(ff_prepare_kernel, dim3(rows), dim3(kRowThreads), 0, stream, static_cast<const B*>(input),
+                 static_cast<const B*>(dense_weight), static_cast<const B*>(expert_weight),
+                 static_cast<const B*>(router_scale), static_cast<B*>(dense_out), static_cast<B*>(expert_out),
+                 static_cast<B*>(router_out));
 }
 
-void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows,
+void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows, const RoutePlan& plan,
                               cudaStream_t stream) {
-  fp8_quantize_rows_kernel<<<rows, kRowThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(input), out,
-                                                              scales);
+  launch_chained(fp8_quantize_rows_kernel, dim3(rows), dim3(kRowThreads), 0, stream,
+                 static_cast<const __nv_bfloat16*>(input), out, scales, rows, plan);
 }
 
 void launch_gelu_quantize_fp8(const void* gate_up, const float* activation_scales, float gate_w_scale,
                               float up_w_scale, uint8_t* out, float* scales, int rows,
                               cudaStream_t stream) {
-  gelu_quantize_fp8_kernel<<<rows, kDenseThreads, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(gate_up), activation_scales, gate_w_scale, up_w_scale, out, scales);
+  launch_chained(gelu_quantize_fp8_kernel, dim3(rows), dim3(kDenseThreads), 0, stream,
+                 static_cast<const __nv_bfloat16*>(gate_up), activation_scales, gate_w_scale, up_w_scale, out, scales);
 }
 
 void launch_ff_finalize(const void* dense, const void* dense_weight, const void* expert_routes,
@@ -294,16 +299,11 @@ void launch_ff_finalize(const void* dense, const void* dense_weight, const void*
                         void* output, int rows, const float* dense_activation_scales,
                         const float* dense_projection_scale, cudaStream_t stream) {
   using B = __nv_bfloat16;
-  ff_finalize_kernel<<<rows, kRowThreads, 0, stream>>>(
-      static_cast<const B*>(dense), static_cast<const B*>(dense_weight), static_cast<const B*>(expert_routes),
-      route_weights, inverse_routes, static_cast<const B*>(expert_weight),
-      static_cast<const B*>(combined_weight), static_cast<const B*>(residual),
-      static_cast<const B*>(layer_scalar), static_cast<B*>(output), dense_activation_scales,
-      dense_projection_scale);
-}
-
-void launch_dense_plan(int rows, const RoutePlan& plan, cudaStream_t stream) {
-  dense_plan_kernel<<<1, kExperts, 0, stream>>>(rows, plan);
+  launch_chained(ff_finalize_kernel, dim3(rows), dim3(kRowThreads), 0, stream, static_cast<const B*>(dense),
+                 static_cast<const B*>(dense_weight), static_cast<const B*>(expert_routes), route_weights, inverse_routes,
+                 static_cast<const B*>(expert_weight), static_cast<const B*>(combined_weight),
+                 static_cast<const B*>(residual), static_cast<const B*>(layer_scalar), static_cast<B*>(output),
+                 dense_activation_scales, dense_projection_scale);
 }
 
 void launch_pack_fp8(const float* w, size_t count, uint8_t* out, float* scale_out, cudaStream_t stream) {

@@ -29,11 +29,12 @@
 // waits for nothing, so weight bytes keep arriving across the boundary.  All CTAs are co-resident (one per
 // SM) and no wait can form a cycle.
 //
-// In its kFront form (at most 128 tokens) the kernel also sorts the routes and quantises the input: every
-// CTA counts the batch's at most 1024 routes and derives the group geometry for itself; CTA t < tokens
-// ranks the routes of token t and quantises it with eleven warps, eight columns a thread (88 threads of
+// In its kFront form the kernel also sorts the routes and quantises the input: every CTA ranks the whole
+// batch's routes by a counting sort (13 warps, a stretch of routes each) and derives the group geometry for
+// itself; CTA c quantises tokens c and c + CTAs with eleven warps, eight columns a thread (88 threads of
 // 32 columns took 4.3 us of the chain, this takes about one), then adds one to a counter that the
-// activation side waits for.  Meanwhile the weight side has filled its stages.  The CTA that finishes last
+// activation side waits for.  At 200 tokens that saves 4 us of a layer against launches of their own; with
+// five tokens a CTA it would lose five (613 tokens: 119.5 against 114.1 us).  Meanwhile the weight side has filled its stages.  The CTA that finishes last
 // puts all counters back to zero.
 #include "gv_common.cuh"
 #include "gv_gemm_parts.cuh"
@@ -63,15 +64,20 @@ constexpr int kStDownTiles = kHidden / 128;               // 22 w2 items a chunk
 constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
 constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192
 constexpr int kStDownLastMmas = 3;
-constexpr int kStMaxChunks = 384;
+constexpr int kStMaxChunks = 256;
 constexpr int kStExchangeRows = 32;
+constexpr int kStWarps = kStThreads / 32;
+constexpr int kStOwnTokens = 2;                           // kFront: tokens a CTA quantises, at most
 
 struct alignas(1024) StreamSmem {
   uint8_t a[kStStages][kStWeightBytes];
   uint8_t b[kStStages][kStTokenBytes];
   uint8_t sfa[kStStages][kSfStageBytes];
   uint8_t sfb[kStStages][kSfStageBytes];
-  __nv_bfloat16 exchange[2][kStExchangeRows][128];  // [token][MMA row]
+  union {
+    __nv_bfloat16 exchange[2][kStExchangeRows][128];  // [token][MMA row]
+    int warp_counts[kStWarps][kExperts];              // the sort's, before
+  };
   uint64_t full[kStStages], empty[kStStages], sf_full[kStStages];
   uint64_t acc_full[kStAccStages], acc_empty[kStAccStages];
   volatile int progress[kStEpilogueWarps];  // w13 items whose rows each epilogue warp has stored
@@ -86,11 +92,13 @@ struct alignas(1024) StreamSmem {
   short chunk_expert[kStMaxChunks];
   short chunk_index[kStMaxChunks];  // which chunk of its expert
   int histogram[kExperts];
-  int own_expert[kTopK];
-  int own_rank[kTopK];
-  alignas(16) int route_row[kTopK];
-  alignas(16) float route_multiplier[kTopK];
-  unsigned long long route_scale_base[kTopK];
+  // kFront: the routes of this CTA's tokens
+  int own_expert[kStOwnTokens * kTopK];
+  int own_rank[kStOwnTokens * kTopK];  // among the routes of its warp's stretch with the same expert
+  int own_warp[kStOwnTokens * kTopK];
+  alignas(16) int route_row[kStOwnTokens * kTopK];
+  alignas(16) float route_multiplier[kStOwnTokens * kTopK];
+  unsigned long long route_scale_base[kStOwnTokens * kTopK];
   float scale_q1[kExperts];
   GegluTables tables;
 };
@@ -225,9 +233,10 @@ __device__ __forceinline__ bool stream_wait_counter(const int* counter, int targ
   return __all_sync(0xffffffffu, ready);
 }
 
-// This CTA's token by 352 threads, eight columns each (`raw`; two threads a 16-value block): the codes and
-// scale bytes of its eight routes go to their sorted rows.  The arithmetic of quantize_routes_of_token.
-__device__ __forceinline__ void stream_quantise_token(const StreamParams& p, const StreamSmem* smem, int q, const uint4& raw) {
+// One token by 352 threads, eight columns each (`raw`; two threads a 16-value block): the codes and
+// scale bytes of its eight routes (entries first..first+7 of the route arrays) go to their sorted rows.  The arithmetic of quantize_routes_of_token.
+__device__ __forceinline__ void stream_quantise_token(const StreamParams& p, const StreamSmem* smem, int first, int q,
+                                                      const uint4& raw) {
   float values[8];
   unpack_bf16x8(raw, values);
   float maximum = 0.0f;
@@ -240,9 +249,9 @@ __device__ __forceinline__ void stream_quantise_token(const StreamParams& p, con
   bool have = false;
 #pragma unroll
   for (int k = 0; k < kTopK; ++k) {
-    const int row = smem->route_row[k];
+    const int row = smem->route_row[first + k];
     if (row < 0) continue;
-    const float multiplier = smem->route_multiplier[k];
+    const float multiplier = smem->route_multiplier[first + k];
     if (!have || __float_as_uint(multiplier) != previous) {  // routes of equal static scale share the result
       have = true;
       previous = __float_as_uint(multiplier);
@@ -257,7 +266,7 @@ __device__ __forceinline__ void stream_quantise_token(const StreamParams& p, con
                    (__shfl_down_sync(0xffffffffu, scale, 6) << 24);
     }
     *reinterpret_cast<uint32_t*>(p.packed + static_cast<size_t>(row) * (kHidden / 2) + 4 * q) = codes;
-    if ((q & 7) == 0) *reinterpret_cast<uint32_t*>(p.scales + smem->route_scale_base[k] + scale_offset) = scale_word;
+    if ((q & 7) == 0) *reinterpret_cast<uint32_t*>(p.scales + smem->route_scale_base[first + k] + scale_offset) = scale_word;
   }
 }
 
@@ -299,8 +308,8 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   load_geglu_tables(&smem->tables);
   __syncthreads();
   fill_geglu_tables(&smem->tables);
-  if (kFront && tid < kExperts) smem->histogram[tid] = 0;
-  if (kFront && tid < kTopK) smem->own_rank[tid] = 0;
+  if (kFront)
+    for (int i = tid; i < kStWarps * kExperts; i += kStThreads) (&smem->warp_counts[0][0])[i] = 0;
   grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
@@ -310,31 +319,49 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
 
   // ---------------- group geometry ----------------
   const bool has_token = kFront && cta < p.tokens;
+  const int ctas = gridDim.x;
   uint4 raw = make_uint4(0, 0, 0, 0);
+  float scale_q1 = 0.0f;
   if constexpr (kFront) {
-    const int routes = p.tokens * kTopK;
-    int mine[kTopK];
-    // the token itself and the static scales are on their way while the geometry is worked out
+    // the first token and the static scales are on their way while the geometry is worked out
     if (has_token && tid >= 32 && tid < 32 + kStQuantiseThreads)
       raw = __ldg(reinterpret_cast<const uint4*>(p.input + static_cast<size_t>(cta) * kHidden) + (tid - 32));
-    if (has_token && tid < kExperts) smem->scale_q1[tid] = p.in_scale_q1[tid];
-    if (has_token) {
-#pragma unroll
-      for (int k = 0; k < kTopK; ++k) mine[k] = p.expert_ids[cta * kTopK + k];
-      if (tid < kTopK) smem->own_expert[tid] = p.expert_ids[cta * kTopK + tid];
-    }
-    for (int route = tid; route < routes; route += kStThreads) {
-      const int expert = p.expert_ids[route];
+    if (has_token && tid < kExperts) scale_q1 = p.in_scale_q1[tid];
+    // warp w ranks routes [w * stretch, (w + 1) * stretch) among those of its own stretch
+    const int routes = p.tokens * kTopK;
+    const int stretch = ((routes + kStWarps - 1) / kStWarps + 31) & ~31;
+    int* counts = smem->warp_counts[warp];
+    for (int base = warp * stretch; base < (warp + 1) * stretch && base < routes; base += 32) {
+      const int route = base + lane;
+      int expert = route < routes ? p.expert_ids[route] : -1;
       if (expert < 0 || expert >= kExperts) {
-        if (cta == 0) atomicExch(status, static_cast<int>(kBadExpertId));
-        continue;
+        if (cta == 0 && route < routes) atomicExch(status, static_cast<int>(kBadExpertId));
+        expert = kExperts;
       }
-      atomicAdd(&smem->histogram[expert], 1);
-      if (has_token) {
+      const uint32_t peers = __match_any_sync(0xffffffffu, expert);
+      const int before = expert < kExperts ? counts[expert] : 0;
+      __syncwarp();
+      if (expert < kExperts && (peers & (0u - peers)) == (1u << lane)) counts[expert] = before + __popc(peers);
+      __syncwarp();
+      const int token = route >> 3;
+      if (route < routes && token % ctas == cta) {
+        const int slot = token / ctas * kTopK + (route & (kTopK - 1));
+        smem->own_expert[slot] = expert;
+        smem->own_rank[slot] = before + __popc(peers & ((1u << lane) - 1u));
+        smem->own_warp[slot] = warp;
+      }
+    }
+    __syncthreads();
+    if (tid < kExperts) {
+      int running = 0;
 #pragma unroll
-        for (int k = 0; k < kTopK; ++k)
-          if (expert == mine[k] && route < cta * kTopK + k) atomicAdd(&smem->own_rank[k], 1);
+      for (int w = 0; w < kStWarps; ++w) {
+        const int c = smem->warp_counts[w][tid];
+        smem->warp_counts[w][tid] = running;
+        running += c;
       }
+      smem->histogram[tid] = running;
+      smem->scale_q1[tid] = scale_q1;
     }
   } else {
     if (tid < kExperts) smem->histogram[tid] = p.plan.expert_offsets[tid + 1] - p.plan.expert_offsets[tid];
@@ -400,25 +427,33 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   bool ok = true;
 
   if (has_token && warp != kStWeightWarp && warp != kStPublishWarp) {
-    // ---------------- this CTA's token: its routes' rows, then its codes ----------------
+    // ---------------- this CTA's tokens: their routes' rows, then their codes ----------------
     const int q = tid - 32;
-    if (q < kTopK) {
-      const int route = cta * kTopK + q;
+    const int own = (p.tokens - 1 - cta) / ctas + 1;
+    if (q < own * kTopK) {
       const int expert = smem->own_expert[q];
       int dst = -1;
-      if (expert >= 0 && expert < kExperts) {  // others are flagged above
-        dst = smem->offsets[expert] + smem->own_rank[q];
+      if (expert < kExperts) {  // others are flagged above
+        const int route = (cta + q / kTopK * ctas) * kTopK + q % kTopK;
+        const int rank = smem->warp_counts[smem->own_warp[q]][expert] + smem->own_rank[q];
+        dst = smem->offsets[expert] + rank;
         p.plan.sorted_experts[dst] = expert;
         p.plan.sorted_routes[dst] = route;
         p.plan.inverse_routes[route] = dst;
         smem->route_multiplier[q] = smem->scale_q1[expert];
         smem->route_scale_base[q] = static_cast<unsigned long long>(smem->scale_rows[expert]) * (kHidden / 16) +
-                                    sf_offset(smem->own_rank[q], 0, kHidden / 16);
+                                    sf_offset(rank, 0, kHidden / 16);
       }
       smem->route_row[q] = dst;
     }
     named_barrier(1, kStQuantiseThreads);
-    stream_quantise_token(p, smem, q, raw);
+    for (int i = 0; i < own; ++i) {
+      uint4 next = raw;
+      if (i + 1 < own)
+        next = __ldg(reinterpret_cast<const uint4*>(p.input + static_cast<size_t>(cta + (i + 1) * ctas) * kHidden) + q);
+      stream_quantise_token(p, smem, i * kTopK, q, raw);
+      raw = next;
+    }
     named_barrier(1, kStQuantiseThreads);
     if (q == 0) {
       __threadfence();
@@ -432,8 +467,8 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     int stage = 0, issued = 0;
     uint32_t phase = 0;
     if (kFront && !weight_side) {
-      // the w13 operand exists once every token's CTA has quantised its token and counted itself
-      ok = stream_wait_counter(p.plan.front_sync, p.tokens, smem, status);
+      // the w13 operand exists once every CTA with tokens has quantised them and counted itself
+      ok = stream_wait_counter(p.plan.front_sync, p.tokens < ctas ? p.tokens : ctas, smem, status);
       asm volatile("fence.proxy.async.global;" ::: "memory");
     }
     for (int i = 0; ok && i < schedule.count; ++i) {
@@ -752,6 +787,11 @@ StreamMaps make_maps(const StreamOperands& op) {
 
 static_assert(kStRows / 8 == kStreamBoxes, "one map per box height");
 static_assert(kExperts + kStreamMaxTokens * kTopK / kStRows <= kStMaxChunks, "chunk list");
+
+bool stream_layer_fits(int tokens, int sm_count) {
+  return tokens <= kStreamMaxTokens && tokens <= sm_count * kStOwnTokens;
+}
+
 
 int prepare_stream_experts() {
   cudaError_t e = cudaFuncSetAttribute(stream_experts_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

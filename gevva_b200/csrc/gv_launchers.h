@@ -152,7 +152,7 @@ int prepare_w13_pairs();
 // Both expert GEMMs of a batch with few rows an expert in one persistent launch with the weights on the
 // MMA's M side (experts_stream.cu).
 constexpr int kStreamBoxes = 8;         // activation boxes of 8, 16, ... 64 rows
-constexpr int kStreamMaxTokens = 2048;  // the kernel's chunk list; where the launch pays is the caller's rule
+constexpr int kStreamMaxTokens = 1024;  // the kernel's chunk list; where the launch pays is the caller's rule
 struct StreamOperands {
   CUtensorMap map_w13;                 // as W13PairOperands::map_w
   CUtensorMap map_w2;                  // [128 * 2816, 352] bytes, box 128 x 128 B
@@ -169,7 +169,8 @@ struct StreamOperands {
 // On a sorted plan and a quantised input; plan.tile_ready (by expert here) and plan.front_sync zero on
 // entry and on exit.
 void launch_stream_experts(const StreamOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
-// With the route sort and the input quantiser inside; tokens <= min(128, sm_count).
+// With the route sort and the input quantiser inside, where stream_layer_fits.
+bool stream_layer_fits(int tokens, int sm_count);
 void launch_stream_layer(const StreamOperands& op, const RoutePlan& plan, const void* input_bf16, const int* expert_ids,
                          const float* in_scale_q1, uint8_t* packed, uint8_t* scales, int tokens, int sm_count,
                          cudaStream_t stream);
@@ -188,7 +189,8 @@ void launch_pack_weights(const float* weights, int experts, int n_out, int k_in,
 void launch_ff_prepare(const void* input, const void* dense_weight, const void* expert_weight,
                        const void* router_scale, void* dense_out, void* expert_out, void* router_out,
                        int rows, cudaStream_t stream);
-void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows,
+// Also writes the plan of the dense projections seen as grouped GEMMs with one group.
+void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows, const RoutePlan& plan,
                               cudaStream_t stream);
 void launch_gelu_quantize_fp8(const void* gate_up, const float* activation_scales, float gate_w_scale,
                               float up_w_scale, uint8_t* out, float* scales, int rows,
@@ -198,7 +200,6 @@ void launch_ff_finalize(const void* dense, const void* dense_weight, const void*
                         const void* combined_weight, const void* residual, const void* layer_scalar,
                         void* output, int rows, const float* dense_activation_scales,
                         const float* dense_projection_scale, cudaStream_t stream);
-void launch_dense_plan(int rows, const RoutePlan& plan, cudaStream_t stream);
 void launch_pack_fp8(const float* w, size_t count, uint8_t* out, float* scale_out, cudaStream_t stream);
 
 }  // namespace gv

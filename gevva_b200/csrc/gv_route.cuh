@@ -116,4 +116,57 @@ __device__ __forceinline__ void route_top8_quad(const uint32_t (&packed)[16], in
   }
 }
 
+// The same for one token by a whole warp, four logits a lane (experts 4 * lane ..), for launches with a few
+// rows, where the quad's chain of some 600 dependent instructions is the time: lanes sort four, and five
+// exchanges merge whole lists.  Same keys, same operations on the winners, hence the same results.
+__device__ __forceinline__ void route_top8_warp(const uint2& packed, int lane, bool use_rescale, float rescale,
+                                                const __nv_bfloat16* expert_scale, float* __restrict__ weights_row,
+                                                int* __restrict__ ids_row) {
+  uint32_t list[kTopK];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t pair = i < 2 ? packed.x : packed.y;
+    uint32_t bits = (i & 1) ? pair >> 16 : pair & 0xffffu;
+    if (use_rescale)
+      bits = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__uint_as_float(bits << 16), rescale))));
+    list[i] = ((route_key16(bits) << 7) | static_cast<uint32_t>(127 - (4 * lane + i))) + 1u;
+  }
+  route_order(list[0], list[1]);
+  route_order(list[2], list[3]);
+  route_order(list[0], list[2]);
+  route_order(list[1], list[3]);
+  route_order(list[1], list[2]);
+  // two descending fours, one reversed, make a bitonic eight
+#pragma unroll
+  for (int i = 0; i < 4; ++i) list[7 - i] = __shfl_xor_sync(0xffffffffu, list[i], 1);
+#pragma unroll
+  for (int distance = 4; distance >= 1; distance >>= 1) {
+#pragma unroll
+    for (int i = 0; i < kTopK; ++i)
+      if ((i & distance) == 0) route_order(list[i], list[i + distance]);
+  }
+#pragma unroll
+  for (int step = 2; step <= 16; step <<= 1) {
+    uint32_t other[kTopK];
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k) other[k] = __shfl_xor_sync(0xffffffffu, list[k], step);
+    route_merge8(list, other);
+  }
+  const int mine = lane & (kTopK - 1);
+  uint32_t winner = list[0];
+#pragma unroll
+  for (int k = 1; k < kTopK; ++k) winner = mine == k ? list[k] : winner;
+  winner -= 1u;
+  const int id = 127 - static_cast<int>(winner & 127u);
+  const float e = gv_expf(__fsub_rn(route_value_of_key16(winner >> 7), route_value_of_key16((list[0] - 1u) >> 7)));
+  // ((e0+e4)+(e2+e6)) + ((e1+e5)+(e3+e7)), as in the quad form
+  float denominator = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 4));
+  denominator = __fadd_rn(denominator, __shfl_xor_sync(0xffffffffu, denominator, 2));
+  denominator = __fadd_rn(denominator, __shfl_xor_sync(0xffffffffu, denominator, 1));
+  if (lane < kTopK) {
+    ids_row[lane] = id;
+    weights_row[lane] = __fmul_rn(__fdiv_rn(e, denominator), __bfloat162float(expert_scale[id]));
+  }
+}
+
 }  // namespace gv

@@ -239,7 +239,7 @@ struct gevva_moe {
   bool w13_pair_form = false;       // GEVVA_MOE_OPTION_W13_PAIRS, or GEVVA_MOE_W13_PAIRS=1 for a whole process
   int sm_count = 0;
   bool pairs = false;               // GEVVA_MOE_OPTION_PAIRS: prefill-sized launches run the expert GEMMs as CTA pairs
-  bool decode_front = true;         // batches of at most 128 tokens: ... and the route sort and the input quantiser in the same launch (GEVVA_MOE_DECODE_FRONT=0: a launch of their own)
+  bool decode_front = true;         // ... and the route sort and the input quantiser in the same launch (GEVVA_MOE_DECODE_FRONT=0: a launch of their own)
   bool merged_decode = true;        // batches of at most kStreamTokens: w13 and w2 in one launch (GEVVA_MOE_DECODE_MERGED=0: two)
   bool nvtx = false;                // GEVVA_MOE_OPTION_NVTX: one range per stage around its launches
 };
@@ -274,10 +274,16 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   const bool use_pairs = runner->pairs && tokens > gv::kFusedSortQuantizeMaxTokens;
   const unsigned front = GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE;
   const unsigned layer_body = front | GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU | GEVVA_MOE_STAGE_W2;
-  if ((stages & layer_body) == layer_body && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode &&
-      runner->decode_front && tokens <= gv::kFusedSortQuantizeMaxTokens && tokens <= sm_count) {
-    // decode-sized batch: sort, quantiser and both GEMMs in one persistent launch; the weights start
-    // streaming while the input is still being quantised
+  // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side
+  // does both GEMMs.  Up to about 40 rows an expert that is faster than the launches with 128-row tiles
+  // (per layer of two distinct ones, us, one B200, with the sort and the quantiser as launches of their own
+  // on both sides: 129 tokens 101.9 against 111.4, 200 103.4 / 112.5, 450 108.0 / 116.8, 613 114.1 / 121.3,
+  // 800 124.0 / 126.9): above, its GeGLU epilogue, which handles a column of a token per thread through
+  // shared memory, outweighs the weights.
+  const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !runner->pairs &&
+                       !runner->w13_pair_form && tokens <= kStreamTokens;
+  if ((stages & layer_body) == layer_body && streams && runner->decode_front && gv::stream_layer_fits(tokens, sm_count)) {
+    // ... and the route sort and the quantiser; the weights stream while the input is being quantised
     StageRange range(runner->nvtx, "gevva_moe.sort+quantize+w13+geglu+w2");
     gv::launch_stream_layer(runner->stream_experts, s->plan, in, ids, runner->weights.in_scale_q1, s->input_codes,
                             s->input_sf, tokens, sm_count, stream);
@@ -300,13 +306,7 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   }
   const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
   const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
-  // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side
-  // does both GEMMs.  Up to about 40 rows an expert that is faster than the two 128-row-tile launches
-  // (per layer of two distinct ones, us, one B200: 129 tokens 101.9 against 111.4, 200 103.4 / 112.5,
-  // 450 108.0 / 116.8, 613 118.4 / 121.3, 800 137.7 / 126.9): above, its GeGLU epilogue, which handles
-  // a column of a token per thread through shared memory, outweighs the weights.
-  if ((stages & gemms) == gemms && !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !runner->pairs &&
-      !runner->w13_pair_form && tokens <= kStreamTokens) {
+  if ((stages & gemms) == gemms && streams) {
     StageRange range(runner->nvtx, "gevva_moe.w13+geglu+w2");
     gv::launch_stream_experts(runner->stream_experts, s->plan, sm_count, stream);
     stages &= ~gemms;

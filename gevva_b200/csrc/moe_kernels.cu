@@ -23,6 +23,8 @@ route_128_top8_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
                       const __nv_bfloat16* __restrict__ expert_scale, float* __restrict__ weights,
                       int* __restrict__ ids, int rows, const float* __restrict__ activation_scales,
                       const float* __restrict__ projection_weight_scale) {
+  grid_launch_dependents();
+  grid_dependency_wait();
   const int row = blockIdx.x * 32 + (threadIdx.x >> 2);
   const int part = threadIdx.x & 3;
   const bool valid = row < rows;
@@ -52,10 +54,9 @@ route_128_top8_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
 void launch_route(const void* logits_bf16, int ld, const void* expert_scale_bf16, float* weights,
                   int* ids, int tokens, const float* activation_scales,
                   const float* projection_weight_scale, cudaStream_t stream) {
-  route_128_top8_kernel<<<(tokens + 31) / 32, 128, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(logits_bf16), ld,
-      static_cast<const __nv_bfloat16*>(expert_scale_bf16), weights, ids, tokens, activation_scales,
-      projection_weight_scale);
+  launch_chained(route_128_top8_kernel, dim3((tokens + 31) / 32), dim3(128), 0, stream,
+                 static_cast<const __nv_bfloat16*>(logits_bf16), ld, static_cast<const __nv_bfloat16*>(expert_scale_bf16),
+                 weights, ids, tokens, activation_scales, projection_weight_scale);
 }
 
 // ---------------------------------------------------------------------------

@@ -32,23 +32,31 @@ namespace {
 // CTAs per cluster = K slices per token tile: 8 for small batches, else 4, 2 or 1, the largest that
 // keeps the launch within one wave of SMs (a tile's pass is a chain of latencies, so waves cost more
 // than depth)
-constexpr int kRpStages = 5;
 constexpr int kRpThreads = 192;
+constexpr int kSmallTile = 64;
+constexpr int kWarpRows = 8;   // rows of a CTA up to which a warp routes a row (two each); above, a quad of lanes does
 constexpr int kRpTileBytes = kTileM * kTileKBytes;  // 16 KiB: 128 rows of one 128-byte K block
 
+// kRows: token rows of a tile that exist at most.  64 is the form of batches of at most 64 tokens, where
+// the launch is a chain of latencies: its CTA's five or six K blocks all fit the ring (half a token tile
+// each; the MMA reads the next tile's bytes as rows 64..127, whose results nobody looks at).
+template <int kRows>
 struct alignas(1024) RouterSmem {
-  uint8_t a[kRpStages][kRpTileBytes];
-  uint8_t b[kRpStages][kRpTileBytes];
-  // Partial sums of this CTA's 32 rows as received from the four CTAs of the cluster (its own
-  // included): [source][local row][128 floats]; the 16-byte chunks of a row are permuted
+  static constexpr int kStages = kRows == 64 ? 6 : 5;
+  static constexpr int kTokenBytes = kRows * kTileKBytes;
+  uint8_t a[kStages][kTokenBytes];
+  uint8_t b[kStages][kRpTileBytes];
+  // Partial sums of this CTA's rows as received from the CTAs of the cluster (its own included):
+  // [source][local row][128 floats]; the 16-byte chunks of a row are permuted
   // (received_chunk_position) so that neither the row-wise stores nor the reduce's reads, where
   // four lanes share a row, meet in a bank.
-  float received[kTileM * kExperts];   // [kSplit][128 / kSplit rows][128 floats]
-  uint64_t full[kRpStages];
-  uint64_t empty[kRpStages];
+  float received[kRows * kExperts];   // [kSplit][kRows / kSplit rows][128 floats]
+  uint64_t full[kStages];
+  uint64_t empty[kStages];
   uint64_t acc_full;
   uint32_t tmem_base;
   volatile int abort;
+  __nv_bfloat16 expert_scale[kExperts];
 };
 
 // Position of 16-byte chunk `chunk` (0..31) inside local row `row`: the chunk's low three bits are
@@ -59,8 +67,8 @@ __device__ __forceinline__ int received_chunk_position(int chunk, int row) {
   return chunk ^ ((row + 2 * (chunk >> 3)) & 7);
 }
 
-constexpr size_t kRpSmemBytes = sizeof(RouterSmem) + 1024;
-static_assert(kRpSmemBytes <= 232448, "shared memory budget of one sm_100 CTA");
+template <int kRows> constexpr size_t router_smem_bytes() { return sizeof(RouterSmem<kRows>) + 1024; }
+static_assert(router_smem_bytes<64>() <= 232448 && router_smem_bytes<128>() <= 232448, "shared memory budget of one sm_100 CTA");
 
 struct RouterParams {
   const float* bias;                   // optional f32 [128], added before the bf16 rounding
@@ -111,17 +119,19 @@ __device__ __forceinline__ void issue_router_k_block(uint32_t tmem_acc, uint32_t
 #undef GV_RP_MMA
 }
 
-template <bool kFp8, int kSplit>
+template <bool kFp8, int kSplit, int kRows>
 __global__ void __launch_bounds__(kRpThreads, 1)
 route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                      const RouterParams p) {
+  using Smem = RouterSmem<kRows>;
+  constexpr int kRpStages = Smem::kStages;
   extern __shared__ uint8_t smem_raw[];
-  RouterSmem* smem = reinterpret_cast<RouterSmem*>(
+  Smem* smem = reinterpret_cast<Smem*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();
-  constexpr int kOwnRows = kTileM / kSplit;   // tile rows this CTA reduces and routes
+  constexpr int kOwnRows = kRows / kSplit;   // tile rows this CTA reduces and routes
   const int m_tile = static_cast<int>(blockIdx.x) / kSplit;
   const int kb_begin = static_cast<int>(rank) * p.k_blocks / kSplit;
   const int kb_end = (static_cast<int>(rank) + 1) * p.k_blocks / kSplit;
@@ -148,6 +158,12 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = smem->tmem_base;
+  // While the previous kernel drains, this CTA's slice of the router matrix is asked into L2 (a hint: the
+  // loads themselves come after the wait); a model's other weights have pushed it out since last time.
+  if (m_tile == 0 && warp == 0 && elect_one())
+    for (int kb = kb_begin; kb < kb_end; ++kb)
+      asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&map_w), "r"(kb * kTileKBytes), "r"(0)
+                   : "memory");
   grid_dependency_wait();  // the previous kernel of the stream has completed and its writes are visible
 
   if (warp == 0) {
@@ -160,7 +176,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status));
       if (!ok) break;
       if (elect_one()) {
-        mbar_arrive_expect_tx(&smem->full[stage], 2u * kRpTileBytes);
+        mbar_arrive_expect_tx(&smem->full[stage], static_cast<uint32_t>(Smem::kTokenBytes + kRpTileBytes));
         tma_load_2d(smem->a[stage], &map_x, &smem->full[stage], kb * kTileKBytes, m_tile * kTileM);
         tma_load_2d(smem->b[stage], &map_w, &smem->full[stage], kb * kTileKBytes, 0);
       }
@@ -194,7 +210,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     for (int kb = kb_begin; kb < kb_end; ++kb) {
       if (!wait_or_abort<false>(&smem->full[stage], phase, smem, p.status)) break;
       if (leader) {
-        issue_router_k_block<kFp8>(tmem_base, a_lo0 + static_cast<uint32_t>(stage) * (kRpTileBytes >> 4),
+        issue_router_k_block<kFp8>(tmem_base, a_lo0 + static_cast<uint32_t>(stage) * (Smem::kTokenBytes >> 4),
                                    b_lo0 + static_cast<uint32_t>(stage) * (kRpTileBytes >> 4),
                                    kb != kb_begin ? 1u : 0u);
         tc_commit(&smem->empty[stage]);
@@ -207,6 +223,8 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     }
   } else {
     // ---------------- epilogue, part 1: partial sums to the rows' owners ----------------
+    // (the per-expert scale, which part 2 would otherwise look up behind its last comparison)
+    smem->expert_scale[threadIdx.x - 64] = p.expert_scale[threadIdx.x - 64];
     const int quarter = warp & 3;  // the tensor-memory lanes this warp may read
     const int row = quarter * 32 + lane;
     const int owner = row % kSplit;
@@ -244,6 +262,34 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
 
   if (warp >= 2 && !smem->abort) {
     // ---------------- epilogue, part 2: reduce this CTA's rows and route them, 32 at a time ----------------
+    const int tile_rows = p.tokens - m_tile * kTileM;   // may exceed the tile
+    // rows kSplit * i + rank < tile_rows
+    const int own_rows = tile_rows >= kRows ? kOwnRows : (tile_rows - static_cast<int>(rank) + kSplit - 1) / kSplit;
+    if (own_rows <= kWarpRows) {
+      // a few rows: one warp per row, four logits a lane (a third of the quads' chain)
+      for (int row_local = warp - 2; row_local < own_rows; row_local += 4) {
+        const int token = m_tile * kTileM + row_local * kSplit + static_cast<int>(rank);
+        float4 acc = make_float4(0, 0, 0, 0);
+#pragma unroll
+        for (int source = 0; source < kSplit; ++source) {
+          const float4 v = reinterpret_cast<const float4*>(
+              smem->received + (source * kOwnRows + row_local) * kExperts)[received_chunk_position(lane, row_local)];
+          acc = source == 0 ? v
+                            : make_float4(__fadd_rn(acc.x, v.x), __fadd_rn(acc.y, v.y), __fadd_rn(acc.z, v.z), __fadd_rn(acc.w, v.w));
+        }
+        if (p.bias) {
+          const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias) + lane);
+          acc = make_float4(__fadd_rn(acc.x, b.x), __fadd_rn(acc.y, b.y), __fadd_rn(acc.z, b.z), __fadd_rn(acc.w, b.w));
+        }
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y);
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(acc.z, acc.w);
+        const uint2 packed = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        if (p.logits_out) reinterpret_cast<uint2*>(p.logits_out + static_cast<size_t>(token) * kExperts)[lane] = packed;
+        const float rescale = kFp8 ? __fmul_rn(p.activation_scales[token], p.weight_scale[0]) : 1.0f;
+        route_top8_warp(packed, lane, kFp8, rescale, smem->expert_scale, p.weights + static_cast<size_t>(token) * kTopK,
+                        p.ids + static_cast<size_t>(token) * kTopK);
+      }
+    } else {
     const int t = threadIdx.x - 64;
     const int part = t & 3;         // columns [32 * part, 32 * part + 32)
 #pragma unroll 1
@@ -298,8 +344,9 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       }
       // the reference's rescale of an unscaled FP8 GEMM output (routing_sampling.cuh:405-411)
       const float rescale = kFp8 ? __fmul_rn(p.activation_scales[safe_token], p.weight_scale[0]) : 1.0f;
-      route_top8_quad(packed, part, kFp8, rescale, valid, p.expert_scale, p.weights + safe_token * kTopK,
+      route_top8_quad(packed, part, kFp8, rescale, valid, smem->expert_scale, p.weights + safe_token * kTopK,
                       p.ids + safe_token * kTopK);
+    }
     }
   }
 
@@ -312,7 +359,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   }
 }
 
-template <bool kFp8, int kSplit>
+template <bool kFp8, int kSplit, int kRows>
 cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, const RouterParams& p,
                            cudaStream_t stream) {
   static bool prepared[64] = {};
@@ -320,8 +367,8 @@ cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, c
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return e;
   if (device >= 0 && device < 64 && !prepared[device]) {
-    e = cudaFuncSetAttribute(route_project_kernel<kFp8, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kRpSmemBytes));
+    e = cudaFuncSetAttribute(route_project_kernel<kFp8, kSplit, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(router_smem_bytes<kRows>()));
     if (e != cudaSuccess) return e;
     prepared[device] = true;
   }
@@ -329,7 +376,7 @@ cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, c
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(m_tiles * kSplit));
   config.blockDim = dim3(kRpThreads);
-  config.dynamicSmemBytes = kRpSmemBytes;
+  config.dynamicSmemBytes = router_smem_bytes<kRows>();
   config.stream = stream;
   // Clusters of kSplit CTAs; and the launch may begin while the previous kernel of the stream is
   // still running (the kernel waits at grid_dependency_wait before it reads or writes global memory),
@@ -343,17 +390,18 @@ cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, c
   attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = 2;
-  return cudaLaunchKernelEx(&config, route_project_kernel<kFp8, kSplit>, map_x, map_w, p);
+  return cudaLaunchKernelEx(&config, route_project_kernel<kFp8, kSplit, kRows>, map_x, map_w, p);
 }
 
 template <bool kFp8>
 cudaError_t launch_split(const CUtensorMap& map_x, const CUtensorMap& map_w, const RouterParams& p,
                          cudaStream_t stream) {
   const int m_tiles = (p.tokens + kTileM - 1) / kTileM;
-  if (m_tiles <= 4) return launch_variant<kFp8, 8>(map_x, map_w, p, stream);
-  if (m_tiles * 4 <= 160) return launch_variant<kFp8, 4>(map_x, map_w, p, stream);
-  if (m_tiles * 2 <= 160) return launch_variant<kFp8, 2>(map_x, map_w, p, stream);
-  return launch_variant<kFp8, 1>(map_x, map_w, p, stream);
+  if (p.tokens <= kSmallTile) return launch_variant<kFp8, 8, kSmallTile>(map_x, map_w, p, stream);
+  if (m_tiles <= 4) return launch_variant<kFp8, 8, kTileM>(map_x, map_w, p, stream);
+  if (m_tiles * 4 <= 160) return launch_variant<kFp8, 4, kTileM>(map_x, map_w, p, stream);
+  if (m_tiles * 2 <= 160) return launch_variant<kFp8, 2, kTileM>(map_x, map_w, p, stream);
+  return launch_variant<kFp8, 1, kTileM>(map_x, map_w, p, stream);
 }
 
 }  // namespace
@@ -364,7 +412,7 @@ int launch_route_project(const void* x, const void* router_w, bool fp8, const fl
                          cudaStream_t stream) {
   const uint64_t row_bytes = fp8 ? kHidden : 2 * kHidden;
   CUtensorMap map_x, map_w;
-  if (!make_operand_tensor_map(&map_x, x, static_cast<uint64_t>(tokens), row_bytes, kTileM) ||
+  if (!make_operand_tensor_map(&map_x, x, static_cast<uint64_t>(tokens), row_bytes, tokens <= kSmallTile ? kSmallTile : kTileM) ||
       !make_operand_tensor_map(&map_w, router_w, kExperts, row_bytes, kTileM))
     return static_cast<int>(cudaErrorInvalidValue);
   RouterParams p{};
