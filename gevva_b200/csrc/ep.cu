@@ -485,6 +485,7 @@ struct gevva_moe_ep {
   uint8_t* inter_sf = nullptr;
   unsigned long long* row_dest = nullptr;
   unsigned long long* row_dest_local = nullptr;  // measurement aid, allocated on first use
+  uint8_t* w2_sf_down = nullptr;
   uint8_t* w13_sf_units = nullptr;
   // the compute phase runs the local experts in two halves so that the NVLink-bound w2 of the
   // first half overlaps the w13 of the second: a side stream and two events order them
@@ -505,6 +506,7 @@ void gevva_moe_ep_destroy(gevva_moe_ep* ep) {
   cudaFree(ep->inter_sf);
   cudaFree(ep->row_dest);
   cudaFree(ep->row_dest_local);
+  cudaFree(ep->w2_sf_down);
   cudaFree(ep->w13_sf_units);
   if (ep->side) cudaStreamDestroy(ep->side);
   if (ep->fork) cudaEventDestroy(ep->fork);
@@ -589,6 +591,7 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&ep->row_dest), cap * sizeof(unsigned long long));
   if (e == cudaSuccess)
     e = cudaMalloc(reinterpret_cast<void**>(&ep->w13_sf_units), gv::w13_unit_scale_bytes(el));
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&ep->w2_sf_down), gv::retiled_w2_scale_bytes(el));
   if (e != cudaSuccess) {
     gevva_moe_ep_destroy(ep);
     return GEVVA_MOE_CUDA_ERROR;
@@ -640,18 +643,17 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
 
   gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(local_weights->w13_sf), ep->w13_sf_units, el,
                                     nullptr);
+  gv::launch_retile_w2_scales(static_cast<const uint8_t*>(local_weights->w2_sf), ep->w2_sf_down, el, nullptr);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   bool ok = e == cudaSuccess;
   ok = ok && make_map(&ep->w13.map_a, ep->dev.peer_codes[rank], cap, kHidden / 2, kTileM);
   ok = ok && make_map(&ep->w13.map_a32, ep->dev.peer_codes[rank], cap, kHidden / 2, 32);
-  ok = ok && make_map(&ep->w2.map_a32, ep->inter_codes, cap, kInter / 2, 32);
   ok = ok && make_map(&ep->w13.map_b, local_weights->w13, static_cast<uint64_t>(el) * kW13Out,
                       kHidden / 2, kTileM);
   ok = ok && gv::make_w13_unit_tensor_map(&ep->w13.map_b_units, local_weights->w13, static_cast<uint64_t>(el));
   ok = ok && make_map(&ep->w2.map_a, ep->inter_codes, cap, kInter / 2, kTileM);
-  ok = ok && make_map(&ep->w2.map_b, local_weights->w2, static_cast<uint64_t>(el) * kHidden, kInter / 2,
-                      kTileM);
+  ok = ok && gv::make_w2_down_tensor_map(&ep->w2.map_b_down, local_weights->w2, static_cast<uint64_t>(el));
   if (!ok) {
     gevva_moe_ep_destroy(ep);
     return GEVVA_MOE_CUDA_ERROR;
@@ -670,6 +672,7 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
   ep->w2.b_scales = static_cast<const uint8_t*>(local_weights->w2_sf);
   ep->w2.alpha = local_weights->alpha2;
   ep->w2.out = nullptr;
+  ep->w2.down_scales = ep->w2_sf_down;
   ep->w2.row_dest = ep->row_dest;
   ep->w2.n_out = kHidden;
   ep->w2.k_in = kInter;

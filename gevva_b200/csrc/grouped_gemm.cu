@@ -10,17 +10,16 @@
 // the accumulators before anything is written.
 //
 // Mapping.  Tokens (sorted routes) sit on MMA-M, weight rows on MMA-N.  A work
-// item is (128-row tile of one expert) x (kN weight rows), kN = 256 for the two expert
-// GEMMs and 128 elsewhere.  The main loop is bound by how fast one thread can issue
-// tcgen05 instructions (about 90 cycles per MMA with its scale copies, against 64 cycles
-// of tensor-pipe time at N = 128), so the wide tile, which does twice the work per
+// item is (128-row tile of one expert) x (kN weight rows), kN = 256 for the fused w13 form,
+// 128 elsewhere.  An MMA of M = 128 takes at least about 105 cycles whatever its
+// N (measured; 128 at N = 256), so the wide tile, which does twice the work per
 // instruction, is what keeps the tensor pipe fed.  Row tiles are listed
 // in device memory by the route sort; CTAs are persistent and take items
 // round-robin.  Warps 0 and 18 are the TMA producers (activation side, weight side),
 // warp 1 allocates tensor memory and issues the MMAs, warps 2..17 drain accumulators (two
-// accumulator stages at N = 128; at N = 256 one, which the epilogue copies to registers and
-// releases before it does its arithmetic, so the epilogue of one item still overlaps the
-// main loop of the next).  Warps 0 and 1 walk
+// accumulator stages; one in the fused form, whose scales take the other half of tensor memory: the
+// epilogue copies it to registers and releases it before it does its arithmetic, so the epilogue of one
+// item still overlaps the main loop of the next).  Warps 0 and 1 walk
 // their loops as whole warps (warp-uniform addresses) and one elected lane issues.
 //
 // Two epilogues:
@@ -62,21 +61,20 @@ constexpr int kWeightProducerWarp = 2 + 4 * kEpilogueWarpsPerQuarter;
 constexpr int kScaleCopyWarp = kWeightProducerWarp + 1;
 constexpr int kGemmThreads = (kScaleCopyWarp + 1) * 32;
 constexpr uint32_t kTmemColumns = 512;
-// Accumulators take tensor-memory columns [0, 256) in every configuration (2 x 128 or
+// With block scales the accumulators take tensor-memory columns [0, 256) (2 x 128 or
 // 1 x 256); scale factors follow, per pipeline stage and K block: a copy for the next K
 // block must not wait for the MMAs of the previous one to finish reading theirs.
 constexpr uint32_t kSfColumn = 256;
 constexpr int kOperandStageBytes = kTileM * kTileKBytes;  // 16 KiB: 128 rows of one K block
 // A pipeline stage holds kAtoms K blocks of 256 elements (one 128-byte swizzle row each) of
-// 128 activation rows and kN weight rows.  At N = 256 a stage is 54 KiB, so four stages fit
-// (three beside the store staging of the plain epilogue); at N = 128 five.
+// 128 activation rows and kN weight rows.  At N = 256 a stage is 54 KiB (48 without scales), so four
+// stages fit; at N = 128 five.
 template <int kMode, int kAtomsPerStage, int kN> struct StageShape {
   static_assert(kN == 128 || kN == 256, "weight rows per item");
   static_assert(kN == 128 || kAtomsPerStage == 1, "wide tiles take one K block per stage");
   static constexpr int kAtoms = kAtomsPerStage;
-  static constexpr int kStages =
-      kN == 256 ? (kMode == kGeglu ? 4 : 3) : 5;
-  static constexpr int kAccStages = kN == 256 ? 1 : 2;
+  static constexpr int kStages = kN == 256 ? 4 : 5;
+  static constexpr int kAccStages = kMode == kGeglu ? 1 : 2;
   static constexpr int kWeightBytes = kN * kTileKBytes;        // per K block
   static constexpr int kWeightSfBytes = (kN / 128) * kSfStageBytes;
   // Scale-factor columns per K block: at N = 128 sixteen for A then sixteen for B; at N = 256
@@ -109,7 +107,7 @@ struct alignas(1024) GemmSmem {
 template <int kMode, int kAtoms, int kN> constexpr size_t gemm_smem_bytes() {
   return sizeof(GemmSmem<kMode, kAtoms, kN>) + 1024;
 }
-static_assert(gemm_smem_bytes<kPlain, 1, 128>() <= 232448 && gemm_smem_bytes<kPlain, 1, 256>() <= 232448 &&
+static_assert(gemm_smem_bytes<kPlain, 1, 128>() <= 232448 &&
                   gemm_smem_bytes<kGeglu, 1, 256>() <= 232448 && gemm_smem_bytes<kFp8, 1, 128>() <= 232448,
               "shared memory budget of one sm_100 CTA");
 static_assert(kSfColumn + 64 * 4 <= kTmemColumns && kSfColumn + 32 * 6 <= kTmemColumns, "tensor memory budget");
@@ -189,7 +187,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   constexpr int kAtoms = Smem::kAtoms;
   constexpr int kAccStages = Smem::kAccStages;
   constexpr bool kWide = kN == 256;
-  static_assert(kMode != kFp8 || !kWide, "the dense path uses 128-row weight tiles");
+  static_assert(kMode == kGeglu || !kWide, "the other forms use 128-row weight tiles");
   static_assert(kMode != kGeglu || kWide, "the fused form exists for 256-row weight tiles only");
   extern __shared__ uint8_t smem_raw[];
   Smem* smem = reinterpret_cast<Smem*>(
@@ -250,9 +248,9 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const int m_tile = item.m_tile;
       const int n_tile = item.n_tile;
       const int expert = p.tile_expert[m_tile];
-      int row = 0, row2 = 0;
+      int row = 0;
       const uint8_t* sf_src;
-      const uint8_t* sf_src2 = nullptr;  // wide tiles: scales of weight rows 128..255
+      const uint8_t* sf_src2 = nullptr;  // fused form: scales of weight rows 128..255
       bool short_tile = false;  // decode-sized groups: fetch 32 activation rows instead of 128
       bool half_item = false;   // fused form: the last item of a row tile has one unit
       if (!weight_side) {
@@ -267,9 +265,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         sf_src2 = sf_src + static_cast<size_t>(p.k_blocks) * kSfStageBytes;
       } else {
         row = expert * p.n_out + n_tile * kN;
-        row2 = row + 128;
         sf_src = p.b_scales + static_cast<size_t>(row) * p.groups;
-        sf_src2 = sf_src + static_cast<size_t>(128) * p.groups;
       }
       for (int kb = 0; kb < p.k_blocks; kb += kAtoms) {
         ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status));
@@ -286,7 +282,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           else if (kWide && kMode == kGeglu)
             expected = (half_item ? 1u : 2u) * (Shape::kWeightBytes / 2 + kSfStageBytes);
           else
-            expected = atoms * Shape::kWeightBytes + (kWide ? 2u : 1u) * sf_bytes;
+            expected = atoms * Shape::kWeightBytes + sf_bytes;
           mbar_arrive_expect_tx(&smem->full[stage], expected);
 #pragma unroll
           for (int atom = 0; atom < kAtoms; ++atom) {
@@ -300,9 +296,6 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               tma_load_3d(smem->b[stage], &map_b, &smem->full[stage], x, row, 2 * expert);
               if (!half_item)
                 tma_load_3d(smem->b[stage] + kOperandStageBytes, &map_b, &smem->full[stage], x, row + 64, 2 * expert);
-            } else if (kWide) {
-              tma_load_2d(smem->b[stage], &map_b, &smem->full[stage], x, row);
-              tma_load_2d(smem->b[stage] + kOperandStageBytes, &map_b, &smem->full[stage], x, row2);
             } else {
               tma_load_2d(smem->b[stage] + atom * kOperandStageBytes, &map_b, &smem->full[stage], x, row);
             }
@@ -320,9 +313,6 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
             } else {
               bulk_load_1d(smem->sfb[stage], sf_src + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes,
                            &smem->full[stage]);
-              if (kWide)
-                bulk_load_1d(smem->sfb[stage] + kSfStageBytes, sf_src2 + static_cast<size_t>(kb) * kSfStageBytes,
-                             sf_bytes, &smem->full[stage]);
             }
           }
         }
@@ -369,7 +359,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       if (!__all_sync(0xffffffffu,
                       wait_or_abort<false>(&smem->acc_empty[acc_stage], acc_phase ^ 1u, smem, p.status)))
         break;
-      const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc_stage * kTileN);
+      const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc_stage * kN);
       const bool half_item = kMode == kGeglu && item.n_tile == p.n_tiles - 1;
       bool ok = true;
       tc_fence_after_sync();  // the epilogue's tensor-memory loads of this accumulator are done
@@ -509,8 +499,8 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       tc_fence_after_sync();
       const int row_local = quarter * 32 + lane;
       const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                                static_cast<uint32_t>(acc_stage * kTileN);
-      if constexpr (kMode != kGeglu && !kWide) {
+                                static_cast<uint32_t>(acc_stage * kN);
+      if constexpr (kMode != kGeglu) {
         uint32_t r[32];
         tmem_load_32x32(tmem_row + sub * 32, r);
         tmem_load_wait();
@@ -519,19 +509,6 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         // same decision in all four warps of the quarter
         if (quarter * 32 < rows_valid)
           stage_and_store(r, alpha, staging, quarter, sub, lane, rows_valid, row0, n_tile * kN, p);
-      } else if constexpr (kMode != kGeglu) {
-        // 256 columns: both halves are taken into registers before the accumulator is released
-        uint32_t r0[32], r1[32];
-        tmem_load_32x32(tmem_row + sub * 32, r0);
-        tmem_load_32x32(tmem_row + kStoreColumns + sub * 32, r1);
-        tmem_load_wait();
-        tc_fence_before_sync();
-        mbar_arrive(&smem->acc_empty[acc_stage]);
-        if (quarter * 32 < rows_valid) {
-          stage_and_store(r0, alpha, staging, quarter, sub, lane, rows_valid, row0, n_tile * kN, p);
-          stage_and_store(r1, alpha, staging, quarter, sub, lane, rows_valid, row0,
-                          n_tile * kN + kStoreColumns, p);
-        }
       } else {
         // Fused GeGLU + NVFP4 requantise, wide tile.  Accumulator columns are [64 up | 64 gate] of unit
         // 2*n_tile, then of the next one; this warp owns the two 16-column blocks 2*sub and 2*sub+1 of
@@ -640,10 +617,10 @@ void launch_variant(const GemmOperands& op, const GemmParams& p, int sm_count, c
 
 int prepare_grouped_gemm() {
   cudaError_t e = raise_smem_limit<kPlain, 1, 128>();
-  if (e == cudaSuccess) e = raise_smem_limit<kPlain, 1, 256>();
   if (e == cudaSuccess) e = raise_smem_limit<kGeglu, 1, 256>();
   if (e == cudaSuccess) e = raise_smem_limit<kFp8, 1, 128>();
   if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_stream_experts());
+  if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_grouped_down());
   if (e == cudaSuccess) return prepare_grouped_gemm_pairs();
   return static_cast<int>(e);
 }
@@ -694,9 +671,8 @@ void launch_grouped_gemm(const GemmOperands& op, const RoutePlan& plan, int sm_c
     GemmOperands fused = op;
     fused.map_b = op.map_b_units;
     launch_variant<kGeglu, 256>(fused, p, sm_count, stream);
-  } else if (op.n_out % 256 == 0) {
-    p.n_tiles = op.n_out / 256;
-    launch_variant<kPlain, 256>(op, p, sm_count, stream);
+  } else if (op.down_scales) {
+    launch_grouped_down(op, plan, sm_count, stream);
   } else {
     p.n_tiles = op.n_out / kTileN;
     launch_variant<kPlain, 128>(op, p, sm_count, stream);

@@ -83,6 +83,7 @@ struct GemmOperands {
   CUtensorMap map_b;        // [128*N, K/2] bytes, same box
   CUtensorMap map_b64;      // CTA-pair fused w13 form: the same matrix through a 64-row box
   CUtensorMap map_b_units;  // fused w13 form: [experts * 2 halves, 704 rows, 1408 bytes], box 2 x 64 rows x 128 B
+  CUtensorMap map_b_down;   // w2: the weights in the column order of grouped_gemm_down.cu
   CUtensorMap map_a_sf;     // CTA-pair form: a_scales as [atoms of 512 B][128 x u32], box of four atoms
   CUtensorMap map_b_sf;     // CTA-pair form: b_scales likewise; box of eight atoms (fused w13) or four (w2)
   const uint8_t* a_scales;  // activation scale regions
@@ -97,6 +98,7 @@ struct GemmOperands {
   // the copy made by launch_retile_w13_scales in b_scales.)
   bool fused_geglu;
   const uint8_t* unit_scales;  // launch_retile_w13_unit_scales
+  const uint8_t* down_scales;  // w2: launch_retile_w2_scales
   bool serial_launch;         // launch the ordinary way: no start before the stream's previous kernel ends
   bool use_pairs;             // NVFP4 forms with 256 weight rows per item: run as CTA pairs (tcgen05 cta_group::2)
                               // when the plan carries a pair list
@@ -121,6 +123,16 @@ bool make_operand_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, 
 
 // w13 codes [experts, 2 halves, 704 rows, 1408 bytes] through a box of both halves x 64 rows x 128 bytes.
 bool make_w13_unit_tensor_map(CUtensorMap* map, const void* base, uint64_t experts);
+
+// w2 codes [experts * 2816 rows, 352 bytes] as [64-row groups][8][4][2] rows with strides of 64, 2, 16 and 1
+// rows, through a box of 192 rows x 128 bytes: the column order of grouped_gemm_down.cu.
+bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t experts);
+
+// The w2 GEMM of prefill-sized batches (grouped_gemm_down.cu): op.map_a, map_b_down, down_scales.
+size_t retiled_w2_scale_bytes(int experts);
+void launch_retile_w2_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, cudaStream_t stream);
+void launch_grouped_down(const GemmOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
+int prepare_grouped_down();
 
 // Scale-factor bytes seen as rows of one 512-byte atom each (128 x u32), through a box of
 // `box_atoms` consecutive atoms; no swizzle.

@@ -116,6 +116,19 @@ bool make_w13_unit_map(CUtensorMap* map, const void* base, uint64_t experts) {
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts) {
+  constexpr cuuint64_t row = kInter / 2;
+  const cuuint64_t dims[5] = {row, 2, 4, 8, experts * kHidden / 64};
+  const cuuint64_t strides[4] = {row, 16 * row, 2 * row, 64 * row};
+  const cuuint32_t box[5] = {static_cast<cuuint32_t>(kTileKBytes), 2, 4, 8, 3};
+  const cuuint32_t element_strides[5] = {1, 1, 1, 1, 1};
+  EncodeTiledFn fn = encode_tiled();
+  if (!fn) return false;
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<void*>(base), dims, strides, box, element_strides,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Scale bytes of an activation operand as [128-row blocks, atoms per block, 128 x u32] through a
 // box of two blocks x four atoms: the scales of one K block for up to 256 rows in one copy.
 bool make_block_scale_map(CUtensorMap* map, const void* base, uint64_t bytes, int atoms_per_block) {
@@ -202,6 +215,9 @@ namespace gv {
 bool make_w13_unit_tensor_map(CUtensorMap* map, const void* base, uint64_t experts) {
   return make_w13_unit_map(map, base, experts);
 }
+bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t experts) {
+  return make_w2_down_map(map, base, experts);
+}
 bool make_operand_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
                              int box_rows) {
   return make_operand_map(map, base, rows, row_bytes, box_rows);
@@ -235,6 +251,7 @@ struct gevva_moe {
   uint8_t* w13_sf_tiled = nullptr;  // runner-owned re-tiling of weights.w13_sf for the CTA-pair tile kernels
   gv::W13PairOperands w13_pairs{};  // the CTA-pair form of the fused w13 stage
   uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf by unit of 64 columns
+  uint8_t* w2_sf_down = nullptr;    // runner-owned re-tiling of weights.w2_sf in the column order of grouped_gemm_down.cu
   gv::StreamOperands stream_experts{};  // few rows an expert: both GEMMs in one launch, weights on the MMA's M side
   bool w13_pair_form = false;       // GEVVA_MOE_OPTION_W13_PAIRS, or GEVVA_MOE_W13_PAIRS=1 for a whole process
   int sm_count = 0;
@@ -423,6 +440,11 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
       gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_units, kExperts, nullptr);
       e = cudaGetLastError();
     }
+    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&m->w2_sf_down), gv::retiled_w2_scale_bytes(kExperts));
+    if (e == cudaSuccess) {
+      gv::launch_retile_w2_scales(static_cast<const uint8_t*>(weights->w2_sf), m->w2_sf_down, kExperts, nullptr);
+      e = cudaGetLastError();
+    }
     if (e == cudaSuccess && m->pairs) {
       // the opt-in CTA-pair form of the tile kernels has a tiling of its own
       e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_tiled), gv::retiled_w13_scale_bytes(kExperts));
@@ -434,7 +456,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
       gevva_moe_destroy(m);
-      return cuda_failure(e, "w13 scale re-tiling");
+      return cuda_failure(e, "weight scale re-tiling");
     }
     if (m->pairs) {
       ok = make_scale_map(&m->w13.map_a_sf, s->input_sf, s->input_sf_bytes, 4) &&
@@ -449,7 +471,8 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
       }
     }
     gv::StreamOperands& st = m->stream_experts;
-    ok = make_w13_unit_map(&st.map_w13, weights->w13, kExperts);
+    ok = make_w13_unit_map(&st.map_w13, weights->w13, kExperts) &&
+         make_w2_down_map(&m->w2.map_b_down, weights->w2, kExperts);
     for (int i = 0; i < gv::kStreamBoxes; ++i)
       ok = ok && make_operand_map(&st.map_up[i], s->input_codes, rows, kHidden / 2, 8 * (i + 1)) &&
            make_operand_map(&st.map_down[i], s->inter_codes, rows, kInter / 2, 8 * (i + 1));
@@ -514,6 +537,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   m->w2.b_scales = static_cast<const uint8_t*>(weights->w2_sf);
   m->w2.alpha = weights->alpha2;
   m->w2.out = s->w2_out;
+  m->w2.down_scales = m->w2_sf_down;
   m->w2.n_out = kHidden;
   m->w2.k_in = kInter;
   *out = m;
@@ -525,6 +549,7 @@ void gevva_moe_destroy(gevva_moe* runner) {
   if (runner->scratch && --runner->scratch->references == 0) free_scratch(runner->scratch);
   cudaFree(runner->w13_sf_tiled);
   cudaFree(runner->w13_sf_units);
+  cudaFree(runner->w2_sf_down);
   delete runner;
 }
 

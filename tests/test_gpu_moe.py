@@ -532,6 +532,42 @@ def test_cta_pair_gemms_equal_the_single_cta_gemms(gm, weights, cuda_device, tok
     assert results[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens", [641, 1000])
+def test_w2_of_large_batches_at_row_tile_edges(gm, weights, cuda_device, tokens):
+    """The w2 kernel of batches above 640 tokens, whose items, units of items and rows end raggedly,
+    against the CTA-pair kernel: the same routed rows with experts of 0, 1, 7..9, 127..129, 255..257 and
+    `tokens` rows, with every stage in one call and each in a call of its own."""
+    from gevva_b200 import runtime as rt
+    edges = [tokens, 1, 7, 8, 9, 127, 128, 129, 255, 256, 257]
+    rng = np.random.default_rng(tokens)
+    ids = np.empty((tokens, TOP_K), dtype=np.int32)
+    mine = [[] for _ in range(tokens)]  # with these seeds no token has more than six of the edge experts
+    for expert, count in enumerate(edges):
+        for t in rng.permutation(tokens)[:count]:
+            mine[t].append(expert)
+    for t in range(tokens):
+        rest = rng.choice(np.arange(20, EXPERTS - 1), TOP_K - len(mine[t]), replace=False)
+        ids[t] = rng.permutation(np.concatenate([np.array(mine[t], dtype=np.int64), rest]))
+    x = hashgen.activations(tokens, HIDDEN, 77, cuda_device)
+    dev_ids = torch.from_numpy(ids).to(cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    results = []
+    for pairs, split in ((True, False), (False, False), (False, True)):
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens, pairs=pairs)
+        out = torch.zeros_like(x)
+        if split:
+            for stage in (rt.STAGE_SORT, rt.STAGE_QUANTIZE, rt.STAGE_W13 | rt.STAGE_GEGLU, rt.STAGE_W2, rt.STAGE_REDUCE):
+                runner.launch_stages(stage, tokens, input=x, expert_ids=dev_ids, route_weights=rw, output=out)
+        else:
+            runner.launch_batch(x, dev_ids, rw, out, tokens)
+        runner.check()
+        results.append((out, runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].clone()))
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            assert torch.equal(a, b)
+    assert results[0][0].float().abs().max() > 0
+
+
 @pytest.mark.parametrize("tokens,kind", [(129, "random"), (130, "skewed"), (300, "skewed"), (777, "random"),
                                          (4096, "random")])
 def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_device, tokens, kind):
