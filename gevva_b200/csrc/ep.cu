@@ -786,7 +786,7 @@ int gevva_moe_ep_reduce(gevva_moe_ep* ep, const float* route_weights, void* out,
                         gevva_stream_t stream) {
   if (!ep || !route_weights || !out || tokens < 1 || tokens > ep->max_tokens) return GEVVA_MOE_BAD_ARGUMENT;
   gv::launch_reduce_routes(ep->dev.peer_combine[ep->dev.rank], route_weights,
-                           ep->send_plan.inverse_routes, tokens, out, stream);
+                           ep->send_plan.inverse_routes, tokens, out, false, stream);
   return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
 }
 

@@ -221,14 +221,17 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     __syncthreads();
     fill_geglu_tables(smem->tables);
   }
-  grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = smem->tmem_base;
   // Everything above touched only this CTA's shared and tensor memory; from here on the
   // kernel reads what earlier kernels of the stream wrote.
-  grid_dependency_wait();
+  // (The weights and the plan may come from before the previous kernel: see GemmOperands::early_weights.)
+  if (!(p.early_weights && warp == kWeightProducerWarp)) {
+    grid_dependency_wait();
+    grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
+  }
 
   const int m_tiles = p.num_m_tiles[0];
   const int tile_first = p.tile_first ? p.tile_first[0] : 0;
@@ -657,6 +660,7 @@ void launch_grouped_gemm(const GemmOperands& op, const RoutePlan& plan, int sm_c
   p.num_m_tiles = plan.num_m_tiles;
   p.tile_first = plan.tile_first;
   p.status = plan.status;
+  p.early_weights = op.early_weights;
   p.n_out = op.n_out;
   const int k_bytes = op.fp8 ? op.k_in : op.k_in / 2;
   p.groups = op.k_in / 16;

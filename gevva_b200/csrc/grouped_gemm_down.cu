@@ -86,6 +86,7 @@ struct DownParams {
   const int* num_m_tiles;
   const int* tile_first;               // optional
   int* status;
+  bool early_weights;
 };
 
 // A row tile of an expert and kDnUnitTiles of its column tiles [begin, end).
@@ -190,12 +191,15 @@ grouped_down_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tmem_alloc(&smem->tmem_base, kDnTmemColumns);
     tmem_relinquish();
   }
-  grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = smem->tmem_base;
-  grid_dependency_wait();
+  // The weights (and the plan) come from before the previous kernel, which let this one start after its own wait.
+  if (!(p.early_weights && warp == kDnWeightWarp)) {
+    grid_dependency_wait();
+    grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
+  }
 
   DownSchedule schedule(p);
   DownUnit unit;
@@ -467,6 +471,7 @@ void launch_grouped_down(const GemmOperands& op, const RoutePlan& plan, int sm_c
   p.num_m_tiles = plan.num_m_tiles;
   p.tile_first = plan.tile_first;
   p.status = plan.status;
+  p.early_weights = op.early_weights;
   if (op.serial_launch) {
     grouped_down_kernel<<<sm_count, kDnThreads, kDnSmemBytes, stream>>>(op.map_a, op.map_b_down, p);
     return;

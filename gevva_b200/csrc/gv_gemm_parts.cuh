@@ -38,6 +38,7 @@ struct GemmParams {
   int groups;       // k_in / 16
   int k_blocks;     // ceil(k_in / 256)
   int last_mmas;    // MMAs (K = 64 each) in the last K block, 1..4
+  bool early_weights;  // see GemmOperands
 };
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

@@ -63,9 +63,10 @@ void launch_route_sort_quantize_small(const void* input_bf16, const int* expert_
                                       const RoutePlan& plan, int tokens, uint8_t* packed, uint8_t* scales,
                                       cudaStream_t stream);
 
-// bf16 [tokens, 2816] -> codes [R, 1408] (sorted order) + swizzled scale bytes.
+// bf16 [tokens, 2816] -> codes [R, 1408] (sorted order) + swizzled scale bytes.  behind_sort: the
+// stream's previous kernel is the route sort of this batch.
 void launch_quantize_input(const void* input_bf16, const int* expert_ids, const float* in_scale_q,
-                           const RoutePlan& plan, int tokens, uint8_t* packed, uint8_t* scales,
+                           const RoutePlan& plan, int tokens, uint8_t* packed, uint8_t* scales, bool behind_sort,
                            cudaStream_t stream);
 
 // bf16 [R, 1408] ([up;gate]) -> codes [R, 352] + swizzled scale bytes.
@@ -73,7 +74,7 @@ void launch_geglu_quantize(const void* fused_bf16, const float* in_scale_q, cons
                            int routes, uint8_t* packed, uint8_t* scales, cudaStream_t stream);
 
 void launch_reduce_routes(const void* routed_bf16, const float* route_weights,
-                          const int* inverse_routes, int tokens, void* output_bf16,
+                          const int* inverse_routes, int tokens, void* output_bf16, bool behind_gemm,
                           cudaStream_t stream);
 
 // Grouped NVFP4 GEMM: out[r, n] = bf16(alpha[e] * sum_k A[r,k] B[e,n,k]).
@@ -99,6 +100,8 @@ struct GemmOperands {
   bool fused_geglu;
   const uint8_t* unit_scales;  // launch_retile_w13_unit_scales
   const uint8_t* down_scales;  // w2: launch_retile_w2_scales
+  bool early_weights;         // the stream's previous kernel is one of this library's that lets its dependents go
+                              // only after its own wait: the weights need not wait for it
   bool serial_launch;         // launch the ordinary way: no start before the stream's previous kernel ends
   bool use_pairs;             // NVFP4 forms with 256 weight rows per item: run as CTA pairs (tcgen05 cta_group::2)
                               // when the plan carries a pair list

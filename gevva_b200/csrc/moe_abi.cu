@@ -319,7 +319,7 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
     StageRange range(runner->nvtx && (stages & GEVVA_MOE_STAGE_QUANTIZE), "gevva_moe.quantize");
     if (stages & GEVVA_MOE_STAGE_QUANTIZE)
       gv::launch_quantize_input(in, ids, runner->weights.in_scale_q1, s->plan, tokens, s->input_codes,
-                                s->input_sf, stream);
+                                s->input_sf, (stages & GEVVA_MOE_STAGE_SORT) != 0, stream);
   }
   const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
   const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
@@ -337,6 +337,7 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
     } else {
       gv::GemmOperands w13 = runner->w13_fused;
       w13.use_pairs = use_pairs;
+      w13.early_weights = (stages & front) == front && tokens > gv::kFusedSortQuantizeMaxTokens;
       gv::launch_grouped_gemm(w13, s->plan, sm_count, stream);
     }
   } else {
@@ -346,15 +347,19 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
       gv::launch_geglu_quantize(s->w13_out, runner->weights.in_scale_q2, s->plan, routes,
                                 s->inter_codes, s->inter_sf, stream);
   }
+  // the fused one-CTA w13 launch of this call is w2's predecessor, and w2 the reduce's
+  const bool behind_w13 = (stages & both) == both && !(stages & GEVVA_MOE_STAGE_UNFUSED) && !use_pairs && !runner->w13_pair_form;
+  const bool behind_w2 = (stages & GEVVA_MOE_STAGE_W2) && !use_pairs && behind_w13;
   if (stages & GEVVA_MOE_STAGE_W2) {
     StageRange range(runner->nvtx, "gevva_moe.w2");
     gv::GemmOperands w2 = runner->w2;
     w2.use_pairs = use_pairs;
+    w2.early_weights = behind_w13;
     gv::launch_grouped_gemm(w2, s->plan, sm_count, stream);
   }
   StageRange reduce_range(runner->nvtx && (stages & GEVVA_MOE_STAGE_REDUCE), "gevva_moe.reduce");
   if (stages & GEVVA_MOE_STAGE_REDUCE)
-    gv::launch_reduce_routes(s->w2_out, route_weights, s->plan.inverse_routes, tokens, out, stream);
+    gv::launch_reduce_routes(s->w2_out, route_weights, s->plan.inverse_routes, tokens, out, behind_w2, stream);
   GV_CUDA(cudaGetLastError(), "moe launch");
   return GEVVA_MOE_OK;
 }

@@ -228,13 +228,13 @@ __device__ __forceinline__ bool grid_barrier(int* sync, int ctas, int* status) {
 // scatters its routes.
 __global__ void __launch_bounds__(kSortChunk)
 route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chunks, RoutePlan plan) {
-  grid_launch_dependents();
   __shared__ int warp_counts[32 * kExperts];
   __shared__ int scan_scratch[16];
   const int tid = threadIdx.x;
   for (int i = tid; i < 32 * kExperts; i += kSortChunk) warp_counts[i] = 0;
   __syncthreads();
   grid_dependency_wait();  // the ids are written, and the plan's last readers are done
+  grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
   const int route = blockIdx.x * kSortChunk + tid;
   int expert = kExperts;
   if (route < routes) {
@@ -347,49 +347,53 @@ void launch_route_sort(const int* expert_ids, int routes, const RoutePlan& plan,
 // quantises them with that expert's static scale, storing 16 code bytes and the two scale
 // bytes (adjacent in the swizzled layout) of the route's sorted row.  Nothing is computed
 // twice: no lane shares a block with another, and routes with equal static scales share one
-// quantisation.  At 4096 tokens the kernel moves 75 MB, 52 MB of them written, in 21 us; a
-// form with 64 columns per thread (whole 4-byte scale words, half as many threads) took 30 us.
+// quantisation.  One token per CTA: small CTAs keep more of them resident, which is what hides the latency
+// of this short kernel.
+//
+// kEarly: launched right behind the route sort of the same batch, which lets it start once everything
+// before the sort is complete.  The token, the ids and the static scales are such things; only the rows
+// come from the sort.  So the loads and the arithmetic of the CTAs that find room happen during the
+// sort, and what follows it is the stores.
 // ---------------------------------------------------------------------------
-template <int kTokensPerBlock, int kBlocks>
-__global__ void __launch_bounds__(kHidden / (16 * kBlocks) * kTokensPerBlock)
+template <bool kEarly>
+__global__ void __launch_bounds__(kQuantizeThreadsPerToken)
 quantize_input_kernel(const __nv_bfloat16* __restrict__ input, const int* __restrict__ expert_ids,
-                      const float* __restrict__ in_scale_q, RoutePlan plan, int tokens,
+                      const float* __restrict__ in_scale_q, RoutePlan plan,
                       uint8_t* __restrict__ packed, uint8_t* __restrict__ scales) {
   constexpr int groups = kHidden / 16;
-  __shared__ float route_multiplier[kTokensPerBlock][kTopK];
-  __shared__ int route_row[kTokensPerBlock][kTopK];  // sorted row, or -1 for a rejected expert id
-  __shared__ unsigned long long route_scale_base[kTokensPerBlock][kTopK];
-  grid_launch_dependents();
-  grid_dependency_wait();  // the route sort's plan, and the previous user of the output buffers
-  if (threadIdx.x < kTokensPerBlock * kTopK) {
-    const int slot = threadIdx.x / kTopK;
-    const int k = threadIdx.x % kTopK;
-    const int token = blockIdx.x * kTokensPerBlock + slot;
-    int dst = -1;
-    if (token < tokens) {
-      const int route = token * kTopK + k;
-      const int expert = expert_ids[route];
-      if (expert >= 0 && expert < kExperts) {  // others are flagged by the route sort
-        dst = plan.inverse_routes[route];
-        const int row = dst - plan.expert_offsets[expert];
-        route_multiplier[slot][k] = in_scale_q[expert];
-        route_scale_base[slot][k] =
-            static_cast<unsigned long long>(plan.scale_row_offsets[expert]) * groups + sf_offset(row, 0, groups);
-      }
-    }
-    route_row[slot][k] = dst;
+  __shared__ float route_multiplier[kTopK];
+  __shared__ int route_row[kTopK];  // sorted row, or -1 for a rejected expert id
+  __shared__ unsigned long long route_scale_base[kTopK];
+  const int token = blockIdx.x;
+  const int part = threadIdx.x;  // columns [32*part, +32)
+  float values[32];
+  float maximum[2];
+  QuantisedBlocks blocks;
+  int expert = -1;
+  if (!kEarly) grid_dependency_wait();  // the route sort's plan, and the previous user of the output buffers
+  load_token_columns(input, token, part, values, maximum);
+  if (threadIdx.x < kTopK) {
+    expert = expert_ids[token * kTopK + threadIdx.x];
+    if (expert >= 0 && expert < kExperts) route_multiplier[threadIdx.x] = in_scale_q[expert];  // others are flagged by the route sort
+    else route_multiplier[threadIdx.x] = 0.0f;
   }
-  constexpr int threads_per_token = kHidden / (16 * kBlocks);
-  const int slot = threadIdx.x / threads_per_token;
-  const int part = threadIdx.x - slot * threads_per_token;  // columns [16*kBlocks*part, +16*kBlocks)
-  const int token = blockIdx.x * kTokensPerBlock + slot;
-  float values[16 * kBlocks];
-  float maximum[kBlocks];
-  if (token < tokens) load_token_columns<kBlocks>(input, token, part, values, maximum);
+  if (kEarly) {
+    __syncthreads();
+    blocks.quantise(values, maximum, route_multiplier[0]);
+    grid_dependency_wait();
+  }
+  grid_launch_dependents();
+  if (threadIdx.x < kTopK) {
+    int dst = -1;
+    if (expert >= 0 && expert < kExperts) {
+      dst = plan.inverse_routes[token * kTopK + threadIdx.x];
+      route_scale_base[threadIdx.x] = static_cast<unsigned long long>(plan.scale_row_offsets[expert]) * groups +
+                                      sf_offset(dst - plan.expert_offsets[expert], 0, groups);
+    }
+    route_row[threadIdx.x] = dst;
+  }
   __syncthreads();
-  if (token >= tokens) return;
-  quantize_routes_of_token<kBlocks>(values, maximum, part, route_row[slot], route_multiplier[slot],
-                                    route_scale_base[slot], packed, scales);
+  quantize_routes_of_token(values, maximum, part, route_row, route_multiplier, route_scale_base, packed, scales, blocks);
 }
 
 // Route sort and input quantiser in one launch, for batches of at most 1024 routes (decode
@@ -497,9 +501,10 @@ route_sort_quantize_small_kernel(const __nv_bfloat16* __restrict__ input, const 
   }
   float values[32];
   float maximum[2];
-  load_token_columns<2>(input, token, tid, values, maximum);
+  load_token_columns(input, token, tid, values, maximum);
   __syncthreads();
-  quantize_routes_of_token<2>(values, maximum, tid, route_row, route_multiplier, route_scale_base, packed, scales);
+  QuantisedBlocks blocks;
+  quantize_routes_of_token(values, maximum, tid, route_row, route_multiplier, route_scale_base, packed, scales, blocks);
 }
 
 void launch_route_sort_quantize_small(const void* input_bf16, const int* expert_ids, const float* in_scale_q,
@@ -511,13 +516,11 @@ void launch_route_sort_quantize_small(const void* input_bf16, const int* expert_
 }
 
 void launch_quantize_input(const void* input_bf16, const int* expert_ids, const float* in_scale_q,
-                           const RoutePlan& plan, int tokens, uint8_t* packed, uint8_t* scales,
+                           const RoutePlan& plan, int tokens, uint8_t* packed, uint8_t* scales, bool behind_sort,
                            cudaStream_t stream) {
   const __nv_bfloat16* input = static_cast<const __nv_bfloat16*>(input_bf16);
-  // One token per CTA at every size: small CTAs keep more of them resident, which is what hides the
-  // latency of this short kernel (4096 tokens: 3 us less per layer than four tokens per CTA).
-  launch_chained(quantize_input_kernel<1, 2>, dim3(tokens), dim3(kQuantizeThreadsPerToken), 0, stream, input,
-                 expert_ids, in_scale_q, plan, tokens, packed, scales);
+  launch_chained(behind_sort ? quantize_input_kernel<true> : quantize_input_kernel<false>, dim3(tokens),
+                 dim3(kQuantizeThreadsPerToken), 0, stream, input, expert_ids, in_scale_q, plan, packed, scales);
 }
 
 // ---------------------------------------------------------------------------
@@ -577,6 +580,9 @@ void launch_geglu_quantize(const void* fused_bf16, const float* in_scale_q, cons
 // src/nvfp4_cutlass.cu:229-247: fp32 fmaf over the eight routes in route order,
 // one bf16 rounding.
 // ---------------------------------------------------------------------------
+// kEarly: launched behind the down GEMM of the same batch, which lets it start once everything before that
+// GEMM is complete: the token's rows and weights are looked up while the GEMM drains.
+template <bool kEarly>
 __global__ void __launch_bounds__(kHidden / 8)
 reduce_routes_kernel(const __nv_bfloat16* __restrict__ routed, const float* __restrict__ route_weights,
                      const int* __restrict__ inverse_routes, __nv_bfloat16* __restrict__ output) {
@@ -584,13 +590,20 @@ reduce_routes_kernel(const __nv_bfloat16* __restrict__ routed, const float* __re
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   unsigned long long read_once;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(read_once));
-  grid_launch_dependents();
-  grid_dependency_wait();  // the down GEMM's rows
+  if (!kEarly) grid_dependency_wait();
+  int sources[kTopK];
+  float route_weight[kTopK];
 #pragma unroll
   for (int k = 0; k < kTopK; ++k) {
-    const int index = token * kTopK + k;
-    const int source = inverse_routes[index];
-    const float weight = route_weights[index];
+    sources[k] = inverse_routes[token * kTopK + k];
+    route_weight[k] = route_weights[token * kTopK + k];
+  }
+  if (kEarly) grid_dependency_wait();  // the down GEMM's rows
+  grid_launch_dependents();
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k) {
+    const int source = sources[k];
+    const float weight = route_weight[k];
     float v[8];
     // read once and dead afterwards: the rows must not push the rows that other CTAs have not yet read out of L2
     uint4 raw;
@@ -613,9 +626,9 @@ reduce_routes_kernel(const __nv_bfloat16* __restrict__ routed, const float* __re
 }
 
 void launch_reduce_routes(const void* routed_bf16, const float* route_weights,
-                          const int* inverse_routes, int tokens, void* output_bf16,
+                          const int* inverse_routes, int tokens, void* output_bf16, bool behind_gemm,
                           cudaStream_t stream) {
-  launch_chained(reduce_routes_kernel, dim3(tokens), dim3(kHidden / 8), 0, stream,
+  launch_chained(behind_gemm ? reduce_routes_kernel<true> : reduce_routes_kernel<false>, dim3(tokens), dim3(kHidden / 8), 0, stream,
                  static_cast<const __nv_bfloat16*>(routed_bf16), route_weights, inverse_routes,
                  static_cast<__nv_bfloat16*>(output_bf16));
 }
