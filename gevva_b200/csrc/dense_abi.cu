@@ -33,14 +33,29 @@ struct gevva_dense {
   cudaEvent_t fork = nullptr, join = nullptr;  // gevva_ff_layer_launch: to the second stream and back
 };
 
+// Whether a GEMM of the dense MLP takes 256 weight rows an item instead of 128.  The launch lasts as many items
+// as its busiest CTA has, and a wide item takes about one and a half times a narrow one (48 KB of operands a K
+// block against 32 KB): wide where that is no longer.  Alone on 148 SMs the MLP takes (us, narrow -> wide)
+// 31.9 -> 35.4 at 301 tokens, where one wave of narrow items is enough, 39.0 -> 35.5 at 600, 74.8 -> 62.6 at 2048
+// and 131.9 -> 108.4 at 4096; on the 16 SMs it gets beside the experts wide is as good or better from 129 tokens on.
+static bool wide_items(int tokens, int n_out, int sms) {
+  const int row_tiles = (tokens + gv::kTileM - 1) / gv::kTileM;
+  const int narrow = (row_tiles * ((n_out + 127) / 128) + sms - 1) / sms;
+  const int wide = (row_tiles * ((n_out + 255) / 256) + sms - 1) / sms;
+  return 3 * wide <= 2 * narrow;
+}
+
 int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
                         int sm_count) {
   gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, d->plan, stream);
-  gv::launch_grouped_gemm(d->gate_up, d->plan, sm_count, stream);
+  gv::GemmOperands gate_up = d->gate_up;
+  gate_up.wide = wide_items(tokens, gate_up.n_out, sm_count);
+  gv::launch_grouped_gemm(gate_up, d->plan, sm_count, stream);
   gv::launch_gelu_quantize_fp8(d->gate_up_out, d->act_scales, d->weights.gate_scale, d->weights.up_scale,
                                d->prod_fp8, d->prod_scales, tokens, stream);
   gv::GemmOperands down = d->down;
   down.out = out_unscaled;
+  down.wide = wide_items(tokens, down.n_out, sm_count);
   gv::launch_grouped_gemm(down, d->plan, sm_count, stream);
   return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
 }

@@ -10,8 +10,8 @@
 // the accumulators before anything is written.
 //
 // Mapping.  Tokens (sorted routes) sit on MMA-M, weight rows on MMA-N.  A work
-// item is (128-row tile of one expert) x (kN weight rows), kN = 256 for the fused w13 form,
-// 128 elsewhere.  An MMA of M = 128 takes at least about 105 cycles whatever its
+// item is (128-row tile of one expert) x (kN weight rows), kN = 256 for the fused w13 form and
+// for dense FP8 batches, 128 elsewhere.  An MMA of M = 128 takes at least about 105 cycles whatever its
 // N (measured; 128 at N = 256), so the wide tile, which does twice the work per
 // instruction, is what keeps the tensor pipe fed.  Row tiles are listed
 // in device memory by the route sort; CTAs are persistent and take items
@@ -64,6 +64,7 @@ constexpr uint32_t kTmemColumns = 512;
 // With block scales the accumulators take tensor-memory columns [0, 256) (2 x 128 or
 // 1 x 256); scale factors follow, per pipeline stage and K block: a copy for the next K
 // block must not wait for the MMAs of the previous one to finish reading theirs.
+// Dense FP8 has no scale factors: at N = 256 its two accumulators take all 512 columns.
 constexpr uint32_t kSfColumn = 256;
 constexpr int kOperandStageBytes = kTileM * kTileKBytes;  // 16 KiB: 128 rows of one K block
 // A pipeline stage holds kAtoms K blocks of 256 elements (one 128-byte swizzle row each) of
@@ -90,8 +91,8 @@ struct alignas(1024) GemmSmem {
   static constexpr int kAccStages = Shape::kAccStages;
   uint8_t a[kStages][kAtoms * kOperandStageBytes];
   uint8_t b[kStages][kAtoms * Shape::kWeightBytes];
-  uint8_t sfa[kStages][kAtoms * kSfStageBytes];
-  uint8_t sfb[kStages][kAtoms * Shape::kWeightSfBytes];
+  uint8_t sfa[kMode == kFp8 ? 1 : kStages][kMode == kFp8 ? 16 : kAtoms * kSfStageBytes];
+  uint8_t sfb[kMode == kFp8 ? 1 : kStages][kMode == kFp8 ? 16 : kAtoms * Shape::kWeightSfBytes];
   uint8_t staging[4][kMode != kGeglu ? kStagingBytesPerWarp : 16];  // plain epilogue only
   uint64_t full[kStages];
   uint64_t empty[kStages];
@@ -107,7 +108,7 @@ struct alignas(1024) GemmSmem {
 template <int kMode, int kAtoms, int kN> constexpr size_t gemm_smem_bytes() {
   return sizeof(GemmSmem<kMode, kAtoms, kN>) + 1024;
 }
-static_assert(gemm_smem_bytes<kPlain, 1, 128>() <= 232448 &&
+static_assert(gemm_smem_bytes<kPlain, 1, 128>() <= 232448 && gemm_smem_bytes<kFp8, 1, 256>() <= 232448 &&
                   gemm_smem_bytes<kGeglu, 1, 256>() <= 232448 && gemm_smem_bytes<kFp8, 1, 128>() <= 232448,
               "shared memory budget of one sm_100 CTA");
 static_assert(kSfColumn + 64 * 4 <= kTmemColumns && kSfColumn + 32 * 6 <= kTmemColumns, "tensor memory budget");
@@ -115,19 +116,20 @@ static_assert(kSfColumn + 64 * 4 <= kTmemColumns && kSfColumn + 32 * 6 <= kTmemC
 // Dense FP8 form of the same: kMmas MMAs of K = 32 E4M3 elements (32 bytes, the same
 // descriptor step), no scale factors.  Instruction descriptor: fp32 accumulate (bit 4),
 // E4M3 x E4M3 (format 0), both K-major, N and M as above.
-constexpr uint32_t kInstrDescFp8 = (1u << 4) | (static_cast<uint32_t>(kTileN >> 3) << 17) |
+template <int kN>
+constexpr uint32_t kInstrDescFp8 = (1u << 4) | (static_cast<uint32_t>(kN >> 3) << 17) |
                                    (static_cast<uint32_t>(kTileM >> 4) << 24);
 
 template <int kMmas>
 __device__ __forceinline__ void issue_k_block_fp8(uint32_t tmem_acc, uint32_t a_lo, uint32_t b_lo,
-                                                  uint32_t hi_ab, uint32_t accumulate) {
+                                                  uint32_t hi_ab, uint32_t descriptor, uint32_t accumulate) {
 #define GV_MMA8(j, pred)                                                   \
   "add.u32 lo, %1, " #j "*2;\n\t"                                          \
   "mov.b64 d0, {lo, %3};\n\t"                                              \
   "add.u32 lo, %2, " #j "*2;\n\t"                                          \
   "mov.b64 d1, {lo, %3};\n\t"                                              \
   "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], d0, d1, %4, " pred ";\n\t"
-#define GV_OPERANDS8 ::"r"(tmem_acc), "r"(a_lo), "r"(b_lo), "r"(hi_ab), "r"(kInstrDescFp8), "r"(accumulate) : "memory"
+#define GV_OPERANDS8 ::"r"(tmem_acc), "r"(a_lo), "r"(b_lo), "r"(hi_ab), "r"(descriptor), "r"(accumulate) : "memory"
 #define GV_PROLOGUE8 "{\n\t.reg .pred p, pt;\n\t.reg .b32 lo;\n\t.reg .b64 d0, d1;\n\t" \
                      "setp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
   asm volatile(GV_PROLOGUE8 GV_MMA8(0, "p") "}" GV_OPERANDS8);
@@ -187,7 +189,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   constexpr int kAtoms = Smem::kAtoms;
   constexpr int kAccStages = Smem::kAccStages;
   constexpr bool kWide = kN == 256;
-  static_assert(kMode == kGeglu || !kWide, "the other forms use 128-row weight tiles");
+  static_assert(kMode != kPlain || !kWide, "the plain form uses 128-row weight tiles");
   static_assert(kMode != kGeglu || kWide, "the fused form exists for 256-row weight tiles only");
   extern __shared__ uint8_t smem_raw[];
   Smem* smem = reinterpret_cast<Smem*>(
@@ -255,7 +257,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const uint8_t* sf_src;
       const uint8_t* sf_src2 = nullptr;  // fused form: scales of weight rows 128..255
       bool short_tile = false;  // decode-sized groups: fetch 32 activation rows instead of 128
-      bool half_item = false;   // fused form: the last item of a row tile has one unit
+      bool half_item = false;   // wide tiles: the last item of a row tile has 128 weight rows
       if (!weight_side) {
         row = p.expert_offsets[expert] + (m_tile * kTileM - p.scale_row_offsets[expert]);
         short_tile = p.expert_offsets[expert + 1] - row <= 32;
@@ -268,6 +270,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         sf_src2 = sf_src + static_cast<size_t>(p.k_blocks) * kSfStageBytes;
       } else {
         row = expert * p.n_out + n_tile * kN;
+        half_item = kWide && (n_tile + 1) * kN > p.n_out;
         sf_src = p.b_scales + static_cast<size_t>(row) * p.groups;
       }
       for (int kb = 0; kb < p.k_blocks; kb += kAtoms) {
@@ -285,7 +288,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           else if (kWide && kMode == kGeglu)
             expected = (half_item ? 1u : 2u) * (Shape::kWeightBytes / 2 + kSfStageBytes);
           else
-            expected = atoms * Shape::kWeightBytes + sf_bytes;
+            expected = half_item ? Shape::kWeightBytes / 2 : atoms * Shape::kWeightBytes + sf_bytes;
           mbar_arrive_expect_tx(&smem->full[stage], expected);
 #pragma unroll
           for (int atom = 0; atom < kAtoms; ++atom) {
@@ -299,11 +302,14 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               tma_load_3d(smem->b[stage], &map_b, &smem->full[stage], x, row, 2 * expert);
               if (!half_item)
                 tma_load_3d(smem->b[stage] + kOperandStageBytes, &map_b, &smem->full[stage], x, row + 64, 2 * expert);
+            } else if (kWide) {
+              tma_load_2d(smem->b[stage], &map_b, &smem->full[stage], x, row);
+              if (!half_item) tma_load_2d(smem->b[stage] + kOperandStageBytes, &map_b, &smem->full[stage], x, row + 128);
             } else {
               tma_load_2d(smem->b[stage] + atom * kOperandStageBytes, &map_b, &smem->full[stage], x, row);
             }
           }
-          if (kMode != kFp8) {
+          if constexpr (kMode != kFp8) {
             if (!weight_side) {
               bulk_load_1d(smem->sfa[stage], sf_src + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes,
                            &smem->full[stage]);
@@ -363,7 +369,8 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                       wait_or_abort<false>(&smem->acc_empty[acc_stage], acc_phase ^ 1u, smem, p.status)))
         break;
       const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc_stage * kN);
-      const bool half_item = kMode == kGeglu && item.n_tile == p.n_tiles - 1;
+      const bool half_item = kMode == kGeglu ? item.n_tile == p.n_tiles - 1 : kWide && (item.n_tile + 1) * kN > p.n_out;
+      const uint32_t descriptor8 = half_item ? kInstrDescFp8<128> : kInstrDescFp8<kN>;
       bool ok = true;
       tc_fence_after_sync();  // the epilogue's tensor-memory loads of this accumulator are done
       for (int kb = 0; kb < p.k_blocks; kb += kAtoms) {
@@ -390,10 +397,10 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
             const uint32_t bb = b_lo + atom * (Shape::kWeightBytes >> 4);
             const uint32_t ts = tmem_sf + atom * Shape::kSfColumns;
             if (kMode == kFp8) {
-              if (k != p.k_blocks - 1 || full_last) issue_k_block_fp8<4>(tmem_acc, aa, bb, hi_ab, accumulate);
-              else if (p.last_mmas == 3) issue_k_block_fp8<3>(tmem_acc, aa, bb, hi_ab, accumulate);
-              else if (p.last_mmas == 2) issue_k_block_fp8<2>(tmem_acc, aa, bb, hi_ab, accumulate);
-              else issue_k_block_fp8<1>(tmem_acc, aa, bb, hi_ab, accumulate);
+              if (k != p.k_blocks - 1 || full_last) issue_k_block_fp8<4>(tmem_acc, aa, bb, hi_ab, descriptor8, accumulate);
+              else if (p.last_mmas == 3) issue_k_block_fp8<3>(tmem_acc, aa, bb, hi_ab, descriptor8, accumulate);
+              else if (p.last_mmas == 2) issue_k_block_fp8<2>(tmem_acc, aa, bb, hi_ab, descriptor8, accumulate);
+              else issue_k_block_fp8<1>(tmem_acc, aa, bb, hi_ab, descriptor8, accumulate);
             } else if (kMode == kGeglu && half_item) {
               issue_mmas<4, kN, kMode == kGeglu>(tmem_acc, ts, aa, bb, hi_ab, accumulate);
             } else if (k != p.k_blocks - 1 || full_last) {
@@ -503,7 +510,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const int row_local = quarter * 32 + lane;
       const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                 static_cast<uint32_t>(acc_stage * kN);
-      if constexpr (kMode != kGeglu) {
+      if constexpr (kMode != kGeglu && !kWide) {
         uint32_t r[32];
         tmem_load_32x32(tmem_row + sub * 32, r);
         tmem_load_wait();
@@ -512,6 +519,19 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         // same decision in all four warps of the quarter
         if (quarter * 32 < rows_valid)
           stage_and_store(r, alpha, staging, quarter, sub, lane, rows_valid, row0, n_tile * kN, p);
+      } else if constexpr (kMode != kGeglu) {
+        // 256 columns: both halves are taken into registers before the accumulator is released
+        uint32_t r0[32], r1[32];
+        tmem_load_32x32(tmem_row + sub * 32, r0);
+        tmem_load_32x32(tmem_row + kStoreColumns + sub * 32, r1);
+        tmem_load_wait();
+        tc_fence_before_sync();
+        mbar_arrive(&smem->acc_empty[acc_stage]);
+        if (quarter * 32 < rows_valid) {
+          stage_and_store(r0, alpha, staging, quarter, sub, lane, rows_valid, row0, n_tile * kN, p);
+          if (n_tile * kN + kStoreColumns < p.n_out)
+            stage_and_store(r1, alpha, staging, quarter, sub, lane, rows_valid, row0, n_tile * kN + kStoreColumns, p);
+        }
       } else {
         // Fused GeGLU + NVFP4 requantise, wide tile.  Accumulator columns are [64 up | 64 gate] of unit
         // 2*n_tile, then of the next one; this warp owns the two 16-column blocks 2*sub and 2*sub+1 of
@@ -622,6 +642,7 @@ int prepare_grouped_gemm() {
   cudaError_t e = raise_smem_limit<kPlain, 1, 128>();
   if (e == cudaSuccess) e = raise_smem_limit<kGeglu, 1, 256>();
   if (e == cudaSuccess) e = raise_smem_limit<kFp8, 1, 128>();
+  if (e == cudaSuccess) e = raise_smem_limit<kFp8, 1, 256>();
   if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_stream_experts());
   if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_grouped_down());
   if (e == cudaSuccess) return prepare_grouped_gemm_pairs();
@@ -666,7 +687,10 @@ void launch_grouped_gemm(const GemmOperands& op, const RoutePlan& plan, int sm_c
   p.groups = op.k_in / 16;
   p.k_blocks = (k_bytes + kTileKBytes - 1) / kTileKBytes;
   p.last_mmas = (k_bytes - (p.k_blocks - 1) * kTileKBytes) / 32;
-  if (op.fp8) {
+  if (op.fp8 && op.wide) {
+    p.n_tiles = (op.n_out + 255) / 256;
+    launch_variant<kFp8, 256>(op, p, sm_count, stream);
+  } else if (op.fp8) {
     p.n_tiles = op.n_out / kTileN;
     launch_variant<kFp8, 128>(op, p, sm_count, stream);
   } else if (op.fused_geglu) {

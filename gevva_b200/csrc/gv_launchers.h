@@ -106,6 +106,7 @@ struct GemmOperands {
   bool use_pairs;             // NVFP4 forms with 256 weight rows per item: run as CTA pairs (tcgen05 cta_group::2)
                               // when the plan carries a pair list
   bool fp8;                   // dense E4M3 x E4M3 (no block scales); k_in counts bytes = elements
+  bool wide;                  // fp8: 256 weight rows per item instead of 128
   uint8_t* next_codes;        // [row capacity, 352]
   uint8_t* next_scales;       // scale regions of the w2 operand
   const float* next_scale_q;  // g2.input_scale_quant [128]

@@ -86,6 +86,25 @@ def test_dense_mlp_stages(dense_oracle, dense_weights, cuda_device, tokens):
     assert rel_l2(bf16_to_f32(bits(out)), bf16_to_f32(want_out)) < 5e-3
 
 
+@pytest.mark.parametrize("tokens", [512, 513, 897, 1025])
+def test_dense_mlp_rows_do_not_depend_on_the_batch(dense_weights, cuda_device, tokens):
+    """Batches whose GEMMs take 256 weight rows an item (4224 leaves half an item over) give every row
+    the bits it has in a batch of 100, whose items have 128."""
+    from gevva_b200 import feedforward as ff
+    gate_up, down, gs, us, ds = dense_weights
+    mlp = ff.DenseMlp(gate_up, down, gs, us, ds, tokens)
+    x = hashgen.activations(tokens, HIDDEN, 82, cuda_device)
+    out, scales = (t.clone() for t in mlp.launch(x))
+    hidden = mlp.buffer(2, torch.bfloat16)[: tokens * 2 * DENSE].view(tokens, -1).clone()
+    for first in range(0, tokens, 100):
+        rows = min(100, tokens - first)
+        part, part_scales = mlp.launch(x[first : first + rows].contiguous())
+        assert torch.equal(mlp.buffer(2, torch.bfloat16)[: rows * 2 * DENSE].view(rows, -1), hidden[first : first + rows])
+        assert torch.equal(part[:rows], out[first : first + rows])
+        assert torch.equal(part_scales[:rows], scales[first : first + rows])
+    assert out.float().abs().max() > 0
+
+
 def test_ff_finalize_bit_exact(dense_oracle, cuda_device):
     from gevva_b200 import feedforward as ff
     rows = 41
