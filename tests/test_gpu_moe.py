@@ -685,6 +685,33 @@ def test_decode_kernel_that_sorts_and_quantises_itself(gm, weights, cuda_device,
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("tokens", [147, 149, 296, 297])
+def test_streaming_front_with_two_tokens_an_sm(gm, weights, cuda_device, tokens, monkeypatch):
+    """Sort and quantiser inside the streaming launch where some CTAs prepare two tokens and others one
+    (up to twice the number of SMs) against launches of their own, with an expert id out of range."""
+    from gevva_b200 import runtime as rt
+    ids = random_ids(tokens, 9)
+    ids[tokens - 1, 7] = 200
+    ids[tokens // 2, 0] = -1
+    x = hashgen.activations(tokens, HIDDEN, 13, cuda_device)
+    keep = torch.ones(tokens * TOP_K, dtype=torch.bool, device=cuda_device)
+    keep[(tokens - 1) * TOP_K + 7] = False
+    keep[tokens // 2 * TOP_K] = False
+    outs = []
+    for front in ("0", "1"):
+        monkeypatch.setenv("GEVVA_MOE_DECODE_FRONT", front)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        for _ in range(2):
+            runner.launch_stages(rt.STAGE_ALL & ~rt.STAGE_REDUCE, tokens, input=x,
+                                 expert_ids=torch.from_numpy(ids).to(cuda_device))
+            assert runner.last_status() == -1
+        inverse = runner.buffer(rt.BUF_INVERSE_ROUTES, torch.int32)[: tokens * TOP_K]
+        rows = runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].view(-1, HIDDEN)
+        outs.append(rows[inverse[keep].long()].clone())
+    assert torch.equal(outs[0], outs[1])
+    assert outs[0].float().abs().max() > 0
+
+
 @pytest.mark.parametrize("tokens", [2, 65, 128, 129, 300, 640])
 def test_streaming_experts_equal_the_two_launches(gm, weights, cuda_device, tokens, monkeypatch):
     """The launch that does both GEMMs with the weights on the MMA's M side (up to 640 tokens) against

@@ -96,6 +96,33 @@ def test_fp8_router_projection(oracle, cuda_device, rows):
     print(f"FP8 router projection {rows} rows: {off} logits one ulp off; {close_rows} close rows, {moved} moved")
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 63, 64, 65])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_router_tiles_of_few_rows(cuda_device, rows, fp8):
+    """The 64-row tile, whose warps take eight rows each, at its edges: every row's logits, experts and
+    weights are those of the same row in a batch of 300, which takes 128-row tiles."""
+    import gevva_b200 as gm
+    gen = torch.Generator().manual_seed(3000 + rows)
+    x = torch.randn((300, HIDDEN), generator=gen).to(cuda_device)
+    router = (torch.randn((EXPERTS, HIDDEN), generator=gen) * 0.02).to(cuda_device)
+    scale = (0.5 + torch.rand(EXPERTS, generator=gen)).to(torch.bfloat16).to(cuda_device)
+    act = ws = None
+    if fp8:
+        act = (x.abs().amax(dim=1) / 448.0).float()
+        ws = (router.abs().max() / 448.0).float().reshape(1)
+        x = (x / act[:, None]).to(torch.float8_e4m3fn).view(torch.uint8)
+        router = (router / ws).to(torch.float8_e4m3fn).view(torch.uint8)
+    else:
+        x, router = x.to(torch.bfloat16), router.to(torch.bfloat16)
+
+    def run(n):
+        extra = dict(activation_scales=act[:n].contiguous(), weight_scale=ws) if fp8 else {}
+        return gm.route_project(x[:n].contiguous(), router, scale, want_logits=True, **extra)
+
+    for few, many in zip(run(rows), run(300)):
+        assert torch.equal(few[:rows], many[:rows])
+
+
 def test_router_projection_feeds_the_layer(oracle, cuda_device):
     """The fused router in front of the expert runner: the layer step made of C-ABI calls only."""
     import gevva_b200 as gm
