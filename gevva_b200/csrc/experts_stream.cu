@@ -20,7 +20,9 @@
 // groups of eight rows), 12 publishes finished w13 items.  Seven stages of one K block (256 elements); four accumulators of 64 columns,
 // so nothing waits for a drain.  In the w13 epilogue a thread holds one weight row for eight tokens, so
 // bf16(alpha * acc), which is what the reference's GEMM stores, changes hands through shared memory and a
-// thread then owns one column of a token: GeGLU, block maximum over sixteen lanes, codes.  The w2
+// thread then owns one column of four tokens: GeGLU, block maxima over sixteen lanes, codes.  (One token at a
+// time, with the scale worked out in all sixteen lanes, this took 87000 of 165000 cycles at 613 tokens and
+// bounded the launch; now 48000, a layer 113.6 -> 110.9 us.)  The w2
 // epilogue pairs two columns by one shuffle per two tokens and stores 64-byte pieces of a row.
 //
 // A w2 item needs the w2 operand rows of its expert: when the epilogue warps have stored an item, a
@@ -699,32 +701,69 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
           stop = true;
           break;
         }
-        for (int token = et >> 6; token < kStExchangeRows; token += 4) {
+        // four tokens a thread (of 16 a round): their chains overlap, and the block's scale is worked out once
+        // for every four lanes instead of in all sixteen
+        for (int token = (et >> 6) * 4; token < kStExchangeRows; token += 16) {
           if (base + token >= rows) break;
-          const float up = __bfloat162float(smem->exchange[buffer][token][column]);
-          const float gate = __bfloat162float(smem->exchange[buffer][token][64 + column]);
-          const float v = __fmul_rn(gelu_of_bf16(gate, &smem->tables), up);
-          float maximum = fabsf(v);
+          float v[4], maximum[4];
+          bool in_table = true;
 #pragma unroll
-          for (int offset = 8; offset; offset >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
-          const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
+          for (int j = 0; j < 4; ++j) {
+            const float up = __bfloat162float(smem->exchange[buffer][token + j][column]);
+            const float gate = __bfloat162float(smem->exchange[buffer][token + j][64 + column]);
+            const int index = erf_index((__float_as_uint(gate) >> 16) & 0x7fffu);
+            in_table &= index >= 0 || base + token + j >= rows;  // rows past the end hold anything
+            v[j] = __fmul_rn(gelu_from_erf(gate, smem->tables.erf_of[max(index, 0)]), up);
+          }
+          if (!in_table) {
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j) {
+              const float exact = __fmul_rn(gelu_of_bf16(__bfloat162float(smem->exchange[buffer][token + j][64 + column]), &smem->tables),
+                                            __bfloat162float(smem->exchange[buffer][token + j][column]));
+              if (j == 0) v[0] = exact;
+              else if (j == 1) v[1] = exact;
+              else if (j == 2) v[2] = exact;
+              else v[3] = exact;
+            }
+          }
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) maximum[j] = fabsf(v[j]);
+          // maxima over the block's sixteen lanes; lane 8a + 4b + c of the block is left with token 2a + b's
+          const bool a = lane & 8, b = lane & 4;
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float received = __shfl_xor_sync(0xffffffffu, a ? maximum[j] : maximum[j + 2], 8);
+            maximum[j] = fmaxf(a ? maximum[j + 2] : maximum[j], received);
+          }
+          float most = fmaxf(b ? maximum[1] : maximum[0], __shfl_xor_sync(0xffffffffu, b ? maximum[0] : maximum[1], 4));
+          most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 2));
+          most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 1));
+          const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, most)));
           const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, smem->tables.reciprocals)
                                                                    : scale_inverse_divided(multiplier, scale);
-          const float scaled = __fmul_rn(v, inverse);
-          // columns 2c and 2c + 1 make byte c of the block's eight code bytes
-          const float other = __shfl_xor_sync(0xffffffffu, scaled, 1);
-          uint32_t word = encode_e2m1x2(scaled, other) << (8 * ((column >> 1) & 3));  // meaningful in even lanes
-          if (column & 1) word = 0;
-          word |= __shfl_xor_sync(0xffffffffu, word, 2);
-          word |= __shfl_xor_sync(0xffffffffu, word, 4);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = __fmul_rn(v[j], __shfl_sync(0xffffffffu, inverse, (lane & 16) | (4 * j)));
+          // Columns 2c and 2c + 1 make byte c of a block's eight code bytes.  Even lanes go on with tokens 0 and 1, odd
+          // ones with 2 and 3; then lane bit 1 picks one of the two, and lanes 0..3 of a block end with a token each.
+          const bool odd = lane & 1, second = lane & 2;
+          const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[2], 1);
+          const float r1 = __shfl_xor_sync(0xffffffffu, odd ? v[1] : v[3], 1);
+          const uint32_t byte0 = odd ? encode_e2m1x2(r0, v[2]) : encode_e2m1x2(v[0], r0);
+          const uint32_t byte1 = odd ? encode_e2m1x2(r1, v[3]) : encode_e2m1x2(v[1], r1);
+          const uint32_t neighbour = __shfl_xor_sync(0xffffffffu, second ? byte0 : byte1, 2);
+          uint32_t word = second ? neighbour | (byte1 << 8) : byte0 | (neighbour << 8);
+          word |= __shfl_down_sync(0xffffffffu, word, 4) << 16;
           const uint32_t high = __shfl_down_sync(0xffffffffu, word, 8);
-          if ((column & 15) == 0) {
-            const int block = it.n_tile * 4 + (column >> 4);
-            *reinterpret_cast<uint2*>(p.inter_codes + static_cast<size_t>(row0 + base + token) * (kInter / 2) + block * 8) =
+          const int block = it.n_tile * 4 + (column >> 4);
+          const int coded = base + token + 2 * (lane & 1) + ((lane >> 1) & 1);
+          if ((column & 15) < 4 && coded < rows)
+            *reinterpret_cast<uint2*>(p.inter_codes + static_cast<size_t>(row0 + coded) * (kInter / 2) + block * 8) =
                 make_uint2(word, high);
+          const int scaled_token = base + token + 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1);
+          if ((lane & 3) == 0 && scaled_token < rows)
             p.inter_scales[static_cast<size_t>(smem->scale_rows[it.expert]) * (kInter / 16) +
-                           sf_offset(first + base + token, block, kInter / 16)] = static_cast<uint8_t>(scale);
-          }
+                           sf_offset(first + scaled_token, block, kInter / 16)] = static_cast<uint8_t>(scale);
         }
         buffer ^= 1;
       }
