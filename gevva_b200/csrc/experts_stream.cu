@@ -32,12 +32,18 @@
 // SM) and no wait can form a cycle.
 //
 // In its kFront form the kernel also sorts the routes and quantises the input: every CTA ranks the whole
-// batch's routes by a counting sort (13 warps, a stretch of routes each) and derives the group geometry for
-// itself; CTA c quantises tokens c and c + CTAs with eleven warps, eight columns a thread (88 threads of
-// 32 columns took 4.3 us of the chain, this takes about one), then adds one to a counter that the
-// activation side waits for.  At 200 tokens that saves 4 us of a layer against launches of their own; with
-// five tokens a CTA it would lose five (613 tokens: 119.5 against 114.1 us).  Meanwhile the weight side has filled its stages.  The CTA that finishes last
-// puts all counters back to zero.
+// batch's routes by a counting sort (12 warps, a stretch of routes each) and derives the group geometry for
+// itself; CTA c quantises tokens c and c + CTAs with eleven warps, a K block each, then adds one to a counter that
+// the activation side waits for.  At 200 tokens that saves 4 us of a layer against launches of their own; with
+// five tokens a CTA it would lose five (613 tokens: 119.5 against 114.1 us).
+// Until that counter is full, all that moves is the weights that fit the ring, and its chain (stores, their
+// release to the GPU, the poll, the copies) takes 5 to 8 us while they do.  So a CTA's first w13 item does not wait: if it has
+// at most eight rows, eleven warps quantise these into the pipeline stages, and the counter is full by the
+// time that the second item needs it.  24.5 -> 22.9 us a layer at 1 token, 36.1 -> 34.1 at 5, 53.7 -> 52.2 at 16, 70.2 -> 69.7
+// at 37, nothing from 64 on, where more rows take as long as the counter (with 24 rows allowed, 5 us slower at 200).
+// The code in front of the roles runs once a launch, and while the weights keep the way to L2 busy an instruction
+// line that has to be fetched costs up to a microsecond: it is kept small, loops are not unrolled.
+// The CTA that finishes last puts all counters back to zero.
 #include "gv_common.cuh"
 #include "gv_gemm_parts.cuh"
 #include "gv_launchers.h"
@@ -54,8 +60,6 @@ constexpr int kStWeightWarp = 0, kStMmaWarp = 1, kStTokenWarp = 2, kStScaleWarp 
 constexpr int kStEpilogueWarps = 8;
 constexpr int kStPublishWarp = kStEpilogueWarp + kStEpilogueWarps;     // 12
 constexpr int kStThreads = (kStPublishWarp + 1) * 32;                  // 416
-constexpr int kStQuantiseThreads = kStThreads - 64;       // warps 1..11: 352 = 2816 / 8
-static_assert(kStQuantiseThreads * 8 == kHidden, "eight columns a thread");
 constexpr uint32_t kStTmemColumns = 512;
 constexpr uint32_t kStSfColumn = kStAccStages * kStRows;  // 256
 constexpr uint32_t kStSfColumnsPerStage = 32;             // 16 for the weights, 16 for the rows
@@ -64,12 +68,17 @@ constexpr int kStWeightBytes = kTileM * kTileKBytes;      // 16 KiB
 constexpr int kStTokenBytes = kStRows * kTileKBytes;      // 8 KiB
 constexpr int kStDownTiles = kHidden / 128;               // 22 w2 items a chunk
 constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
+static_assert(kStMmaWarp == 1 && kStPublishWarp - 1 == kStUpKBlocks, "warps 1..11 quantise a K block each");
 constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192
 constexpr int kStDownLastMmas = 3;
 constexpr int kStMaxChunks = 256;
 constexpr int kStExchangeRows = 32;
 constexpr int kStWarps = kStThreads / 32;
 constexpr int kStOwnTokens = 2;                           // kFront: tokens a CTA quantises, at most
+constexpr int kStRankWarps = kStWarps - 1;                // kFront: all but the first rank the routes
+constexpr int kStStretch = 224;                           // routes of each, at most
+constexpr int kStFrontTokens = kStStretch * kStRankWarps / kTopK;  // 336
+constexpr int kStSelfRows = 8;                            // kFront: rows of a first item that the CTA quantises itself, at most
 
 struct alignas(1024) StreamSmem {
   uint8_t a[kStStages][kStWeightBytes];
@@ -78,7 +87,10 @@ struct alignas(1024) StreamSmem {
   uint8_t sfb[kStStages][kSfStageBytes];
   union {
     __nv_bfloat16 exchange[2][kStExchangeRows][128];  // [token][MMA row]
-    int warp_counts[kStWarps][kExperts];              // the sort's, before
+    struct {                                          // the sort's, before
+      int warp_counts[kStRankWarps][kExperts];
+      uint8_t route_expert[kStRankWarps * kStStretch];
+    };
   };
   uint64_t full[kStStages], empty[kStStages], sf_full[kStStages];
   uint64_t acc_full[kStAccStages], acc_empty[kStAccStages];
@@ -102,6 +114,7 @@ struct alignas(1024) StreamSmem {
   alignas(16) float route_multiplier[kStOwnTokens * kTopK];
   unsigned long long route_scale_base[kStOwnTokens * kTopK];
   float scale_q1[kExperts];
+  short first_token[kStSelfRows];          // kFront: tokens of the CTA's first w13 item's rows
   GegluTables tables;
 };
 constexpr size_t kStSmemBytes = sizeof(StreamSmem) + 1024;
@@ -217,6 +230,11 @@ __device__ __forceinline__ int stream_load_acquire(const int* address) {
   return value;
 }
 
+// Adds one, after everything that happened before in this thread and in those it has synchronised with.
+__device__ __forceinline__ void stream_add_release(int* address) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(address) : "memory");
+}
+
 // Bounded acquire spin of a whole warp on a counter in global memory.
 __device__ __forceinline__ bool stream_wait_counter(const int* counter, int target, StreamSmem* smem, int* status) {
   const long long start = clock64();
@@ -235,21 +253,39 @@ __device__ __forceinline__ bool stream_wait_counter(const int* counter, int targ
   return __all_sync(0xffffffffu, ready);
 }
 
-// One token by 352 threads, eight columns each (`raw`; two threads a 16-value block): the codes and
-// scale bytes of its eight routes (entries first..first+7 of the route arrays) go to their sorted rows.  The arithmetic of quantize_routes_of_token.
-__device__ __forceinline__ void stream_quantise_token(const StreamParams& p, const StreamSmem* smem, int first, int q,
-                                                      const uint4& raw) {
-  float values[8];
+// Eight columns a lane (two lanes a 16-value block): code bytes and scale of the block.  The arithmetic of
+// quantize_routes_of_token.
+__device__ __forceinline__ uint32_t stream_quantise(const float (&values)[8], float maximum, float multiplier,
+                                                    const float* reciprocals, uint32_t& codes) {
+  const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
+  const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, reciprocals)
+                                                           : scale_inverse_divided(multiplier, scale);
+  codes = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    codes |= encode_e2m1x2(__fmul_rn(values[2 * i], inverse), __fmul_rn(values[2 * i + 1], inverse)) << (8 * i);
+  return scale;
+}
+
+__device__ __forceinline__ float stream_block_maximum(const uint4& raw, float (&values)[8]) {
   unpack_bf16x8(raw, values);
   float maximum = 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) maximum = fmaxf(maximum, fabsf(values[i]));
-  maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, 1));
-  // scale groups q/2 of a row, four to an aligned word of the swizzled layout: eight threads a word
-  const uint32_t scale_offset = static_cast<uint32_t>(q >> 3) * kSfAtomBytes;
+  return fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, 1));
+}
+
+// K block `kb` of one token by a warp: the codes and scale bytes of its eight routes (entries first..first+7 of
+// the route arrays) go to their sorted rows.
+__device__ __forceinline__ void stream_quantise_token(const StreamParams& p, const StreamSmem* smem, int first, int kb,
+                                                      int lane, const uint4& raw) {
+  float values[8];
+  const float maximum = stream_block_maximum(raw, values);
+  // scale groups of a row go four to an aligned word of the swizzled layout: eight lanes a word
+  const uint32_t scale_offset = static_cast<uint32_t>(4 * kb + (lane >> 3)) * kSfAtomBytes;
   uint32_t codes = 0, scale_word = 0, previous = 0;
   bool have = false;
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < kTopK; ++k) {
     const int row = smem->route_row[first + k];
     if (row < 0) continue;
@@ -257,19 +293,54 @@ __device__ __forceinline__ void stream_quantise_token(const StreamParams& p, con
     if (!have || __float_as_uint(multiplier) != previous) {  // routes of equal static scale share the result
       have = true;
       previous = __float_as_uint(multiplier);
-      const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
-      const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, smem->tables.reciprocals)
-                                                               : scale_inverse_divided(multiplier, scale);
-      codes = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        codes |= encode_e2m1x2(__fmul_rn(values[2 * i], inverse), __fmul_rn(values[2 * i + 1], inverse)) << (8 * i);
+      const uint32_t scale = stream_quantise(values, maximum, multiplier, smem->tables.reciprocals, codes);
       scale_word = scale | (__shfl_down_sync(0xffffffffu, scale, 2) << 8) | (__shfl_down_sync(0xffffffffu, scale, 4) << 16) |
                    (__shfl_down_sync(0xffffffffu, scale, 6) << 24);
     }
-    *reinterpret_cast<uint32_t*>(p.packed + static_cast<size_t>(row) * (kHidden / 2) + 4 * q) = codes;
-    if ((q & 7) == 0) *reinterpret_cast<uint32_t*>(p.scales + smem->route_scale_base[first + k] + scale_offset) = scale_word;
+    *reinterpret_cast<uint32_t*>(p.packed + static_cast<size_t>(row) * (kHidden / 2) + kb * kTileKBytes + 4 * lane) = codes;
+    if ((lane & 7) == 0) *reinterpret_cast<uint32_t*>(p.scales + smem->route_scale_base[first + k] + scale_offset) = scale_word;
   }
+}
+
+// K block `kb` of an item's `rows` tokens (smem->first_token) by a warp, straight into a pipeline stage: codes in
+// the 128B-swizzled layout of the row side, scale bytes at rows scale_row.. of the stage's four atoms.  The tokens
+// are fetched into the stage first, twelve at a time and 512 bytes each from its byte 2048 on, where the codes that replace them
+// never reach a token that is still to be read (up to 24 rows: code row 12 + j lies below byte 2048 + 512 j).
+// Everything here runs once a launch, while the weights keep the way to L2 busy, and an instruction line that has to
+// be fetched takes about a microsecond: hence one copy of the code and no unrolling.
+__device__ __noinline__ void stream_quantise_stage(const uint4* input, StreamSmem* smem, int stage, int kb, int rows,
+                                                   int scale_row, float multiplier, int lane) {
+  constexpr int kAhead = 12;
+  static_assert(kStSelfRows <= 2 * kAhead && 2048 + kAhead * 512 == kStTokenBytes, "codes and tokens in one stage");
+  uint8_t* const b = smem->b[stage];
+  uint8_t* const sf = smem->sfb[stage] + (lane >> 3) * kSfAtomBytes + ((lane >> 1) & 3);
+  input += kb * (kTileK / 8) + lane;
+#pragma unroll 1
+  for (int base = 0; base < rows; base += kAhead) {
+    const int end = rows < base + kAhead ? rows : base + kAhead;
+    uint8_t* token = b + 2048 + lane * 16;
+    __syncwarp();
+#pragma unroll 1
+    for (int r = base; r < end; ++r, token += 512)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(token)),
+                   "l"(input + static_cast<size_t>(smem->first_token[r]) * (kHidden / 8))
+                   : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    token = b + 2048 + lane * 16;
+#pragma unroll 1
+    for (int r = base; r < end; ++r, token += 512) {
+      float values[8];
+      const float maximum = stream_block_maximum(*reinterpret_cast<const uint4*>(token), values);
+      uint32_t codes;
+      const uint32_t scale = stream_quantise(values, maximum, multiplier, smem->tables.reciprocals, codes);
+      *reinterpret_cast<uint32_t*>(b + r * kTileKBytes + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) = codes;
+      const int n = scale_row + r;
+      if ((lane & 1) == 0) sf[(n & 31) * 16 + ((n >> 5) & 3) * 4] = static_cast<uint8_t>(scale);
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&smem->full[stage]);
 }
 
 template <bool kFront>
@@ -311,7 +382,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   __syncthreads();
   fill_geglu_tables(&smem->tables);
   if (kFront)
-    for (int i = tid; i < kStWarps * kExperts; i += kStThreads) (&smem->warp_counts[0][0])[i] = 0;
+    for (int i = tid; i < kStRankWarps * kExperts; i += kStThreads) (&smem->warp_counts[0][0])[i] = 0;
   grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
@@ -322,42 +393,59 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   // ---------------- group geometry ----------------
   const bool has_token = kFront && cta < p.tokens;
   const int ctas = gridDim.x;
-  uint4 raw = make_uint4(0, 0, 0, 0);
-  float scale_q1 = 0.0f;
+  const int routes = kFront ? p.tokens * kTopK : 0;
+  // warp 1 + w ranks routes [w * stretch, (w + 1) * stretch) among those of its own stretch
+  const int rank_warp = warp > 0 ? warp - 1 : 0;
+  const int stretch = ((routes + kStRankWarps - 1) / kStRankWarps + 31) & ~31;
+  const int stretch_begin = warp > 0 ? rank_warp * stretch : routes;
+  const int stretch_end = stretch_begin + stretch < routes ? stretch_begin + stretch : routes;
+  const int own = has_token ? (p.tokens - 1 - cta) / ctas + 1 : 0;
+  const int kb = warp - kStMmaWarp;  // 0..10: the K block that the warp quantises
+  uint4 own_raw[kStOwnTokens];
   if constexpr (kFront) {
-    // the first token and the static scales are on their way while the geometry is worked out
-    if (has_token && tid >= 32 && tid < 32 + kStQuantiseThreads)
-      raw = __ldg(reinterpret_cast<const uint4*>(p.input + static_cast<size_t>(cta) * kHidden) + (tid - 32));
-    if (has_token && tid < kExperts) scale_q1 = p.in_scale_q1[tid];
-    // warp w ranks routes [w * stretch, (w + 1) * stretch) among those of its own stretch
-    const int routes = p.tokens * kTopK;
-    const int stretch = ((routes + kStWarps - 1) / kStWarps + 31) & ~31;
-    int* counts = smem->warp_counts[warp];
-    for (int base = warp * stretch; base < (warp + 1) * stretch && base < routes; base += 32) {
+    const float scale_q1 = tid < kExperts ? p.in_scale_q1[tid] : 0.0f;
+    int* const counts = smem->warp_counts[rank_warp];
+    uint8_t* const route_expert = smem->route_expert + rank_warp * kStStretch + lane;
+    uint32_t ids[kStStretch / 32];
+#pragma unroll
+    for (int k = 0; k < kStStretch / 32; ++k) {
+      const int route = stretch_begin + 32 * k + lane;
+      ids[k] = route < stretch_end ? static_cast<uint32_t>(p.expert_ids[route]) : kExperts;
+    }
+    // of this CTA's tokens, a K block each that the warp will quantise (see below) is on its way meanwhile
+    const uint4* const own_input = reinterpret_cast<const uint4*>(p.input) + static_cast<size_t>(cta) * (kHidden / 8) + kb * (kTileK / 8) + lane;
+    if (kb >= 0 && kb < kStUpKBlocks) {
+#pragma unroll
+      for (int t = 0; t < kStOwnTokens; ++t)
+        if (t < own) own_raw[t] = __ldg(own_input + static_cast<size_t>(t) * ctas * (kHidden / 8));
+    }
+    if (warp > 0)
+#pragma unroll
+      for (int k = 0; k < kStStretch / 32; ++k) route_expert[32 * k] = static_cast<uint8_t>(ids[k] < kExperts ? ids[k] : kExperts);
+    __syncwarp();
+#pragma unroll 1
+    for (int base = stretch_begin; base < stretch_end; base += 32) {
       const int route = base + lane;
-      int expert = route < routes ? p.expert_ids[route] : -1;
-      if (expert < 0 || expert >= kExperts) {
-        if (cta == 0 && route < routes) atomicExch(status, static_cast<int>(kBadExpertId));
-        expert = kExperts;
-      }
+      const int expert = route_expert[base - stretch_begin];
+      if (expert == kExperts && cta == 0 && route < stretch_end) atomicExch(status, static_cast<int>(kBadExpertId));
       const uint32_t peers = __match_any_sync(0xffffffffu, expert);
       const int before = expert < kExperts ? counts[expert] : 0;
       __syncwarp();
       if (expert < kExperts && (peers & (0u - peers)) == (1u << lane)) counts[expert] = before + __popc(peers);
       __syncwarp();
-      const int token = route >> 3;
-      if (route < routes && token % ctas == cta) {
-        const int slot = token / ctas * kTopK + (route & (kTopK - 1));
+      int token = (route >> 3) - cta;  // this CTA's are 0 and ctas
+      if (route < stretch_end && (token == 0 || token == ctas)) {
+        const int slot = (token ? kTopK : 0) + (route & (kTopK - 1));
         smem->own_expert[slot] = expert;
         smem->own_rank[slot] = before + __popc(peers & ((1u << lane) - 1u));
-        smem->own_warp[slot] = warp;
+        smem->own_warp[slot] = rank_warp;
       }
     }
     __syncthreads();
     if (tid < kExperts) {
       int running = 0;
 #pragma unroll
-      for (int w = 0; w < kStWarps; ++w) {
+      for (int w = 0; w < kStRankWarps; ++w) {
         const int c = smem->warp_counts[w][tid];
         smem->warp_counts[w][tid] = running;
         running += c;
@@ -428,11 +516,37 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   const StreamSchedule schedule(smem->chunks);
   bool ok = true;
 
-  if (has_token && warp != kStWeightWarp && warp != kStPublishWarp) {
-    // ---------------- this CTA's tokens: their routes' rows, then their codes ----------------
-    const int q = tid - 32;
-    const int own = (p.tokens - 1 - cta) / ctas + 1;
-    if (q < own * kTopK) {
+  // kFront: the CTA's first w13 item does not wait for the grid's quantised rows: its own warps put them into
+  // the pipeline stages (not the weight warp's concern, which leaves it out)
+  bool self_first = kFront && schedule.up_count > 0;
+  if (kFront && warp != kStWeightWarp) {  // the weights are under way meanwhile
+    StreamItem it{};
+    int first = 0, first_rows = 0;
+    if (self_first) {
+      it = schedule.item(0, smem);
+      first = it.chunk * kStRows;
+      first_rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
+      first_rows = first_rows > kStRows ? kStRows : first_rows;
+      self_first = first_rows <= kStSelfRows;  // with more, the grid's rows are there as early
+    }
+    if (self_first) {
+      // the tokens of its rows, by the order of the sort
+      if (stretch_begin < stretch_end) {
+        int rank = smem->warp_counts[rank_warp][it.expert] - first;
+#pragma unroll 1
+        for (int base = stretch_begin; base < stretch_end; base += 32) {
+          const int route = base + lane;
+          const bool mine = smem->route_expert[rank_warp * kStStretch + route - stretch_begin] == it.expert;
+          const uint32_t all = __ballot_sync(0xffffffffu, mine);
+          const int r = rank + __popc(all & ((1u << lane) - 1u));
+          if (mine && r >= 0 && r < kStSelfRows) smem->first_token[r] = static_cast<short>(route >> 3);
+          rank += __popc(all);
+        }
+      }
+    }
+    const int q = tid - kStPublishWarp * 32;
+    if (q >= 0 && q < own * kTopK) {
+      // where this CTA's tokens' routes go
       const int expert = smem->own_expert[q];
       int dst = -1;
       if (expert < kExperts) {  // others are flagged above
@@ -444,22 +558,29 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
         p.plan.inverse_routes[route] = dst;
         smem->route_multiplier[q] = smem->scale_q1[expert];
         smem->route_scale_base[q] = static_cast<unsigned long long>(smem->scale_rows[expert]) * (kHidden / 16) +
-                                    sf_offset(rank, 0, kHidden / 16);
+                                      sf_offset(rank, 0, kHidden / 16);
       }
       smem->route_row[q] = dst;
     }
-    named_barrier(1, kStQuantiseThreads);
-    for (int i = 0; i < own; ++i) {
-      uint4 next = raw;
-      if (i + 1 < own)
-        next = __ldg(reinterpret_cast<const uint4*>(p.input + static_cast<size_t>(cta + (i + 1) * ctas) * kHidden) + q);
-      stream_quantise_token(p, smem, i * kTopK, q, raw);
-      raw = next;
+    named_barrier(3, kStThreads - 32);
+    const float multiplier = self_first ? smem->scale_q1[it.expert] : 0.0f;
+    if (has_token && kb >= 0) {
+      constexpr int kOwnThreads = (kStUpKBlocks + 1) * 32;
+      if (warp == kStPublishWarp) {
+        named_barrier(1, kOwnThreads);
+        if (lane == 0) stream_add_release(p.plan.front_sync);
+      } else {
+#pragma unroll 1
+        for (int t = 0; t < own; ++t) stream_quantise_token(p, smem, t * kTopK, kb, lane, own_raw[t ? 1 : 0]);
+        asm volatile("bar.arrive 1, %0;" ::"n"(kOwnThreads) : "memory");
+      }
     }
-    named_barrier(1, kStQuantiseThreads);
-    if (q == 0) {
-      __threadfence();
-      atomicAdd(p.plan.front_sync, 1);
+    if (self_first && kb >= 0 && kb < kStStages)
+      stream_quantise_stage(reinterpret_cast<const uint4*>(p.input), smem, kb, kb, first_rows, first % kTileM, multiplier, lane);
+    if (self_first && kb >= kStStages && kb < kStUpKBlocks) {
+      // the stage's second use
+      if (__all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[kb - kStStages], 0u, smem, status)))
+        stream_quantise_stage(reinterpret_cast<const uint4*>(p.input), smem, kb - kStStages, kb, first_rows, first % kTileM, multiplier, lane);
     }
   }
 
@@ -468,12 +589,12 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     const bool weight_side = warp == kStWeightWarp;
     int stage = 0, issued = 0;
     uint32_t phase = 0;
-    if (kFront && !weight_side) {
-      // the w13 operand exists once every CTA with tokens has quantised them and counted itself
-      ok = stream_wait_counter(p.plan.front_sync, p.tokens < ctas ? p.tokens : ctas, smem, status);
-      asm volatile("fence.proxy.async.global;" ::: "memory");
+    const int begin = self_first && !weight_side ? 1 : 0;
+    if (begin) {
+      stage = kStUpKBlocks % kStStages;
+      phase = kStUpKBlocks / kStStages & 1;
     }
-    for (int i = 0; ok && i < schedule.count; ++i) {
+    for (int i = begin; ok && i < schedule.count; ++i) {
       const StreamItem it = schedule.item(i, smem);
       const int k_blocks = it.down ? kStDownKBlocks : kStUpKBlocks;
       const int first = it.chunk * kStRows;
@@ -486,6 +607,12 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
                      : p.w13_scales + static_cast<size_t>(it.expert * kUnitSlots + it.n_tile) * kStUpKBlocks * kSfStageBytes;
       } else {
         const size_t scale_row = smem->scale_rows[it.expert] + first / kTileM * kTileM;
+        if (kFront && i == begin && !it.down) {
+          // the w13 operand exists once every CTA with tokens has quantised them and counted itself
+          ok = stream_wait_counter(p.plan.front_sync, p.tokens < ctas ? p.tokens : ctas, smem, status);
+          if (!ok) break;
+          asm volatile("fence.proxy.async.global;" ::: "memory");
+        }
         sf = it.down ? p.inter_scales + scale_row * (kInter / 16) : p.input_scales + scale_row * (kHidden / 16);
         if (it.down) {
           // the rows exist once every w13 item of the expert has been counted; they were written by ordinary stores of other SMs and are read through the async proxy
@@ -605,8 +732,8 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   } else if (warp == kStPublishWarp) {
     // ---------------- publisher ----------------
     // Making an item's stores visible to the grid takes one to two microseconds under load.  The epilogue
-    // warps leave that to this warp (their progress is a release to the CTA, the fence here extends it to
-    // the GPU) and go on; several items that finish meanwhile share one fence.
+    // warps leave that to this warp (their progress is a release to the CTA, the additions here extend it to
+    // the GPU) and go on.
     int published = 0;
     const long long start = clock64();
     while (published < schedule.up_count) {
@@ -617,9 +744,10 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
         __nanosleep(64);
         continue;
       }
-      if (lane == 0) __threadfence();
+      __threadfence_block();
       __syncwarp();
-      for (int i = published + lane; i < done; i += 32) atomicAdd(p.plan.tile_ready + schedule.item(i, smem).expert, 1);
+      for (int i = published + lane; i < done; i += 32) stream_add_release(p.plan.tile_ready + schedule.item(i, smem).expert);
+      __syncwarp();
       published = done;
     }
   } else {
@@ -824,11 +952,12 @@ StreamMaps make_maps(const StreamOperands& op) {
 
 }  // namespace
 
+static_assert(kStOwnTokens == 2 && kExperts <= 255, "the front's indexes");
 static_assert(kStRows / 8 == kStreamBoxes, "one map per box height");
 static_assert(kExperts + kStreamMaxTokens * kTopK / kStRows <= kStMaxChunks, "chunk list");
 
 bool stream_layer_fits(int tokens, int sm_count) {
-  return tokens <= kStreamMaxTokens && tokens <= sm_count * kStOwnTokens;
+  return tokens <= kStFrontTokens && tokens <= sm_count * kStOwnTokens;
 }
 
 

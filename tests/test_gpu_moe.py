@@ -685,6 +685,36 @@ def test_decode_kernel_that_sorts_and_quantises_itself(gm, weights, cuda_device,
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("tokens", [8, 9, 65, 72, 73, 137])
+def test_streaming_front_first_items(gm, weights, cuda_device, tokens, monkeypatch):
+    """The streaming launch's CTAs quantise the rows of their first items themselves up to eight rows, also
+    those of a second or third 64-row chunk of an expert (65, 72 and 137 tokens: one, eight and nine rows of
+    it): the routed rows of a runner that sorts and quantises in launches of its own."""
+    from gevva_b200 import runtime as rt
+    edges = [c for c in (tokens, 1, 7, 8, 9) if c <= tokens]
+    rng = np.random.default_rng(100 + tokens)
+    mine = [[] for _ in range(tokens)]
+    for expert, count in enumerate(edges):
+        for t in rng.permutation(tokens)[:count]:
+            mine[t].append(expert)
+    ids = np.array([rng.permutation(m + list(rng.choice(np.arange(8, EXPERTS), TOP_K - len(m), replace=False)))
+                    for m in mine], dtype=np.int32)
+    x = hashgen.activations(tokens, HIDDEN, 14, cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    outs = []
+    for front in ("0", "1"):
+        monkeypatch.setenv("GEVVA_MOE_DECODE_FRONT", front)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        out = torch.zeros_like(x)
+        for _ in range(2):
+            runner.launch_batch(x, torch.from_numpy(ids).to(cuda_device), rw, out, tokens)
+        runner.check()
+        outs.append((out, runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].clone()))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    assert outs[0][0].float().abs().max() > 0
+
+
 @pytest.mark.parametrize("tokens", [147, 149, 296, 297])
 def test_streaming_front_with_two_tokens_an_sm(gm, weights, cuda_device, tokens, monkeypatch):
     """Sort and quantiser inside the streaming launch where some CTAs prepare two tokens and others one
