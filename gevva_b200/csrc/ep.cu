@@ -642,7 +642,7 @@ int gevva_moe_ep_create(gevva_moe_ep** out, const gevva_moe_weights* local_weigh
   sp.remap = remap;
 
   gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(local_weights->w13_sf), ep->w13_sf_units, el,
-                                    nullptr);
+                                    false, nullptr);
   gv::launch_retile_w2_scales(static_cast<const uint8_t*>(local_weights->w2_sf), ep->w2_sf_down, el, nullptr);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);

@@ -1,30 +1,31 @@
 // Fused w13 GEMM + GeGLU + NVFP4 requantisation run by CTA pairs, weights on the MMA's M side.
 //
-// Why this shape.  An SM takes in at most about 140 GB/s through TMA (measured with all SMs
-// streaming from L2), and one K block of 256 elements of a 128 x 256 tile needs 54 KiB for 512
-// tensor-pipe cycles: the one-CTA kernel (grouped_gemm.cu) is bound by that intake, not by the
-// tensor pipe.  Here a CTA pair (tcgen05 cta_group::2, M = 256) holds 256 weight rows, 128 per
-// CTA, against up to 256 token rows of one expert on the N side, half of them loaded by each CTA:
-// at most 38 KiB per CTA and K block.  And because the tokens sit on N, which may be any multiple
-// of 16, a group of 300 rows costs 304 rows of tensor work instead of three 128-row tiles.
+// What bounds it.  One K block of 256 elements of a 128 x 256 tile costs 512 tensor-pipe cycles, but in the
+// one-CTA kernel (grouped_gemm.cu) shared memory has to take in 54 KiB and give the MMAs 48 KiB for it: 800
+// cycles.  Here a CTA pair (tcgen05 cta_group::2, M = 256) holds 256 weight rows, 128 per CTA, against up to 208
+// token rows of one expert on the N side, half of them loaded by each CTA: at most 35 KiB in and 29 out.  And because
+// the tokens sit on N, which may be any multiple of 16, a group of 200 rows is one item and not two 128-row tiles.
+// An item is 44 MMAs of about 105 cycles and their scale copies, 5345 cycles with neither loads nor epilogue and
+// 6600 in all (4096 tokens).  Beside large batches the clock drops to 1.5 GHz under the power limit.
+// Alone (us, one-CTA kernel -> this one; uniform routing): 53.1 -> 53.2 at 1024 tokens, 63.9 -> 58.9 at 2048,
+// 83.5 -> 70 at 3000, 97 -> 95 at 4096, 172 -> 151 at 8192, 330 -> 293 at 16384.
 //
-// Work.  A chunk is one entry of the route plan's tile-pair list: up to 256 consecutive rows of
-// one expert starting at a 128-row tile (so its activation scales are whole 128-row blocks).  The
-// intermediate width 704 is cut into 11 units of 64 columns; a CTA computes one unit as 128 MMA
-// rows, the unit's 64 up rows on lanes 0..63 and its 64 gate rows on lanes 64..127, so that up
-// and gate of a column end in the same CTA.  A work item is (chunk, two units); the second CTA of
-// the sixth item has no unit (its weight scales are zero and its results are dropped).
+// Work.  A chunk is up to 208 consecutive rows of an expert; one with more is cut into stretches of 192, so that a
+// chunk's scales start at a 64-row boundary of their 128-row blocks.  The intermediate width 704 is cut into 11 units
+// of 64 columns; a CTA computes one unit as 128 MMA rows, the unit's up and gate rows interleaved so that a thread
+// of the epilogue finds both of a column in its registers (see there; the order costs nothing: it is a
+// five-dimensional view of the same weights, and the scales have a re-tiled copy made at runner creation).  A work
+// item is (chunk, two units); the second CTA of the sixth item has no unit (its weight scales are zero and its
+// results are dropped).
 //
-// Protocol.  As in every kernel here: a TMA producer (one warp per CTA) fills a ring of stages,
+// Protocol.  Two TMA producers in each CTA (weight side, token side) fill a ring of six stages,
 // all loads of both CTAs complete on the `full` barrier of the first CTA (tensor-map loads in
 // their cta_group::2 form, no multicast; the scale atoms travel through tensor maps too).  There
 // the MMA thread copies the scale atoms of a landed stage into tensor memory, issues four MMAs
-// (copies and MMAs of one thread execute in order) and commits to `empty` of both CTAs.  Spills
-// are expensive here (shared memory leaves almost no L1), which is why the epilogue holds one
-// 32-column load at a time.  The 16 epilogue warps of each CTA copy the accumulator (lanes = weight
-// rows, columns = tokens) to registers as bf16(alpha * acc), release it, transpose it through
-// shared memory and then, one thread per (token, 16 columns), apply erf-GELU(gate) * up and
-// quantise exactly like the two-kernel form.  Every wait is bounded.
+// (copies and MMAs of one thread execute in order) and commits to `empty` of both CTAs.  Two accumulators, so that the
+// eight epilogue warps of each CTA work on one item while the next is computed.  (With the accumulator transposed
+// through shared memory by sixteen warps that traffic bounded the kernel, 107 us at 4096 tokens; with this epilogue
+// twelve or sixteen warps are 3 to 8 % slower than eight, and five stages up to 8 % slower than six.)  Every wait is bounded.
 #include "gv_common.cuh"
 #include "gv_gemm_parts.cuh"
 #include "gv_launchers.h"
@@ -33,37 +34,41 @@ namespace gv {
 
 namespace {
 
-constexpr int kWpStages = 4;
-constexpr int kWpThreads = (2 + 4 * kEpilogueWarpsPerQuarter) * 32;     // 576: leaves 112 registers per thread
+constexpr int kWpStages = 6;
+constexpr int kWpParts = 2;                    // epilogue warps a block of 16 columns
+constexpr int kWpTokenWarp = 0, kWpMmaWarp = 1, kWpEpilogueWarp = 2, kWpWeightWarp = kWpEpilogueWarp + 4 * kWpParts;
+constexpr int kWpThreads = (kWpWeightWarp + 1) * 32;
 constexpr uint32_t kWpTmemColumns = 512;
-constexpr uint32_t kWpSfColumn = 256;          // accumulator: columns [0, 256)
-constexpr uint32_t kWpSfColumnsPerStage = 48;  // per MMA j: weights at +12j, tokens 0..127 at +12j+4, 128..255 at +12j+8
+constexpr int kWpRows = 208;                   // rows of a chunk at most (MMA N), and accumulator columns
+constexpr int kWpChunk = 192;                  // rows of every chunk but the last of an expert with more than kWpRows
+constexpr int kWpAccStages = 2;
+// One K block's scales, per MMA j: weights at +12j, the chunk's two 128-row blocks at +12j+4 and +12j+8.
+constexpr uint32_t kWpSfColumn = kWpAccStages * kWpRows;
+static_assert(kWpSfColumn + 48 <= kWpTmemColumns, "tensor memory budget");
+constexpr int kWpTokenBytes = kWpRows / 2 * kTileKBytes;  // 13 KiB
 constexpr int kWpTileBytes = 128 * kTileKBytes;  // 16 KiB
 constexpr int kWpUnits = kInter / 64;            // 11
 constexpr int kWpUnitSlots = 12;                 // the re-tiled scales carry a twelfth, all-zero unit
 constexpr int kWpItemsPerChunk = kWpUnitSlots / 2;
-constexpr int kWpStagePitch = 256;               // one token of the transposed tile: 128 lanes x bf16
-constexpr int kWpStagingBytes = 32 * kWpStagePitch;
 
 struct alignas(1024) WpSmem {
   uint8_t w[kWpStages][kWpTileBytes];          // this CTA's 64 up + 64 gate weight rows
-  uint8_t x[kWpStages][kWpTileBytes];          // this CTA's half of the chunk's token rows
+  uint8_t x[kWpStages][kWpTokenBytes];         // this CTA's half of the chunk's token rows
   uint8_t sfw[kWpStages][kSfStageBytes];       // scales of this CTA's weight rows
   uint8_t sfx[kWpStages][2 * kSfStageBytes];   // scales of the chunk's one or two 128-row blocks
-  uint8_t staging[4][kWpStagingBytes];         // per token group of the epilogue: 32 tokens x 128 lanes, bf16
   uint64_t full[kWpStages];    // leader: the stage's bytes have landed in both CTAs
   uint64_t empty[kWpStages];   // both CTAs: the MMAs that read the stage have completed
-  uint64_t acc_full;           // both CTAs: the item's accumulator is complete
-  uint64_t acc_empty;          // leader: both CTAs' epilogues have copied the accumulator out
+  uint64_t acc_full[kWpAccStages];   // both CTAs: the item's accumulator is complete
+  uint64_t acc_empty[kWpAccStages];  // leader: both CTAs' epilogues have copied the accumulator out
   uint32_t tmem_base;
   volatile int abort;
-  int group_left[4];
+  // group geometry, by expert: first row, first scale row, chunks before it
+  int offsets[kExperts + 1], scale_rows[kExperts + 1], chunks[kExperts + 1], scan[4];
   GegluTables tables;
 };
 
 constexpr size_t kWpSmemBytes = sizeof(WpSmem) + 1024;
 static_assert(kWpSmemBytes <= 232448, "shared memory budget");
-static_assert(kWpSfColumn + kWpSfColumnsPerStage * kWpStages <= kWpTmemColumns, "tensor memory budget");
 
 __device__ __forceinline__ void wp_arrive_remote(uint64_t* local_bar, uint32_t target_cta) {
   const uint32_t remote = cluster_map_shared(smem_u32(local_bar), target_cta);
@@ -102,15 +107,13 @@ __device__ __forceinline__ void wp_load_3d(void* smem_dst, const void* tensor_ma
       : "memory");
 }
 
-// Asks for a box to be brought into L2 (no shared-memory destination, nothing to wait for).
-__device__ __forceinline__ void wp_prefetch_3d(const void* tensor_map, int x, int y, int z) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(tensor_map), "r"(x), "r"(y),
-               "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void wp_prefetch_2d(const void* tensor_map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tensor_map), "r"(x), "r"(y)
-               : "memory");
+// The 128 weight rows of a unit in the kernel's order: see make_w13_fragment_tensor_map.
+__device__ __forceinline__ void wp_load_weights(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int block) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%2, %3, %3, %3, %4}], [%5];" ::"r"(smem_u32(smem_dst)),
+      "l"(tensor_map), "r"(x), "r"(0), "r"(block), "r"(barrier)
+      : "memory");
 }
 
 __device__ __forceinline__ void wp_copy_sf(uint32_t tmem_address, uint32_t hi, uint32_t lo) {
@@ -146,61 +149,70 @@ __device__ __forceinline__ void wp_issue_sf_copies(uint32_t tmem_sf, uint32_t sf
   }
 }
 
-__device__ __forceinline__ void wp_issue_mmas(uint32_t tmem_acc, uint32_t tmem_sf, uint32_t w_lo, uint32_t x_lo,
+__device__ __forceinline__ void wp_issue_mmas(uint32_t tmem_acc, uint32_t tmem_sf, uint32_t shift, uint32_t w_lo, uint32_t x_lo,
                                               uint32_t idesc, uint32_t accumulate) {
   constexpr uint32_t hi_ab = (1024u >> 4) | (1u << 14) | (2u << 29);  // 8 rows x 128 B, 128B swizzle
 #pragma unroll
   for (uint32_t j = 0; j < 4; ++j)
-    wp_mma(tmem_acc, hi_ab, w_lo + 2 * j, x_lo + 2 * j, idesc, tmem_sf + 12 * j, tmem_sf + 12 * j + 4,
+    wp_mma(tmem_acc, hi_ab, w_lo + 2 * j, x_lo + 2 * j, idesc, tmem_sf + 12 * j, tmem_sf + 12 * j + 4 + shift,
            j == 0 ? accumulate : 1u);
 }
 
+// 16 lanes x 32 columns: register 4g + i holds columns 8g + 2t + (i & 1) of row lane/4 + 8 * (i / 2).
+__device__ __forceinline__ void wp_load_16x32(uint32_t tmem_address, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(tmem_address)
+      : "memory");
+}
+
+// erf-GELU where the table does not reach: one gate in 20000 of unit variance.
+__device__ __noinline__ float wp_gelu_small(float gate, const float* erf_table) { return gv_gelu_erf(gate, erf_table); }
+
 struct WpItem {
-  int first;     // first 128-row tile of the chunk
   int expert;
+  int first;     // first 128-row scale tile of the chunk
+  int shift;     // tensor-memory columns (of 32 rows) by which the chunk starts inside that tile: 0 or 2
+  int local;     // first row of the chunk within the expert
   int row0;      // first sorted row of the chunk
-  int valid;     // rows of the chunk, 1..256
+  int valid;     // rows of the chunk, 1..224
   int n;         // MMA N: valid rounded up to 16
   int unit_pair; // 0..5
 };
 
-struct WpPlan {
-  const int* pair_tile;
-  const int* tile_expert;
-  const int* expert_offsets;
-  const int* scale_row_offsets;
-  int pair_begin;
-  int total_items;
-  int rounds;
-};
+// Chunks of an expert: one if its rows fit an accumulator, else stretches of 192 (a multiple of 64, so that
+// a chunk's scales start at a column of its first scale tile's atom and end within the next tile's).
+__host__ __device__ __forceinline__ int wp_chunks_of(int rows) {
+  return rows <= kWpRows ? (rows > 0) : (rows + kWpChunk - 1) / kWpChunk;
+}
 
 // Items in snake order over the pairs of the grid: the unit pairs of a chunk go to neighbouring
 // clusters, which then read the same token rows from L2 at about the same time.
-__device__ __forceinline__ bool wp_item(const WpPlan& plan, int round, WpItem& item) {
+__device__ __forceinline__ bool wp_item(const WpSmem* smem, int round, WpItem& item) {
   const int slots = static_cast<int>(gridDim.x) >> 1;
   const int mine = static_cast<int>(blockIdx.x) >> 1;
   const int slot = (round & 1) ? slots - 1 - mine : mine;
   const int index = round * slots + slot;
-  if (index >= plan.total_items) return false;
   const int chunk = index / kWpItemsPerChunk;
+  if (chunk >= smem->chunks[kExperts]) return false;
   item.unit_pair = index - chunk * kWpItemsPerChunk;
-  item.first = plan.pair_tile[plan.pair_begin + chunk] >> 1;
-  item.expert = plan.tile_expert[item.first];
-  const int local0 = item.first * kTileM - plan.scale_row_offsets[item.expert];
-  item.row0 = plan.expert_offsets[item.expert] + local0;
-  const int rows_after = plan.expert_offsets[item.expert + 1] - item.row0;
-  item.valid = rows_after < 2 * kTileM ? rows_after : 2 * kTileM;
+  int expert = 0;  // the last expert with chunks[expert] <= chunk
+#pragma unroll
+  for (int step = kExperts / 2; step; step >>= 1)
+    if (smem->chunks[expert + step] <= chunk) expert += step;
+  item.expert = expert;
+  item.local = (chunk - smem->chunks[expert]) * kWpChunk;
+  item.row0 = smem->offsets[expert] + item.local;
+  item.first = (smem->scale_rows[expert] + item.local) / kTileM;
+  item.shift = (item.local & (kTileM - 1)) >> 5;
+  const int rows = smem->offsets[expert + 1] - smem->offsets[expert];
+  const int rows_after = rows - item.local;
+  item.valid = rows <= kWpRows || rows_after < kWpChunk ? rows_after : kWpChunk;
   item.n = (item.valid + 15) & ~15;
   return true;
-}
-
-__device__ __forceinline__ int wp_lower_bound(const int* __restrict__ pair_tile, int count, int tile) {
-  int lo = 0, hi = count;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if ((pair_tile[mid] >> 1) < tile) lo = mid + 1; else hi = mid;
-  }
-  return lo;
 }
 
 struct WpTokenMaps {
@@ -212,14 +224,10 @@ struct WpParams {
   uint8_t* next_codes;         // [row capacity, 352] w2 operand codes
   uint8_t* next_scales;        // scale regions of the w2 operand
   const float* next_scale_q;   // [experts] g2.input_scale_quant
-  const int* tile_expert;
   const int* expert_offsets;
   const int* scale_row_offsets;
-  const int* num_m_tiles;
-  const int* tile_first;       // optional: the launch covers tiles [tile_first, tile_first + num_m_tiles)
-  const int* pair_tile;
-  const int* num_pairs;
   int* status;
+  bool early_weights;
 };
 
 __global__ void __launch_bounds__(kWpThreads, 1)
@@ -235,81 +243,86 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kWpStages; ++s) {
-      mbar_init(&smem->full[s], 1);   // the leader's producer announces both CTAs' byte count
+      mbar_init(&smem->full[s], 2);   // the leader's two producers each announce both CTAs' byte count
       mbar_init(&smem->empty[s], 1);
     }
-    mbar_init(&smem->acc_full, 1);
-    mbar_init(&smem->acc_empty, kEpilogueThreads + kEpilogueThreads / 32);  // leader's threads + the second CTA's warps
+    for (int b = 0; b < kWpAccStages; ++b) {
+      mbar_init(&smem->acc_full[b], 1);
+      mbar_init(&smem->acc_empty[b], 2 * 4 * kWpParts);  // the epilogue warps of both CTAs
+    }
     smem->abort = 0;
-    for (int s = 0; s < 4; ++s) smem->group_left[s] = 0;
     fence_barrier_init();
     prefetch_tensor_map(&map_w);
     prefetch_tensor_map(&map_x_sf);
     prefetch_tensor_map(&map_w_sf);
   }
-  if (warp == 1) {
+  if (warp == kWpMmaWarp) {
     tmem_alloc(&smem->tmem_base, kWpTmemColumns);  // the whole tensor memory: both CTAs get address 0
     tmem_relinquish();
   }
   load_geglu_tables(&smem->tables);
   __syncthreads();
   fill_geglu_tables(&smem->tables);
-  grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   // Barriers of both CTAs exist before either CTA arrives on the other's.
   cluster_sync_all();
   const uint32_t tmem_base = smem->tmem_base;
-  grid_dependency_wait();
+  // The plan and the weights may come from before the previous kernel: see W13PairOperands::early_weights.
+  if (!p.early_weights) grid_dependency_wait();
 
-  WpPlan plan;
-  plan.pair_tile = p.pair_tile;
-  plan.tile_expert = p.tile_expert;
-  plan.expert_offsets = p.expert_offsets;
-  plan.scale_row_offsets = p.scale_row_offsets;
-  plan.pair_begin = 0;
-  int pair_count = p.num_pairs[0];
-  if (p.tile_first) {
-    const int first = p.tile_first[0];
-    plan.pair_begin = wp_lower_bound(p.pair_tile, pair_count, first);
-    pair_count = wp_lower_bound(p.pair_tile, pair_count, first + p.num_m_tiles[0]) - plan.pair_begin;
+  if (warp < 4) {
+    // thread = expert: chunks before it
+    const int e = threadIdx.x;
+    const int row = p.expert_offsets[e], next_row = p.expert_offsets[e + 1];
+    const int own = wp_chunks_of(next_row - row);
+    int inclusive = own;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
+      if (lane >= offset) inclusive += other;
+    }
+    if (lane == 31) smem->scan[warp] = inclusive;
+    smem->offsets[e] = row;
+    smem->scale_rows[e] = p.scale_row_offsets[e];
+    if (e == kExperts - 1) smem->offsets[kExperts] = next_row;
+    named_barrier(5, 128);
+    for (int w = 0; w < warp; ++w) inclusive += smem->scan[w];
+    smem->chunks[e] = inclusive - own;
+    if (e == kExperts - 1) smem->chunks[kExperts] = inclusive;
   }
-  plan.total_items = pair_count * kWpItemsPerChunk;
+  __syncthreads();
+  if (warp != kWpWeightWarp) {
+    grid_dependency_wait();
+    grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
+  }
+  const int total_items = smem->chunks[kExperts] * kWpItemsPerChunk;
   const int slots = static_cast<int>(gridDim.x) >> 1;
-  plan.rounds = (plan.total_items + slots - 1) / slots;
+  const int rounds = (total_items + slots - 1) / slots;
   constexpr int k_blocks = kHidden / 2 / kTileKBytes;   // 11
 
-  if (warp == 0) {
-    // ---------------- TMA producer (one warp in each CTA) ----------------
+  if (warp == kWpTokenWarp || warp == kWpWeightWarp) {
+    // ---------------- TMA producers (one warp for each side in each CTA) ----------------
+    const bool weight_side = warp == kWpWeightWarp;
     int stage = 0;
     uint32_t phase = 0;
     int issued = 0;
     bool ok = true;
-    for (int round = 0; ok && round < plan.rounds; ++round) {
+    for (int round = 0; ok && round < rounds; ++round) {
       WpItem item;
-      if (!wp_item(plan, round, item)) continue;
+      if (!wp_item(smem, round, item)) continue;
       const int unit = 2 * item.unit_pair + static_cast<int>(rank);
       const bool unit_exists = unit < kWpUnits;
       const int half = item.n >> 1;                            // token rows per CTA, a multiple of 8
       const int token_row = item.row0 + static_cast<int>(rank) * half;
       const bool second_exists = 2 * item.unit_pair + 1 < kWpUnits;
-      // per K block and CTA: the weight scales (2 KiB), the scales of two 128-row blocks of tokens
-      // (4 KiB; the second block is fetched, and ignored, also when the chunk has one), the token rows,
-      // and the unit's weight rows
-      const uint32_t both_bytes = 2 * (3 * kSfStageBytes + static_cast<uint32_t>(half) * kTileKBytes) + kWpTileBytes +
-                                  (second_exists ? kWpTileBytes : 0);
+      // Per K block and CTA: the unit's weight rows and their scales (2 KiB), or the token rows and the scales of two
+      // 128-row blocks of tokens (4 KiB; the second block is fetched, and ignored, also when the chunk has one).
+      const uint32_t both_bytes = weight_side ? 2 * kSfStageBytes + kWpTileBytes + (second_exists ? kWpTileBytes : 0)
+                                              : 2 * (2 * kSfStageBytes + static_cast<uint32_t>(half) * kTileKBytes);
       const CUtensorMap* token_map = &map_x.rows[(half >> 3) - 1];
       const int w_sf_row = ((item.expert * kWpUnitSlots + unit) * k_blocks) * 4;
-      // While this item streams, the bytes of this CTA's next item are asked into L2, K block by K
-      // block: the ring holds at most five stages, too few to cover the latency of a load that
-      // misses L2 (the weights are read from HBM about once per chunk).
-      WpItem next;
-      const bool has_next = round + 1 < plan.rounds && wp_item(plan, round + 1, next);
-      const int next_unit = has_next ? 2 * next.unit_pair + static_cast<int>(rank) : kWpUnits;
-      const int next_half = has_next ? next.n >> 1 : 8;
-      const CUtensorMap* next_token_map = &map_x.rows[(next_half >> 3) - 1];
-      const int next_token_row = has_next ? next.row0 + static_cast<int>(rank) * next_half : 0;
       for (int kb = 0; kb < k_blocks; ++kb) {
         ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status));
         if (!ok) break;
@@ -318,13 +331,12 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           const uint32_t bar = is_leader ? smem_u32(&smem->full[stage])
                                          : cluster_map_shared(smem_u32(&smem->full[stage]), 0);
           if (is_leader) mbar_arrive_expect_tx(&smem->full[stage], both_bytes);
-          if (unit_exists) wp_load_3d(smem->w[stage], &map_w, bar, x, unit * 64, item.expert * 2);
-          wp_load(smem->x[stage], token_map, bar, x, token_row);
-          wp_load(smem->sfw[stage], &map_w_sf, bar, 0, w_sf_row + 4 * kb);
-          wp_load_3d(smem->sfx[stage], &map_x_sf, bar, 0, 4 * kb, item.first);
-          if (has_next) {
-            if (next_unit < kWpUnits) wp_prefetch_3d(&map_w, x, next_unit * 64, next.expert * 2);
-            wp_prefetch_2d(next_token_map, x, next_token_row);
+          if (weight_side) {
+            if (unit_exists) wp_load_weights(smem->w[stage], &map_w, bar, x, item.expert * (kW13Out / 16) + unit * 4);
+            wp_load(smem->sfw[stage], &map_w_sf, bar, 0, w_sf_row + 4 * kb);
+          } else {
+            wp_load(smem->x[stage], token_map, bar, x, token_row);
+            wp_load_3d(smem->sfx[stage], &map_x_sf, bar, 0, 4 * kb, item.first);
           }
         }
         __syncwarp();
@@ -349,26 +361,27 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
         mbar_wait_bounded(&smem->full[s], ph, 40000000ll);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == kWpMmaWarp) {
     if (is_leader) {
       // ---------------- leader: scale copies and MMAs for both CTAs ----------------
       int stage = 0;
       uint32_t phase = 0;
+      int acc = 0;
       uint32_t acc_phase = 0;
       const uint32_t w_lo0 = (smem_u32(smem->w[0]) & 0x3ffffu) >> 4;
       const uint32_t x_lo0 = (smem_u32(smem->x[0]) & 0x3ffffu) >> 4;
       const uint32_t sfw_lo0 = (smem_u32(smem->sfw[0]) & 0x3ffffu) >> 4;
       const uint32_t sfx_lo0 = (smem_u32(smem->sfx[0]) & 0x3ffffu) >> 4;
       const bool leader_lane = elect_one();
-      for (int round = 0; round < plan.rounds; ++round) {
+      for (int round = 0; round < rounds; ++round) {
         WpItem item;
-        if (!wp_item(plan, round, item)) continue;
-        const bool two_blocks = item.n > kTileM;
+        if (!wp_item(smem, round, item)) continue;
+        const bool two_blocks = item.shift * 32 + item.n > kTileM;
         // E2M1 x E2M1, both K-major, UE4M3 scales; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
         const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(item.n >> 3) << 17) |
                                (static_cast<uint32_t>(256 >> 4) << 24);
-        if (!__all_sync(0xffffffffu, wait_or_abort<false>(&smem->acc_empty, acc_phase ^ 1u, smem, p.status))) break;
-        acc_phase ^= 1u;
+        if (!__all_sync(0xffffffffu, wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status))) break;
+        const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc) * kWpRows;
         bool ok = true;
         tc_fence_after_sync();
         for (int kb = 0; kb < k_blocks; ++kb) {
@@ -377,16 +390,17 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           tc_fence_after_sync();
           if (leader_lane) {
             const uint32_t w_lo = w_lo0 + static_cast<uint32_t>(stage) * (kWpTileBytes >> 4);
-            const uint32_t x_lo = x_lo0 + static_cast<uint32_t>(stage) * (kWpTileBytes >> 4);
+            const uint32_t x_lo = x_lo0 + static_cast<uint32_t>(stage) * (kWpTokenBytes >> 4);
             const uint32_t sfw_lo = sfw_lo0 + static_cast<uint32_t>(stage) * (kSfStageBytes >> 4);
             const uint32_t sfx_lo = sfx_lo0 + static_cast<uint32_t>(stage) * (2 * kSfStageBytes >> 4);
-            const uint32_t tmem_sf = tmem_base + kWpSfColumn + kWpSfColumnsPerStage * stage;
-            // copies and MMAs of one thread execute in order in the tensor pipe
+            const uint32_t tmem_sf = tmem_base + kWpSfColumn;
+            // copies and MMAs of one thread execute in order in the tensor pipe, so one set of scale
+            // columns serves every K block
             if (two_blocks) wp_issue_sf_copies<true>(tmem_sf, sfw_lo, sfx_lo);
             else wp_issue_sf_copies<false>(tmem_sf, sfw_lo, sfx_lo);
-            wp_issue_mmas(tmem_base, tmem_sf, w_lo, x_lo, idesc, kb != 0 ? 1u : 0u);
+            wp_issue_mmas(tmem_acc, tmem_sf, item.shift, w_lo, x_lo, idesc, kb != 0 ? 1u : 0u);
             wp_commit_both(&smem->empty[stage]);   // both CTAs may refill the stage
-            if (kb + 1 == k_blocks) wp_commit_both(&smem->acc_full);
+            if (kb + 1 == k_blocks) wp_commit_both(&smem->acc_full[acc]);
           }
           if (++stage == kWpStages) {
             stage = 0;
@@ -394,102 +408,142 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           }
         }
         if (!ok) break;
+        if (++acc == kWpAccStages) {
+          acc = 0;
+          acc_phase ^= 1u;
+        }
       }
     }
   } else {
-    // ---------------- epilogue: 16 warps in each CTA ----------------
-    // A warp may touch only the tensor-memory lanes 32*(warp%4)..+31 (here: 32 of the CTA's 128
-    // weight rows); the four warps with the same `group` take the same 32 tokens of a pass and
-    // share one staging tile.
-    const int quarter = warp & 3;
-    const int group = (warp - 2) >> 2;  // 0..3
+    // ---------------- epilogue: eight warps in each CTA ----------------
+    // A warp may touch only the tensor-memory lanes 32*(warp%4)..+31: one block of 16 intermediate columns,
+    // 16b + 2i + o being the up row of lane 16o + i and the gate row of lane 16o + 8 + i.  In the 16x256b layout a
+    // thread holds rows lane/4 and lane/4 + 8, so up and gate of columns 2i and 2i + 1 (i = lane / 4), for eight of
+    // 32 tokens: GeGLU needs no exchange, a block's maximum is one over the eight lanes of equal lane % 4, and the
+    // thread's two codes are byte i of the block's eight.  Three steps of exchange leave lane i with the maximum,
+    // and then the code bytes, of the i-th of its eight tokens.
+    const int block = warp & 3;
+    const int part = (warp - kWpEpilogueWarp) >> 2;
+    const bool a = lane & 16, b = lane & 8, c = lane & 4;
+    const uint32_t keep_b = b ? 0x7632u : 0x5410u, send_b = b ? 0x5410u : 0x7632u;
+    const uint32_t keep_c = c ? 0x7531u : 0x6420u, send_c = c ? 0x6420u : 0x7531u;
+    const uint32_t low_word = b ? 0x4062u : 0x6240u, high_word = b ? 0x5173u : 0x7351u;
+    const int own_token = 8 * (lane >> 3) + 2 * (lane & 3) + ((lane >> 2) & 1);  // of the 32: the (lane / 4)-th of the thread's
+    constexpr int groups = kInter / 16;
+    int acc = 0;
     uint32_t acc_phase = 0;
-    uint8_t* staging = smem->staging[group];
-    const int in_group = quarter * 32 + lane;       // 0..127: this thread's weight row, later its (token, block)
-    for (int round = 0; round < plan.rounds; ++round) {
+    for (int round = 0; round < rounds; ++round) {
       WpItem item;
-      if (!wp_item(plan, round, item)) continue;
+      if (!wp_item(smem, round, item)) continue;
       const int unit = 2 * item.unit_pair + static_cast<int>(rank);
-      const bool unit_exists = unit < kWpUnits;
+      const int steps = unit < kWpUnits ? (item.valid + 31) >> 5 : 0;  // of 32 tokens, dealt to the four warps of a block
       const float alpha = p.alpha[item.expert];
       const float multiplier = p.next_scale_q[item.expert];
-      const bool acc_ready = wait_or_abort<true>(&smem->acc_full, acc_phase, smem, p.status);
-      acc_phase ^= 1u;
-      if (!acc_ready) smem->group_left[group] = 1;
-      named_barrier(1 + group, 4 * 32);
-      if (*reinterpret_cast<volatile int*>(&smem->group_left[group])) break;
+      if (!__all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, p.status))) break;
       tc_fence_after_sync();
-      const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-      // pass 0: tokens [32 group, +32); pass 1: tokens [128 + 32 group, +32)
-      const bool has0 = unit_exists && 32 * group < item.valid;
-      const bool has1 = unit_exists && 128 + 32 * group < item.valid;
-      uint32_t packed[2][16];
-      {
-        uint32_t r[32];
-        if (has0) {
-          tmem_load_32x32(tmem_row + 32 * group, r);
+      const uint32_t tmem_rows = tmem_base + (static_cast<uint32_t>(block * 32) << 16) + static_cast<uint32_t>(acc) * kWpRows;
+      uint8_t* const scales = p.next_scales + static_cast<size_t>(smem->scale_rows[item.expert]) * groups;
+      int step = (part + round) % kWpParts;
+      bool released = false;
+#pragma unroll 1
+      do {
+        uint32_t even[16], odd[16];
+        if (step < steps) {
+          wp_load_16x32(tmem_rows + 32 * step, even);
+          wp_load_16x32(tmem_rows + (16u << 16) + 32 * step, odd);
           tmem_load_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            packed[0][i] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(r[2 * i])), __fmul_rn(alpha, __uint_as_float(r[2 * i + 1])));
         }
-        if (has1) {
-          tmem_load_32x32(tmem_row + 128 + 32 * group, r);
-          tmem_load_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            packed[1][i] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(r[2 * i])), __fmul_rn(alpha, __uint_as_float(r[2 * i + 1])));
+        if (step + kWpParts >= steps) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            if (is_leader) mbar_arrive(&smem->acc_empty[acc]);
+            else wp_arrive_remote(&smem->acc_empty[acc], 0);
+          }
+          released = true;
         }
-      }
-      tc_fence_before_sync();
-      if (is_leader) {
-        mbar_arrive(&smem->acc_empty);
-      } else {
+        if (step >= steps) break;
+        const int token = 32 * step + own_token;
+        // bf16(alpha * acc), columns 2i and 2i + 1 of token k = 2g + s (8g + 2 (lane % 4) + s of the 32)
+        uint32_t up[8], gate[8];
+        int smallest = 0;  // its sign bit: some magnitude lies below the table
+        float v0[8], v1[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = 4 * (k >> 1) + (k & 1);
+          up[k] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(even[r])), __fmul_rn(alpha, __uint_as_float(odd[r])));
+          gate[k] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(even[r + 2])), __fmul_rn(alpha, __uint_as_float(odd[r + 2])));
+          const int index0 = erf_index(gate[k] & 0x7fffu), index1 = erf_index((gate[k] >> 16) & 0x7fffu);
+          smallest |= index0 | index1;
+          v0[k] = gelu_from_erf(__uint_as_float(gate[k] << 16), smem->tables.erf_of[max(index0, 0)]);
+          v1[k] = gelu_from_erf(__uint_as_float(gate[k] & 0xffff0000u), smem->tables.erf_of[max(index1, 0)]);
+        }
+        if (smallest < 0) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            if (erf_index(gate[k] & 0x7fffu) < 0) v0[k] = wp_gelu_small(__uint_as_float(gate[k] << 16), smem->tables.erf_table);
+            if (erf_index((gate[k] >> 16) & 0x7fffu) < 0)
+              v1[k] = wp_gelu_small(__uint_as_float(gate[k] & 0xffff0000u), smem->tables.erf_table);
+          }
+        }
         __syncwarp();
-        if (lane == 0) wp_arrive_remote(&smem->acc_empty, 0);
-      }
+        float most[8];
 #pragma unroll
-      for (int pass = 0; pass < 2; ++pass) {
-        if (!(pass == 0 ? has0 : has1)) continue;
-        // transposed write: token i of the pass, this thread's weight row; the 16-byte chunk c of a
-        // token lives at chunk position c ^ (token & 7)
-        const int chunk = in_group >> 3;
-        const int within = (in_group & 7) * 2;
+        for (int k = 0; k < 8; ++k) {
+          v0[k] = __fmul_rn(v0[k], __uint_as_float(up[k] << 16));
+          v1[k] = __fmul_rn(v1[k], __uint_as_float(up[k] & 0xffff0000u));
+          most[k] = fmaxf(fabsf(v0[k]), fabsf(v1[k]));
+        }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const uint32_t pair = packed[pass][i >> 1];
-          const uint16_t value = static_cast<uint16_t>((i & 1) ? pair >> 16 : pair & 0xffffu);
-          *reinterpret_cast<uint16_t*>(staging + i * kWpStagePitch + ((chunk ^ (i & 7)) << 4) + within) = value;
+        for (int k = 0; k < 4; ++k) {
+          const float received = __shfl_xor_sync(0xffffffffu, a ? most[k] : most[k + 4], 16);
+          most[k] = fmaxf(a ? most[k + 4] : most[k], received);
         }
-        named_barrier(1 + group, 4 * 32);
-        // one thread per (token, 16 columns): lanes [16 b, +16) are up, [64 + 16 b, +16) gate
-        const int t = in_group >> 2;
-        const int b = in_group & 3;
-        const uint8_t* row = staging + t * kWpStagePitch;
-        const int swz = t & 7;
-        const uint4 u0 = *reinterpret_cast<const uint4*>(row + (((2 * b) ^ swz) << 4));
-        const uint4 u1 = *reinterpret_cast<const uint4*>(row + (((2 * b + 1) ^ swz) << 4));
-        const uint4 g0 = *reinterpret_cast<const uint4*>(row + (((8 + 2 * b) ^ swz) << 4));
-        const uint4 g1 = *reinterpret_cast<const uint4*>(row + (((8 + 2 * b + 1) ^ swz) << 4));
-        uint2 codes;
-        const uint32_t ups[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-        const uint32_t gates[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        uint32_t scale = geglu_block_of_bf16(ups, gates, multiplier, &smem->tables, codes.x, codes.y);
-        const int token = 128 * pass + 32 * group + t;
-        const bool valid = token < item.valid;
-        if (valid)
-          *reinterpret_cast<uint2*>(p.next_codes + static_cast<size_t>(item.row0 + token) * (kInter / 2) + unit * 32 + b * 8) = codes;
-        // the four scale bytes of a token's unit are one aligned word of the w2 operand's scale atom
-        scale <<= 8 * b;
-        scale |= __shfl_xor_sync(0xffffffffu, scale, 1);
-        scale |= __shfl_xor_sync(0xffffffffu, scale, 2);
-        if (valid && b == 0) {
-          constexpr int groups = kInter / 16;
-          const int tile = item.first + (token >> 7);
-          *reinterpret_cast<uint32_t*>(p.next_scales + static_cast<size_t>(tile) * kTileM * groups +
-                                       sf_offset(token & 127, 4 * unit, groups)) = scale;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float received = __shfl_xor_sync(0xffffffffu, b ? most[k] : most[k + 2], 8);
+          most[k] = fmaxf(b ? most[k + 2] : most[k], received);
         }
-        named_barrier(1 + group, 4 * 32);  // the staging tile is rewritten by the next pass or item
+        const float maximum = fmaxf(c ? most[1] : most[0], __shfl_xor_sync(0xffffffffu, c ? most[0] : most[1], 4));
+        const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
+        const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, smem->tables.reciprocals)
+                                                                 : scale_inverse_divided(multiplier, scale);
+        uint32_t words[2];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float inverses[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) inverses[k] = __shfl_sync(0xffffffffu, inverse, (lane & 3) | (16 * half + 4 * k));
+          const float *x0 = v0 + 4 * half, *x1 = v1 + 4 * half;
+          asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+              "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+              "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+              "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+              "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+              "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+              : "=r"(words[half])
+              : "f"(__fmul_rn(x0[0], inverses[0])), "f"(__fmul_rn(x1[0], inverses[0])), "f"(__fmul_rn(x0[1], inverses[1])),
+                "f"(__fmul_rn(x1[1], inverses[1])), "f"(__fmul_rn(x0[2], inverses[2])), "f"(__fmul_rn(x1[2], inverses[2])),
+                "f"(__fmul_rn(x0[3], inverses[3])), "f"(__fmul_rn(x1[3], inverses[3])));
+        }
+        // 8 x 8 bytes over the eight lanes, transposed: bits 2, 1 and 0 of the lane number in turn
+        const uint32_t received_a = __shfl_xor_sync(0xffffffffu, a ? words[0] : words[1], 16);
+        const uint32_t lo = a ? received_a : words[0], hi = a ? words[1] : received_a;
+        const uint32_t received_b = __shfl_xor_sync(0xffffffffu, __byte_perm(lo, hi, send_b), 8);
+        const uint32_t kept_b = __byte_perm(lo, hi, keep_b);
+        const uint32_t received_c = __shfl_xor_sync(0xffffffffu, __byte_perm(kept_b, received_b, send_c), 4);
+        const uint32_t kept_c = __byte_perm(kept_b, received_b, keep_c);
+        const uint32_t first = c ? received_c : kept_c, second = c ? kept_c : received_c;
+        if (token < item.valid) {
+          *reinterpret_cast<uint2*>(p.next_codes + static_cast<size_t>(item.row0 + token) * (kInter / 2) + unit * 32 + block * 8) =
+              make_uint2(__byte_perm(first, second, low_word), __byte_perm(first, second, high_word));
+          scales[sf_offset(item.local + token, 4 * unit + block, groups)] = static_cast<uint8_t>(scale);
+        }
+        step += kWpParts;
+      } while (!released);
+      if (++acc == kWpAccStages) {
+        acc = 0;
+        acc_phase ^= 1u;
       }
     }
   }
@@ -497,17 +551,18 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
   tc_fence_before_sync();
   // Both CTAs stay until neither can still receive a remote arrive, a copy or a multicast commit.
   cluster_sync_all();
-  if (warp == 1) {
+  if (warp == kWpMmaWarp) {
     tc_fence_after_sync();
     __syncwarp();
     tmem_dealloc(tmem_base, kWpTmemColumns);
   }
 }
 
-// Re-tiles the w13 block scales for this kernel: unit u of an expert (intermediate columns
-// [64u, 64u+64)) is 128 MMA rows, up rows on 0..63 and gate rows on 64..127.  Per expert, unit
-// (twelve slots, the last all zero) and K block of 256 the copy holds [MMA 0..3][512-byte atom],
-// the atom being (n%32)*16 + (n/32)*4 + k over the 128 rows n.  One thread per byte.
+// Re-tiles the w13 block scales by unit of 64 intermediate columns, twelve slots an expert of which the last is
+// all zero: [expert][unit][K block of 256][MMA 0..3][512-byte atom], the atom being (n%32)*16 + (n/32)*4 + k over
+// the unit's 128 MMA rows n.  kFragments: in this file's row order; else the 64 up rows, then the 64 gate rows.
+// One thread per byte.
+template <bool kFragments>
 __global__ void retile_w13_unit_scales_kernel(const uint8_t* __restrict__ sidecar, uint8_t* __restrict__ tiled,
                                               int experts) {
   constexpr int groups = kHidden / 16;          // 176
@@ -527,7 +582,9 @@ __global__ void retile_w13_unit_scales_kernel(const uint8_t* __restrict__ sideca
   const int k = byte & 3;
   uint8_t value = 0;
   if (unit < kWpUnits) {
-    const int source_row = n < 64 ? unit * 64 + n : kInter + unit * 64 + (n - 64);
+    const bool gate = kFragments ? (n & 8) != 0 : n >= 64;
+    const int column = kFragments ? 16 * (n >> 5) + 2 * (n & 7) + ((n >> 4) & 1) : n & 63;
+    const int source_row = (gate ? kInter : 0) + unit * 64 + column;
     value = sidecar[static_cast<size_t>(expert) * kW13Out * groups +
                     sf_offset(source_row, (k_block * 4 + mma) * 4 + k, groups)];
   }
@@ -540,10 +597,11 @@ size_t w13_unit_scale_bytes(int experts) {
   return static_cast<size_t>(experts) * kWpUnitSlots * (kHidden / 256) * 4 * kSfAtomBytes;
 }
 
-void launch_retile_w13_unit_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, cudaStream_t stream) {
-  const size_t total = w13_unit_scale_bytes(experts);
-  retile_w13_unit_scales_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(sidecar_scales, tiled,
-                                                                                                 experts);
+void launch_retile_w13_unit_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, bool fragments,
+                                   cudaStream_t stream) {
+  const unsigned blocks = static_cast<unsigned>((w13_unit_scale_bytes(experts) + 255) / 256);
+  if (fragments) retile_w13_unit_scales_kernel<true><<<blocks, 256, 0, stream>>>(sidecar_scales, tiled, experts);
+  else retile_w13_unit_scales_kernel<false><<<blocks, 256, 0, stream>>>(sidecar_scales, tiled, experts);
 }
 
 int prepare_w13_pairs() {
@@ -557,14 +615,10 @@ void launch_w13_pairs(const W13PairOperands& op, const RoutePlan& plan, int sm_c
   p.next_codes = op.next_codes;
   p.next_scales = op.next_scales;
   p.next_scale_q = op.next_scale_q;
-  p.tile_expert = plan.tile_expert;
   p.expert_offsets = plan.expert_offsets;
   p.scale_row_offsets = plan.scale_row_offsets;
-  p.num_m_tiles = plan.num_m_tiles;
-  p.tile_first = plan.tile_first;
-  p.pair_tile = plan.pair_tile;
-  p.num_pairs = plan.num_pairs;
   p.status = plan.status;
+  p.early_weights = op.early_weights;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(sm_count & ~1));
   config.blockDim = dim3(kWpThreads);

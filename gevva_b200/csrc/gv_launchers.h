@@ -147,11 +147,10 @@ void launch_grouped_gemm_pairs(const GemmOperands& op, const RoutePlan& plan, in
 int prepare_grouped_gemm_pairs();
 
 // Fused w13 + GeGLU + requantise run by CTA pairs with the weights on the MMA's M side and up to
-// 256 rows of one expert on its N side (grouped_gemm_w13_pair.cu); needs the plan's tile-pair list.
+// 208 rows of one expert on its N side (grouped_gemm_w13_pair.cu).
 struct W13PairOperands {
   CUtensorMap map_x[16];  // activation codes [row capacity, 1408] bytes through boxes of 8, 16, ... 128 rows x 128 B
-  CUtensorMap map_w;      // w13 codes as [experts * 2 halves, 704 rows, 1408] bytes, box 2 x 64 rows x 128 B: the
-                          // up rows and the gate rows of one unit in one copy
+  CUtensorMap map_w;      // w13 codes in the row order of its MMAs, a unit of 64 columns (up and gate rows) a copy
   CUtensorMap map_x_sf;   // activation scale regions as [128-row blocks, 44 atoms, 512 B], box 2 blocks x 4 atoms
   CUtensorMap map_w_sf;   // unit-tiled weight scales (launch_retile_w13_unit_scales), box of four atoms
   const float* alpha;           // [experts]
@@ -159,9 +158,11 @@ struct W13PairOperands {
   uint8_t* next_scales;         // scale regions of the w2 operand
   const float* next_scale_q;    // [experts]
   bool serial_launch;
+  bool early_weights;           // as in GemmOperands; the route plan too comes from before the previous kernel
 };
 size_t w13_unit_scale_bytes(int experts);
-void launch_retile_w13_unit_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, cudaStream_t stream);
+void launch_retile_w13_unit_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, bool fragments,
+                                   cudaStream_t stream);
 void launch_w13_pairs(const W13PairOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
 int prepare_w13_pairs();
 

@@ -116,6 +116,22 @@ bool make_w13_unit_map(CUtensorMap* map, const void* base, uint64_t experts) {
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// w13 codes [experts, up and gate halves of 704 rows, 1408 bytes] in the row order of grouped_gemm_w13_pair.cu:
+// row 32b + 16o + 8h + i of a 128-row box is row 16b + 2i + o of half h, b counting blocks of 16 rows.
+bool make_w13_fragment_map(CUtensorMap* map, const void* base, uint64_t experts) {
+  constexpr cuuint64_t row = kHidden / 2;
+  // the last dimension starts in an up half; its extent keeps the gate half, 704 rows on, inside the matrix
+  const cuuint64_t dims[5] = {row, 8, 2, 2, (experts * kW13Out - kInter) / 16};
+  const cuuint64_t strides[4] = {2 * row, kInter * row, row, 16 * row};
+  const cuuint32_t box[5] = {static_cast<cuuint32_t>(kTileKBytes), 8, 2, 2, 4};
+  const cuuint32_t element_strides[5] = {1, 1, 1, 1, 1};
+  EncodeTiledFn fn = encode_tiled();
+  if (!fn) return false;
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<void*>(base), dims, strides, box, element_strides,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts) {
   constexpr cuuint64_t row = kInter / 2;
   const cuuint64_t dims[5] = {row, 2, 4, 8, experts * kHidden / 64};
@@ -251,6 +267,7 @@ struct gevva_moe {
   uint8_t* w13_sf_tiled = nullptr;  // runner-owned re-tiling of weights.w13_sf for the CTA-pair tile kernels
   gv::W13PairOperands w13_pairs{};  // the CTA-pair form of the fused w13 stage
   uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf by unit of 64 columns
+  uint8_t* w13_sf_fragments = nullptr;  // the same in the row order of grouped_gemm_w13_pair.cu
   uint8_t* w2_sf_down = nullptr;    // runner-owned re-tiling of weights.w2_sf in the column order of grouped_gemm_down.cu
   gv::StreamOperands stream_experts{};  // few rows an expert: both GEMMs in one launch, weights on the MMA's M side
   bool w13_pair_form = false;       // GEVVA_MOE_OPTION_W13_PAIRS, or GEVVA_MOE_W13_PAIRS=1 for a whole process
@@ -323,6 +340,10 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   }
   const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
   const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
+  // Weights on the MMA's M side, by CTA pairs: faster than (2048 tokens on) or as fast as the one-CTA tile kernel
+  // wherever a batch does not stream (figures in grouped_gemm_w13_pair.cu).
+  const bool w13_by_pairs = !use_pairs && sm_count >= 2 &&
+                            (tokens > kStreamTokens || (runner->w13_pair_form && tokens > gv::kFusedSortQuantizeMaxTokens));
   if ((stages & gemms) == gemms && streams) {
     StageRange range(runner->nvtx, "gevva_moe.w13+geglu+w2");
     gv::launch_stream_experts(runner->stream_experts, s->plan, sm_count, stream);
@@ -331,9 +352,10 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   if ((stages & both) == both && !(stages & GEVVA_MOE_STAGE_UNFUSED)) {
     // production path: GeGLU + requantise inside the w13 epilogue, no bf16 w13 output
     StageRange range(runner->nvtx, "gevva_moe.w13+geglu");
-    if (runner->w13_pair_form && tokens > gv::kFusedSortQuantizeMaxTokens && s->plan.pair_tile &&
-        sm_count >= 2) {
-      gv::launch_w13_pairs(runner->w13_pairs, s->plan, sm_count, stream);
+    if (w13_by_pairs) {
+      gv::W13PairOperands w13 = runner->w13_pairs;
+      w13.early_weights = (stages & front) == front;
+      gv::launch_w13_pairs(w13, s->plan, sm_count, stream);
     } else {
       gv::GemmOperands w13 = runner->w13_fused;
       w13.use_pairs = use_pairs;
@@ -347,8 +369,8 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
       gv::launch_geglu_quantize(s->w13_out, runner->weights.in_scale_q2, s->plan, routes,
                                 s->inter_codes, s->inter_sf, stream);
   }
-  // the fused one-CTA w13 launch of this call is w2's predecessor, and w2 the reduce's
-  const bool behind_w13 = (stages & both) == both && !(stages & GEVVA_MOE_STAGE_UNFUSED) && !use_pairs && !runner->w13_pair_form;
+  // the fused w13 launch of this call is w2's predecessor, and w2 the reduce's
+  const bool behind_w13 = (stages & both) == both && !(stages & GEVVA_MOE_STAGE_UNFUSED) && !use_pairs;
   const bool behind_w2 = (stages & GEVVA_MOE_STAGE_W2) && !use_pairs && behind_w13;
   if (stages & GEVVA_MOE_STAGE_W2) {
     StageRange range(runner->nvtx, "gevva_moe.w2");
@@ -442,7 +464,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   {
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_units), gv::w13_unit_scale_bytes(kExperts));
     if (e == cudaSuccess) {
-      gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_units, kExperts, nullptr);
+      gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_units, kExperts, false, nullptr);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&m->w2_sf_down), gv::retiled_w2_scale_bytes(kExperts));
@@ -499,8 +521,14 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   }
   const char* w13_pairs_env = std::getenv("GEVVA_MOE_W13_PAIRS");
   m->w13_pair_form = (options && (options->flags & GEVVA_MOE_OPTION_W13_PAIRS)) || (w13_pairs_env && w13_pairs_env[0] == '1');
-  if (m->w13_pair_form) {
-    const cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
+  {
+    cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
+    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_fragments), gv::w13_unit_scale_bytes(kExperts));
+    if (e == cudaSuccess) {
+      gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_fragments, kExperts, true, nullptr);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
       gevva_moe_destroy(m);
       return cuda_failure(e, "w13 pair form");
@@ -509,9 +537,9 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
     ok = true;
     for (int i = 0; i < 16; ++i)
       ok = ok && make_operand_map(&wp.map_x[i], s->input_codes, rows, kHidden / 2, 8 * (i + 1));
-    ok = ok && make_w13_unit_map(&wp.map_w, weights->w13, kExperts) &&
+    ok = ok && make_w13_fragment_map(&wp.map_w, weights->w13, kExperts) &&
          make_block_scale_map(&wp.map_x_sf, s->input_sf, s->input_sf_bytes, kHidden / 64) &&
-         make_scale_map(&wp.map_w_sf, m->w13_sf_units, gv::w13_unit_scale_bytes(kExperts), 4);
+         make_scale_map(&wp.map_w_sf, m->w13_sf_fragments, gv::w13_unit_scale_bytes(kExperts), 4);
     if (!ok) {
       gevva_moe_destroy(m);
       std::snprintf(g_error_text, sizeof(g_error_text), "cuTensorMapEncodeTiled failed (w13 pair maps)");
@@ -554,6 +582,7 @@ void gevva_moe_destroy(gevva_moe* runner) {
   if (runner->scratch && --runner->scratch->references == 0) free_scratch(runner->scratch);
   cudaFree(runner->w13_sf_tiled);
   cudaFree(runner->w13_sf_units);
+  cudaFree(runner->w13_sf_fragments);
   cudaFree(runner->w2_sf_down);
   delete runner;
 }

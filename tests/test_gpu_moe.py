@@ -532,13 +532,14 @@ def test_cta_pair_gemms_equal_the_single_cta_gemms(gm, weights, cuda_device, tok
     assert results[0][0].float().abs().max() > 0
 
 
-@pytest.mark.parametrize("tokens", [641, 1000])
-def test_w2_of_large_batches_at_row_tile_edges(gm, weights, cuda_device, tokens):
-    """The w2 kernel of batches above 640 tokens, whose items, units of items and rows end raggedly,
-    against the CTA-pair kernel: the same routed rows with experts of 0, 1, 7..9, 127..129, 255..257 and
-    `tokens` rows, with every stage in one call and each in a call of its own."""
+@pytest.mark.parametrize("tokens,edges", [(641, [1, 7, 8, 9, 127, 128, 129, 255, 256, 257]),
+                                          (1000, [15, 16, 17, 33, 191, 192, 193, 208, 209, 385])])
+def test_large_batches_at_tile_and_chunk_edges(gm, weights, cuda_device, tokens, edges):
+    """The w13 and w2 kernels of batches above 640 tokens, whose chunks of up to 208 rows, 128-row tiles, items
+    and units of items end raggedly, against the CTA-pair kernels that share weight tiles: the same w2 operand
+    and routed rows, with every stage in one call and each in a call of its own."""
     from gevva_b200 import runtime as rt
-    edges = [tokens, 1, 7, 8, 9, 127, 128, 129, 255, 256, 257]
+    edges = [tokens] + edges
     rng = np.random.default_rng(tokens)
     ids = np.empty((tokens, TOP_K), dtype=np.int32)
     mine = [[] for _ in range(tokens)]  # with these seeds no token has more than six of the edge experts
@@ -561,7 +562,8 @@ def test_w2_of_large_batches_at_row_tile_edges(gm, weights, cuda_device, tokens)
         else:
             runner.launch_batch(x, dev_ids, rw, out, tokens)
         runner.check()
-        results.append((out, runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].clone()))
+        results.append((out, runner.buffer(rt.BUF_INTER_CODES)[: tokens * TOP_K * INTER // 2].clone(),
+                        runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].clone()))
     for other in results[1:]:
         for a, b in zip(results[0], other):
             assert torch.equal(a, b)
