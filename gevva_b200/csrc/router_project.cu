@@ -6,7 +6,7 @@
 // route_128_top8_kernel<<<tokens,128>>>).  Here both are one kernel and the logits never
 // reach HBM: tokens sit on MMA-M (128 per tile), the 128 experts on MMA-N, K = 2816.
 //
-// A tile's K range is split over a cluster of four CTAs (two, or one, for batches whose tiles
+// A tile (of 64 tokens in batches of up to 2048) has its K range split over a cluster of four CTAs (two, or one, for batches whose tiles
 // would otherwise not fit one wave of SMs; eight for batches of at most 512 tokens), so a
 // 4096-token batch runs on 128 SMs and a decode-sized batch streams the router matrix through
 // eight SMs instead of one.  Each
@@ -34,11 +34,16 @@ namespace {
 // than depth)
 constexpr int kRpThreads = 192;
 constexpr int kSmallTile = 64;
+// Batches up to which the tiles have 64 rows: twice as many CTAs, each with half the partial sums to send, reduce
+// and route.  9.7 -> 6.8 us at 128 and 200 tokens, 10.2 -> 7.6 at 512, 10.2 -> 9.3 at 1024, 10.5 -> 9.7 at 2048; above,
+// the clusters no longer run all at once (2368 tokens: 11.0 against 17.3).  The K split, which decides the
+// order of the sums, depends on the number of 128-row tiles either way.
+constexpr int kSmallTileTokens = 2048;
 constexpr int kWarpRows = 8;   // rows of a CTA up to which a warp routes a row (two each); above, a quad of lanes does
 constexpr int kRpTileBytes = kTileM * kTileKBytes;  // 16 KiB: 128 rows of one 128-byte K block
 
-// kRows: token rows of a tile that exist at most.  64 is the form of batches of at most 64 tokens, where
-// the launch is a chain of latencies: its CTA's five or six K blocks all fit the ring (half a token tile
+// kRows: token rows of a tile.  64 is the form of batches of at most kSmallTileTokens tokens, where
+// the launch is a chain of latencies: with eight CTAs a tile the five or six K blocks of each all fit the ring (half a token tile
 // each; the MMA reads the next tile's bytes as rows 64..127, whose results nobody looks at).
 template <int kRows>
 struct alignas(1024) RouterSmem {
@@ -177,7 +182,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       if (!ok) break;
       if (elect_one()) {
         mbar_arrive_expect_tx(&smem->full[stage], static_cast<uint32_t>(Smem::kTokenBytes + kRpTileBytes));
-        tma_load_2d(smem->a[stage], &map_x, &smem->full[stage], kb * kTileKBytes, m_tile * kTileM);
+        tma_load_2d(smem->a[stage], &map_x, &smem->full[stage], kb * kTileKBytes, m_tile * kRows);
         tma_load_2d(smem->b[stage], &map_w, &smem->full[stage], kb * kTileKBytes, 0);
       }
       __syncwarp();
@@ -231,8 +236,8 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const int owner_row = row / kSplit;
     // rows past the end of the batch (most rows of a decode-sized batch) are not sent; the
     // tensor-memory loads are warp-wide, so a warp takes part if any of its 32 rows exists
-    const bool row_exists = m_tile * kTileM + row < p.tokens;
-    const bool warp_has_rows = m_tile * kTileM + quarter * 32 < p.tokens;
+    const bool row_exists = row < kRows && m_tile * kRows + row < p.tokens;
+    const bool warp_has_rows = quarter * 32 < kRows && m_tile * kRows + quarter * 32 < p.tokens;
     if (wait_or_abort<true>(&smem->acc_full, 0, smem, p.status) && warp_has_rows) {
       tc_fence_after_sync();
       const uint32_t remote_row =
@@ -262,13 +267,13 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
 
   if (warp >= 2 && !smem->abort) {
     // ---------------- epilogue, part 2: reduce this CTA's rows and route them, 32 at a time ----------------
-    const int tile_rows = p.tokens - m_tile * kTileM;   // may exceed the tile
+    const int tile_rows = p.tokens - m_tile * kRows;   // may exceed the tile
     // rows kSplit * i + rank < tile_rows
     const int own_rows = tile_rows >= kRows ? kOwnRows : (tile_rows - static_cast<int>(rank) + kSplit - 1) / kSplit;
     if (own_rows <= kWarpRows) {
       // a few rows: one warp per row, four logits a lane (a third of the quads' chain)
       for (int row_local = warp - 2; row_local < own_rows; row_local += 4) {
-        const int token = m_tile * kTileM + row_local * kSplit + static_cast<int>(rank);
+        const int token = m_tile * kRows + row_local * kSplit + static_cast<int>(rank);
         float4 acc = make_float4(0, 0, 0, 0);
 #pragma unroll
         for (int source = 0; source < kSplit; ++source) {
@@ -294,12 +299,12 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const int part = t & 3;         // columns [32 * part, 32 * part + 32)
 #pragma unroll 1
     for (int pass = 0; pass < (kOwnRows + 31) / 32; ++pass) {
-      if (m_tile * kTileM + pass * 32 * kSplit >= p.tokens) break;   // no row of this pass exists
+      if (m_tile * kRows + pass * 32 * kSplit >= p.tokens) break;   // no row of this pass exists
       // tile row kSplit * row_local + rank; with eight owners a CTA has 16 rows and half of the
       // threads only keep their quads company (they read row 15 again and store nothing)
       const bool row_owned = pass * 32 + (t >> 2) < kOwnRows;
       const int row_local = row_owned ? pass * 32 + (t >> 2) : kOwnRows - 1;
-      const int token = m_tile * kTileM + row_local * kSplit + static_cast<int>(rank);
+      const int token = m_tile * kRows + row_local * kSplit + static_cast<int>(rank);
       const bool valid = row_owned && token < p.tokens;
       float4 acc[8];
 #pragma unroll
@@ -372,7 +377,7 @@ cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, c
     if (e != cudaSuccess) return e;
     prepared[device] = true;
   }
-  const int m_tiles = (p.tokens + kTileM - 1) / kTileM;
+  const int m_tiles = (p.tokens + kRows - 1) / kRows;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(m_tiles * kSplit));
   config.blockDim = dim3(kRpThreads);
@@ -397,8 +402,8 @@ template <bool kFp8>
 cudaError_t launch_split(const CUtensorMap& map_x, const CUtensorMap& map_w, const RouterParams& p,
                          cudaStream_t stream) {
   const int m_tiles = (p.tokens + kTileM - 1) / kTileM;
-  if (p.tokens <= kSmallTile) return launch_variant<kFp8, 8, kSmallTile>(map_x, map_w, p, stream);
-  if (m_tiles <= 4) return launch_variant<kFp8, 8, kTileM>(map_x, map_w, p, stream);
+  if (m_tiles <= 4) return launch_variant<kFp8, 8, kSmallTile>(map_x, map_w, p, stream);
+  if (p.tokens <= kSmallTileTokens) return launch_variant<kFp8, 4, kSmallTile>(map_x, map_w, p, stream);
   if (m_tiles * 4 <= 160) return launch_variant<kFp8, 4, kTileM>(map_x, map_w, p, stream);
   if (m_tiles * 2 <= 160) return launch_variant<kFp8, 2, kTileM>(map_x, map_w, p, stream);
   return launch_variant<kFp8, 1, kTileM>(map_x, map_w, p, stream);
@@ -412,7 +417,7 @@ int launch_route_project(const void* x, const void* router_w, bool fp8, const fl
                          cudaStream_t stream) {
   const uint64_t row_bytes = fp8 ? kHidden : 2 * kHidden;
   CUtensorMap map_x, map_w;
-  if (!make_operand_tensor_map(&map_x, x, static_cast<uint64_t>(tokens), row_bytes, tokens <= kSmallTile ? kSmallTile : kTileM) ||
+  if (!make_operand_tensor_map(&map_x, x, static_cast<uint64_t>(tokens), row_bytes, tokens <= kSmallTileTokens ? kSmallTile : kTileM) ||
       !make_operand_tensor_map(&map_w, router_w, kExperts, row_bytes, kTileM))
     return static_cast<int>(cudaErrorInvalidValue);
   RouterParams p{};

@@ -96,14 +96,16 @@ def test_fp8_router_projection(oracle, cuda_device, rows):
     print(f"FP8 router projection {rows} rows: {off} logits one ulp off; {close_rows} close rows, {moved} moved")
 
 
-@pytest.mark.parametrize("rows", [1, 8, 9, 63, 64, 65])
+@pytest.mark.parametrize("rows,of", [(1, 512), (8, 512), (9, 512), (63, 512), (64, 512), (65, 512), (129, 512),
+                                     (513, 2049), (577, 2049), (2048, 2049)])
 @pytest.mark.parametrize("fp8", [False, True])
-def test_router_tiles_of_few_rows(cuda_device, rows, fp8):
-    """The 64-row tile, whose warps take eight rows each, at its edges: every row's logits, experts and
-    weights are those of the same row in a batch of 300, which takes 128-row tiles."""
+def test_router_tiles_of_few_rows(cuda_device, rows, of, fp8):
+    """64-row tiles, whose warps take up to eight rows each, at their edges: every row's logits, experts and
+    weights are those of the same row in a batch of `of`, whose K range is split the same way (over eight CTAs up
+    to 512 tokens, over four above; a batch of 2049 has 128-row tiles)."""
     import gevva_b200 as gm
     gen = torch.Generator().manual_seed(3000 + rows)
-    x = torch.randn((300, HIDDEN), generator=gen).to(cuda_device)
+    x = torch.randn((of, HIDDEN), generator=gen).to(cuda_device)
     router = (torch.randn((EXPERTS, HIDDEN), generator=gen) * 0.02).to(cuda_device)
     scale = (0.5 + torch.rand(EXPERTS, generator=gen)).to(torch.bfloat16).to(cuda_device)
     act = ws = None
@@ -119,7 +121,7 @@ def test_router_tiles_of_few_rows(cuda_device, rows, fp8):
         extra = dict(activation_scales=act[:n].contiguous(), weight_scale=ws) if fp8 else {}
         return gm.route_project(x[:n].contiguous(), router, scale, want_logits=True, **extra)
 
-    for few, many in zip(run(rows), run(300)):
+    for few, many in zip(run(rows), run(of)):
         assert torch.equal(few[:rows], many[:rows])
 
 
