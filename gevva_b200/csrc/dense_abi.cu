@@ -80,17 +80,18 @@ void gevva_dense_destroy(gevva_dense* d) {
 int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, int max_tokens) {
   if (!out || !weights || !weights->gate_up || !weights->down || max_tokens < 1) return GEVVA_MOE_BAD_ARGUMENT;
   if (max_tokens > 131072) return GEVVA_MOE_TOO_LARGE;
-  cudaDeviceProp prop;
+  int major = 0, sms = 0;
   int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || cudaGetDeviceProperties(&prop, device) != cudaSuccess)
+  if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
     return GEVVA_MOE_CUDA_ERROR;
-  if (prop.major != 10) return GEVVA_MOE_NO_DEVICE;
+  if (major != 10) return GEVVA_MOE_NO_DEVICE;
   if (gv::prepare_grouped_gemm() != 0) return GEVVA_MOE_CUDA_ERROR;
   gevva_dense* d = new (std::nothrow) gevva_dense;
   if (!d) return GEVVA_MOE_CUDA_ERROR;
   d->weights = *weights;
   d->max_tokens = max_tokens;
-  d->sm_count = prop.multiProcessorCount;
+  d->sm_count = sms;
   const size_t t = static_cast<size_t>(max_tokens);
   const size_t tiles = t / gv::kTileM + gv::kExperts + 1;
   const size_t int_count = 2 * (gv::kExperts + 1) + tiles + 2;

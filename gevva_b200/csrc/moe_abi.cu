@@ -266,9 +266,10 @@ struct gevva_moe {
   gv::GemmOperands w2{};
   uint8_t* w13_sf_tiled = nullptr;  // runner-owned re-tiling of weights.w13_sf for the CTA-pair tile kernels
   gv::W13PairOperands w13_pairs{};  // the CTA-pair form of the fused w13 stage
-  uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf by unit of 64 columns
+  uint8_t* w13_sf_units = nullptr;  // runner-owned re-tiling of weights.w13_sf by unit of 64 columns (and its allocation,
+                                    // which the next two share)
   uint8_t* w13_sf_fragments = nullptr;  // the same in the row order of grouped_gemm_w13_pair.cu
-  uint8_t* w2_sf_down = nullptr;    // runner-owned re-tiling of weights.w2_sf in the column order of grouped_gemm_down.cu
+  uint8_t* w2_sf_down = nullptr;    // re-tiling of weights.w2_sf in the column order of grouped_gemm_down.cu
   gv::StreamOperands stream_experts{};  // few rows an expert: both GEMMs in one launch, weights on the MMA's M side
   bool w13_pair_form = false;       // GEVVA_MOE_OPTION_W13_PAIRS, or GEVVA_MOE_W13_PAIRS=1 for a whole process
   int sm_count = 0;
@@ -308,12 +309,12 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   const bool use_pairs = runner->pairs && tokens > gv::kFusedSortQuantizeMaxTokens;
   const unsigned front = GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE;
   const unsigned layer_body = front | GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU | GEVVA_MOE_STAGE_W2;
-  // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side
-  // does both GEMMs.  Up to about 40 rows an expert that is faster than the launches with 128-row tiles
-  // (per layer of two distinct ones, us, one B200, with the sort and the quantiser as launches of their own
-  // on both sides: 129 tokens 101.9 against 111.4, 200 103.4 / 112.5, 450 108.0 / 116.8, 613 114.1 / 121.3,
-  // 800 124.0 / 126.9): above, its GeGLU epilogue, which handles a column of a token per thread through
-  // shared memory, outweighs the weights.
+  // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side does both GEMMs.
+  // Against the two launches, per layer of two distinct ones, us, one B200, uniform routing: 310 tokens 101.8 against 101.1,
+  // 400 102.7 / 103.8, 500 104.5 / 106.9, 613 109.1 / 112.5, 800 113.7 / 116.4, 1000 126.4 / 122.0 (up to 296 tokens it
+  // also takes in the sort and the quantiser and is 5 to 10 us faster).  A skewed router gives a few experts many 64-row
+  // chunks, each with the whole of the weights: Zipf, 400 tokens 90.8 / 87.6, 613 110.8 / 105.2, 800 124.8 / 110.1.  The host
+  // does not know the routes, so the line lies where the one gains what the other loses.
   const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !runner->pairs &&
                        !runner->w13_pair_form && tokens <= kStreamTokens;
   if ((stages & layer_body) == layer_body && streams && runner->decode_front && gv::stream_layer_fits(tokens, sm_count)) {
@@ -414,9 +415,10 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
     return GEVVA_MOE_BAD_ARGUMENT;  // "shared expert capacity mismatch", src/nvfp4_cutlass.cu:1788
   int device = 0;
   GV_CUDA(cudaGetDevice(&device), "cudaGetDevice");
-  cudaDeviceProp prop;
-  GV_CUDA(cudaGetDeviceProperties(&prop, device), "cudaGetDeviceProperties");
-  if (prop.major != 10 || !encode_tiled()) return GEVVA_MOE_NO_DEVICE;
+  int major = 0, sms = 0;  // (all properties of a device take 3 ms to ask for)
+  GV_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device), "cudaDeviceGetAttribute");
+  GV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
+  if (major != 10 || !encode_tiled()) return GEVVA_MOE_NO_DEVICE;
   GV_CUDA(static_cast<cudaError_t>(gv::prepare_grouped_gemm()), "cudaFuncSetAttribute");
 
   gevva_moe* m = new (std::nothrow) gevva_moe;
@@ -432,7 +434,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   m->decode_front = !(front_env && front_env[0] == '0');
   const char* pairs_env = std::getenv("GEVVA_MOE_PAIRS");
   m->pairs = (options && (options->flags & GEVVA_MOE_OPTION_PAIRS)) || (pairs_env && pairs_env[0] == '1');
-  m->sm_count = prop.multiProcessorCount;
+  m->sm_count = sms;
   if (share_scratch_with) {
     m->scratch = share_scratch_with->scratch;
     ++m->scratch->references;
@@ -462,13 +464,14 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   // The fused w13 epilogues pair up rows with gate rows inside one MMA tile; their weight scales are a
   // one-off re-tiling of the caller's tensor (the caller's memory is not touched).
   {
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_units), gv::w13_unit_scale_bytes(kExperts));
+    // one allocation for the three: of a runner's creation most goes into allocations
+    const size_t unit_bytes = gv::w13_unit_scale_bytes(kExperts);  // a multiple of 2 KiB
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_units), 2 * unit_bytes + gv::retiled_w2_scale_bytes(kExperts));
     if (e == cudaSuccess) {
+      m->w13_sf_fragments = m->w13_sf_units + unit_bytes;
+      m->w2_sf_down = m->w13_sf_fragments + unit_bytes;
       gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_units, kExperts, false, nullptr);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&m->w2_sf_down), gv::retiled_w2_scale_bytes(kExperts));
-    if (e == cudaSuccess) {
+      gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_fragments, kExperts, true, nullptr);
       gv::launch_retile_w2_scales(static_cast<const uint8_t*>(weights->w2_sf), m->w2_sf_down, kExperts, nullptr);
       e = cudaGetLastError();
     }
@@ -522,13 +525,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   const char* w13_pairs_env = std::getenv("GEVVA_MOE_W13_PAIRS");
   m->w13_pair_form = (options && (options->flags & GEVVA_MOE_OPTION_W13_PAIRS)) || (w13_pairs_env && w13_pairs_env[0] == '1');
   {
-    cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&m->w13_sf_fragments), gv::w13_unit_scale_bytes(kExperts));
-    if (e == cudaSuccess) {
-      gv::launch_retile_w13_unit_scales(static_cast<const uint8_t*>(weights->w13_sf), m->w13_sf_fragments, kExperts, true, nullptr);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    const cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
     if (e != cudaSuccess) {
       gevva_moe_destroy(m);
       return cuda_failure(e, "w13 pair form");
@@ -582,8 +579,6 @@ void gevva_moe_destroy(gevva_moe* runner) {
   if (runner->scratch && --runner->scratch->references == 0) free_scratch(runner->scratch);
   cudaFree(runner->w13_sf_tiled);
   cudaFree(runner->w13_sf_units);
-  cudaFree(runner->w13_sf_fragments);
-  cudaFree(runner->w2_sf_down);
   delete runner;
 }
 
