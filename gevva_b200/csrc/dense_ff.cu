@@ -49,30 +49,33 @@ __device__ __forceinline__ float bf16_round(float v) {
   return __bfloat162float(__float2bfloat16_rn(v));
 }
 
-// Block-wide sum of squares of 8 values per thread, in the fixed order described above.
-// `scratch` holds blockDim/32 + 1 floats.  Every thread gets the total.
-__device__ __forceinline__ float block_sum_squares(const float* v, float* scratch) {
+// A thread's sum of squares of its 8 values, then the warp's in lane 0, by a shuffle-down tree (lanes beyond the
+// tree keep their own value).
+__device__ __forceinline__ float warp_sum_squares(const float* v) {
   float s = 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) s = __fmaf_rn(v[i], v[i], s);
-  // shuffle-down tree; lanes beyond the tree keep their own value, lane 0 ends with the sum
 #pragma unroll
   for (int offset = 16; offset; offset >>= 1) {
     const float other = __shfl_down_sync(0xffffffffu, s, offset);
     if ((threadIdx.x & 31) + offset < 32) s = __fadd_rn(s, other);
   }
-  const int warps = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float total = scratch[0];
-    for (int w = 1; w < warps; ++w) total = __fadd_rn(total, scratch[w]);
-    scratch[warps] = total;
-  }
-  __syncthreads();
-  const float total = scratch[warps];
-  __syncthreads();
+  return s;
+}
+
+// The warps' sums folded in order, by every thread for itself: these kernels are chains of latencies (a row a
+// block), and one thread that folds for all costs two more barriers and eleven dependent loads.
+constexpr int kRowWarps = kRowThreads / 32;  // 11
+__device__ __forceinline__ float fold_warps(const float* sums) {
+  float total = sums[0];
+#pragma unroll
+  for (int w = 1; w < kRowWarps; ++w) total = __fadd_rn(total, sums[w]);
   return total;
+}
+
+// Inverse root mean square from a row's sum of squares.
+__device__ __forceinline__ float inverse_rms(float sum) {
+  return gv_rsqrtf(__fadd_rn(__fdiv_rn(sum, static_cast<float>(kHidden)), 1e-6f));
 }
 
 __global__ void __launch_bounds__(kRowThreads)
@@ -80,7 +83,7 @@ ff_prepare_kernel(const __nv_bfloat16* __restrict__ input, const __nv_bfloat16* 
                   const __nv_bfloat16* __restrict__ expert_weight,
                   const __nv_bfloat16* __restrict__ router_scale, __nv_bfloat16* __restrict__ dense_out,
                   __nv_bfloat16* __restrict__ expert_out, __nv_bfloat16* __restrict__ router_out) {
-  __shared__ float scratch[kRowThreads / 32 + 1];
+  __shared__ float sums[kRowWarps];
   grid_launch_dependents();
   grid_dependency_wait();
   const size_t base = static_cast<size_t>(blockIdx.x) * kHidden;
@@ -89,8 +92,10 @@ ff_prepare_kernel(const __nv_bfloat16* __restrict__ input, const __nv_bfloat16* 
   unpack8(__ldg(reinterpret_cast<const uint4*>(dense_weight) + threadIdx.x), dw);
   unpack8(__ldg(reinterpret_cast<const uint4*>(expert_weight) + threadIdx.x), ew);
   unpack8(__ldg(reinterpret_cast<const uint4*>(router_scale) + threadIdx.x), rs);
-  const float sum = block_sum_squares(x, scratch);
-  const float inverse = gv_rsqrtf(__fadd_rn(__fdiv_rn(sum, static_cast<float>(kHidden)), 1e-6f));
+  const float warp_sum = warp_sum_squares(x);
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = warp_sum;
+  __syncthreads();
+  const float inverse = inverse_rms(fold_warps(sums));
   const float root = gv_rsqrtf(static_cast<float>(kHidden));
   float d[8], e[8], r[8];
 #pragma unroll
@@ -106,15 +111,15 @@ ff_prepare_kernel(const __nv_bfloat16* __restrict__ input, const __nv_bfloat16* 
   reinterpret_cast<uint4*>(router_out + base)[threadIdx.x] = pack8(r);
 }
 
+template <int kWarps>
 __device__ __forceinline__ float block_max(float v, float* scratch) {
 #pragma unroll
   for (int offset = 16; offset; offset >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, offset));
-  const int warps = blockDim.x >> 5;
   if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
   __syncthreads();
   float total = scratch[0];
-  for (int w = 1; w < warps; ++w) total = fmaxf(total, scratch[w]);
-  __syncthreads();
+#pragma unroll
+  for (int w = 1; w < kWarps; ++w) total = fmaxf(total, scratch[w]);
   return total;
 }
 
@@ -131,7 +136,7 @@ __device__ __forceinline__ uint2 encode_e4m3x8(const float* v, float inverse) {
 __global__ void __launch_bounds__(kRowThreads)
 fp8_quantize_rows_kernel(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ out,
                          float* __restrict__ scales, int rows, RoutePlan plan) {
-  __shared__ float scratch[kRowThreads / 32 + 1];
+  __shared__ float scratch[kRowWarps];
   __shared__ int scan_scratch[16];
   grid_launch_dependents();
   grid_dependency_wait();
@@ -143,7 +148,7 @@ fp8_quantize_rows_kernel(const __nv_bfloat16* __restrict__ input, uint8_t* __res
   float maximum = 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) maximum = fmaxf(maximum, fabsf(x[i]));
-  maximum = block_max(maximum, scratch);
+  maximum = block_max<kRowWarps>(maximum, scratch);
   const float scale = fmaxf(__fdiv_rn(maximum, 448.0f), 1.17549435e-38f);
   if (threadIdx.x == 0) scales[blockIdx.x] = scale;
   const float inverse = __fdiv_rn(1.0f, scale);
@@ -154,7 +159,7 @@ __global__ void __launch_bounds__(kDenseThreads)
 gelu_quantize_fp8_kernel(const __nv_bfloat16* __restrict__ gate_up,
                          const float* __restrict__ activation_scales, float gate_w_scale,
                          float up_w_scale, uint8_t* __restrict__ out, float* __restrict__ scales) {
-  __shared__ float scratch[kDenseThreads / 32 + 1];
+  __shared__ float scratch[kDenseThreads / 32];
   grid_launch_dependents();
   grid_dependency_wait();
   const int row = blockIdx.x;
@@ -176,7 +181,7 @@ gelu_quantize_fp8_kernel(const __nv_bfloat16* __restrict__ gate_up,
       maximum = fmaxf(maximum, fabsf(value[i]));
     }
   }
-  maximum = block_max(maximum, scratch);
+  maximum = block_max<kDenseThreads / 32>(maximum, scratch);
   const float scale = fmaxf(__fdiv_rn(maximum, 448.0f), 1.17549435e-38f);
   if (threadIdx.x == 0) scales[row] = scale;
   const float inverse = __fdiv_rn(1.0f, scale);
@@ -195,15 +200,36 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
                    const __nv_bfloat16* __restrict__ layer_scalar, __nv_bfloat16* __restrict__ output,
                    const float* __restrict__ dense_activation_scales,
                    const float* __restrict__ dense_projection_scale) {
-  __shared__ float scratch[kRowThreads / 32 + 1];
+  __shared__ float dense_sums[kRowWarps], expert_sums[kRowWarps], combined_sums[kRowWarps];
   grid_launch_dependents();
   grid_dependency_wait();
   const int row = blockIdx.x;
   const size_t base = static_cast<size_t>(row) * kHidden;
+  // Everything is asked for at once: the norm weights have left L2 since the last layer (the experts' weights went
+  // through it), and a load behind each sum would put a trip to HBM into the chain each time.
+  int sources[kTopK];
+  float weights[kTopK];
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k) {
+    const int index = row * kTopK + k;
+    sources[k] = inverse_routes ? inverse_routes[index] : index;
+    weights[k] = route_weights[index];
+  }
+  const uint4 dense_raw = __ldg(reinterpret_cast<const uint4*>(dense + base) + threadIdx.x);
+  const uint4 dense_weight_raw = __ldg(reinterpret_cast<const uint4*>(dense_weight) + threadIdx.x);
+  const uint4 expert_weight_raw = __ldg(reinterpret_cast<const uint4*>(expert_weight) + threadIdx.x);
+  const uint4 combined_weight_raw = __ldg(reinterpret_cast<const uint4*>(combined_weight) + threadIdx.x);
+  const uint4 residual_raw = __ldg(reinterpret_cast<const uint4*>(residual + base) + threadIdx.x);
+  const float scalar = __bfloat162float(*layer_scalar);
+  const float scale = dense_activation_scales ? __fmul_rn(dense_activation_scales[row], dense_projection_scale[0]) : 1.0f;
+  uint4 routes[kTopK];
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k)
+    routes[k] = __ldg(reinterpret_cast<const uint4*>(expert_routes + static_cast<size_t>(sources[k]) * kHidden) + threadIdx.x);
+
   float d[8], e[8], w[8];
-  unpack8(__ldg(reinterpret_cast<const uint4*>(dense + base) + threadIdx.x), d);
+  unpack8(dense_raw, d);
   if (dense_activation_scales) {
-    const float scale = __fmul_rn(dense_activation_scales[row], dense_projection_scale[0]);
 #pragma unroll
     for (int i = 0; i < 8; ++i) d[i] = bf16_round(__fmul_rn(d[i], scale));
   }
@@ -211,36 +237,36 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
   for (int i = 0; i < 8; ++i) e[i] = 0.0f;
 #pragma unroll
   for (int k = 0; k < kTopK; ++k) {
-    const int index = row * kTopK + k;
-    const int source = inverse_routes ? inverse_routes[index] : index;
-    const float weight = route_weights[index];
     float v[8];
-    unpack8(__ldg(reinterpret_cast<const uint4*>(expert_routes + static_cast<size_t>(source) * kHidden) +
-                  threadIdx.x),
-            v);
+    unpack8(routes[k], v);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) e[i] = __fmaf_rn(v[i], weight, e[i]);
+    for (int i = 0; i < 8; ++i) e[i] = __fmaf_rn(v[i], weights[k], e[i]);
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) e[i] = bf16_round(e[i]);
-  const float dense_inverse =
-      gv_rsqrtf(__fadd_rn(__fdiv_rn(block_sum_squares(d, scratch), static_cast<float>(kHidden)), 1e-6f));
-  const float expert_inverse =
-      gv_rsqrtf(__fadd_rn(__fdiv_rn(block_sum_squares(e, scratch), static_cast<float>(kHidden)), 1e-6f));
+  const float dense_sum = warp_sum_squares(d), expert_sum = warp_sum_squares(e);
+  if ((threadIdx.x & 31) == 0) {
+    dense_sums[threadIdx.x >> 5] = dense_sum;
+    expert_sums[threadIdx.x >> 5] = expert_sum;
+  }
+  __syncthreads();
+  const float dense_inverse = inverse_rms(fold_warps(dense_sums));
+  const float expert_inverse = inverse_rms(fold_warps(expert_sums));
   float combined[8];
-  unpack8(__ldg(reinterpret_cast<const uint4*>(dense_weight) + threadIdx.x), w);
+  unpack8(dense_weight_raw, w);
 #pragma unroll
   for (int i = 0; i < 8; ++i) combined[i] = bf16_round(__fmul_rn(__fmul_rn(d[i], dense_inverse), w[i]));
-  unpack8(__ldg(reinterpret_cast<const uint4*>(expert_weight) + threadIdx.x), w);
+  unpack8(expert_weight_raw, w);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     combined[i] = bf16_round(__fadd_rn(combined[i], bf16_round(__fmul_rn(__fmul_rn(e[i], expert_inverse), w[i]))));
-  const float combined_inverse = gv_rsqrtf(
-      __fadd_rn(__fdiv_rn(block_sum_squares(combined, scratch), static_cast<float>(kHidden)), 1e-6f));
+  const float combined_sum = warp_sum_squares(combined);
+  if ((threadIdx.x & 31) == 0) combined_sums[threadIdx.x >> 5] = combined_sum;
+  __syncthreads();
+  const float combined_inverse = inverse_rms(fold_warps(combined_sums));
   float r[8], out[8];
-  unpack8(__ldg(reinterpret_cast<const uint4*>(combined_weight) + threadIdx.x), w);
-  unpack8(__ldg(reinterpret_cast<const uint4*>(residual + base) + threadIdx.x), r);
-  const float scalar = __bfloat162float(*layer_scalar);
+  unpack8(combined_weight_raw, w);
+  unpack8(residual_raw, r);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float normalized = bf16_round(__fmul_rn(__fmul_rn(combined[i], combined_inverse), w[i]));
