@@ -232,11 +232,12 @@ struct LayerWorkspace {
 // SMs that the dense MLP of a decode-sized layer gets beside the experts.  An expert launch of this size
 // holds its SMs from the router to its end, and its time is that of its weights' way through HBM, which 132
 // SMs fill as well as 148; the 18 MB of dense weights pass meanwhile.  With a few tokens the experts are
-// few and the dense side is the longer chain, so it gets more (whole layers in a graph, us, at 16 / 24 /
-// 32 / 48 SMs: 1 token 51.8 / 43.1 / 43.0 / 33.6, 4 tokens 58.4 / 49.5 / 48.8 / 46.5, 8 tokens 65.5 / 57.9 /
-// 57.5 / 61.9, 16 tokens 74.8 / 76.4 / 77.7 / 82.3, 40 tokens 97.1 / 98.8 / 101.4 / 108.0).
+// few and the dense side is the longer chain, so it gets more; 33 SMs hold the first projection's items of 128
+// weight rows in one wave, 17 those of 256 (whole layers in a graph, us, at 16 / 17 / 33 / 48 SMs: 1 token 46.4 / 38.9 / 34.4 /
+// 32.3, 4 tokens 52.8 / 45.0 / 44.2 / 43.4, 5 tokens 55.5 / 47.7 / 44.9 / 47.2, 8 tokens 60.5 / 52.1 / 54.2 / 57.4, 12 tokens
+// 62.7 / 62.3 / 64.2 / 68.1, 40 tokens 93.6 / 94.6 / 99.6 / -, 128 tokens 107.4 / 108.4 / 109.9 / -).
 int dense_sms_beside(int tokens, int sms) {
-  const int wanted = tokens <= 4 ? 48 : tokens <= 8 ? 32 : 16;
+  const int wanted = tokens <= 4 ? 48 : tokens <= 6 ? 33 : tokens <= 12 ? 17 : 16;
   return wanted * 2 < sms ? wanted : sms / 2;
 }
 }  // namespace
