@@ -186,8 +186,9 @@ class Nvfp4ExpertRunner:
     def __init__(self, experts: ExpertWeights, maximum_tokens: int = 1, shared_scratch=None, nvtx=False,
                  pairs=False, w13_pairs=False):
         """nvtx: wrap every stage's launches in a named NVTX range; pairs: run the expert GEMMs of
-        batches above 128 tokens as CTA pairs; w13_pairs: run the fused w13 stage of such batches as
-        CTA pairs with the weights on the MMA's M side (all additions of this build, same bits)."""
+        batches above 128 tokens as CTA pairs; w13_pairs: run batches of 129 to 640 tokens as larger ones
+        run by default, with the weights of the fused w13 stage on the MMA's M side (additions to the reference's
+        interface, same bits)."""
         experts.validate()
         self._weights = experts  # keeps the tensors alive, as the DeviceModel arena does
         self._device = experts.w13.device

@@ -779,6 +779,33 @@ def test_streaming_experts_equal_the_two_launches(gm, weights, cuda_device, toke
     assert results[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens", [297, 1000])
+def test_captured_layer_equals_the_eager_one(gm, weights, cuda_device, tokens):
+    """A batch whose route sort is one cooperative launch, captured into a graph (where that launch is an
+    ordinary successor) and replayed with new inputs: the eager call's bits."""
+    runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+    x = hashgen.activations(tokens, HIDDEN, 61, cuda_device)
+    ids = torch.from_numpy(random_ids(tokens, 21)).to(cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    out = torch.empty_like(x)
+    runner.launch_batch(x, ids, rw, out, tokens)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(2):
+            runner.launch_batch(x, ids, rw, out, tokens)
+    for seed in (62, 63):
+        x.copy_(hashgen.activations(tokens, HIDDEN, seed, cuda_device))
+        ids.copy_(torch.from_numpy(random_ids(tokens, seed)))
+        out.zero_()
+        graph.replay()
+        runner.check()
+        replayed = out.clone()
+        runner.launch_batch(x, ids, rw, out, tokens)
+        runner.check()
+        assert torch.equal(replayed, out) and out.float().abs().max() > 0
+
+
 def test_nvtx_ranges_do_not_change_results(gm, weights, cuda_device):
     """A runner created with the NVTX option marks its stages and computes the same bits; unknown
     option flags are refused."""
