@@ -12,12 +12,13 @@
 //              are the unit's up rows, 64..127 its gate rows (one 3-D box brings both; their scales come
 //              from a copy re-tiled by unit, made at runner creation)
 //   w2 item    (chunk) x (128 output columns)
-// One list per launch, all w13 items chunk by chunk, then all w2 items; dealt round-robin, the w2 part
-// so that the CTAs that are one w13 item short (180 KB) get four w2 items (48 KB each) first.
+// One list per launch, all w13 items chunk by chunk, then all w2 items.  A CTA's first w13 item is given by its number,
+// further ones are claimed one by one, a little ahead; the w2 items are dealt in the order in which the CTAs run out of
+// w13 items, so that those that are one short (180 KB) get four w2 items (48 KB each) first.
 //
-// Roles (13 warps): 0 fetches weights, 1 issues MMAs, 2 fetches activations, 3 copies scale factors to
+// Roles (14 warps): 0 fetches weights, 1 issues MMAs, 2 fetches activations, 3 copies scale factors to
 // tensor memory one stage ahead, 4..11 are the epilogue (two warps per 32-lane quarter, alternating
-// groups of eight rows), 12 publishes finished w13 items.  Seven stages of one K block (256 elements); four accumulators of 64 columns,
+// groups of eight rows), 12 publishes finished w13 items, 13 claims the next ones.  Seven stages of one K block (256 elements); four accumulators of 64 columns,
 // so nothing waits for a drain.  In the w13 epilogue a thread holds one weight row for eight tokens, so
 // bf16(alpha * acc), which is what the reference's GEMM stores, changes hands through shared memory and a
 // thread then owns one column of four tokens: GeGLU, block maxima over sixteen lanes, codes.  (One token at a
@@ -28,8 +29,14 @@
 // A w2 item needs the w2 operand rows of its expert: when the epilogue warps have stored an item, a
 // publisher warp adds one to the expert's counter (release); the activation side of a w2 item waits for
 // 11 x chunks of them (bounded acquire spin), crosses to the async proxy and loads.  The weight side
-// waits for nothing, so weight bytes keep arriving across the boundary.  All CTAs are co-resident (one per
-// SM) and no wait can form a cycle.
+// waits for nothing, so weight bytes keep arriving across the boundary.
+//
+// What other streams run may keep a part of the grid from starting for any time, and another such grid that waits for
+// SMs that this one holds must not be waited for.  So no wait depends on a CTA that is not running: of what is
+// waited for, w13 items lie with CTAs that run (gv_stream_schedule.h), and tokens that are not quantised
+// after 20 us are quantised by the CTAs that wait (stream_rescue_tokens).  Items dealt in advance to CTAs that were
+// assumed to run, with a cooperative launch to have that, cost 2 us a layer in a graph and 4 us eagerly (64
+// tokens, 87.7 -> 90 and 91 us), because such a launch starts only once all SMs are free.
 //
 // In its kFront form the kernel also sorts the routes and quantises the input: every CTA ranks the whole
 // batch's routes by a counting sort (12 warps, a stretch of routes each) and derives the group geometry for
@@ -48,6 +55,7 @@
 #include "gv_gemm_parts.cuh"
 #include "gv_launchers.h"
 #include "gv_quantize.cuh"
+#include "gv_stream_schedule.h"
 
 namespace gv {
 
@@ -59,26 +67,29 @@ constexpr int kStAccStages = 4;
 constexpr int kStWeightWarp = 0, kStMmaWarp = 1, kStTokenWarp = 2, kStScaleWarp = 3, kStEpilogueWarp = 4;
 constexpr int kStEpilogueWarps = 8;
 constexpr int kStPublishWarp = kStEpilogueWarp + kStEpilogueWarps;     // 12
-constexpr int kStThreads = (kStPublishWarp + 1) * 32;                  // 416
+constexpr int kStClaimWarp = kStPublishWarp + 1;                       // 13
+constexpr int kStThreads = (kStClaimWarp + 1) * 32;                    // 448
 constexpr uint32_t kStTmemColumns = 512;
 constexpr uint32_t kStSfColumn = kStAccStages * kStRows;  // 256
 constexpr uint32_t kStSfColumnsPerStage = 32;             // 16 for the weights, 16 for the rows
 static_assert(kStSfColumn + kStSfColumnsPerStage * kStStages <= kStTmemColumns, "tensor memory budget");
 constexpr int kStWeightBytes = kTileM * kTileKBytes;      // 16 KiB
 constexpr int kStTokenBytes = kStRows * kTileKBytes;      // 8 KiB
-constexpr int kStDownTiles = kHidden / 128;               // 22 w2 items a chunk
+static_assert(kStreamUpItems == kUnits && kStreamDownItems == kHidden / 128, "items of a chunk");
 constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
 static_assert(kStMmaWarp == 1 && kStPublishWarp - 1 == kStUpKBlocks, "warps 1..11 quantise a K block each");
 constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192
 constexpr int kStDownLastMmas = 3;
 constexpr int kStMaxChunks = 256;
 constexpr int kStExchangeRows = 32;
-constexpr int kStWarps = kStThreads / 32;
 constexpr int kStOwnTokens = 2;                           // kFront: tokens a CTA quantises, at most
-constexpr int kStRankWarps = kStWarps - 1;                // kFront: all but the first rank the routes
+constexpr int kStRankWarps = 12;                          // kFront: warps 1..12 rank the routes
 constexpr int kStStretch = 224;                           // routes of each, at most
 constexpr int kStFrontTokens = kStStretch * kStRankWarps / kTopK;  // 336
 constexpr int kStSelfRows = 8;                            // kFront: rows of a first item that the CTA quantises itself, at most
+constexpr int kStClaims = 32;                             // claims on their way from the claim warp to the others, at most
+constexpr uint32_t kStNoMoreClaims = 1u << 15, kStNoTurn = kStNoMoreClaims - 1;
+constexpr long long kStRescueCycles = 40000;              // 20 us without progress
 
 struct alignas(1024) StreamSmem {
   uint8_t a[kStStages][kStWeightBytes];
@@ -95,6 +106,11 @@ struct alignas(1024) StreamSmem {
   uint64_t full[kStStages], empty[kStStages], sf_full[kStStages];
   uint64_t acc_full[kStAccStages], acc_empty[kStAccStages];
   volatile int progress[kStEpilogueWarps];  // w13 items whose rows each epilogue warp has stored
+  volatile int published;                   // w13 items that the publisher has counted
+  volatile int first_mine;                  // whether the CTA's first w13 item is its to count; -1: not known yet
+  volatile int begun;                       // w13 items that the weight warp has begun
+  volatile uint32_t claims[kStClaims];      // the CTA's w13 items, then its turn among the w2 items: see StreamCursor
+  volatile int downs;                       // w2 items of the CTA, once its turn is announced
   uint32_t tmem_base;
   volatile int abort;
   volatile int left;  // an epilogue warp gave up waiting
@@ -152,47 +168,72 @@ struct StreamItem {
   int n_tile;  // unit of 64 intermediate columns, or tile of 128 output columns
 };
 
-// This CTA's items in order.
-struct StreamSchedule {
-  int up_count, count;
-  int first_extra, lacking, pre;  // w2: CTAs >= first_extra are one w13 item short and take `pre` items first
-  __device__ StreamSchedule(int chunks) {
-    const int ctas = gridDim.x, cta = blockIdx.x;
-    const int up = chunks * kUnits, down = chunks * kStDownTiles;
-    up_count = up > cta ? (up - 1 - cta) / ctas + 1 : 0;
-    first_extra = up % ctas;
-    lacking = first_extra == 0 ? 0 : ctas - first_extra;
-    pre = lacking > 0 && down >= 4 * lacking + 4 * ctas ? 4 : 0;  // a short list is spread evenly instead
-    const int rest = down - pre * lacking;
-    const int turn = cta >= first_extra ? cta - first_extra : cta - first_extra + ctas;  // lacking CTAs come first
-    const int mine = (cta >= first_extra ? pre : 0) + (rest > turn ? (rest - 1 - turn) / ctas + 1 : 0);
-    count = up_count + mine;
+// Claim `i` of this CTA: the number of a w13 item, or kStNoMoreClaims + the CTA's turn among the w2 items (kStNoTurn: it
+// gave up).  The claim warp announces one after the other, the last one also when it gives up; its own waits are
+// bounded, so this wait ends.
+__device__ __forceinline__ uint32_t stream_claim(const StreamSmem* smem, int i) {
+  const uint32_t round = static_cast<uint32_t>(i / kStClaims + 1);
+  uint32_t word = smem->claims[i % kStClaims];
+  while ((word >> 16) != round) {
+    __nanosleep(32);
+    word = smem->claims[i % kStClaims];
   }
-  __device__ __forceinline__ StreamItem item(int i, const StreamSmem* smem) const {
-    const int ctas = gridDim.x, cta = blockIdx.x;
-    StreamItem it;
-    int index, per_chunk;
-    it.down = i >= up_count;
-    if (!it.down) {
-      index = cta + i * ctas;
-      per_chunk = kUnits;
-    } else {
-      int k = i - up_count;
-      const bool is_short = cta >= first_extra;
-      const int turn = is_short ? cta - first_extra : cta - first_extra + ctas;
-      if (is_short && k < pre) {
-        index = turn + k * lacking;
-      } else {
-        if (is_short) k -= pre;
-        index = pre * lacking + turn + k * ctas;
-      }
-      per_chunk = kStDownTiles;
-    }
+  return word & 0xffffu;
+}
+
+// By one thread of the claim warp.  No reader is further behind than the publisher (pipeline and accumulators hold six items).
+__device__ __forceinline__ void stream_announce(StreamSmem* smem, int i, uint32_t claim) {
+  const long long start = clock64();
+  while (smem->published + kStClaims <= i && !smem->abort && clock64() - start < kWaitLimitCycles) __nanosleep(64);
+  __threadfence_block();
+  smem->claims[i % kStClaims] = static_cast<uint32_t>(i / kStClaims + 1) << 16 | claim;
+}
+
+// The lane's view of the CTAs' first items: one that is not taken, or `firsts`.
+__device__ __forceinline__ int stream_open_first(const int* sync, int firsts, int lane) {
+  int taken[kStreamMaxCtas / 32], open = firsts;
+#pragma unroll
+  for (int j = 0; j < kStreamMaxCtas / 32; ++j)
+    taken[j] = lane + 32 * j < firsts ? *reinterpret_cast<const volatile int*>(sync + kStreamFirsts + lane + 32 * j) : 1;
+#pragma unroll
+  for (int j = 0; j < kStreamMaxCtas / 32; ++j)
+    if (taken[j] == 0) open = lane + 32 * j;
+  return open;
+}
+
+// This CTA's items in order, as each role walks them.
+struct StreamCursor {
+  int taken = 0;      // items so far
+  int ups = -1;       // w13 items of the CTA, once known
+  int turn = 0, downs = 0;
+
+  __device__ __forceinline__ StreamItem item_of(int index, bool down, const StreamSmem* smem) const {
+    const int per_chunk = down ? kStreamDownItems : kStreamUpItems;
     const int chunk = index / per_chunk;
+    StreamItem it;
+    it.down = down;
     it.n_tile = index - chunk * per_chunk;
     it.expert = smem->chunk_expert[chunk];
     it.chunk = smem->chunk_index[chunk];
     return it;
+  }
+  __device__ __forceinline__ bool next(const StreamShares& shares, const StreamSmem* smem, StreamItem& it) {
+    if (ups < 0) {
+      const uint32_t claim = stream_claim(smem, taken);
+      if (!(claim & kStNoMoreClaims)) {
+        it = item_of(static_cast<int>(claim), false, smem);
+        ++taken;
+        return true;
+      }
+      ups = taken;
+      turn = static_cast<int>(claim & kStNoTurn);
+      __threadfence_block();
+      downs = smem->downs;
+    }
+    if (taken - ups >= downs) return false;
+    it = item_of(shares.down_item(turn, taken - ups), true, smem);
+    ++taken;
+    return true;
   }
 };
 
@@ -235,13 +276,18 @@ __device__ __forceinline__ void stream_add_release(int* address) {
   asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(address) : "memory");
 }
 
-// Bounded acquire spin of a whole warp on a counter in global memory.
-__device__ __forceinline__ bool stream_wait_counter(const int* counter, int target, StreamSmem* smem, int* status) {
+// Bounded acquire spin of a whole warp on a counter in global memory; or, where one is given, on a second one.
+__device__ __forceinline__ bool stream_wait_counter(const int* counter, int target, StreamSmem* smem, int* status,
+                                                    const int* other = nullptr, int other_target = 0) {
   const long long start = clock64();
   bool ready = false;
   for (uint32_t spin = 1; !ready; ++spin) {
     ready = stream_load_acquire(counter) >= target;
     if (!ready && (spin & 63u) == 0) {
+      if (other && stream_load_acquire(other) >= other_target) {
+        ready = true;
+        break;
+      }
       if (smem->abort) break;
       if (clock64() - start > kWaitLimitCycles) {
         smem->abort = 1;
@@ -343,9 +389,49 @@ __device__ __noinline__ void stream_quantise_stage(const uint4* input, StreamSme
   if (lane == 0) mbar_arrive(&smem->full[stage]);
 }
 
+// By the publisher warp of a CTA that has had nothing to do for a while: the grid's CTAs quantise two tokens each at most,
+// and some may not be running.  The ones that are go over all tokens, token by token; a CTA that starts after all writes the
+// same bytes again.  (Their ranks are counted anew: the sort's tables have given way to the exchange tile.)
+__device__ __noinline__ void stream_rescue_tokens(const StreamParams& p, StreamSmem* smem, int lane) {
+  int* const sync = p.plan.stream_sync;
+  const int owners = p.tokens < static_cast<int>(gridDim.x) ? p.tokens : static_cast<int>(gridDim.x);
+  if (stream_load_acquire(sync + kStreamQuantised) >= owners) return;
+#pragma unroll 1
+  for (;;) {
+    int token = 0;
+    if (lane == 0) token = atomicAdd(sync + kStreamRescueClaims, 1);
+    token = __shfl_sync(0xffffffffu, token, 0);
+    if (token >= p.tokens || smem->abort) return;
+#pragma unroll 1
+    for (int k = 0; k < kTopK; ++k) {
+      const int route = token * kTopK + k;
+      const int expert = p.expert_ids[route];
+      int rank = 0;
+#pragma unroll 1
+      for (int base = 0; base < route; base += 32)
+        rank += __popc(__ballot_sync(0xffffffffu, base + lane < route && p.expert_ids[base + lane] == expert));
+      if (lane == 0) {
+        const bool valid = expert >= 0 && expert < kExperts;
+        smem->route_row[k] = valid ? smem->offsets[expert] + rank : -1;
+        if (valid) {
+          smem->route_multiplier[k] = smem->scale_q1[expert];
+          smem->route_scale_base[k] = static_cast<unsigned long long>(smem->scale_rows[expert]) * (kHidden / 16) +
+                                      sf_offset(rank, 0, kHidden / 16);
+        }
+      }
+    }
+    __syncwarp();
+    const uint4* const input = reinterpret_cast<const uint4*>(p.input) + static_cast<size_t>(token) * (kHidden / 8) + lane;
+#pragma unroll 1
+    for (int kb = 0; kb < kStUpKBlocks; ++kb) stream_quantise_token(p, smem, 0, kb, lane, __ldg(input + kb * (kTileK / 8)));
+    __syncwarp();
+    if (lane == 0) stream_add_release(sync + kStreamRescued);
+  }
+}
+
 template <bool kFront>
 __global__ void __launch_bounds__(kStThreads, 1)
-stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParams p) {
+stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_constant__ StreamParams p) {
   extern __shared__ uint8_t smem_raw[];
   StreamSmem* smem =
       reinterpret_cast<StreamSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -366,6 +452,9 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
       mbar_init(&smem->acc_empty[s], kStEpilogueWarps);
     }
     for (int w = 0; w < kStEpilogueWarps; ++w) smem->progress[w] = 0;
+    smem->published = 0;
+    smem->first_mine = -1;
+    smem->begun = 0;
     smem->abort = 0;
     smem->left = 0;
     fence_barrier_init();
@@ -374,6 +463,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     prefetch_tensor_map(&maps.up[0]);
     prefetch_tensor_map(&maps.down[0]);
   }
+  if (tid < kStClaims) smem->claims[tid] = 0;
   if (warp == kStMmaWarp) {
     tmem_alloc(&smem->tmem_base, kStTmemColumns);
     tmem_relinquish();
@@ -389,15 +479,19 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   tc_fence_after_sync();
   const uint32_t tmem_base = smem->tmem_base;
   grid_dependency_wait();  // what earlier kernels of the stream wrote is visible from here on
+  int* const sync = p.plan.stream_sync;
+  int first_taken = 0;
+  if (tid == kStClaimWarp * 32) first_taken = atomicExch(sync + kStreamFirsts + cta, 1);
 
   // ---------------- group geometry ----------------
   const bool has_token = kFront && cta < p.tokens;
   const int ctas = gridDim.x;
   const int routes = kFront ? p.tokens * kTopK : 0;
   // warp 1 + w ranks routes [w * stretch, (w + 1) * stretch) among those of its own stretch
-  const int rank_warp = warp > 0 ? warp - 1 : 0;
+  const bool ranks = warp > 0 && warp <= kStRankWarps;
+  const int rank_warp = ranks ? warp - 1 : 0;
   const int stretch = ((routes + kStRankWarps - 1) / kStRankWarps + 31) & ~31;
-  const int stretch_begin = warp > 0 ? rank_warp * stretch : routes;
+  const int stretch_begin = ranks ? rank_warp * stretch : routes;
   const int stretch_end = stretch_begin + stretch < routes ? stretch_begin + stretch : routes;
   const int own = has_token ? (p.tokens - 1 - cta) / ctas + 1 : 0;
   const int kb = warp - kStMmaWarp;  // 0..10: the K block that the warp quantises
@@ -419,7 +513,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
       for (int t = 0; t < kStOwnTokens; ++t)
         if (t < own) own_raw[t] = __ldg(own_input + static_cast<size_t>(t) * ctas * (kHidden / 8));
     }
-    if (warp > 0)
+    if (ranks)
 #pragma unroll
       for (int k = 0; k < kStStretch / 32; ++k) route_expert[32 * k] = static_cast<uint8_t>(ids[k] < kExperts ? ids[k] : kExperts);
     __syncwarp();
@@ -502,6 +596,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
       chunk += expert_chunks;
     }
     if (lane == 31) {
+      if (cta < chunk * kStreamUpItems) smem->claims[0] = 1u << 16 | static_cast<uint32_t>(cta);
       smem->offsets[kExperts] = row;
       smem->scale_rows[kExperts] = tile * kTileM;
       smem->chunks = chunk;
@@ -513,17 +608,18 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     }
   }
   __syncthreads();
-  const StreamSchedule schedule(smem->chunks);
+  const StreamShares shares(smem->chunks, ctas);
+  StreamCursor cursor;
+  StreamItem it{};
   bool ok = true;
 
   // kFront: the CTA's first w13 item does not wait for the grid's quantised rows: its own warps put them into
-  // the pipeline stages (not the weight warp's concern, which leaves it out)
-  bool self_first = kFront && schedule.up_count > 0;
-  if (kFront && warp != kStWeightWarp) {  // the weights are under way meanwhile
-    StreamItem it{};
+  // the pipeline stages (not the concern of the weight and claim warps, which leave it out)
+  bool self_first = kFront && cta < shares.up;
+  if (kFront && warp != kStWeightWarp && warp != kStClaimWarp) {  // the weights are under way meanwhile
     int first = 0, first_rows = 0;
     if (self_first) {
-      it = schedule.item(0, smem);
+      it = cursor.item_of(cta, false, smem);
       first = it.chunk * kStRows;
       first_rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
       first_rows = first_rows > kStRows ? kStRows : first_rows;
@@ -562,13 +658,13 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
       }
       smem->route_row[q] = dst;
     }
-    named_barrier(3, kStThreads - 32);
+    named_barrier(3, kStThreads - 64);
     const float multiplier = self_first ? smem->scale_q1[it.expert] : 0.0f;
     if (has_token && kb >= 0) {
       constexpr int kOwnThreads = (kStUpKBlocks + 1) * 32;
       if (warp == kStPublishWarp) {
         named_barrier(1, kOwnThreads);
-        if (lane == 0) stream_add_release(p.plan.front_sync);
+        if (lane == 0) stream_add_release(sync + kStreamQuantised);
       } else {
 #pragma unroll 1
         for (int t = 0; t < own; ++t) stream_quantise_token(p, smem, t * kTopK, kb, lane, own_raw[t ? 1 : 0]);
@@ -589,13 +685,14 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     const bool weight_side = warp == kStWeightWarp;
     int stage = 0, issued = 0;
     uint32_t phase = 0;
-    const int begin = self_first && !weight_side ? 1 : 0;
-    if (begin) {
+    bool rows_pending = kFront && !weight_side;
+    if (self_first && !weight_side) {
+      (void)cursor.next(shares, smem, it);
       stage = kStUpKBlocks % kStStages;
       phase = kStUpKBlocks / kStStages & 1;
     }
-    for (int i = begin; ok && i < schedule.count; ++i) {
-      const StreamItem it = schedule.item(i, smem);
+    while (ok && cursor.next(shares, smem, it)) {
+      if (weight_side && !it.down && lane == 0) smem->begun = cursor.taken;
       const int k_blocks = it.down ? kStDownKBlocks : kStUpKBlocks;
       const int first = it.chunk * kStRows;
       const int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
@@ -607,10 +704,12 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
                      : p.w13_scales + static_cast<size_t>(it.expert * kUnitSlots + it.n_tile) * kStUpKBlocks * kSfStageBytes;
       } else {
         const size_t scale_row = smem->scale_rows[it.expert] + first / kTileM * kTileM;
-        if (kFront && i == begin && !it.down) {
+        if (rows_pending && !it.down) {
           // the w13 operand exists once every CTA with tokens has quantised them and counted itself
-          ok = stream_wait_counter(p.plan.front_sync, p.tokens < ctas ? p.tokens : ctas, smem, status);
+          ok = stream_wait_counter(sync + kStreamQuantised, p.tokens < ctas ? p.tokens : ctas, smem, status,
+                                   sync + kStreamRescued, p.tokens);
           if (!ok) break;
+          rows_pending = false;
           asm volatile("fence.proxy.async.global;" ::: "memory");
         }
         sf = it.down ? p.inter_scales + scale_row * (kInter / 16) : p.input_scales + scale_row * (kHidden / 16);
@@ -647,7 +746,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
         }
       }
     }
-    if (!ok && lane == 0) {
+    if ((!ok || smem->abort) && lane == 0) {
       // unwinding: the copies already issued land before shared memory is given up
       const int pending = issued < kStStages ? issued : kStStages;
       for (int i = 0; i < pending; ++i) {
@@ -665,8 +764,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     const uint32_t a_lo0 = (smem_u32(smem->a[0]) & 0x3ffffu) >> 4;
     const uint32_t b_lo0 = (smem_u32(smem->b[0]) & 0x3ffffu) >> 4;
     const bool leader = elect_one();
-    for (int i = 0; ok && i < schedule.count; ++i) {
-      const StreamItem it = schedule.item(i, smem);
+    while (ok && cursor.next(shares, smem, it)) {
       const int k_blocks = it.down ? kStDownKBlocks : kStUpKBlocks;
       const int first = it.chunk * kStRows;
       int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
@@ -709,8 +807,8 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     const uint32_t sfb_lo0 = (smem_u32(smem->sfb[0]) & 0x3ffffu) >> 4;
     constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);  // 8 rows x 16 B, no swizzle
     const bool leader = elect_one();
-    for (int i = 0; ok && i < schedule.count; ++i) {
-      const bool down = i >= schedule.up_count;
+    while (ok && cursor.next(shares, smem, it)) {
+      const bool down = it.down;
       const int k_blocks = down ? kStDownKBlocks : kStUpKBlocks;
       for (int kb = 0; kb < k_blocks; ++kb) {
         ok = wait_or_abort<false>(&smem->full[stage], phase, smem, status);
@@ -729,26 +827,96 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
         }
       }
     }
+  } else if (warp == kStClaimWarp) {
+    // ---------------- claims ----------------
+    // Two items ahead of the weight warp, which is busy with one for four microseconds: a claim takes one to two under
+    // load, and weights that are asked for that much later are lost time (by the weight warp itself, 37 tokens took 3.4 us a
+    // layer more).
+    if (lane == 0) smem->first_mine = first_taken == 0;
+    int turn = shares.fixed_turn(cta);
+    bool exhausted = shares.up <= ctas, all_started = false;
+#pragma unroll 1
+    for (int i = cta < shares.up ? 1 : 0;; ++i) {
+      if (!all_started) all_started = __all_sync(0xffffffffu, stream_open_first(sync, shares.firsts, lane) == shares.firsts);
+      const long long start = clock64();
+      bool wanted = i <= 2 || smem->begun >= i - 1;
+      while (!wanted && !smem->abort && clock64() - start < 2 * kWaitLimitCycles) {
+        __nanosleep(64);
+        wanted = smem->begun >= i - 1;
+      }
+      uint32_t claim = kStNoMoreClaims | kStNoTurn;
+      if (__all_sync(0xffffffffu, wanted)) {
+        if (!exhausted) {
+          int index = 0;
+          if (lane == 0) index = shares.firsts + atomicAdd(sync + kStreamItemClaims, 1);
+          index = __shfl_sync(0xffffffffu, index, 0);
+          claim = static_cast<uint32_t>(index);
+          exhausted = index >= shares.up;
+          turn = index - shares.up;
+        }
+        while (exhausted) {
+          // the end, unless a CTA has not started: after a while its first item is this one's
+          const int open = all_started ? shares.firsts : stream_open_first(sync, shares.firsts, lane);
+          const uint32_t any = __ballot_sync(0xffffffffu, open < shares.firsts);
+          if (any == 0) {
+            claim = kStNoMoreClaims | static_cast<uint32_t>(turn);
+            break;
+          }
+          claim = kStNoMoreClaims | kStNoTurn;
+          if (__any_sync(0xffffffffu, smem->abort)) break;
+          if (__any_sync(0xffffffffu, clock64() - start > kStRescueCycles)) {
+            const int source = __ffs(static_cast<int>(any)) - 1;
+            int taken = 1;
+            if (lane == source) taken = atomicExch(sync + kStreamFirsts + open, 1);
+            claim = static_cast<uint32_t>(__shfl_sync(0xffffffffu, open, source));
+            if (__shfl_sync(0xffffffffu, taken, source) == 0) break;
+          }
+          __nanosleep(64);
+        }
+      }
+      if (lane == 0) {
+        if (claim & kStNoMoreClaims) smem->downs = claim == (kStNoMoreClaims | kStNoTurn) ? 0 : shares.down_count(turn);
+        stream_announce(smem, i, claim);
+      }
+      __syncwarp();
+      if (claim & kStNoMoreClaims) break;
+    }
   } else if (warp == kStPublishWarp) {
     // ---------------- publisher ----------------
     // Making an item's stores visible to the grid takes one to two microseconds under load.  The epilogue
     // warps leave that to this warp (their progress is a release to the CTA, the additions here extend it to
     // the GPU) and go on.
     int published = 0;
-    const long long start = clock64();
-    while (published < schedule.up_count) {
-      int done = lane < kStEpilogueWarps ? smem->progress[lane] : schedule.up_count;
-      done = __reduce_min_sync(0xffffffffu, done);
+    bool rescue = kFront;
+    long long start = clock64();
+    for (;;) {
+      int done = __reduce_min_sync(0xffffffffu, smem->progress[lane & (kStEpilogueWarps - 1)]);
+      const int first_mine = __shfl_sync(0xffffffffu, smem->first_mine, 0);
+      if (first_mine < 0) done = published;
       if (done == published) {
-        if (smem->abort || clock64() - start > 2 * kWaitLimitCycles) break;
+        const uint32_t next = smem->claims[published % kStClaims];
+        const bool over = (next >> 16) == static_cast<uint32_t>(published / kStClaims + 1) && (next & kStNoMoreClaims);
+        const long long idle = clock64() - start;
+        if (__any_sync(0xffffffffu, over || smem->abort || idle > 2 * kWaitLimitCycles)) break;
+        if (kFront && rescue && __any_sync(0xffffffffu, idle > kStRescueCycles)) {
+          stream_rescue_tokens(p, smem, lane);
+          rescue = false;
+        }
         __nanosleep(64);
         continue;
       }
       __threadfence_block();
       __syncwarp();
-      for (int i = published + lane; i < done; i += 32) stream_add_release(p.plan.tile_ready + schedule.item(i, smem).expert);
+      for (int i = published + lane; i < done; i += 32) {
+        const uint32_t word = smem->claims[i % kStClaims];
+        // (overwritten only where the claim warp gave up waiting; a first item that another CTA took is that CTA's to count)
+        if ((word >> 16) == static_cast<uint32_t>(i / kStClaims + 1) && (i > 0 || first_mine > 0))
+          stream_add_release(p.plan.tile_ready + cursor.item_of(static_cast<int>(word & 0xffffu), false, smem).expert);
+      }
       __syncwarp();
       published = done;
+      if (lane == 0) smem->published = done;
+      start = clock64();
     }
   } else {
     // ---------------- epilogue ----------------
@@ -757,8 +925,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
     const int et = tid - kStEpilogueWarp * 32;
     int acc = 0, buffer = 0;
     uint32_t acc_phase = 0;
-    for (int i = 0; i < schedule.count; ++i) {
-      const StreamItem it = schedule.item(i, smem);
+    while (cursor.next(shares, smem, it)) {
       const int first = it.chunk * kStRows;
       const int row0 = smem->offsets[it.expert] + first;
       int rows = smem->offsets[it.expert + 1] - row0;
@@ -899,7 +1066,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
       __syncwarp();
       if (lane == 0) {
         __threadfence_block();
-        smem->progress[warp - kStEpilogueWarp] = i + 1;
+        smem->progress[warp - kStEpilogueWarp] = cursor.taken;
       }
     }
   }
@@ -915,12 +1082,12 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const StreamParam
   // before a CTA's end.
   if (tid == 0) {
     __threadfence();
-    smem->last = atomicAdd(p.plan.front_sync + 1, 1) == static_cast<int>(gridDim.x) - 1;
+    smem->last = atomicAdd(sync + kStreamFinished, 1) == static_cast<int>(gridDim.x) - 1;
   }
   __syncthreads();
   if (smem->last) {
     if (tid < kExperts) p.plan.tile_ready[tid] = 0;
-    if (tid < 2) p.plan.front_sync[tid] = 0;
+    for (int i = tid; i < kStreamSyncInts; i += kStThreads) sync[i] = 0;
   }
 }
 
@@ -971,7 +1138,7 @@ int prepare_stream_experts() {
 }
 
 void launch_stream_experts(const StreamOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream) {
-  launch_chained(stream_experts_kernel<false>, dim3(sm_count), dim3(kStThreads), kStSmemBytes, stream, make_maps(op),
+  launch_chained(stream_experts_kernel<false>, dim3(sm_count < kStreamMaxCtas ? sm_count : kStreamMaxCtas), dim3(kStThreads), kStSmemBytes, stream, make_maps(op),
                  make_params(op, plan));
 }
 
@@ -985,7 +1152,7 @@ void launch_stream_layer(const StreamOperands& op, const RoutePlan& plan, const 
   p.packed = packed;
   p.scales = scales;
   p.tokens = tokens;
-  launch_chained(stream_experts_kernel<true>, dim3(sm_count), dim3(kStThreads), kStSmemBytes, stream, make_maps(op), p);
+  launch_chained(stream_experts_kernel<true>, dim3(sm_count < kStreamMaxCtas ? sm_count : kStreamMaxCtas), dim3(kStThreads), kStSmemBytes, stream, make_maps(op), p);
 }
 
 }  // namespace gv

@@ -39,8 +39,8 @@ struct RoutePlan {
   int* status;             // [1]   device status word (gv::Status)
   const int* remap;        // optional [128]: sort key = remap[expert id] (expert-parallel placement)
   int* sync;               // optional [2], zero on entry: arrival/departure counters of the one-launch sort
-  int* front_sync;         // optional [2], zero on entry and on exit: tokens quantised / CTAs finished, of the
-                           // streaming kernel
+  int* stream_sync;        // optional [kStreamSyncInts], zero on entry and on exit: counters of the streaming
+                           // kernel (gv_stream_schedule.h)
 };
 
 void launch_route(const void* logits_bf16, int ld, const void* expert_scale_bf16, float* weights,
@@ -183,7 +183,7 @@ struct StreamOperands {
   void* routed;                        // bf16 [row capacity, 2816]
   const float *alpha1, *alpha2, *in_scale_q2;
 };
-// On a sorted plan and a quantised input; plan.tile_ready (by expert here) and plan.front_sync zero on
+// On a sorted plan and a quantised input; plan.tile_ready (by expert here) and plan.stream_sync zero on
 // entry and on exit.
 void launch_stream_experts(const StreamOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
 // With the route sort and the input quantiser inside, where stream_layer_fits.

@@ -17,8 +17,10 @@
 
 #if defined(__CUDACC__)
 #define GV_HD __host__ __device__ __forceinline__
+#define GV_HD_MEMBER __host__ __device__ __forceinline__
 #else
 #define GV_HD static inline
+#define GV_HD_MEMBER inline
 #endif
 
 #if defined(__CUDA_ARCH__)

@@ -18,6 +18,7 @@
 #include "gv_common.cuh"
 #include "gv_launchers.h"
 #include "gv_scratch.h"
+#include "gv_stream_schedule.h"
 
 namespace {
 
@@ -220,7 +221,7 @@ int make_scratch(int tokens, Scratch** out) {
   s->plan.chunk_hist = carve(chunks * kExperts);
   s->plan.status = carve(1);
   s->plan.sync = carve(2);  // taken from the 64 spare ints; zero like everything else here
-  s->plan.front_sync = carve(2);  // likewise
+  s->plan.stream_sync = carve(gv::kStreamSyncInts);
   *out = s;
   return GEVVA_MOE_OK;
 }

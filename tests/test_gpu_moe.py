@@ -717,6 +717,60 @@ def test_streaming_front_first_items(gm, weights, cuda_device, tokens, monkeypat
     assert outs[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("first,second", [(64, 64), (200, 16), (400, 300)])
+def test_streaming_launches_on_two_streams(gm, weights, cuda_device, first, second):
+    """Runners with scratch of their own may run on streams of their own, also of different priority: of two streaming
+    launches, whose CTAs wait for one another, neither may keep the other from ending with half of the SMs each."""
+    cases = []
+    for tokens, priority in ((first, 0), (second, -1)):
+        x = hashgen.activations(tokens, HIDDEN, 15 + priority, cuda_device)
+        ids = torch.from_numpy(random_ids(tokens, 16 + priority)).to(cuda_device)
+        rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        want = torch.zeros_like(x)
+        runner.launch_batch(x, ids, rw, want, tokens)
+        runner.check()
+        cases.append((runner, x, ids, rw, want, torch.zeros_like(x), torch.cuda.Stream(device=cuda_device, priority=priority)))
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for runner, x, ids, rw, _, out, stream in cases:
+            runner.launch_batch(x, ids, rw, out, x.shape[0], stream=stream)
+    torch.cuda.synchronize()
+    for runner, _, _, _, want, out, _ in cases:
+        runner.check()
+        assert torch.equal(want, out)
+
+
+@pytest.mark.parametrize("tokens", [1, 13, 128, 296, 500])
+def test_streaming_launch_beside_a_prefill(gm, weights, cuda_device, tokens):
+    """A streaming launch whose CTAs start one by one, as those of a large batch on another stream give up their SMs:
+    items and tokens of CTAs that have not started are done by those that have, and the bits stay."""
+    x = hashgen.activations(tokens, HIDDEN, 18, cuda_device)
+    ids = torch.from_numpy(random_ids(tokens, 19)).to(cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+    want = torch.zeros_like(x)
+    runner.launch_batch(x, ids, rw, want, tokens)
+    runner.check()
+    large = 8192
+    big_x = hashgen.activations(large, HIDDEN, 20, cuda_device)
+    big_ids = torch.from_numpy(skewed_ids(large)).to(cuda_device)
+    big_rw = torch.full((large, TOP_K), 0.125, device=cuda_device)
+    big_out = torch.empty_like(big_x)
+    big = gm.Nvfp4ExpertRunner(weights[0], large)
+    other = torch.cuda.Stream(device=cuda_device, priority=-1)
+    torch.cuda.synchronize()
+    outs = [torch.zeros_like(x) for _ in range(16)]
+    for step, out in enumerate(outs):
+        if step % 4 == 0:
+            big.launch_batch(big_x, big_ids, big_rw, big_out, large, stream=other)
+        runner.launch_batch(x, ids, rw, out, tokens)
+    torch.cuda.synchronize()
+    runner.check()
+    big.check()
+    assert all(torch.equal(want, out) for out in outs)
+
+
 @pytest.mark.parametrize("tokens", [147, 149, 296, 297])
 def test_streaming_front_with_two_tokens_an_sm(gm, weights, cuda_device, tokens, monkeypatch):
     """Sort and quantiser inside the streaming launch where some CTAs prepare two tokens and others one

@@ -1,0 +1,24 @@
+"""The streaming kernel's items are shared out so that a running CTA never waits for one that has not started, as
+happens when another stream holds a part of the SMs (host form of csrc/gv_stream_schedule.h)."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def probe(tmp_path_factory):
+    binary = str(tmp_path_factory.mktemp("schedule") / "probe")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-o", binary,
+                    os.path.join(ROOT, "tests", "stream_schedule_probe.cpp")], check=True)
+    return binary
+
+
+@pytest.mark.parametrize("chunks", [1, 8, 27, 128, 148, 160, 256])
+@pytest.mark.parametrize("ctas,running", [(148, 148), (148, 147), (148, 74), (148, 1), (132, 16), (1, 1)])
+def test_no_wait_on_a_cta_that_is_not_running(probe, chunks, ctas, running):
+    for seed in range(3):
+        result = subprocess.run([probe, str(chunks), str(ctas), str(running), str(seed)], capture_output=True, text=True)
+        assert result.stdout.strip() == "ok", (chunks, ctas, running, seed, result.stdout)
