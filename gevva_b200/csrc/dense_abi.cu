@@ -249,8 +249,9 @@ int gevva_ff_layer_launch(const gevva_ff_layer* layer, const void* hidden, void*
   if (!layer || !layer->dense_pre || !layer->expert_pre || !layer->router_scale || !layer->router_weight ||
       !layer->expert_scale || !layer->dense_post || !layer->expert_post || !layer->combined_post ||
       !layer->layer_scalar || !layer->experts || !layer->dense || !hidden || !out || !workspace ||
-      (reinterpret_cast<uintptr_t>(workspace) & 255) || tokens < 1 || tokens > layer->dense->max_tokens)
-    return GEVVA_MOE_BAD_ARGUMENT;
+      (reinterpret_cast<uintptr_t>(workspace) & 255) || (reinterpret_cast<uintptr_t>(layer->router_weight) & 15) ||
+      tokens < 1 || tokens > layer->dense->max_tokens || tokens > gv::moe_max_tokens(layer->experts))
+    return GEVVA_MOE_BAD_ARGUMENT;  // (what the parts would refuse, before the first of them is launched)
   const LayerWorkspace w(workspace, tokens);
   gevva_dense* dense = layer->dense;
   const bool beside = aux_stream != stream;

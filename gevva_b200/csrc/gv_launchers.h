@@ -18,6 +18,7 @@ int moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, cons
 int dense_launch_on(gevva_dense* dense, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
                     int sm_count);
 int moe_sm_count(const gevva_moe* runner);
+int moe_max_tokens(const gevva_moe* runner);
 
 // Device-resident description of one launch's routing, written by the route sort
 // and read by every later stage without a host round trip.

@@ -295,6 +295,7 @@ struct StageRange {
 }  // namespace
 
 int gv::moe_sm_count(const gevva_moe* runner) { return runner->sm_count; }
+int gv::moe_max_tokens(const gevva_moe* runner) { return runner->scratch->max_tokens; }
 
 int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, const float* route_weights, void* out,
                              int tokens, unsigned stages, cudaStream_t stream, int sm_count) {

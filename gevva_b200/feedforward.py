@@ -6,7 +6,7 @@ from dataclasses import dataclass
 
 import torch
 
-from .runtime import (HIDDEN, GevvaMoeError, Nvfp4ExpertRunner, _address, _check, _enqueue, _ptr, _stream_handle,
+from .runtime import (EXPERTS, HIDDEN, GevvaMoeError, Nvfp4ExpertRunner, _address, _check, _enqueue, _ptr, _stream_handle,
                       _view, library)
 
 DENSE = 2112
@@ -154,6 +154,8 @@ class FeedForwardLayer:
         Python they took 137 us of host time a layer, four times what the GPU needs for one token."""
         tokens = hidden.shape[0]
         _check(hidden, torch.bfloat16, (tokens, HIDDEN), "input")
+        _check(self.router_w, torch.bfloat16, (EXPERTS, HIDDEN), "router_weight")
+        _check(self.expert_scale, torch.bfloat16, (EXPERTS,), "expert_scale")
         lib = _lib()
         out = torch.empty_like(hidden)
         workspace = torch.empty(lib.gevva_ff_layer_workspace_bytes(tokens), dtype=torch.uint8, device=hidden.device)

@@ -1,0 +1,147 @@
+"""Which kernels a call launches, without a GPU: the library's sources compiled over a CUDA runtime that records
+launches instead of making them (launch_recorder.cpp)."""
+import ctypes
+import os
+import re
+import shutil
+import subprocess
+from concurrent.futures import ThreadPoolExecutor
+
+import pytest
+import torch
+
+from gevva_b200 import build
+from gevva_b200 import feedforward as ff
+from gevva_b200 import runtime as rt
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+NVCC = shutil.which(build.NVCC)
+STREAM, AUX_STREAM = 64, 65
+ADDRESS = 4096  # stands for every pointer that the recording runtime does not follow
+
+
+def kernel_name(mangled):
+    """The function's own name, followed by <0> or <1> where its first template argument is a bool."""
+    for digits in re.finditer(r"\d+", mangled):
+        for start in range(digits.start(), digits.end()):
+            length = int(mangled[start : digits.end()])
+            name = mangled[digits.end() : digits.end() + length]
+            if len(name) == length and name.endswith("_kernel"):
+                flag = re.match(r"ILb([01])E", mangled[digits.end() + length :])
+                return name + (f"<{flag[1]}>" if flag else "")
+    return mangled
+
+
+class Recorder:
+    def __init__(self, path):
+        self.lib = lib = ctypes.CDLL(path)
+        lib.recorder_take_log.restype = ctypes.c_char_p
+        vp, i32 = ctypes.c_void_p, ctypes.c_int
+        lib.gevva_moe_create.argtypes = [ctypes.POINTER(vp), ctypes.POINTER(rt._Weights), i32, vp, ctypes.POINTER(rt._Options)]
+        lib.gevva_moe_destroy.argtypes = [vp]
+        lib.gevva_moe_launch_stages.argtypes = [vp, vp, vp, vp, vp, i32, ctypes.c_uint, vp]
+        lib.gevva_dense_create.argtypes = [ctypes.POINTER(vp), ctypes.POINTER(ff._DenseWeights), i32]
+        lib.gevva_dense_destroy.argtypes = [vp]
+        lib.gevva_ff_layer_launch.argtypes = [ctypes.POINTER(ff._Layer), vp, vp, vp, i32, vp, vp]
+
+    def runner(self, max_tokens, flags=0):
+        handle = ctypes.c_void_p()
+        assert self.lib.gevva_moe_create(ctypes.byref(handle), ctypes.byref(rt._Weights(*[ADDRESS] * 8)), max_tokens, None,
+                                         ctypes.byref(rt._Options(flags))) == 0
+        self.launches()
+        return handle
+
+    def dense(self, max_tokens):
+        handle = ctypes.c_void_p()
+        assert self.lib.gevva_dense_create(ctypes.byref(handle), ctypes.byref(ff._DenseWeights(ADDRESS, ADDRESS, 1, 1, 1)),
+                                           max_tokens) == 0
+        self.launches()
+        return handle
+
+    def launches(self):
+        """The launches since the last call: dicts with the kernel's name and the launch's attributes."""
+        out = []
+        for line in self.lib.recorder_take_log().decode().splitlines():
+            mangled, rest = line.split(" ", 1)
+            out.append({key: int(value) for key, value in re.findall(r"(\w+)=(\d+)", rest)})
+            out[-1]["kernel"] = kernel_name(mangled)
+        return out
+
+    def layer(self, runner, tokens, stages=rt.STAGE_ALL):
+        assert self.lib.gevva_moe_launch_stages(runner, ADDRESS, ADDRESS, ADDRESS, ADDRESS, tokens, stages, STREAM) == 0
+        return self.launches()
+
+
+@pytest.fixture(scope="module")
+def recorder(tmp_path_factory):
+    if NVCC is None:
+        pytest.skip("needs nvcc")
+    folder = tmp_path_factory.mktemp("recorder")
+
+    def compile_one(source):
+        target = str(folder / (os.path.splitext(os.path.basename(source))[0] + ".o"))
+        # PTX only: the device code is not run
+        subprocess.run([NVCC, "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=compute_100a", "-Xcompiler", "-fPIC",
+                        "-c", "-o", target, source], check=True, capture_output=True)
+        return target
+
+    sources = [os.path.join(build.CSRC, s) for s in build.SOURCES if s.endswith(".cu")]
+    with ThreadPoolExecutor(os.cpu_count()) as pool:
+        objects = list(pool.map(compile_one, sources + [os.path.join(ROOT, "tests", "launch_recorder.cpp")]))
+    library = str(folder / "librecorder.so")
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", library] + objects + ["-ldl"], check=True, capture_output=True)
+    return Recorder(library)
+
+
+def kernels(launches):
+    return [launch["kernel"] for launch in launches]
+
+
+def layer_launch(recorder, runner, dense, tokens, router_weight=ADDRESS, workspace=ADDRESS):
+    layer = ff._Layer(*[ADDRESS] * 9, runner, dense)
+    layer.router_weight = router_weight
+    return recorder.lib.gevva_ff_layer_launch(ctypes.byref(layer), ADDRESS, ADDRESS, workspace, tokens, STREAM, AUX_STREAM)
+
+
+def test_feed_forward_layer_launches(recorder):
+    runner, dense = recorder.runner(64), recorder.dense(64)
+    assert layer_launch(recorder, runner, dense, 64) == 0
+    launches = recorder.launches()
+    assert kernels([l for l in launches if l["stream"] == AUX_STREAM]) == [
+        "fp8_quantize_rows_kernel", "grouped_nvfp4_gemm_kernel", "gelu_quantize_fp8_kernel", "grouped_nvfp4_gemm_kernel"]
+    assert kernels([l for l in launches if l["stream"] == STREAM]) == [
+        "ff_prepare_kernel", "route_project_kernel<0>", "stream_experts_kernel<1>", "ff_finalize_kernel"]
+
+
+@pytest.mark.parametrize("capacity,dense_capacity,tokens,router_weight", [(4, 64, 5, ADDRESS), (64, 4, 5, ADDRESS),
+                                                                         (64, 64, 0, ADDRESS), (64, 64, 5, ADDRESS + 8)])
+def test_feed_forward_layer_refuses_before_it_launches(recorder, capacity, dense_capacity, tokens, router_weight):
+    """A call that one of its parts would refuse launches nothing: neither of the parts in front of it, on either stream."""
+    runner, dense = recorder.runner(capacity), recorder.dense(dense_capacity)
+    assert layer_launch(recorder, runner, dense, tokens, router_weight) == -3  # GEVVA_MOE_BAD_ARGUMENT
+    assert recorder.launches() == []
+
+
+class _Cuda:
+    """What forward() checks of a tensor."""
+    is_cuda = True
+    device = "cuda:0"
+
+    def __init__(self, shape, dtype, contiguous=True):
+        self.shape, self.dtype, self._contiguous = torch.Size(shape), dtype, contiguous
+
+    def is_contiguous(self):
+        return self._contiguous
+
+
+@pytest.mark.parametrize("router_w,expert_scale", [
+    (_Cuda((128, 2816), torch.uint8), None), (_Cuda((128, 2816), torch.float32), None),
+    (_Cuda((64, 2816), torch.bfloat16), None), (_Cuda((128, 2816), torch.bfloat16, False), None),
+    (None, _Cuda((128,), torch.float32)), (None, _Cuda((64,), torch.bfloat16))])
+def test_feed_forward_layer_checks_its_router(router_w, expert_scale):
+    """forward() hands addresses to one native call, so what route_project() would refuse it has to refuse itself."""
+    router_w = router_w or _Cuda((128, 2816), torch.bfloat16)
+    expert_scale = expert_scale or _Cuda((128,), torch.bfloat16)
+    layer = ff.FeedForwardLayer(*[None] * 3, router_w, expert_scale, *[None] * 6)
+    with pytest.raises(ValueError, match="router_weight|expert_scale"):
+        layer.forward(_Cuda((3, 2816), torch.bfloat16))
