@@ -317,8 +317,10 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   // also takes in the sort and the quantiser and is 5 to 10 us faster).  A skewed router gives a few experts many 64-row
   // chunks, each with the whole of the weights: Zipf, 400 tokens 90.8 / 87.6, 613 110.8 / 105.2, 800 124.8 / 110.1.  The host
   // does not know the routes, so the line lies where the one gains what the other loses.
-  const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !runner->pairs &&
-                       !runner->w13_pair_form && tokens <= kStreamTokens;
+  // (The pair options leave batches of at most 128 tokens alone.)
+  const bool pair_options = (runner->pairs || runner->w13_pair_form) && tokens > gv::kFusedSortQuantizeMaxTokens;
+  const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !pair_options &&
+                       tokens <= kStreamTokens;
   if ((stages & layer_body) == layer_body && streams && runner->decode_front && gv::stream_layer_fits(tokens, sm_count)) {
     // ... and the route sort and the quantiser; the weights stream while the input is being quantised
     StageRange range(runner->nvtx, "gevva_moe.sort+quantize+w13+geglu+w2");

@@ -97,6 +97,24 @@ def kernels(launches):
     return [launch["kernel"] for launch in launches]
 
 
+@pytest.mark.parametrize("flags", [0, rt.OPTION_PAIRS, rt.OPTION_W13_PAIRS])
+@pytest.mark.parametrize("tokens", [1, 64, 128, 129, 296, 297, 640, 641])
+def test_kernels_of_a_layer(recorder, flags, tokens):
+    """The pair options are for batches of more than 128 tokens; smaller ones run as without them."""
+    runner = recorder.runner(1024, flags)
+    got = kernels(recorder.layer(runner, tokens))
+    plain_front = ["route_sort_fused_kernel", "quantize_input_kernel<1>"]
+    if tokens <= 128 or (flags == 0 and tokens <= 296):
+        assert got == ["stream_experts_kernel<1>", "reduce_routes_kernel<0>"]
+    elif flags == 0 and tokens <= 640:
+        assert got == plain_front + ["stream_experts_kernel<0>", "reduce_routes_kernel<0>"]
+    elif flags == rt.OPTION_PAIRS:
+        assert got == plain_front + ["grouped_nvfp4_gemm_pair_kernel"] * 2 + ["reduce_routes_kernel<0>"]
+    else:
+        assert got == plain_front + ["w13_geglu_pair_kernel", "grouped_down_kernel", "reduce_routes_kernel<1>"]
+    recorder.lib.gevva_moe_destroy(runner)
+
+
 def layer_launch(recorder, runner, dense, tokens, router_weight=ADDRESS, workspace=ADDRESS):
     layer = ff._Layer(*[ADDRESS] * 9, runner, dense)
     layer.router_weight = router_weight
