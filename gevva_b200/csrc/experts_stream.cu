@@ -1033,7 +1033,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
           }
           float most = fmaxf(b ? maximum[1] : maximum[0], __shfl_xor_sync(0xffffffffu, b ? maximum[0] : maximum[1], 4));
           most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 2));
-          most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 1));
+          most = fmaxf(fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 1)), 0.0f);  // (a block of NaN has scale zero)
           const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, most)));
           const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, smem->tables.reciprocals)
                                                                    : scale_inverse_divided(multiplier, scale);

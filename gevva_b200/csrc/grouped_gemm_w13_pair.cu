@@ -504,7 +504,8 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           const float received = __shfl_xor_sync(0xffffffffu, b ? most[k] : most[k + 2], 8);
           most[k] = fmaxf(b ? most[k + 2] : most[k], received);
         }
-        const float maximum = fmaxf(c ? most[1] : most[0], __shfl_xor_sync(0xffffffffu, c ? most[0] : most[1], 4));
+        // (a block of NaN has scale zero)
+        const float maximum = fmaxf(fmaxf(c ? most[1] : most[0], __shfl_xor_sync(0xffffffffu, c ? most[0] : most[1], 4)), 0.0f);
         const uint32_t scale = encode_e4m3(gv_sixth(__fmul_rn(multiplier, maximum)));
         const float inverse = gv_scale_inverse_exact(multiplier) ? gv_scale_inverse(multiplier, scale, smem->tables.reciprocals)
                                                                  : scale_inverse_divided(multiplier, scale);

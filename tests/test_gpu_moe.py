@@ -717,6 +717,36 @@ def test_streaming_front_first_items(gm, weights, cuda_device, tokens, monkeypat
     assert outs[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("kind", ["nan", "inf", "magnitudes"])
+@pytest.mark.parametrize("tokens,form", [(8, ""), (200, ""), (400, ""), (200, "two launches"), (200, "w13_pairs"), (700, "")])
+def test_fused_w13_of_special_values(gm, weights, cuda_device, tokens, form, kind, monkeypatch):
+    """Every fused form of the w13 stage against the separate GeGLU and quantiser, on outputs that random weights do not
+    give: blocks that are NaN throughout (their scale is zero, as in the oracle: NaN does not count towards a maximum) or
+    hold infinities, and gates of every bf16 magnitude from 2^-27 to 2^7, below and above the erf table too."""
+    from gevva_b200 import runtime as rt
+    base = weights[0]
+    index = torch.arange(EXPERTS, device=cuda_device)
+    alpha1, scale_q2 = base.alpha1.clone(), base.in_scale_q2.clone()
+    if kind == "magnitudes":
+        factor = torch.exp2((index % 27 - 20).float())
+        alpha1 *= factor
+        scale_q2 /= factor * factor
+    else:
+        alpha1[index % 3 == 0] = float(kind)
+    w = gm.ExpertWeights(base.w13, base.w13_sf, base.w2, base.w2_sf, alpha1, base.alpha2, base.in_scale_q1, scale_q2)
+    x = hashgen.activations(tokens, HIDDEN, 21, cuda_device)
+    ids = torch.from_numpy(random_ids(tokens, 22)).to(cuda_device)
+    monkeypatch.setenv("GEVVA_MOE_DECODE_MERGED", "0" if form == "two launches" else "1")
+    records = []
+    for stages in (rt.STAGE_ALL & ~rt.STAGE_REDUCE | rt.STAGE_UNFUSED, rt.STAGE_ALL & ~rt.STAGE_REDUCE):
+        runner = gm.Nvfp4ExpertRunner(w, tokens, w13_pairs=form == "w13_pairs")
+        runner.launch_stages(stages, tokens, input=x, expert_ids=ids)
+        runner.check()
+        records.append([runner.buffer(b).clone() for b in (rt.BUF_INTER_SF, rt.BUF_INTER_CODES, rt.BUF_W2_OUT)])
+    for name, a, b in zip(("scales", "codes", "routed rows"), *records):
+        assert torch.equal(a, b), f"{name}: {(a != b).sum().item()} bytes differ"
+
+
 @pytest.mark.parametrize("first,second", [(64, 64), (200, 16), (400, 300)])
 def test_streaming_launches_on_two_streams(gm, weights, cuda_device, first, second):
     """Runners with scratch of their own may run on streams of their own, also of different priority: of two streaming
