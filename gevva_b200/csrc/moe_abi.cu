@@ -273,6 +273,8 @@ struct gevva_moe {
   uint8_t* w2_sf_down = nullptr;    // re-tiling of weights.w2_sf in the column order of grouped_gemm_down.cu
   gv::StreamOperands stream_experts{};  // few rows an expert: both GEMMs in one launch, weights on the MMA's M side
   bool w13_pair_form = false;       // GEVVA_MOE_OPTION_W13_PAIRS, or GEVVA_MOE_W13_PAIRS=1 for a whole process
+  bool w13_single = false;          // GEVVA_MOE_W13_PAIRS=0: the fused w13 of large batches by the one-CTA kernel, which
+                                    // expert-parallel ranks use (to compare the two)
   int sm_count = 0;
   bool pairs = false;               // GEVVA_MOE_OPTION_PAIRS: prefill-sized launches run the expert GEMMs as CTA pairs
   bool decode_front = true;         // ... and the route sort and the input quantiser in the same launch (GEVVA_MOE_DECODE_FRONT=0: a launch of their own)
@@ -347,7 +349,7 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
   // Weights on the MMA's M side, by CTA pairs: faster than (2048 tokens on) or as fast as the one-CTA tile kernel
   // wherever a batch does not stream (figures in grouped_gemm_w13_pair.cu).
-  const bool w13_by_pairs = !use_pairs && sm_count >= 2 &&
+  const bool w13_by_pairs = !use_pairs && sm_count >= 2 && !runner->w13_single &&
                             (tokens > kStreamTokens || (runner->w13_pair_form && tokens > gv::kFusedSortQuantizeMaxTokens));
   if ((stages & gemms) == gemms && streams) {
     StageRange range(runner->nvtx, "gevva_moe.w13+geglu+w2");
@@ -528,6 +530,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   }
   const char* w13_pairs_env = std::getenv("GEVVA_MOE_W13_PAIRS");
   m->w13_pair_form = (options && (options->flags & GEVVA_MOE_OPTION_W13_PAIRS)) || (w13_pairs_env && w13_pairs_env[0] == '1');
+  m->w13_single = !m->w13_pair_form && w13_pairs_env && w13_pairs_env[0] == '0';
   {
     const cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
     if (e != cudaSuccess) {

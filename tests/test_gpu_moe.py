@@ -509,10 +509,12 @@ def test_against_committed_golden_vectors(gm, packed, weights, cuda_device):
 
 
 @pytest.mark.parametrize("tokens,kind", [(130, "random"), (300, "skewed"), (4096, "random")])
-def test_cta_pair_gemms_equal_the_single_cta_gemms(gm, weights, cuda_device, tokens, kind):
+def test_cta_pair_gemms_equal_the_single_cta_gemms(gm, weights, cuda_device, tokens, kind, monkeypatch):
     """The two expert GEMMs run by CTA pairs (tcgen05 cta_group::2: two row tiles of an expert
     against shared weight rows, odd last tiles alone in their pair) give the bits of the
     one-CTA-per-tile kernels: w2 operand codes and scales, routed rows, layer output."""
+    monkeypatch.setenv("GEVVA_MOE_DECODE_MERGED", "0")
+    monkeypatch.setenv("GEVVA_MOE_W13_PAIRS", "0")
     from gevva_b200 import runtime as rt
     ids = random_ids(tokens, 5) if kind == "random" else skewed_ids(tokens)
     x = hashgen.activations(tokens, HIDDEN, 71, cuda_device)
@@ -572,10 +574,11 @@ def test_large_batches_at_tile_and_chunk_edges(gm, weights, cuda_device, tokens,
 
 @pytest.mark.parametrize("tokens,kind", [(129, "random"), (130, "skewed"), (300, "skewed"), (777, "random"),
                                          (4096, "random")])
-def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_device, tokens, kind):
-    """The fused w13 stage run by CTA pairs with the weights on the MMA's M side and up to 256 rows of
+def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_device, tokens, kind, monkeypatch):
+    """The fused w13 stage run by CTA pairs with the weights on the MMA's M side and up to 208 rows of
     an expert on its N side (any multiple of 16) writes the same w2 operand codes and scale bytes as
-    the one-CTA-per-tile kernel, and the layer output follows."""
+    the one-CTA-per-tile kernel (in its short and, with more than eight rounds of items, its long order),
+    and the layer output follows."""
     from gevva_b200 import runtime as rt
     ids = random_ids(tokens, 23) if kind == "random" else skewed_ids(tokens)
     x = hashgen.activations(tokens, HIDDEN, 79, cuda_device)
@@ -583,8 +586,10 @@ def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_devic
     rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
     routes = tokens * TOP_K
     results = []
-    for form in (False, True):
-        runner = gm.Nvfp4ExpertRunner(weights[0], tokens, w13_pairs=form)
+    monkeypatch.setenv("GEVVA_MOE_DECODE_MERGED", "0")
+    for form in ("0", "1"):
+        monkeypatch.setenv("GEVVA_MOE_W13_PAIRS", form)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
         out = torch.empty_like(x)
         runner.buffer(rt.BUF_INTER_CODES).zero_()
         runner.buffer(rt.BUF_INTER_SF).zero_()
@@ -604,9 +609,9 @@ def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_devic
 @pytest.mark.parametrize("tokens,kind", [(1, "random"), (8, "random"), (40, "skewed"), (64, "random"),
                                          (128, "skewed")])
 def test_merged_decode_launch_equals_two_launches(gm, weights, cuda_device, tokens, kind, monkeypatch):
-    """Batches of at most 128 tokens run both expert GEMMs in one persistent launch (w2 items wait
-    on per-tile readiness counters); the bits must be those of the two separate launches, also when
-    the launch is repeated on the same scratch (the counters are reset by the sort)."""
+    """Decode batches run both expert GEMMs in one persistent launch (w2 items wait on their expert's
+    readiness counter); the bits must be those of the two separate launches, also when the launch is
+    repeated on the same scratch (the CTA that finishes last puts the counters back)."""
     from gevva_b200 import runtime as rt
     ids = random_ids(tokens, 17) if kind == "random" else skewed_ids(tokens)
     x = hashgen.activations(tokens, HIDDEN, 73, cuda_device)
@@ -630,7 +635,7 @@ def test_merged_decode_launch_equals_two_launches(gm, weights, cuda_device, toke
 
 
 def test_decode_kernel_that_sorts_and_quantises_itself(gm, weights, cuda_device, monkeypatch):
-    """Batches of at most 128 tokens sort their routes and quantise their input inside the merged
+    """Batches of at most two tokens an SM sort their routes and quantise their input inside the merged
     expert launch.  Against a runner that keeps the sort + quantise launch of its own
     (GEVVA_MOE_DECODE_FRONT=0): the same route plan, operand bytes, routed rows and output, over a
     sequence of batch sizes on one runner (the launch puts its counters back itself), and an expert

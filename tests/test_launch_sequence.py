@@ -115,6 +115,16 @@ def test_kernels_of_a_layer(recorder, flags, tokens):
     recorder.lib.gevva_moe_destroy(runner)
 
 
+@pytest.mark.parametrize("tokens", [129, 641, 1024])
+def test_switches_give_the_one_cta_kernels(recorder, monkeypatch, tokens):
+    """What the other forms of the two GEMMs are compared with bit by bit."""
+    monkeypatch.setenv("GEVVA_MOE_DECODE_MERGED", "0")
+    monkeypatch.setenv("GEVVA_MOE_W13_PAIRS", "0")
+    runner = recorder.runner(1024)
+    assert kernels(recorder.layer(runner, tokens))[2:4] == ["grouped_nvfp4_gemm_kernel", "grouped_down_kernel"]
+    recorder.lib.gevva_moe_destroy(runner)
+
+
 def layer_launch(recorder, runner, dense, tokens, router_weight=ADDRESS, workspace=ADDRESS):
     layer = ff._Layer(*[ADDRESS] * 9, runner, dense)
     layer.router_weight = router_weight
