@@ -37,7 +37,8 @@ struct gevva_dense {
 // as its busiest CTA has, and a wide item takes about one and a half times a narrow one (48 KB of operands a K
 // block against 32 KB): wide where that is no longer.  Alone on 148 SMs the MLP takes (us, narrow -> wide)
 // 31.9 -> 35.4 at 301 tokens, where one wave of narrow items is enough, 39.0 -> 35.5 at 600, 74.8 -> 62.6 at 2048
-// and 131.9 -> 108.4 at 4096; on the 16 SMs it gets beside the experts wide is as good or better from 129 tokens on.
+// and 131.9 -> 108.4 at 4096.  On the few SMs that it gets beside the experts of a decode batch (whole layers in a graph):
+// 57.5 -> 53.7 at 8 tokens, 71.6 -> 71.8 at 16, 91.4 -> 91.9 at 40, 95.9 -> 95.7 at 64, 104.1 -> 103.2 at 128.
 static bool wide_items(int tokens, int n_out, int sms) {
   const int row_tiles = (tokens + gv::kTileM - 1) / gv::kTileM;
   const int narrow = (row_tiles * ((n_out + 127) / 128) + sms - 1) / sms;
@@ -236,6 +237,8 @@ struct LayerWorkspace {
 // weight rows in one wave, 17 those of 256 (whole layers in a graph, us, at 16 / 17 / 33 / 48 SMs: 1 token 46.4 / 38.9 / 34.4 /
 // 32.3, 4 tokens 52.8 / 45.0 / 44.2 / 43.4, 5 tokens 55.5 / 47.7 / 44.9 / 47.2, 8 tokens 60.5 / 52.1 / 54.2 / 57.4, 12 tokens
 // 62.7 / 62.3 / 64.2 / 68.1, 40 tokens 93.6 / 94.6 / 99.6 / -, 128 tokens 107.4 / 108.4 / 109.9 / -).
+// (48 and 16 SMs are the table's, not a matter of waves.)
+constexpr int kBesideTokens = 128;  // the range of the table; above it both sides take all SMs (sharing was not measured there)
 int dense_sms_beside(int tokens, int sms) {
   const int wanted = tokens <= 4 ? 48 : tokens <= 6 ? 33 : tokens <= 12 ? 17 : 16;
   return wanted * 2 < sms ? wanted : sms / 2;
@@ -258,7 +261,7 @@ int gevva_ff_layer_launch(const gevva_ff_layer* layer, const void* hidden, void*
   // The dense MLP starts as soon as its input exists, on SMs that the router leaves idle; beside a
   // decode-sized expert launch on SMs of its own.
   const int sms = gv::moe_sm_count(layer->experts);
-  const bool split = beside && tokens <= gv::kFusedSortQuantizeMaxTokens && sms > 1;
+  const bool split = beside && tokens <= kBesideTokens && sms > 1;
   const int dense_sms = split ? dense_sms_beside(tokens, sms) : sms;
   const int expert_sms = split ? sms - dense_sms : sms;
   gv::launch_ff_prepare(hidden, layer->dense_pre, layer->expert_pre, layer->router_scale, w.dense_in, w.expert_in,

@@ -45,6 +45,7 @@ constexpr int kWpAccStages = 2;
 // One K block's scales, per MMA j: weights at +12j, the chunk's two 128-row blocks at +12j+4 and +12j+8.
 constexpr uint32_t kWpSfColumn = kWpAccStages * kWpRows;
 static_assert(kWpSfColumn + 48 <= kWpTmemColumns, "tensor memory budget");
+static_assert(kWpRows / 2 == 8 * kW13PairBoxes, "a box for each half of a chunk");
 constexpr int kWpTokenBytes = kWpRows / 2 * kTileKBytes;  // 13 KiB
 constexpr int kWpTileBytes = 128 * kTileKBytes;  // 16 KiB
 constexpr int kWpUnits = kInter / 64;            // 11
@@ -107,7 +108,7 @@ __device__ __forceinline__ void wp_load_3d(void* smem_dst, const void* tensor_ma
       : "memory");
 }
 
-// The 128 weight rows of a unit in the kernel's order: see make_w13_fragment_tensor_map.
+// The 128 weight rows of a unit in the kernel's order: see make_w13_fragment_map (moe_abi.cu).
 __device__ __forceinline__ void wp_load_weights(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int block) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
@@ -178,7 +179,7 @@ struct WpItem {
   int shift;     // tensor-memory columns (of 32 rows) by which the chunk starts inside that tile: 0 or 2
   int local;     // first row of the chunk within the expert
   int row0;      // first sorted row of the chunk
-  int valid;     // rows of the chunk, 1..224
+  int valid;     // rows of the chunk, 1..208
   int n;         // MMA N: valid rounded up to 16
   int unit_pair; // 0..5
 };
@@ -216,7 +217,7 @@ __device__ __forceinline__ bool wp_item(const WpSmem* smem, int round, WpItem& i
 }
 
 struct WpTokenMaps {
-  CUtensorMap rows[16];   // boxes of 8, 16, ... 128 token rows x 128 bytes
+  CUtensorMap rows[kW13PairBoxes];   // boxes of 8, 16, ... 104 token rows x 128 bytes
 };
 
 struct WpParams {
@@ -436,7 +437,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
       WpItem item;
       if (!wp_item(smem, round, item)) continue;
       const int unit = 2 * item.unit_pair + static_cast<int>(rank);
-      const int steps = unit < kWpUnits ? (item.valid + 31) >> 5 : 0;  // of 32 tokens, dealt to the four warps of a block
+      const int steps = unit < kWpUnits ? (item.valid + 31) >> 5 : 0;  // of 32 tokens, dealt to the two warps of a block
       const float alpha = p.alpha[item.expert];
       const float multiplier = p.next_scale_q[item.expert];
       if (!__all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, p.status))) break;
@@ -635,7 +636,7 @@ void launch_w13_pairs(const W13PairOperands& op, const RoutePlan& plan, int sm_c
   config.attrs = attributes;
   config.numAttrs = op.serial_launch ? 1 : 2;
   WpTokenMaps token_maps;
-  for (int i = 0; i < 16; ++i) token_maps.rows[i] = op.map_x[i];
+  for (int i = 0; i < kW13PairBoxes; ++i) token_maps.rows[i] = op.map_x[i];
   cudaLaunchKernelEx(&config, w13_geglu_pair_kernel, token_maps, op.map_w, op.map_x_sf, op.map_w_sf, p);
 }
 

@@ -149,8 +149,9 @@ int prepare_grouped_gemm_pairs();
 
 // Fused w13 + GeGLU + requantise run by CTA pairs with the weights on the MMA's M side and up to
 // 208 rows of one expert on its N side (grouped_gemm_w13_pair.cu).
+constexpr int kW13PairBoxes = 13;
 struct W13PairOperands {
-  CUtensorMap map_x[16];  // activation codes [row capacity, 1408] bytes through boxes of 8, 16, ... 128 rows x 128 B
+  CUtensorMap map_x[kW13PairBoxes];  // activation codes [row capacity, 1408] bytes through boxes of 8, 16, ... 104 rows x 128 B
   CUtensorMap map_w;      // w13 codes in the row order of its MMAs, a unit of 64 columns (up and gate rows) a copy
   CUtensorMap map_x_sf;   // activation scale regions as [128-row blocks, 44 atoms, 512 B], box 2 blocks x 4 atoms
   CUtensorMap map_w_sf;   // unit-tiled weight scales (launch_retile_w13_unit_scales), box of four atoms
@@ -172,7 +173,7 @@ int prepare_w13_pairs();
 constexpr int kStreamBoxes = 8;         // activation boxes of 8, 16, ... 64 rows
 constexpr int kStreamMaxTokens = 1024;  // the kernel's chunk list; where the launch pays is the caller's rule
 struct StreamOperands {
-  CUtensorMap map_w13;                 // as W13PairOperands::map_w
+  CUtensorMap map_w13;                 // make_w13_unit_tensor_map
   CUtensorMap map_w2;                  // [128 * 2816, 352] bytes, box 128 x 128 B
   CUtensorMap map_up[kStreamBoxes];    // input codes [row capacity, 1408] through boxes of 8(i+1) rows x 128 B
   CUtensorMap map_down[kStreamBoxes];  // w2 operand codes [row capacity, 352] likewise

@@ -314,11 +314,12 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   const unsigned front = GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE;
   const unsigned layer_body = front | GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU | GEVVA_MOE_STAGE_W2;
   // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side does both GEMMs.
-  // Against the two launches, per layer of two distinct ones, us, one B200, uniform routing: 310 tokens 101.8 against 101.1,
-  // 400 102.7 / 103.8, 500 104.5 / 106.9, 613 109.1 / 112.5, 800 113.7 / 116.4, 1000 126.4 / 122.0 (up to 296 tokens it
-  // also takes in the sort and the quantiser and is 5 to 10 us faster).  A skewed router gives a few experts many 64-row
-  // chunks, each with the whole of the weights: Zipf, 400 tokens 90.8 / 87.6, 613 110.8 / 105.2, 800 124.8 / 110.1.  The host
-  // does not know the routes, so the line lies where the one gains what the other loses.
+  // Against the launches of larger batches (w13 by CTA pairs, then w2), us a layer of four distinct ones in a graph, one B200:
+  // router logits without bias, 300 tokens 96.7 against 99.7, 400 98.4 / 101.8, 500 101 / 105.5, 640 108.2 / 112.8 (up to 296
+  // tokens it also takes in the sort and the quantiser); with a bias of deviation 0.5 96.9 / 99.2, 100.3 / 102.4, 106.1 / 104.9,
+  // 114.8 / 112.5; with a Zipf(1.1) bias 83.9 / 84.5, 90.3 / 86.5, 96.4 / 91.2, 110.7 / 103.7: a heavy expert has many 64-row
+  // chunks, each with the whole of its weights.  The host does not know the routes.  The line is that of evenly loaded
+  // experts, for which the launch pays all the way; strongly skewed batches of 400 to 640 tokens lose 4 to 7 us by it.
   // (The pair options leave batches of at most 128 tokens alone.)
   const bool pair_options = (runner->pairs || runner->w13_pair_form) && tokens > gv::kFusedSortQuantizeMaxTokens;
   const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !pair_options &&
@@ -539,7 +540,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
     }
     gv::W13PairOperands& wp = m->w13_pairs;
     ok = true;
-    for (int i = 0; i < 16; ++i)
+    for (int i = 0; i < gv::kW13PairBoxes; ++i)
       ok = ok && make_operand_map(&wp.map_x[i], s->input_codes, rows, kHidden / 2, 8 * (i + 1));
     ok = ok && make_w13_fragment_map(&wp.map_w, weights->w13, kExperts) &&
          make_block_scale_map(&wp.map_x_sf, s->input_sf, s->input_sf_bytes, kHidden / 64) &&

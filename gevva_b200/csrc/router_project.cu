@@ -4,7 +4,7 @@
 // (src/cuda/runtime/prefill.cuh:414-422, :1203-1210: cublasGemmEx / cuBLASLt FP8
 // [tokens,2816] x [128,2816]^T -> bf16 [tokens,128], followed by
 // route_128_top8_kernel<<<tokens,128>>>).  Here both are one kernel and the logits never
-// reach HBM: tokens sit on MMA-M (128 per tile), the 128 experts on MMA-N, K = 2816.
+// reach HBM: tokens sit on MMA-M (64 or 128 per tile), the 128 experts on MMA-N, K = 2816.
 //
 // A tile (of 64 tokens in batches of up to 2048) has its K range split over a cluster of four CTAs (two, or one, for batches whose tiles
 // would otherwise not fit one wave of SMs; eight for batches of at most 512 tokens), so a
@@ -12,11 +12,11 @@
 // eight SMs instead of one.  Each
 // CTA accumulates its K slice in tensor memory (tcgen05.mma kind::f16 for bf16 operands,
 // kind::f8f6f4 for E4M3).  Tile row r belongs to CTA r % split of the cluster: every CTA stores
-// its 128 x 128 fp32 partial sums row by row straight into the owners' shared memory (posted
+// its fp32 partial sums (128 a row) row by row straight into the owners' shared memory (posted
 // st.shared::cluster stores), and after one cluster barrier each owner sums the partials of its
-// 128 / split rows in rank order (a fixed order: results do not depend on timing), adds the optional
-// per-expert bias, rounds to bf16 as the GEMM would have stored it, and routes its rows with four
-// lanes per token (gv_route.cuh).
+// rows (a tile's / split) in rank order (a fixed order: results do not depend on timing), adds the optional
+// per-expert bias, rounds to bf16 as the GEMM would have stored it, and routes its rows (gv_route.cuh): a warp per
+// token where it has at most eight, else four lanes per token.
 //
 // Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer and owner of tensor memory, warps
 // 2..5 epilogue (thread = accumulator row).  Every mbarrier wait is bounded (status word
@@ -270,7 +270,8 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const int tile_rows = p.tokens - m_tile * kRows;   // may exceed the tile
     // rows kSplit * i + rank < tile_rows
     const int own_rows = tile_rows >= kRows ? kOwnRows : (tile_rows - static_cast<int>(rank) + kSplit - 1) / kSplit;
-    if (own_rows <= kWarpRows) {
+    const bool few = kOwnRows <= kWarpRows || own_rows <= kWarpRows;
+    if (few) {
       // a few rows: one warp per row, four logits a lane (a third of the quads' chain)
       for (int row_local = warp - 2; row_local < own_rows; row_local += 4) {
         const int token = m_tile * kRows + row_local * kSplit + static_cast<int>(rank);
@@ -294,13 +295,14 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         route_top8_warp(packed, lane, kFp8, rescale, smem->expert_scale, p.weights + static_cast<size_t>(token) * kTopK,
                         p.ids + static_cast<size_t>(token) * kTopK);
       }
-    } else {
+    }
+    if constexpr (kOwnRows > kWarpRows) if (!few) {
     const int t = threadIdx.x - 64;
     const int part = t & 3;         // columns [32 * part, 32 * part + 32)
 #pragma unroll 1
     for (int pass = 0; pass < (kOwnRows + 31) / 32; ++pass) {
       if (m_tile * kRows + pass * 32 * kSplit >= p.tokens) break;   // no row of this pass exists
-      // tile row kSplit * row_local + rank; with eight owners a CTA has 16 rows and half of the
+      // tile row kSplit * row_local + rank; where a CTA has 16 rows (64-row tiles, four owners) half of the
       // threads only keep their quads company (they read row 15 again and store nothing)
       const bool row_owned = pass * 32 + (t >> 2) < kOwnRows;
       const int row_local = row_owned ? pass * 32 + (t >> 2) : kOwnRows - 1;

@@ -14,7 +14,8 @@
  * of the call itself; every launch only enqueues work on `stream`; functions
  * return 0 or a negative gevva_moe_status and never throw.  A runner is used
  * from one host thread; runners that share scratch must be launched on one
- * stream (include/gevva/gpu.hpp:222).
+ * stream (include/gevva/gpu.hpp:222).  Runners with scratch of their own may run on streams of their own, of any
+ * priority, at the same time: no launch waits for a block that the device has not started.
  */
 #ifndef GEVVA_MOE_H_
 #define GEVVA_MOE_H_
@@ -47,7 +48,8 @@ enum gevva_moe_status {
  *   w2_sf   u8  [128,2816,44]
  *   alpha1, alpha2            f32 [128]   g1.alpha, g2.alpha
  *   in_scale_q1, in_scale_q2  f32 [128]   g1/g2.input_scale_quant
- * They must stay valid for the life of the runner (pointers are cached). */
+ * They must stay valid and unchanged for the life of the runner: pointers are cached, and re-tiled copies of the two
+ * scale tensors (93 MB) are made at creation. */
 typedef struct {
   const void* w13;
   const void* w13_sf;
