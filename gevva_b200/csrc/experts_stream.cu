@@ -3,13 +3,13 @@
 // What bounds it.  Every routed expert's 3.3 MB come from HBM once: 65 us of it when all 128 experts are
 // hit, whatever the batch; with a handful of tokens the time is the chain sort -> quantise -> w13 ->
 // GeGLU -> w2.  So the weights sit on MMA-M (128 rows a tile, all of them real) and the rows of an
-// expert on MMA-N, in multiples of 16.  What that buys is not tensor time (an MMA takes about 105 cycles at any N up to
+// expert on MMA-N, in multiples of 16.  What that buys is not tensor time (an MMA takes 40 to 64 cycles at N up to
 // 128, and the pipe is 4 to 8 % busy) but finer steps: a pipeline stage carries 18 KB of weights instead of 34, and
 // a w13 item is 64 intermediate columns (11 an expert, 180 KB), so one token's eight experts keep 88 SMs busy
 // instead of 48.  A chunk ends at 64 rows because four accumulators of 64 columns and seven stages' scales fill tensor
 // memory, and seven stages with 8 KB of rows each shared memory; an expert with more rows reads its weights once a chunk.
 // Alone and from a cold L2: 64 tokens 81 us for 430 MB of DRAM traffic, 400 tokens (kFront false) 81 us for 450 MB,
-// 5.3 and 5.5 TB/s over the whole launch.
+// 5.3 and 5.5 TB/s over the whole launch (before the K loops were unrolled; 6.4 from the first load to the last).
 //
 //   w13 item   (chunk of at most 64 rows of an expert) x (unit of 64 intermediate columns): MMA rows 0..63
 //              are the unit's up rows, 64..127 its gate rows (one 3-D box brings both; their scales come
@@ -19,10 +19,13 @@
 // further ones are claimed one by one, a little ahead; the w2 items are dealt in the order in which the CTAs run out of
 // w13 items, so that those that are one short (180 KB) get four w2 items (48 KB each) first.
 //
-// Roles (14 warps): 0 fetches weights, 1 issues MMAs, 2 fetches activations, 3 copies scale factors to
-// tensor memory one stage ahead, 4..11 are the epilogue (two warps per 32-lane quarter, alternating
+// Roles (14 warps): 0 fetches weights, 1 copies scale factors to tensor memory and issues MMAs, 2 fetches activations
+// (one thread each), 3 only takes part in the sort and the quantiser, 4..11 are the epilogue (two warps per 32-lane quarter, alternating
 // groups of eight rows), 12 publishes finished w13 items, 13 claims the next ones.  Seven stages of one K block (256 elements); four accumulators of 64 columns,
-// so nothing waits for a drain.  In the w13 epilogue a thread holds one weight row for eight tokens, so
+// so nothing waits for a drain.  How fast a CTA gets through K blocks is a matter of how those three threads are written, not of
+// bytes: with a warp of its own for the scale copies (a commit and a barrier more a stage), waits by whole warps and rolled K
+// loops a w13 item whose weights lay in L2 took 3.8 us, with one thread a role and the K loops unrolled by two and four
+// 2.6 (unrolled by eleven 3.4: its code no longer stays in the instruction cache).  64 tokens 86.2 -> 83.6 us a layer, 1 token 22.7 -> 21.9.  In the w13 epilogue a thread holds one weight row for eight tokens, so
 // bf16(alpha * acc), which is what the reference's GEMM stores, changes hands through shared memory and a
 // thread then owns one column of four tokens: GeGLU, block maxima over sixteen lanes, codes.  (One token at a
 // time, with the scale worked out in all sixteen lanes, this took 87000 of 165000 cycles at 613 tokens and
@@ -67,7 +70,7 @@ namespace {
 constexpr int kStStages = 7;
 constexpr int kStRows = 64;                               // rows of a chunk at most (MMA-N)
 constexpr int kStAccStages = 4;
-constexpr int kStWeightWarp = 0, kStMmaWarp = 1, kStTokenWarp = 2, kStScaleWarp = 3, kStEpilogueWarp = 4;
+constexpr int kStWeightWarp = 0, kStMmaWarp = 1, kStTokenWarp = 2, kStEpilogueWarp = 4;
 constexpr int kStEpilogueWarps = 8;
 constexpr int kStPublishWarp = kStEpilogueWarp + kStEpilogueWarps;     // 12
 constexpr int kStClaimWarp = kStPublishWarp + 1;                       // 13
@@ -81,6 +84,7 @@ constexpr int kStTokenBytes = kStRows * kTileKBytes;      // 8 KiB
 static_assert(kStreamUpItems == kUnits && kStreamDownItems == kHidden / 128, "items of a chunk");
 constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
 static_assert(kStMmaWarp == 1 && kStPublishWarp - 1 == kStUpKBlocks, "warps 1..11 quantise a K block each");
+constexpr int kStLoadUnroll = 2, kStMmaUnroll = 4;        // K blocks of w13 items
 constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192
 constexpr int kStDownLastMmas = 3;
 constexpr int kStMaxChunks = 256;
@@ -106,7 +110,7 @@ struct alignas(1024) StreamSmem {
       uint8_t route_expert[kStRankWarps * kStStretch];
     };
   };
-  uint64_t full[kStStages], empty[kStStages], sf_full[kStStages];
+  uint64_t full[kStStages], empty[kStStages];
   uint64_t acc_full[kStAccStages], acc_empty[kStAccStages];
   volatile int progress[kStEpilogueWarps];  // w13 items whose rows each epilogue warp has stored
   volatile int published;                   // w13 items that the publisher has counted
@@ -247,6 +251,12 @@ __device__ __forceinline__ void tmem_load_32x8(uint32_t tmem_address, uint32_t (
                : "memory");
 }
 
+// A number of MMAs as a type.
+template <int kCount>
+struct MmaCount {
+  __device__ constexpr int operator()() const { return kCount; }
+};
+
 // The MMAs of one K block (K = 64 each) with a runtime instruction descriptor (its N field).  Scale
 // columns of the stage: weights of MMA j at +4j; rows at +16 + 4j, plus two where the chunk is the second
 // half of its 128-row scale atom.
@@ -279,7 +289,7 @@ __device__ __forceinline__ void stream_add_release(int* address) {
   asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(address) : "memory");
 }
 
-// Bounded acquire spin of a whole warp on a counter in global memory; or, where one is given, on a second one.
+// Bounded acquire spin of one thread on a counter in global memory; or, where one is given, on a second one.
 __device__ __forceinline__ bool stream_wait_counter(const int* counter, int target, StreamSmem* smem, int* status,
                                                     const int* other = nullptr, int other_target = 0) {
   const long long start = clock64();
@@ -299,7 +309,7 @@ __device__ __forceinline__ bool stream_wait_counter(const int* counter, int targ
       }
     }
   }
-  return __all_sync(0xffffffffu, ready);
+  return ready;
 }
 
 // Eight columns a lane (two lanes a 16-value block): code bytes and scale of the block.  The arithmetic of
@@ -448,7 +458,6 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     for (int s = 0; s < kStStages; ++s) {
       mbar_init(&smem->full[s], 2);  // one arrival (with its byte count) per producer warp
       mbar_init(&smem->empty[s], 1);
-      mbar_init(&smem->sf_full[s], 1);
     }
     for (int s = 0; s < kStAccStages; ++s) {
       mbar_init(&smem->acc_full[s], 1);
@@ -684,7 +693,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
   }
 
   if (warp == kStWeightWarp || warp == kStTokenWarp) {
-    // ---------------- producers ----------------
+    // ---------------- producers, a thread each ----------------
     const bool weight_side = warp == kStWeightWarp;
     int stage = 0, issued = 0;
     uint32_t phase = 0;
@@ -694,40 +703,40 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       stage = kStUpKBlocks % kStStages;
       phase = kStUpKBlocks / kStStages & 1;
     }
-    while (ok && cursor.next(shares, smem, it)) {
-      if (weight_side && !it.down && lane == 0) smem->begun = cursor.taken;
-      const int k_blocks = it.down ? kStDownKBlocks : kStUpKBlocks;
-      const int first = it.chunk * kStRows;
-      const int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
-      const int boxes = rows >= kStRows ? kStRows / 8 : (rows + 7) / 8;
-      const int row = smem->offsets[it.expert] + first;
-      const uint8_t* sf;
-      if (weight_side) {
-        sf = it.down ? p.w2_scales + static_cast<size_t>(it.expert * kHidden + it.n_tile * 128) * (kInter / 16)
-                     : p.w13_scales + static_cast<size_t>(it.expert * kUnitSlots + it.n_tile) * kStUpKBlocks * kSfStageBytes;
-      } else {
-        const size_t scale_row = smem->scale_rows[it.expert] + first / kTileM * kTileM;
-        if (rows_pending && !it.down) {
-          // the w13 operand exists once every CTA with tokens has quantised them and counted itself
-          ok = stream_wait_counter(sync + kStreamQuantised, p.tokens < ctas ? p.tokens : ctas, smem, status,
-                                   sync + kStreamRescued, p.tokens);
-          if (!ok) break;
-          rows_pending = false;
-          asm volatile("fence.proxy.async.global;" ::: "memory");
+    if (elect_one()) {
+      while (ok && cursor.next(shares, smem, it)) {
+        if (weight_side && !it.down) smem->begun = cursor.taken;
+        const int first = it.chunk * kStRows;
+        const int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
+        const int boxes = rows >= kStRows ? kStRows / 8 : (rows + 7) / 8;
+        const int row = smem->offsets[it.expert] + first;
+        const uint8_t* sf;
+        if (weight_side) {
+          sf = it.down ? p.w2_scales + static_cast<size_t>(it.expert * kHidden + it.n_tile * 128) * (kInter / 16)
+                       : p.w13_scales + static_cast<size_t>(it.expert * kUnitSlots + it.n_tile) * kStUpKBlocks * kSfStageBytes;
+        } else {
+          const size_t scale_row = smem->scale_rows[it.expert] + first / kTileM * kTileM;
+          if (rows_pending && !it.down) {
+            // the w13 operand exists once every CTA with tokens has quantised them and counted itself
+            ok = stream_wait_counter(sync + kStreamQuantised, p.tokens < ctas ? p.tokens : ctas, smem, status,
+                                     sync + kStreamRescued, p.tokens);
+            if (!ok) break;
+            rows_pending = false;
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+          }
+          sf = it.down ? p.inter_scales + scale_row * (kInter / 16) : p.input_scales + scale_row * (kHidden / 16);
+          if (it.down) {
+            // the rows exist once every w13 item of the expert has been counted; they were written by ordinary stores of other SMs and are read through the async proxy
+            ok = stream_wait_counter(p.plan.tile_ready + it.expert, kUnits * smem->chunks_of[it.expert], smem, status);
+            if (!ok) break;
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+          }
         }
-        sf = it.down ? p.inter_scales + scale_row * (kInter / 16) : p.input_scales + scale_row * (kHidden / 16);
-        if (it.down) {
-          // the rows exist once every w13 item of the expert has been counted; they were written by ordinary stores of other SMs and are read through the async proxy
-          ok = stream_wait_counter(p.plan.tile_ready + it.expert, kUnits * smem->chunks_of[it.expert], smem, status);
-          if (!ok) break;
-          asm volatile("fence.proxy.async.global;" ::: "memory");
-        }
-      }
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, status));
-        if (!ok) break;
-        if (elect_one()) {
-          const uint32_t sf_bytes = static_cast<uint32_t>(it.down && kb + 1 == k_blocks ? kStDownLastMmas : 4) * kSfAtomBytes;
+        // One K block.  The loops around it are unrolled because a trip of a rolled one takes 320 cycles, whatever it loads (the
+        // back edge waits until the copy has read its operands); unrolled it is as fast as 128 rows arrive from L2, 226 cycles.
+        const auto load = [&](int kb, uint32_t sf_bytes) {
+          ok = wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, status);
+          if (!ok) return false;
           const int x = kb * kTileKBytes;
           uint64_t* bar = &smem->full[stage];
           if (weight_side) {
@@ -740,96 +749,95 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
             tma_load_2d(smem->b[stage], it.down ? &maps.down[boxes - 1] : &maps.up[boxes - 1], bar, x, row);
             bulk_load_1d(smem->sfb[stage], sf + static_cast<size_t>(kb) * kSfStageBytes, sf_bytes, bar);
           }
+          ++issued;
+          if (++stage == kStStages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+          return true;
+        };
+        if (it.down) {
+#pragma unroll
+          for (int kb = 0; kb < kStDownKBlocks; ++kb)
+            if (!load(kb, (kb + 1 == kStDownKBlocks ? kStDownLastMmas : 4) * kSfAtomBytes)) break;
+        } else {
+#pragma unroll kStLoadUnroll
+          for (int kb = 0; kb < kStUpKBlocks; ++kb)
+            if (!load(kb, kSfStageBytes)) break;
         }
-        __syncwarp();
-        ++issued;
-        if (++stage == kStStages) {
-          stage = 0;
-          phase ^= 1u;
+      }
+      if (!ok || smem->abort) {
+        // unwinding: the copies already issued land before shared memory is given up
+        const int pending = issued < kStStages ? issued : kStStages;
+        for (int i = 0; i < pending; ++i) {
+          if (--stage < 0) {
+            stage = kStStages - 1;
+            phase ^= 1u;
+          }
+          mbar_wait_bounded(&smem->full[stage], phase, 40000000ll);
         }
       }
     }
-    if ((!ok || smem->abort) && lane == 0) {
-      // unwinding: the copies already issued land before shared memory is given up
-      const int pending = issued < kStStages ? issued : kStStages;
-      for (int i = 0; i < pending; ++i) {
-        if (--stage < 0) {
-          stage = kStStages - 1;
-          phase ^= 1u;
-        }
-        mbar_wait_bounded(&smem->full[stage], phase, 40000000ll);
-      }
-    }
+    __syncwarp();
   } else if (warp == kStMmaWarp) {
-    // ---------------- MMA issuer ----------------
-    int stage = 0, acc = 0;
-    uint32_t phase = 0, acc_phase = 0;
-    const uint32_t a_lo0 = (smem_u32(smem->a[0]) & 0x3ffffu) >> 4;
-    const uint32_t b_lo0 = (smem_u32(smem->b[0]) & 0x3ffffu) >> 4;
-    const bool leader = elect_one();
-    while (ok && cursor.next(shares, smem, it)) {
-      const int k_blocks = it.down ? kStDownKBlocks : kStUpKBlocks;
-      const int first = it.chunk * kStRows;
-      int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
-      rows = rows > kStRows ? kStRows : rows;
-      // E2M1 x E2M1, both K-major, UE4M3 scales, M = 128; N = the rows in multiples of 16
-      const uint32_t descriptor = (1u << 7) | (1u << 10) | (static_cast<uint32_t>((rows + 15) / 16 * 2) << 17) |
-                                  (static_cast<uint32_t>(kTileM >> 4) << 24);
-      const uint32_t half = (first % kTileM) / 32;
-      if (!__all_sync(0xffffffffu, wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, status))) break;
-      tc_fence_after_sync();
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = wait_or_abort<false>(&smem->sf_full[stage], phase, smem, status);
-        if (!ok) break;
-        tc_fence_after_sync();
-        if (leader) {
+    // ---------------- scale copies and MMAs, in one thread ----------------
+    if (elect_one()) {
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      const uint32_t a_lo0 = (smem_u32(smem->a[0]) & 0x3ffffu) >> 4;
+      const uint32_t b_lo0 = (smem_u32(smem->b[0]) & 0x3ffffu) >> 4;
+      const uint32_t sfa_lo0 = (smem_u32(smem->sfa[0]) & 0x3ffffu) >> 4;
+      const uint32_t sfb_lo0 = (smem_u32(smem->sfb[0]) & 0x3ffffu) >> 4;
+      constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);  // 8 rows x 16 B, no swizzle
+      bool landed = false;  // the next stage's bytes have been seen
+      while (ok && cursor.next(shares, smem, it)) {
+        const int first = it.chunk * kStRows;
+        int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
+        rows = rows > kStRows ? kStRows : rows;
+        // E2M1 x E2M1, both K-major, UE4M3 scales, M = 128; N = the rows in multiples of 16
+        const uint32_t descriptor = (1u << 7) | (1u << 10) | (static_cast<uint32_t>((rows + 15) / 16 * 2) << 17) |
+                                    (static_cast<uint32_t>(kTileM >> 4) << 24);
+        const uint32_t half = (first % kTileM) / 32;
+        if (!wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, status)) break;
+        const uint32_t d = tmem_base + static_cast<uint32_t>(acc) * kStRows;
+        // One K block, unrolled for the producers' reason.
+        const auto multiply = [&](int kb, auto mmas, bool last) {
+          if (!landed) ok = wait_or_abort<false>(&smem->full[stage], phase, smem, status);
+          if (!ok) return false;
+          tc_fence_after_sync();
           const uint32_t sf = tmem_base + kStSfColumn + kStSfColumnsPerStage * stage;
           const uint32_t a_lo = a_lo0 + static_cast<uint32_t>(stage) * (kStWeightBytes >> 4);
           const uint32_t b_lo = b_lo0 + static_cast<uint32_t>(stage) * (kStTokenBytes >> 4);
-          const uint32_t d = tmem_base + static_cast<uint32_t>(acc) * kStRows;
-          if (it.down && kb + 1 == k_blocks) stream_mmas<kStDownLastMmas>(d, sf, sf + 16 + half, a_lo, b_lo, descriptor, kb != 0);
-          else stream_mmas<4>(d, sf, sf + 16 + half, a_lo, b_lo, descriptor, kb != 0);
-          tc_commit(&smem->empty[stage]);
-          if (kb + 1 == k_blocks) tc_commit(&smem->acc_full[acc]);
+          const uint32_t sf_offset = static_cast<uint32_t>(stage) * (kSfStageBytes >> 4);
+          uint64_t* const empty = &smem->empty[stage];
+          if (++stage == kStStages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+          issue_sf_copies<mmas(), 128>(sf, sfa_lo0 + sf_offset, sfb_lo0 + sf_offset, hi_sf);
+          stream_mmas<mmas()>(d, sf, sf + 16 + half, a_lo, b_lo, descriptor, kb != 0);
+          landed = mbar_try_wait(&smem->full[stage], phase);
+          tc_commit(empty);
+          if (last) tc_commit(&smem->acc_full[acc]);
+          return true;
+        };
+        if (it.down) {
+#pragma unroll
+          for (int kb = 0; kb < kStDownKBlocks - 1; ++kb)
+            if (!multiply(kb, MmaCount<4>(), false)) break;
+          if (ok) (void)multiply(kStDownKBlocks - 1, MmaCount<kStDownLastMmas>(), true);
+        } else {
+#pragma unroll kStMmaUnroll
+          for (int kb = 0; kb < kStUpKBlocks; ++kb)
+            if (!multiply(kb, MmaCount<4>(), kb + 1 == kStUpKBlocks)) break;
         }
-        if (++stage == kStStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
-      }
-      if (++acc == kStAccStages) {
-        acc = 0;
-        acc_phase ^= 1u;
-      }
-    }
-  } else if (warp == kStScaleWarp) {
-    // ---------------- scale-factor copier ----------------
-    int stage = 0;
-    uint32_t phase = 0;
-    const uint32_t sfa_lo0 = (smem_u32(smem->sfa[0]) & 0x3ffffu) >> 4;
-    const uint32_t sfb_lo0 = (smem_u32(smem->sfb[0]) & 0x3ffffu) >> 4;
-    constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);  // 8 rows x 16 B, no swizzle
-    const bool leader = elect_one();
-    while (ok && cursor.next(shares, smem, it)) {
-      const bool down = it.down;
-      const int k_blocks = down ? kStDownKBlocks : kStUpKBlocks;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = wait_or_abort<false>(&smem->full[stage], phase, smem, status);
-        if (!ok) break;
-        if (leader) {
-          const uint32_t sfa = sfa_lo0 + static_cast<uint32_t>(stage) * (kSfStageBytes >> 4);
-          const uint32_t sfb = sfb_lo0 + static_cast<uint32_t>(stage) * (kSfStageBytes >> 4);
-          const uint32_t sf = tmem_base + kStSfColumn + kStSfColumnsPerStage * stage;
-          if (down && kb + 1 == k_blocks) issue_sf_copies<kStDownLastMmas, 128>(sf, sfa, sfb, hi_sf);
-          else issue_sf_copies<4, 128>(sf, sfa, sfb, hi_sf);
-          tc_commit(&smem->sf_full[stage]);
-        }
-        if (++stage == kStStages) {
-          stage = 0;
-          phase ^= 1u;
+        if (++acc == kStAccStages) {
+          acc = 0;
+          acc_phase ^= 1u;
         }
       }
     }
+    __syncwarp();
   } else if (warp == kStClaimWarp) {
     // ---------------- claims ----------------
     // Two items ahead of the weight warp, which is busy with one for four microseconds: a claim takes one to two under
@@ -921,7 +929,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       if (lane == 0) smem->published = done;
       start = clock64();
     }
-  } else {
+  } else if (warp >= kStEpilogueWarp) {
     // ---------------- epilogue ----------------
     const int quarter = warp & 3;                        // the tensor-memory lanes this warp may read
     const int side = (warp - kStEpilogueWarp) >> 2;      // groups side, side + 2, ... of eight rows
