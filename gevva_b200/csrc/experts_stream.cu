@@ -45,8 +45,9 @@
 // tokens, 87.7 -> 90 and 91 us), because such a launch starts only once all SMs are free.
 //
 // In its kFront form the kernel also sorts the routes and quantises the input: every CTA ranks the whole
-// batch's routes by a counting sort (12 warps, a stretch of routes each) and derives the group geometry for
-// itself; CTA c quantises tokens c and c + CTAs with eleven warps, a K block each, then adds one to a counter that
+// batch's routes for itself, with a bit per expert and token (a route's rank is the number of bits before its own; a token that names
+// an expert twice is seen when its bit is set already, and the routes are then counted one by one) and derives the group geometry;
+// CTA c quantises tokens c and c + CTAs with ten warps, a K block each, then adds one to a counter that
 // the activation side waits for.  At 200 tokens that saves 4 us of a layer against launches of their own; with
 // five tokens a CTA it would lose five (613 tokens: 119.5 against 114.1 us).
 // Until that counter is full, all that moves is the weights that fit the ring, and its chain (stores, their
@@ -54,8 +55,13 @@
 // at most eight rows, eleven warps quantise these into the pipeline stages, and the counter is full by the
 // time that the second item needs it.  24.5 -> 22.9 us a layer at 1 token, 36.1 -> 34.1 at 5, 53.7 -> 52.2 at 16, 70.2 -> 69.7
 // at 37, nothing from 64 on, where more rows take as long as the counter (with 24 rows allowed, 5 us slower at 200).
+// Time stamps at 64 tokens, from the end of the dependency wait: geometry 2.8 us with counts by match.any and three scans, 1.5
+// with bits and one scan of packed words (200 tokens 3.8 and 1.9); the grid's own tokens 4.7 and 3.6.  Those come before the
+// first item's rows wherever some CTA has a second item, and the MMA warp leaves its share of them to warp 3.
+// 1 token 177 -> 172 us a pass of eight layers, 64 tokens 656 -> 646, 200 tokens (four layers) 360 -> 356.
 // The code in front of the roles runs once a launch, and while the weights keep the way to L2 busy an instruction
-// line that has to be fetched costs up to a microsecond: it is kept small, loops are not unrolled.
+// line that has to be fetched costs up to a microsecond: it is kept small, loops are not unrolled, and the two quantisers
+// are run once on nothing in front of the dependency wait (37 tokens 615 -> 611, 40-token feed-forward layers 343 -> 338).
 // The CTA that finishes last puts all counters back to zero.
 #include "gv_common.cuh"
 #include "gv_gemm_parts.cuh"
@@ -70,7 +76,7 @@ namespace {
 constexpr int kStStages = 7;
 constexpr int kStRows = 64;                               // rows of a chunk at most (MMA-N)
 constexpr int kStAccStages = 4;
-constexpr int kStWeightWarp = 0, kStMmaWarp = 1, kStTokenWarp = 2, kStEpilogueWarp = 4;
+constexpr int kStWeightWarp = 0, kStMmaWarp = 1, kStTokenWarp = 2, kStSpareWarp = 3, kStEpilogueWarp = 4;
 constexpr int kStEpilogueWarps = 8;
 constexpr int kStPublishWarp = kStEpilogueWarp + kStEpilogueWarps;     // 12
 constexpr int kStClaimWarp = kStPublishWarp + 1;                       // 13
@@ -84,15 +90,17 @@ constexpr int kStTokenBytes = kStRows * kTileKBytes;      // 8 KiB
 static_assert(kStreamUpItems == kUnits && kStreamDownItems == kHidden / 128, "items of a chunk");
 constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
 static_assert(kStMmaWarp == 1 && kStPublishWarp - 1 == kStUpKBlocks, "warps 1..11 quantise a K block each");
+static_assert(kStWeightWarp == 0 && kExperts == 128, "threads 0..127 scan the experts");
 constexpr int kStLoadUnroll = 2, kStMmaUnroll = 4;        // K blocks of w13 items
 constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192
 constexpr int kStDownLastMmas = 3;
 constexpr int kStMaxChunks = 256;
 constexpr int kStExchangeRows = 32;
 constexpr int kStOwnTokens = 2;                           // kFront: tokens a CTA quantises, at most
-constexpr int kStRankWarps = 12;                          // kFront: warps 1..12 rank the routes
-constexpr int kStStretch = 224;                           // routes of each, at most
-constexpr int kStFrontTokens = kStStretch * kStRankWarps / kTopK;  // 336
+constexpr int kStFrontRoutes = 6;                         // kFront: routes a thread looks at, at most
+constexpr int kStFrontTokens = kStFrontRoutes * kStThreads / kTopK;  // 336
+constexpr int kStFrontWords = (kStFrontTokens + 31) / 32; // 11, odd: an expert's words lie in banks of their own
+constexpr uint32_t kStNoRow = 0xffffffffu;
 constexpr int kStSelfRows = 8;                            // kFront: rows of a first item that the CTA quantises itself, at most
 constexpr int kStClaims = 32;                             // claims on their way from the claim warp to the others, at most
 constexpr uint32_t kStNoMoreClaims = 1u << 15, kStNoTurn = kStNoMoreClaims - 1;
@@ -105,10 +113,7 @@ struct alignas(1024) StreamSmem {
   uint8_t sfb[kStStages][kSfStageBytes];
   union {
     __nv_bfloat16 exchange[2][kStExchangeRows][128];  // [token][MMA row]
-    struct {                                          // the sort's, before
-      int warp_counts[kStRankWarps][kExperts];
-      uint8_t route_expert[kStRankWarps * kStStretch];
-    };
+    uint32_t tokens_of[kExperts][kStFrontWords];      // the sort's, before: a bit per token
   };
   uint64_t full[kStStages], empty[kStStages];
   uint64_t acc_full[kStAccStages], acc_empty[kStAccStages];
@@ -128,16 +133,15 @@ struct alignas(1024) StreamSmem {
   int chunks_of[kExperts];
   short chunk_expert[kStMaxChunks];
   short chunk_index[kStMaxChunks];  // which chunk of its expert
-  int histogram[kExperts];
-  // kFront: the routes of this CTA's tokens
-  int own_expert[kStOwnTokens * kTopK];
-  int own_rank[kStOwnTokens * kTopK];  // among the routes of its warp's stretch with the same expert
-  int own_warp[kStOwnTokens * kTopK];
-  alignas(16) int route_row[kStOwnTokens * kTopK];
+  uint32_t scan[kExperts / 32];
+  // kFront
+  volatile int repeats;                // a token names an expert twice: tokens_of does not count its routes
+  int histogram[kExperts];             // ... which these two do
+  int own_rank[kStOwnTokens * kTopK];
+  // the routes of this CTA's tokens
+  alignas(16) uint2 route_at[kStOwnTokens * kTopK];  // where the row's codes and its scale bytes begin
   alignas(16) float route_multiplier[kStOwnTokens * kTopK];
-  unsigned long long route_scale_base[kStOwnTokens * kTopK];
   float scale_q1[kExperts];
-  short first_token[kStSelfRows];          // kFront: tokens of the CTA's first w13 item's rows
   GegluTables tables;
 };
 constexpr size_t kStSmemBytes = sizeof(StreamSmem) + 1024;
@@ -278,6 +282,13 @@ __device__ __forceinline__ void stream_mmas(uint32_t tmem_acc, uint32_t tmem_sfa
   }
 }
 
+// A load that is issued here; the compiler puts an ordinary one where its value is used, a trip to memory later.
+__device__ __forceinline__ uint4 stream_load_now(const uint4* address) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(address) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ int stream_load_acquire(const int* address) {
   int value;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(value) : "l"(address) : "memory");
@@ -335,71 +346,130 @@ __device__ __forceinline__ float stream_block_maximum(const uint4& raw, float (&
 }
 
 // K block `kb` of one token by a warp: the codes and scale bytes of its eight routes (entries first..first+7 of
-// the route arrays) go to their sorted rows.
-__device__ __forceinline__ void stream_quantise_token(const StreamParams& p, const StreamSmem* smem, int first, int kb,
-                                                      int lane, const uint4& raw) {
+// the route arrays) go to their sorted rows.  (Arguments by value: a kernel parameter's fields read through a reference
+// come from memory, a microsecond away.)
+__device__ __noinline__ void stream_quantise_token(uint8_t* packed, uint8_t* scales, const StreamSmem* smem, int first, int kb,
+                                                   int lane, uint4 raw, bool dry) {
   float values[8];
   const float maximum = stream_block_maximum(raw, values);
+  packed += kb * kTileKBytes + 4 * lane;
   // scale groups of a row go four to an aligned word of the swizzled layout: eight lanes a word
-  const uint32_t scale_offset = static_cast<uint32_t>(4 * kb + (lane >> 3)) * kSfAtomBytes;
-  uint32_t codes = 0, scale_word = 0, previous = 0;
-  bool have = false;
+  scales += static_cast<uint32_t>(4 * kb + (lane >> 3)) * kSfAtomBytes;
+  uint4 at[kTopK / 2];  // code offset and scale offset of two routes each
+#pragma unroll
+  for (int i = 0; i < kTopK / 2; ++i) at[i] = reinterpret_cast<const uint4*>(smem->route_at + first)[i];
+  const float4 m0 = *reinterpret_cast<const float4*>(smem->route_multiplier + first);
+  const float4 m1 = *reinterpret_cast<const float4*>(smem->route_multiplier + first + 4);
+  const float multipliers[kTopK] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+  uint32_t codes = 0, scale_word = 0;
 #pragma unroll 1
-  for (int k = 0; k < kTopK; ++k) {
-    const int row = smem->route_row[first + k];
-    if (row < 0) continue;
-    const float multiplier = smem->route_multiplier[first + k];
-    if (!have || __float_as_uint(multiplier) != previous) {  // routes of equal static scale share the result
-      have = true;
-      previous = __float_as_uint(multiplier);
-      const uint32_t scale = stream_quantise(values, maximum, multiplier, smem->tables.reciprocals, codes);
-      scale_word = scale | (__shfl_down_sync(0xffffffffu, scale, 2) << 8) | (__shfl_down_sync(0xffffffffu, scale, 4) << 16) |
-                   (__shfl_down_sync(0xffffffffu, scale, 6) << 24);
+  for (int done = 0; done < kTopK;) {
+    // the routes from `done` on that share a static scale share the result
+    float multiplier = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k)
+      if (k == done) multiplier = multipliers[k];
+    const uint32_t scale = stream_quantise(values, maximum, multiplier, smem->tables.reciprocals, codes);
+    scale_word = scale | (__shfl_down_sync(0xffffffffu, scale, 2) << 8) | (__shfl_down_sync(0xffffffffu, scale, 4) << 16) |
+                 (__shfl_down_sync(0xffffffffu, scale, 6) << 24);
+    const int from = done;
+    bool same = true;
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k) {
+      const uint32_t code_at = k & 1 ? at[k / 2].z : at[k / 2].x, scale_at = k & 1 ? at[k / 2].w : at[k / 2].y;
+      same = same && (k < from || __float_as_uint(multipliers[k]) == __float_as_uint(multiplier));
+      const bool store = same && k >= from && code_at != kStNoRow && !dry;
+      if (store) *reinterpret_cast<uint32_t*>(packed + code_at) = codes;
+      if (store && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(scales + scale_at) = scale_word;
+      done = same && k >= from ? k + 1 : done;
     }
-    *reinterpret_cast<uint32_t*>(p.packed + static_cast<size_t>(row) * (kHidden / 2) + kb * kTileKBytes + 4 * lane) = codes;
-    if ((lane & 7) == 0) *reinterpret_cast<uint32_t*>(p.scales + smem->route_scale_base[first + k] + scale_offset) = scale_word;
   }
 }
 
-// K block `kb` of an item's `rows` tokens (smem->first_token) by a warp, straight into a pipeline stage: codes in
+// The token of row `target` of an expert (rows in the order of the sort).
+__device__ __forceinline__ int stream_token_of_row(const StreamSmem* smem, int expert, int target, int words) {
+#pragma unroll 1
+  for (int w = 0; w < words; ++w) {
+    uint32_t bits = smem->tokens_of[expert][w];
+    const int count = __popc(bits);
+    if (target < count) {
+      for (; target > 0; --target) bits &= bits - 1;
+      return 32 * w + __ffs(static_cast<int>(bits)) - 1;
+    }
+    target -= count;
+  }
+  return 0;
+}
+
+// The same from the ids, by a warp, for rows first + lane; and a route's rank among those of its expert: where a token
+// names an expert twice.
+__device__ __noinline__ int stream_token_of_row_repeated(const int* expert_ids, int routes, int expert, int first, int lane) {
+  int before = 0, token = 0;
+#pragma unroll 4
+  for (int base = 0; base < routes; base += 32) {
+    uint32_t all = __ballot_sync(0xffffffffu, base + lane < routes && expert_ids[base + lane] == expert);
+    const int count = __popc(all);
+    int target = first + lane - before;
+    if (target >= 0 && target < count) {
+      for (; target > 0; --target) all &= all - 1;
+      token = (base + __ffs(static_cast<int>(all)) - 1) / kTopK;
+    }
+    before += count;
+  }
+  return token;
+}
+__device__ __noinline__ int stream_rank_repeated(const int* expert_ids, int route, int lane) {
+  const int expert = expert_ids[route];
+  int rank = 0;
+#pragma unroll 4
+  for (int base = 0; base < route; base += 32)
+    rank += __popc(__ballot_sync(0xffffffffu, base + lane < route && expert_ids[base + lane] == expert));
+  return rank;
+}
+
+// K block `kb` of an item's `rows` tokens (lane r holds the one of row r) by a warp, straight into a pipeline stage: codes in
 // the 128B-swizzled layout of the row side, scale bytes at rows scale_row.. of the stage's four atoms.  The tokens
-// are fetched into the stage first, twelve at a time and 512 bytes each from its byte 2048 on, where the codes that replace them
-// never reach a token that is still to be read (up to 24 rows: code row 12 + j lies below byte 2048 + 512 j).
+// are fetched into the stage first, 512 bytes each from its byte 2048 on, where the codes that replace them
+// never reach a token that is still to be read; or, in a batch of a few, they lie there already, in their own order.
 // Everything here runs once a launch, while the weights keep the way to L2 busy, and an instruction line that has to
 // be fetched takes about a microsecond: hence one copy of the code and no unrolling.
-__device__ __noinline__ void stream_quantise_stage(const uint4* input, StreamSmem* smem, int stage, int kb, int rows,
-                                                   int scale_row, float multiplier, int lane) {
-  constexpr int kAhead = 12;
-  static_assert(kStSelfRows <= 2 * kAhead && 2048 + kAhead * 512 == kStTokenBytes, "codes and tokens in one stage");
+constexpr int kStTokensAt = 2048;
+__device__ __forceinline__ void stream_fetch_token(uint8_t* stage_rows, int slot, const uint4* input, int token, int kb, int lane) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(stage_rows + kStTokensAt + slot * 512 + lane * 16)),
+               "l"(input + static_cast<size_t>(token) * (kHidden / 8) + kb * (kTileK / 8) + lane)
+               : "memory");
+}
+static_assert(kStTokensAt + kStSelfRows * 512 <= kStTokenBytes && kStSelfRows * kTileKBytes <= kStTokensAt, "codes and tokens in one stage");
+__device__ __noinline__ void stream_quantise_stage(const uint4* input, StreamSmem* smem, int stage, int kb, int rows, int tokens,
+                                                   bool fetched, int scale_row, float multiplier, int lane, bool dry) {
   uint8_t* const b = smem->b[stage];
   uint8_t* const sf = smem->sfb[stage] + (lane >> 3) * kSfAtomBytes + ((lane >> 1) & 3);
-  input += kb * (kTileK / 8) + lane;
+  if (!fetched) {
 #pragma unroll 1
-  for (int base = 0; base < rows; base += kAhead) {
-    const int end = rows < base + kAhead ? rows : base + kAhead;
-    uint8_t* token = b + 2048 + lane * 16;
-    __syncwarp();
-#pragma unroll 1
-    for (int r = base; r < end; ++r, token += 512)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(token)),
-                   "l"(input + static_cast<size_t>(smem->first_token[r]) * (kHidden / 8))
-                   : "memory");
+    for (int r = 0; r < rows; ++r) stream_fetch_token(b, r, input, __shfl_sync(0xffffffffu, tokens, r), kb, lane);
     asm volatile("cp.async.wait_all;" ::: "memory");
-    token = b + 2048 + lane * 16;
+  }
 #pragma unroll 1
-    for (int r = base; r < end; ++r, token += 512) {
-      float values[8];
-      const float maximum = stream_block_maximum(*reinterpret_cast<const uint4*>(token), values);
-      uint32_t codes;
-      const uint32_t scale = stream_quantise(values, maximum, multiplier, smem->tables.reciprocals, codes);
-      *reinterpret_cast<uint32_t*>(b + r * kTileKBytes + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) = codes;
-      const int n = scale_row + r;
-      if ((lane & 1) == 0) sf[(n & 31) * 16 + ((n >> 5) & 3) * 4] = static_cast<uint8_t>(scale);
-    }
+  for (int r = 0; r < rows; ++r) {
+    const int slot = fetched ? __shfl_sync(0xffffffffu, tokens, r) : r;
+    float values[8];
+    const float maximum = stream_block_maximum(*reinterpret_cast<const uint4*>(b + kStTokensAt + slot * 512 + lane * 16), values);
+    uint32_t codes;
+    const uint32_t scale = stream_quantise(values, maximum, multiplier, smem->tables.reciprocals, codes);
+    *reinterpret_cast<uint32_t*>(b + r * kTileKBytes + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) = codes;
+    const int n = scale_row + r;
+    if ((lane & 1) == 0) sf[(n & 31) * 16 + ((n >> 5) & 3) * 4] = static_cast<uint8_t>(scale);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();
-  if (lane == 0) mbar_arrive(&smem->full[stage]);
+  if (lane == 0 && !dry) mbar_arrive(&smem->full[stage]);
+}
+
+// Offsets of the codes and the scale bytes of an expert's row (below 4 MB in batches of this size).
+__device__ __forceinline__ uint2 stream_route_at(const StreamSmem* smem, int expert, int rank) {
+  return make_uint2(static_cast<uint32_t>(smem->offsets[expert] + rank) * (kHidden / 2),
+                    static_cast<uint32_t>(smem->scale_rows[expert]) * (kHidden / 16) +
+                        static_cast<uint32_t>(sf_offset(rank, 0, kHidden / 16)));
 }
 
 // By the publisher warp of a CTA that has had nothing to do for a while: the grid's CTAs quantise two tokens each at most,
@@ -425,18 +495,14 @@ __device__ __noinline__ void stream_rescue_tokens(const StreamParams& p, StreamS
         rank += __popc(__ballot_sync(0xffffffffu, base + lane < route && p.expert_ids[base + lane] == expert));
       if (lane == 0) {
         const bool valid = expert >= 0 && expert < kExperts;
-        smem->route_row[k] = valid ? smem->offsets[expert] + rank : -1;
-        if (valid) {
-          smem->route_multiplier[k] = smem->scale_q1[expert];
-          smem->route_scale_base[k] = static_cast<unsigned long long>(smem->scale_rows[expert]) * (kHidden / 16) +
-                                      sf_offset(rank, 0, kHidden / 16);
-        }
+        smem->route_at[k] = valid ? stream_route_at(smem, expert, rank) : make_uint2(kStNoRow, 0);
+        smem->route_multiplier[k] = valid ? smem->scale_q1[expert] : 0.0f;
       }
     }
     __syncwarp();
     const uint4* const input = reinterpret_cast<const uint4*>(p.input) + static_cast<size_t>(token) * (kHidden / 8) + lane;
 #pragma unroll 1
-    for (int kb = 0; kb < kStUpKBlocks; ++kb) stream_quantise_token(p, smem, 0, kb, lane, __ldg(input + kb * (kTileK / 8)));
+    for (int kb = 0; kb < kStUpKBlocks; ++kb) stream_quantise_token(p.packed, p.scales, smem, 0, kb, lane, __ldg(input + kb * (kTileK / 8)), false);
     __syncwarp();
     if (lane == 0) stream_add_release(sync + kStreamRescued);
   }
@@ -467,6 +533,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     smem->published = 0;
     smem->first_mine = -1;
     smem->begun = 0;
+    smem->repeats = 0;
     smem->abort = 0;
     smem->left = 0;
     fence_barrier_init();
@@ -476,6 +543,10 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     prefetch_tensor_map(&maps.down[0]);
   }
   if (tid < kStClaims) smem->claims[tid] = 0;
+  if (kFront && tid < kTopK) {
+    smem->route_at[tid] = make_uint2(kStNoRow, 0);
+    smem->route_multiplier[tid] = 1.0f;
+  }
   if (warp == kStMmaWarp) {
     tmem_alloc(&smem->tmem_base, kStTmemColumns);
     tmem_relinquish();
@@ -484,12 +555,17 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
   __syncthreads();
   fill_geglu_tables(&smem->tables);
   if (kFront)
-    for (int i = tid; i < kStRankWarps * kExperts; i += kStThreads) (&smem->warp_counts[0][0])[i] = 0;
+    for (int i = tid; i < kExperts * kStFrontWords; i += kStThreads) (&smem->tokens_of[0][0])[i] = 0;
   grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = smem->tmem_base;
+  if (kFront && p.tokens > kStSelfRows && warp >= 4 && warp < 8) {
+    // the quantisers' code is brought in while the CTA has nothing else to do
+    stream_quantise_token(p.packed, p.scales, smem, 0, 0, lane, make_uint4(0, 0, 0, 0), true);
+    stream_quantise_stage(nullptr, smem, warp - 4, 0, 1, 0, true, 0, 1.0f, lane, true);
+  }
   grid_dependency_wait();  // what earlier kernels of the stream wrote is visible from here on
   int* const sync = p.plan.stream_sync;
   int first_taken = 0;
@@ -499,125 +575,118 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
   const bool has_token = kFront && cta < p.tokens;
   const int ctas = gridDim.x;
   const int routes = kFront ? p.tokens * kTopK : 0;
-  // warp 1 + w ranks routes [w * stretch, (w + 1) * stretch) among those of its own stretch
-  const bool ranks = warp > 0 && warp <= kStRankWarps;
-  const int rank_warp = ranks ? warp - 1 : 0;
-  const int stretch = ((routes + kStRankWarps - 1) / kStRankWarps + 31) & ~31;
-  const int stretch_begin = ranks ? rank_warp * stretch : routes;
-  const int stretch_end = stretch_begin + stretch < routes ? stretch_begin + stretch : routes;
+  const int words = (p.tokens + 31) >> 5;
   const int own = has_token ? (p.tokens - 1 - cta) / ctas + 1 : 0;
   const int kb = warp - kStMmaWarp;  // 0..10: the K block that the warp quantises
-  uint4 own_raw[kStOwnTokens];
+  // in a batch this small every token may be in the CTA's first item
+  const bool fetched = kFront && p.tokens <= kStSelfRows && kb < kStStages;
+  // Of the CTA's own tokens, that goes for warps 2..11; warp 3, which has no role later, takes the MMA warp's K block, too.
+  uint4 own_raw[kStOwnTokens], mma_raw[kStOwnTokens];
+  int own_expert = -1;  // publisher warp, a lane each of the CTA's own routes
+  int count = 0;  // threads 0..127: rows of expert tid
   if constexpr (kFront) {
     const float scale_q1 = tid < kExperts ? p.in_scale_q1[tid] : 0.0f;
-    int* const counts = smem->warp_counts[rank_warp];
-    uint8_t* const route_expert = smem->route_expert + rank_warp * kStStretch + lane;
-    uint32_t ids[kStStretch / 32];
+    int ids[kStFrontRoutes];
 #pragma unroll
-    for (int k = 0; k < kStStretch / 32; ++k) {
-      const int route = stretch_begin + 32 * k + lane;
-      ids[k] = route < stretch_end ? static_cast<uint32_t>(p.expert_ids[route]) : kExperts;
-    }
-    // of this CTA's tokens, a K block each that the warp will quantise (see below) is on its way meanwhile
-    const uint4* const own_input = reinterpret_cast<const uint4*>(p.input) + static_cast<size_t>(cta) * (kHidden / 8) + kb * (kTileK / 8) + lane;
-    if (kb >= 0 && kb < kStUpKBlocks) {
+    for (int k = 0; k < kStFrontRoutes; ++k) ids[k] = tid + k * kStThreads < routes ? p.expert_ids[tid + k * kStThreads] : -1;
+    const int own_route = (cta + lane / kTopK * ctas) * kTopK + lane % kTopK;
+    if (warp == kStPublishWarp && lane < own * kTopK) own_expert = p.expert_ids[own_route];
+    // what the warp will quantise (see below) is on its way meanwhile
+    const uint4* const input = reinterpret_cast<const uint4*>(p.input);
+    if (fetched && kb >= 0)
+      for (int t = 0; t < p.tokens; ++t) stream_fetch_token(smem->b[kb], t, input, t, kb, lane);
+    if (kb > 0 && kb < kStUpKBlocks) {
 #pragma unroll
       for (int t = 0; t < kStOwnTokens; ++t)
-        if (t < own) own_raw[t] = __ldg(own_input + static_cast<size_t>(t) * ctas * (kHidden / 8));
+        if (t < own) {
+          const uint4* const token = input + static_cast<size_t>(cta + t * ctas) * (kHidden / 8) + lane;
+          own_raw[t] = stream_load_now(token + kb * (kTileK / 8));
+          if (warp == kStSpareWarp) mma_raw[t] = stream_load_now(token);
+        }
     }
-    if (ranks)
+    // Every expert's tokens as bits; a bit found set is a token that names its expert twice.
+    uint32_t repeated = 0;
 #pragma unroll
-      for (int k = 0; k < kStStretch / 32; ++k) route_expert[32 * k] = static_cast<uint8_t>(ids[k] < kExperts ? ids[k] : kExperts);
-    __syncwarp();
-#pragma unroll 1
-    for (int base = stretch_begin; base < stretch_end; base += 32) {
-      const int route = base + lane;
-      const int expert = route_expert[base - stretch_begin];
-      if (expert == kExperts && cta == 0 && route < stretch_end) atomicExch(status, static_cast<int>(kBadExpertId));
-      const uint32_t peers = __match_any_sync(0xffffffffu, expert);
-      const int before = expert < kExperts ? counts[expert] : 0;
-      __syncwarp();
-      if (expert < kExperts && (peers & (0u - peers)) == (1u << lane)) counts[expert] = before + __popc(peers);
-      __syncwarp();
-      int token = (route >> 3) - cta;  // this CTA's are 0 and ctas
-      if (route < stretch_end && (token == 0 || token == ctas)) {
-        const int slot = (token ? kTopK : 0) + (route & (kTopK - 1));
-        smem->own_expert[slot] = expert;
-        smem->own_rank[slot] = before + __popc(peers & ((1u << lane) - 1u));
-        smem->own_warp[slot] = rank_warp;
+    for (int k = 0; k < kStFrontRoutes; ++k) {
+      const int route = tid + k * kStThreads;
+      if (route < routes) {
+        const uint32_t bit = 1u << ((route / kTopK) & 31);
+        if (ids[k] >= 0 && ids[k] < kExperts) repeated |= atomicOr(&smem->tokens_of[ids[k]][route / (32 * kTopK)], bit) & bit;
+        else if (cta == 0) atomicExch(status, static_cast<int>(kBadExpertId));
       }
+    }
+    if (repeated) smem->repeats = 1;
+    if (tid < kExperts) {
+      smem->scale_q1[tid] = scale_q1;
+      smem->histogram[tid] = 0;
     }
     __syncthreads();
-    if (tid < kExperts) {
-      int running = 0;
+    if (smem->repeats) {
+      // not what a router gives: counted one by one
 #pragma unroll
-      for (int w = 0; w < kStRankWarps; ++w) {
-        const int c = smem->warp_counts[w][tid];
-        smem->warp_counts[w][tid] = running;
-        running += c;
+      for (int k = 0; k < kStFrontRoutes; ++k)
+        if (ids[k] >= 0 && ids[k] < kExperts) atomicAdd(&smem->histogram[ids[k]], 1);
+      for (int q = warp; q < own * kTopK; q += kStThreads / 32) {
+        const int rank = stream_rank_repeated(p.expert_ids, (cta + q / kTopK * ctas) * kTopK + q % kTopK, lane);
+        if (lane == 0) smem->own_rank[q] = rank;
       }
-      smem->histogram[tid] = running;
-      smem->scale_q1[tid] = scale_q1;
+      __syncthreads();
+      if (tid < kExperts) count = smem->histogram[tid];
+    } else if (tid < kExperts) {
+#pragma unroll
+      for (int w = 0; w < kStFrontWords; ++w)
+        if (w < words) count += __popc(smem->tokens_of[tid][w]);
     }
   } else {
-    if (tid < kExperts) smem->histogram[tid] = p.plan.expert_offsets[tid + 1] - p.plan.expert_offsets[tid];
+    if (tid < kExperts) count = p.plan.expert_offsets[tid + 1] - p.plan.expert_offsets[tid];
   }
-  __syncthreads();
-  if (warp == 0) {
-    // lane l scans experts 4l..4l+3: rows, 128-row scale tiles, chunks
-    int counts[4], rows = 0, tiles = 0, chunks = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      counts[i] = smem->histogram[4 * lane + i];
-      rows += counts[i];
-      tiles += (counts[i] + kTileM - 1) / kTileM;
-      chunks += (counts[i] + kStRows - 1) / kStRows;
-    }
-    int rows_inclusive = rows, tiles_inclusive = tiles, chunks_inclusive = chunks;
+  if (tid < kExperts) {
+    // rows, 128-row scale tiles and chunks of the experts before this one, in one word
+    static_assert(kStreamMaxTokens * kTopK < (1 << 14) && kExperts + kStreamMaxTokens * kTopK / kTileM < (1 << 9) && kStMaxChunks < (1 << 9), "scan in one word");
+    const int tiles = (count + kTileM - 1) / kTileM, chunks = (count + kStRows - 1) / kStRows;
+    const uint32_t packed = static_cast<uint32_t>(count) | static_cast<uint32_t>(tiles) << 14 | static_cast<uint32_t>(chunks) << 23;
+    uint32_t inclusive = packed;
 #pragma unroll
     for (int offset = 1; offset < 32; offset <<= 1) {
-      const int r = __shfl_up_sync(0xffffffffu, rows_inclusive, offset);
-      const int t = __shfl_up_sync(0xffffffffu, tiles_inclusive, offset);
-      const int c = __shfl_up_sync(0xffffffffu, chunks_inclusive, offset);
-      if (lane >= offset) {
-        rows_inclusive += r;
-        tiles_inclusive += t;
-        chunks_inclusive += c;
-      }
+      const uint32_t other = __shfl_up_sync(0xffffffffu, inclusive, offset);
+      if (lane >= offset) inclusive += other;
     }
-    int row = rows_inclusive - rows, tile = tiles_inclusive - tiles, chunk = chunks_inclusive - chunks;
+    if (lane == 31) smem->scan[warp] = inclusive;
+    named_barrier(4, kExperts);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int expert = 4 * lane + i;
-      const int expert_tiles = (counts[i] + kTileM - 1) / kTileM;
-      const int expert_chunks = (counts[i] + kStRows - 1) / kStRows;
-      smem->offsets[expert] = row;
-      smem->scale_rows[expert] = tile * kTileM;
-      smem->chunks_of[expert] = expert_chunks;
-      for (int c = 0; c < expert_chunks; ++c) {
-        smem->chunk_expert[chunk + c] = static_cast<short>(expert);
-        smem->chunk_index[chunk + c] = static_cast<short>(c);
-      }
-      if (kFront && cta == 0) {
-        p.plan.expert_offsets[expert] = row;
-        p.plan.scale_row_offsets[expert] = tile * kTileM;
-        for (int t = 0; t < expert_tiles; ++t) p.plan.tile_expert[tile + t] = expert;
-      }
-      row += counts[i];
-      tile += expert_tiles;
-      chunk += expert_chunks;
+    for (int w = 0; w < kExperts / 32 - 1; ++w)
+      if (w < warp) inclusive += smem->scan[w];
+    const uint32_t before = inclusive - packed;
+    const int row = before & 0x3fffu, tile = before >> 14 & 0x1ffu, chunk = before >> 23;
+    smem->offsets[tid] = row;
+    smem->scale_rows[tid] = tile * kTileM;
+    smem->chunks_of[tid] = chunks;
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+      smem->chunk_expert[chunk + c] = static_cast<short>(tid);
+      smem->chunk_index[chunk + c] = static_cast<short>(c);
     }
-    if (lane == 31) {
-      if (cta < chunk * kStreamUpItems) smem->claims[0] = 1u << 16 | static_cast<uint32_t>(cta);
-      smem->offsets[kExperts] = row;
-      smem->scale_rows[kExperts] = tile * kTileM;
-      smem->chunks = chunk;
-      if (kFront && cta == 0) {
-        p.plan.expert_offsets[kExperts] = row;
-        p.plan.scale_row_offsets[kExperts] = tile * kTileM;
-        p.plan.num_m_tiles[0] = tile;
+    if (tid == kExperts - 1) {
+      const int all_chunks = chunk + chunks;
+      if (cta < all_chunks * kStreamUpItems) smem->claims[0] = 1u << 16 | static_cast<uint32_t>(cta);
+      smem->offsets[kExperts] = row + count;
+      smem->scale_rows[kExperts] = (tile + tiles) * kTileM;
+      smem->chunks = all_chunks;
+    }
+    if (kFront && cta == 0) {
+      p.plan.expert_offsets[tid] = row;
+      p.plan.scale_row_offsets[tid] = tile * kTileM;
+      for (int t = 0; t < tiles; ++t) p.plan.tile_expert[tile + t] = tid;
+      if (tid == kExperts - 1) {
+        p.plan.expert_offsets[kExperts] = row + count;
+        p.plan.scale_row_offsets[kExperts] = (tile + tiles) * kTileM;
+        p.plan.num_m_tiles[0] = tile + tiles;
       }
     }
+  }
+  if (fetched) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_proxy_async_smem();  // a stage whose tokens are not used after all is filled by a tensor-map copy
   }
   __syncthreads();
   const StreamShares shares(smem->chunks, ctas);
@@ -629,6 +698,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
   // the pipeline stages (not the concern of the weight and claim warps, which leave it out)
   bool self_first = kFront && cta < shares.up;
   if (kFront && warp != kStWeightWarp && warp != kStClaimWarp) {  // the weights are under way meanwhile
+    const uint4* const input = reinterpret_cast<const uint4*>(p.input);
     int first = 0, first_rows = 0;
     if (self_first) {
       it = cursor.item_of(cta, false, smem);
@@ -637,58 +707,67 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       first_rows = first_rows > kStRows ? kStRows : first_rows;
       self_first = first_rows <= kStSelfRows;  // with more, the grid's rows are there as early
     }
-    if (self_first) {
-      // the tokens of its rows, by the order of the sort
-      if (stretch_begin < stretch_end) {
-        int rank = smem->warp_counts[rank_warp][it.expert] - first;
+    float multiplier = 0.0f;
+    int tokens = 0;  // lane r: the token of row r of that item
+    if (self_first && warp != kStPublishWarp) {
+      multiplier = smem->scale_q1[it.expert];
+      if (smem->repeats) tokens = stream_token_of_row_repeated(p.expert_ids, routes, it.expert, first, lane);
+      else if (lane < first_rows) tokens = stream_token_of_row(smem, it.expert, first + lane, words);
+      __syncwarp();
+    }
+    // The CTA's own tokens come first where some CTA has a second item, which needs the grid's.
+    const bool own_first = shares.up > ctas;
 #pragma unroll 1
-        for (int base = stretch_begin; base < stretch_end; base += 32) {
-          const int route = base + lane;
-          const bool mine = smem->route_expert[rank_warp * kStStretch + route - stretch_begin] == it.expert;
-          const uint32_t all = __ballot_sync(0xffffffffu, mine);
-          const int r = rank + __popc(all & ((1u << lane) - 1u));
-          if (mine && r >= 0 && r < kStSelfRows) smem->first_token[r] = static_cast<short>(route >> 3);
-          rank += __popc(all);
+    for (int step = 0; step < 2; ++step) {
+      if ((step == 0) != own_first) {
+        if (self_first && warp != kStPublishWarp && kb < kStStages)
+          stream_quantise_stage(input, smem, kb, kb, first_rows, tokens, fetched, first % kTileM, multiplier, lane, false);
+      } else if (has_token && warp != kStMmaWarp) {
+        constexpr int kOwnThreads = kStUpKBlocks * 32;  // warps 2..12
+        if (warp == kStPublishWarp) {
+          // where this CTA's tokens' routes go
+          if (lane < own * kTopK) {
+            const int route = (cta + lane / kTopK * ctas) * kTopK + lane % kTopK;
+            const int expert = own_expert;
+            const bool valid = expert >= 0 && expert < kExperts;  // others are flagged above
+            if (valid) {
+              int rank = 0;
+              if (smem->repeats) {
+                rank = smem->own_rank[lane];
+              } else {
+                const int token = route / kTopK;
+#pragma unroll 1
+                for (int w = 0; w < token >> 5; ++w) rank += __popc(smem->tokens_of[expert][w]);
+                rank += __popc(smem->tokens_of[expert][token >> 5] & ((1u << (token & 31)) - 1u));
+              }
+              const int dst = smem->offsets[expert] + rank;
+              p.plan.sorted_experts[dst] = expert;
+              p.plan.sorted_routes[dst] = route;
+              p.plan.inverse_routes[route] = dst;
+              smem->route_at[lane] = stream_route_at(smem, expert, rank);
+            } else {
+              smem->route_at[lane] = make_uint2(kStNoRow, 0);
+            }
+            smem->route_multiplier[lane] = valid ? smem->scale_q1[expert] : 0.0f;
+          }
+          named_barrier(3, kOwnThreads);
+          named_barrier(1, kOwnThreads);
+          if (lane == 0) stream_add_release(sync + kStreamQuantised);
+        } else {
+          named_barrier(3, kOwnThreads);
+#pragma unroll 1
+          for (int t = 0; t < own; ++t) {
+            stream_quantise_token(p.packed, p.scales, smem, t * kTopK, kb, lane, own_raw[t ? 1 : 0], false);
+            if (warp == kStSpareWarp) stream_quantise_token(p.packed, p.scales, smem, t * kTopK, 0, lane, mma_raw[t ? 1 : 0], false);
+          }
+          asm volatile("bar.arrive 1, %0;" ::"n"(kOwnThreads) : "memory");
         }
       }
     }
-    const int q = tid - kStPublishWarp * 32;
-    if (q >= 0 && q < own * kTopK) {
-      // where this CTA's tokens' routes go
-      const int expert = smem->own_expert[q];
-      int dst = -1;
-      if (expert < kExperts) {  // others are flagged above
-        const int route = (cta + q / kTopK * ctas) * kTopK + q % kTopK;
-        const int rank = smem->warp_counts[smem->own_warp[q]][expert] + smem->own_rank[q];
-        dst = smem->offsets[expert] + rank;
-        p.plan.sorted_experts[dst] = expert;
-        p.plan.sorted_routes[dst] = route;
-        p.plan.inverse_routes[route] = dst;
-        smem->route_multiplier[q] = smem->scale_q1[expert];
-        smem->route_scale_base[q] = static_cast<unsigned long long>(smem->scale_rows[expert]) * (kHidden / 16) +
-                                      sf_offset(rank, 0, kHidden / 16);
-      }
-      smem->route_row[q] = dst;
-    }
-    named_barrier(3, kStThreads - 64);
-    const float multiplier = self_first ? smem->scale_q1[it.expert] : 0.0f;
-    if (has_token && kb >= 0) {
-      constexpr int kOwnThreads = (kStUpKBlocks + 1) * 32;
-      if (warp == kStPublishWarp) {
-        named_barrier(1, kOwnThreads);
-        if (lane == 0) stream_add_release(sync + kStreamQuantised);
-      } else {
-#pragma unroll 1
-        for (int t = 0; t < own; ++t) stream_quantise_token(p, smem, t * kTopK, kb, lane, own_raw[t ? 1 : 0]);
-        asm volatile("bar.arrive 1, %0;" ::"n"(kOwnThreads) : "memory");
-      }
-    }
-    if (self_first && kb >= 0 && kb < kStStages)
-      stream_quantise_stage(reinterpret_cast<const uint4*>(p.input), smem, kb, kb, first_rows, first % kTileM, multiplier, lane);
     if (self_first && kb >= kStStages && kb < kStUpKBlocks) {
       // the stage's second use
       if (__all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[kb - kStStages], 0u, smem, status)))
-        stream_quantise_stage(reinterpret_cast<const uint4*>(p.input), smem, kb - kStStages, kb, first_rows, first % kTileM, multiplier, lane);
+        stream_quantise_stage(input, smem, kb - kStStages, kb, first_rows, tokens, false, first % kTileM, multiplier, lane, false);
     }
   }
 

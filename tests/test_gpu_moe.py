@@ -692,6 +692,39 @@ def test_decode_kernel_that_sorts_and_quantises_itself(gm, weights, cuda_device,
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("tokens", [1, 8, 9, 32, 33, 65, 296])
+def test_streaming_front_with_experts_named_twice(gm, weights, cuda_device, tokens, monkeypatch):
+    """No router does it, but a token may name an expert more than once: the streaming launch, which ranks routes by
+    a bit per token and expert, then counts them one by one.  Against a runner that sorts and quantises in launches of its own:
+    plan, operand bytes, routed rows and output, and the same once more with ordinary ids on the same scratch."""
+    from gevva_b200 import runtime as rt
+    ids = random_ids(tokens, 61)
+    ids[tokens // 2, 5] = ids[tokens // 2, 2]
+    ids[:: 3, 7] = ids[:: 3, 0]
+    ids[-1] = 77
+    x = hashgen.activations(tokens, HIDDEN, 15, cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    routes = tokens * TOP_K
+    seen = []
+    for front in ("0", "1"):
+        monkeypatch.setenv("GEVVA_MOE_DECODE_FRONT", front)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        record = []
+        for batch in (ids, random_ids(tokens, 62)):
+            out = torch.zeros_like(x)
+            runner.launch_batch(x, torch.from_numpy(batch).to(cuda_device), rw, out, tokens)
+            runner.check()
+            record += [out, runner.buffer(rt.BUF_INPUT_CODES)[: routes * HIDDEN // 2].clone(),
+                       runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: routes * HIDDEN].clone(),
+                       runner.buffer(rt.BUF_EXPERT_OFFSETS, torch.int32).clone()]
+            record += [runner.buffer(b, torch.int32)[:routes].clone()
+                       for b in (rt.BUF_SORTED_EXPERTS, rt.BUF_SORTED_ROUTES, rt.BUF_INVERSE_ROUTES)]
+        seen.append(record)
+    for a, b in zip(*seen):
+        assert torch.equal(a, b)
+    assert seen[0][0].float().abs().max() > 0
+
+
 @pytest.mark.parametrize("tokens", [8, 9, 65, 72, 73, 137])
 def test_streaming_front_first_items(gm, weights, cuda_device, tokens, monkeypatch):
     """The streaming launch's CTAs quantise the rows of their first items themselves up to eight rows, also
