@@ -858,6 +858,33 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       }
     }
     __syncwarp();
+  } else if (kFront && warp == kStSpareWarp) {
+    // ---------------- what does not fit the ring ----------------
+    // A CTA whose first item waits for the grid's quantised rows has its ring full of weights meanwhile, and nothing moves.  So
+    // the rest of the item's weights and the start of the next item's are asked into L2: 100 tokens 502.6 -> 501.6 us a pass of six
+    // layers, 150 tokens 346.9 -> 344.4 (four), 200 tokens 356.5 -> 352.5, 290 tokens 368.8 -> 364.  (From every CTA: 1 token 171 -> 177,
+    // 64 tokens 647 -> 651, because there the ring is at work all the time; the whole next item: no better at 200, 657 at 64.)
+    if (!self_first && cta < shares.up && elect_one()) {
+#pragma unroll 1
+      for (int n = 0; n < 2; ++n) {
+        uint32_t word = smem->claims[n];
+        for (int spin = 0; (word >> 16) != 1 && spin < 200 && !smem->abort; ++spin) {
+          __nanosleep(32);
+          word = smem->claims[n];
+        }
+        if ((word >> 16) != 1 || (word & kStNoMoreClaims)) break;
+        const StreamItem ahead = cursor.item_of(static_cast<int>(word & 0xffffu), false, smem);
+        const uint8_t* sf = p.w13_scales + static_cast<size_t>(ahead.expert * kUnitSlots + ahead.n_tile) * kStUpKBlocks * kSfStageBytes;
+#pragma unroll 2
+        for (int k = n ? 0 : kStStages; k < (n ? kStUpKBlocks - kStStages : kStUpKBlocks); ++k) {
+          asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(&maps.w13), "r"(k * kTileKBytes),
+                       "r"(ahead.n_tile * 64), "r"(2 * ahead.expert)
+                       : "memory");
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(sf + k * kSfStageBytes), "r"(kSfStageBytes) : "memory");
+        }
+      }
+    }
+    __syncwarp();
   } else if (warp == kStMmaWarp) {
     // ---------------- scale copies and MMAs, in one thread ----------------
     if (elect_one()) {
