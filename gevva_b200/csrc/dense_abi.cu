@@ -52,8 +52,13 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
   gv::GemmOperands gate_up = d->gate_up;
   gate_up.wide = wide_items(tokens, gate_up.n_out, sm_count);
   gv::launch_grouped_gemm(gate_up, d->plan, sm_count, stream);
+  // Beside the experts this kernel is launched the ordinary way: its CTAs, one a token, would otherwise wait out the first
+  // projection on SMs that the streaming launch's last CTAs need (296 tokens with 16 dense SMs: 373 -> 2000 us for three layers,
+  // because tokens of CTAs that are not running are then quantised by the others one by one).  Whole layers in a graph, us, chained and
+  // ordinary: 16 tokens 271 and 268 (four layers), 100 tokens 371 and 368, 128 tokens 390 and 380.  A dozen CTAs fit anywhere.
+  const bool beside = sm_count < d->sm_count;
   gv::launch_gelu_quantize_fp8(d->gate_up_out, d->act_scales, d->weights.gate_scale, d->weights.up_scale,
-                               d->prod_fp8, d->prod_scales, tokens, stream);
+                               d->prod_fp8, d->prod_scales, tokens, beside && tokens > 12, stream);
   gv::GemmOperands down = d->down;
   down.out = out_unscaled;
   down.wide = wide_items(tokens, down.n_out, sm_count);
@@ -230,17 +235,22 @@ struct LayerWorkspace {
     bytes = used;
   }
 };
-// SMs that the dense MLP of a decode-sized layer gets beside the experts.  An expert launch of this size
+// SMs that the dense MLP of a layer whose experts stream gets beside them.  An expert launch of this size
 // holds its SMs from the router to its end, and its time is that of its weights' way through HBM, which 132
 // SMs fill as well as 148; the 18 MB of dense weights pass meanwhile.  With a few tokens the experts are
 // few and the dense side is the longer chain, so it gets more; 33 SMs hold the first projection's items of 128
 // weight rows in one wave, 17 those of 256 (whole layers in a graph, us, at 16 / 17 / 33 / 48 SMs: 1 token 46.4 / 38.9 / 34.4 /
 // 32.3, 4 tokens 52.8 / 45.0 / 44.2 / 43.4, 5 tokens 55.5 / 47.7 / 44.9 / 47.2, 8 tokens 60.5 / 52.1 / 54.2 / 57.4, 12 tokens
 // 62.7 / 62.3 / 64.2 / 68.1, 40 tokens 93.6 / 94.6 / 99.6 / -, 128 tokens 107.4 / 108.4 / 109.9 / -).
-// (48 and 16 SMs are the table's, not a matter of waves.)
-constexpr int kBesideTokens = 128;  // the range of the table; above it both sides take all SMs (sharing was not measured there)
+// Three layers at 0 (both sides take all SMs) / 20 / 24 / 28 / 33 / 40 / 48: 130 tokens 333 / 284 / 285 / 290 / 289 / 292 / 299,
+// 200 tokens 344 / 296 / 297 / 302 / 301 / 305 / 312, 256 tokens - / 306 / 305 / - / - / - / -, 296 tokens 363 / 333 / 325 / 316 / 313 / 317 / 324,
+// 400 tokens 355 / 364 / 331 / 335 / 333 / 333 / 338, 512 tokens 368 / - / 348 / - / 350 / 350 / 354, 640 tokens 390 / - / 403 / - / 376 / 379 / 385.
+// Above 640 tokens, where the experts no longer stream, sharing gains nothing (700 tokens 425 at 0, 422 at 40, 1024 479 and 488,
+// 2048 448 and 469).
+// (48, 22 and 16 SMs are the table's, not a matter of waves.)
+constexpr int kBesideTokens = 640;
 int dense_sms_beside(int tokens, int sms) {
-  const int wanted = tokens <= 4 ? 48 : tokens <= 6 ? 33 : tokens <= 12 ? 17 : 16;
+  const int wanted = tokens <= 4 ? 48 : tokens <= 6 ? 33 : tokens <= 12 ? 17 : tokens <= 128 ? 16 : tokens <= 256 ? 22 : 33;
   return wanted * 2 < sms ? wanted : sms / 2;
 }
 }  // namespace

@@ -160,8 +160,8 @@ gelu_quantize_fp8_kernel(const __nv_bfloat16* __restrict__ gate_up,
                          const float* __restrict__ activation_scales, float gate_w_scale,
                          float up_w_scale, uint8_t* __restrict__ out, float* __restrict__ scales) {
   __shared__ float scratch[kDenseThreads / 32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();  // the second projection's CTAs take the SMs that the first one leaves, not others
   const int row = blockIdx.x;
   const bool active = threadIdx.x < kDense / 8;
   const float gate_scale = __fmul_rn(activation_scales[row], gate_w_scale);
@@ -313,8 +313,13 @@ void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, in
 }
 
 void launch_gelu_quantize_fp8(const void* gate_up, const float* activation_scales, float gate_w_scale,
-                              float up_w_scale, uint8_t* out, float* scales, int rows,
+                              float up_w_scale, uint8_t* out, float* scales, int rows, bool serial_launch,
                               cudaStream_t stream) {
+  if (serial_launch) {
+    gelu_quantize_fp8_kernel<<<rows, kDenseThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(gate_up), activation_scales,
+                                                                 gate_w_scale, up_w_scale, out, scales);
+    return;
+  }
   launch_chained(gelu_quantize_fp8_kernel, dim3(rows), dim3(kDenseThreads), 0, stream,
                  static_cast<const __nv_bfloat16*>(gate_up), activation_scales, gate_w_scale, up_w_scale, out, scales);
 }

@@ -241,3 +241,24 @@ def test_layer_call_equals_its_parts(cuda_device, tokens):
         torch.cuda.synchronize()
         assert torch.equal(got, want)
     layer.experts.check()
+
+
+@pytest.mark.parametrize("tokens", [130, 256, 257, 296, 640, 641])
+def test_layers_beside_the_dense_mlp_in_a_graph(cuda_device, tokens):
+    """Layers of the sizes whose experts stream share the SMs with the dense MLP: a captured stack of three gives the bits of
+    the same layers on one stream, at the edges of the table of shares and of the range."""
+    from gevva_b200.synthetic import SyntheticStack
+    stack = SyntheticStack(3, 641, cuda_device, seed=9, distinct_experts=False)
+    hidden = hashgen.activations(tokens, HIDDEN, 5 + tokens, cuda_device)
+    want = stack.forward(hidden, concurrent=False).clone()
+    stack.forward(hidden)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = stack.forward(hidden)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    for layer in stack.layers:
+        layer.experts.check()
