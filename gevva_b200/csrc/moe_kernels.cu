@@ -222,20 +222,29 @@ __device__ __forceinline__ bool grid_barrier(int* sync, int ctas, int* status) {
   return passed != 0;
 }
 
-// The three phases above in one cooperative launch (chunks <= number of SMs): every CTA
-// counts its chunk, all meet at a grid barrier, every CTA scans the chunk histograms for
-// its own base (the group geometry is written by all of them with identical values) and
-// scatters its routes.
+// The three phases above in one launch.  Up to kSortAloneChunks chunks every CTA counts the others' routes, too, and waits for
+// none: the launch may then begin behind its predecessor, which a cooperative one does not here (3 us from the router's end
+// to the sort's first instruction), and counting takes less than meeting.  Beyond, the launch is cooperative (chunks <= number of
+// SMs): every CTA counts its chunk, all meet at a grid barrier, every CTA scans the chunk histograms.
+// Either way every CTA has its own base then (the group geometry is written by all of them with identical values) and
+// scatters its routes.  Cooperative and alone, same box, us a pass: 613 tokens 198.3 -> 191.9 (two layers), 1000 tokens 244.3 -> 237.5, 1500
+// tokens 267.4 -> 262, feed-forward layers of 300 tokens 331 -> 322 (three), 1024 tokens 323.5 -> 313.5 (two), 1500 tokens 383.7 -> 379.2; 2048
+// tokens 304.5 -> 301.5, but feed-forward layers of that size 437 -> 449, where the sort then takes SMs before the dense MLP does.
+constexpr int kSortAloneChunks = 12;
 __global__ void __launch_bounds__(kSortChunk)
-route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chunks, RoutePlan plan) {
+route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chunks, bool alone, RoutePlan plan) {
+  constexpr int kCopies = 16;  // of the counts of other chunks, so that fewer warps meet at a counter
   __shared__ int warp_counts[32 * kExperts];
+  __shared__ int fetched[32 * kExperts];  // alone: [before this chunk, behind it][copy][expert]
+  __shared__ int remapped[kExperts];
   __shared__ int scan_scratch[16];
   const int tid = threadIdx.x;
-  for (int i = tid; i < 32 * kExperts; i += kSortChunk) warp_counts[i] = 0;
+  for (int i = tid; i < 32 * kExperts; i += kSortChunk) warp_counts[i] = fetched[i] = 0;
   __syncthreads();
   grid_dependency_wait();  // the ids are written, and the plan's last readers are done
   grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
-  const int route = blockIdx.x * kSortChunk + tid;
+  const int chunk = blockIdx.x;
+  const int route = chunk * kSortChunk + tid;
   int expert = kExperts;
   if (route < routes) {
     expert = expert_ids[route];
@@ -246,31 +255,63 @@ route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chun
       expert = plan.remap[expert];
     }
   }
+  if (alone) {
+    if (plan.remap) {
+      if (tid < kExperts) remapped[tid] = plan.remap[tid];
+      __syncthreads();
+    }
+    int* const counts = fetched + (tid >> 5) % kCopies * kExperts;
+    constexpr int kAhead = 8;
+    for (int first = 0; first < chunks; first += kAhead) {
+      int ids[kAhead];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const int other = (first + k) * kSortChunk + tid;
+        ids[k] = first + k < chunks && first + k != chunk && other < routes ? expert_ids[other] : -1;
+      }
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k)
+        if (ids[k] >= 0 && ids[k] < kExperts)
+          atomicAdd(counts + (first + k > chunk ? kCopies * kExperts : 0) + (plan.remap ? remapped[ids[k]] : ids[k]), 1);
+    }
+  }
   const uint32_t peers = count_chunk(expert, warp_counts);
   __syncthreads();
-  if (tid < kExperts) {
-    int total = 0;
-    for (int w = 0; w < 32; ++w) total += warp_counts[w * kExperts + tid];
-    plan.chunk_hist[blockIdx.x * kExperts + tid] = total;
-  }
-  if (!grid_barrier(plan.sync, chunks, plan.status)) return;
-  // All chunk histograms, 32 chunks at a time: the whole CTA fetches them in one round of loads
-  // (128 threads walking them chunk by chunk is a chain of trips to L2), then expert `tid` adds
-  // its column from shared memory.
-  __shared__ int fetched[32 * kExperts];
   int before = 0, total = 0;
-  for (int first = 0; first < chunks; first += 32) {
-    const int count = chunks - first < 32 ? chunks - first : 32;
-    for (int i = tid; i < count * kExperts; i += kSortChunk) fetched[i] = __ldcg(&plan.chunk_hist[first * kExperts + i]);
-    __syncthreads();
+  if (tid < kExperts) {
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) total += warp_counts[w * kExperts + tid];
+  }
+  if (alone) {
     if (tid < kExperts) {
-      for (int c = 0; c < count; ++c) {
-        const int v = fetched[c * kExperts + tid];
-        if (first + c < static_cast<int>(blockIdx.x)) before += v;
-        total += v;
+      int behind = 0;
+#pragma unroll
+      for (int copy = 0; copy < kCopies; ++copy) {
+        before += fetched[copy * kExperts + tid];
+        behind += fetched[(kCopies + copy) * kExperts + tid];
       }
+      total += before + behind;
     }
-    __syncthreads();
+  } else {
+    if (tid < kExperts) plan.chunk_hist[chunk * kExperts + tid] = total;
+    total = 0;
+    if (!grid_barrier(plan.sync, chunks, plan.status)) return;
+    // All chunk histograms, 32 chunks at a time: the whole CTA fetches them in one round of loads
+    // (128 threads walking them chunk by chunk is a chain of trips to L2), then expert `tid` adds
+    // its column from shared memory.
+    for (int first = 0; first < chunks; first += 32) {
+      const int count = chunks - first < 32 ? chunks - first : 32;
+      for (int i = tid; i < count * kExperts; i += kSortChunk) fetched[i] = __ldcg(&plan.chunk_hist[first * kExperts + i]);
+      __syncthreads();
+      if (tid < kExperts) {
+        for (int c = 0; c < count; ++c) {
+          const int v = fetched[c * kExperts + tid];
+          if (first + c < chunk) before += v;
+          total += v;
+        }
+      }
+      __syncthreads();
+    }
   }
   if (tid < kExperts) {
     int running = publish_groups(total, routes, plan, scan_scratch) + before;
@@ -311,6 +352,10 @@ void launch_route_sort(const int* expert_ids, int routes, const RoutePlan& plan,
     return;
   }
   int chunks = (routes + kSortChunk - 1) / kSortChunk;
+  if (plan.sync != nullptr && chunks <= kSortAloneChunks) {
+    launch_chained(route_sort_fused_kernel, dim3(chunks), dim3(kSortChunk), 0, stream, expert_ids, routes, chunks, true, plan);
+    return;
+  }
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (plan.sync != nullptr && chunks <= current_sm_count() && cudaStreamIsCapturing(stream, &capture) == cudaSuccess) {
     // A cooperative launch (its CTAs meet at a grid barrier) that may also begin while the previous
@@ -329,7 +374,7 @@ void launch_route_sort(const int* expert_ids, int routes, const RoutePlan& plan,
     // A graph's kernel node may be cooperative; captured, the launch begins behind its predecessor in the
     // ordinary way (three plain launches before: 2 to 4 us of a layer in a graph, 297 to 2048 tokens).
     config.numAttrs = capture == cudaStreamCaptureStatusNone ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&config, route_sort_fused_kernel, expert_ids, routes, chunks, plan);
+    const cudaError_t e = cudaLaunchKernelEx(&config, route_sort_fused_kernel, expert_ids, routes, chunks, false, plan);
     if (e == cudaSuccess) return;
     (void)cudaGetLastError();  // not launchable as one grid here: fall through to the three launches
   }

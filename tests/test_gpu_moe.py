@@ -209,6 +209,22 @@ def test_route_sort_matches_oracle(gm, oracle, big_runner, cuda_device, tokens, 
     assert (got["tile_expert"][:tiles.sum()] == np.repeat(np.arange(EXPERTS), tiles)).all()
 
 
+@pytest.mark.parametrize("tokens", [256, 257, 640, 1151, 1153, 1535, 1536, 1537])
+def test_route_sort_at_the_edges_of_its_forms(gm, oracle, big_runner, cuda_device, tokens):
+    """Up to twelve chunks of 1024 routes every CTA of the one-launch sort counts the other chunks itself, beyond they meet: whole and
+    ragged last chunks on both sides, with experts that a token names twice and one that takes a route of every token."""
+    from gevva_b200 import runtime as rt
+    ids = random_ids(tokens, 7 + tokens)
+    ids[::5, 6] = ids[::5, 1]
+    ids[:, 3] = 99
+    big_runner.launch_stages(rt.STAGE_SORT, tokens, expert_ids=torch.from_numpy(ids).to(cuda_device))
+    assert big_runner.last_status() == 0
+    got = plan_arrays(gm, big_runner, tokens * TOP_K)
+    want = oracle.sort(ids)
+    for key in ("sorted_experts", "sorted_routes", "inverse", "offsets", "scale_rows"):
+        assert (got[key] == want[key]).all(), key
+
+
 def test_bad_expert_id_is_reported(gm, big_runner, cuda_device):
     from gevva_b200 import runtime as rt
     for tokens in (4, 300):
