@@ -1,0 +1,474 @@
+// The grouped w2 GEMM of the largest batches by CTA pairs: two 128-row tiles of an expert against the same output columns.
+//
+// What bounds it.  Operands in and rows out share the way between an SM and L2: 100 KB in take 0.72 us an item there, 48 KB out 0.84 to
+// 1.0 us, both 1.4 to 2.1.  One CTA a tile (grouped_gemm_down.cu) fetches 103 KB for 128 rows x 192 columns and takes 2 us; a pair
+// (tcgen05 cta_group::2, M = 256) needs the weights once for two row tiles, each CTA half of them: 66 KB an item and CTA.
+// Alone, one CTA a tile -> this (us): 2048 tokens 46.7 -> 47.5, 3000 tokens 57 -> 53, 4096 tokens 71 -> 68, 8192 tokens 132 -> 118, 16384 tokens
+// 248 -> 203; without its stores 44 at 4096 tokens and 115 at 16384.  Below, most experts have a single tile, whose pair fetches 132 KB
+// where one CTA fetches 103 (1024 tokens 36.2 -> 42.4).  Eight epilogue warps and stores without a cache hint make no difference.
+// Everything else is as in that file, whose column order, re-tiled scales and schedule this one shares: items of 192 columns, five to a
+// unit (three there: 2 % more at 16384 tokens), a tile's activations fetched once a unit, two accumulators, results stored from registers.  The last tile of an expert
+// with an odd number has no partner: its pair's second CTA fetches its half of the weights and stores nothing.
+//
+// Roles of each CTA (8 warps): 0 fetches weights, 1 copies scale factors and issues MMAs (in the first CTA, for both), 2 fetches
+// activations, 4..7 the epilogue; one thread each but for the last.  Loads of both CTAs complete on the first one's barriers, MMAs on
+// both's.  Every wait is bounded.
+#include "gv_common.cuh"
+#include "gv_cta_pair.cuh"
+#include "gv_gemm_parts.cuh"
+#include "gv_launchers.h"
+
+namespace gv {
+
+namespace {
+
+constexpr int kDpStages = 7;                    // weight stages: one K block of this CTA's half of 192 output columns
+constexpr int kDpSlots = 6;                     // K blocks of row tiles: the unit at work and the next
+constexpr int kDpKBlocks = 3;                   // 704 = 256 + 256 + 192
+constexpr int kDpLastMmas = 3;
+constexpr int kDpAtoms = kInter / 64;           // 11 scale atoms a row tile
+constexpr int kDpColumns = 192;                 // output columns of an item (MMA N)
+constexpr int kDpTiles = (kHidden + kDpColumns - 1) / kDpColumns;       // 15
+constexpr int kDpLastColumns = kHidden - (kDpTiles - 1) * kDpColumns;   // 128
+constexpr int kDpUnitTiles = 5;                 // items of a unit
+constexpr int kDpPairUnits = kDpTiles / kDpUnitTiles;                   // 5
+static_assert(kDpTiles % kDpUnitTiles == 0 && kDpLastColumns == 128, "units of whole items, the last one of N = 128");
+constexpr int kDpPieceRows = 32;                // weight rows of a copy: half a 64-column group
+// Tensor memory: two accumulators, the scales of the row tile at work (four columns an MMA), two K blocks'
+// weight scales (eight columns an MMA).
+constexpr int kDpAccStages = 2;
+constexpr uint32_t kDpSfaColumn = kDpAccStages * kDpColumns;
+constexpr uint32_t kDpSfbColumn = kDpSfaColumn + kDpAtoms * 4;
+constexpr uint32_t kDpTmemColumns = 512;
+static_assert(kDpSfbColumn + 2 * 32 <= kDpTmemColumns, "tensor memory budget");
+constexpr int kDpTokenBytes = 128 * kTileKBytes;            // 16 KiB
+constexpr int kDpPieceBytes = kDpPieceRows * kTileKBytes;   // 4 KiB
+constexpr int kDpWeightBytes = kDpColumns / 2 * kTileKBytes;  // 12 KiB
+constexpr int kDpWeightSfBytes = 2 * kSfStageBytes;
+constexpr int kDpWeightWarp = 0, kDpMmaWarp = 1, kDpTokenWarp = 2, kDpEpilogueWarp = 4;
+constexpr int kDpEpilogueWarps = 4;
+constexpr int kDpThreads = (kDpEpilogueWarp + kDpEpilogueWarps) * 32;
+
+struct alignas(1024) DownPairSmem {
+  uint8_t a[kDpSlots][kDpTokenBytes];
+  uint8_t b[kDpStages][kDpWeightBytes];
+  uint8_t sfa[kDpSlots][kSfStageBytes];
+  uint8_t sfb[kDpStages][kDpWeightSfBytes];
+  uint64_t a_full[kDpSlots], b_full[kDpStages];    // first CTA: the bytes have landed in both
+  uint64_t a_empty[kDpSlots], b_empty[kDpStages];  // both CTAs: the MMAs that read them have completed
+  uint64_t acc_full[kDpAccStages];                 // both CTAs
+  uint64_t acc_empty[kDpAccStages];                // first CTA: both CTAs' epilogues have copied the accumulator out
+  uint32_t tmem_base;
+  volatile int abort;
+  // by expert: first row, first row tile, pairs before it
+  int offsets[kExperts + 1], tiles[kExperts], pairs[kExperts + 1], scan[kExperts / 32];
+};
+constexpr size_t kDpSmemBytes = sizeof(DownPairSmem) + 1024;
+static_assert(kDpSmemBytes <= 232448, "shared memory budget of one sm_100 CTA");
+
+struct DownPairParams {
+  const float* alpha;
+  __nv_bfloat16* out;
+  const int* expert_offsets;
+  const int* scale_row_offsets;
+  int* status;
+  bool early_weights;
+};
+
+// A pair of row tiles of an expert, of which this CTA has one, and kDpUnitTiles column tiles [begin, begin + kDpUnitTiles).
+struct DownPairUnit {
+  int expert, begin;
+  int tile;        // this CTA's row tile
+  int row0, rows;  // its first sorted row, and how many it has (none: an odd tile's partner)
+  bool both;       // the pair's second tile exists
+};
+
+// Units are numbered pair by pair and dealt to the clusters in snake order, so that at any time the grid works on neighbouring
+// row tiles and an expert's weights are fetched from HBM once.
+struct DownPairSchedule {
+  const DownPairSmem* smem;
+  int round = 0, units;
+  __device__ explicit DownPairSchedule(const DownPairSmem* s) : smem(s), units(s->pairs[kExperts] * kDpPairUnits) {}
+  __device__ bool next(uint32_t rank, DownPairUnit& unit) {
+    const int clusters = static_cast<int>(gridDim.x) >> 1, mine = static_cast<int>(blockIdx.x) >> 1;
+    const int index = round * clusters + ((round & 1) ? clusters - 1 - mine : mine);
+    ++round;
+    if (index >= units) return false;  // only the last round is incomplete
+    const int pair = index / kDpPairUnits;
+    unit.begin = (index - pair * kDpPairUnits) * kDpUnitTiles;
+    int expert = 0;  // the last one with pairs[expert] <= pair
+#pragma unroll
+    for (int step = kExperts / 2; step; step >>= 1)
+      if (smem->pairs[expert + step] <= pair) expert += step;
+    unit.expert = expert;
+    const int first = 2 * (pair - smem->pairs[expert]);
+    const int expert_rows = smem->offsets[expert + 1] - smem->offsets[expert];
+    const int local = (first + static_cast<int>(rank)) * kTileM;
+    unit.tile = smem->tiles[expert] + first + static_cast<int>(rank);
+    unit.row0 = smem->offsets[expert] + local;
+    unit.rows = expert_rows - local < kTileM ? expert_rows - local : kTileM;
+    unit.both = expert_rows > (first + 1) * kTileM;
+    return true;
+  }
+};
+
+// 32 weight rows in the column order of grouped_gemm_down.cu: half `half` of 64-column group `group`.
+__device__ __forceinline__ void down_pair_load_weights(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int half,
+                                                       int group) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%2, %3, %3, %4, %5}], [%6];" ::"r"(smem_u32(smem_dst)),
+      "l"(tensor_map), "r"(x), "r"(0), "r"(half * 4), "r"(group), "r"(barrier)
+      : "memory");
+}
+
+// 16 lanes x 64 columns: register 4g + i holds columns 8g + 2t + (i & 1) of row lane/4 + 8 * (i / 2).
+__device__ __forceinline__ void down_pair_load_16x64(uint32_t tmem_address, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(tmem_address)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(kDpThreads, 1)
+grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_sf,
+                         const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b_sf,
+                         const DownPairParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  DownPairSmem* smem = reinterpret_cast<DownPairSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_cta_rank();
+  const bool is_leader = rank == 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kDpSlots; ++s) {
+      mbar_init(&smem->a_full[s], 1);   // the first CTA's producer announces both CTAs' byte count
+      mbar_init(&smem->a_empty[s], 1);
+    }
+    for (int s = 0; s < kDpStages; ++s) {
+      mbar_init(&smem->b_full[s], 1);
+      mbar_init(&smem->b_empty[s], 1);
+    }
+    for (int s = 0; s < kDpAccStages; ++s) {
+      mbar_init(&smem->acc_full[s], 1);
+      mbar_init(&smem->acc_empty[s], 2 * kDpEpilogueWarps);
+    }
+    smem->abort = 0;
+    fence_barrier_init();
+    prefetch_tensor_map(&map_a);
+    prefetch_tensor_map(&map_a_sf);
+    prefetch_tensor_map(&map_b);
+    prefetch_tensor_map(&map_b_sf);
+  }
+  if (warp == kDpMmaWarp) {
+    tmem_alloc(&smem->tmem_base, kDpTmemColumns);  // the whole tensor memory: both CTAs get address 0
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  // Barriers of both CTAs exist before either CTA arrives on the other's.
+  cluster_sync_all();
+  const uint32_t tmem_base = smem->tmem_base;
+  // The weights and the plan come from before the previous kernel, which let this one start after its own wait.
+  if (!p.early_weights) grid_dependency_wait();
+  if (warp < kExperts / 32) {
+    // thread = expert: pairs before it
+    const int e = threadIdx.x;
+    const int row = p.expert_offsets[e], next_row = p.expert_offsets[e + 1];
+    const int own = (next_row - row + 2 * kTileM - 1) / (2 * kTileM);
+    int inclusive = own;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
+      if (lane >= offset) inclusive += other;
+    }
+    if (lane == 31) smem->scan[warp] = inclusive;
+    smem->offsets[e] = row;
+    smem->tiles[e] = p.scale_row_offsets[e] / kTileM;
+    if (e == kExperts - 1) smem->offsets[kExperts] = next_row;
+    named_barrier(1, kExperts);
+    for (int w = 0; w < warp; ++w) inclusive += smem->scan[w];
+    smem->pairs[e] = inclusive - own;
+    if (e == kExperts - 1) smem->pairs[kExperts] = inclusive;
+  }
+  __syncthreads();
+  if (warp != kDpWeightWarp) {
+    grid_dependency_wait();
+    grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
+  }
+
+  DownPairSchedule schedule(smem);
+  DownPairUnit unit;
+  bool ok = true;
+
+  if (warp == kDpWeightWarp) {
+    // ---------------- weights: this CTA's half of every column tile of every unit, three K blocks each ----------------
+    if (elect_one()) {
+      const uint32_t full0 = is_leader ? smem_u32(&smem->b_full[0]) : cluster_map_shared(smem_u32(&smem->b_full[0]), 0);
+      int stage = 0, issued = 0;
+      uint32_t phase = 0;
+      while (ok && schedule.next(rank, unit)) {
+        for (int n = unit.begin; ok && n < unit.begin + kDpUnitTiles; ++n) {
+          const int pieces = n + 1 == kDpTiles ? kDpLastColumns / 2 / kDpPieceRows : kDpColumns / 2 / kDpPieceRows;
+          const int group0 = unit.expert * (kHidden / 64) + (kDpColumns / 64) * n;
+          const int sf_row = (unit.expert * kDpTiles + n) * kDpKBlocks * 8;
+#pragma unroll
+          for (int kb = 0; kb < kDpKBlocks; ++kb) {
+            ok = wait_or_abort<true>(&smem->b_empty[stage], phase ^ 1u, smem, p.status);
+            if (!ok) break;
+            const uint32_t bar = full0 + 8 * stage;
+            if (is_leader)
+              mbar_arrive_expect_tx(&smem->b_full[stage], 2u * (static_cast<uint32_t>(pieces) * kDpPieceBytes + kDpWeightSfBytes));
+#pragma unroll
+            for (int j = 0; j < kDpColumns / 2 / kDpPieceRows; ++j) {
+              const int piece = static_cast<int>(rank) * pieces + j;
+              if (j < pieces)
+                down_pair_load_weights(smem->b[stage] + j * kDpPieceBytes, &map_b, bar, kb * kTileKBytes, piece & 1, group0 + (piece >> 1));
+            }
+            pair_load(smem->sfb[stage], &map_b_sf, bar, 0, sf_row + 8 * kb);
+            ++issued;
+            if (++stage == kDpStages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+        }
+      }
+      if (!ok && is_leader) {
+        // Unwinding: the copies already issued (by either CTA) land before shared memory is given up; the second CTA stays
+        // resident until the cluster barrier at the end.
+        const int pending = issued < kDpStages ? issued : kDpStages;
+        for (int i = 0; i < pending; ++i) {
+          if (--stage < 0) {
+            stage = kDpStages - 1;
+            phase ^= 1u;
+          }
+          mbar_wait_bounded(&smem->b_full[stage], phase, 40000000ll);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == kDpTokenWarp) {
+    // ---------------- activations: this CTA's row tile of every unit once ----------------
+    if (elect_one()) {
+      const uint32_t full0 = is_leader ? smem_u32(&smem->a_full[0]) : cluster_map_shared(smem_u32(&smem->a_full[0]), 0);
+      int slot = 0, issued = 0;
+      uint32_t phase = 0;
+      while (ok && schedule.next(rank, unit)) {
+#pragma unroll
+        for (int kb = 0; kb < kDpKBlocks; ++kb) {
+          ok = wait_or_abort<true>(&smem->a_empty[slot], phase ^ 1u, smem, p.status);
+          if (!ok) break;
+          const uint32_t bar = full0 + 8 * slot;
+          if (is_leader) mbar_arrive_expect_tx(&smem->a_full[slot], (unit.both ? 2u : 1u) * (kDpTokenBytes + kSfStageBytes));
+          if (is_leader || unit.both) {
+            // (the last K block's fourth atom is the next tile's first; nothing reads it)
+            pair_load(smem->a[slot], &map_a, bar, kb * kTileKBytes, unit.row0);
+            pair_load(smem->sfa[slot], &map_a_sf, bar, 0, unit.tile * kDpAtoms + 4 * kb);
+          }
+          ++issued;
+          if (++slot == kDpSlots) {
+            slot = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      if (!ok && is_leader) {
+        const int pending = issued < kDpSlots ? issued : kDpSlots;
+        for (int i = 0; i < pending; ++i) {
+          if (--slot < 0) {
+            slot = kDpSlots - 1;
+            phase ^= 1u;
+          }
+          mbar_wait_bounded(&smem->a_full[slot], phase, 40000000ll);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == kDpMmaWarp) {
+    // ---------------- first CTA: scale copies and MMAs for both, in one thread ----------------
+    // They execute in order, so two buffers for the weight scales are enough.  The scales of a row tile are copied once a unit.
+    if (is_leader && elect_one()) {
+      constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);                // 8 rows x 16 B, no swizzle
+      constexpr uint32_t hi_ab = (1024u >> 4) | (1u << 14) | (2u << 29);  // 8 rows x 128 B, 128B swizzle
+      const uint32_t a_lo0 = (smem_u32(smem->a[0]) & 0x3ffffu) >> 4, b_lo0 = (smem_u32(smem->b[0]) & 0x3ffffu) >> 4;
+      const uint32_t sfa_lo0 = (smem_u32(smem->sfa[0]) & 0x3ffffu) >> 4, sfb_lo0 = (smem_u32(smem->sfb[0]) & 0x3ffffu) >> 4;
+      int stage = 0, buffer = 0, acc = 0, slot0 = 0;  // slot0: the unit's first K block
+      uint32_t phase = 0, acc_phase = 0, slot0_phase = 0;
+      bool landed = false;  // the next stage's bytes have been seen
+      while (ok && schedule.next(rank, unit)) {
+        for (int n = unit.begin; ok && n < unit.begin + kDpUnitTiles; ++n) {
+          ok = wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status);
+          if (!ok) break;
+          tc_fence_after_sync();
+          // E2M1 x E2M1, both K-major, UE4M3 scales; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
+          const uint32_t columns = n + 1 == kDpTiles ? kDpLastColumns : kDpColumns;
+          const uint32_t descriptor = (1u << 7) | (1u << 10) | ((columns >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
+          const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc) * kDpColumns;
+#pragma unroll
+          for (int kb = 0; kb < kDpKBlocks; ++kb) {
+            constexpr int kMmas[kDpKBlocks] = {4, 4, kDpLastMmas};
+            const int slot = slot0 + kb;  // units start at slot 0 or 3
+            if (n == unit.begin) ok = wait_or_abort<false>(&smem->a_full[slot], slot0_phase, smem, p.status);
+            if (ok && !landed) ok = wait_or_abort<false>(&smem->b_full[stage], phase, smem, p.status);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint32_t tmem_sfa = tmem_base + kDpSfaColumn + static_cast<uint32_t>(16 * kb);
+            const uint32_t tmem_sfb = tmem_base + kDpSfbColumn + static_cast<uint32_t>(buffer) * 32;
+            if (n == unit.begin) {
+              const uint32_t sfa = sfa_lo0 + static_cast<uint32_t>(slot) * (kSfStageBytes >> 4);
+#pragma unroll
+              for (int j = 0; j < kMmas[kb]; ++j) pair_copy_sf(tmem_sfa + 4 * j, hi_sf, sfa + 32 * j);
+            }
+            const uint32_t sfb = sfb_lo0 + static_cast<uint32_t>(stage) * (kDpWeightSfBytes >> 4);
+            const uint32_t a = a_lo0 + static_cast<uint32_t>(slot) * (kDpTokenBytes >> 4);
+            const uint32_t b = b_lo0 + static_cast<uint32_t>(stage) * (kDpWeightBytes >> 4);
+            uint64_t* const empty = &smem->b_empty[stage];
+            if (++stage == kDpStages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+#pragma unroll
+            for (int j = 0; j < kMmas[kb]; ++j) {
+              pair_copy_sf(tmem_sfb + 8 * j, hi_sf, sfb + 32 * j);
+              pair_copy_sf(tmem_sfb + 8 * j + 4, hi_sf, sfb + 128 + 32 * j);
+            }
+#pragma unroll
+            for (int j = 0; j < kMmas[kb]; ++j)
+              pair_mma(tmem_acc, hi_ab, a + 2 * j, b + 2 * j, descriptor, tmem_sfa + 4 * j, tmem_sfb + 8 * j, (kb | j) != 0 ? 1u : 0u);
+            landed = mbar_try_wait(&smem->b_full[stage], phase);
+            pair_commit_both(empty);
+            if (n + 1 == unit.begin + kDpUnitTiles) pair_commit_both(&smem->a_empty[slot]);
+            if (kb + 1 == kDpKBlocks) pair_commit_both(&smem->acc_full[acc]);
+            buffer ^= 1;
+          }
+          if (++acc == kDpAccStages) {
+            acc = 0;
+            acc_phase ^= 1u;
+          }
+        }
+        slot0 += kDpKBlocks;
+        if (slot0 == kDpSlots) {
+          slot0 = 0;
+          slot0_phase ^= 1u;
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp >= kDpEpilogueWarp) {
+    // ---------------- epilogue: 64 columns of 16 rows at a time ----------------
+    static_assert(kDpEpilogueWarps == 4 && kDpSlots == 2 * kDpKBlocks, "a quarter of the rows each; units start at slot 0 or 3");
+    const int quarter = warp & 3;                        // the tensor-memory lanes this warp may read
+    constexpr int kParts = 2;                            // 16-row parts of the quarter
+    const int row_in_tile = quarter * 32 + (lane >> 2);  // and 8, 16 and 24 further down
+    const uint32_t tmem_rows = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    unsigned long long keep_in_l2;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep_in_l2));
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    while (ok && schedule.next(rank, unit)) {
+      const float alpha = p.alpha[unit.expert];
+      const int warp_rows = unit.rows - quarter * 32;  // of this warp's quarter that exist
+      for (int n = unit.begin; n < unit.begin + kDpUnitTiles; ++n) {
+        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, p.status));
+        if (!ok) break;
+        tc_fence_after_sync();
+        const int groups = n + 1 == kDpTiles ? kDpLastColumns / 64 : kDpColumns / 64;
+        const int steps = warp_rows <= 0 ? 0 : (warp_rows <= 16 ? 1 : kParts) * groups;  // none of rows that do not exist
+        bool released = false;
+        int step = 0;
+#pragma unroll 1
+        do {
+          uint32_t r[32];
+          const int part = step >= groups ? 1 : 0, group = step - part * groups;
+          if (step < steps) {
+            down_pair_load_16x64(tmem_rows + (static_cast<uint32_t>(part * 16) << 16) + static_cast<uint32_t>(acc) * kDpColumns + 64 * group, r);
+            tmem_load_wait();
+          }
+          if (step + 1 >= steps) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+              if (is_leader) mbar_arrive(&smem->acc_empty[acc]);
+              else pair_arrive_remote(&smem->acc_empty[acc], 0);
+            }
+            released = true;
+          }
+          if (step >= steps) break;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int row = row_in_tile + 16 * part + 8 * half;
+            if (row >= unit.rows) continue;
+            uint32_t v[8];
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              v[g] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(r[4 * g + 2 * half])),
+                                 __fmul_rn(alpha, __uint_as_float(r[4 * g + 2 * half + 1])));
+            const int column = n * kDpColumns + 64 * group + (lane & 3) * 16;
+            // read back by the weighted reduce right after this launch: L2 is asked to keep it
+            asm volatile("st.global.L2::cache_hint.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8}, %9;" ::"l"(
+                             p.out + static_cast<size_t>(unit.row0 + row) * kHidden + column),
+                         "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "l"(keep_in_l2)
+                         : "memory");
+          }
+          ++step;
+        } while (!released);
+        if (++acc == kDpAccStages) {
+          acc = 0;
+          acc_phase ^= 1u;
+        }
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  // Both CTAs stay until neither can still receive a remote arrive, a copy or a commit.
+  cluster_sync_all();
+  if (warp == kDpMmaWarp) {
+    tc_fence_after_sync();
+    __syncwarp();
+    tmem_dealloc(tmem_base, kDpTmemColumns);
+  }
+}
+
+}  // namespace
+
+int prepare_grouped_down_pairs() {
+  return static_cast<int>(cudaFuncSetAttribute(grouped_down_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kDpSmemBytes)));
+}
+
+void launch_grouped_down_pairs(const GemmOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream) {
+  DownPairParams p{};
+  p.alpha = op.alpha;
+  p.out = static_cast<__nv_bfloat16*>(op.out);
+  p.expert_offsets = plan.expert_offsets;
+  p.scale_row_offsets = plan.scale_row_offsets;
+  p.status = plan.status;
+  p.early_weights = op.early_weights;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(sm_count & ~1));
+  config.blockDim = dim3(kDpThreads);
+  config.dynamicSmemBytes = kDpSmemBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = 2;
+  attributes[0].val.clusterDim.y = 1;
+  attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = 2;
+  cudaLaunchKernelEx(&config, grouped_down_pair_kernel, op.map_a, op.map_down_a_sf, op.map_down_pieces, op.map_down_b_sf, p);
+}
+
+}  // namespace gv

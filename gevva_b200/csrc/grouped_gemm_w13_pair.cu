@@ -27,6 +27,7 @@
 // through shared memory by sixteen warps that traffic bounded the kernel, 107 us at 4096 tokens; with this epilogue
 // twelve or sixteen warps are 3 to 8 % slower than eight, and five stages up to 8 % slower than six.)  Every wait is bounded.
 #include "gv_common.cuh"
+#include "gv_cta_pair.cuh"
 #include "gv_gemm_parts.cuh"
 #include "gv_launchers.h"
 
@@ -71,69 +72,12 @@ struct alignas(1024) WpSmem {
 constexpr size_t kWpSmemBytes = sizeof(WpSmem) + 1024;
 static_assert(kWpSmemBytes <= 232448, "shared memory budget");
 
-__device__ __forceinline__ void wp_arrive_remote(uint64_t* local_bar, uint32_t target_cta) {
-  const uint32_t remote = cluster_map_shared(smem_u32(local_bar), target_cta);
-  // Relaxed: the arrive announces that tensor-memory reads have completed (tcgen05.wait::ld came
-  // before it); no memory written by this thread has to be visible to the leader, and a release
-  // here would first wait for the thread's earlier global stores.
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
-}
-
-// Arrives on the barrier at the same shared-memory offset in both CTAs of the pair once every
-// tcgen05 operation issued so far by this thread has completed.
-__device__ __forceinline__ void wp_commit_both(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(static_cast<uint16_t>(3))
-      : "memory");
-}
-
-// Tensor-map load into this CTA's shared memory that completes on a barrier of either CTA of the
-// pair (`barrier` is a shared::cluster address).  No multicast: every CTA loads its own bytes.
-__device__ __forceinline__ void wp_load(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(smem_dst)),
-      "l"(tensor_map), "r"(x), "r"(y), "r"(barrier)
-      : "memory");
-}
-
-__device__ __forceinline__ void wp_load_3d(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int y,
-                                           int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(smem_dst)),
-      "l"(tensor_map), "r"(x), "r"(y), "r"(z), "r"(barrier)
-      : "memory");
-}
-
 // The 128 weight rows of a unit in the kernel's order: see make_w13_fragment_map (moe_abi.cu).
 __device__ __forceinline__ void wp_load_weights(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int block) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
       " [%0], [%1, {%2, %3, %3, %3, %4}], [%5];" ::"r"(smem_u32(smem_dst)),
       "l"(tensor_map), "r"(x), "r"(0), "r"(block), "r"(barrier)
-      : "memory");
-}
-
-__device__ __forceinline__ void wp_copy_sf(uint32_t tmem_address, uint32_t hi, uint32_t lo) {
-  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_address),
-               "l"((static_cast<uint64_t>(hi) << 32) | lo)
-               : "memory");
-}
-
-__device__ __forceinline__ void wp_mma(uint32_t tmem_d, uint32_t hi, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
-                                       uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X"
-      " [%0], %1, %2, %3, [%5], [%6], p;\n\t"
-      "}" ::"r"(tmem_d),
-      "l"((static_cast<uint64_t>(hi) << 32) | a_lo), "l"((static_cast<uint64_t>(hi) << 32) | b_lo), "r"(idesc),
-      "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
       : "memory");
 }
 
@@ -144,9 +88,9 @@ __device__ __forceinline__ void wp_issue_sf_copies(uint32_t tmem_sf, uint32_t sf
   constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);                // 8 rows x 16 B, no swizzle
 #pragma unroll
   for (uint32_t j = 0; j < 4; ++j) {
-    wp_copy_sf(tmem_sf + 12 * j, hi_sf, sfw_lo + 32 * j);
-    wp_copy_sf(tmem_sf + 12 * j + 4, hi_sf, sfx_lo + 32 * j);
-    if (kTwoBlocks) wp_copy_sf(tmem_sf + 12 * j + 8, hi_sf, sfx_lo + 128 + 32 * j);
+    pair_copy_sf(tmem_sf + 12 * j, hi_sf, sfw_lo + 32 * j);
+    pair_copy_sf(tmem_sf + 12 * j + 4, hi_sf, sfx_lo + 32 * j);
+    if (kTwoBlocks) pair_copy_sf(tmem_sf + 12 * j + 8, hi_sf, sfx_lo + 128 + 32 * j);
   }
 }
 
@@ -155,7 +99,7 @@ __device__ __forceinline__ void wp_issue_mmas(uint32_t tmem_acc, uint32_t tmem_s
   constexpr uint32_t hi_ab = (1024u >> 4) | (1u << 14) | (2u << 29);  // 8 rows x 128 B, 128B swizzle
 #pragma unroll
   for (uint32_t j = 0; j < 4; ++j)
-    wp_mma(tmem_acc, hi_ab, w_lo + 2 * j, x_lo + 2 * j, idesc, tmem_sf + 12 * j, tmem_sf + 12 * j + 4 + shift,
+    pair_mma(tmem_acc, hi_ab, w_lo + 2 * j, x_lo + 2 * j, idesc, tmem_sf + 12 * j, tmem_sf + 12 * j + 4 + shift,
            j == 0 ? accumulate : 1u);
 }
 
@@ -334,10 +278,10 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           if (is_leader) mbar_arrive_expect_tx(&smem->full[stage], both_bytes);
           if (weight_side) {
             if (unit_exists) wp_load_weights(smem->w[stage], &map_w, bar, x, item.expert * (kW13Out / 16) + unit * 4);
-            wp_load(smem->sfw[stage], &map_w_sf, bar, 0, w_sf_row + 4 * kb);
+            pair_load(smem->sfw[stage], &map_w_sf, bar, 0, w_sf_row + 4 * kb);
           } else {
-            wp_load(smem->x[stage], token_map, bar, x, token_row);
-            wp_load_3d(smem->sfx[stage], &map_x_sf, bar, 0, 4 * kb, item.first);
+            pair_load(smem->x[stage], token_map, bar, x, token_row);
+            pair_load_3d(smem->sfx[stage], &map_x_sf, bar, 0, 4 * kb, item.first);
           }
         }
         __syncwarp();
@@ -400,8 +344,8 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
             if (two_blocks) wp_issue_sf_copies<true>(tmem_sf, sfw_lo, sfx_lo);
             else wp_issue_sf_copies<false>(tmem_sf, sfw_lo, sfx_lo);
             wp_issue_mmas(tmem_acc, tmem_sf, item.shift, w_lo, x_lo, idesc, kb != 0 ? 1u : 0u);
-            wp_commit_both(&smem->empty[stage]);   // both CTAs may refill the stage
-            if (kb + 1 == k_blocks) wp_commit_both(&smem->acc_full[acc]);
+            pair_commit_both(&smem->empty[stage]);   // both CTAs may refill the stage
+            if (kb + 1 == k_blocks) pair_commit_both(&smem->acc_full[acc]);
           }
           if (++stage == kWpStages) {
             stage = 0;
@@ -459,7 +403,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           __syncwarp();
           if (lane == 0) {
             if (is_leader) mbar_arrive(&smem->acc_empty[acc]);
-            else wp_arrive_remote(&smem->acc_empty[acc], 0);
+            else pair_arrive_remote(&smem->acc_empty[acc], 0);
           }
           released = true;
         }

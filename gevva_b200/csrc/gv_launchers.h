@@ -86,6 +86,7 @@ struct GemmOperands {
   CUtensorMap map_b64;      // CTA-pair fused w13 form: the same matrix through a 64-row box
   CUtensorMap map_b_units;  // fused w13 form: [experts * 2 halves, 704 rows, 1408 bytes], box 2 x 64 rows x 128 B
   CUtensorMap map_b_down;   // w2: the weights in the column order of grouped_gemm_down.cu
+  CUtensorMap map_down_pieces, map_down_a_sf, map_down_b_sf;  // grouped_gemm_down_pair.cu: 32 rows of it, and the scales
   CUtensorMap map_a_sf;     // CTA-pair form: a_scales as [atoms of 512 B][128 x u32], box of four atoms
   CUtensorMap map_b_sf;     // CTA-pair form: b_scales likewise; box of eight atoms (fused w13) or four (w2)
   const uint8_t* a_scales;  // activation scale regions
@@ -136,6 +137,9 @@ bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t expert
 // The w2 GEMM of prefill-sized batches (grouped_gemm_down.cu): op.map_a, map_b_down, down_scales.
 size_t retiled_w2_scale_bytes(int experts);
 void launch_retile_w2_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, cudaStream_t stream);
+// The same by CTA pairs (grouped_gemm_down_pair.cu): op.map_a, map_down_pieces, map_down_a_sf, map_down_b_sf; all row tiles, no row_dest.
+int prepare_grouped_down_pairs();
+void launch_grouped_down_pairs(const GemmOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
 void launch_grouped_down(const GemmOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
 int prepare_grouped_down();
 

@@ -26,6 +26,9 @@ using namespace gv;
 
 constexpr int kMaxTokens = 131072;
 constexpr int kStreamTokens = 640;  // see moe_launch_stages_on
+// w2 by CTA pairs that share weights between two row tiles of an expert: from 160 rows an expert on average (figures in
+// grouped_gemm_down_pair.cu; 2048 tokens 46.7 us by one CTA a tile and 47.5 by pairs, 3000 tokens 57 and 53).
+constexpr int kDownPairTokens = 2560;
 static_assert(kStreamTokens <= gv::kStreamMaxTokens, "the streaming kernel's chunk list");
 
 // The CUDA face of the allocator that gv_scratch.h takes as a parameter.
@@ -133,11 +136,12 @@ bool make_w13_fragment_map(CUtensorMap* map, const void* base, uint64_t experts)
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts) {
+// w2 codes in the row order of grouped_gemm_down.cu: a box of `groups` 64-row groups, or of half a one (0).
+bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts, int groups = 3) {
   constexpr cuuint64_t row = kInter / 2;
   const cuuint64_t dims[5] = {row, 2, 4, 8, experts * kHidden / 64};
   const cuuint64_t strides[4] = {row, 16 * row, 2 * row, 64 * row};
-  const cuuint32_t box[5] = {static_cast<cuuint32_t>(kTileKBytes), 2, 4, 8, 3};
+  const cuuint32_t box[5] = {static_cast<cuuint32_t>(kTileKBytes), 2, 4, groups ? 8u : 4u, groups ? static_cast<cuuint32_t>(groups) : 1u};
   const cuuint32_t element_strides[5] = {1, 1, 1, 1, 1};
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return false;
@@ -385,7 +389,8 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
     gv::GemmOperands w2 = runner->w2;
     w2.use_pairs = use_pairs;
     w2.early_weights = behind_w13;
-    gv::launch_grouped_gemm(w2, s->plan, sm_count, stream);
+    if (!use_pairs && sm_count >= 2 && tokens >= kDownPairTokens) gv::launch_grouped_down_pairs(w2, s->plan, sm_count, stream);
+    else gv::launch_grouped_gemm(w2, s->plan, sm_count, stream);
   }
   StageRange reduce_range(runner->nvtx && (stages & GEVVA_MOE_STAGE_REDUCE), "gevva_moe.reduce");
   if (stages & GEVVA_MOE_STAGE_REDUCE)
@@ -509,7 +514,9 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
     }
     gv::StreamOperands& st = m->stream_experts;
     ok = make_w13_unit_map(&st.map_w13, weights->w13, kExperts) &&
-         make_w2_down_map(&m->w2.map_b_down, weights->w2, kExperts);
+         make_w2_down_map(&m->w2.map_b_down, weights->w2, kExperts) && make_w2_down_map(&m->w2.map_down_pieces, weights->w2, kExperts, 0) &&
+         make_scale_map(&m->w2.map_down_a_sf, s->inter_sf, s->inter_sf_bytes, 4) &&
+         make_scale_map(&m->w2.map_down_b_sf, m->w2_sf_down, gv::retiled_w2_scale_bytes(kExperts), 8);
     for (int i = 0; i < gv::kStreamBoxes; ++i)
       ok = ok && make_operand_map(&st.map_up[i], s->input_codes, rows, kHidden / 2, 8 * (i + 1)) &&
            make_operand_map(&st.map_down[i], s->inter_codes, rows, kInter / 2, 8 * (i + 1));
@@ -533,10 +540,11 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
   m->w13_pair_form = (options && (options->flags & GEVVA_MOE_OPTION_W13_PAIRS)) || (w13_pairs_env && w13_pairs_env[0] == '1');
   m->w13_single = !m->w13_pair_form && w13_pairs_env && w13_pairs_env[0] == '0';
   {
-    const cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
+    cudaError_t e = static_cast<cudaError_t>(gv::prepare_w13_pairs());
+    if (e == cudaSuccess) e = static_cast<cudaError_t>(gv::prepare_grouped_down_pairs());
     if (e != cudaSuccess) {
       gevva_moe_destroy(m);
-      return cuda_failure(e, "w13 pair form");
+      return cuda_failure(e, "CTA-pair forms");
     }
     gv::W13PairOperands& wp = m->w13_pairs;
     ok = true;

@@ -550,6 +550,40 @@ def test_cta_pair_gemms_equal_the_single_cta_gemms(gm, weights, cuda_device, tok
     assert results[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens,edges", [(2559, [1, 127, 128, 129, 256]), (2560, [1, 127, 128, 129, 255, 256, 257, 383, 384, 385]),
+                                          (3001, [16, 17, 112, 113, 272, 273, 511, 512, 513, 640])])
+def test_w2_pairs_at_tile_edges(gm, weights, cuda_device, tokens, edges):
+    """From 2560 tokens on w2 runs by CTA pairs, a row tile of an expert each: experts whose last pair has one tile or
+    two, whole and ragged to the 16 rows that an epilogue step takes, against the pair kernels that share weight tiles in another
+    way; with every stage in one call and each in a call of its own."""
+    from gevva_b200 import runtime as rt
+    edges = [tokens] + edges
+    rng = np.random.default_rng(tokens)
+    mine = [[] for _ in range(tokens)]
+    for expert, count in enumerate(edges):
+        for t in rng.permutation(tokens)[:count]:
+            mine[t].append(expert)
+    ids = np.array([rng.permutation(m[:TOP_K] + list(rng.choice(np.arange(20, EXPERTS - 1), TOP_K - len(m[:TOP_K]), replace=False)))
+                    for m in mine], dtype=np.int32)
+    x = hashgen.activations(tokens, HIDDEN, 79, cuda_device)
+    dev_ids = torch.from_numpy(ids).to(cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    results = []
+    for pairs, split in ((True, False), (False, False), (False, True)):
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens, pairs=pairs)
+        out = torch.zeros_like(x)
+        if split:
+            for stage in (rt.STAGE_SORT, rt.STAGE_QUANTIZE, rt.STAGE_W13 | rt.STAGE_GEGLU, rt.STAGE_W2, rt.STAGE_REDUCE):
+                runner.launch_stages(stage, tokens, input=x, expert_ids=dev_ids, route_weights=rw, output=out)
+        else:
+            runner.launch_batch(x, dev_ids, rw, out, tokens)
+        runner.check()
+        results.append((out, runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].clone()))
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("tokens,edges", [(641, [1, 7, 8, 9, 127, 128, 129, 255, 256, 257]),
                                           (1000, [15, 16, 17, 33, 191, 192, 193, 208, 209, 385])])
 def test_large_batches_at_tile_and_chunk_edges(gm, weights, cuda_device, tokens, edges):
