@@ -51,7 +51,12 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
   gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, d->plan, stream);
   gv::GemmOperands gate_up = d->gate_up;
   gate_up.wide = wide_items(tokens, gate_up.n_out, sm_count);
-  gv::launch_grouped_gemm(gate_up, d->plan, sm_count, stream);
+  // By CTA pairs where the MLP has all SMs (figures in dense_gemm_pair.cu).  On the few that it gets beside the experts, whose weight
+  // stream bounds the layer, the one-CTA kernels are as fast or faster: whole layers in a graph 16 tokens 264.8 and 266.6 us by pairs, 40 tokens
+  // 337 and 343, 301 tokens 321 and 322, 640 tokens 363.5 and 366.
+  const bool pairs = sm_count >= 2 && sm_count == d->sm_count;
+  if (pairs) gv::launch_dense_pairs(gate_up, tokens, d->plan.status, sm_count, stream);
+  else gv::launch_grouped_gemm(gate_up, d->plan, sm_count, stream);
   // Beside the experts this kernel is launched the ordinary way: its CTAs, one a token, would otherwise wait out the first
   // projection on SMs that the streaming launch's last CTAs need (296 tokens with 16 dense SMs: 373 -> 2000 us for three layers,
   // because tokens of CTAs that are not running are then quantised by the others one by one).  Whole layers in a graph, us, chained and
@@ -62,7 +67,8 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
   gv::GemmOperands down = d->down;
   down.out = out_unscaled;
   down.wide = wide_items(tokens, down.n_out, sm_count);
-  gv::launch_grouped_gemm(down, d->plan, sm_count, stream);
+  if (pairs) gv::launch_dense_pairs(down, tokens, d->plan.status, sm_count, stream);
+  else gv::launch_grouped_gemm(down, d->plan, sm_count, stream);
   return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
 }
 
@@ -137,6 +143,9 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
   ok = ok && gv::make_operand_tensor_map(&d->gate_up.map_b, weights->gate_up, 2 * kDense, gv::kHidden, gv::kTileM);
   ok = ok && gv::make_operand_tensor_map(&d->down.map_a, d->prod_fp8, t, kDense, gv::kTileM);
   ok = ok && gv::make_operand_tensor_map(&d->down.map_b, weights->down, gv::kHidden, kDense, gv::kTileM);
+  ok = ok && gv::make_piece_tensor_map(&d->gate_up.map_down_pieces, weights->gate_up, 2 * kDense, gv::kHidden);
+  ok = ok && gv::make_piece_tensor_map(&d->down.map_down_pieces, weights->down, gv::kHidden, kDense);
+  ok = ok && gv::prepare_dense_pairs() == 0;
   if (!ok) {
     gevva_dense_destroy(d);
     return GEVVA_MOE_CUDA_ERROR;

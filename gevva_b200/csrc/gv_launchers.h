@@ -86,7 +86,8 @@ struct GemmOperands {
   CUtensorMap map_b64;      // CTA-pair fused w13 form: the same matrix through a 64-row box
   CUtensorMap map_b_units;  // fused w13 form: [experts * 2 halves, 704 rows, 1408 bytes], box 2 x 64 rows x 128 B
   CUtensorMap map_b_down;   // w2: the weights in the column order of grouped_gemm_down.cu
-  CUtensorMap map_down_pieces, map_down_a_sf, map_down_b_sf;  // grouped_gemm_down_pair.cu: 32 rows of it, and the scales
+  CUtensorMap map_down_pieces;  // grouped_gemm_down_pair.cu, dense_gemm_pair.cu: 32 weight rows in that order
+  CUtensorMap map_down_a_sf, map_down_b_sf;  // grouped_gemm_down_pair.cu: the scales
   CUtensorMap map_a_sf;     // CTA-pair form: a_scales as [atoms of 512 B][128 x u32], box of four atoms
   CUtensorMap map_b_sf;     // CTA-pair form: b_scales likewise; box of eight atoms (fused w13) or four (w2)
   const uint8_t* a_scales;  // activation scale regions
@@ -132,12 +133,16 @@ bool make_w13_unit_tensor_map(CUtensorMap* map, const void* base, uint64_t exper
 
 // w2 codes [experts * 2816 rows, 352 bytes] as [64-row groups][8][4][2] rows with strides of 64, 2, 16 and 1
 // rows, through a box of 192 rows x 128 bytes: the column order of grouped_gemm_down.cu.
+bool make_piece_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes);  // 32 rows in that order
 bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t experts);
 
 // The w2 GEMM of prefill-sized batches (grouped_gemm_down.cu): op.map_a, map_b_down, down_scales.
 size_t retiled_w2_scale_bytes(int experts);
 void launch_retile_w2_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, cudaStream_t stream);
-// The same by CTA pairs (grouped_gemm_down_pair.cu): op.map_a, map_down_pieces, map_down_a_sf, map_down_b_sf; all row tiles, no row_dest.
+// The dense projections by CTA pairs (dense_gemm_pair.cu): op.map_a, map_down_pieces, out, n_out, k_in.
+int prepare_dense_pairs();
+void launch_dense_pairs(const GemmOperands& op, int tokens, int* status, int sm_count, cudaStream_t stream);
+// w2 by CTA pairs (grouped_gemm_down_pair.cu): op.map_a, map_down_pieces, map_down_a_sf, map_down_b_sf; all row tiles, no row_dest.
 int prepare_grouped_down_pairs();
 void launch_grouped_down_pairs(const GemmOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);
 void launch_grouped_down(const GemmOperands& op, const RoutePlan& plan, int sm_count, cudaStream_t stream);

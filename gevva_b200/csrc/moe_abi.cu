@@ -136,10 +136,10 @@ bool make_w13_fragment_map(CUtensorMap* map, const void* base, uint64_t experts)
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// w2 codes in the row order of grouped_gemm_down.cu: a box of `groups` 64-row groups, or of half a one (0).
-bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts, int groups = 3) {
-  constexpr cuuint64_t row = kInter / 2;
-  const cuuint64_t dims[5] = {row, 2, 4, 8, experts * kHidden / 64};
+// Weight rows in the order of grouped_gemm_down.cu, row 8g + 2t + i of a 64-row group being row 16t + 2g + i: a box of `groups` groups,
+// or of half a one (0).
+bool make_column_order_map(CUtensorMap* map, const void* base, uint64_t rows, cuuint64_t row, int groups) {
+  const cuuint64_t dims[5] = {row, 2, 4, 8, rows / 64};
   const cuuint64_t strides[4] = {row, 16 * row, 2 * row, 64 * row};
   const cuuint32_t box[5] = {static_cast<cuuint32_t>(kTileKBytes), 2, 4, groups ? 8u : 4u, groups ? static_cast<cuuint32_t>(groups) : 1u};
   const cuuint32_t element_strides[5] = {1, 1, 1, 1, 1};
@@ -148,6 +148,10 @@ bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts, int 
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<void*>(base), dims, strides, box, element_strides,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts) {
+  return make_column_order_map(map, base, experts * kHidden, kInter / 2, 3);
 }
 
 // Scale bytes of an activation operand as [128-row blocks, atoms per block, 128 x u32] through a
@@ -238,6 +242,9 @@ bool make_w13_unit_tensor_map(CUtensorMap* map, const void* base, uint64_t exper
 }
 bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t experts) {
   return make_w2_down_map(map, base, experts);
+}
+bool make_piece_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes) {
+  return make_column_order_map(map, base, rows, row_bytes, 0);
 }
 bool make_operand_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
                              int box_rows) {
@@ -514,7 +521,7 @@ int gevva_moe_create(gevva_moe** out, const gevva_moe_weights* weights, int max_
     }
     gv::StreamOperands& st = m->stream_experts;
     ok = make_w13_unit_map(&st.map_w13, weights->w13, kExperts) &&
-         make_w2_down_map(&m->w2.map_b_down, weights->w2, kExperts) && make_w2_down_map(&m->w2.map_down_pieces, weights->w2, kExperts, 0) &&
+         make_w2_down_map(&m->w2.map_b_down, weights->w2, kExperts) && gv::make_piece_tensor_map(&m->w2.map_down_pieces, weights->w2, static_cast<uint64_t>(kExperts) * kHidden, kInter / 2) &&
          make_scale_map(&m->w2.map_down_a_sf, s->inter_sf, s->inter_sf_bytes, 4) &&
          make_scale_map(&m->w2.map_down_b_sf, m->w2_sf_down, gv::retiled_w2_scale_bytes(kExperts), 8);
     for (int i = 0; i < gv::kStreamBoxes; ++i)

@@ -262,3 +262,24 @@ def test_layers_beside_the_dense_mlp_in_a_graph(cuda_device, tokens):
     assert torch.equal(got, want)
     for layer in stack.layers:
         layer.experts.check()
+
+
+@pytest.mark.parametrize("tokens", [17, 127, 129, 255, 257, 1153, 2048])
+def test_dense_pairs_at_tile_edges(dense_weights, cuda_device, tokens):
+    """The dense GEMMs by CTA pairs take 256 tokens and 256 or 192 columns an item and store 16 rows a step: whole and ragged last
+    tiles, with either width, give every row the bits it has in a batch of 112 (one ragged tile), and store nothing past the end."""
+    from gevva_b200 import feedforward as ff
+    gate_up, down, gs, us, ds = dense_weights
+    mlp = ff.DenseMlp(gate_up, down, gs, us, ds, tokens + 300)
+    x = hashgen.activations(tokens, HIDDEN, 83, cuda_device)
+    guarded = torch.full((tokens + 256, HIDDEN), 7.0, device=cuda_device, dtype=torch.bfloat16)
+    mlp.buffer(2, torch.bfloat16).fill_(5.0)
+    mlp.launch(x, out=guarded[:tokens])
+    hidden = mlp.buffer(2, torch.bfloat16).view(-1, 2 * DENSE).clone()
+    assert (guarded[tokens:] == 7.0).all() and (hidden[tokens:] == 5.0).all()
+    for first in range(0, tokens, 112):
+        rows = min(112, tokens - first)
+        part, _ = mlp.launch(x[first : first + rows].contiguous())
+        assert torch.equal(mlp.buffer(2, torch.bfloat16)[: rows * 2 * DENSE].view(rows, -1), hidden[first : first + rows])
+        assert torch.equal(part[:rows], guarded[first : first + rows])
+    assert guarded[:tokens].float().abs().max() > 0
