@@ -10,6 +10,7 @@
 
 #include "../../include/gevva_moe.h"
 #include "gv_common.cuh"
+#include "gv_exact.h"
 #include "gv_launchers.h"
 
 namespace {
@@ -28,6 +29,7 @@ struct gevva_dense {
   uint8_t* prod_fp8 = nullptr;    // [T, 2112]
   float* prod_scales = nullptr;   // [T]
   float* ones = nullptr;          // [128]
+  float* gelu_table = nullptr;    // [GV_GELU_FLOATS]
   float* down_scale = nullptr;    // [1]: weights.down_scale on the device, for gevva_ff_finalize
   int* ints = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;  // gevva_ff_layer_launch: to the second stream and back
@@ -63,7 +65,7 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
   // ordinary: 16 tokens 271 and 268 (four layers), 100 tokens 371 and 368, 128 tokens 390 and 380.  A dozen CTAs fit anywhere.
   const bool beside = sm_count < d->sm_count;
   gv::launch_gelu_quantize_fp8(d->gate_up_out, d->act_scales, d->weights.gate_scale, d->weights.up_scale,
-                               d->prod_fp8, d->prod_scales, tokens, beside && tokens > 12, stream);
+                               d->gelu_table, d->prod_fp8, d->prod_scales, tokens, sm_count, beside && tokens > 12, stream);
   gv::GemmOperands down = d->down;
   down.out = out_unscaled;
   down.wide = wide_items(tokens, down.n_out, sm_count);
@@ -82,6 +84,7 @@ void gevva_dense_destroy(gevva_dense* d) {
   cudaFree(d->prod_fp8);
   cudaFree(d->prod_scales);
   cudaFree(d->ones);
+  cudaFree(d->gelu_table);
   cudaFree(d->down_scale);
   cudaFree(d->ints);
   if (d->fork) cudaEventDestroy(d->fork);
@@ -124,6 +127,12 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
     float host_ones[gv::kExperts];
     for (float& v : host_ones) v = 1.0f;
     e = cudaMemcpy(d->ones, host_ones, sizeof(host_ones), cudaMemcpyHostToDevice);
+  }
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->gelu_table), GV_GELU_FLOATS * sizeof(float));
+  if (e == cudaSuccess) {
+    float host_table[GV_GELU_FLOATS];
+    for (uint32_t i = 0; i < GV_GELU_FLOATS; ++i) host_table[i] = gv_gelu_entry(i);
+    e = cudaMemcpy(d->gelu_table, host_table, sizeof(host_table), cudaMemcpyHostToDevice);
   }
   if (e != cudaSuccess) {
     gevva_dense_destroy(d);

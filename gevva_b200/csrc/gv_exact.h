@@ -40,3 +40,36 @@ GV_HD float gv_scale_inverse(float multiplier, uint32_t code, const float* recip
   const float q = GV_FMA(GV_FMA(reciprocals[2 * k + 1], q0, multiplier), r, q0);
   return GV_MUL(q, gv_bits_to_float((137u - (exponent ? exponent : 1u)) << 23));
 }
+
+// gv_gelu_tanh(x) as x times a factor from a table, for an x that is a bf16 number of magnitude 2^-14 and up (or zero): one entry for each bf16
+// number of [2^-14, 2^3), for each sign; from 2^3 on the factor is the last entry's, 1 or 0 (tanh has long reached its limit).  The entries come
+// from the function itself, and its halving is exact wherever it stands in the product, so that both give the same bits
+// (tests/test_exact_divisions.py compares every argument).
+#define GV_GELU_FIRST (113u << 7)                  // 2^-14 as bf16
+#define GV_GELU_LAST ((130u << 7) - 1u)            // the last bf16 number below 2^3
+#define GV_GELU_SIGN 4096u                         // where the entries of the negative numbers start
+#define GV_GELU_FLOATS (GV_GELU_SIGN + GV_GELU_LAST - GV_GELU_FIRST + 1u)
+
+GV_HD float gv_gelu_entry(uint32_t index) {
+  const uint32_t sign = index >= GV_GELU_SIGN ? 1u : 0u;
+  uint32_t magnitude = GV_GELU_FIRST + index - sign * GV_GELU_SIGN;
+  if (magnitude > GV_GELU_LAST) magnitude = GV_GELU_LAST;  // the gap before the negative numbers
+  return GV_MUL(0.5f, gv_gelu_factor(gv_bits_to_float((sign << 31) | (magnitude << 16))));
+}
+
+// Two bf16 numbers in a word -> the byte offsets of their factors, in a word.  Magnitudes below the table's get the
+// first entry, which is right for zero only.
+GV_HD uint32_t gv_gelu_offsets(uint32_t pair) {
+  const uint32_t magnitude = pair & 0x7fff7fffu;
+#if defined(__CUDA_ARCH__)
+  const uint32_t clamped = __vmaxu2(__vminu2(magnitude, GV_GELU_LAST * 0x10001u), GV_GELU_FIRST * 0x10001u);
+#else
+  uint32_t clamped = 0;
+  for (int half = 0; half < 32; half += 16) {
+    uint32_t m = (magnitude >> half) & 0xffffu;
+    m = m > GV_GELU_LAST ? GV_GELU_LAST : m < GV_GELU_FIRST ? GV_GELU_FIRST : m;
+    clamped |= m << half;
+  }
+#endif
+  return ((clamped - GV_GELU_FIRST * 0x10001u) << 2) | ((pair >> 1) & 0x40004000u);
+}

@@ -221,8 +221,8 @@ void launch_ff_prepare(const void* input, const void* dense_weight, const void* 
 void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows, const RoutePlan& plan,
                               cudaStream_t stream);
 void launch_gelu_quantize_fp8(const void* gate_up, const float* activation_scales, float gate_w_scale,
-                              float up_w_scale, uint8_t* out, float* scales, int rows,
-                              bool serial_launch, cudaStream_t stream);
+                              float up_w_scale, const float* gelu_table, uint8_t* out, float* scales, int rows,
+                              int sm_count, bool serial_launch, cudaStream_t stream);
 void launch_ff_finalize(const void* dense, const void* dense_weight, const void* expert_routes,
                         const float* route_weights, const int* inverse_routes, const void* expert_weight,
                         const void* combined_weight, const void* residual, const void* layer_scalar,

@@ -149,11 +149,13 @@ GV_HD float gv_tanhf(float y) {
 
 // tanh-GELU times up, rounded to bf16 by the caller: 0.5*x*(1+tanh(k*(x+0.044715*x^3))),
 // operations in the order the reference writes them.
-GV_HD float gv_gelu_tanh(float x) {
+GV_HD float gv_gelu_factor(float x) {
   const float cube = GV_MUL(GV_MUL(GV_MUL(0.044715f, x), x), x);
   const float inner = GV_MUL(0.7978845608028654f, GV_ADD(x, cube));
-  return GV_MUL(GV_MUL(0.5f, x), GV_ADD(1.0f, gv_tanhf(inner)));
+  return GV_ADD(1.0f, gv_tanhf(inner));
 }
+
+GV_HD float gv_gelu_tanh(float x) { return GV_MUL(GV_MUL(0.5f, x), gv_gelu_factor(x)); }
 
 // 1/sqrt(x) with IEEE square root and division (the reference calls the approximate rsqrtf).
 GV_HD float gv_rsqrtf(float x) {

@@ -1,6 +1,6 @@
 // Compares the two divisions of gv_exact.h with IEEE division: every significand for the constant
-// divisor and for every integer divisor 1..15, a spread of exponents, and every E4M3 scale code.
-// Prints the number of differences.
+// divisor and for every integer divisor 1..15, a spread of exponents, and every E4M3 scale code; and the
+// table form of the tanh GELU with the function itself for every bf16 argument.  Prints the number of differences.
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -42,6 +42,17 @@ int main() {
         differences += gv_scale_inverse_exact(m) && gv_scale_inverse(m, code, reciprocals) != quotient(m, code);
       }
   differences += gv_sixth(0.0f) != 0.0f || !std::isinf(gv_sixth(INFINITY));
+  static float table[GV_GELU_FLOATS];
+  for (uint32_t i = 0; i < GV_GELU_FLOATS; ++i) table[i] = gv_gelu_entry(i);
+  for (uint32_t magnitude = 0; magnitude < 32768; ++magnitude) {
+    if (magnitude && magnitude < GV_GELU_FIRST) continue;
+    const uint32_t offsets = gv_gelu_offsets(magnitude | (magnitude | 0x8000u) << 16);  // the number and its negative
+    for (uint32_t sign = 0; sign < 2; ++sign) {
+      const float x = gv_bits_to_float(sign << 31 | magnitude << 16);
+      const float direct = gv_gelu_tanh(x), looked_up = x * table[(sign ? offsets >> 16 : offsets & 0xffffu) / 4];
+      differences += gv_float_to_bits(direct) != gv_float_to_bits(looked_up) && !(direct != direct && looked_up != looked_up);
+    }
+  }
   std::printf("%ld\n", differences);
   return 0;
 }

@@ -1,4 +1,4 @@
-"""The division-free quotients of the block quantiser (csrc/gv_exact.h) equal IEEE division."""
+"""The division-free quotients of the block quantiser (csrc/gv_exact.h) equal IEEE division, the tanh GELU by table the function."""
 import os
 import subprocess
 

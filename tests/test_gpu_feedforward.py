@@ -283,3 +283,24 @@ def test_dense_pairs_at_tile_edges(dense_weights, cuda_device, tokens):
         assert torch.equal(mlp.buffer(2, torch.bfloat16)[: rows * 2 * DENSE].view(rows, -1), hidden[first : first + rows])
         assert torch.equal(part[:rows], guarded[first : first + rows])
     assert guarded[:tokens].float().abs().max() > 0
+
+
+@pytest.mark.parametrize("tokens,gate_scale", [(593, 1.0), (600, 1e-6), (1023, 1e6), (1024, 1e-5), (2369, 3e-6)])
+def test_activation_of_large_batches_equals_the_small_ones(dense_weights, cuda_device, tokens, gate_scale):
+    """From five tokens an SM the GELU step takes a warp a row and looks its tanh factor up, from 1024 tokens the first quantiser takes a
+    warp a row: all bytes and scales as in batches of 64, for gates inside the table, past both of its ends, and zero."""
+    from gevva_b200 import feedforward as ff
+    gate_up, down, gs, us, ds = dense_weights
+    mlp = ff.DenseMlp(gate_up, down, gs * gate_scale, us, ds, tokens)
+    x = hashgen.activations(tokens, HIDDEN, 89, cuda_device)
+    x[tokens // 2].zero_()
+    views = lambda rows: (mlp.buffer(0, torch.uint8)[: rows * HIDDEN].view(rows, -1), mlp.buffer(1, torch.float32)[:rows],
+                          mlp.buffer(3, torch.uint8)[: rows * DENSE].view(rows, -1), mlp.buffer(4, torch.float32)[:rows])
+    mlp.launch(x)
+    whole = [v.clone() for v in views(tokens)]
+    for first in range(0, tokens, 64):
+        rows = min(64, tokens - first)
+        mlp.launch(x[first : first + rows].contiguous())
+        for part, all_rows in zip(views(rows), whole):
+            assert torch.equal(part, all_rows[first : first + rows])
+    assert whole[2].count_nonzero() > 0
