@@ -2,7 +2,7 @@
 // expert path (declared in include/gevva_moe.h).  The reference runs the three dense
 // projections through cuBLASLt (Fp8LinearRunner::launch_unscaled,
 // src/cuda/runtime/fp8_linear.cuh:215-473, called at src/cuda/runtime/prefill.cuh:1211-1230);
-// here they are the tcgen05 kernel of grouped_gemm.cu in its FP8 form.
+// here they are the tcgen05 kernels of dense_gemm_pair.cu or, beside the experts, of grouped_gemm.cu in its FP8 form.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -37,7 +37,7 @@ struct gevva_dense {
 
 // Whether a GEMM of the dense MLP takes 256 weight rows an item instead of 128.  The launch lasts as many items
 // as its busiest CTA has, and a wide item takes about one and a half times a narrow one (48 KB of operands a K
-// block against 32 KB): wide where that is no longer.  Alone on 148 SMs the MLP takes (us, narrow -> wide)
+// block against 32 KB): wide where that is no longer.  Alone on 148 SMs (where pairs of CTAs run now) the MLP took (us, narrow -> wide)
 // 31.9 -> 35.4 at 301 tokens, where one wave of narrow items is enough, 39.0 -> 35.5 at 600, 74.8 -> 62.6 at 2048
 // and 131.9 -> 108.4 at 4096.  On the few SMs that it gets beside the experts of a decode batch (whole layers in a graph):
 // 57.5 -> 53.7 at 8 tokens, 71.6 -> 71.8 at 16, 91.4 -> 91.9 at 40, 95.9 -> 95.7 at 64, 104.1 -> 103.2 at 128.

@@ -4,7 +4,7 @@
 // takes in 73 bytes a cycle: 660 cycles.  A pair (tcgen05 cta_group::2, M = 256) computes 256 tokens x 256 columns with half of either
 // operand in each CTA, 32 KB: 450 cycles, under the MMAs' 512.  The whole MLP, one CTA a tile -> pairs
 // (us): 1 token 25.5 -> 22.8, 128 tokens 29.0 -> 24.8, 301 tokens 31.3 -> 25.1, 640 tokens 34.9 -> 30.1, 1024 tokens 38.0 -> 33.6, 2048 tokens 62.8 ->
-// 54.2, 4096 tokens 106 -> 94 (of the last two 23 and 38 are its quantisers).
+// 54.2, 4096 tokens 106 -> 94 (of the last two 23 and 38 were its quantisers; 48 and 81 with those of today).
 // 192 columns an item where that leaves the clusters less to do (the second projection at 2048 tokens: 88 items of 256 are two
 // rounds of 74 clusters as 120 items of 192 are).  The weight rows are taken in the column order of grouped_gemm_down.cu, in copies of 32
 // rows, so that a quad of lanes stores whole 128-byte lines of a row from registers.  Two accumulators of up to 256 columns fill

@@ -11,8 +11,8 @@
 //
 // Mapping.  Tokens (sorted routes) sit on MMA-M, weight rows on MMA-N.  A work
 // item is (128-row tile of one expert) x (kN weight rows), kN = 256 for the fused w13 form and
-// for dense FP8 batches, 128 elsewhere.  An MMA of M = 128 takes at least about 105 cycles whatever its
-// N (measured; 128 at N = 256), so the wide tile, which does twice the work per
+// for dense FP8 batches, 128 elsewhere.  An MMA of M = 128 keeps the pipe busy for N / 2 cycles from N = 128 on, but with its
+// scale copies it takes about 105 to issue, so the wide tile, which does twice the work per
 // instruction, is what keeps the tensor pipe fed.  Row tiles are listed
 // in device memory by the route sort; CTAs are persistent and take items
 // round-robin.  Warps 0 and 18 are the TMA producers (activation side, weight side),

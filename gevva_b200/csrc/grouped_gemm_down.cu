@@ -9,8 +9,8 @@
 // reads, the arriving operands and the staged results, had no bandwidth left.  Here 35.7, 46, 70 and 227:
 //   * an item is 192 output columns (15 to a row tile, the last of 128): two accumulators fit beside the
 //     scales in tensor memory, so that draining one overlaps the next item's MMAs.  128-column items with
-//     three accumulators took 76 us at 4096 tokens (an MMA takes 105 cycles at any N up to 128 and 111 at
-//     192), 256-column items with one 80;
+//     three accumulators took 76 us at 4096 tokens (an MMA and its share of the scale copies take 105 cycles to issue at
+//     any N up to 128 and 111 at 192), 256-column items with one 80;
 //   * a unit of work is a row tile against three of its items, and the tile's activations and their scales are
 //     fetched and copied once a unit;
 //   * scale copies and MMAs are issued by one thread (see there);
@@ -21,7 +21,7 @@
 //     128-byte line of a row.  The order costs nothing: it is a five-dimensional view of the same weights
 //     ([64-column group][g][t][pair] with strides of 64, 2, 16 and 1 rows), and the scales have a
 //     re-tiled copy made at runner creation.
-// What is left at 4096 tokens is the way between an SM and L2, which stores and TMA loads share: the stores of
+// From 2560 tokens on grouped_gemm_down_pair.cu takes its place. What is left is the way between an SM and L2, which stores and TMA loads share: the stores of
 // an item (48 KB) raise the wait for its operands from 500 to 1700 cycles.
 //
 // Roles (8 warps): 0 fetches weights, 1 copies scale factors and issues MMAs, 2 fetches activations, 4..7 the

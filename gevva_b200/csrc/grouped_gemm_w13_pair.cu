@@ -5,8 +5,8 @@
 // cycles.  Here a CTA pair (tcgen05 cta_group::2, M = 256) holds 256 weight rows, 128 per CTA, against up to 208
 // token rows of one expert on the N side, half of them loaded by each CTA: at most 35 KiB in and 29 out.  And because
 // the tokens sit on N, which may be any multiple of 16, a group of 200 rows is one item and not two 128-row tiles.
-// An item is 44 MMAs of about 105 cycles and their scale copies, 5345 cycles with neither loads nor epilogue and
-// 6600 in all (4096 tokens).  Beside large batches the clock drops to 1.5 GHz under the power limit.
+// An item is 44 MMAs and their scale copies. The tensor pipe takes N / 2 cycles an MMA from 128 rows on (39 to 64 below), issuing it
+// and its share of the copies about 105: 5345 cycles with neither loads nor epilogue and 6600 in all (4096 tokens).  Beside large batches the clock drops to 1.5 GHz under the power limit.
 // Alone (us, one-CTA kernel -> this one; uniform routing): 53.1 -> 53.2 at 1024 tokens, 63.9 -> 58.9 at 2048,
 // 83.5 -> 70 at 3000, 97 -> 95 at 4096, 172 -> 151 at 8192, 330 -> 293 at 16384.
 //
