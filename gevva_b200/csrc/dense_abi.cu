@@ -51,14 +51,21 @@ static bool wide_items(int tokens, int n_out, int sms) {
 int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
                         int sm_count) {
   gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, d->plan, stream);
-  gv::GemmOperands gate_up = d->gate_up;
-  gate_up.wide = wide_items(tokens, gate_up.n_out, sm_count);
   // By CTA pairs where the MLP has all SMs (figures in dense_gemm_pair.cu).  On the few that it gets beside the experts, whose weight
   // stream bounds the layer, the one-CTA kernels are as fast or faster: whole layers in a graph 16 tokens 264.8 and 266.6 us by pairs, 40 tokens
   // 337 and 343, 301 tokens 321 and 322, 640 tokens 363.5 and 366.
+  // The pair kernel stores 32 bytes at a time; rows are whole multiples of that, so an output that is aligned to 16 only, as the
+  // one-CTA kernel takes it, goes there (same bits; the MLP takes 54.4 us instead of 46.5 then at 2048 tokens, 27.4 instead of 24.6 at 301).
   const bool pairs = sm_count >= 2 && sm_count == d->sm_count;
-  if (pairs) gv::launch_dense_pairs(gate_up, tokens, d->plan.status, sm_count, stream);
-  else gv::launch_grouped_gemm(gate_up, d->plan, sm_count, stream);
+  const auto project = [&](gv::GemmOperands op) {
+    if (pairs && (reinterpret_cast<uintptr_t>(op.out) & 31) == 0) {
+      gv::launch_dense_pairs(op, tokens, d->plan.status, sm_count, stream);
+    } else {
+      op.wide = wide_items(tokens, op.n_out, sm_count);
+      gv::launch_grouped_gemm(op, d->plan, sm_count, stream);
+    }
+  };
+  project(d->gate_up);
   // Beside the experts this kernel is launched the ordinary way: its CTAs, one a token, would otherwise wait out the first
   // projection on SMs that the streaming launch's last CTAs need (296 tokens with 16 dense SMs: 373 -> 2000 us for three layers,
   // because tokens of CTAs that are not running are then quantised by the others one by one).  Whole layers in a graph, us, chained and
@@ -68,9 +75,7 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
                                d->gelu_table, d->prod_fp8, d->prod_scales, tokens, sm_count, beside && tokens > 12, stream);
   gv::GemmOperands down = d->down;
   down.out = out_unscaled;
-  down.wide = wide_items(tokens, down.n_out, sm_count);
-  if (pairs) gv::launch_dense_pairs(down, tokens, d->plan.status, sm_count, stream);
-  else gv::launch_grouped_gemm(down, d->plan, sm_count, stream);
+  project(down);
   return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
 }
 
@@ -174,7 +179,9 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
 
 int gevva_dense_launch(gevva_dense* d, const void* in, void* out_unscaled, int tokens,
                        gevva_stream_t stream) {
-  if (!d || !in || !out_unscaled || tokens < 1 || tokens > d->max_tokens) return GEVVA_MOE_BAD_ARGUMENT;
+  if (!d || !in || !out_unscaled || tokens < 1 || tokens > d->max_tokens ||
+      ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out_unscaled)) & 15))
+    return GEVVA_MOE_BAD_ARGUMENT;  // (rows are read and written 16 bytes at a time at least)
   return gv::dense_launch_on(d, in, out_unscaled, tokens, stream, d->sm_count);
 }
 

@@ -310,7 +310,8 @@ int gevva_ff_finalize(const void* dense, const void* dense_weight, const void* e
  * src/cuda/kernels/fp8.cuh:2-26, :299-364).  gate_up is the gate matrix [2112,2816] followed by
  * the up matrix [2112,2816]; down is [2816,2112].  The output is the UNSCALED bf16 down
  * projection; gevva_dense_output_scales gives the per-row activation scale that, times
- * down_scale, gevva_ff_finalize applies. */
+ * down_scale, gevva_ff_finalize applies.  Input and output are 16-byte aligned (others are refused); an
+ * output that is 32-byte aligned, as every allocation is, takes the faster down projection. */
 typedef struct gevva_dense gevva_dense;
 typedef struct {
   const void* gate_up; /* e4m3 [4224,2816] */

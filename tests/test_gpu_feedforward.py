@@ -285,6 +285,21 @@ def test_dense_pairs_at_tile_edges(dense_weights, cuda_device, tokens):
     assert guarded[:tokens].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens", [1, 129, 600])
+def test_dense_output_aligned_to_16_bytes(dense_weights, cuda_device, tokens):
+    """An output that starts between two 32-byte lines gets the bits of one that does not, and nothing around it."""
+    from gevva_b200 import feedforward as ff
+    gate_up, down, gs, us, ds = dense_weights
+    mlp = ff.DenseMlp(gate_up, down, gs, us, ds, tokens)
+    x = hashgen.activations(tokens, HIDDEN, 84, cuda_device)
+    want = mlp.launch(x)[0].clone()
+    flat = torch.full((tokens * HIDDEN + 16,), 7.0, device=cuda_device, dtype=torch.bfloat16)
+    assert flat.data_ptr() % 32 == 0
+    mlp.launch(x, out=flat[8:-8].view(tokens, HIDDEN))
+    assert torch.equal(flat[8:-8].view(tokens, HIDDEN), want)
+    assert (flat[:8] == 7.0).all() and (flat[-8:] == 7.0).all()
+
+
 @pytest.mark.parametrize("tokens,gate_scale", [(593, 1.0), (600, 1e-6), (1023, 1e6), (1024, 1e-5), (2369, 3e-6)])
 def test_activation_of_large_batches_equals_the_small_ones(dense_weights, cuda_device, tokens, gate_scale):
     """From five tokens an SM the GELU step takes a warp a row and looks its tanh factor up, from 1024 tokens the first quantiser takes a

@@ -42,6 +42,7 @@ class Recorder:
         lib.gevva_moe_launch_stages.argtypes = [vp, vp, vp, vp, vp, i32, ctypes.c_uint, vp]
         lib.gevva_dense_create.argtypes = [ctypes.POINTER(vp), ctypes.POINTER(ff._DenseWeights), i32]
         lib.gevva_dense_destroy.argtypes = [vp]
+        lib.gevva_dense_launch.argtypes = [vp, vp, vp, i32, vp]
         lib.gevva_ff_layer_launch.argtypes = [ctypes.POINTER(ff._Layer), vp, vp, vp, i32, vp, vp]
 
     def runner(self, max_tokens, flags=0):
@@ -139,6 +140,22 @@ def test_feed_forward_layer_launches(recorder):
         "fp8_quantize_rows_kernel", "grouped_nvfp4_gemm_kernel", "gelu_quantize_fp8_kernel", "grouped_nvfp4_gemm_kernel"]
     assert kernels([l for l in launches if l["stream"] == STREAM]) == [
         "ff_prepare_kernel", "route_project_kernel<0>", "stream_experts_kernel<1>", "ff_finalize_kernel"]
+
+
+@pytest.mark.parametrize("offset,last", [(0, "dense_fp8_pair_kernel"), (16, "grouped_nvfp4_gemm_kernel"),
+                                         (32, "dense_fp8_pair_kernel"), (48, "grouped_nvfp4_gemm_kernel")])
+def test_dense_outputs_between_32_byte_lines(recorder, offset, last):
+    """The pair kernel stores 32 bytes at a time: into an output that is aligned to 16 only, the one-CTA kernel stores."""
+    dense = recorder.dense(64)
+    assert recorder.lib.gevva_dense_launch(dense, ADDRESS, ADDRESS + offset, 64, STREAM) == 0
+    assert kernels(recorder.launches()) == ["fp8_quantize_rows_kernel", "dense_fp8_pair_kernel", "gelu_quantize_fp8_kernel", last]
+
+
+@pytest.mark.parametrize("in_offset,out_offset", [(8, 0), (2, 0), (0, 8), (0, 2)])
+def test_dense_refuses_unaligned_rows(recorder, in_offset, out_offset):
+    dense = recorder.dense(64)
+    assert recorder.lib.gevva_dense_launch(dense, ADDRESS + in_offset, ADDRESS + out_offset, 64, STREAM) == -3
+    assert recorder.launches() == []
 
 
 @pytest.mark.parametrize("capacity,dense_capacity,tokens,router_weight", [(4, 64, 5, ADDRESS), (64, 4, 5, ADDRESS),
