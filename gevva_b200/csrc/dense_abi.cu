@@ -49,8 +49,10 @@ static bool wide_items(int tokens, int n_out, int sms) {
 }
 
 int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
-                        int sm_count) {
-  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, d->plan, stream);
+                        int sm_count, int* status) {
+  gv::RoutePlan plan = d->plan;
+  plan.status = status;
+  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, plan, stream);
   // By CTA pairs where the MLP has all SMs (figures in dense_gemm_pair.cu).  On the few that it gets beside the experts, whose weight
   // stream bounds the layer, the one-CTA kernels are as fast or faster: whole layers in a graph 16 tokens 264.8 and 266.6 us by pairs, 40 tokens
   // 337 and 343, 301 tokens 321 and 322, 640 tokens 363.5 and 366.
@@ -59,10 +61,10 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
   const bool pairs = sm_count >= 2 && sm_count == d->sm_count;
   const auto project = [&](gv::GemmOperands op) {
     if (pairs && (reinterpret_cast<uintptr_t>(op.out) & 31) == 0) {
-      gv::launch_dense_pairs(op, tokens, d->plan.status, sm_count, stream);
+      gv::launch_dense_pairs(op, tokens, status, sm_count, stream);
     } else {
       op.wide = wide_items(tokens, op.n_out, sm_count);
-      gv::launch_grouped_gemm(op, d->plan, sm_count, stream);
+      gv::launch_grouped_gemm(op, plan, sm_count, stream);
     }
   };
   project(d->gate_up);
@@ -182,7 +184,19 @@ int gevva_dense_launch(gevva_dense* d, const void* in, void* out_unscaled, int t
   if (!d || !in || !out_unscaled || tokens < 1 || tokens > d->max_tokens ||
       ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out_unscaled)) & 15))
     return GEVVA_MOE_BAD_ARGUMENT;  // (rows are read and written 16 bytes at a time at least)
-  return gv::dense_launch_on(d, in, out_unscaled, tokens, stream, d->sm_count);
+  return gv::dense_launch_on(d, in, out_unscaled, tokens, stream, d->sm_count, d->plan.status);
+}
+
+int* gevva_dense_status_word(gevva_dense* d) { return d ? d->plan.status : nullptr; }
+
+int gevva_dense_last_status(gevva_dense* d) {
+  if (!d) return GEVVA_MOE_BAD_ARGUMENT;
+  int status = 0;
+  if (cudaDeviceSynchronize() != cudaSuccess ||
+      cudaMemcpy(&status, d->plan.status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+      (status != 0 && cudaMemset(d->plan.status, 0, sizeof(int)) != cudaSuccess))
+    return GEVVA_MOE_CUDA_ERROR;
+  return -status;
 }
 
 const float* gevva_dense_output_scales(const gevva_dense* d) { return d ? d->prod_scales : nullptr; }
@@ -306,11 +320,13 @@ int gevva_ff_layer_launch(const gevva_ff_layer* layer, const void* hidden, void*
         cudaStreamWaitEvent(aux_stream, dense->fork, 0) != cudaSuccess)
       return GEVVA_MOE_CUDA_ERROR;
   }
-  int status = gv::dense_launch_on(dense, w.dense_in, w.dense_out, tokens, beside ? aux_stream : stream, dense_sms);
+  // One word for the whole layer: what gevva_moe_last_status of its experts reads.
+  int* const status_word = gevva_moe_status_word(layer->experts);
+  int status = gv::dense_launch_on(dense, w.dense_in, w.dense_out, tokens, beside ? aux_stream : stream, dense_sms, status_word);
   if (beside && cudaEventRecord(dense->join, aux_stream) != cudaSuccess) return GEVVA_MOE_CUDA_ERROR;
   if (status == GEVVA_MOE_OK)
     status = gevva_moe_route_project(w.router_in, layer->router_weight, nullptr, layer->expert_scale, w.route_weights,
-                                     w.ids, nullptr, tokens, gevva_moe_status_word(layer->experts), stream);
+                                     w.ids, nullptr, tokens, status_word, stream);
   if (status == GEVVA_MOE_OK)
     status = gv::moe_launch_stages_on(layer->experts, w.expert_in, w.ids, nullptr, nullptr, tokens,
                                       GEVVA_MOE_STAGE_ALL & ~static_cast<unsigned>(GEVVA_MOE_STAGE_REDUCE), stream,

@@ -15,8 +15,9 @@ namespace gv {
 // take one CTA per SM): what lets the two sides of a feed-forward layer run beside each other.
 int moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, const float* route_weights, void* out,
                          int tokens, unsigned stages, cudaStream_t stream, int sm_count);
+// (`status`: the word into which the dense kernels report a wait that ran out.)
 int dense_launch_on(gevva_dense* dense, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
-                    int sm_count);
+                    int sm_count, int* status);
 int moe_sm_count(const gevva_moe* runner);
 int moe_max_tokens(const gevva_moe* runner);
 

@@ -34,6 +34,9 @@ def _lib():
     lib.gevva_dense_destroy.argtypes = [vp]
     lib.gevva_dense_destroy.restype = None
     lib.gevva_dense_launch.argtypes = [vp, vp, vp, i32, vp]
+    lib.gevva_dense_last_status.argtypes = [vp]
+    lib.gevva_dense_status_word.argtypes = [vp]
+    lib.gevva_dense_status_word.restype = vp
     lib.gevva_dense_output_scales.argtypes = [vp]
     lib.gevva_dense_output_scales.restype = vp
     lib.gevva_dense_projection_scale.argtypes = [vp]
@@ -122,6 +125,14 @@ class DenseMlp:
         scales = _view(_lib().gevva_dense_output_scales(self._handle), (tokens,), torch.int32,
                        self.device).view(torch.float32)
         return out, scales
+
+    def last_status(self):
+        """Synchronises, then returns and clears the status of launch() (0 = ok); a layer's is its experts'."""
+        with torch.cuda.device(self.device):
+            return _lib().gevva_dense_last_status(self._handle)
+
+    def check(self):
+        _status(self.last_status(), "device status")
 
     def buffer(self, which, dtype):
         ptr, size = ctypes.c_void_p(), ctypes.c_size_t()

@@ -322,6 +322,12 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
 void gevva_dense_destroy(gevva_dense* dense);
 int gevva_dense_launch(gevva_dense* dense, const void* in, void* out_unscaled, int tokens,
                        gevva_stream_t stream);
+/* Reads and clears the device status word of gevva_dense_launch (synchronises the device): GEVVA_MOE_WAIT_TIMEOUT
+ * after a bounded wait that expired, whose output rows are not to be used.  A layer (gevva_ff_layer_launch) reports
+ * into its experts' word instead: gevva_moe_last_status. */
+int gevva_dense_last_status(gevva_dense* dense);
+/* The word itself, on the device. */
+int* gevva_dense_status_word(gevva_dense* dense);
 const float* gevva_dense_output_scales(const gevva_dense* dense);
 /* f32 [1] on the device: weights->down_scale, in the form gevva_ff_finalize takes it */
 const float* gevva_dense_projection_scale(const gevva_dense* dense);
@@ -332,7 +338,8 @@ int gevva_dense_buffer(const gevva_dense* dense, int which, void** device_ptr, s
  * gevva_ff_prepare, gevva_moe_route_project, the experts unreduced, the dense MLP and
  * gevva_ff_finalize.  The dense MLP runs on `aux_stream`, forked from and joined to `stream` by
  * events, and shares the SMs with the expert kernels; aux_stream == stream runs everything in
- * order on one stream.  Same bits as the five calls.  `workspace` is device memory of at least
+ * order on one stream.  Same bits as the five calls; waits that expire, the dense MLP's too, are reported
+ * by gevva_moe_last_status(experts).  `workspace` is device memory of at least
  * gevva_ff_layer_workspace_bytes(tokens) bytes, 256-byte aligned, used until `stream` has passed the
  * call; every weight pointer is bf16 as in the calls above. */
 typedef struct {

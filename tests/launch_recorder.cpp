@@ -1,6 +1,7 @@
 // A CUDA runtime that launches nothing: it stands in for libcudart under the library's own host code (see
 // test_launch_sequence.py) and writes down every kernel launch, one line each:
-//   <mangled kernel name> grid=<x> cluster=<x> cooperative=<0|1> programmatic=<0|1> stream=<handle>
+//   <mangled kernel name> grid=<x> cluster=<x> cooperative=<0|1> programmatic=<0|1> stream=<handle> status=<address>
+// (status: the word into which the kernels of the dense MLP report a wait that ran out; 0 for others).
 // "Device" memory is host memory that nothing reads; events, copies and attributes succeed.
 #include <cuda.h>
 #include <cuda_runtime_api.h>
@@ -22,10 +23,19 @@ struct Pending {
   cudaStream_t stream;
 } pending;
 
-void record(const void* function, unsigned grid, unsigned cluster, bool cooperative, bool programmatic, cudaStream_t stream) {
+// DensePairParams::status of dense_gemm_pair.cu and GemmParams::status of gv_gemm_parts.cuh, by their places.
+size_t status_of(const std::string& name, void** arguments) {
+  if (name.find("dense_fp8_pair_kernel") != std::string::npos) return static_cast<size_t*>(arguments[2])[1];
+  if (name.find("grouped_nvfp4_gemm_kernel") != std::string::npos) return static_cast<size_t*>(arguments[3])[13];
+  return 0;
+}
+
+void record(const void* function, unsigned grid, unsigned cluster, bool cooperative, bool programmatic, cudaStream_t stream,
+            void** arguments) {
   char line[512];
-  std::snprintf(line, sizeof(line), "%s grid=%u cluster=%u cooperative=%d programmatic=%d stream=%zu\n",
-                names()[function].c_str(), grid, cluster, cooperative, programmatic, reinterpret_cast<size_t>(stream));
+  std::snprintf(line, sizeof(line), "%s grid=%u cluster=%u cooperative=%d programmatic=%d stream=%zu status=%zu\n",
+                names()[function].c_str(), grid, cluster, cooperative, programmatic, reinterpret_cast<size_t>(stream),
+                status_of(names()[function], arguments));
   log_text += line;
 }
 
@@ -66,11 +76,11 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* shared, 
   *static_cast<cudaStream_t*>(stream) = pending.stream;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* function, dim3 grid, dim3, void**, size_t, cudaStream_t stream) {
-  record(function, grid.x, 1, false, false, stream);
+cudaError_t cudaLaunchKernel(const void* function, dim3 grid, dim3, void** arguments, size_t, cudaStream_t stream) {
+  record(function, grid.x, 1, false, false, stream, arguments);
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* function, void**) {
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* function, void** arguments) {
   unsigned cluster = 1;
   bool cooperative = false, programmatic = false;
   for (unsigned i = 0; i < config->numAttrs; ++i) {
@@ -80,7 +90,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* fu
     if (a.id == cudaLaunchAttributeProgrammaticStreamSerialization)
       programmatic = a.val.programmaticStreamSerializationAllowed != 0;
   }
-  record(function, config->gridDim.x, cluster, cooperative, programmatic, config->stream);
+  record(function, config->gridDim.x, cluster, cooperative, programmatic, config->stream, arguments);
   return cudaSuccess;
 }
 cudaError_t cudaGetLastError() { return cudaSuccess; }

@@ -300,6 +300,20 @@ def test_dense_output_aligned_to_16_bytes(dense_weights, cuda_device, tokens):
     assert (flat[:8] == 7.0).all() and (flat[-8:] == 7.0).all()
 
 
+def test_dense_status_is_read_and_cleared(dense_weights, cuda_device):
+    """The word that an expired wait of the dense kernels sets (here a store stands in for it) is what last_status() returns, once."""
+    import gevva_b200 as gm
+    from gevva_b200 import feedforward as ff
+    from gevva_b200.runtime import _view
+    mlp = ff.DenseMlp(*dense_weights, 300)
+    mlp.launch(hashgen.activations(300, HIDDEN, 85, cuda_device))
+    mlp.check()
+    _view(ff._lib().gevva_dense_status_word(mlp._handle), (1,), torch.int32, cuda_device).fill_(2)
+    with pytest.raises(gm.GevvaMoeError, match="wait expired"):
+        mlp.check()
+    assert mlp.last_status() == 0
+
+
 @pytest.mark.parametrize("tokens,gate_scale", [(593, 1.0), (600, 1e-6), (1023, 1e6), (1024, 1e-5), (2369, 3e-6)])
 def test_activation_of_large_batches_equals_the_small_ones(dense_weights, cuda_device, tokens, gate_scale):
     """From five tokens an SM the GELU step takes a warp a row and looks its tanh factor up, from 1024 tokens the first quantiser takes a

@@ -43,6 +43,8 @@ class Recorder:
         lib.gevva_dense_create.argtypes = [ctypes.POINTER(vp), ctypes.POINTER(ff._DenseWeights), i32]
         lib.gevva_dense_destroy.argtypes = [vp]
         lib.gevva_dense_launch.argtypes = [vp, vp, vp, i32, vp]
+        lib.gevva_dense_status_word.argtypes = lib.gevva_moe_status_word.argtypes = [vp]
+        lib.gevva_dense_status_word.restype = lib.gevva_moe_status_word.restype = ctypes.c_size_t
         lib.gevva_ff_layer_launch.argtypes = [ctypes.POINTER(ff._Layer), vp, vp, vp, i32, vp, vp]
 
     def runner(self, max_tokens, flags=0):
@@ -149,6 +151,19 @@ def test_dense_outputs_between_32_byte_lines(recorder, offset, last):
     dense = recorder.dense(64)
     assert recorder.lib.gevva_dense_launch(dense, ADDRESS, ADDRESS + offset, 64, STREAM) == 0
     assert kernels(recorder.launches()) == ["fp8_quantize_rows_kernel", "dense_fp8_pair_kernel", "gelu_quantize_fp8_kernel", last]
+
+
+@pytest.mark.parametrize("offset", [0, 16])
+def test_dense_waits_report_where_they_are_read(recorder, offset):
+    """A wait of the dense MLP that runs out is reported into a word that a status call reads: its own, in a layer the experts'."""
+    runner, dense = recorder.runner(1024), recorder.dense(1024)
+    assert recorder.lib.gevva_dense_launch(dense, ADDRESS, ADDRESS + offset, 600, STREAM) == 0
+    words = [l["status"] for l in recorder.launches() if l["status"]]
+    assert len(words) == 2 and set(words) == {recorder.lib.gevva_dense_status_word(dense)}
+    for tokens in (40, 600, 1000):
+        assert layer_launch(recorder, runner, dense, tokens) == 0
+        words = [l["status"] for l in recorder.launches() if l["stream"] == AUX_STREAM and l["status"]]
+        assert len(words) == 2 and set(words) == {recorder.lib.gevva_moe_status_word(runner)}
 
 
 @pytest.mark.parametrize("in_offset,out_offset", [(8, 0), (2, 0), (0, 8), (0, 2)])
