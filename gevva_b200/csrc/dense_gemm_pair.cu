@@ -129,15 +129,13 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     prefetch_tensor_map(&map_a);
     prefetch_tensor_map(&map_b);
   }
-  if (warp == kFpMmaWarp) {
-    tmem_alloc(&smem->tmem_base, kFpTmemColumns);  // the whole tensor memory: both CTAs get address 0
-    tmem_relinquish();
-  }
+  // Both CTAs run and their barriers exist before either touches the other's tensor memory or arrives there.
+  __syncwarp();
+  cluster_sync_all();
+  if (warp == kFpMmaWarp) pair_tmem_alloc(&smem->tmem_base, kFpTmemColumns);  // the whole tensor memory
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  // Barriers of both CTAs exist before either CTA arrives on the other's.
-  cluster_sync_all();
   const uint32_t tmem_base = smem->tmem_base;
   grid_dependency_wait();
   grid_launch_dependents();
@@ -293,7 +291,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   if (warp == kFpMmaWarp) {
     tc_fence_after_sync();
     __syncwarp();
-    tmem_dealloc(tmem_base, kFpTmemColumns);
+    pair_tmem_dealloc(tmem_base, kFpTmemColumns);
   }
 }
 

@@ -167,15 +167,13 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     prefetch_tensor_map(&map_b);
     prefetch_tensor_map(&map_b_sf);
   }
-  if (warp == kDpMmaWarp) {
-    tmem_alloc(&smem->tmem_base, kDpTmemColumns);  // the whole tensor memory: both CTAs get address 0
-    tmem_relinquish();
-  }
+  // Both CTAs run and their barriers exist before either touches the other's tensor memory or arrives there.
+  __syncwarp();
+  cluster_sync_all();
+  if (warp == kDpMmaWarp) pair_tmem_alloc(&smem->tmem_base, kDpTmemColumns);  // the whole tensor memory
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  // Barriers of both CTAs exist before either CTA arrives on the other's.
-  cluster_sync_all();
   const uint32_t tmem_base = smem->tmem_base;
   // The weights and the plan come from before the previous kernel, which let this one start after its own wait.
   if (!p.early_weights) grid_dependency_wait();
@@ -435,7 +433,7 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (warp == kDpMmaWarp) {
     tc_fence_after_sync();
     __syncwarp();
-    tmem_dealloc(tmem_base, kDpTmemColumns);
+    pair_tmem_dealloc(tmem_base, kDpTmemColumns);
   }
 }
 

@@ -23,10 +23,10 @@
 // to `empty` of both CTAs (the commit's multicast form), and after the last K block to both
 // `acc_full`.  The epilogue warps of both CTAs drain their own 128 accumulator rows exactly as in
 // the single-CTA kernel and release the accumulator to the leader (the second CTA by remote
-// arrives).  Tensor memory is allocated by each CTA for itself (all 512 columns, so both get the
-// same addresses).  Every wait is bounded; a CTA that gives up still reaches the cluster barrier
+// arrives).  Tensor memory is allocated for both CTAs at once.  Every wait is bounded; a CTA that gives up still reaches the cluster barrier
 // at the end, which keeps both CTAs resident until no remote arrive or copy can be in flight.
 #include "gv_common.cuh"
+#include "gv_cta_pair.cuh"
 #include "gv_gemm_parts.cuh"
 #include "gv_launchers.h"
 
@@ -222,17 +222,15 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
     prefetch_tensor_map(&map_a_sf);
     prefetch_tensor_map(&map_b_sf);
   }
-  if (warp == 1) {
-    tmem_alloc(&smem->tmem_base, kPairTmemColumns);  // the whole tensor memory: both CTAs get address 0
-    tmem_relinquish();
-  }
+  // Both CTAs run and their barriers exist before either touches the other's tensor memory or arrives there.
+  __syncwarp();
+  cluster_sync_all();
+  if (warp == 1) pair_tmem_alloc(&smem->tmem_base, kPairTmemColumns);  // the whole tensor memory
   if (kMode == kGeglu) load_erf_table(smem->erf_table);
   grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  // Barriers of both CTAs exist before either CTA arrives on the other's.
-  cluster_sync_all();
   const uint32_t tmem_base = smem->tmem_base;
   grid_dependency_wait();
 
@@ -475,7 +473,7 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
   if (warp == 1) {
     tc_fence_after_sync();
     __syncwarp();
-    tmem_dealloc(tmem_base, kPairTmemColumns);
+    pair_tmem_dealloc(tmem_base, kPairTmemColumns);
   }
 }
 

@@ -201,18 +201,16 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
     prefetch_tensor_map(&map_x_sf);
     prefetch_tensor_map(&map_w_sf);
   }
-  if (warp == kWpMmaWarp) {
-    tmem_alloc(&smem->tmem_base, kWpTmemColumns);  // the whole tensor memory: both CTAs get address 0
-    tmem_relinquish();
-  }
+  // Both CTAs run and their barriers exist before either touches the other's tensor memory or arrives there.
+  __syncwarp();
+  cluster_sync_all();
+  if (warp == kWpMmaWarp) pair_tmem_alloc(&smem->tmem_base, kWpTmemColumns);  // the whole tensor memory
   load_geglu_tables(&smem->tables);
   __syncthreads();
   fill_geglu_tables(&smem->tables);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  // Barriers of both CTAs exist before either CTA arrives on the other's.
-  cluster_sync_all();
   const uint32_t tmem_base = smem->tmem_base;
   // The plan and the weights may come from before the previous kernel: see W13PairOperands::early_weights.
   if (!p.early_weights) grid_dependency_wait();
@@ -500,7 +498,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
   if (warp == kWpMmaWarp) {
     tc_fence_after_sync();
     __syncwarp();
-    tmem_dealloc(tmem_base, kWpTmemColumns);
+    pair_tmem_dealloc(tmem_base, kWpTmemColumns);
   }
 }
 

@@ -5,6 +5,20 @@
 
 namespace gv {
 
+// Tensor memory of both CTAs at once, `columns` in each and at the same address: PTX wants one value of .cta_group for all tcgen05
+// instructions of a kernel.  A warp of either CTA takes part, both after a cluster barrier (both CTAs run) and the release before either
+// exits.  No CTA of the pair can hold its half while the other waits for a neighbour's: every kernel here that allocates
+// tensor memory asks for more than half of an SM's shared memory, so that no two of them share one.
+__device__ __forceinline__ void pair_tmem_alloc(uint32_t* smem_result, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(columns)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void pair_tmem_dealloc(uint32_t address, uint32_t columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(address), "r"(columns) : "memory");
+}
+
 __device__ __forceinline__ void pair_arrive_remote(uint64_t* local_bar, uint32_t target_cta) {
   const uint32_t remote = cluster_map_shared(smem_u32(local_bar), target_cta);
   // Relaxed: the arrive announces that tensor-memory reads have completed (tcgen05.wait::ld came

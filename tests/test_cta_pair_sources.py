@@ -1,0 +1,38 @@
+"""A kernel that issues tcgen05 instructions for a CTA pair (cta_group::2) issues no other form: PTX wants one value of
+.cta_group for all of them, allocation and release of tensor memory among them."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gevva_b200", "csrc")
+
+
+def code(path):
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+
+
+def one_cta_helpers():
+    """Functions of the shared headers that hold a cta_group::1 instruction."""
+    names = set()
+    for path in glob.glob(os.path.join(CSRC, "*.cuh")):
+        for function in re.finditer(r"__device__ __forceinline__ \w+ (\w+)\(.*?\n}\n", code(path), flags=re.S):
+            if "cta_group::1" in function[0]:
+                names.add(function[1])
+    return names
+
+
+PAIR_SOURCES = sorted(os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cu")) if "cta_group::2" in code(p))
+
+
+def test_helpers_are_found():
+    assert {"tmem_alloc", "tmem_relinquish", "tmem_dealloc", "tc_commit", "issue_mmas", "issue_sf_copies"} <= one_cta_helpers()
+    assert len(PAIR_SOURCES) == 4
+
+
+@pytest.mark.parametrize("source", PAIR_SOURCES)
+def test_pair_kernels_use_the_pair_forms_alone(source):
+    text = code(os.path.join(CSRC, source))
+    assert "cta_group::1" not in text
+    assert [name for name in sorted(one_cta_helpers()) if re.search(rf"\b{name}\s*[<(]", text)] == []
