@@ -284,10 +284,10 @@ struct LayerWorkspace {
 // Three layers at 0 (both sides take all SMs) / 20 / 24 / 28 / 33 / 40 / 48: 130 tokens 333 / 284 / 285 / 290 / 289 / 292 / 299,
 // 200 tokens 344 / 296 / 297 / 302 / 301 / 305 / 312, 256 tokens - / 306 / 305 / - / - / - / -, 296 tokens 363 / 333 / 325 / 316 / 313 / 317 / 324,
 // 400 tokens 355 / 364 / 331 / 335 / 333 / 333 / 338, 512 tokens 368 / - / 348 / - / 350 / 350 / 354, 640 tokens 390 / - / 403 / - / 376 / 379 / 385.
-// Above 640 tokens, where the experts no longer stream, sharing gains nothing (700 tokens 425 at 0, 422 at 40, 1024 479 and 488,
-// 2048 448 and 469).
+// Where the experts do not stream, above 640 tokens or under an option, sharing gains nothing (700 tokens 425 at 0, 422 at 40, 1024 479 and 488,
+// 2048 448 and 469; three layers at 0 and the table's share: runners with GEVVA_MOE_OPTION_W13_PAIRS 130 tokens 317 and 323, 400 345 and 388,
+// with GEVVA_MOE_OPTION_PAIRS 484 and 532, 550 and 641, with GEVVA_MOE_DECODE_MERGED=0 319 and 331, 363 and 374).
 // (48, 22 and 16 SMs are the table's, not a matter of waves.)
-constexpr int kBesideTokens = 640;
 int dense_sms_beside(int tokens, int sms) {
   const int wanted = tokens <= 4 ? 48 : tokens <= 6 ? 33 : tokens <= 12 ? 17 : tokens <= 128 ? 16 : tokens <= 256 ? 22 : 33;
   return wanted * 2 < sms ? wanted : sms / 2;
@@ -310,7 +310,7 @@ int gevva_ff_layer_launch(const gevva_ff_layer* layer, const void* hidden, void*
   // The dense MLP starts as soon as its input exists, on SMs that the router leaves idle; beside a
   // decode-sized expert launch on SMs of its own.
   const int sms = gv::moe_sm_count(layer->experts);
-  const bool split = beside && tokens <= kBesideTokens && sms > 1;
+  const bool split = beside && sms > 1 && (tokens <= gv::kFusedSortQuantizeMaxTokens || gv::moe_streams(layer->experts, tokens));
   const int dense_sms = split ? dense_sms_beside(tokens, sms) : sms;
   const int expert_sms = split ? sms - dense_sms : sms;
   gv::launch_ff_prepare(hidden, layer->dense_pre, layer->expert_pre, layer->router_scale, w.dense_in, w.expert_in,

@@ -25,7 +25,7 @@ namespace {
 using namespace gv;
 
 constexpr int kMaxTokens = 131072;
-constexpr int kStreamTokens = 640;  // see moe_launch_stages_on
+constexpr int kStreamTokens = 640;  // see moe_streams
 // w2 by CTA pairs that share weights between two row tiles of an expert: from 160 rows an expert on average (figures in
 // grouped_gemm_down_pair.cu; 2048 tokens 46.7 us by one CTA a tile and 47.5 by pairs, 3000 tokens 57 and 53).
 constexpr int kDownPairTokens = 2560;
@@ -310,6 +310,19 @@ struct StageRange {
 int gv::moe_sm_count(const gevva_moe* runner) { return runner->sm_count; }
 int gv::moe_max_tokens(const gevva_moe* runner) { return runner->scratch->max_tokens; }
 
+// Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side does both GEMMs.
+// Against the launches of larger batches (w13 by CTA pairs, then w2), us a layer of four distinct ones in a graph, one B200:
+// router logits without bias, 300 tokens 96.7 against 99.7, 400 98.4 / 101.8, 500 101 / 105.5, 640 108.2 / 112.8 (up to 296
+// tokens it also takes in the sort and the quantiser); with a bias of deviation 0.5 96.9 / 99.2, 100.3 / 102.4, 106.1 / 104.9,
+// 114.8 / 112.5; with a Zipf(1.1) bias 83.9 / 84.5, 90.3 / 86.5, 96.4 / 91.2, 110.7 / 103.7: a heavy expert has many 64-row
+// chunks, each with the whole of its weights.  The host does not know the routes.  The line is that of evenly loaded
+// experts, for which the launch pays all the way; strongly skewed batches of 400 to 640 tokens lose 4 to 7 us by it.
+// (The pair options leave batches of at most 128 tokens alone.)
+bool gv::moe_streams(const gevva_moe* runner, int tokens) {
+  const bool pair_options = (runner->pairs || runner->w13_pair_form) && tokens > gv::kFusedSortQuantizeMaxTokens;
+  return runner->merged_decode && !pair_options && tokens <= kStreamTokens;
+}
+
 int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, const float* route_weights, void* out,
                              int tokens, unsigned stages, cudaStream_t stream, int sm_count) {
   Scratch* s = runner->scratch;
@@ -324,17 +337,7 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   const bool use_pairs = runner->pairs && tokens > gv::kFusedSortQuantizeMaxTokens;
   const unsigned front = GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE;
   const unsigned layer_body = front | GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU | GEVVA_MOE_STAGE_W2;
-  // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side does both GEMMs.
-  // Against the launches of larger batches (w13 by CTA pairs, then w2), us a layer of four distinct ones in a graph, one B200:
-  // router logits without bias, 300 tokens 96.7 against 99.7, 400 98.4 / 101.8, 500 101 / 105.5, 640 108.2 / 112.8 (up to 296
-  // tokens it also takes in the sort and the quantiser); with a bias of deviation 0.5 96.9 / 99.2, 100.3 / 102.4, 106.1 / 104.9,
-  // 114.8 / 112.5; with a Zipf(1.1) bias 83.9 / 84.5, 90.3 / 86.5, 96.4 / 91.2, 110.7 / 103.7: a heavy expert has many 64-row
-  // chunks, each with the whole of its weights.  The host does not know the routes.  The line is that of evenly loaded
-  // experts, for which the launch pays all the way; strongly skewed batches of 400 to 640 tokens lose 4 to 7 us by it.
-  // (The pair options leave batches of at most 128 tokens alone.)
-  const bool pair_options = (runner->pairs || runner->w13_pair_form) && tokens > gv::kFusedSortQuantizeMaxTokens;
-  const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && runner->merged_decode && !pair_options &&
-                       tokens <= kStreamTokens;
+  const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && gv::moe_streams(runner, tokens);
   if ((stages & layer_body) == layer_body && streams && runner->decode_front && gv::stream_layer_fits(tokens, sm_count)) {
     // ... and the route sort and the quantiser; the weights stream while the input is being quantised
     StageRange range(runner->nvtx, "gevva_moe.sort+quantize+w13+geglu+w2");

@@ -144,6 +144,22 @@ def test_feed_forward_layer_launches(recorder):
         "ff_prepare_kernel", "route_project_kernel<0>", "stream_experts_kernel<1>", "ff_finalize_kernel"]
 
 
+@pytest.mark.parametrize("tokens,share", [(40, 16), (128, 16), (129, 22), (640, 33), (641, 0)])
+@pytest.mark.parametrize("flags,merged", [(0, "1"), (rt.OPTION_PAIRS, "1"), (rt.OPTION_W13_PAIRS, "1"), (0, "0")])
+def test_sms_of_the_two_sides_of_a_layer(recorder, monkeypatch, flags, merged, tokens, share):
+    """Above 128 tokens the dense MLP gets SMs of its own only where the experts stream; else both sides take all of them."""
+    monkeypatch.setenv("GEVVA_MOE_DECODE_MERGED", merged)
+    runner, dense = recorder.runner(1024, flags), recorder.dense(1024)
+    assert layer_launch(recorder, runner, dense, tokens) == 0
+    launches = recorder.launches()
+    gemms = lambda stream: [l for l in launches if l["stream"] == stream and re.match("stream|grouped|w13|dense_fp8", l["kernel"])]
+    if tokens > 128 and (flags or merged == "0"):
+        share = 0
+    assert {l["grid"] for l in gemms(STREAM)} == {148 - share}
+    assert {(l["kernel"], l["grid"]) for l in gemms(AUX_STREAM)} == (
+        {("grouped_nvfp4_gemm_kernel", share)} if share else {("dense_fp8_pair_kernel", 148)})
+
+
 @pytest.mark.parametrize("offset,last", [(0, "dense_fp8_pair_kernel"), (16, "grouped_nvfp4_gemm_kernel"),
                                          (32, "dense_fp8_pair_kernel"), (48, "grouped_nvfp4_gemm_kernel")])
 def test_dense_outputs_between_32_byte_lines(recorder, offset, last):
