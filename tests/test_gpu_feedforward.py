@@ -1,6 +1,8 @@
 """Dense FP8 GeGLU MLP and the feed-forward pre/post steps against the CPU oracle.
 Bit-exact where both sides see the same bytes (norm outputs, FP8 codes, row scales,
 finalize); 2e-2 relative L2 for the FP8 GEMM outputs."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -88,8 +90,7 @@ def test_dense_mlp_stages(dense_oracle, dense_weights, cuda_device, tokens):
 
 @pytest.mark.parametrize("tokens", [512, 513, 897, 1025])
 def test_dense_mlp_rows_do_not_depend_on_the_batch(dense_weights, cuda_device, tokens):
-    """Batches whose GEMMs take 256 weight rows an item (4224 leaves half an item over) give every row
-    the bits it has in a batch of 100, whose items have 128."""
+    """Batches of several row tiles give every row the bits it has in a batch of 100, which is one tile."""
     from gevva_b200 import feedforward as ff
     gate_up, down, gs, us, ds = dense_weights
     mlp = ff.DenseMlp(gate_up, down, gs, us, ds, tokens)
@@ -220,8 +221,7 @@ def test_thirty_layers_captured_into_one_graph_at_verifier_size(cuda_device):
 @pytest.mark.parametrize("tokens", [1, 16, 128, 129, 301])
 def test_layer_call_equals_its_parts(cuda_device, tokens):
     """gevva_ff_layer_launch against the calls it stands for, made one by one: the same bits, on one
-    stream and with the dense MLP on a second one, on both sides of the size (128 tokens) up to which
-    the dense MLP and the experts share the SMs."""
+    stream and with the dense MLP on a second one, where the two sides share the SMs."""
     from gevva_b200 import feedforward as ff
     from gevva_b200.runtime import route_project
     from gevva_b200.synthetic import SyntheticStack
@@ -241,6 +241,41 @@ def test_layer_call_equals_its_parts(cuda_device, tokens):
         torch.cuda.synchronize()
         assert torch.equal(got, want)
     layer.experts.check()
+
+
+@pytest.mark.parametrize("tokens,widths", [(1, (128, 128)), (5, (128, 128)), (8, (256, 256)), (100, (256, 256)), (200, (256, 256)),
+                                           (300, (256, 256)), (512, (128, 256)), (640, (256, 256))])
+def test_dense_mlp_beside_the_experts(cuda_device, tokens, widths):
+    """The one-CTA kernels that the dense MLP takes on its share of a layer's SMs, with 128 or 256 weight rows an item in either
+    projection, against the pair kernels of the MLP alone: its input, its gate and up projection and its unscaled output."""
+    from gevva_b200 import feedforward as ff
+    from gevva_b200.synthetic import SyntheticStack
+    sms = next(share for last, share in ((4, 48), (6, 33), (12, 17), (128, 16), (256, 22), (640, 33)) if tokens <= last)
+    tiles = (tokens + 127) // 128
+    items = lambda n_out, width: -(-tiles * -(-n_out // width) // sms)
+    assert widths == tuple(256 if 3 * items(n, 256) <= 2 * items(n, 128) else 128 for n in (2 * DENSE, HIDDEN))  # the library's rule
+    layer = SyntheticStack(1, 640, cuda_device, seed=6).layers[0]
+    lib = ff._lib()
+    hidden = hashgen.activations(tokens, HIDDEN, 55 + tokens, cuda_device)
+    out = torch.empty_like(hidden)
+    workspace = torch.zeros(lib.gevva_ff_layer_workspace_bytes(tokens), dtype=torch.uint8, device=cuda_device)
+    parts = ("dense_pre", "expert_pre", "router_scale", "router_w", "expert_scale", "dense_post", "expert_post", "combined_post",
+             "layer_scalar")
+    native = ff._Layer(*[getattr(layer, p).data_ptr() for p in parts], layer.experts._handle, layer.dense._handle)
+    aux = torch.cuda.Stream(device=cuda_device)
+    torch.cuda.synchronize()
+    assert lib.gevva_ff_layer_launch(ctypes.byref(native), hidden.data_ptr(), out.data_ptr(), workspace.data_ptr(), tokens,
+                                     torch.cuda.current_stream().cuda_stream, aux.cuda_stream) == 0
+    torch.cuda.synchronize()
+    layer.experts.check()
+    rows = tokens * HIDDEN * 2  # a multiple of 256, so the workspace's four row buffers lie end to end
+    dense_in = workspace[:rows].view(torch.bfloat16).view(tokens, HIDDEN)
+    dense_out = workspace[3 * rows : 4 * rows].view(torch.bfloat16).view(tokens, HIDDEN)
+    gate_up = layer.dense.buffer(2, torch.bfloat16)[: tokens * 2 * DENSE].clone()
+    alone, _ = layer.dense.launch(dense_in)
+    layer.dense.check()
+    assert torch.equal(layer.dense.buffer(2, torch.bfloat16)[: tokens * 2 * DENSE], gate_up)
+    assert torch.equal(alone, dense_out) and alone.float().abs().max() > 0
 
 
 @pytest.mark.parametrize("tokens", [130, 256, 257, 296, 640, 641])

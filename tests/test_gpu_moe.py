@@ -225,6 +225,51 @@ def test_route_sort_at_the_edges_of_its_forms(gm, oracle, big_runner, cuda_devic
         assert (got[key] == want[key]).all(), key
 
 
+@pytest.mark.parametrize("tokens", [128, 129, 300, 1535, 1536, 1537])
+def test_route_sort_by_owner_at_one_rank(gm, varied_weights, cuda_device, tokens):
+    """Expert-parallel ranks sort by the key that a placement table gives each expert: one rank alone, whose table is a permutation
+    of its own experts, has the bits of the plain runner in all three one-launch forms of the sort, twice over."""
+    import ctypes
+    from gevva_b200.expert_parallel import _EpConfig, local_expert_weights
+    from gevva_b200.runtime import _Weights
+    full = varied_weights[0]
+    rng = np.random.default_rng(tokens)
+    placement = [int(v) for v in rng.permutation(EXPERTS)]
+    local = local_expert_weights(full, 0, 1, placement)
+    routes = tokens * TOP_K
+    buffers = [torch.zeros(n, dtype=torch.uint8, device=cuda_device)
+               for n in (routes * (HIDDEN // 2), routes * (HIDDEN // 16), routes * HIDDEN * 2, EXPERTS * 4, 256)]
+    lists = [(ctypes.c_void_p * 1)(b.data_ptr()) for b in buffers]
+    table = (ctypes.c_int * EXPERTS)(*placement)
+    config = _EpConfig(0, 1, tokens, routes, *[ctypes.cast(l, ctypes.POINTER(ctypes.c_void_p)) for l in lists], table)
+    lib, vp = gm.library(), ctypes.c_void_p
+    address = lambda t: vp(t.data_ptr())
+    packed_weights = _Weights(*[t.data_ptr() for t in (local.w13, local.w13_sf, local.w2, local.w2_sf, local.alpha1, local.alpha2,
+                                                       local.in_scale_q1, local.in_scale_q2)])
+    ep = vp()
+    assert lib.gevva_moe_ep_create(ctypes.byref(ep), ctypes.byref(packed_weights), address(full.in_scale_q1), ctypes.byref(config)) == 0
+    runner = gm.Nvfp4ExpertRunner(full, tokens)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    for step in range(2):
+        host_ids = random_ids(tokens, 70 + step)
+        host_ids[:, 3] = 99  # an expert that is much longer than the others
+        ids = torch.from_numpy(host_ids).to(cuda_device)
+        x = hashgen.activations(tokens, HIDDEN, 41 + step, cuda_device)
+        want, got = torch.zeros_like(x), torch.zeros_like(x)
+        runner.launch_batch(x, ids, rw, want, tokens)
+        runner.check()
+        stream = vp(torch.cuda.current_stream().cuda_stream)
+        assert lib.gevva_moe_ep_route_sort(ep, address(ids), tokens, stream) == 0
+        assert lib.gevva_moe_ep_dispatch(ep, address(x), address(ids), tokens, stream) == 0
+        assert lib.gevva_moe_ep_compute(ep, stream) == 0
+        assert lib.gevva_moe_ep_barrier(ep, stream) == 0
+        assert lib.gevva_moe_ep_reduce(ep, address(rw), address(got), tokens, stream) == 0
+        rows = ctypes.c_int(0)
+        assert lib.gevva_moe_ep_status(ep, ctypes.byref(rows)) == 0 and rows.value == routes
+        assert torch.equal(got, want) and got.float().abs().max() > 0
+    lib.gevva_moe_ep_destroy(ep)
+
+
 def test_bad_expert_id_is_reported(gm, big_runner, cuda_device):
     from gevva_b200 import runtime as rt
     for tokens in (4, 300):
