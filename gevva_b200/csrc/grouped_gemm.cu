@@ -639,14 +639,11 @@ void launch_variant(const GemmOperands& op, const GemmParams& p, int sm_count, c
 }  // namespace
 
 int prepare_grouped_gemm() {
-  // This call brings a kernel's code into device memory, and where the streaming kernel's lies is worth 3 % of a layer of a few tokens, whose
-  // instructions are fetched while the weights saturate L2: loaded first 276 us (eight layers of 5 tokens), behind the others 286.
-  cudaError_t e = static_cast<cudaError_t>(prepare_stream_experts());
-  if (e != cudaSuccess) return static_cast<int>(e);
-  e = raise_smem_limit<kPlain, 1, 128>();
+  cudaError_t e = raise_smem_limit<kPlain, 1, 128>();
   if (e == cudaSuccess) e = raise_smem_limit<kGeglu, 1, 256>();
   if (e == cudaSuccess) e = raise_smem_limit<kFp8, 1, 128>();
   if (e == cudaSuccess) e = raise_smem_limit<kFp8, 1, 256>();
+  if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_stream_experts());
   if (e == cudaSuccess) e = static_cast<cudaError_t>(prepare_grouped_down());
   if (e == cudaSuccess) return prepare_grouped_gemm_pairs();
   return static_cast<int>(e);
