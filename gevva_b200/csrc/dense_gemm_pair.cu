@@ -70,35 +70,12 @@ __device__ __forceinline__ bool dense_pair_item(const DensePairParams& p, int ro
   return tile * 256 < p.tokens;
 }
 
-__device__ __forceinline__ void dense_pair_load_weights(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int half,
-                                                        int group) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
-      " [%0], [%1, {%2, %3, %3, %4, %5}], [%6];" ::"r"(smem_u32(smem_dst)),
-      "l"(tensor_map), "r"(x), "r"(0), "r"(half * 4), "r"(group), "r"(barrier)
-      : "memory");
-}
-
 __device__ __forceinline__ void dense_pair_mma(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t descriptor, uint32_t accumulate) {
   constexpr uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // 8 rows x 128 B, 128B swizzle
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"((static_cast<uint64_t>(hi) << 32) | a_lo), "l"((static_cast<uint64_t>(hi) << 32) | b_lo), "r"(descriptor), "r"(accumulate)
-      : "memory");
-}
-
-// 16 lanes x 64 columns: register 4g + i holds columns 8g + 2t + (i & 1) of row lane/4 + 8 * (i / 2).
-__device__ __forceinline__ void dense_pair_load_16x64(uint32_t tmem_address, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(tmem_address)
       : "memory");
 }
 
@@ -162,7 +139,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 #pragma unroll
             for (int j = 0; j < kPieces; ++j)
               if (j < item.pieces)
-                dense_pair_load_weights(smem->b[stage] + j * kFpPieceBytes, &map_b, bar, kb * kTileKBytes, (piece0 + j) & 1,
+                pair_load_piece(smem->b[stage] + j * kFpPieceBytes, &map_b, bar, kb * kTileKBytes, (piece0 + j) & 1,
                                         group0 + ((piece0 + j) >> 1));
           } else {
             pair_load(smem->a[stage], &map_a, bar, kb * kTileKBytes, item.token0);  // (rows past the end are not stored)
@@ -250,7 +227,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         uint32_t r[32];
         const int part = step >= groups ? 1 : 0, group = step - part * groups;
         if (step < steps) {
-          dense_pair_load_16x64(tmem_rows + (static_cast<uint32_t>(part * 16) << 16) + static_cast<uint32_t>(acc) * kN + 64 * group, r);
+          tmem_load_16x64(tmem_rows + (static_cast<uint32_t>(part * 16) << 16) + static_cast<uint32_t>(acc) * kN + 64 * group, r);
           tmem_load_wait();
         }
         if (step + 1 >= steps) {

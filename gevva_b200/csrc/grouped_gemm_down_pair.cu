@@ -31,7 +31,7 @@ constexpr int kDpColumns = 192;                 // output columns of an item (MM
 constexpr int kDpTiles = (kHidden + kDpColumns - 1) / kDpColumns;       // 15
 constexpr int kDpLastColumns = kHidden - (kDpTiles - 1) * kDpColumns;   // 128
 constexpr int kDpUnitTiles = 5;                 // items of a unit
-constexpr int kDpPairUnits = kDpTiles / kDpUnitTiles;                   // 5
+constexpr int kDpPairUnits = kDpTiles / kDpUnitTiles;                   // 3
 static_assert(kDpTiles % kDpUnitTiles == 0 && kDpLastColumns == 128, "units of whole items, the last one of N = 128");
 constexpr int kDpPieceRows = 32;                // weight rows of a copy: half a 64-column group
 // Tensor memory: two accumulators, the scales of the row tile at work (four columns an MMA), two K blocks'
@@ -111,30 +111,6 @@ struct DownPairSchedule {
     return true;
   }
 };
-
-// 32 weight rows in the column order of grouped_gemm_down.cu: half `half` of 64-column group `group`.
-__device__ __forceinline__ void down_pair_load_weights(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int half,
-                                                       int group) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
-      " [%0], [%1, {%2, %3, %3, %4, %5}], [%6];" ::"r"(smem_u32(smem_dst)),
-      "l"(tensor_map), "r"(x), "r"(0), "r"(half * 4), "r"(group), "r"(barrier)
-      : "memory");
-}
-
-// 16 lanes x 64 columns: register 4g + i holds columns 8g + 2t + (i & 1) of row lane/4 + 8 * (i / 2).
-__device__ __forceinline__ void down_pair_load_16x64(uint32_t tmem_address, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(tmem_address)
-      : "memory");
-}
 
 __global__ void __launch_bounds__(kDpThreads, 1)
 grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_sf,
@@ -229,7 +205,7 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             for (int j = 0; j < kDpColumns / 2 / kDpPieceRows; ++j) {
               const int piece = static_cast<int>(rank) * pieces + j;
               if (j < pieces)
-                down_pair_load_weights(smem->b[stage] + j * kDpPieceBytes, &map_b, bar, kb * kTileKBytes, piece & 1, group0 + (piece >> 1));
+                pair_load_piece(smem->b[stage] + j * kDpPieceBytes, &map_b, bar, kb * kTileKBytes, piece & 1, group0 + (piece >> 1));
             }
             pair_load(smem->sfb[stage], &map_b_sf, bar, 0, sf_row + 8 * kb);
             ++issued;
@@ -388,7 +364,7 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           uint32_t r[32];
           const int part = step >= groups ? 1 : 0, group = step - part * groups;
           if (step < steps) {
-            down_pair_load_16x64(tmem_rows + (static_cast<uint32_t>(part * 16) << 16) + static_cast<uint32_t>(acc) * kDpColumns + 64 * group, r);
+            tmem_load_16x64(tmem_rows + (static_cast<uint32_t>(part * 16) << 16) + static_cast<uint32_t>(acc) * kDpColumns + 64 * group, r);
             tmem_load_wait();
           }
           if (step + 1 >= steps) {

@@ -74,27 +74,6 @@ __device__ __forceinline__ void mbar_arrive_remote(uint64_t* local_bar, uint32_t
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
 
-// Arrives on the barrier at the same shared-memory offset in both CTAs of the pair once every
-// tcgen05 operation issued so far by this thread has completed.
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(static_cast<uint16_t>(3))
-      : "memory");
-}
-
-// Tensor-map load into this CTA's shared memory that completes on a barrier of either CTA of the
-// pair (`barrier` is a shared::cluster address).  No multicast: every CTA loads its own bytes.
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tensor_map, uint32_t barrier, int x,
-                                                 int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(smem_dst)),
-      "l"(tensor_map), "r"(x), "r"(y), "r"(barrier)
-      : "memory");
-}
-
 // Scale copies of one K block for both CTAs (each from its own shared memory at these offsets
 // into its own tensor memory): per MMA j the A atom, and the two weight halves.
 template <int kMmas>
@@ -302,16 +281,16 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
           if (my_bytes == 0) {
             // second CTA of a pair with one tile: no activation rows
           } else if (!weight_side) {
-            tma_load_2d_pair(smem->a[stage], short_tile ? &map_a32 : &map_a, bar, x, row);
-            tma_load_2d_pair(smem->sfa[stage], &map_a_sf, bar, 0, sf_row + 4 * kb);
+            pair_load(smem->a[stage], short_tile ? &map_a32 : &map_a, bar, x, row);
+            pair_load(smem->sfa[stage], &map_a_sf, bar, 0, sf_row + 4 * kb);
           } else if (kMode == kGeglu) {
-            tma_load_2d_pair(smem->b[stage], half_item ? &map_b64 : &map_b, bar, x, row);
+            pair_load(smem->b[stage], half_item ? &map_b64 : &map_b, bar, x, row);
             // re-tiled scales: [rows 0..127 | rows 128..255] x four MMAs, 4 KiB per K block
-            tma_load_2d_pair(smem->sfb[stage], &map_b_sf, bar, 0, sf_row + 8 * kb);
+            pair_load(smem->sfb[stage], &map_b_sf, bar, 0, sf_row + 8 * kb);
           } else {
-            tma_load_2d_pair(smem->b[stage], &map_b, bar, x, row);
-            tma_load_2d_pair(smem->sfb[stage], &map_b_sf, bar, 0, sf_row + 4 * kb);
-            tma_load_2d_pair(smem->sfb[stage] + kSfStageBytes, &map_b_sf, bar, 0, sf_row2 + 4 * kb);
+            pair_load(smem->b[stage], &map_b, bar, x, row);
+            pair_load(smem->sfb[stage], &map_b_sf, bar, 0, sf_row + 4 * kb);
+            pair_load(smem->sfb[stage] + kSfStageBytes, &map_b_sf, bar, 0, sf_row2 + 4 * kb);
           }
         }
         __syncwarp();
@@ -381,8 +360,8 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
               issue_pair_sf_copies<1>(tmem_sf, sfa_lo, sfb_lo, hi_sf);
               issue_pair_mmas<1>(tmem_base, tmem_sf, a_lo, b_lo, hi_ab, accumulate);
             }
-            tc_commit_pair(&smem->empty[stage]);   // both CTAs may refill the stage
-            if (kb + 1 == p.k_blocks) tc_commit_pair(&smem->acc_full);
+            pair_commit_both(&smem->empty[stage]);   // both CTAs may refill the stage
+            if (kb + 1 == p.k_blocks) pair_commit_both(&smem->acc_full);
           }
           if (++stage == kPairStages) {
             stage = 0;

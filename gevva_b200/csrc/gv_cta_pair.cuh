@@ -56,6 +56,16 @@ __device__ __forceinline__ void pair_load_3d(void* smem_dst, const void* tensor_
       : "memory");
 }
 
+// 32 weight rows in the column order of grouped_gemm_down.cu (map_down_pieces): half `half` of 64-column group `group`.
+__device__ __forceinline__ void pair_load_piece(void* smem_dst, const void* tensor_map, uint32_t barrier, int x, int half,
+                                                int group) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%2, %3, %3, %4, %5}], [%6];" ::"r"(smem_u32(smem_dst)),
+      "l"(tensor_map), "r"(x), "r"(0), "r"(half * 4), "r"(group), "r"(barrier)
+      : "memory");
+}
+
 __device__ __forceinline__ void pair_copy_sf(uint32_t tmem_address, uint32_t hi, uint32_t lo) {
   asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_address),
                "l"((static_cast<uint64_t>(hi) << 32) | lo)

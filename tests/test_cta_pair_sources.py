@@ -23,7 +23,7 @@ def one_cta_helpers():
     return names
 
 
-PAIR_SOURCES = sorted(os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cu")) if "cta_group::2" in code(p))
+PAIR_SOURCES = sorted(os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cu")) if re.search(r"cta_group::2|gv_cta_pair\.cuh", code(p)))
 
 
 def test_helpers_are_found():
