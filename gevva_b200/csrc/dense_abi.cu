@@ -37,7 +37,8 @@ struct gevva_dense {
 
 // Whether a GEMM of the dense MLP takes 256 weight rows an item instead of 128.  The launch lasts as many items
 // as its busiest CTA has, and a wide item takes about one and a half times a narrow one (48 KB of operands a K
-// block against 32 KB): wide where that is no longer.  Alone on 148 SMs (where pairs of CTAs run now) the MLP took (us, narrow -> wide)
+// block against 32 KB): wide where that is no longer.  Alone on 148 SMs (where pairs of CTAs run now, but for outputs that they cannot store)
+// the MLP took (us, narrow -> wide)
 // 31.9 -> 35.4 at 301 tokens, where one wave of narrow items is enough, 39.0 -> 35.5 at 600, 74.8 -> 62.6 at 2048
 // and 131.9 -> 108.4 at 4096.  On the few SMs that it gets beside the experts of a decode batch (whole layers in a graph):
 // 57.5 -> 53.7 at 8 tokens, 71.6 -> 71.8 at 16, 91.4 -> 91.9 at 40, 95.9 -> 95.7 at 64, 104.1 -> 103.2 at 128.
@@ -287,6 +288,10 @@ struct LayerWorkspace {
 // Where the experts do not stream, above 640 tokens or under an option, sharing gains nothing (700 tokens 425 at 0, 422 at 40, 1024 479 and 488,
 // 2048 448 and 469; three layers at 0 and the table's share: runners with GEVVA_MOE_OPTION_W13_PAIRS 130 tokens 317 and 323, 400 345 and 388,
 // with GEVVA_MOE_OPTION_PAIRS 484 and 532, 550 and 641, with GEVVA_MOE_DECODE_MERGED=0 319 and 331, 363 and 374).
+// Loads other than even ones, three layers in a graph at 0 / 20 / 22 / 24 / 33 SMs: bias of deviation 0.5 on the router logits, 130 tokens 290 / 257 / 258 / 256 / 263,
+// 256 tokens 324 / 292 / 293 / 295 / 298; Zipf(1.1), 130 tokens 235 / 215 / 203 / 198 / 192, 256 tokens 279 / 257 / 231 / 233 / 236 (even 340 / 304 / 305 / 306 / 308, 250
+// and 253 tokens, on both sides of the last batch whose sort 126 SMs take in, 301 / 304 at 22).  At 0 / 28 / 33 / 40: bias 0.5, 400 tokens 336 / 329 / 330 / 342, 640 tokens
+// 405 / 407 / 412 / 430, the one place where sharing gains nothing; Zipf 288 / 280 / 285 / 289 and 379 / 368 / 376 / 386.
 // (48, 22 and 16 SMs are the table's, not a matter of waves.)
 int dense_sms_beside(int tokens, int sms) {
   const int wanted = tokens <= 4 ? 48 : tokens <= 6 ? 33 : tokens <= 12 ? 17 : tokens <= 128 ? 16 : tokens <= 256 ? 22 : 33;

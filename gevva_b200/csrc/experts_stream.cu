@@ -8,8 +8,8 @@
 // a w13 item is 64 intermediate columns (11 an expert, 180 KB), so one token's eight experts keep 88 SMs busy
 // instead of 48.  A chunk ends at 64 rows because four accumulators of 64 columns and seven stages' scales fill tensor
 // memory, and seven stages with 8 KB of rows each shared memory; an expert with more rows reads its weights once a chunk.
-// Alone and from a cold L2: 64 tokens 81 us for 430 MB of DRAM traffic, 400 tokens (kFront false) 81 us for 450 MB,
-// 5.3 and 5.5 TB/s over the whole launch (before the K loops were unrolled; 6.4 from the first load to the last).
+// Alone and from a cold L2: 64 tokens 77.4 us for 422 MB of DRAM traffic, 400 tokens (kFront false) 75.2 us for 447 MB,
+// 5.5 and 5.9 TB/s over the whole launch.
 //
 //   w13 item   (chunk of at most 64 rows of an expert) x (unit of 64 intermediate columns): MMA rows 0..63
 //              are the unit's up rows, 64..127 its gate rows (one 3-D box brings both; their scales come
@@ -89,7 +89,7 @@ constexpr int kStWeightBytes = kTileM * kTileKBytes;      // 16 KiB
 constexpr int kStTokenBytes = kStRows * kTileKBytes;      // 8 KiB
 static_assert(kStreamUpItems == kUnits && kStreamDownItems == kHidden / 128, "items of a chunk");
 constexpr int kStUpKBlocks = kHidden / kTileK;            // 11
-static_assert(kStMmaWarp == 1 && kStPublishWarp - 1 == kStUpKBlocks, "warps 1..11 quantise a K block each");
+static_assert(kStMmaWarp == 1 && kStPublishWarp - 1 == kStUpKBlocks, "warps 1..11 quantise a K block of the first item each; of the CTA's own tokens warps 2..11, warp 3 two");
 static_assert(kStWeightWarp == 0 && kExperts == 128, "threads 0..127 scan the experts");
 constexpr int kStLoadUnroll = 2, kStMmaUnroll = 4;        // K blocks of w13 items
 constexpr int kStDownKBlocks = 3;                         // 704 = 256 + 256 + 192

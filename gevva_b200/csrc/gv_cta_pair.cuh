@@ -8,7 +8,8 @@ namespace gv {
 // Tensor memory of both CTAs at once, `columns` in each and at the same address: PTX wants one value of .cta_group for all tcgen05
 // instructions of a kernel.  A warp of either CTA takes part, both after a cluster barrier (both CTAs run) and the release before either
 // exits.  No CTA of the pair can hold its half while the other waits for a neighbour's: every kernel here that allocates
-// tensor memory asks for more than half of an SM's shared memory, so that no two of them share one.
+// tensor memory asks for more than half of an SM's shared memory, so that no two of them share one.  (Allocated by either CTA
+// for itself, as before: two feed-forward layers of 2048 tokens 390.2 us at their fastest, together 392.3; the dense MLP alone takes the same.)
 __device__ __forceinline__ void pair_tmem_alloc(uint32_t* smem_result, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(columns)
                : "memory");

@@ -26,8 +26,9 @@ using namespace gv;
 
 constexpr int kMaxTokens = 131072;
 constexpr int kStreamTokens = 640;  // see moe_streams
-// w2 by CTA pairs that share weights between two row tiles of an expert: from 160 rows an expert on average (figures in
-// grouped_gemm_down_pair.cu; 2048 tokens 46.7 us by one CTA a tile and 47.5 by pairs, 3000 tokens 57 and 53).
+// w2 by CTA pairs that share weights between two row tiles of an expert: from 160 rows an expert on average, where most experts
+// have two tiles.  Two layers in a graph, one CTA a tile and pairs, us: 1536 tokens 262 and 278, 2048 308 and 320, 2304 341 and 332, 2432 347 and
+// 344, 2560 362 and 361, 2688 365 and 361, 3072 383 and 371, 4096 496 and 494.  (Evenly loaded experts; the sides cross between 2048 and 2304.)
 constexpr int kDownPairTokens = 2560;
 static_assert(kStreamTokens <= gv::kStreamMaxTokens, "the streaming kernel's chunk list");
 

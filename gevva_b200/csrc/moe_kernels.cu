@@ -228,8 +228,10 @@ __device__ __forceinline__ bool grid_barrier(int* sync, int ctas, int* status) {
 // SMs): every CTA counts its chunk, all meet at a grid barrier, every CTA scans the chunk histograms.
 // Either way every CTA has its own base then (the group geometry is written by all of them with identical values) and
 // scatters its routes.  Cooperative and alone, same box, us a pass: 613 tokens 198.3 -> 191.9 (two layers), 1000 tokens 244.3 -> 237.5, 1500
-// tokens 267.4 -> 262, feed-forward layers of 300 tokens 331 -> 322 (three), 1024 tokens 323.5 -> 313.5 (two), 1500 tokens 383.7 -> 379.2; 2048
-// tokens 304.5 -> 301.5, but feed-forward layers of that size 437 -> 449, where the sort then takes SMs before the dense MLP does.
+// tokens 267.4 -> 262, feed-forward layers of 300 tokens 331 -> 322 (three), 1024 tokens 323.5 -> 313.5 (two), 1500 tokens 383.7 -> 379.2.
+// The line is where it still paid when it was drawn.  Around it, with the kernels of today, two layers called from Python and two feed-forward layers:
+// 1536 tokens 276 -> 270 and 354 -> 347, 1664 281 -> 275 and 372 -> 360, 1792 295 -> 291 and 385 -> 377, 1920 308 -> 305 and 403 -> 404, 2048 328 -> 322 and
+// 427 -> 426 (in graphs half of that and less): up to fifteen chunks would gain, too.
 constexpr int kSortAloneChunks = 12;
 __global__ void __launch_bounds__(kSortChunk)
 route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chunks, bool alone, RoutePlan plan) {
