@@ -17,11 +17,17 @@
 //   w2 item    (chunk) x (128 output columns)
 // One list per launch, all w13 items chunk by chunk, then all w2 items.  A CTA's first w13 item is given by its number,
 // further ones are claimed one by one, a little ahead; the w2 items are dealt in the order in which the CTAs run out of
-// w13 items, so that those that are one short (180 KB) get four w2 items (48 KB each) first.
+// w13 items, so that those that are one short (180 KB) get four w2 items (48 KB each) first, and the last three of each share lie in
+// a pool.  SMs get through their weights at different rates, and the CTAs on SMs that the router held start 1.7 us late: with fixed
+// shares the CTAs of 64 tokens ended between 60.4 and 67.5 us (median 62.7).
+// A CTA's items are worked out by the claim warp, ahead of their use, and the other roles read them as words from a ring.  Worked out
+// from numbers by each role for itself, and with fixed shares, us a layer: 1 token 21.05 (now 20.75), 5 33.6 (33.9), 16 55.1 (53.3), 37 72.0 (69.3), 64 77.3
+// (74.9), 200 83.5 (81.4), 613 95.9 (95.6), Zipf(1.1) 64 tokens 45.8 (45.7), 200 62.5 (60.9).  (The pool without the ring: 1 token 21.3, 5 33.5, 16 54.3,
+// 37 71.4, 64 77.9, 200 85.3 against 21.0, 33.2, 55.2, 73.2, 79.0, 86.4 on that box; two or six items of a share in it: the same.)
 //
 // Roles (14 warps): 0 fetches weights, 1 copies scale factors to tensor memory and issues MMAs, 2 fetches activations
 // (one thread each), 3 only takes part in the sort and the quantiser, 4..11 are the epilogue (two warps per 32-lane quarter, alternating
-// groups of eight rows), 12 publishes finished w13 items, 13 claims the next ones.  Seven stages of one K block (256 elements); four accumulators of 64 columns,
+// groups of eight rows), 12 publishes finished w13 items, 13 works out the next ones.  Seven stages of one K block (256 elements); four accumulators of 64 columns,
 // so nothing waits for a drain.  How fast a CTA gets through K blocks is a matter of how those three threads are written, not of
 // bytes: with a warp of its own for the scale copies (a commit and a barrier more a stage), waits by whole warps and rolled K
 // loops a w13 item whose weights lay in L2 took 3.8 us, with one thread a role and the K loops unrolled by two and four
@@ -67,7 +73,6 @@
 // Us a layer (eight in a graph, one box): 1 token 21.5 -> 21.0, 5 34.2 -> 33.0, 16 57.1 -> 55.1, 37 75.2 -> 73.0, 64 80.9 -> 77.5, 200 87.2 -> 83.6,
 // 400 92.6 -> 89.5, 613 99.7 -> 95.4.  Experts with several chunks, whose weights are read once a chunk, gain as much (Zipf(1.1), 200 tokens
 // 65.1 -> 62.5, 613 96.7 -> 94; bias of deviation 0.5, 613 tokens 102.3 -> 98.7; theirs left without the policy: 64.0, 97.0, 103).
-// The CTA that finishes last puts all counters back to zero.
 #include "gv_common.cuh"
 #include "gv_gemm_parts.cuh"
 #include "gv_launchers.h"
@@ -107,8 +112,10 @@ constexpr int kStFrontTokens = kStFrontRoutes * kStThreads / kTopK;  // 336
 constexpr int kStFrontWords = (kStFrontTokens + 31) / 32; // 11, odd: an expert's words lie in banks of their own
 constexpr uint32_t kStNoRow = 0xffffffffu;
 constexpr int kStSelfRows = 8;                            // kFront: rows of a first item that the CTA quantises itself, at most
-constexpr int kStClaims = 32;                             // claims on their way from the claim warp to the others, at most
-constexpr uint32_t kStNoMoreClaims = 1u << 15, kStNoTurn = kStNoMoreClaims - 1;
+constexpr int kStItems = 32;                              // items on their way from the claim warp to the others, at most
+constexpr int kStItemsAhead = 2;                          // item i is worked out once this many before it are still to be begun
+constexpr uint32_t kStItemDown = 1u << 21, kStItemEnd = 1u << 22;
+constexpr int kStAllPublished = 1 << 20;
 constexpr long long kStRescueCycles = 40000;              // 20 us without progress
 
 struct alignas(1024) StreamSmem {
@@ -123,11 +130,10 @@ struct alignas(1024) StreamSmem {
   uint64_t full[kStStages], empty[kStStages];
   uint64_t acc_full[kStAccStages], acc_empty[kStAccStages];
   volatile int progress[kStEpilogueWarps];  // w13 items whose rows each epilogue warp has stored
-  volatile int published;                   // w13 items that the publisher has counted
+  volatile int published;                   // w13 items that the publisher has counted; kStAllPublished at its end
   volatile int first_mine;                  // whether the CTA's first w13 item is its to count; -1: not known yet
-  volatile int begun;                       // w13 items that the weight warp has begun
-  volatile uint32_t claims[kStClaims];      // the CTA's w13 items, then its turn among the w2 items: see StreamCursor
-  volatile int downs;                       // w2 items of the CTA, once its turn is announced
+  volatile int begun;                       // items that the weight warp has begun
+  volatile uint32_t items[kStItems];        // the CTA's items: see stream_item
   uint32_t tmem_base;
   volatile int abort;
   volatile int left;  // an epilogue warp gave up waiting
@@ -184,25 +190,43 @@ struct StreamItem {
   int n_tile;  // unit of 64 intermediate columns, or tile of 128 output columns
 };
 
-// Claim `i` of this CTA: the number of a w13 item, or kStNoMoreClaims + the CTA's turn among the w2 items (kStNoTurn: it
-// gave up).  The claim warp announces one after the other, the last one also when it gives up; its own waits are
-// bounded, so this wait ends.
-__device__ __forceinline__ uint32_t stream_claim(const StreamSmem* smem, int i) {
-  const uint32_t round = static_cast<uint32_t>(i / kStClaims + 1);
-  uint32_t word = smem->claims[i % kStClaims];
-  while ((word >> 16) != round) {
+// An item as a word: expert, n_tile << 7, chunk << 12, kStItemDown; or kStItemEnd behind the last one.
+__device__ __forceinline__ uint32_t stream_word(int expert, int chunk, int n_tile) {
+  return static_cast<uint32_t>(expert) | static_cast<uint32_t>(n_tile) << 7 | static_cast<uint32_t>(chunk) << 12;
+}
+__device__ __forceinline__ StreamItem stream_unpack(uint32_t word) {
+  StreamItem it;
+  it.down = word & kStItemDown;
+  it.expert = word & 127u;
+  it.n_tile = word >> 7 & 31u;
+  it.chunk = word >> 12 & 511u;
+  return it;
+}
+static_assert(kExperts == 128 && kStreamDownItems <= 32 && kStreamUpItems <= 32 && kStMaxChunks <= 512, "fields of an item's word");
+
+// The word of item `i` of this CTA, w13 items first, with the turn of its place in the ring above it.  The claim warp works the items out and
+// announces one after the other, the end also when it gives up; its own waits are bounded, so the wait below ends.
+__device__ __forceinline__ uint32_t stream_turn(int i) { return static_cast<uint32_t>(i / kStItems + 1) << 24; }
+__device__ __forceinline__ bool stream_announced(uint32_t word, int i) { return (word & 0xff000000u) == stream_turn(i); }
+__device__ __forceinline__ bool stream_next(const StreamSmem* smem, int& taken, StreamItem& it) {
+  uint32_t word = smem->items[taken % kStItems];
+  while (!stream_announced(word, taken)) {
     __nanosleep(32);
-    word = smem->claims[i % kStClaims];
+    word = smem->items[taken % kStItems];
   }
-  return word & 0xffffu;
+  if (word & kStItemEnd) return false;
+  it = stream_unpack(word);
+  ++taken;
+  return true;
 }
 
-// By one thread of the claim warp.  No reader is further behind than the publisher (pipeline and accumulators hold six items).
-__device__ __forceinline__ void stream_announce(StreamSmem* smem, int i, uint32_t claim) {
+// By one thread of the claim warp, which is never more than three items ahead of the weight warp.  No other reader is further than nine
+// items behind that one (pipeline and accumulators), but for the publisher, which reads the w13 items.
+__device__ __forceinline__ void stream_announce(StreamSmem* smem, int i, uint32_t word) {
   const long long start = clock64();
-  while (smem->published + kStClaims <= i && !smem->abort && clock64() - start < kWaitLimitCycles) __nanosleep(64);
+  while (smem->published + kStItems <= i && !smem->abort && clock64() - start < kWaitLimitCycles) __nanosleep(64);
   __threadfence_block();
-  smem->claims[i % kStClaims] = static_cast<uint32_t>(i / kStClaims + 1) << 16 | claim;
+  smem->items[i % kStItems] = stream_turn(i) | word;
 }
 
 // The lane's view of the CTAs' first items: one that is not taken, or `firsts`.
@@ -217,41 +241,12 @@ __device__ __forceinline__ int stream_open_first(const int* sync, int firsts, in
   return open;
 }
 
-// This CTA's items in order, as each role walks them.
-struct StreamCursor {
-  int taken = 0;      // items so far
-  int ups = -1;       // w13 items of the CTA, once known
-  int turn = 0, downs = 0;
-
-  __device__ __forceinline__ StreamItem item_of(int index, bool down, const StreamSmem* smem) const {
-    const int per_chunk = down ? kStreamDownItems : kStreamUpItems;
-    const int chunk = index / per_chunk;
-    StreamItem it;
-    it.down = down;
-    it.n_tile = index - chunk * per_chunk;
-    it.expert = smem->chunk_expert[chunk];
-    it.chunk = smem->chunk_index[chunk];
-    return it;
-  }
-  __device__ __forceinline__ bool next(const StreamShares& shares, const StreamSmem* smem, StreamItem& it) {
-    if (ups < 0) {
-      const uint32_t claim = stream_claim(smem, taken);
-      if (!(claim & kStNoMoreClaims)) {
-        it = item_of(static_cast<int>(claim), false, smem);
-        ++taken;
-        return true;
-      }
-      ups = taken;
-      turn = static_cast<int>(claim & kStNoTurn);
-      __threadfence_block();
-      downs = smem->downs;
-    }
-    if (taken - ups >= downs) return false;
-    it = item_of(shares.down_item(turn, taken - ups), true, smem);
-    ++taken;
-    return true;
-  }
-};
+// Item `index` of the list of w13 items, or of that of w2 items.
+__device__ __forceinline__ uint32_t stream_word_of(int index, bool down, const StreamSmem* smem) {
+  const int per_chunk = down ? kStreamDownItems : kStreamUpItems;
+  const int chunk = index / per_chunk;
+  return stream_word(smem->chunk_expert[chunk], smem->chunk_index[chunk], index - chunk * per_chunk) | (down ? kStItemDown : 0u);
+}
 
 __device__ __forceinline__ void tmem_load_32x8(uint32_t tmem_address, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -547,7 +542,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     prefetch_tensor_map(&maps.up[0]);
     prefetch_tensor_map(&maps.down[0]);
   }
-  if (tid < kStClaims) smem->claims[tid] = 0;
+  if (tid < kStItems) smem->items[tid] = 0;
   if (kFront && tid < kTopK) {
     smem->route_at[tid] = make_uint2(kStNoRow, 0);
     smem->route_multiplier[tid] = 1.0f;
@@ -571,6 +566,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     stream_quantise_token(p.packed, p.scales, smem, 0, 0, lane, make_uint4(0, 0, 0, 0), true);
     stream_quantise_stage(nullptr, smem, warp - 4, 0, 1, 0, true, 0, 1.0f, lane, true);
   }
+  const int first_chunk = cta / kStreamUpItems, first_unit = cta - first_chunk * kStreamUpItems;  // the CTA's first w13 item
   grid_dependency_wait();  // what earlier kernels of the stream wrote is visible from here on
   int* const sync = p.plan.stream_sync;
   int first_taken = 0;
@@ -670,10 +666,10 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     for (int c = 0; c < chunks; ++c) {
       smem->chunk_expert[chunk + c] = static_cast<short>(tid);
       smem->chunk_index[chunk + c] = static_cast<short>(c);
+      if (chunk + c == first_chunk) smem->items[0] = stream_turn(0) | stream_word(tid, c, first_unit);
     }
     if (tid == kExperts - 1) {
       const int all_chunks = chunk + chunks;
-      if (cta < all_chunks * kStreamUpItems) smem->claims[0] = 1u << 16 | static_cast<uint32_t>(cta);
       smem->offsets[kExperts] = row + count;
       smem->scale_rows[kExperts] = (tile + tiles) * kTileM;
       smem->chunks = all_chunks;
@@ -694,19 +690,19 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     fence_proxy_async_smem();  // a stage whose tokens are not used after all is filled by a tensor-map copy
   }
   __syncthreads();
-  const StreamShares shares(smem->chunks, ctas);
-  StreamCursor cursor;
+  const int ups = smem->chunks * kStreamUpItems;  // w13 items of the launch
+  int taken = 0;                                  // items that this thread's role has walked past
   StreamItem it{};
   bool ok = true;
 
   // kFront: the CTA's first w13 item does not wait for the grid's quantised rows: its own warps put them into
   // the pipeline stages (not the concern of the weight and claim warps, which leave it out)
-  bool self_first = kFront && cta < shares.up;
+  bool self_first = kFront && cta < ups;
   if (kFront && warp != kStWeightWarp && warp != kStClaimWarp) {  // the weights are under way meanwhile
     const uint4* const input = reinterpret_cast<const uint4*>(p.input);
     int first = 0, first_rows = 0;
     if (self_first) {
-      it = cursor.item_of(cta, false, smem);
+      it = stream_unpack(smem->items[0]);
       first = it.chunk * kStRows;
       first_rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
       first_rows = first_rows > kStRows ? kStRows : first_rows;
@@ -721,7 +717,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       __syncwarp();
     }
     // The CTA's own tokens come first where some CTA has a second item, which needs the grid's.
-    const bool own_first = shares.up > ctas;
+    const bool own_first = ups > ctas;
 #pragma unroll 1
     for (int step = 0; step < 2; ++step) {
       if ((step == 0) != own_first) {
@@ -784,13 +780,13 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     uint32_t phase = 0;
     bool rows_pending = kFront && !weight_side;
     if (self_first && !weight_side) {
-      (void)cursor.next(shares, smem, it);
+      (void)stream_next(smem, taken, it);
       stage = kStUpKBlocks % kStStages;
       phase = kStUpKBlocks / kStStages & 1;
     }
     if (elect_one()) {
-      while (ok && cursor.next(shares, smem, it)) {
-        if (weight_side && !it.down) smem->begun = cursor.taken;
+      while (ok && stream_next(smem, taken, it)) {
+        if (weight_side) smem->begun = taken;
         const int first = it.chunk * kStRows;
         const int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
         const int boxes = rows >= kStRows ? kStRows / 8 : (rows + 7) / 8;
@@ -870,16 +866,16 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     // the rest of the item's weights and the start of the next item's are asked into L2: 100 tokens 502.6 -> 501.6 us a pass of six
     // layers, 150 tokens 346.9 -> 344.4 (four), 200 tokens 356.5 -> 352.5, 290 tokens 368.8 -> 364.  (From every CTA: 1 token 171 -> 177,
     // 64 tokens 647 -> 651, because there the ring is at work all the time; the whole next item: no better at 200, 657 at 64.)
-    if (!self_first && cta < shares.up && elect_one()) {
+    if (!self_first && cta < ups && elect_one()) {
 #pragma unroll 1
       for (int n = 0; n < 2; ++n) {
-        uint32_t word = smem->claims[n];
-        for (int spin = 0; (word >> 16) != 1 && spin < 200 && !smem->abort; ++spin) {
+        uint32_t word = smem->items[n];
+        for (int spin = 0; !stream_announced(word, n) && spin < 200 && !smem->abort; ++spin) {
           __nanosleep(32);
-          word = smem->claims[n];
+          word = smem->items[n];
         }
-        if ((word >> 16) != 1 || (word & kStNoMoreClaims)) break;
-        const StreamItem ahead = cursor.item_of(static_cast<int>(word & 0xffffu), false, smem);
+        if (!stream_announced(word, n) || (word & (kStItemDown | kStItemEnd))) break;
+        const StreamItem ahead = stream_unpack(word);
         const uint8_t* sf = p.w13_scales + static_cast<size_t>(ahead.expert * kUnitSlots + ahead.n_tile) * kStUpKBlocks * kSfStageBytes;
 #pragma unroll 2
         for (int k = n ? 0 : kStStages; k < (n ? kStUpKBlocks - kStStages : kStUpKBlocks); ++k) {
@@ -902,7 +898,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       const uint32_t sfb_lo0 = (smem_u32(smem->sfb[0]) & 0x3ffffu) >> 4;
       constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);  // 8 rows x 16 B, no swizzle
       bool landed = false;  // the next stage's bytes have been seen
-      while (ok && cursor.next(shares, smem, it)) {
+      while (ok && stream_next(smem, taken, it)) {
         const int first = it.chunk * kStRows;
         int rows = smem->offsets[it.expert + 1] - smem->offsets[it.expert] - first;
         rows = rows > kStRows ? kStRows : rows;
@@ -956,54 +952,82 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     // load, and weights that are asked for that much later are lost time (by the weight warp itself, 37 tokens took 3.4 us a
     // layer more).
     if (lane == 0) smem->first_mine = first_taken == 0;
+    const StreamShares shares(smem->chunks, ctas);
     int turn = shares.fixed_turn(cta);
-    bool exhausted = shares.up <= ctas, all_started = false;
+    bool exhausted = shares.up <= ctas, all_started = false, gave_up = false;
+    int i = cta < shares.up ? 1 : 0;
 #pragma unroll 1
-    for (int i = cta < shares.up ? 1 : 0;; ++i) {
+    for (;; ++i) {
       if (!all_started) all_started = __all_sync(0xffffffffu, stream_open_first(sync, shares.firsts, lane) == shares.firsts);
       const long long start = clock64();
-      bool wanted = i <= 2 || smem->begun >= i - 1;
+      bool wanted = i <= kStItemsAhead || smem->begun >= i - kStItemsAhead + 1;
       while (!wanted && !smem->abort && clock64() - start < 2 * kWaitLimitCycles) {
         __nanosleep(64);
-        wanted = smem->begun >= i - 1;
+        wanted = smem->begun >= i - kStItemsAhead + 1;
       }
-      uint32_t claim = kStNoMoreClaims | kStNoTurn;
-      if (__all_sync(0xffffffffu, wanted)) {
+      gave_up = !__all_sync(0xffffffffu, wanted);
+      int index = -1;  // the claimed item, if any
+      if (!gave_up) {
         if (!exhausted) {
-          int index = 0;
           if (lane == 0) index = shares.firsts + atomicAdd(sync + kStreamItemClaims, 1);
           index = __shfl_sync(0xffffffffu, index, 0);
-          claim = static_cast<uint32_t>(index);
           exhausted = index >= shares.up;
           turn = index - shares.up;
+          if (exhausted) index = -1;
         }
         while (exhausted) {
           // the end, unless a CTA has not started: after a while its first item is this one's
           const int open = all_started ? shares.firsts : stream_open_first(sync, shares.firsts, lane);
           const uint32_t any = __ballot_sync(0xffffffffu, open < shares.firsts);
-          if (any == 0) {
-            claim = kStNoMoreClaims | static_cast<uint32_t>(turn);
-            break;
-          }
-          claim = kStNoMoreClaims | kStNoTurn;
-          if (__any_sync(0xffffffffu, smem->abort)) break;
+          if (any == 0) break;
+          gave_up = __any_sync(0xffffffffu, smem->abort);
+          if (gave_up) break;
           if (__any_sync(0xffffffffu, clock64() - start > kStRescueCycles)) {
             const int source = __ffs(static_cast<int>(any)) - 1;
-            int taken = 1;
-            if (lane == source) taken = atomicExch(sync + kStreamFirsts + open, 1);
-            claim = static_cast<uint32_t>(__shfl_sync(0xffffffffu, open, source));
-            if (__shfl_sync(0xffffffffu, taken, source) == 0) break;
+            int was_taken = 1;
+            if (lane == source) was_taken = atomicExch(sync + kStreamFirsts + open, 1);
+            index = __shfl_sync(0xffffffffu, open, source);
+            if (__shfl_sync(0xffffffffu, was_taken, source) == 0) break;
+            index = -1;
           }
           __nanosleep(64);
         }
       }
-      if (lane == 0) {
-        if (claim & kStNoMoreClaims) smem->downs = claim == (kStNoMoreClaims | kStNoTurn) ? 0 : shares.down_count(turn);
-        stream_announce(smem, i, claim);
-      }
+      if (index < 0) break;
+      if (lane == 0) stream_announce(smem, i, stream_word_of(index, false, smem));
       __syncwarp();
-      if (claim & kStNoMoreClaims) break;
     }
+    // The CTA's share of the w2 items but for its last ones; those of all shares lie in a pool.  SMs get through their weights at
+    // different rates, and the CTAs that waited for the router's SMs start late.  A claim takes as long as an item, so two are on their way at a time.
+    if (lane == 0) {
+      const int pooled = gave_up ? 0 : shares.pooled(), pool = pooled * ctas;
+      const int share = gave_up ? 0 : shares.down_count(turn) - pooled;
+      int next = pool, after = pool;
+#pragma unroll 1
+      for (int k = 0;; ++k, ++i) {
+        const long long start = clock64();
+        bool near = true;
+        while (near && smem->begun < i - kStItemsAhead) {
+          __nanosleep(64);
+          near = !smem->abort && clock64() - start < 2 * kWaitLimitCycles;
+        }
+        if (k + 1 == share || (k == 0 && share == 0)) {
+          if (pooled) {
+            next = atomicAdd(sync + kStreamDownClaims, 1);
+            after = atomicAdd(sync + kStreamDownClaims, 1);
+          }
+        }
+        const bool fixed = k < share;
+        if (!near || !(fixed || next < pool)) break;
+        stream_announce(smem, i, stream_word_of(fixed ? shares.down_item(turn, k) : shares.pool_item(next), true, smem));
+        if (!fixed) {
+          next = after;
+          if (after < pool) after = atomicAdd(sync + kStreamDownClaims, 1);
+        }
+      }
+      stream_announce(smem, i, kStItemEnd);
+    }
+    __syncwarp();
   } else if (warp == kStPublishWarp) {
     // ---------------- publisher ----------------
     // Making an item's stores visible to the grid takes one to two microseconds under load.  The epilogue
@@ -1017,8 +1041,8 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       const int first_mine = __shfl_sync(0xffffffffu, smem->first_mine, 0);
       if (first_mine < 0) done = published;
       if (done == published) {
-        const uint32_t next = smem->claims[published % kStClaims];
-        const bool over = (next >> 16) == static_cast<uint32_t>(published / kStClaims + 1) && (next & kStNoMoreClaims);
+        const uint32_t next = smem->items[published % kStItems];
+        const bool over = stream_announced(next, published) && (next & (kStItemDown | kStItemEnd));
         const long long idle = clock64() - start;
         if (__any_sync(0xffffffffu, over || smem->abort || idle > 2 * kWaitLimitCycles)) break;
         if (kFront && rescue && __any_sync(0xffffffffu, idle > kStRescueCycles)) {
@@ -1031,16 +1055,17 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       __threadfence_block();
       __syncwarp();
       for (int i = published + lane; i < done; i += 32) {
-        const uint32_t word = smem->claims[i % kStClaims];
+        const uint32_t word = smem->items[i % kStItems];
         // (overwritten only where the claim warp gave up waiting; a first item that another CTA took is that CTA's to count)
-        if ((word >> 16) == static_cast<uint32_t>(i / kStClaims + 1) && (i > 0 || first_mine > 0))
-          stream_add_release(p.plan.tile_ready + cursor.item_of(static_cast<int>(word & 0xffffu), false, smem).expert);
+        if (stream_announced(word, i) && (i > 0 || first_mine > 0))
+          stream_add_release(p.plan.tile_ready + stream_unpack(word).expert);
       }
       __syncwarp();
       published = done;
       if (lane == 0) smem->published = done;
       start = clock64();
     }
+    if (lane == 0) smem->published = kStAllPublished;
   } else if (warp >= kStEpilogueWarp) {
     // ---------------- epilogue ----------------
     const int quarter = warp & 3;                        // the tensor-memory lanes this warp may read
@@ -1048,7 +1073,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     const int et = tid - kStEpilogueWarp * 32;
     int acc = 0, buffer = 0;
     uint32_t acc_phase = 0;
-    while (cursor.next(shares, smem, it)) {
+    while (stream_next(smem, taken, it)) {
       const int first = it.chunk * kStRows;
       const int row0 = smem->offsets[it.expert] + first;
       int rows = smem->offsets[it.expert + 1] - row0;
@@ -1189,7 +1214,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       __syncwarp();
       if (lane == 0) {
         __threadfence_block();
-        smem->progress[warp - kStEpilogueWarp] = cursor.taken;
+        smem->progress[warp - kStEpilogueWarp] = taken;
       }
     }
   }
@@ -1205,7 +1230,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
   // before a CTA's end.
   if (tid == 0) {
     __threadfence();
-    smem->last = atomicAdd(sync + kStreamFinished, 1) == static_cast<int>(gridDim.x) - 1;
+    smem->last = atomicAdd(sync + kStreamFinished, 1) == ctas - 1;
   }
   __syncthreads();
   if (smem->last) {

@@ -22,12 +22,17 @@ constexpr int kStreamFinished = 1;      // CTAs at their end
 constexpr int kStreamRescued = 2;       // tokens quantised in place of CTAs that are not running
 constexpr int kStreamItemClaims = 32;
 constexpr int kStreamRescueClaims = 33;
+constexpr int kStreamDownClaims = 34;
 constexpr int kStreamFirsts = 64;       // per CTA: its first w13 item is taken
 constexpr int kStreamMaxCtas = 256;
 constexpr int kStreamSyncInts = kStreamFirsts + kStreamMaxCtas;
 
 constexpr int kStreamUpItems = 11;      // w13 items (64 intermediate columns) of a chunk
 constexpr int kStreamDownItems = 22;    // w2 items (128 output columns)
+
+// A pool of each share's last three w2 items (ends the launch evenly, see experts_stream.cu), from eight items a share on: with a
+// pool of two from six on, 8 tokens took 41.45 us a layer instead of 41.3.
+constexpr int kStreamPooled = 3, kStreamLongShare = 8;
 
 struct StreamShares {
   int ctas, up, down, firsts;  // w13 items 0 .. firsts - 1 are CTAs' first ones, firsts .. up - 1 are claimed
@@ -55,6 +60,13 @@ struct StreamShares {
       k -= pre;
     }
     return pre * lacking + turn + k * ctas;
+  }
+  // The last w2 items of every share go to whoever comes for them, where the smallest share has some to spare.
+  GV_HD_MEMBER int pooled() const { return down - pre * lacking >= kStreamLongShare * ctas ? kStreamPooled : 0; }
+  // The j-th of them, one of each share after the other.
+  GV_HD_MEMBER int pool_item(int j) const {
+    const int turn = j % ctas;
+    return down_item(turn, down_count(turn) - kStreamPooled + j / ctas);
   }
 };
 

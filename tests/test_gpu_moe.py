@@ -996,6 +996,28 @@ def test_streaming_experts_equal_the_two_launches(gm, weights, cuda_device, toke
     assert results[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens,experts", [(6, 48), (7, 56), (8, 64), (16, 128), (640, 78)])
+def test_streaming_items_from_the_pool(gm, weights, cuda_device, tokens, experts, monkeypatch):
+    """Shares of w2 items just too short for a pool, just long enough and longer, and more items a CTA than the ring of their words
+    has places (78 experts of 65 or 66 rows, two chunks each): the rows of the two launches, three times on one scratch."""
+    from gevva_b200 import runtime as rt
+    ids = (np.arange(tokens * TOP_K, dtype=np.int32) % experts).reshape(tokens, TOP_K)
+    x = hashgen.activations(tokens, HIDDEN, 31, cuda_device)
+    dev_ids = torch.from_numpy(ids).to(cuda_device)
+    rows = []
+    for merged in ("0", "1"):
+        monkeypatch.setenv("GEVVA_MOE_DECODE_MERGED", merged)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        out = runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN]
+        for _ in range(3 if merged == "1" else 1):
+            out.zero_()
+            runner.launch_batch_unreduced(x, dev_ids, tokens)
+            runner.check()
+            rows.append(out.clone())
+    assert rows[0].float().abs().max() > 0
+    assert all(torch.equal(rows[0], other) for other in rows[1:])
+
+
 @pytest.mark.parametrize("tokens", [297, 1000])
 def test_captured_layer_equals_the_eager_one(gm, weights, cuda_device, tokens):
     """A batch whose route sort is one cooperative launch, captured into a graph (where that launch is an

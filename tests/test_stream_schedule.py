@@ -22,3 +22,13 @@ def test_no_wait_on_a_cta_that_is_not_running(probe, chunks, ctas, running):
     for seed in range(3):
         result = subprocess.run([probe, str(chunks), str(ctas), str(running), str(seed)], capture_output=True, text=True)
         assert result.stdout.strip() == "ok", (chunks, ctas, running, seed, result.stdout)
+
+
+@pytest.mark.parametrize("ctas", [1, 2, 16, 115, 126, 132, 148, 256])
+def test_shares_and_pool_hold_every_item_once(tmp_path, ctas):
+    """Every number of chunks: both sides of the shortest share that gives items to the pool, and of the shares that begin with extra items."""
+    binary = str(tmp_path / "probe")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-o", binary, os.path.join(ROOT, "tests", "stream_pool_probe.cpp")], check=True)
+    for chunks in range(1, 257):
+        result = subprocess.run([binary, str(chunks), str(ctas)], capture_output=True, text=True)
+        assert result.stdout.strip() == "ok", (chunks, ctas, result.stdout)
