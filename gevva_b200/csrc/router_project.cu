@@ -4,9 +4,9 @@
 // (src/cuda/runtime/prefill.cuh:414-422, :1203-1210: cublasGemmEx / cuBLASLt FP8
 // [tokens,2816] x [128,2816]^T -> bf16 [tokens,128], followed by
 // route_128_top8_kernel<<<tokens,128>>>).  Here both are one kernel and the logits never
-// reach HBM: tokens sit on MMA-M (64 or 128 per tile), the 128 experts on MMA-N, K = 2816.
+// reach HBM: tokens sit on MMA-M (16 to 128 per tile), the 128 experts on MMA-N, K = 2816.
 //
-// A tile (of 64 tokens in batches of up to 2048) has its K range split over a cluster of four CTAs (two, or one, for batches whose tiles
+// A tile (of 16, 32 or 64 tokens in batches of up to 2048) has its K range split over a cluster of four CTAs (two, or one, for batches whose tiles
 // would otherwise not fit one wave of SMs; eight for batches of at most 512 tokens), so a
 // 4096-token batch runs on 128 SMs and a decode-sized batch streams the router matrix through
 // eight SMs instead of one.  Each
@@ -16,10 +16,10 @@
 // st.shared::cluster stores), and after one cluster barrier each owner sums the partials of its
 // rows (a tile's / split) in rank order (a fixed order: results do not depend on timing), adds the optional
 // per-expert bias, rounds to bf16 as the GEMM would have stored it, and routes its rows (gv_route.cuh): a warp per
-// token where it has at most eight, else four lanes per token.
+// token where it has at most two a warp, else four lanes per token.
 //
 // Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer and owner of tensor memory, warps
-// 2..5 epilogue (thread = accumulator row).  Every mbarrier wait is bounded (status word
+// from 2 on epilogue (thread = accumulator row, the columns shared by warps of equal lanes).  Every mbarrier wait is bounded (status word
 // kWaitTimeout); the cluster barrier is reached by every thread whatever happened before.
 #include "gv_common.cuh"
 #include "gv_launchers.h"
@@ -32,22 +32,27 @@ namespace {
 // CTAs per cluster = K slices per token tile: 8 for small batches, else 4, 2 or 1, the largest that
 // keeps the launch within one wave of SMs (a tile's pass is a chain of latencies, so waves cost more
 // than depth)
-constexpr int kRpThreads = 192;
-constexpr int kSmallTile = 64;
-// Batches up to which the tiles have 64 rows: twice as many CTAs, each with half the partial sums to send, reduce
-// and route.  9.7 -> 6.8 us at 128 and 200 tokens, 10.2 -> 7.6 at 512, 10.2 -> 9.3 at 1024, 10.5 -> 9.7 at 2048; above,
-// the clusters no longer run all at once (2368 tokens: 11.0 against 17.3).  The K split, which decides the
-// order of the sums, depends on the number of 128-row tiles either way.
-constexpr int kSmallTileTokens = 2048;
-constexpr int kWarpRows = 8;   // rows of a CTA up to which a warp routes a row (two each); above, a quad of lanes does
+// Epilogue warps.  64 rows keep eight busy (four -> eight, us alone: 37 tokens 5.9 -> 5.5, 64 6.7 -> 6.4, 613 9.0 -> 8.2, 1024 9.2 -> 8.4,
+// 2048 10.0 -> 9.1); with fewer rows eight are 0.1 slower than four.
+template <int kRows> constexpr int kRpEpilogueWarps = kRows == 64 ? 8 : 4;
+template <int kRows> constexpr int kRpThreads = (2 + kRpEpilogueWarps<kRows>) * 32;
+// Rows of a tile.  In batches of up to 2048 tokens the launch is a chain of latencies, and the fewer rows a cluster has, the fewer partial sums
+// each CTA has to send, reduce and route.  128 -> 64 rows, us alone: 9.7 -> 6.8 at 128 and 200 tokens, 10.2 -> 7.6 at 512, 10.2 -> 9.3 at 1024, 10.5 -> 9.7
+// at 2048; above, the clusters no longer run all at once (2368 tokens: 11.0 against 17.3).  64 -> 32 rows: 37 tokens 5.5 -> 5.2, 64 6.2 -> 5.4,
+// 200 6.4 -> 5.6, 400 6.7 -> 5.8, but 512, whose 16 clusters of eight do not run all at once, 6.7 -> 10.3.  32 -> 16 rows: 37 tokens 5.2 -> 4.9,
+// 64 5.4 -> 4.9, 128 5.4 -> 5.0; whole layers 37 tokens 69.6 -> 69.2 us, 64 75.3 -> 75.1, but 128 76.4 -> 76.6 (the fastest runs): the experts' CTAs
+// start late on the SMs of a router's CTAs, so that the line for 16 rows is drawn at 64 tokens.
+// The K split, which decides the order of the sums, depends on the number of 128-row tiles either way.
+constexpr int kSmallTile = 64, kSmallTileTokens = 2048;
+constexpr int tile_rows(int tokens) { return tokens <= 64 ? 16 : tokens <= 400 ? 32 : tokens <= kSmallTileTokens ? kSmallTile : kTileM; }
+template <int kRows> constexpr int kWarpRows = 2 * kRpEpilogueWarps<kRows>;  // rows of a CTA up to which a warp routes a row (two each); above, a quad of lanes does
 constexpr int kRpTileBytes = kTileM * kTileKBytes;  // 16 KiB: 128 rows of one 128-byte K block
 
-// kRows: token rows of a tile.  64 is the form of batches of at most kSmallTileTokens tokens, where
-// the launch is a chain of latencies: with eight CTAs a tile the five or six K blocks of each all fit the ring (half a token tile
-// each; the MMA reads the next tile's bytes as rows 64..127, whose results nobody looks at).
+// kRows: token rows of a tile.  Below 128, with eight CTAs a tile, the five or six K blocks of each all fit the ring; the MMA, whose
+// M is 128, reads what lies behind the tile (always inside this structure) as its further rows, whose results nobody looks at.
 template <int kRows>
 struct alignas(1024) RouterSmem {
-  static constexpr int kStages = kRows == 64 ? 6 : 5;
+  static constexpr int kStages = kRows <= 64 ? 6 : 5;
   static constexpr int kTokenBytes = kRows * kTileKBytes;
   uint8_t a[kStages][kTokenBytes];
   uint8_t b[kStages][kRpTileBytes];
@@ -125,7 +130,7 @@ __device__ __forceinline__ void issue_router_k_block(uint32_t tmem_acc, uint32_t
 }
 
 template <bool kFp8, int kSplit, int kRows>
-__global__ void __launch_bounds__(kRpThreads, 1)
+__global__ void __launch_bounds__(kRpThreads<kRows>, 1)
 route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                      const RouterParams p) {
   using Smem = RouterSmem<kRows>;
@@ -229,8 +234,10 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   } else {
     // ---------------- epilogue, part 1: partial sums to the rows' owners ----------------
     // (the per-expert scale, which part 2 would otherwise look up behind its last comparison)
-    smem->expert_scale[threadIdx.x - 64] = p.expert_scale[threadIdx.x - 64];
+    if (threadIdx.x - 64 < kExperts) smem->expert_scale[threadIdx.x - 64] = p.expert_scale[threadIdx.x - 64];
     const int quarter = warp & 3;  // the tensor-memory lanes this warp may read
+    constexpr int kParts = 4 / (kRpEpilogueWarps<kRows> / 4);  // the columns of a row are shared by the quarter's warps
+    const int first_part = (warp - 2) / 4 * kParts;
     const int row = quarter * 32 + lane;
     const int owner = row % kSplit;
     const int owner_row = row / kSplit;
@@ -244,7 +251,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
           cluster_map_shared(smem_u32(smem->received + (rank * kOwnRows + owner_row) * kExperts),
                              static_cast<uint32_t>(owner));
 #pragma unroll 1
-      for (int part = 0; part < 4; ++part) {
+      for (int part = first_part; part < first_part + kParts; ++part) {
         uint32_t r[32];
         tmem_load_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 32, r);
         tmem_load_wait();
@@ -270,10 +277,11 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const int tile_rows = p.tokens - m_tile * kRows;   // may exceed the tile
     // rows kSplit * i + rank < tile_rows
     const int own_rows = tile_rows >= kRows ? kOwnRows : (tile_rows - static_cast<int>(rank) + kSplit - 1) / kSplit;
-    const bool few = kOwnRows <= kWarpRows || own_rows <= kWarpRows;
+    constexpr int kWarps = kRpEpilogueWarps<kRows>;
+    const bool few = kOwnRows <= kWarpRows<kRows> || own_rows <= kWarpRows<kRows>;
     if (few) {
       // a few rows: one warp per row, four logits a lane (a third of the quads' chain)
-      for (int row_local = warp - 2; row_local < own_rows; row_local += 4) {
+      for (int row_local = warp - 2; row_local < own_rows; row_local += kWarps) {
         const int token = m_tile * kRows + row_local * kSplit + static_cast<int>(rank);
         float4 acc = make_float4(0, 0, 0, 0);
 #pragma unroll
@@ -296,7 +304,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                         p.ids + static_cast<size_t>(token) * kTopK);
       }
     }
-    if constexpr (kOwnRows > kWarpRows) if (!few) {
+    if constexpr (kOwnRows > kWarpRows<kRows>) if (!few) {
     const int t = threadIdx.x - 64;
     const int part = t & 3;         // columns [32 * part, 32 * part + 32)
 #pragma unroll 1
@@ -382,7 +390,7 @@ cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, c
   const int m_tiles = (p.tokens + kRows - 1) / kRows;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(m_tiles * kSplit));
-  config.blockDim = dim3(kRpThreads);
+  config.blockDim = dim3(kRpThreads<kRows>);
   config.dynamicSmemBytes = router_smem_bytes<kRows>();
   config.stream = stream;
   // Clusters of kSplit CTAs; and the launch may begin while the previous kernel of the stream is
@@ -404,8 +412,11 @@ template <bool kFp8>
 cudaError_t launch_split(const CUtensorMap& map_x, const CUtensorMap& map_w, const RouterParams& p,
                          cudaStream_t stream) {
   const int m_tiles = (p.tokens + kTileM - 1) / kTileM;
+  const int tile = tile_rows(p.tokens);
+  if (tile == 16) return launch_variant<kFp8, 8, 16>(map_x, map_w, p, stream);
+  if (tile == 32) return launch_variant<kFp8, 8, 32>(map_x, map_w, p, stream);
   if (m_tiles <= 4) return launch_variant<kFp8, 8, kSmallTile>(map_x, map_w, p, stream);
-  if (p.tokens <= kSmallTileTokens) return launch_variant<kFp8, 4, kSmallTile>(map_x, map_w, p, stream);
+  if (tile == kSmallTile) return launch_variant<kFp8, 4, kSmallTile>(map_x, map_w, p, stream);
   if (m_tiles * 4 <= 160) return launch_variant<kFp8, 4, kTileM>(map_x, map_w, p, stream);
   if (m_tiles * 2 <= 160) return launch_variant<kFp8, 2, kTileM>(map_x, map_w, p, stream);
   return launch_variant<kFp8, 1, kTileM>(map_x, map_w, p, stream);
@@ -419,7 +430,7 @@ int launch_route_project(const void* x, const void* router_w, bool fp8, const fl
                          cudaStream_t stream) {
   const uint64_t row_bytes = fp8 ? kHidden : 2 * kHidden;
   CUtensorMap map_x, map_w;
-  if (!make_operand_tensor_map(&map_x, x, static_cast<uint64_t>(tokens), row_bytes, tokens <= kSmallTileTokens ? kSmallTile : kTileM) ||
+  if (!make_operand_tensor_map(&map_x, x, static_cast<uint64_t>(tokens), row_bytes, tile_rows(tokens)) ||
       !make_operand_tensor_map(&map_w, router_w, kExperts, row_bytes, kTileM))
     return static_cast<int>(cudaErrorInvalidValue);
   RouterParams p{};

@@ -125,6 +125,13 @@ def test_router_tiles_of_few_rows(cuda_device, rows, of, fp8):
         assert torch.equal(few[:rows], many[:rows])
 
 
+@pytest.mark.parametrize("rows", [7, 15, 16, 17, 31, 33, 48, 97, 161, 383, 400, 401, 416, 417])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_router_tiles_of_16_and_32_rows(cuda_device, rows, fp8):
+    """Tiles of 16, 32 and 64 rows, whole and ragged, with the same split of K: the rows of a larger batch, bit by bit."""
+    test_router_tiles_of_few_rows(cuda_device, rows, 512, fp8)
+
+
 def test_router_projection_feeds_the_layer(oracle, cuda_device):
     """The fused router in front of the expert runner: the layer step made of C-ABI calls only."""
     import gevva_b200 as gm
