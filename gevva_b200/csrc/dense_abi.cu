@@ -28,6 +28,7 @@ struct gevva_dense {
   void* gate_up_out = nullptr;    // bf16 [T, 4224], unscaled
   uint8_t* prod_fp8 = nullptr;    // [T, 2112]
   float* prod_scales = nullptr;   // [T]
+  void* few_products = nullptr;   // bf16 [kDenseFewTokens, 2112]
   float* ones = nullptr;          // [128]
   float* gelu_table = nullptr;    // [GV_GELU_FLOATS]
   float* down_scale = nullptr;    // [1]: weights.down_scale on the device, for gevva_ff_finalize
@@ -51,6 +52,25 @@ static bool wide_items(int tokens, int n_out, int sms) {
 
 int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
                         int sm_count, int* status) {
+  if (tokens <= gv::kDenseFewTokens) {
+    // (these have no waits that could run out, and need no plan)
+    gv::DenseFewOperands op{};
+    op.input = in;
+    op.gate_up_weights = static_cast<const uint8_t*>(d->weights.gate_up);
+    op.down_weights = static_cast<const uint8_t*>(d->weights.down);
+    op.gate_scale = d->weights.gate_scale;
+    op.up_scale = d->weights.up_scale;
+    op.act_codes = d->act_fp8;
+    op.prod_codes = d->prod_fp8;
+    op.act_scales = d->act_scales;
+    op.prod_scales = d->prod_scales;
+    op.gate_up = d->gate_up_out;
+    op.products = d->few_products;
+    op.out = out_unscaled;
+    op.serial_launch = sm_count < d->sm_count;
+    gv::launch_dense_few(op, tokens, stream);
+    return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
+  }
   gv::RoutePlan plan = d->plan;
   plan.status = status;
   gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, plan, stream);
@@ -91,6 +111,7 @@ void gevva_dense_destroy(gevva_dense* d) {
   cudaFree(d->gate_up_out);
   cudaFree(d->prod_fp8);
   cudaFree(d->prod_scales);
+  cudaFree(d->few_products);
   cudaFree(d->ones);
   cudaFree(d->gelu_table);
   cudaFree(d->down_scale);
@@ -123,6 +144,7 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
   if (e == cudaSuccess) e = cudaMalloc(&d->gate_up_out, t * 2 * kDense * 2);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->prod_fp8), t * kDense);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->prod_scales), t * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&d->few_products, gv::kDenseFewTokens * kDense * 2);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->ones), gv::kExperts * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->down_scale), sizeof(float));
   if (e == cudaSuccess)
@@ -282,6 +304,8 @@ struct LayerWorkspace {
 // weight rows in one wave, 17 those of 256 (whole layers in a graph, us, at 16 / 17 / 33 / 48 SMs: 1 token 46.4 / 38.9 / 34.4 /
 // 32.3, 4 tokens 52.8 / 45.0 / 44.2 / 43.4, 5 tokens 55.5 / 47.7 / 44.9 / 47.2, 8 tokens 60.5 / 52.1 / 54.2 / 57.4, 12 tokens
 // 62.7 / 62.3 / 64.2 / 68.1, 40 tokens 93.6 / 94.6 / 99.6 / -, 128 tokens 107.4 / 108.4 / 109.9 / -).
+// (With one or two tokens the dense side is dense_few_rows.cu now, whose CTAs take no notice of the share: at 48 / 40 / 32 / 16 SMs
+// 1 token 25.8 / 25.7 / 26.7 / 32.4, 2 tokens 29.2 / 28.9 / 30.5 / 35.7.)
 // Three layers at 0 (both sides take all SMs) / 20 / 24 / 28 / 33 / 40 / 48: 130 tokens 333 / 284 / 285 / 290 / 289 / 292 / 299,
 // 200 tokens 344 / 296 / 297 / 302 / 301 / 305 / 312, 256 tokens - / 306 / 305 / - / - / - / -, 296 tokens 363 / 333 / 325 / 316 / 313 / 317 / 324,
 // 400 tokens 355 / 364 / 331 / 335 / 333 / 333 / 338, 512 tokens 368 / - / 348 / - / 350 / 350 / 354, 640 tokens 390 / - / 403 / - / 376 / 379 / 385.

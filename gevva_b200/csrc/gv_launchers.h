@@ -142,6 +142,21 @@ bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t expert
 // The w2 GEMM of prefill-sized batches (grouped_gemm_down.cu): op.map_a, map_b_down, down_scales.
 size_t retiled_w2_scale_bytes(int experts);
 void launch_retile_w2_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, cudaStream_t stream);
+// The dense MLP of a few tokens (dense_few_rows.cu): rows of the caller's tensors aligned to 16 bytes, weights to 16.
+constexpr int kDenseFewTokens = 2;
+struct DenseFewOperands {
+  const void* input;               // bf16 [tokens, 2816]
+  const uint8_t* gate_up_weights;  // [4224, 2816]
+  const uint8_t* down_weights;     // [2816, 2112]
+  float gate_scale, up_scale;
+  uint8_t *act_codes, *prod_codes;
+  float *act_scales, *prod_scales;
+  void* gate_up;                   // bf16 [tokens, 4224], unscaled
+  void* products;                  // bf16 [kDenseFewTokens, 2112]
+  void* out;                       // bf16 [tokens, 2816], unscaled
+  bool serial_launch;              // the second launch does not begin before the first one has ended
+};
+void launch_dense_few(const DenseFewOperands& op, int tokens, cudaStream_t stream);
 // The dense projections by CTA pairs (dense_gemm_pair.cu): op.map_a, map_down_pieces, out, n_out, k_in.
 int prepare_dense_pairs();
 void launch_dense_pairs(const GemmOperands& op, int tokens, int* status, int sm_count, cudaStream_t stream);

@@ -88,6 +88,12 @@ def test_dense_mlp_stages(dense_oracle, dense_weights, cuda_device, tokens):
     assert rel_l2(bf16_to_f32(bits(out)), bf16_to_f32(want_out)) < 5e-3
 
 
+@pytest.mark.parametrize("tokens", [2, 3])
+def test_dense_mlp_of_a_few_rows(dense_oracle, dense_weights, cuda_device, tokens):
+    """The two launches of up to two tokens (one token above), and the first size beyond."""
+    test_dense_mlp_stages(dense_oracle, dense_weights, cuda_device, tokens)
+
+
 @pytest.mark.parametrize("tokens", [512, 513, 897, 1025])
 def test_dense_mlp_rows_do_not_depend_on_the_batch(dense_weights, cuda_device, tokens):
     """Batches of several row tiles give every row the bits it has in a batch of 100, which is one tile."""

@@ -169,6 +169,16 @@ def test_dense_outputs_between_32_byte_lines(recorder, offset, last):
     assert kernels(recorder.launches()) == ["fp8_quantize_rows_kernel", "dense_fp8_pair_kernel", "gelu_quantize_fp8_kernel", last]
 
 
+@pytest.mark.parametrize("tokens,few", [(1, True), (2, True), (3, False)])
+def test_dense_mlp_of_a_few_tokens(recorder, tokens, few):
+    dense = recorder.dense(64)
+    assert recorder.lib.gevva_dense_launch(dense, ADDRESS, ADDRESS + 16, tokens, STREAM) == 0
+    got = kernels(recorder.launches())
+    want = (["dense_few_gate_up_kernel", "dense_few_down_kernel"] if few else
+            ["fp8_quantize_rows_kernel", "dense_fp8_pair_kernel", "gelu_quantize_fp8_kernel", "grouped_nvfp4_gemm_kernel"])
+    assert len(got) == len(want) and all(name.endswith(end) for name, end in zip(got, want))
+
+
 @pytest.mark.parametrize("offset", [0, 16])
 def test_dense_waits_report_where_they_are_read(recorder, offset):
     """A wait of the dense MLP that runs out is reported into a word that a status call reads: its own, in a layer the experts'."""
