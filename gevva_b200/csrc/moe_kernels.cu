@@ -51,9 +51,41 @@ route_128_top8_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
                   weights + static_cast<size_t>(safe_row) * kTopK, ids + static_cast<size_t>(safe_row) * kTopK);
 }
 
+// The same, a warp a token (a third of the quad's chain), while the warps are few: us alone, a quad and a warp a token: 1 token 3.9 and 1.8, 200 3.6 and 1.85,
+// 613 3.8 and 2.1, 1024 3.6 and 2.1, 2048 3.6 and 2.7, 4096 3.9 and 3.6, but 8192 4.4 and 5.4, 16384 6.4 and 8.5.
+constexpr int kWarpRouteTokens = 4096;
+__global__ void __launch_bounds__(128)
+route_128_top8_warp_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
+                           const __nv_bfloat16* __restrict__ expert_scale, float* __restrict__ weights,
+                           int* __restrict__ ids, int rows, const float* __restrict__ activation_scales,
+                           const float* __restrict__ projection_weight_scale) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(logits) + static_cast<size_t>(row) * ld + 4 * lane;
+  uint2 packed;
+  if ((reinterpret_cast<uintptr_t>(logits) & 7) == 0 && (ld & 3) == 0) {
+    packed = __ldg(reinterpret_cast<const uint2*>(src));
+  } else {  // a view whose rows are not 8-byte aligned
+    packed.x = static_cast<uint32_t>(src[0]) | (static_cast<uint32_t>(src[1]) << 16);
+    packed.y = static_cast<uint32_t>(src[2]) | (static_cast<uint32_t>(src[3]) << 16);
+  }
+  float rescale = 1.0f;
+  if (activation_scales) rescale = __fmul_rn(activation_scales[row], projection_weight_scale[0]);
+  route_top8_warp(packed, lane, activation_scales != nullptr, rescale, expert_scale, weights + static_cast<size_t>(row) * kTopK,
+                  ids + static_cast<size_t>(row) * kTopK);
+}
+
 void launch_route(const void* logits_bf16, int ld, const void* expert_scale_bf16, float* weights,
                   int* ids, int tokens, const float* activation_scales,
                   const float* projection_weight_scale, cudaStream_t stream) {
+  if (tokens <= kWarpRouteTokens) {
+    launch_chained(route_128_top8_warp_kernel, dim3((tokens + 3) / 4), dim3(128), 0, stream,
+                   static_cast<const __nv_bfloat16*>(logits_bf16), ld, static_cast<const __nv_bfloat16*>(expert_scale_bf16),
+                   weights, ids, tokens, activation_scales, projection_weight_scale);
+    return;
+  }
   launch_chained(route_128_top8_kernel, dim3((tokens + 31) / 32), dim3(128), 0, stream,
                  static_cast<const __nv_bfloat16*>(logits_bf16), ld, static_cast<const __nv_bfloat16*>(expert_scale_bf16),
                  weights, ids, tokens, activation_scales, projection_weight_scale);

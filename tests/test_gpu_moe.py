@@ -996,6 +996,27 @@ def test_streaming_experts_equal_the_two_launches(gm, weights, cuda_device, toke
     assert results[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("rows", [1, 3, 4, 5, 613, 4096])
+@pytest.mark.parametrize("stride,offset", [(EXPERTS, 0), (EXPERTS + 4, 4), (EXPERTS + 2, 2), (EXPERTS + 1, 1)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_router_by_warps_equals_router_by_quads(gm, cuda_device, rows, stride, offset, fp8):
+    """Up to 4096 tokens a warp routes a token, above four lanes do: the same rows in a batch of 4097, ties, infinities and NaN among
+    them, from rows that are aligned to 16, 8, 4 and 2 bytes."""
+    logits = hashgen.activations(4097, stride, 17, cuda_device)
+    logits[::3] = (logits[::3].float() * 4).round().to(torch.bfloat16) / 4  # ties
+    logits[1::7, 5::16] = float("inf")
+    logits[2::7, 3::16] = float("-inf")
+    logits[3::11, 9::32] = float("nan")
+    view = logits[:, offset : offset + EXPERTS]
+    scale = (0.5 + torch.arange(EXPERTS, device=cuda_device) / EXPERTS).to(torch.bfloat16)
+    act = torch.rand(4097, device=cuda_device) + 0.5 if fp8 else None
+    ws = torch.full((1,), 0.75, device=cuda_device) if fp8 else None
+    few_weights, few_ids = gm.route_128_top8(view[:rows], scale, activation_scales=act[:rows] if fp8 else None, projection_weight_scale=ws)
+    all_weights, all_ids = gm.route_128_top8(view, scale, activation_scales=act, projection_weight_scale=ws)
+    assert torch.equal(few_ids, all_ids[:rows])
+    assert torch.equal(few_weights.view(torch.int32), all_weights[:rows].view(torch.int32))
+
+
 @pytest.mark.parametrize("tokens,experts", [(6, 48), (7, 56), (8, 64), (16, 128), (640, 78)])
 def test_streaming_items_from_the_pool(gm, weights, cuda_device, tokens, experts, monkeypatch):
     """Shares of w2 items just too short for a pool, just long enough and longer, and more items a CTA than the ring of their words
