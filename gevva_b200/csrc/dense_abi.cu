@@ -2,7 +2,8 @@
 // expert path (declared in include/gevva_moe.h).  The reference runs the three dense
 // projections through cuBLASLt (Fp8LinearRunner::launch_unscaled,
 // src/cuda/runtime/fp8_linear.cuh:215-473, called at src/cuda/runtime/prefill.cuh:1211-1230);
-// here they are the tcgen05 kernels of dense_gemm_pair.cu or, beside the experts, of grouped_gemm.cu in its FP8 form.
+// here they are the tcgen05 kernels of dense_gemm_pair.cu or, beside the experts, of grouped_gemm.cu in its FP8 form; dense_few_rows.cu for
+// one or two tokens.
 #include <cuda.h>
 #include <cuda_runtime.h>
 

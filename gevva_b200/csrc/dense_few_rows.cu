@@ -11,6 +11,8 @@
 //   * E4M3 values are exact in fp16, and so are the products of two in fp32: mma.m16n8k16 with fp32 sums, the tokens on its N side (a shape
 //     that tcgen05 would fill with 128 rows).  A lane's 16 consecutive bytes are four MMAs' share of K for it, in the same order on both
 //     sides.  The warps' sums are added in a fixed order.
+//     Against sums in 64 bits the projections are as far off as the tcgen05 ones: 1.7e-3 of the norm, all of it the bf16
+//     result; 2 to 4 results in ten thousand are not the nearest bf16 (those: 2 to 5).
 // MLP alone, us, those launches -> these: 1 token 23.3 -> 8.8, 2 22.5 -> 8.5 (a variant for four tokens 22.4 -> 9.9, for eight 22.5 -> 15: every CTA
 // quantises all of them).  Feed-forward layers in a graph, us a layer: 1 token 31.0 -> 25.7, 2 31.5 -> 29.1, 3 32.0 -> 32.4, 4 34.7 -> 35.8, 5 39.8 -> 45
 // to 51: the longer these CTAs hold SMs, the later the experts' start, which want them all.  Hence the line at two tokens, and beside the

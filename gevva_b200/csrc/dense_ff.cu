@@ -8,7 +8,8 @@
 //                (gelu_quantize_fp8_2112_kernel, src/cuda/kernels/fp8.cuh:308-364)
 //   ff_finalize  8-route weighted reduce + three RMSNorms + residual + layer scalar
 //                (finalize_feedforward_routes_2816_kernel, normalization.cuh:249-377)
-// The projections themselves are in dense_gemm_pair.cu and, for the few SMs beside the experts, grouped_gemm.cu in its FP8 form.
+// The projections themselves are in dense_gemm_pair.cu and, for the few SMs beside the experts, grouped_gemm.cu in its FP8 form; the whole
+// MLP of one or two tokens is dense_few_rows.cu, with the arithmetic of the row kernels here.
 // Rows are 2816 wide: 352 threads x 8 columns, 16-byte loads and stores.  Sums of squares
 // are folded in one fixed order (thread, shuffle-down tree, warps in order) and the
 // reciprocal square root is IEEE, so a CPU can reproduce every bit.

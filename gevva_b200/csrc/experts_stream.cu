@@ -8,8 +8,8 @@
 // a w13 item is 64 intermediate columns (11 an expert, 180 KB), so one token's eight experts keep 88 SMs busy
 // instead of 48.  A chunk ends at 64 rows because four accumulators of 64 columns and seven stages' scales fill tensor
 // memory, and seven stages with 8 KB of rows each shared memory; an expert with more rows reads its weights once a chunk.
-// Alone and from a cold L2: 64 tokens 77.4 us for 422 MB of DRAM traffic, 400 tokens (kFront false) 75.2 us for 447 MB,
-// 5.5 and 5.9 TB/s over the whole launch.
+// Alone and from a cold L2: 64 tokens 75.8 us for 430 MB of DRAM traffic, 400 tokens (kFront false) 72.2 us for 440 MB,
+// 5.7 and 6.1 TB/s over the whole launch.
 //
 //   w13 item   (chunk of at most 64 rows of an expert) x (unit of 64 intermediate columns): MMA rows 0..63
 //              are the unit's up rows, 64..127 its gate rows (one 3-D box brings both; their scales come
@@ -23,7 +23,7 @@
 // A CTA's items are worked out by the claim warp, ahead of their use, and the other roles read them as words from a ring.  Worked out
 // from numbers by each role for itself, and with fixed shares, us a layer: 1 token 21.05 (now 20.75), 5 33.6 (33.9), 16 55.1 (53.3), 37 72.0 (69.3), 64 77.3
 // (74.9), 200 83.5 (81.4), 613 95.9 (95.6), Zipf(1.1) 64 tokens 45.8 (45.7), 200 62.5 (60.9).  (The pool without the ring: 1 token 21.3, 5 33.5, 16 54.3,
-// 37 71.4, 64 77.9, 200 85.3 against 21.0, 33.2, 55.2, 73.2, 79.0, 86.4 on that box; two or six items of a share in it: the same.)
+// 37 71.4, 64 77.9, 200 85.3 against 21.0, 33.2, 55.2, 73.2, 79.0, 86.4 in that comparison; two or six items of a share in it: the same.)
 //
 // Roles (14 warps): 0 fetches weights, 1 copies scale factors to tensor memory and issues MMAs, 2 fetches activations
 // (one thread each), 3 only takes part in the sort and the quantiser, 4..11 are the epilogue (two warps per 32-lane quarter, alternating
@@ -70,7 +70,7 @@
 // are run once on nothing in front of the dependency wait (37 tokens 615 -> 611, 40-token feed-forward layers 343 -> 338).
 // Weights are asked for with an L2 policy that lets them give way first.  A launch passes 400 MB through L2, and without
 // the policy that pushes out what the next launches start with: their code, the router's matrix, tokens, rows and counters.
-// Us a layer (eight in a graph, one box): 1 token 21.5 -> 21.0, 5 34.2 -> 33.0, 16 57.1 -> 55.1, 37 75.2 -> 73.0, 64 80.9 -> 77.5, 200 87.2 -> 83.6,
+// Us a layer (eight in a graph, one GPU): 1 token 21.5 -> 21.0, 5 34.2 -> 33.0, 16 57.1 -> 55.1, 37 75.2 -> 73.0, 64 80.9 -> 77.5, 200 87.2 -> 83.6,
 // 400 92.6 -> 89.5, 613 99.7 -> 95.4.  Experts with several chunks, whose weights are read once a chunk, gain as much (Zipf(1.1), 200 tokens
 // 65.1 -> 62.5, 613 96.7 -> 94; bias of deviation 0.5, 613 tokens 102.3 -> 98.7; theirs left without the policy: 64.0, 97.0, 103).
 #include "gv_common.cuh"
