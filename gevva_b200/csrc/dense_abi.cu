@@ -24,6 +24,7 @@ struct gevva_dense {
   int sm_count = 0;
   gv::RoutePlan plan{};
   gv::GemmOperands gate_up{}, down{};
+  CUtensorMap map_few_gate_up{}, map_few_down{};  // of the weights, for up to kDenseFewTokens tokens
   uint8_t* act_fp8 = nullptr;     // [T, 2816]
   float* act_scales = nullptr;    // [T]
   void* gate_up_out = nullptr;    // bf16 [T, 4224], unscaled
@@ -54,11 +55,11 @@ static bool wide_items(int tokens, int n_out, int sms) {
 int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int tokens, cudaStream_t stream,
                         int sm_count, int* status) {
   if (tokens <= gv::kDenseFewTokens) {
-    // (these have no waits that could run out, and need no plan)
+    // (these need no plan)
     gv::DenseFewOperands op{};
     op.input = in;
-    op.gate_up_weights = static_cast<const uint8_t*>(d->weights.gate_up);
-    op.down_weights = static_cast<const uint8_t*>(d->weights.down);
+    op.map_gate_up = &d->map_few_gate_up;
+    op.map_down = &d->map_few_down;
     op.gate_scale = d->weights.gate_scale;
     op.up_scale = d->weights.up_scale;
     op.act_codes = d->act_fp8;
@@ -68,6 +69,7 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
     op.gate_up = d->gate_up_out;
     op.products = d->few_products;
     op.out = out_unscaled;
+    op.status = status;
     op.serial_launch = sm_count < d->sm_count;
     gv::launch_dense_few(op, tokens, stream);
     return cudaGetLastError() == cudaSuccess ? GEVVA_MOE_OK : GEVVA_MOE_CUDA_ERROR;
@@ -185,7 +187,9 @@ int gevva_dense_create(gevva_dense** out, const gevva_dense_weights* weights, in
   ok = ok && gv::make_operand_tensor_map(&d->down.map_b, weights->down, gv::kHidden, kDense, gv::kTileM);
   ok = ok && gv::make_piece_tensor_map(&d->gate_up.map_down_pieces, weights->gate_up, 2 * kDense, gv::kHidden);
   ok = ok && gv::make_piece_tensor_map(&d->down.map_down_pieces, weights->down, gv::kHidden, kDense);
-  ok = ok && gv::prepare_dense_pairs() == 0;
+  ok = ok && gv::make_halves_tensor_map(&d->map_few_gate_up, weights->gate_up, kDense, gv::kHidden, gv::kDenseFewUpRows);
+  ok = ok && gv::make_operand_tensor_map(&d->map_few_down, weights->down, gv::kHidden, kDense, gv::kDenseFewDownRows);
+  ok = ok && gv::prepare_dense_pairs() == 0 && gv::prepare_dense_few() == 0;
   if (!ok) {
     gevva_dense_destroy(d);
     return GEVVA_MOE_CUDA_ERROR;
@@ -305,8 +309,8 @@ struct LayerWorkspace {
 // weight rows in one wave, 17 those of 256 (whole layers in a graph, us, at 16 / 17 / 33 / 48 SMs: 1 token 46.4 / 38.9 / 34.4 /
 // 32.3, 4 tokens 52.8 / 45.0 / 44.2 / 43.4, 5 tokens 55.5 / 47.7 / 44.9 / 47.2, 8 tokens 60.5 / 52.1 / 54.2 / 57.4, 12 tokens
 // 62.7 / 62.3 / 64.2 / 68.1, 40 tokens 93.6 / 94.6 / 99.6 / -, 128 tokens 107.4 / 108.4 / 109.9 / -).
-// (With one or two tokens the dense side is dense_few_rows.cu now, whose CTAs take no notice of the share: at 48 / 40 / 32 / 16 SMs
-// 1 token 25.8 / 25.7 / 26.7 / 32.4, 2 tokens 29.2 / 28.9 / 30.5 / 35.7.)
+// (With one or two tokens the dense side is dense_few_rows.cu now, 44 CTAs of an SM each: at 48 / 44 / 40 / 32 / 16 SMs 1 token 24.5 / 24.6 / 27.2 / 27.5 / 33.3,
+// 2 tokens 27.7 / 27.8 / 29.7 / 30.3 / 35.3.)
 // Three layers at 0 (both sides take all SMs) / 20 / 24 / 28 / 33 / 40 / 48: 130 tokens 333 / 284 / 285 / 290 / 289 / 292 / 299,
 // 200 tokens 344 / 296 / 297 / 302 / 301 / 305 / 312, 256 tokens - / 306 / 305 / - / - / - / -, 296 tokens 363 / 333 / 325 / 316 / 313 / 317 / 324,
 // 400 tokens 355 / 364 / 331 / 335 / 333 / 333 / 338, 512 tokens 368 / - / 348 / - / 350 / 350 / 354, 640 tokens 390 / - / 403 / - / 376 / 379 / 385.

@@ -113,35 +113,6 @@ static_assert(gemm_smem_bytes<kPlain, 1, 128>() <= 232448 && gemm_smem_bytes<kFp
               "shared memory budget of one sm_100 CTA");
 static_assert(kSfColumn + 64 * 4 <= kTmemColumns && kSfColumn + 32 * 6 <= kTmemColumns, "tensor memory budget");
 
-// Dense FP8 form of the same: kMmas MMAs of K = 32 E4M3 elements (32 bytes, the same
-// descriptor step), no scale factors.  Instruction descriptor: fp32 accumulate (bit 4),
-// E4M3 x E4M3 (format 0), both K-major, N and M as above.
-template <int kN>
-constexpr uint32_t kInstrDescFp8 = (1u << 4) | (static_cast<uint32_t>(kN >> 3) << 17) |
-                                   (static_cast<uint32_t>(kTileM >> 4) << 24);
-
-template <int kMmas>
-__device__ __forceinline__ void issue_k_block_fp8(uint32_t tmem_acc, uint32_t a_lo, uint32_t b_lo,
-                                                  uint32_t hi_ab, uint32_t descriptor, uint32_t accumulate) {
-#define GV_MMA8(j, pred)                                                   \
-  "add.u32 lo, %1, " #j "*2;\n\t"                                          \
-  "mov.b64 d0, {lo, %3};\n\t"                                              \
-  "add.u32 lo, %2, " #j "*2;\n\t"                                          \
-  "mov.b64 d1, {lo, %3};\n\t"                                              \
-  "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], d0, d1, %4, " pred ";\n\t"
-#define GV_OPERANDS8 ::"r"(tmem_acc), "r"(a_lo), "r"(b_lo), "r"(hi_ab), "r"(descriptor), "r"(accumulate) : "memory"
-#define GV_PROLOGUE8 "{\n\t.reg .pred p, pt;\n\t.reg .b32 lo;\n\t.reg .b64 d0, d1;\n\t" \
-                     "setp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
-  asm volatile(GV_PROLOGUE8 GV_MMA8(0, "p") "}" GV_OPERANDS8);
-  if constexpr (kMmas >= 2) asm volatile(GV_PROLOGUE8 GV_MMA8(1, "pt") "}" GV_OPERANDS8);
-  if constexpr (kMmas >= 3) asm volatile(GV_PROLOGUE8 GV_MMA8(2, "pt") "}" GV_OPERANDS8);
-  if constexpr (kMmas >= 4) asm volatile(GV_PROLOGUE8 GV_MMA8(3, "pt") "}" GV_OPERANDS8);
-#undef GV_MMA8
-#undef GV_OPERANDS8
-#undef GV_PROLOGUE8
-}
-
-
 // Work distribution.  Items are dealt to the persistent CTAs in snake order: round r goes to
 // CTA b as item r*G + b for even r and r*G + (G-1-b) for odd r.  In a short launch of the fused
 // wide form (at most eight rounds) the items are numbered with the expensive ones first, the

@@ -41,6 +41,33 @@ struct GemmParams {
   bool early_weights;  // see GemmOperands
 };
 
+// One 128-byte K block of the dense FP8 projections: kMmas MMAs of K = 32 E4M3 elements (32 bytes, a descriptor step of 2), no scale
+// factors.  Instruction descriptor: fp32 accumulate (bit 4), E4M3 x E4M3 (format 0), both K-major, N at [17,23) in units of 8, M at [24,29) in units of 16.
+template <int kN>
+constexpr uint32_t kInstrDescFp8 = (1u << 4) | (static_cast<uint32_t>(kN >> 3) << 17) |
+                                   (static_cast<uint32_t>(kTileM >> 4) << 24);
+
+template <int kMmas>
+__device__ __forceinline__ void issue_k_block_fp8(uint32_t tmem_acc, uint32_t a_lo, uint32_t b_lo,
+                                                  uint32_t hi_ab, uint32_t descriptor, uint32_t accumulate) {
+#define GV_MMA8(j, pred)                                                   \
+  "add.u32 lo, %1, " #j "*2;\n\t"                                          \
+  "mov.b64 d0, {lo, %3};\n\t"                                              \
+  "add.u32 lo, %2, " #j "*2;\n\t"                                          \
+  "mov.b64 d1, {lo, %3};\n\t"                                              \
+  "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], d0, d1, %4, " pred ";\n\t"
+#define GV_OPERANDS8 ::"r"(tmem_acc), "r"(a_lo), "r"(b_lo), "r"(hi_ab), "r"(descriptor), "r"(accumulate) : "memory"
+#define GV_PROLOGUE8 "{\n\t.reg .pred p, pt;\n\t.reg .b32 lo;\n\t.reg .b64 d0, d1;\n\t" \
+                     "setp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
+  asm volatile(GV_PROLOGUE8 GV_MMA8(0, "p") "}" GV_OPERANDS8);
+  if constexpr (kMmas >= 2) asm volatile(GV_PROLOGUE8 GV_MMA8(1, "pt") "}" GV_OPERANDS8);
+  if constexpr (kMmas >= 3) asm volatile(GV_PROLOGUE8 GV_MMA8(2, "pt") "}" GV_OPERANDS8);
+  if constexpr (kMmas >= 4) asm volatile(GV_PROLOGUE8 GV_MMA8(3, "pt") "}" GV_OPERANDS8);
+#undef GV_MMA8
+#undef GV_OPERANDS8
+#undef GV_PROLOGUE8
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   const __nv_bfloat162 pair = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&pair);

@@ -142,20 +142,25 @@ bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t expert
 // The w2 GEMM of prefill-sized batches (grouped_gemm_down.cu): op.map_a, map_b_down, down_scales.
 size_t retiled_w2_scale_bytes(int experts);
 void launch_retile_w2_scales(const uint8_t* sidecar_scales, uint8_t* tiled, int experts, cudaStream_t stream);
-// The dense MLP of a few tokens (dense_few_rows.cu): rows of the caller's tensors aligned to 16 bytes, weights to 16.
+// The dense MLP of a few tokens (dense_few_rows.cu): rows of the caller's tensors aligned to 16 bytes.
 constexpr int kDenseFewTokens = 2;
+constexpr int kDenseFewUpRows = 48, kDenseFewDownRows = 32;  // weight rows of a CTA: of the gate and as many of the up projection, and of the down projection
 struct DenseFewOperands {
   const void* input;               // bf16 [tokens, 2816]
-  const uint8_t* gate_up_weights;  // [4224, 2816]
-  const uint8_t* down_weights;     // [2816, 2112]
+  const CUtensorMap* map_gate_up;  // weights [2 (gate, up), 2112, 2816], boxes of kDenseFewUpRows rows of both
+  const CUtensorMap* map_down;     // weights [2816, 2112], boxes of kDenseFewDownRows rows
   float gate_scale, up_scale;
   uint8_t *act_codes, *prod_codes;
   float *act_scales, *prod_scales;
   void* gate_up;                   // bf16 [tokens, 4224], unscaled
   void* products;                  // bf16 [kDenseFewTokens, 2112]
   void* out;                       // bf16 [tokens, 2816], unscaled
+  int* status;
   bool serial_launch;              // the second launch does not begin before the first one has ended
 };
+// Weights [2, rows, row_bytes] through boxes of `box_rows` rows of both halves, 128-byte swizzle.
+bool make_halves_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, int box_rows);
+int prepare_dense_few();
 void launch_dense_few(const DenseFewOperands& op, int tokens, cudaStream_t stream);
 // The dense projections by CTA pairs (dense_gemm_pair.cu): op.map_a, map_down_pieces, out, n_out, k_in.
 int prepare_dense_pairs();

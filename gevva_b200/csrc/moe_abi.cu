@@ -107,18 +107,23 @@ bool make_scale_map(CUtensorMap* map, const void* base, uint64_t bytes, int box_
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// w13 codes [experts, 2 halves (up, gate), 704 rows, 1408 bytes] through a box of both halves x
-// 64 rows x 128 bytes (128-byte swizzle): one copy brings a unit's up rows and gate rows.
-bool make_w13_unit_map(CUtensorMap* map, const void* base, uint64_t experts) {
-  const cuuint64_t dims[3] = {kHidden / 2, kInter, experts * 2};
-  const cuuint64_t strides[2] = {kHidden / 2, static_cast<cuuint64_t>(kInter) * (kHidden / 2)};
-  const cuuint32_t box[3] = {static_cast<cuuint32_t>(kTileKBytes), 64, 2};
+// Bytes [halves, rows, row_bytes] through a box of two halves x box_rows rows x 128 bytes (128-byte swizzle).
+bool make_halves_map(CUtensorMap* map, const void* base, uint64_t halves, uint64_t rows, uint64_t row_bytes, int box_rows) {
+  const cuuint64_t dims[3] = {row_bytes, rows, halves};
+  const cuuint64_t strides[2] = {row_bytes, rows * row_bytes};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(kTileKBytes), static_cast<cuuint32_t>(box_rows), 2};
   const cuuint32_t element_strides[3] = {1, 1, 1};
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return false;
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box,
             element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// w13 codes [experts, 2 halves (up, gate), 704 rows, 1408 bytes] through a box of both halves x
+// 64 rows: one copy brings a unit's up rows and gate rows.
+bool make_w13_unit_map(CUtensorMap* map, const void* base, uint64_t experts) {
+  return make_halves_map(map, base, experts * 2, kInter, kHidden / 2, 64);
 }
 
 // w13 codes [experts, up and gate halves of 704 rows, 1408 bytes] in the row order of grouped_gemm_w13_pair.cu:
@@ -240,6 +245,9 @@ int make_scratch(int tokens, Scratch** out) {
 namespace gv {
 bool make_w13_unit_tensor_map(CUtensorMap* map, const void* base, uint64_t experts) {
   return make_w13_unit_map(map, base, experts);
+}
+bool make_halves_tensor_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, int box_rows) {
+  return make_halves_map(map, base, 2, rows, row_bytes, box_rows);
 }
 bool make_w2_down_tensor_map(CUtensorMap* map, const void* base, uint64_t experts) {
   return make_w2_down_map(map, base, experts);

@@ -23,10 +23,11 @@ struct Pending {
   cudaStream_t stream;
 } pending;
 
-// DensePairParams::status of dense_gemm_pair.cu and GemmParams::status of gv_gemm_parts.cuh, by their places.
+// DensePairParams::status of dense_gemm_pair.cu, GemmParams::status of gv_gemm_parts.cuh and FewParams::status of dense_few_rows.cu, by their places.
 size_t status_of(const std::string& name, void** arguments) {
   if (name.find("dense_fp8_pair_kernel") != std::string::npos) return static_cast<size_t*>(arguments[2])[1];
   if (name.find("grouped_nvfp4_gemm_kernel") != std::string::npos) return static_cast<size_t*>(arguments[3])[13];
+  if (name.find("dense_few_") != std::string::npos) return static_cast<size_t*>(arguments[1])[5];
   return 0;
 }
 

@@ -112,6 +112,47 @@ def test_dense_mlp_rows_do_not_depend_on_the_batch(dense_weights, cuda_device, t
     assert out.float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens", [1, 2])
+@pytest.mark.parametrize("of", [3, 100])
+def test_dense_mlp_of_a_few_rows_has_the_bits_of_a_larger_batch(dense_weights, cuda_device, tokens, of):
+    """One and two tokens have launches of their own (dense_few_rows.cu): every row of theirs, codes, scales, unscaled projections and all, has
+    the bits that it has in a batch of three or of a hundred."""
+    from gevva_b200 import feedforward as ff
+    gate_up, down, gs, us, ds = dense_weights
+    mlp = ff.DenseMlp(gate_up, down, gs, us, ds, of)
+
+    def launch(x):
+        rows = len(x)
+        out, _ = mlp.launch(x.contiguous())
+        parts = [mlp.buffer(i, dtype)[: rows * width].view(rows, width)
+                 for i, dtype, width in ((0, torch.uint8, HIDDEN), (1, torch.float32, 1), (2, torch.bfloat16, 2 * DENSE),
+                                         (3, torch.uint8, DENSE), (4, torch.float32, 1))] + [out]
+        return [part.clone().view(torch.uint8) for part in parts]
+
+    x = hashgen.activations(of, HIDDEN, 84, cuda_device)
+    x[1] *= 4096.0
+    x[2] = 0.0
+    whole = launch(x)
+    for first in range(0, of - tokens + 1):
+        for got, want in zip(launch(x[first : first + tokens]), whole):
+            assert torch.equal(got, want[first : first + tokens]), first
+    mlp.check()
+
+
+@pytest.mark.parametrize("tokens", [1, 2])
+@pytest.mark.parametrize("concurrent", [False, True])
+def test_layers_of_a_few_tokens_have_the_bits_of_a_larger_batch(cuda_device, tokens, concurrent):
+    """A token decoded alone and the same one among forty, through four whole layers."""
+    from gevva_b200.synthetic import SyntheticStack
+    stack = SyntheticStack(4, 40, cuda_device, seed=12)
+    hidden = hashgen.activations(40, HIDDEN, 85, cuda_device)
+    want = stack.forward(hidden, concurrent=False).clone()
+    for first in range(0, 40, 4):
+        assert torch.equal(stack.forward(hidden[first : first + tokens].contiguous(), concurrent=concurrent), want[first : first + tokens]), first
+    for layer in stack.layers:
+        layer.experts.check()
+
+
 def test_ff_finalize_bit_exact(dense_oracle, cuda_device):
     from gevva_b200 import feedforward as ff
     rows = 41
@@ -224,7 +265,7 @@ def test_thirty_layers_captured_into_one_graph_at_verifier_size(cuda_device):
         layer.experts.check()
 
 
-@pytest.mark.parametrize("tokens", [1, 16, 128, 129, 301])
+@pytest.mark.parametrize("tokens", [1, 2, 16, 128, 129, 301])
 def test_layer_call_equals_its_parts(cuda_device, tokens):
     """gevva_ff_layer_launch against the calls it stands for, made one by one: the same bits, on one
     stream and with the dense MLP on a second one, where the two sides share the SMs."""
@@ -249,11 +290,12 @@ def test_layer_call_equals_its_parts(cuda_device, tokens):
     layer.experts.check()
 
 
-@pytest.mark.parametrize("tokens,widths", [(1, (128, 128)), (5, (128, 128)), (8, (256, 256)), (100, (256, 256)), (200, (256, 256)),
+@pytest.mark.parametrize("tokens,widths", [(1, (128, 128)), (3, (128, 128)), (5, (128, 128)), (8, (256, 256)), (100, (256, 256)), (200, (256, 256)),
                                            (300, (256, 256)), (512, (128, 256)), (640, (256, 256))])
 def test_dense_mlp_beside_the_experts(cuda_device, tokens, widths):
     """The one-CTA kernels that the dense MLP takes on its share of a layer's SMs, with 128 or 256 weight rows an item in either
-    projection, against the pair kernels of the MLP alone: its input, its gate and up projection and its unscaled output."""
+    projection, against the pair kernels of the MLP alone: its input, its gate and up projection and its unscaled output.
+    (One token: the kernels of dense_few_rows.cu in both places.)"""
     from gevva_b200 import feedforward as ff
     from gevva_b200.synthetic import SyntheticStack
     sms = next(share for last, share in ((4, 48), (6, 33), (12, 17), (128, 16), (256, 22), (640, 33)) if tokens <= last)
@@ -326,7 +368,7 @@ def test_dense_pairs_at_tile_edges(dense_weights, cuda_device, tokens):
     assert guarded[:tokens].float().abs().max() > 0
 
 
-@pytest.mark.parametrize("tokens", [1, 129, 600])
+@pytest.mark.parametrize("tokens", [1, 3, 129, 600])
 def test_dense_output_aligned_to_16_bytes(dense_weights, cuda_device, tokens):
     """An output that starts between two 32-byte lines gets the bits of one that does not, and nothing around it."""
     from gevva_b200 import feedforward as ff

@@ -186,7 +186,9 @@ def test_dense_waits_report_where_they_are_read(recorder, offset):
     assert recorder.lib.gevva_dense_launch(dense, ADDRESS, ADDRESS + offset, 600, STREAM) == 0
     words = [l["status"] for l in recorder.launches() if l["status"]]
     assert len(words) == 2 and set(words) == {recorder.lib.gevva_dense_status_word(dense)}
-    for tokens in (40, 600, 1000):
+    assert recorder.lib.gevva_dense_launch(dense, ADDRESS, ADDRESS + offset, 2, STREAM) == 0
+    assert [l["status"] for l in recorder.launches()] == [recorder.lib.gevva_dense_status_word(dense)] * 2
+    for tokens in (1, 2, 40, 600, 1000):
         assert layer_launch(recorder, runner, dense, tokens) == 0
         words = [l["status"] for l in recorder.launches() if l["stream"] == AUX_STREAM and l["status"]]
         assert len(words) == 2 and set(words) == {recorder.lib.gevva_moe_status_word(runner)}
