@@ -295,12 +295,8 @@ __device__ __forceinline__ int stream_load_acquire(const int* address) {
   return value;
 }
 
-// Adds one, after everything that happened before in this thread and in those it has synchronised with.
-__device__ __forceinline__ void stream_add_release(int* address) {
-  asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(address) : "memory");
-}
-
-// The same, and it is there when this returns (a count in flight could arrive behind the zeros of the CTA that finishes last).
+// Adds one, after everything that happened before in this thread and in those it has synchronised with; it has arrived when this returns (one in
+// flight could come behind the zeros of the CTA that finishes last).
 __device__ __forceinline__ void stream_count_release(int* address, StreamSmem* smem) {
   int before;
   asm volatile("atom.release.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(address) : "memory");
@@ -1005,33 +1001,26 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       __syncwarp();
     }
     // The CTA's share of the w2 items but for its last ones; those of all shares lie in a pool.  SMs get through their weights at
-    // different rates, and the CTAs that waited for the router's SMs start late.  A claim takes as long as an item, so two are on their way at a time.
+    // different rates, and the CTAs that waited for the router's SMs start late.
     if (lane == 0) {
-      const int pooled = gave_up ? 0 : shares.pooled(), pool = pooled * ctas;
-      const int share = gave_up ? 0 : shares.down_count(turn) - pooled;
-      int next = pool, after = pool;
+      StreamDownWalk<int> walk(shares, turn);
 #pragma unroll 1
-      for (int k = 0;; ++k, ++i) {
+      for (; !gave_up; ++i) {
         const long long start = clock64();
-        bool near = true;
-        while (near && smem->begun < i - kStItemsAhead) {
+        while (!gave_up && smem->begun < i - kStItemsAhead) {
           __nanosleep(64);
-          near = !smem->abort && clock64() - start < 2 * kWaitLimitCycles;
+          gave_up = smem->abort || clock64() - start > 2 * kWaitLimitCycles;
         }
-        if (k + 1 == share || (k == 0 && share == 0)) {
-          if (pooled) {
-            next = atomicAdd(sync + kStreamDownClaims, 1);
-            after = atomicAdd(sync + kStreamDownClaims, 1);
-          }
+        if (walk.asks()) {
+          walk.next = atomicAdd(sync + kStreamDownClaims, 1);
+          walk.after = atomicAdd(sync + kStreamDownClaims, 1);
         }
-        const bool fixed = k < share;
-        if (!near || !(fixed || next < pool)) break;
-        stream_announce(smem, i, stream_word_of(fixed ? shares.down_item(turn, k) : shares.pool_item(next), true, smem));
-        if (!fixed) {
-          next = after;
-          if (after < pool) after = atomicAdd(sync + kStreamDownClaims, 1);
-        }
+        const int item = walk.item();
+        if (gave_up || item < 0) break;
+        stream_announce(smem, i, stream_word_of(item, true, smem));
+        if (walk.advance()) walk.after = atomicAdd(sync + kStreamDownClaims, 1);
       }
+      if (!walk.answered()) smem->abort = 1;  // never: what waits for the answers
       stream_announce(smem, i, kStItemEnd);
     }
     __syncwarp();
@@ -1065,7 +1054,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
         const uint32_t word = smem->items[i % kStItems];
         // (overwritten only where the claim warp gave up waiting; a first item that another CTA took is that CTA's to count)
         if (stream_announced(word, i) && (i > 0 || first_mine > 0))
-          stream_add_release(p.plan.tile_ready + stream_unpack(word).expert);
+          stream_count_release(p.plan.tile_ready + stream_unpack(word).expert, smem);
       }
       __syncwarp();
       published = done;
@@ -1234,8 +1223,8 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     tmem_dealloc(tmem_base, kStTmemColumns);
   }
   // The CTA that finishes last puts the counters back for the next launch.  No fence is needed in front of this: all waits of the CTA lie before
-  // it, its claims and its counts of tokens have returned, and its counts of w13 items have been waited for by the w2 items of their
-  // experts.  (With one, which waits for the CTA's last rows to arrive, 0.5 us a layer more: 1 token 20.75 and 20.2, 64 tokens 74.9 and 74.3.)
+  // it, and whatever the CTA has added to a counter has arrived, also where a wait ran out: the answer of every claim and every count has been
+  // looked at.  (With a fence, which waits for the CTA's last rows to arrive, 0.5 us a layer more: 1 token 20.75 and 20.2, 64 tokens 74.9 and 74.3.)
   if (tid == 0) smem->last = atomicAdd(sync + kStreamFinished, 1) == ctas - 1;
   __syncthreads();
   if (smem->last) {

@@ -70,4 +70,28 @@ struct StreamShares {
   }
 };
 
+// A CTA's walk over its w2 items: its share but for the pooled ones, then what it claims from the pool.  A claim takes as long as an
+// item, so two are on their way at a time, the first two with the last item of the share.  The walk ends with the first answer that lies
+// behind the pool; the other claim's is looked at by `answered`, without which a CTA must not end (a claim in flight could arrive behind the zeros of the
+// CTA that finishes last, and the next launch would leave an item out).
+// Index: int, or in a test a type that notices when it is looked at.
+template <class Index>
+struct StreamDownWalk {
+  StreamShares shares;
+  int turn, pool, share;  // `share`: items of the CTA's own
+  int k = 0;
+  Index next, after;      // claims
+
+  GV_HD_MEMBER StreamDownWalk(const StreamShares& s, int t) : shares(s), turn(t), pool(s.pooled() * s.ctas), share(s.down_count(t) - s.pooled()), next(pool), after(pool) {}
+  GV_HD_MEMBER bool asks() const { return pool > 0 && (k + 1 == share || (k == 0 && share == 0)); }  // for `next` and `after`
+  GV_HD_MEMBER int item() const { return k < share ? shares.down_item(turn, k) : next < pool ? shares.pool_item(next) : -1; }
+  // To the item behind this one; true where `after` is to be claimed anew.
+  GV_HD_MEMBER bool advance() {
+    if (k++ < share) return false;
+    next = after;
+    return after < pool;
+  }
+  GV_HD_MEMBER bool answered() const { return next >= 0 && after >= 0; }
+};
+
 }  // namespace gv

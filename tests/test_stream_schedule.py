@@ -1,6 +1,7 @@
 """The streaming kernel's items are shared out so that a running CTA never waits for one that has not started, as
 happens when another stream holds a part of the SMs (host form of csrc/gv_stream_schedule.h)."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -22,6 +23,17 @@ def test_no_wait_on_a_cta_that_is_not_running(probe, chunks, ctas, running):
     for seed in range(3):
         result = subprocess.run([probe, str(chunks), str(ctas), str(running), str(seed)], capture_output=True, text=True)
         assert result.stdout.strip() == "ok", (chunks, ctas, running, seed, result.stdout)
+
+
+def test_counts_have_arrived_when_a_cta_ends():
+    """The CTA that finishes last puts the counters back to zero, so whatever another one adds has to have arrived before that one ends: every
+    addition is one whose answer is waited for, none is sent off without (`red`, or an atomic whose result nothing uses)."""
+    with open(os.path.join(ROOT, "gevva_b200", "csrc", "experts_stream.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    assert not re.search(r"\bred\.", text)
+    for line in text.splitlines():
+        if re.search(r"atomic(Add|Exch)\((sync|p\.plan)", line):
+            assert re.search(r"[=?+] *atomic", line), line
 
 
 @pytest.mark.parametrize("ctas", [1, 2, 16, 115, 126, 132, 148, 256])
