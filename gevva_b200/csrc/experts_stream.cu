@@ -303,6 +303,17 @@ __device__ __forceinline__ void stream_count_release(int* address, StreamSmem* s
   if (before < 0) smem->abort = 1;  // never: what waits for the answer
 }
 
+// Of the claim warp: until the weight warp has begun `items` of the CTA's.
+__device__ __forceinline__ bool stream_wait_begun(StreamSmem* smem, int items, int* status) {
+  return stream_wait(
+      2 * kWaitLimitCycles, [&] { return smem->begun >= items; }, [&] { return smem->abort != 0; }, [] { return clock64(); },
+      [] { __nanosleep(64); },
+      [&] {
+        smem->abort = 1;
+        atomicExch(status, static_cast<int>(kWaitTimeout));
+      });
+}
+
 // Bounded acquire spin of one thread on a counter in global memory; or, where one is given, on a second one.
 __device__ __forceinline__ bool stream_wait_counter(const int* counter, int target, StreamSmem* smem, int* status,
                                                     const int* other = nullptr, int other_target = 0) {
@@ -963,12 +974,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     for (;; ++i) {
       if (!all_started) all_started = __all_sync(0xffffffffu, stream_open_first(sync, shares.firsts, lane) == shares.firsts);
       const long long start = clock64();
-      bool wanted = i <= kStItemsAhead || smem->begun >= i - kStItemsAhead + 1;
-      while (!wanted && !smem->abort && clock64() - start < 2 * kWaitLimitCycles) {
-        __nanosleep(64);
-        wanted = smem->begun >= i - kStItemsAhead + 1;
-      }
-      gave_up = !__all_sync(0xffffffffu, wanted);
+      gave_up = !__all_sync(0xffffffffu, i <= kStItemsAhead || stream_wait_begun(smem, i - kStItemsAhead + 1, status));
       int index = -1;  // the claimed item, if any
       if (!gave_up) {
         if (!exhausted) {
@@ -1006,11 +1012,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       StreamDownWalk<int> walk(shares, turn);
 #pragma unroll 1
       for (; !gave_up; ++i) {
-        const long long start = clock64();
-        while (!gave_up && smem->begun < i - kStItemsAhead) {
-          __nanosleep(64);
-          gave_up = smem->abort || clock64() - start > 2 * kWaitLimitCycles;
-        }
+        gave_up = !stream_wait_begun(smem, i - kStItemsAhead, status);
         if (walk.asks()) {
           walk.next = atomicAdd(sync + kStreamDownClaims, 1);
           walk.after = atomicAdd(sync + kStreamDownClaims, 1);

@@ -94,4 +94,24 @@ struct StreamDownWalk {
   GV_HD_MEMBER bool answered() const { return next >= 0 && after >= 0; }
 };
 
+// A bounded wait of a thread that others rely on: until ready(), with pause() between two looks.  It ends early where stopped(): somebody has given up, and
+// reported it.  Past the limit it gives up, and calls report(), but not without another look: the thread itself may be what was not running meanwhile.
+#ifdef __CUDACC__
+#pragma nv_exec_check_disable
+#endif
+template <class Ready, class Stopped, class Now, class Pause, class Report>
+GV_HD bool stream_wait(long long limit, Ready ready, Stopped stopped, Now now, Pause pause, Report report) {
+  const long long start = now();
+  for (;;) {
+    const bool late = now() - start > limit;
+    if (ready()) return true;
+    if (stopped()) return false;
+    if (late) {
+      report();
+      return false;
+    }
+    pause();
+  }
+}
+
 }  // namespace gv

@@ -25,6 +25,17 @@ def test_no_wait_on_a_cta_that_is_not_running(probe, chunks, ctas, running):
         assert result.stdout.strip() == "ok", (chunks, ctas, running, seed, result.stdout)
 
 
+def test_claim_warp_gives_up_only_what_is_not_there(tmp_path):
+    """A claim warp that gave up would leave w2 items out, which nobody waits for: it looks again before it does, and reports it."""
+    binary = str(tmp_path / "probe")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-o", binary, os.path.join(ROOT, "tests", "stream_wait_probe.cpp")], check=True)
+    assert subprocess.run([binary], capture_output=True, text=True).stdout.strip() == "ok"
+    with open(os.path.join(ROOT, "gevva_b200", "csrc", "experts_stream.cu")) as f:
+        text = f.read()
+    claims = text[text.index("---------------- claims") : text.index("---------------- publisher")]
+    assert "kWaitLimitCycles" not in claims  # its waits are that one
+
+
 def test_counts_have_arrived_when_a_cta_ends():
     """The CTA that finishes last puts the counters back to zero, so whatever another one adds has to have arrived before that one ends: every
     addition is one whose answer is waited for, none is sent off without (`red`, or an atomic whose result nothing uses)."""
