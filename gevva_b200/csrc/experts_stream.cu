@@ -133,7 +133,7 @@ struct alignas(1024) StreamSmem {
   volatile int published;                   // w13 items that the publisher has counted; kStAllPublished at its end
   volatile int first_mine;                  // whether the CTA's first w13 item is its to count; -1: not known yet
   volatile int begun;                       // items that the weight warp has begun
-  volatile uint32_t items[kStItems];        // the CTA's items: see stream_item
+  volatile uint32_t items[kStItems];        // the CTA's items: see stream_word
   uint32_t tmem_base;
   volatile int abort;
   volatile int left;  // an epilogue warp gave up waiting

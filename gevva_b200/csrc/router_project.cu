@@ -40,8 +40,8 @@ template <int kRows> constexpr int kRpThreads = (2 + kRpEpilogueWarps<kRows>) * 
 // each CTA has to send, reduce and route.  128 -> 64 rows, us alone: 9.7 -> 6.8 at 128 and 200 tokens, 10.2 -> 7.6 at 512, 10.2 -> 9.3 at 1024, 10.5 -> 9.7
 // at 2048; above, the clusters no longer run all at once (2368 tokens: 11.0 against 17.3).  64 -> 32 rows: 37 tokens 5.5 -> 5.2, 64 6.2 -> 5.4,
 // 200 6.4 -> 5.6, 400 6.7 -> 5.8, but 512, whose 16 clusters of eight do not run all at once, 6.7 -> 10.3.  32 -> 16 rows: 37 tokens 5.2 -> 4.9,
-// 64 5.4 -> 4.9, 128 5.4 -> 5.0; whole layers 37 tokens 69.6 -> 69.2 us, 64 75.3 -> 75.1, but 128 76.4 -> 76.6 (the fastest runs): the experts' CTAs
-// start late on the SMs of a router's CTAs, so that the line for 16 rows is drawn at 64 tokens.
+// 64 5.4 -> 4.9, 128 5.4 -> 5.0; whole layers 37 tokens 69.6 -> 69.2 us, 64 75.3 -> 75.1, 128 76.4 -> 76.6, each
+// hardly beyond its spread: with more tokens the experts' CTAs start late on the SMs of a router's CTAs, so 16 rows are taken up to 64 tokens only.
 // The K split, which decides the order of the sums, depends on the number of 128-row tiles either way.
 constexpr int kSmallTile = 64, kSmallTileTokens = 2048;
 constexpr int tile_rows(int tokens) { return tokens <= 64 ? 16 : tokens <= 400 ? 32 : tokens <= kSmallTileTokens ? kSmallTile : kTileM; }
@@ -305,17 +305,15 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       }
     }
     if constexpr (kOwnRows > kWarpRows<kRows>) if (!few) {
+    static_assert(kOwnRows % 32 == 0 && kWarps == 4, "128-row tiles: whole passes of 32 rows by all epilogue threads");
     const int t = threadIdx.x - 64;
     const int part = t & 3;         // columns [32 * part, 32 * part + 32)
 #pragma unroll 1
-    for (int pass = 0; pass < (kOwnRows + 31) / 32; ++pass) {
+    for (int pass = 0; pass < kOwnRows / 32; ++pass) {
       if (m_tile * kRows + pass * 32 * kSplit >= p.tokens) break;   // no row of this pass exists
-      // tile row kSplit * row_local + rank; where a CTA has 16 rows (64-row tiles, four owners) half of the
-      // threads only keep their quads company (they read row 15 again and store nothing)
-      const bool row_owned = pass * 32 + (t >> 2) < kOwnRows;
-      const int row_local = row_owned ? pass * 32 + (t >> 2) : kOwnRows - 1;
+      const int row_local = pass * 32 + (t >> 2);   // tile row kSplit * row_local + rank
       const int token = m_tile * kRows + row_local * kSplit + static_cast<int>(rank);
-      const bool valid = row_owned && token < p.tokens;
+      const bool valid = token < p.tokens;
       float4 acc[8];
 #pragma unroll
       for (int source = 0; source < kSplit; ++source) {

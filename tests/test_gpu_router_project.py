@@ -100,9 +100,9 @@ def test_fp8_router_projection(oracle, cuda_device, rows):
                                      (513, 2049), (577, 2049), (2048, 2049)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_router_tiles_of_few_rows(cuda_device, rows, of, fp8):
-    """64-row tiles, whose warps take up to eight rows each, at their edges: every row's logits, experts and
+    """Tiles of 16 rows (up to 64 tokens), 32 (up to 400) and 64 (up to 2048) at their edges: every row's logits, experts and
     weights are those of the same row in a batch of `of`, whose K range is split the same way (over eight CTAs up
-    to 512 tokens, over four above; a batch of 2049 has 128-row tiles)."""
+    to 512 tokens, over four above; a batch of 512 has 64-row tiles, one of 2049 128-row ones)."""
     import gevva_b200 as gm
     gen = torch.Generator().manual_seed(3000 + rows)
     x = torch.randn((of, HIDDEN), generator=gen).to(cuda_device)
