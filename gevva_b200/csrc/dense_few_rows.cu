@@ -18,6 +18,7 @@
 // experts the second launch starts when the first has ended: as a programmatic one its CTAs, waiting, would hold SMs of the experts' (and gain nothing: 24.4 so,
 // 24.75 with it).
 #include "gv_common.cuh"
+#include "gv_dense_rows.cuh"
 #include "gv_gemm_parts.cuh"
 #include "gv_launchers.h"
 
@@ -29,11 +30,10 @@ constexpr int kFwWarps = 11;                 // that quantise: 8 columns of a to
 constexpr int kFwRowThreads = kFwWarps * 32;
 constexpr int kFwWeightWarp = kFwWarps, kFwMmaWarp = kFwWarps + 1;
 constexpr int kFwThreads = kFwRowThreads + 64;
-constexpr int kFwDense = 2112;
 constexpr int kFwTokenBytes = 8 * kTileKBytes;  // a K block of the tokens: eight rows, the first one or two of which are tokens
 constexpr int kFwMmaBytes = 32;                 // K of an MMA
 constexpr int kFwMaxSmem = 232448;
-static_assert(kHidden == kFwRowThreads * 8 && kFwDense % kFwMmaBytes == 0 && kHidden % kFwMmaBytes == 0, "whole MMAs");
+static_assert(kHidden == kFwRowThreads * 8 && kDense % kFwMmaBytes == 0 && kHidden % kFwMmaBytes == 0, "whole MMAs");
 
 // kRows: weight rows of a CTA, MMA-N.
 template <int kTokens, int kK, int kRows>
@@ -166,24 +166,7 @@ __device__ __forceinline__ float few_scale(const Smem* smem, int token) {
   float maximum = smem->maxima[token][0];
 #pragma unroll
   for (int w = 1; w < kFwWarps; ++w) maximum = fmaxf(maximum, smem->maxima[token][w]);
-  return fmaxf(__fdiv_rn(maximum, 448.0f), 1.17549435e-38f);
-}
-
-__device__ __forceinline__ uint2 few_encode(const float* v, float inverse) {
-  uint32_t pairs[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    pairs[i] = __nv_cvt_float2_to_fp8x2(float2{__fmul_rn(v[2 * i], inverse), __fmul_rn(v[2 * i + 1], inverse)}, __NV_SATFINITE, __NV_E4M3);
-  return make_uint2(pairs[0] | pairs[1] << 16, pairs[2] | pairs[3] << 16);
-}
-
-__device__ __forceinline__ void few_unpack(const uint4& raw, float* v) {
-  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[2 * i] = __uint_as_float(words[i] << 16);
-    v[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000u);
-  }
+  return e4m3_row_scale(maximum);
 }
 
 // Maxima, scales and codes of the tokens, `raw` being the thread's eight columns of each, into shared memory; CTA 0 also keeps them in
@@ -194,7 +177,7 @@ __device__ __forceinline__ void few_quantise(Smem* smem, const uint4 (&raw)[kTok
 #pragma unroll
   for (int t = 0; t < kTokens; ++t) {
     float x[8], maximum = 0.0f;
-    few_unpack(raw[t], x);
+    unpack8(raw[t], x);
 #pragma unroll
     for (int i = 0; i < 8; ++i) maximum = fmaxf(maximum, fabsf(x[i]));
     few_maximum(smem, t, maximum);
@@ -204,9 +187,9 @@ __device__ __forceinline__ void few_quantise(Smem* smem, const uint4 (&raw)[kTok
 #pragma unroll
   for (int t = 0; t < kTokens; ++t) {
     float x[8];
-    few_unpack(raw[t], x);
+    unpack8(raw[t], x);
     const float scale = few_scale(smem, t);
-    const uint2 code = few_encode(x, __fdiv_rn(1.0f, scale));
+    const uint2 code = encode_e4m3x8(x, __fdiv_rn(1.0f, scale));
     few_store_codes(smem, t, thread, code);
     if (blockIdx.x == 0 && t < p.tokens) {
       reinterpret_cast<uint2*>(p.codes + static_cast<size_t>(t) * kK)[thread] = code;
@@ -271,12 +254,11 @@ dense_few_gate_up_kernel(const __grid_constant__ CUtensorMap map, const FewParam
     if (token < p.tokens) {
       const __nv_bfloat16 gate = __float2bfloat16_rn(__uint_as_float(gate_bits)), up = __float2bfloat16_rn(__uint_as_float(up_bits));
       const int column = column0 + unit * 16 + row;
-      p.out[static_cast<size_t>(token) * (2 * kFwDense) + column] = gate;
-      p.out[static_cast<size_t>(token) * (2 * kFwDense) + kFwDense + column] = up;
+      p.out[static_cast<size_t>(token) * (2 * kDense) + column] = gate;
+      p.out[static_cast<size_t>(token) * (2 * kDense) + kDense + column] = up;
       const float scale = few_scale(smem, token);
-      const float g = __bfloat162float(__float2bfloat16_rn(__fmul_rn(__bfloat162float(gate), __fmul_rn(scale, p.gate_w_scale))));
-      const float u = __bfloat162float(__float2bfloat16_rn(__fmul_rn(__bfloat162float(up), __fmul_rn(scale, p.up_w_scale))));
-      p.products[token * kFwDense + column] = __float2bfloat16_rn(__fmul_rn(gv_gelu_tanh(g), u));
+      p.products[token * kDense + column] =
+          __float2bfloat16_rn(geglu_tanh(__bfloat162float(gate), __bfloat162float(up), __fmul_rn(scale, p.gate_w_scale), __fmul_rn(scale, p.up_w_scale)));
     }
   }
   few_end<kRows>(smem, tmem_acc);
@@ -286,7 +268,7 @@ dense_few_gate_up_kernel(const __grid_constant__ CUtensorMap map, const FewParam
 template <int kTokens, int kRows>
 __global__ void __launch_bounds__(kFwThreads, 1)
 dense_few_down_kernel(const __grid_constant__ CUtensorMap map, const FewParams p) {
-  using Smem = FewSmem<kTokens, kFwDense, kRows>;
+  using Smem = FewSmem<kTokens, kDense, kRows>;
   static_assert(Smem::kStages == Smem::kBlocks, "every block has a place");
   extern __shared__ uint8_t smem_raw[];
   Smem* smem = reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -309,15 +291,15 @@ dense_few_down_kernel(const __grid_constant__ CUtensorMap map, const FewParams p
     uint4 raw[kTokens];
 #pragma unroll
     for (int t = 0; t < kTokens; ++t)
-      raw[t] = threadIdx.x < kFwDense / 8 && t < p.tokens ? reinterpret_cast<const uint4*>(p.input + t * kFwDense)[threadIdx.x] : uint4{};
-    few_quantise<kTokens, kFwDense>(smem, raw, p);
+      raw[t] = threadIdx.x < kDense / 8 && t < p.tokens ? reinterpret_cast<const uint4*>(p.input + t * kDense)[threadIdx.x] : uint4{};
+    few_quantise<kTokens, kDense>(smem, raw, p);
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_acc = smem->tmem_base;
   if (warp == kFwMmaWarp) {
-    if (elect_one()) few_multiply<kFwDense, kRows>(smem, tmem_acc, p.status);
+    if (elect_one()) few_multiply<kDense, kRows>(smem, tmem_acc, p.status);
     __syncwarp();
   } else if ((warp & 3) == 0 && warp < kFwWarps && warp / 4 < kRows / 16 && few_sums_there(smem, p.status)) {
     constexpr int kEpilogueWarps = (kFwWarps + 3) / 4;
@@ -345,10 +327,10 @@ dense_few_down_kernel(const __grid_constant__ CUtensorMap map, const FewParams p
 
 static_assert(kDenseFewTokens == 2, "variants");
 constexpr int kFwUnits = kDenseFewUpRows / 16;
-static_assert(kDenseFewUpRows % 16 == 0 && kFwDense % kDenseFewUpRows == 0 && kHidden % kDenseFewDownRows == 0, "whole CTAs");
+static_assert(kDenseFewUpRows % 16 == 0 && kDense % kDenseFewUpRows == 0 && kHidden % kDenseFewDownRows == 0, "whole CTAs");
 
 template <int kTokens> constexpr size_t few_up_bytes() { return few_smem_bytes<kTokens, kHidden, 2 * kDenseFewUpRows>(); }
-template <int kTokens> constexpr size_t few_down_bytes() { return few_smem_bytes<kTokens, kFwDense, kDenseFewDownRows>(); }
+template <int kTokens> constexpr size_t few_down_bytes() { return few_smem_bytes<kTokens, kDense, kDenseFewDownRows>(); }
 static_assert(few_up_bytes<kDenseFewTokens>() <= kFwMaxSmem && few_down_bytes<kDenseFewTokens>() <= kFwMaxSmem, "shared memory of a CTA");
 
 template <int kTokens>
@@ -372,7 +354,7 @@ void launch(const DenseFewOperands& op, int tokens, cudaStream_t stream) {
   up.gate_w_scale = op.gate_scale;
   up.up_w_scale = op.up_scale;
   up.tokens = tokens;
-  launch_chained(dense_few_gate_up_kernel<kTokens, kFwUnits>, dim3(kFwDense / kDenseFewUpRows), dim3(kFwThreads), few_up_bytes<kTokens>(), stream,
+  launch_chained(dense_few_gate_up_kernel<kTokens, kFwUnits>, dim3(kDense / kDenseFewUpRows), dim3(kFwThreads), few_up_bytes<kTokens>(), stream,
                  *op.map_gate_up, up);
   FewParams down{};
   down.input = up.products;

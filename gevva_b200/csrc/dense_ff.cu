@@ -14,6 +14,7 @@
 // are folded in one fixed order (thread, shuffle-down tree, warps in order) and the
 // reciprocal square root is IEEE, so a CPU can reproduce every bit.
 #include "gv_common.cuh"
+#include "gv_dense_rows.cuh"
 #include "gv_exact.h"
 #include "gv_launchers.h"
 #include "gv_plan.cuh"
@@ -23,19 +24,7 @@ namespace gv {
 namespace {
 
 constexpr int kRowThreads = kHidden / 8;  // 352
-constexpr int kDense = 2112;
 constexpr int kDenseThreads = 288;        // 264 active threads x 8 columns
-
-__device__ __forceinline__ void unpack8(const uint4& raw, float* out) {
-  out[0] = __uint_as_float(raw.x << 16);
-  out[1] = __uint_as_float(raw.x & 0xffff0000u);
-  out[2] = __uint_as_float(raw.y << 16);
-  out[3] = __uint_as_float(raw.y & 0xffff0000u);
-  out[4] = __uint_as_float(raw.z << 16);
-  out[5] = __uint_as_float(raw.z & 0xffff0000u);
-  out[6] = __uint_as_float(raw.w << 16);
-  out[7] = __uint_as_float(raw.w & 0xffff0000u);
-}
 
 __device__ __forceinline__ uint4 pack8(const float* v) {
   uint4 out;
@@ -45,10 +34,6 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   p = __floats2bfloat162_rn(v[4], v[5]); out.z = *reinterpret_cast<uint32_t*>(&p);
   p = __floats2bfloat162_rn(v[6], v[7]); out.w = *reinterpret_cast<uint32_t*>(&p);
   return out;
-}
-
-__device__ __forceinline__ float bf16_round(float v) {
-  return __bfloat162float(__float2bfloat16_rn(v));
 }
 
 // A thread's sum of squares of its 8 values, then the warp's in lane 0, by a shuffle-down tree (lanes beyond the
@@ -160,16 +145,6 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
   return total;
 }
 
-// Two values a conversion: half the instructions of one at a time, the same bytes.
-__device__ __forceinline__ uint2 encode_e4m3x8(const float* v, float inverse) {
-  uint32_t pairs[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    pairs[i] = __nv_cvt_float2_to_fp8x2(float2{__fmul_rn(v[2 * i], inverse), __fmul_rn(v[2 * i + 1], inverse)}, __NV_SATFINITE,
-                                        __NV_E4M3);
-  return make_uint2(pairs[0] | pairs[1] << 16, pairs[2] | pairs[3] << 16);
-}
-
 // Larger of a and |b|, two bf16 numbers a word.  A NaN counts as nothing, as in fmaxf.
 __device__ __forceinline__ uint32_t abs_max_pair(uint32_t a, uint32_t b) {
   const uint32_t magnitude = b & 0x7fff7fffu;
@@ -193,7 +168,7 @@ fp8_quantize_rows_kernel(const __nv_bfloat16* __restrict__ input, uint8_t* __res
 #pragma unroll
   for (int i = 0; i < 8; ++i) maximum = fmaxf(maximum, fabsf(x[i]));
   maximum = block_max<kRowWarps>(maximum, scratch);
-  const float scale = fmaxf(__fdiv_rn(maximum, 448.0f), 1.17549435e-38f);
+  const float scale = e4m3_row_scale(maximum);
   if (threadIdx.x == 0) scales[blockIdx.x] = scale;
   const float inverse = __fdiv_rn(1.0f, scale);
   reinterpret_cast<uint2*>(out + base)[threadIdx.x] = encode_e4m3x8(x, inverse);
@@ -226,7 +201,7 @@ fp8_quantize_warp_rows_kernel(const __nv_bfloat16* __restrict__ input, uint8_t* 
   float maximum = fmaxf(__uint_as_float(maxima << 16), __uint_as_float(maxima & 0xffff0000u));
 #pragma unroll
   for (int offset = 16; offset; offset >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
-  const float scale = fmaxf(__fdiv_rn(maximum, 448.0f), 1.17549435e-38f);
+  const float scale = e4m3_row_scale(maximum);
   if (lane == 0) scales[row] = scale;
   const float inverse = __fdiv_rn(1.0f, scale);
 #pragma unroll
@@ -257,14 +232,12 @@ gelu_quantize_fp8_kernel(const __nv_bfloat16* __restrict__ gate_up,
     unpack8(__ldg(src + kDense / 8 + threadIdx.x), u);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float gv = bf16_round(__fmul_rn(g[i], gate_scale));
-      const float uv = bf16_round(__fmul_rn(u[i], up_scale));
-      value[i] = bf16_round(__fmul_rn(gv_gelu_tanh(gv), uv));
+      value[i] = geglu_tanh(g[i], u[i], gate_scale, up_scale);
       maximum = fmaxf(maximum, fabsf(value[i]));
     }
   }
   maximum = block_max<kDenseThreads / 32>(maximum, scratch);
-  const float scale = fmaxf(__fdiv_rn(maximum, 448.0f), 1.17549435e-38f);
+  const float scale = e4m3_row_scale(maximum);
   if (threadIdx.x == 0) scales[row] = scale;
   const float inverse = __fdiv_rn(1.0f, scale);
   if (active)
@@ -353,7 +326,7 @@ gelu_table_quantize_fp8_kernel(const __nv_bfloat16* __restrict__ gate_up, const 
     float maximum = fmaxf(__uint_as_float(maxima << 16), __uint_as_float(maxima & 0xffff0000u));
 #pragma unroll
     for (int offset = 16; offset; offset >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
-    const float scale = fmaxf(__fdiv_rn(maximum, 448.0f), 1.17549435e-38f);
+    const float scale = e4m3_row_scale(maximum);
     if (lane == 0) scales[row] = scale;
     const float inverse = __fdiv_rn(1.0f, scale);
     uint2* dst = reinterpret_cast<uint2*>(out + static_cast<size_t>(row) * kDense) + lane;
@@ -471,7 +444,7 @@ __global__ void fp8_amax_kernel(const float* __restrict__ w, size_t count, unsig
 
 __global__ void fp8_pack_kernel(const float* __restrict__ w, size_t count, const unsigned int* amax_bits,
                                 uint8_t* __restrict__ out, float* __restrict__ scale_out) {
-  const float scale = fmaxf(__fdiv_rn(__uint_as_float(*amax_bits), 448.0f), 1.17549435e-38f);
+  const float scale = e4m3_row_scale(__uint_as_float(*amax_bits));
   if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
        i += static_cast<size_t>(gridDim.x) * blockDim.x)
