@@ -94,7 +94,7 @@ __device__ __forceinline__ void few_fetch(Smem* smem, int first, int last, int* 
 #pragma unroll 1
   for (int kb = first; kb < last; ++kb) {
     const int stage = kb % Smem::kStages;
-    if (kb >= Smem::kStages && !wait_or_abort<true>(&smem->empty[stage], (kb / Smem::kStages - 1) & 1, smem, status)) return;
+    if (kb >= Smem::kStages && !wait_or_abort(&smem->empty[stage], (kb / Smem::kStages - 1) & 1, smem, status)) return;
     mbar_arrive_expect_tx(&smem->full[stage], Smem::kWeightBytes);
     load(smem->w[stage], &smem->full[stage], kb * kTileKBytes);
   }
@@ -111,7 +111,7 @@ __device__ __forceinline__ void few_multiply(Smem* smem, uint32_t tmem_acc, int*
 #pragma unroll 1
   for (int kb = 0; kb < Smem::kBlocks; ++kb) {
     const int stage = kb % Smem::kStages;
-    if (!wait_or_abort<false>(&smem->full[stage], kb / Smem::kStages & 1, smem, status)) {
+    if (!wait_or_abort(&smem->full[stage], kb / Smem::kStages & 1, smem, status)) {
       // what was asked for lands, and what was issued ends, before shared memory is given up
       for (int b = kb; b < kb + Smem::kStages && b < Smem::kBlocks; ++b)
         mbar_wait_bounded(&smem->full[b % Smem::kStages], b / Smem::kStages & 1, 40000000ll);
@@ -131,7 +131,7 @@ __device__ __forceinline__ void few_multiply(Smem* smem, uint32_t tmem_acc, int*
 // Whether the sums are there, by a warp of the epilogue.
 template <class Smem>
 __device__ __forceinline__ bool few_sums_there(Smem* smem, int* status) {
-  const bool there = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full, 0, smem, status)) && !smem->abort;
+  const bool there = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_full, 0, smem, status)) && !smem->abort;
   tc_fence_after_sync();
   return __all_sync(0xffffffffu, there);
 }

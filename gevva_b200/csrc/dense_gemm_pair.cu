@@ -131,7 +131,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         const int piece0 = static_cast<int>(rank) * item.pieces, group0 = item.column0 / 64;
 #pragma unroll kFpUnroll
         for (int kb = 0; kb < p.k_blocks; ++kb) {
-          ok = wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status);
+          ok = wait_or_abort(&smem->empty[stage], phase ^ 1u, smem, p.status);
           if (!ok) break;
           const uint32_t bar = full0 + 8 * stage;
           if (is_leader) mbar_arrive_expect_tx(&smem->full[stage], both_bytes);
@@ -173,7 +173,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       uint32_t phase = 0, acc_phase = 0;
       bool landed = false;  // the next stage's bytes have been seen
       for (int round = 0; ok && dense_pair_item<kN>(p, round, rank, item); ++round) {
-        ok = wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status);
+        ok = wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status);
         if (!ok) break;
         tc_fence_after_sync();
         // fp32 accumulation (bit 4), E4M3 x E4M3, both K-major; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
@@ -181,7 +181,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc) * kN;
 #pragma unroll kFpUnroll
         for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!landed) ok = wait_or_abort<false>(&smem->full[stage], phase, smem, p.status);
+          if (!landed) ok = wait_or_abort(&smem->full[stage], phase, smem, p.status);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t a = a_lo0 + static_cast<uint32_t>(stage) * (kFpTokenBytes >> 4);
@@ -214,7 +214,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int round = 0; ok && dense_pair_item<kN>(p, round, rank, item); ++round) {
-      ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, p.status));
+      ok = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc], acc_phase, smem, p.status));
       if (!ok) break;
       tc_fence_after_sync();
       const int groups = item.pieces;                                        // of 64 columns

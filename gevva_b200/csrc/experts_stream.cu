@@ -781,7 +781,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
     }
     if (self_first && kb >= kStStages && kb < kStUpKBlocks) {
       // the stage's second use
-      if (__all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[kb - kStStages], 0u, smem, status)))
+      if (__all_sync(0xffffffffu, wait_or_abort(&smem->empty[kb - kStStages], 0u, smem, status)))
         stream_quantise_stage(input, smem, kb - kStStages, kb, first_rows, tokens, false, first % kTileM, multiplier, lane, false);
     }
   }
@@ -830,7 +830,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
         // One K block.  The loops around it are unrolled because a trip of a rolled one takes 320 cycles, whatever it loads (the
         // back edge waits until the copy has read its operands); unrolled it is as fast as 128 rows arrive from L2, 226 cycles.
         const auto load = [&](int kb, uint32_t sf_bytes) {
-          ok = wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, status);
+          ok = wait_or_abort(&smem->empty[stage], phase ^ 1u, smem, status);
           if (!ok) return false;
           const int x = kb * kTileKBytes;
           uint64_t* bar = &smem->full[stage];
@@ -920,11 +920,11 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
         const uint32_t descriptor = (1u << 7) | (1u << 10) | (static_cast<uint32_t>((rows + 15) / 16 * 2) << 17) |
                                     (static_cast<uint32_t>(kTileM >> 4) << 24);
         const uint32_t half = (first % kTileM) / 32;
-        if (!wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, status)) break;
+        if (!wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, status)) break;
         const uint32_t d = tmem_base + static_cast<uint32_t>(acc) * kStRows;
         // One K block, unrolled for the producers' reason.
         const auto multiply = [&](int kb, auto mmas, bool last) {
-          if (!landed) ok = wait_or_abort<false>(&smem->full[stage], phase, smem, status);
+          if (!landed) ok = wait_or_abort(&smem->full[stage], phase, smem, status);
           if (!ok) return false;
           tc_fence_after_sync();
           const uint32_t sf = tmem_base + kStSfColumn + kStSfColumnsPerStage * stage;
@@ -1078,7 +1078,7 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
       rows = rows > kStRows ? kStRows : rows;
       const float alpha = it.down ? p.alpha2[it.expert] : p.alpha1[it.expert];
       const float multiplier = it.down ? 0.0f : p.in_scale_q2[it.expert];
-      const bool ready = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, status));
+      const bool ready = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc], acc_phase, smem, status));
       uint32_t r[4][8];
       if (ready) {
         tc_fence_after_sync();

@@ -245,7 +245,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         sf_src = p.b_scales + static_cast<size_t>(row) * p.groups;
       }
       for (int kb = 0; kb < p.k_blocks; kb += kAtoms) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->empty[stage], phase ^ 1u, smem, p.status));
         if (!ok) break;
         if (elect_one()) {
           const int atoms = p.k_blocks - kb < kAtoms ? p.k_blocks - kb : kAtoms;
@@ -337,7 +337,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       WorkItem item;
       if (!work_item<kMode, kN>(round, total_items, m_tiles, p.n_tiles, tile_first, item)) continue;
       if (!__all_sync(0xffffffffu,
-                      wait_or_abort<false>(&smem->acc_empty[acc_stage], acc_phase ^ 1u, smem, p.status)))
+                      wait_or_abort(&smem->acc_empty[acc_stage], acc_phase ^ 1u, smem, p.status)))
         break;
       const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc_stage * kN);
       const bool half_item = kMode == kGeglu ? item.n_tile == p.n_tiles - 1 : kWide && (item.n_tile + 1) * kN > p.n_out;
@@ -350,7 +350,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         // the barrier's transaction count is what orders the two, no tcgen05 fence is needed.
         // With block scales the stage is ready once the copier's scale copies have landed in
         // tensor memory (which implies that the operands have landed in shared memory).
-        ok = wait_or_abort<false>(kMode == kFp8 ? &smem->full[stage] : &smem->sf_full[stage], phase, smem, p.status);
+        ok = wait_or_abort(kMode == kFp8 ? &smem->full[stage] : &smem->sf_full[stage], phase, smem, p.status);
         if (!ok) break;
         if (kMode != kFp8) tc_fence_after_sync();
         // Descriptor low words advance by whole stages and K atoms; the K offset of each MMA
@@ -419,7 +419,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         if (!work_item<kMode, kN>(round, total_items, m_tiles, p.n_tiles, tile_first, item)) continue;
         const bool half_item = kMode == kGeglu && item.n_tile == p.n_tiles - 1;
         for (int kb = 0; kb < p.k_blocks; kb += kAtoms) {
-          ok = wait_or_abort<false>(&smem->full[stage], phase, smem, p.status);
+          ok = wait_or_abort(&smem->full[stage], phase, smem, p.status);
           if (!ok) break;
           const uint32_t sfa_lo = sfa_lo0 + static_cast<uint32_t>(stage) * (kAtoms * kSfStageBytes >> 4);
           const uint32_t sfb_lo = sfb_lo0 + static_cast<uint32_t>(stage) * (kAtoms * Shape::kWeightSfBytes >> 4);
@@ -466,7 +466,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const int row0 = p.expert_offsets[expert] + local0;
       const int rows_valid = p.expert_offsets[expert + 1] - row0;  // may exceed 128
       const float alpha = p.alpha[expert];
-      const bool acc_ready = wait_or_abort<true>(&smem->acc_full[acc_stage], acc_phase, smem, p.status);
+      const bool acc_ready = wait_or_abort(&smem->acc_full[acc_stage], acc_phase, smem, p.status);
       if constexpr (kMode != kGeglu) {
         // The four warps of a quarter meet at named barriers while they store, so they must
         // leave together: a warp whose wait failed says so, and all four read the answer behind

@@ -199,7 +199,7 @@ grouped_down_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       for (int n = unit.begin; ok && n < unit.end; ++n) {
         const uint8_t* sf = p.b_scales + static_cast<size_t>(unit.expert * kDnTiles + n) * (kDnKBlocks * kDnWeightSfBytes);
         for (int kb = 0; kb < kDnKBlocks; ++kb) {
-          ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->b_empty[stage], phase ^ 1u, smem, p.status));
+          ok = __all_sync(0xffffffffu, wait_or_abort(&smem->b_empty[stage], phase ^ 1u, smem, p.status));
           if (!ok) break;
           if (elect_one()) {
             mbar_arrive_expect_tx(&smem->b_full[stage], kDnWeightBytes + kDnWeightSfBytes);
@@ -235,7 +235,7 @@ grouped_down_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int row = p.expert_offsets[unit.expert] + unit.tile * kTileM - p.scale_row_offsets[unit.expert];
       const uint8_t* sf = p.a_scales + static_cast<size_t>(unit.tile) * (kDnAtoms * kSfAtomBytes);
       for (int kb = 0; kb < kDnKBlocks; ++kb) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->a_empty[slot], phase ^ 1u, smem, p.status));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->a_empty[slot], phase ^ 1u, smem, p.status));
         if (!ok) break;
         if (elect_one()) {
           const uint32_t sf_bytes = static_cast<uint32_t>(kb + 1 == kDnKBlocks ? kDnLastMmas : 4) * kSfAtomBytes;
@@ -273,7 +273,7 @@ grouped_down_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint32_t phase = 0, acc_phase = 0, slot0_phase = 0;
     while (ok && schedule.next(unit)) {
       for (int n = unit.begin; ok && n < unit.end; ++n) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status));
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t descriptor = n + 1 == kDnTiles ? kInstrDesc<kDnLastColumns> : kInstrDesc<kDnColumns>;
@@ -283,8 +283,8 @@ grouped_down_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           constexpr int kMmas[kDnKBlocks] = {4, 4, kDnLastMmas};
           const int slot = slot0 + kb < kDnSlots ? slot0 + kb : slot0 + kb - kDnSlots;
           if (n == unit.begin)
-            ok = wait_or_abort<false>(&smem->a_full[slot], slot < slot0 ? slot0_phase ^ 1u : slot0_phase, smem, p.status);
-          if (ok) ok = wait_or_abort<false>(&smem->b_full[stage], phase, smem, p.status);
+            ok = wait_or_abort(&smem->a_full[slot], slot < slot0 ? slot0_phase ^ 1u : slot0_phase, smem, p.status);
+          if (ok) ok = wait_or_abort(&smem->b_full[stage], phase, smem, p.status);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           if (leader) {
@@ -344,7 +344,7 @@ grouped_down_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int row_end = p.expert_offsets[unit.expert + 1];
       const float alpha = p.alpha[unit.expert];
       for (int n = unit.begin; n < unit.end; ++n) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, p.status));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc], acc_phase, smem, p.status));
         if (!ok) break;
         tc_fence_after_sync();
         const int groups = n + 1 == kDnTiles ? kDnLastColumns / 64 : kDnColumns / 64;

@@ -196,7 +196,7 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const int sf_row = (unit.expert * kDpTiles + n) * kDpKBlocks * 8;
 #pragma unroll
           for (int kb = 0; kb < kDpKBlocks; ++kb) {
-            ok = wait_or_abort<true>(&smem->b_empty[stage], phase ^ 1u, smem, p.status);
+            ok = wait_or_abort(&smem->b_empty[stage], phase ^ 1u, smem, p.status);
             if (!ok) break;
             const uint32_t bar = full0 + 8 * stage;
             if (is_leader)
@@ -239,7 +239,7 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       while (ok && schedule.next(rank, unit)) {
 #pragma unroll
         for (int kb = 0; kb < kDpKBlocks; ++kb) {
-          ok = wait_or_abort<true>(&smem->a_empty[slot], phase ^ 1u, smem, p.status);
+          ok = wait_or_abort(&smem->a_empty[slot], phase ^ 1u, smem, p.status);
           if (!ok) break;
           const uint32_t bar = full0 + 8 * slot;
           if (is_leader) mbar_arrive_expect_tx(&smem->a_full[slot], (unit.both ? 2u : 1u) * (kDpTokenBytes + kSfStageBytes));
@@ -280,7 +280,7 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       bool landed = false;  // the next stage's bytes have been seen
       while (ok && schedule.next(rank, unit)) {
         for (int n = unit.begin; ok && n < unit.begin + kDpUnitTiles; ++n) {
-          ok = wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status);
+          ok = wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status);
           if (!ok) break;
           tc_fence_after_sync();
           // E2M1 x E2M1, both K-major, UE4M3 scales; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
@@ -291,8 +291,8 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           for (int kb = 0; kb < kDpKBlocks; ++kb) {
             constexpr int kMmas[kDpKBlocks] = {4, 4, kDpLastMmas};
             const int slot = slot0 + kb;  // units start at slot 0 or 3
-            if (n == unit.begin) ok = wait_or_abort<false>(&smem->a_full[slot], slot0_phase, smem, p.status);
-            if (ok && !landed) ok = wait_or_abort<false>(&smem->b_full[stage], phase, smem, p.status);
+            if (n == unit.begin) ok = wait_or_abort(&smem->a_full[slot], slot0_phase, smem, p.status);
+            if (ok && !landed) ok = wait_or_abort(&smem->b_full[stage], phase, smem, p.status);
             if (!ok) break;
             tc_fence_after_sync();
             const uint32_t tmem_sfa = tmem_base + kDpSfaColumn + static_cast<uint32_t>(16 * kb);
@@ -352,7 +352,7 @@ grouped_down_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const float alpha = p.alpha[unit.expert];
       const int warp_rows = unit.rows - quarter * 32;  // of this warp's quarter that exist
       for (int n = unit.begin; n < unit.begin + kDpUnitTiles; ++n) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, p.status));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc], acc_phase, smem, p.status));
         if (!ok) break;
         tc_fence_after_sync();
         const int groups = n + 1 == kDpTiles ? kDpLastColumns / 64 : kDpColumns / 64;

@@ -271,7 +271,7 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
         both_bytes = 2 * my_bytes;
       }
       for (int kb = 0; kb < p.k_blocks; ++kb) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->empty[stage], phase ^ 1u, smem, p.status));
         if (!ok) break;
         if (elect_one()) {
           const int x = kb * kTileKBytes;
@@ -332,12 +332,12 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
       for (int round = 0; round < rounds; ++round) {
         PairItem item;
         if (!pair_item(round, total_items, p.n_tiles, pair_begin, pair_tile, rank, item)) continue;
-        if (!__all_sync(0xffffffffu, wait_or_abort<false>(&smem->acc_empty, acc_phase ^ 1u, smem, p.status))) break;
+        if (!__all_sync(0xffffffffu, wait_or_abort(&smem->acc_empty, acc_phase ^ 1u, smem, p.status))) break;
         acc_phase ^= 1u;
         bool ok = true;
         tc_fence_after_sync();
         for (int kb = 0; kb < p.k_blocks; ++kb) {
-          ok = wait_or_abort<false>(&smem->full[stage], phase, smem, p.status);
+          ok = wait_or_abort(&smem->full[stage], phase, smem, p.status);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t a_lo = a_lo0 + static_cast<uint32_t>(stage) * (kPairTileBytes >> 4);
@@ -391,7 +391,7 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
         rows_valid = p.expert_offsets[expert + 1] - row0;  // may exceed 128
         alpha = p.alpha[expert];
       }
-      const bool acc_ready = wait_or_abort<true>(&smem->acc_full, acc_phase, smem, p.status);
+      const bool acc_ready = wait_or_abort(&smem->acc_full, acc_phase, smem, p.status);
       acc_phase ^= 1u;
       if constexpr (kMode != kGeglu) {
         if (!acc_ready) smem->quarter_left[quarter] = 1;

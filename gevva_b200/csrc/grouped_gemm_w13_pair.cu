@@ -267,7 +267,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
       const CUtensorMap* token_map = &map_x.rows[(half >> 3) - 1];
       const int w_sf_row = ((item.expert * kWpUnitSlots + unit) * k_blocks) * 4;
       for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->empty[stage], phase ^ 1u, smem, p.status));
         if (!ok) break;
         if (elect_one()) {
           const int x = kb * kTileKBytes;
@@ -323,12 +323,12 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
         // E2M1 x E2M1, both K-major, UE4M3 scales; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
         const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(item.n >> 3) << 17) |
                                (static_cast<uint32_t>(256 >> 4) << 24);
-        if (!__all_sync(0xffffffffu, wait_or_abort<false>(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status))) break;
+        if (!__all_sync(0xffffffffu, wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status))) break;
         const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc) * kWpRows;
         bool ok = true;
         tc_fence_after_sync();
         for (int kb = 0; kb < k_blocks; ++kb) {
-          ok = wait_or_abort<false>(&smem->full[stage], phase, smem, p.status);
+          ok = wait_or_abort(&smem->full[stage], phase, smem, p.status);
           if (!ok) break;
           tc_fence_after_sync();
           if (leader_lane) {
@@ -382,7 +382,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
       const int steps = unit < kWpUnits ? (item.valid + 31) >> 5 : 0;  // of 32 tokens, dealt to the two warps of a block
       const float alpha = p.alpha[item.expert];
       const float multiplier = p.next_scale_q[item.expert];
-      if (!__all_sync(0xffffffffu, wait_or_abort<true>(&smem->acc_full[acc], acc_phase, smem, p.status))) break;
+      if (!__all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc], acc_phase, smem, p.status))) break;
       tc_fence_after_sync();
       const uint32_t tmem_rows = tmem_base + (static_cast<uint32_t>(block * 32) << 16) + static_cast<uint32_t>(acc) * kWpRows;
       uint8_t* const scales = p.next_scales + static_cast<size_t>(smem->scale_rows[item.expert]) * groups;

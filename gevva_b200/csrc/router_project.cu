@@ -183,7 +183,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     int issued = 0;
     bool ok = true;
     for (int kb = kb_begin; kb < kb_end; ++kb) {
-      ok = __all_sync(0xffffffffu, wait_or_abort<true>(&smem->empty[stage], phase ^ 1u, smem, p.status));
+      ok = __all_sync(0xffffffffu, wait_or_abort(&smem->empty[stage], phase ^ 1u, smem, p.status));
       if (!ok) break;
       if (elect_one()) {
         mbar_arrive_expect_tx(&smem->full[stage], static_cast<uint32_t>(Smem::kTokenBytes + kRpTileBytes));
@@ -218,7 +218,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const uint32_t b_lo0 = (smem_u32(smem->b[0]) & 0x3ffffu) >> 4;
     const bool leader = elect_one();
     for (int kb = kb_begin; kb < kb_end; ++kb) {
-      if (!wait_or_abort<false>(&smem->full[stage], phase, smem, p.status)) break;
+      if (!wait_or_abort(&smem->full[stage], phase, smem, p.status)) break;
       if (leader) {
         issue_router_k_block<kFp8>(tmem_base, a_lo0 + static_cast<uint32_t>(stage) * (Smem::kTokenBytes >> 4),
                                    b_lo0 + static_cast<uint32_t>(stage) * (kRpTileBytes >> 4),
@@ -245,7 +245,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     // tensor-memory loads are warp-wide, so a warp takes part if any of its 32 rows exists
     const bool row_exists = row < kRows && m_tile * kRows + row < p.tokens;
     const bool warp_has_rows = quarter * 32 < kRows && m_tile * kRows + quarter * 32 < p.tokens;
-    if (wait_or_abort<true>(&smem->acc_full, 0, smem, p.status) && warp_has_rows) {
+    if (wait_or_abort(&smem->acc_full, 0, smem, p.status) && warp_has_rows) {
       tc_fence_after_sync();
       const uint32_t remote_row =
           cluster_map_shared(smem_u32(smem->received + (rank * kOwnRows + owner_row) * kExperts),
