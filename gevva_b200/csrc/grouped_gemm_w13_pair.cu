@@ -2,15 +2,18 @@
 //
 // What bounds it.  One K block of 256 elements of a 128 x 256 tile costs 512 tensor-pipe cycles, but in the
 // one-CTA kernel (grouped_gemm.cu) shared memory has to take in 54 KiB and give the MMAs 48 KiB for it: 800
-// cycles.  Here a CTA pair (tcgen05 cta_group::2, M = 256) holds 256 weight rows, 128 per CTA, against up to 208
-// token rows of one expert on the N side, half of them loaded by each CTA: at most 35 KiB in and 29 out.  And because
+// cycles.  Here a CTA pair (tcgen05 cta_group::2, M = 256) holds 256 weight rows, 128 per CTA, against up to 256
+// token rows of one expert on the N side, half of them loaded by each CTA: at most 38 KiB in and 38 out, scales included.  And because
 // the tokens sit on N, which may be any multiple of 16, a group of 200 rows is one item and not two 128-row tiles.
-// An item is 44 MMAs and their scale copies. The tensor pipe takes N / 2 cycles an MMA from 128 rows on (39 to 64 below), issuing it
-// and its share of the copies about 105: 5345 cycles with neither loads nor epilogue and 6600 in all (4096 tokens).  Beside large batches the clock drops to 1.5 GHz under the power limit.
-// Alone (us, one-CTA kernel -> this one; uniform routing): 53.1 -> 53.2 at 1024 tokens, 63.9 -> 58.9 at 2048,
+// An item is 11 K blocks, each of four MMAs of N / 2 tensor cycles (39 at least) and eight or twelve scale copies.  Issuing those takes one
+// thread some 300 cycles a K block, and beside the epilogue's warps on its scheduler more, so a narrow item costs nearly what one of
+// 170 rows does: chunks are as wide as the MMA allows.  Chunks of 208 rows and a loop of the whole warp -> this (us, alone): 4096 tokens 96.5 -> 88.2,
+// of uneven loads 94.2 -> 87.4, 16384 290 -> 269; a whole layer of 700 tokens 109.5 -> 108.5, 4096 254 -> 245, 16384 795 -> 770.
+// Beside large batches the clock drops to 1.35 GHz under the power limit (this kernel repeated for seconds at 4096 tokens).
+// Alone (us, one-CTA kernel -> the first form of this one; uniform routing): 53.1 -> 53.2 at 1024 tokens, 63.9 -> 58.9 at 2048,
 // 83.5 -> 70 at 3000, 97 -> 95 at 4096, 172 -> 151 at 8192, 330 -> 293 at 16384.
 //
-// Work.  A chunk is up to 208 consecutive rows of an expert; one with more is cut into stretches of 192, so that a
+// Work.  A chunk is up to 256 consecutive rows of an expert; one with more is cut into as few chunks as that takes, of 192 or 256 rows but for the last, so that a
 // chunk's scales start at a 64-row boundary of their 128-row blocks.  The intermediate width 704 is cut into 11 units
 // of 64 columns; a CTA computes one unit as 128 MMA rows, the unit's up and gate rows interleaved so that a thread
 // of the epilogue finds both of a column in its registers (see there; the order costs nothing: it is a
@@ -18,12 +21,14 @@
 // item is (chunk, two units); the second CTA of the sixth item has no unit (its weight scales are zero and its
 // results are dropped).
 //
-// Protocol.  Two TMA producers in each CTA (weight side, token side) fill a ring of six stages,
+// Protocol.  Two TMA producers in each CTA (weight side, token side) fill a ring of six stages (where some chunk has more than 208 rows,
+// the tokens' has five: 227 KB of shared memory hold no more),
 // all loads of both CTAs complete on the `full` barrier of the first CTA (tensor-map loads in
 // their cta_group::2 form, no multicast; the scale atoms travel through tensor maps too).  There
 // the MMA thread copies the scale atoms of a landed stage into tensor memory, issues four MMAs
 // (copies and MMAs of one thread execute in order) and commits to `empty` of both CTAs.  Two accumulators, so that the
-// eight epilogue warps of each CTA work on one item while the next is computed.  (With the accumulator transposed
+// eight epilogue warps of each CTA work on one item while the next is computed; two of 256 columns do not fit beside the scales, so they have 48 in common,
+// which the epilogue reads first and releases by themselves (an item waits for that where the two would meet).  The items of a pair are worked out once, by all threads.  (With the accumulator transposed
 // through shared memory by sixteen warps that traffic bounded the kernel, 107 us at 4096 tokens; with this epilogue
 // twelve or sixteen warps are 3 to 8 % slower than eight, and five stages up to 8 % slower than six.)  Every wait is bounded.
 #include "gv_common.cuh"
@@ -35,37 +40,48 @@ namespace gv {
 
 namespace {
 
-constexpr int kWpStages = 6;
+constexpr int kWpStages = 6;                   // K blocks of weights in flight
 constexpr int kWpParts = 2;                    // epilogue warps a block of 16 columns
 constexpr int kWpTokenWarp = 0, kWpMmaWarp = 1, kWpEpilogueWarp = 2, kWpWeightWarp = kWpEpilogueWarp + 4 * kWpParts;
 constexpr int kWpThreads = (kWpWeightWarp + 1) * 32;
 constexpr uint32_t kWpTmemColumns = 512;
-constexpr int kWpRows = 208;                   // rows of a chunk at most (MMA N), and accumulator columns
-constexpr int kWpChunk = 192;                  // rows of every chunk but the last of an expert with more than kWpRows
+constexpr int kWpRows = 256;                   // rows of a chunk at most (MMA N)
 constexpr int kWpAccStages = 2;
-// One K block's scales, per MMA j: weights at +12j, the chunk's two 128-row blocks at +12j+4 and +12j+8.
-constexpr uint32_t kWpSfColumn = kWpAccStages * kWpRows;
+// Tensor memory: two accumulators of up to kWpRows columns, the second from kWpSecond on, so that they share the columns between if
+// the first is wider than that; then one K block's scales, per MMA j: weights at +12j, the chunk's two 128-row blocks at +12j+4 and +12j+8.
+constexpr int kWpSecond = 208;
+constexpr uint32_t kWpSfColumn = kWpSecond + kWpRows;
 static_assert(kWpSfColumn + 48 <= kWpTmemColumns, "tensor memory budget");
+static_assert(kWpRows - kWpSecond <= 2 * 32 && kWpSecond >= kWpRows - 2 * 32, "shared columns: in the first step of the two parts of the epilogue");
 static_assert(kWpRows / 2 == 8 * kW13PairBoxes, "a box for each half of a chunk");
-constexpr int kWpTokenBytes = kWpRows / 2 * kTileKBytes;  // 13 KiB
+// Token rows in flight: six K blocks of up to kWpSecond / 2 rows or, where some chunk of the batch has more, five of up to kWpRows / 2.
+constexpr int kWpTokenBytes = kWpSecond / 2 * kTileKBytes;     // 13 KiB
+constexpr int kWpWideTokenBytes = kWpRows / 2 * kTileKBytes;   // 16 KiB
+constexpr int kWpWideStages = 5;
+constexpr int kWpTokenRing = kWpWideStages * kWpWideTokenBytes;
+static_assert(kWpStages * kWpTokenBytes <= kWpTokenRing, "token ring");
 constexpr int kWpTileBytes = 128 * kTileKBytes;  // 16 KiB
 constexpr int kWpUnits = kInter / 64;            // 11
 constexpr int kWpUnitSlots = 12;                 // the re-tiled scales carry a twelfth, all-zero unit
 constexpr int kWpItemsPerChunk = kWpUnitSlots / 2;
+constexpr int kWpTable = 512;                    // rounds whose items are worked out once (131072 tokens on 148 SMs have 343)
 
 struct alignas(1024) WpSmem {
   uint8_t w[kWpStages][kWpTileBytes];          // this CTA's 64 up + 64 gate weight rows
-  uint8_t x[kWpStages][kWpTokenBytes];         // this CTA's half of the chunk's token rows
+  uint8_t x[kWpTokenRing];                     // this CTA's half of the chunk's token rows
   uint8_t sfw[kWpStages][kSfStageBytes];       // scales of this CTA's weight rows
   uint8_t sfx[kWpStages][2 * kSfStageBytes];   // scales of the chunk's one or two 128-row blocks
   uint64_t full[kWpStages];    // leader: the stage's bytes have landed in both CTAs
   uint64_t empty[kWpStages];   // both CTAs: the MMAs that read the stage have completed
   uint64_t acc_full[kWpAccStages];   // both CTAs: the item's accumulator is complete
   uint64_t acc_empty[kWpAccStages];  // leader: both CTAs' epilogues have copied the accumulator out
+  uint64_t acc_shared[kWpAccStages]; // leader: ... or the columns of it that the other accumulator may have in common
+  uint64_t table;                    // `items` is there
   uint32_t tmem_base;
   volatile int abort;
   // group geometry, by expert: first row, first scale row, chunks before it
   int offsets[kExperts + 1], scale_rows[kExperts + 1], chunks[kExperts + 1], scan[4];
+  uint32_t items[kWpTable];    // this pair's items but the first, see wp_pack
   GegluTables tables;
 };
 
@@ -83,15 +99,16 @@ __device__ __forceinline__ void wp_load_weights(void* smem_dst, const void* tens
 
 // Scale copies of one K block (four MMAs of K = 64) for both CTAs: per MMA j the atom of the
 // weight rows and the atoms of the chunk's one or two 128-row blocks of tokens.
-template <bool kTwoBlocks>
-__device__ __forceinline__ void wp_issue_sf_copies(uint32_t tmem_sf, uint32_t sfw_lo, uint32_t sfx_lo) {
+__device__ __forceinline__ void wp_issue_sf_copies(uint32_t tmem_sf, uint32_t sfw_lo, uint32_t sfx_lo, bool two_blocks) {
   constexpr uint32_t hi_sf = (128u >> 4) | (1u << 14);                // 8 rows x 16 B, no swizzle
 #pragma unroll
   for (uint32_t j = 0; j < 4; ++j) {
     pair_copy_sf(tmem_sf + 12 * j, hi_sf, sfw_lo + 32 * j);
     pair_copy_sf(tmem_sf + 12 * j + 4, hi_sf, sfx_lo + 32 * j);
-    if (kTwoBlocks) pair_copy_sf(tmem_sf + 12 * j + 8, hi_sf, sfx_lo + 128 + 32 * j);
   }
+  if (two_blocks)
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) pair_copy_sf(tmem_sf + 12 * j + 8, hi_sf, sfx_lo + 128 + 32 * j);
 }
 
 __device__ __forceinline__ void wp_issue_mmas(uint32_t tmem_acc, uint32_t tmem_sf, uint32_t shift, uint32_t w_lo, uint32_t x_lo,
@@ -114,6 +131,11 @@ __device__ __forceinline__ void wp_load_16x32(uint32_t tmem_address, uint32_t (&
       : "memory");
 }
 
+__device__ __forceinline__ void wp_arrive(uint64_t* bar, bool is_leader) {
+  if (is_leader) mbar_arrive(bar);
+  else pair_arrive_remote(bar, 0);
+}
+
 // erf-GELU where the table does not reach: one gate in 20000 of unit variance.
 __device__ __noinline__ float wp_gelu_small(float gate, const float* erf_table) { return gv_gelu_erf(gate, erf_table); }
 
@@ -123,46 +145,68 @@ struct WpItem {
   int shift;     // tensor-memory columns (of 32 rows) by which the chunk starts inside that tile: 0 or 2
   int local;     // first row of the chunk within the expert
   int row0;      // first sorted row of the chunk
-  int valid;     // rows of the chunk, 1..208
+  int valid;     // rows of the chunk, 1..256
   int n;         // MMA N: valid rounded up to 16
   int unit_pair; // 0..5
 };
 
-// Chunks of an expert: one if its rows fit an accumulator, else stretches of 192 (a multiple of 64, so that
-// a chunk's scales start at a column of its first scale tile's atom and end within the next tile's).
-__host__ __device__ __forceinline__ int wp_chunks_of(int rows) {
-  return rows <= kWpRows ? (rows > 0) : (rows + kWpChunk - 1) / kWpChunk;
+// Chunks of an expert: as few as cover its rows, and all but the last of the same multiple of 64 (192 or 256), so that a chunk's scales
+// start at a column of its first scale tile's atom and end within the next tile's.
+__host__ __device__ __forceinline__ int wp_chunks_of(int rows) { return (rows + kWpRows - 1) / kWpRows; }
+__host__ __device__ __forceinline__ int wp_chunk_rows(int rows) {
+  const int chunks = wp_chunks_of(rows);
+  return chunks <= 1 ? rows : (rows + 64 * chunks - 1) / (64 * chunks) * 64;
 }
 
-// Items in snake order over the pairs of the grid: the unit pairs of a chunk go to neighbouring
-// clusters, which then read the same token rows from L2 at about the same time.
-__device__ __forceinline__ bool wp_item(const WpSmem* smem, int round, WpItem& item) {
+// An item in a word: expert, unit pair, N / 16 (never zero), first row / 64; zero: none.
+__device__ __noinline__ uint32_t wp_pack(const WpSmem* smem, int round) {
+  // Snake order over the pairs of the grid: the unit pairs of a chunk go to neighbouring
+  // clusters, which then read the same token rows from L2 at about the same time.
   const int slots = static_cast<int>(gridDim.x) >> 1;
   const int mine = static_cast<int>(blockIdx.x) >> 1;
   const int slot = (round & 1) ? slots - 1 - mine : mine;
   const int index = round * slots + slot;
   const int chunk = index / kWpItemsPerChunk;
-  if (chunk >= smem->chunks[kExperts]) return false;
-  item.unit_pair = index - chunk * kWpItemsPerChunk;
+  if (chunk >= smem->chunks[kExperts]) return 0;
   int expert = 0;  // the last expert with chunks[expert] <= chunk
 #pragma unroll
   for (int step = kExperts / 2; step; step >>= 1)
     if (smem->chunks[expert + step] <= chunk) expert += step;
-  item.expert = expert;
-  item.local = (chunk - smem->chunks[expert]) * kWpChunk;
-  item.row0 = smem->offsets[expert] + item.local;
-  item.first = (smem->scale_rows[expert] + item.local) / kTileM;
-  item.shift = (item.local & (kTileM - 1)) >> 5;
   const int rows = smem->offsets[expert + 1] - smem->offsets[expert];
-  const int rows_after = rows - item.local;
-  item.valid = rows <= kWpRows || rows_after < kWpChunk ? rows_after : kWpChunk;
-  item.n = (item.valid + 15) & ~15;
+  const int chunk_rows = wp_chunk_rows(rows);
+  const int local = (chunk - smem->chunks[expert]) * chunk_rows;
+  const int valid = rows - local < chunk_rows ? rows - local : chunk_rows;
+  return static_cast<uint32_t>(expert) | static_cast<uint32_t>(index - chunk * kWpItemsPerChunk) << 7 |
+         static_cast<uint32_t>((valid + 15) >> 4) << 10 | static_cast<uint32_t>(local >> 6) << 15;
+}
+
+// Behind a wait for `table` but for the first round, whose loads do not wait for it.
+__device__ __forceinline__ uint32_t wp_word(const WpSmem* smem, int round) {
+  return round != 0 && round < kWpTable ? smem->items[round] : wp_pack(smem, round);
+}
+
+// False if there is none; then there is none in any later round either.
+__device__ __forceinline__ bool wp_item(const WpSmem* smem, int round, WpItem& item) {
+  const uint32_t word = wp_word(smem, round);
+  if (word == 0) return false;
+  item.expert = static_cast<int>(word & 127u);
+  item.unit_pair = static_cast<int>((word >> 7) & 7u);
+  item.n = static_cast<int>((word >> 10) & 31u) << 4;
+  item.local = static_cast<int>(word >> 15) << 6;
+  item.row0 = smem->offsets[item.expert] + item.local;
+  item.first = (smem->scale_rows[item.expert] + item.local) / kTileM;
+  item.shift = (item.local & (kTileM - 1)) >> 5;
+  item.valid = min(item.n, smem->offsets[item.expert + 1] - item.row0);
   return true;
 }
 
+__device__ __forceinline__ bool wp_two_blocks(const WpItem& item) { return item.shift * 32 + item.n > kTileM; }
+
 struct WpTokenMaps {
-  CUtensorMap rows[kW13PairBoxes];   // boxes of 8, 16, ... 104 token rows x 128 bytes
+  CUtensorMap rows[kW13PairBoxes];   // boxes of 8, 16, ... 128 token rows x 128 bytes
 };
+
+constexpr int kWpKBlocks = kHidden / 2 / kTileKBytes;   // 11
 
 struct WpParams {
   const float* alpha;          // [experts] g1 output scale
@@ -174,6 +218,62 @@ struct WpParams {
   int* status;
   bool early_weights;
 };
+
+// The leader's MMA thread.  In one thread, with running addresses and a look at the next stage's barrier ahead of the issue; not unrolled over the stages,
+// which takes 20 to 80 cycles off a K block when the code is there, but every launch of a layer fetches its code anew: 34 KB more of it
+// cost layers of 700 to 2500 tokens 3 us.
+__device__ __forceinline__ void wp_issue(WpSmem* smem, uint32_t tmem_base, bool wide, int* status) {
+  const uint32_t w_lo0 = (smem_u32(smem->w[0]) & 0x3ffffu) >> 4, x_lo0 = (smem_u32(smem->x) & 0x3ffffu) >> 4;
+  const uint32_t sfw_lo0 = (smem_u32(smem->sfw[0]) & 0x3ffffu) >> 4, sfx_lo0 = (smem_u32(smem->sfx[0]) & 0x3ffffu) >> 4;
+  const uint32_t token_step = (wide ? kWpWideTokenBytes : kWpTokenBytes) >> 4;
+  const uint32_t x_end = x_lo0 + (wide ? kWpWideStages : kWpStages) * token_step;
+  const uint32_t tmem_sf = tmem_base + kWpSfColumn;
+  uint32_t phase = 0, acc_phase = 0, acc = 0, word = wp_word(smem, 0), next = 0;
+  uint32_t x_lo = x_lo0, stage = 0;
+  bool shares = false;   // the item before this one had the first accumulator and more columns than are its own
+  bool landed = false;   // the next stage's bytes have been seen
+  for (int round = 0; word != 0; ++round, word = next) {
+    if (round == 0 && !wait_or_abort(&smem->table, 0, smem, status)) return;
+    next = wp_word(smem, round + 1);
+    const uint32_t n16 = (word >> 10) & 31u;
+    const uint32_t shift = (word >> 14) & 2u;  // an odd multiple of 64 rows into the expert: two columns of 32 rows into its scale tile
+    const bool two_blocks = shift * 2 + n16 > 8;
+    // E2M1 x E2M1, both K-major, UE4M3 scales; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
+    const uint32_t idesc = (1u << 7) | (1u << 10) | (n16 << 18) | (static_cast<uint32_t>(256 >> 4) << 24);
+    const uint32_t tmem_acc = tmem_base + acc * kWpSecond;
+    if (!wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, status)) return;
+    const bool wider = n16 > kWpSecond / 16;
+    if (round != 0 && (acc == 0 ? wider : shares) &&
+        !wait_or_abort(&smem->acc_shared[acc ^ 1u], acc == 0 ? acc_phase ^ 1u : acc_phase, smem, status))
+      return;
+    shares = wider;
+#pragma unroll 1
+    for (uint32_t kb = 0; kb < kWpKBlocks; ++kb) {
+      if (!landed && !wait_or_abort(&smem->full[stage], phase, smem, status)) return;
+      tc_fence_after_sync();
+      const uint32_t w_lo = w_lo0 + stage * (kWpTileBytes >> 4);
+      const uint32_t sfw_lo = sfw_lo0 + stage * (kSfStageBytes >> 4), sfx_lo = sfx_lo0 + stage * (2 * kSfStageBytes >> 4);
+      uint64_t* const empty = &smem->empty[stage];
+      if (++stage == kWpStages) {
+        stage = 0;
+        phase ^= 1u;
+      }
+      landed = mbar_try_wait(&smem->full[stage], phase);
+      // copies and MMAs of one thread execute in order in the tensor pipe, so one set of scale
+      // columns serves every K block
+      wp_issue_sf_copies(tmem_sf, sfw_lo, sfx_lo, two_blocks);
+      wp_issue_mmas(tmem_acc, tmem_sf, shift, w_lo, x_lo, idesc, kb);
+      pair_commit_both(empty);   // both CTAs may refill the stage
+      x_lo += token_step;
+      if (x_lo == x_end) x_lo = x_lo0;
+    }
+    pair_commit_both(&smem->acc_full[acc]);
+    if (++acc == kWpAccStages) {
+      acc = 0;
+      acc_phase ^= 1u;
+    }
+  }
+}
 
 __global__ void __launch_bounds__(kWpThreads, 1)
 w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_constant__ CUtensorMap map_w,
@@ -194,7 +294,9 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
     for (int b = 0; b < kWpAccStages; ++b) {
       mbar_init(&smem->acc_full[b], 1);
       mbar_init(&smem->acc_empty[b], 2 * 4 * kWpParts);  // the epilogue warps of both CTAs
+      mbar_init(&smem->acc_shared[b], 2 * 4 * kWpParts);
     }
+    mbar_init(&smem->table, 4 * kWpParts);
     smem->abort = 0;
     fence_barrier_init();
     prefetch_tensor_map(&map_w);
@@ -215,11 +317,13 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
   // The plan and the weights may come from before the previous kernel: see W13PairOperands::early_weights.
   if (!p.early_weights) grid_dependency_wait();
 
+  bool wide = false;  // some chunk has more than kWpSecond rows
   if (warp < 4) {
     // thread = expert: chunks before it
     const int e = threadIdx.x;
     const int row = p.expert_offsets[e], next_row = p.expert_offsets[e + 1];
     const int own = wp_chunks_of(next_row - row);
+    wide = wp_chunk_rows(next_row - row) > kWpSecond;
     int inclusive = own;
 #pragma unroll
     for (int offset = 1; offset < 32; offset <<= 1) {
@@ -235,15 +339,11 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
     smem->chunks[e] = inclusive - own;
     if (e == kExperts - 1) smem->chunks[kExperts] = inclusive;
   }
-  __syncthreads();
+  wide = __syncthreads_or(wide);
   if (warp != kWpWeightWarp) {
     grid_dependency_wait();
     grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
   }
-  const int total_items = smem->chunks[kExperts] * kWpItemsPerChunk;
-  const int slots = static_cast<int>(gridDim.x) >> 1;
-  const int rounds = (total_items + slots - 1) / slots;
-  constexpr int k_blocks = kHidden / 2 / kTileKBytes;   // 11
 
   if (warp == kWpTokenWarp || warp == kWpWeightWarp) {
     // ---------------- TMA producers (one warp for each side in each CTA) ----------------
@@ -252,22 +352,26 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
     uint32_t phase = 0;
     int issued = 0;
     bool ok = true;
-    for (int round = 0; ok && round < rounds; ++round) {
-      WpItem item;
-      if (!wp_item(smem, round, item)) continue;
+    // The token side may be fewer K blocks ahead; what it waits for is then a younger stage's MMAs.
+    const int token_stages = wide ? kWpWideStages : kWpStages, token_bytes = wide ? kWpWideTokenBytes : kWpTokenBytes;
+    int wait_stage = weight_side ? 0 : kWpStages - token_stages, slot = 0;
+    uint32_t wait_phase = 1;
+    WpItem item;
+    for (int round = 0; ok && wp_item(smem, round, item); ++round) {
       const int unit = 2 * item.unit_pair + static_cast<int>(rank);
       const bool unit_exists = unit < kWpUnits;
       const int half = item.n >> 1;                            // token rows per CTA, a multiple of 8
       const int token_row = item.row0 + static_cast<int>(rank) * half;
       const bool second_exists = 2 * item.unit_pair + 1 < kWpUnits;
-      // Per K block and CTA: the unit's weight rows and their scales (2 KiB), or the token rows and the scales of two
-      // 128-row blocks of tokens (4 KiB; the second block is fetched, and ignored, also when the chunk has one).
+      // Per K block and CTA: the unit's weight rows and their scales (2 KiB), or the token rows and the scales (2 KiB each) of the
+      // one or two 128-row blocks that the chunk has rows in.
+      const bool two_blocks = wp_two_blocks(item);
       const uint32_t both_bytes = weight_side ? 2 * kSfStageBytes + kWpTileBytes + (second_exists ? kWpTileBytes : 0)
-                                              : 2 * (2 * kSfStageBytes + static_cast<uint32_t>(half) * kTileKBytes);
+                                              : 2 * ((two_blocks ? 2 : 1) * kSfStageBytes + static_cast<uint32_t>(half) * kTileKBytes);
       const CUtensorMap* token_map = &map_x.rows[(half >> 3) - 1];
-      const int w_sf_row = ((item.expert * kWpUnitSlots + unit) * k_blocks) * 4;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->empty[stage], phase ^ 1u, smem, p.status));
+      const int w_sf_row = ((item.expert * kWpUnitSlots + unit) * kWpKBlocks) * 4;
+      for (int kb = 0; kb < kWpKBlocks; ++kb) {
+        ok = __all_sync(0xffffffffu, wait_or_abort(&smem->empty[wait_stage], wait_phase, smem, p.status));
         if (!ok) break;
         if (elect_one()) {
           const int x = kb * kTileKBytes;
@@ -278,8 +382,9 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
             if (unit_exists) wp_load_weights(smem->w[stage], &map_w, bar, x, item.expert * (kW13Out / 16) + unit * 4);
             pair_load(smem->sfw[stage], &map_w_sf, bar, 0, w_sf_row + 4 * kb);
           } else {
-            pair_load(smem->x[stage], token_map, bar, x, token_row);
+            pair_load(smem->x + slot * token_bytes, token_map, bar, x, token_row);
             pair_load_3d(smem->sfx[stage], &map_x_sf, bar, 0, 4 * kb, item.first);
+            if (two_blocks) pair_load_3d(smem->sfx[stage] + kSfStageBytes, &map_x_sf, bar, 0, 4 * kb, item.first + 1);
           }
         }
         __syncwarp();
@@ -288,7 +393,13 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           stage = 0;
           phase ^= 1u;
         }
+        if (++wait_stage == kWpStages) {
+          wait_stage = 0;
+          wait_phase ^= 1u;
+        }
+        if (++slot == token_stages) slot = 0;
       }
+      if (round == 0 && ok) ok = __all_sync(0xffffffffu, wait_or_abort(&smem->table, 0, smem, p.status));
     }
     if (!ok && lane == 0 && is_leader) {
       // Unwinding: let the copies already issued (by either CTA) land before shared memory is
@@ -305,58 +416,11 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
       }
     }
   } else if (warp == kWpMmaWarp) {
-    if (is_leader) {
-      // ---------------- leader: scale copies and MMAs for both CTAs ----------------
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      const uint32_t w_lo0 = (smem_u32(smem->w[0]) & 0x3ffffu) >> 4;
-      const uint32_t x_lo0 = (smem_u32(smem->x[0]) & 0x3ffffu) >> 4;
-      const uint32_t sfw_lo0 = (smem_u32(smem->sfw[0]) & 0x3ffffu) >> 4;
-      const uint32_t sfx_lo0 = (smem_u32(smem->sfx[0]) & 0x3ffffu) >> 4;
-      const bool leader_lane = elect_one();
-      for (int round = 0; round < rounds; ++round) {
-        WpItem item;
-        if (!wp_item(smem, round, item)) continue;
-        const bool two_blocks = item.shift * 32 + item.n > kTileM;
-        // E2M1 x E2M1, both K-major, UE4M3 scales; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
-        const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(item.n >> 3) << 17) |
-                               (static_cast<uint32_t>(256 >> 4) << 24);
-        if (!__all_sync(0xffffffffu, wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, p.status))) break;
-        const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(acc) * kWpRows;
-        bool ok = true;
-        tc_fence_after_sync();
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          ok = wait_or_abort(&smem->full[stage], phase, smem, p.status);
-          if (!ok) break;
-          tc_fence_after_sync();
-          if (leader_lane) {
-            const uint32_t w_lo = w_lo0 + static_cast<uint32_t>(stage) * (kWpTileBytes >> 4);
-            const uint32_t x_lo = x_lo0 + static_cast<uint32_t>(stage) * (kWpTokenBytes >> 4);
-            const uint32_t sfw_lo = sfw_lo0 + static_cast<uint32_t>(stage) * (kSfStageBytes >> 4);
-            const uint32_t sfx_lo = sfx_lo0 + static_cast<uint32_t>(stage) * (2 * kSfStageBytes >> 4);
-            const uint32_t tmem_sf = tmem_base + kWpSfColumn;
-            // copies and MMAs of one thread execute in order in the tensor pipe, so one set of scale
-            // columns serves every K block
-            if (two_blocks) wp_issue_sf_copies<true>(tmem_sf, sfw_lo, sfx_lo);
-            else wp_issue_sf_copies<false>(tmem_sf, sfw_lo, sfx_lo);
-            wp_issue_mmas(tmem_acc, tmem_sf, item.shift, w_lo, x_lo, idesc, kb != 0 ? 1u : 0u);
-            pair_commit_both(&smem->empty[stage]);   // both CTAs may refill the stage
-            if (kb + 1 == k_blocks) pair_commit_both(&smem->acc_full[acc]);
-          }
-          if (++stage == kWpStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
-        }
-        if (!ok) break;
-        if (++acc == kWpAccStages) {
-          acc = 0;
-          acc_phase ^= 1u;
-        }
-      }
+    // ---------------- leader: scale copies and MMAs for both CTAs, in one thread ----------------
+    if (is_leader && elect_one()) {
+      wp_issue(smem, tmem_base, wide, p.status);
     }
+    __syncwarp();
   } else {
     // ---------------- epilogue: eight warps in each CTA ----------------
     // A warp may touch only the tensor-memory lanes 32*(warp%4)..+31: one block of 16 intermediate columns,
@@ -373,39 +437,45 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
     const uint32_t low_word = b ? 0x4062u : 0x6240u, high_word = b ? 0x5173u : 0x7351u;
     const int own_token = 8 * (lane >> 3) + 2 * (lane & 3) + ((lane >> 2) & 1);  // of the 32: the (lane / 4)-th of the thread's
     constexpr int groups = kInter / 16;
+    for (int round = threadIdx.x - 32 * kWpEpilogueWarp; round < kWpTable; round += 32 * 4 * kWpParts) smem->items[round] = wp_pack(smem, round);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&smem->table);
+    const bool there = __all_sync(0xffffffffu, wait_or_abort(&smem->table, 0, smem, p.status));
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int round = 0; round < rounds; ++round) {
-      WpItem item;
-      if (!wp_item(smem, round, item)) continue;
+    WpItem item;
+    for (int round = 0; there && wp_item(smem, round, item); ++round) {
       const int unit = 2 * item.unit_pair + static_cast<int>(rank);
       const int steps = unit < kWpUnits ? (item.valid + 31) >> 5 : 0;  // of 32 tokens, dealt to the two warps of a block
       const float alpha = p.alpha[item.expert];
       const float multiplier = p.next_scale_q[item.expert];
       if (!__all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc], acc_phase, smem, p.status))) break;
       tc_fence_after_sync();
-      const uint32_t tmem_rows = tmem_base + (static_cast<uint32_t>(block * 32) << 16) + static_cast<uint32_t>(acc) * kWpRows;
+      const uint32_t tmem_rows = tmem_base + (static_cast<uint32_t>(block * 32) << 16) + static_cast<uint32_t>(acc) * kWpSecond;
       uint8_t* const scales = p.next_scales + static_cast<size_t>(smem->scale_rows[item.expert]) * groups;
-      int step = (part + round) % kWpParts;
-      bool released = false;
+      // from the end that the two accumulators share
+      int turn = (part + round) % kWpParts;
+      bool first = true, released = false;
 #pragma unroll 1
       do {
         uint32_t even[16], odd[16];
-        if (step < steps) {
+        const int step = acc == 0 ? steps - 1 - turn : turn;
+        if (turn < steps) {
           wp_load_16x32(tmem_rows + 32 * step, even);
           wp_load_16x32(tmem_rows + (16u << 16) + 32 * step, odd);
           tmem_load_wait();
         }
-        if (step + kWpParts >= steps) {
+        released = turn + kWpParts >= steps;
+        if (first || released) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
-            if (is_leader) mbar_arrive(&smem->acc_empty[acc]);
-            else pair_arrive_remote(&smem->acc_empty[acc], 0);
+            if (first) wp_arrive(&smem->acc_shared[acc], is_leader);
+            if (released) wp_arrive(&smem->acc_empty[acc], is_leader);
           }
-          released = true;
+          first = false;
         }
-        if (step >= steps) break;
+        if (turn >= steps) break;
         const int token = 32 * step + own_token;
         // bf16(alpha * acc), columns 2i and 2i + 1 of token k = 2g + s (8g + 2 (lane % 4) + s of the 32)
         uint32_t up[8], gate[8];
@@ -483,7 +553,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
               make_uint2(__byte_perm(first, second, low_word), __byte_perm(first, second, high_word));
           scales[sf_offset(item.local + token, 4 * unit + block, groups)] = static_cast<uint8_t>(scale);
         }
-        step += kWpParts;
+        turn += kWpParts;
       } while (!released);
       if (++acc == kWpAccStages) {
         acc = 0;

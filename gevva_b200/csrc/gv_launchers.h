@@ -181,9 +181,9 @@ int prepare_grouped_gemm_pairs();
 
 // Fused w13 + GeGLU + requantise run by CTA pairs with the weights on the MMA's M side and up to
 // 208 rows of one expert on its N side (grouped_gemm_w13_pair.cu).
-constexpr int kW13PairBoxes = 13;
+constexpr int kW13PairBoxes = 16;
 struct W13PairOperands {
-  CUtensorMap map_x[kW13PairBoxes];  // activation codes [row capacity, 1408] bytes through boxes of 8, 16, ... 104 rows x 128 B
+  CUtensorMap map_x[kW13PairBoxes];  // activation codes [row capacity, 1408] bytes through boxes of 8, 16, ... 128 rows x 128 B
   CUtensorMap map_w;      // w13 codes in the row order of its MMAs, a unit of 64 columns (up and gate rows) a copy
   CUtensorMap map_x_sf;   // activation scale regions as [128-row blocks, 44 atoms, 512 B], box 2 blocks x 4 atoms
   CUtensorMap map_w_sf;   // unit-tiled weight scales (launch_retile_w13_unit_scales), box of four atoms

@@ -161,12 +161,12 @@ bool make_w2_down_map(CUtensorMap* map, const void* base, uint64_t experts) {
 }
 
 // Scale bytes of an activation operand as [128-row blocks, atoms per block, 128 x u32] through a
-// box of two blocks x four atoms: the scales of one K block for up to 256 rows in one copy.
+// box of one block x four atoms: the scales of one K block of up to 128 rows.
 bool make_block_scale_map(CUtensorMap* map, const void* base, uint64_t bytes, int atoms_per_block) {
   const uint64_t block_bytes = static_cast<uint64_t>(atoms_per_block) * 512;
   const cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(atoms_per_block), bytes / block_bytes};
   const cuuint64_t strides[2] = {512, block_bytes};
-  const cuuint32_t box[3] = {128, 4, 2};
+  const cuuint32_t box[3] = {128, 4, 1};
   const cuuint32_t element_strides[3] = {1, 1, 1};
   EncodeTiledFn fn = encode_tiled();
   if (!fn || dims[2] == 0) return false;

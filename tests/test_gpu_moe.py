@@ -701,6 +701,46 @@ def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_devic
     assert results[0][0].float().abs().max() > 0
 
 
+def ids_with_counts(tokens, counts):
+    """Expert ids in which expert e has counts[e] tokens, exactly; the other experts share the rest."""
+    counts = list(counts) + [0] * (EXPERTS - len(counts))
+    rest = tokens * TOP_K - sum(counts)
+    others = [e for e in range(EXPERTS) if counts[e] == 0]
+    for i, e in enumerate(others):
+        counts[e] = rest // len(others) + (i < rest % len(others))
+    assert max(counts) <= tokens and sum(counts) == tokens * TOP_K
+    # an expert's routes are consecutive and so go to different tokens
+    return np.repeat(np.arange(EXPERTS), counts).reshape(TOP_K, tokens).T.astype(np.int32).copy()
+
+
+@pytest.mark.parametrize("tokens,counts", [
+    (2600, [207, 208, 209, 1, 224, 225, 16, 240, 241, 255, 256, 257, 17, 383, 384, 385, 448, 449, 512, 513, 576, 577, 769, 1025]),
+    (2600, [256, 12, 256, 15, 256, 224, 208, 256, 2, 209] * 3), (4096, [256] * EXPERTS)])
+def test_w13_pairs_at_chunk_and_accumulator_edges(gm, weights, cuda_device, tokens, counts, monkeypatch):
+    """w13 by CTA pairs takes up to 256 rows of an expert at once, two accumulators of which have columns in common when one has
+    more than 208: experts at either side of those lines and of every cut into chunks, wide items behind wide and narrow
+    ones, and nothing but the widest; the same codes and scale bytes as from the one-CTA kernel."""
+    from gevva_b200 import runtime as rt
+    dev_ids = torch.from_numpy(ids_with_counts(tokens, counts)).to(cuda_device)
+    x = hashgen.activations(tokens, HIDDEN, 83, cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    results = []
+    for form in ("0", "1"):
+        monkeypatch.setenv("GEVVA_MOE_W13_PAIRS", form)
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        out = torch.empty_like(x)
+        runner.buffer(rt.BUF_INTER_CODES).zero_()
+        runner.buffer(rt.BUF_INTER_SF).zero_()
+        for _ in range(2):
+            runner.launch_batch(x, dev_ids, rw, out, tokens)
+        runner.check()
+        results.append((out, runner.buffer(rt.BUF_INTER_CODES)[: tokens * TOP_K * INTER // 2].clone(),
+                        runner.buffer(rt.BUF_INTER_SF).clone()))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert results[0][0].float().abs().max() > 0
+
+
 @pytest.mark.parametrize("tokens,kind", [(1, "random"), (8, "random"), (40, "skewed"), (64, "random"),
                                          (128, "skewed")])
 def test_merged_decode_launch_equals_two_launches(gm, weights, cuda_device, tokens, kind, monkeypatch):
