@@ -105,28 +105,7 @@ __device__ __forceinline__ uint32_t bf16_pair(float low, float high) {
   return *reinterpret_cast<const uint32_t*>(&p);
 }
 
-// Two floats in a register pair: one instruction works on both, each rounded as by itself.
-__device__ __forceinline__ unsigned long long two(float low, float high) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(low), "f"(high));
-  return r;
-}
-__device__ __forceinline__ unsigned long long two(uint32_t pair) { return two(low_half(pair), high_half(pair)); }
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
+__device__ __forceinline__ unsigned long long two_of(uint32_t pair) { return two(low_half(pair), high_half(pair)); }
 __device__ __forceinline__ uint32_t round2(unsigned long long v) {
   float low, high;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(low), "=f"(high) : "l"(v));
@@ -383,7 +362,7 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
   const float scale = dense_activation_scales ? __fmul_rn(dense_activation_scales[row], dense_projection_scale[0]) : 1.0f;
   if (dense_activation_scales) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) d[i] = round2(mul2(two(d[i]), two(scale, scale)));
+    for (int i = 0; i < 4; ++i) d[i] = round2(mul2(two_of(d[i]), two(scale, scale)));
   }
   const float dense_sum = warp_sum_squares_of(d);
   unsigned long long sum[4] = {};
@@ -392,7 +371,7 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
     const float weight = route_weights[row * kTopK + k];
     words(routes[k], v);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) sum[i] = fma2(two(v[i]), two(weight, weight), sum[i]);
+    for (int i = 0; i < 4; ++i) sum[i] = fma2(two_of(v[i]), two(weight, weight), sum[i]);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) e[i] = round2(sum[i]);
@@ -411,12 +390,12 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
   const float expert_inverse = inverse_rms(fold_warps(expert_sums));
   words(dense_weight_raw, w);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) d[i] = round2(mul2(mul2(two(d[i]), two(dense_inverse, dense_inverse)), two(w[i])));
+  for (int i = 0; i < 4; ++i) d[i] = round2(mul2(mul2(two_of(d[i]), two(dense_inverse, dense_inverse)), two_of(w[i])));
   words(expert_weight_raw, w);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    e[i] = round2(mul2(mul2(two(e[i]), two(expert_inverse, expert_inverse)), two(w[i])));
-    d[i] = round2(add2(two(d[i]), two(e[i])));
+    e[i] = round2(mul2(mul2(two_of(e[i]), two(expert_inverse, expert_inverse)), two_of(w[i])));
+    d[i] = round2(add2(two_of(d[i]), two_of(e[i])));
   }
   const float combined_sum = warp_sum_squares_of(d);
   if ((threadIdx.x & 31) == 0) combined_sums[threadIdx.x >> 5] = combined_sum;
@@ -426,8 +405,8 @@ ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16*
   words(residual_raw, v);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint32_t normalized = round2(mul2(mul2(two(d[i]), two(combined_inverse, combined_inverse)), two(w[i])));
-    v[i] = round2(mul2(two(round2(add2(two(v[i]), two(normalized)))), two(scalar, scalar)));
+    const uint32_t normalized = round2(mul2(mul2(two_of(d[i]), two(combined_inverse, combined_inverse)), two_of(w[i])));
+    v[i] = round2(mul2(two_of(round2(add2(two_of(v[i]), two_of(normalized)))), two(scalar, scalar)));
   }
   reinterpret_cast<uint4*>(output + base)[threadIdx.x] = uint4{v[0], v[1], v[2], v[3]};
 }

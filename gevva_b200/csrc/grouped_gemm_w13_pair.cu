@@ -27,8 +27,12 @@
 // their cta_group::2 form, no multicast; the scale atoms travel through tensor maps too).  There
 // the MMA thread copies the scale atoms of a landed stage into tensor memory, issues four MMAs
 // (copies and MMAs of one thread execute in order) and commits to `empty` of both CTAs.  Two accumulators, so that the
-// eight epilogue warps of each CTA work on one item while the next is computed; two of 256 columns do not fit beside the scales, so they have 48 in common,
-// which the epilogue reads first and releases by themselves (an item waits for that where the two would meet).  The items of a pair are worked out once, by all threads.  (With the accumulator transposed
+// eight epilogue warps of each CTA work on one item while the next is computed; two of 256 columns do not fit beside the scales, so such two have 48 in common,
+// which the epilogue reads first and releases by themselves (an item waits for that where the two would meet).  The items of a pair are worked out once, by all threads.  A step of the
+// epilogue (32 tokens, 1800 cycles) took 3500 more when a gate was zero or tiny, which 3 to 25 % of the steps have: such gates now take the
+// polynomial's first interval in line (of the accumulators' columns that no row owns, too).  With that, pairs of values to an instruction and the next
+// accumulators fetched ahead: 700 tokens 53.2 -> 51.6 us, 4096 88.2 -> 85.2, 16384 269 -> 263; a layer of 700 tokens 108.5 -> 107.4,
+// of 4096 245 -> 240.  (With the accumulator transposed
 // through shared memory by sixteen warps that traffic bounded the kernel, 107 us at 4096 tokens; with this epilogue
 // twelve or sixteen warps are 3 to 8 % slower than eight, and five stages up to 8 % slower than six.)  Every wait is bounded.
 #include "gv_common.cuh"
@@ -47,15 +51,14 @@ constexpr int kWpThreads = (kWpWeightWarp + 1) * 32;
 constexpr uint32_t kWpTmemColumns = 512;
 constexpr int kWpRows = 256;                   // rows of a chunk at most (MMA N)
 constexpr int kWpAccStages = 2;
-// Tensor memory: two accumulators of up to kWpRows columns, the second from kWpSecond on, so that they share the columns between if
-// the first is wider than that; then one K block's scales, per MMA j: weights at +12j, the chunk's two 128-row blocks at +12j+4 and +12j+8.
-constexpr int kWpSecond = 208;
-constexpr uint32_t kWpSfColumn = kWpSecond + kWpRows;
-static_assert(kWpSfColumn + 48 <= kWpTmemColumns, "tensor memory budget");
-static_assert(kWpRows - kWpSecond <= 2 * 32 && kWpSecond >= kWpRows - 2 * 32, "shared columns: in the first step of the two parts of the epilogue");
-static_assert(kWpRows / 2 == 8 * kW13PairBoxes, "a box for each half of a chunk");
-// Token rows in flight: six K blocks of up to kWpSecond / 2 rows or, where some chunk of the batch has more, five of up to kWpRows / 2.
-constexpr int kWpTokenBytes = kWpSecond / 2 * kTileKBytes;     // 13 KiB
+// Tensor memory: two accumulators, the first from column 0 on, the second up to where the scales begin, so that two of more than
+// kWpSfColumn columns together have their inner ends in common; then one K block's scales, per MMA j: weights at +12j, the chunk's two
+// 128-row blocks at +12j+4 and +12j+8.
+constexpr uint32_t kWpSfColumn = kWpTmemColumns - 48;
+static_assert(2 * kWpRows - kWpSfColumn <= 2 * 32 - 16, "shared columns: in the first step of the two parts of the epilogue");
+// Token rows in flight: six K blocks of chunks of up to kWpNarrow rows or, where some chunk of the batch has more, five of up to kWpRows.
+constexpr int kWpNarrow = 208;
+constexpr int kWpTokenBytes = kWpNarrow / 2 * kTileKBytes;     // 13 KiB
 constexpr int kWpWideTokenBytes = kWpRows / 2 * kTileKBytes;   // 16 KiB
 constexpr int kWpWideStages = 5;
 constexpr int kWpTokenRing = kWpWideStages * kWpWideTokenBytes;
@@ -135,9 +138,6 @@ __device__ __forceinline__ void wp_arrive(uint64_t* bar, bool is_leader) {
   if (is_leader) mbar_arrive(bar);
   else pair_arrive_remote(bar, 0);
 }
-
-// erf-GELU where the table does not reach: one gate in 20000 of unit variance.
-__device__ __noinline__ float wp_gelu_small(float gate, const float* erf_table) { return gv_gelu_erf(gate, erf_table); }
 
 struct WpItem {
   int expert;
@@ -230,7 +230,7 @@ __device__ __forceinline__ void wp_issue(WpSmem* smem, uint32_t tmem_base, bool 
   const uint32_t tmem_sf = tmem_base + kWpSfColumn;
   uint32_t phase = 0, acc_phase = 0, acc = 0, word = wp_word(smem, 0), next = 0;
   uint32_t x_lo = x_lo0, stage = 0;
-  bool shares = false;   // the item before this one had the first accumulator and more columns than are its own
+  uint32_t before = 0;   // N / 16 of the item before
   bool landed = false;   // the next stage's bytes have been seen
   for (int round = 0; word != 0; ++round, word = next) {
     if (round == 0 && !wait_or_abort(&smem->table, 0, smem, status)) return;
@@ -240,13 +240,10 @@ __device__ __forceinline__ void wp_issue(WpSmem* smem, uint32_t tmem_base, bool 
     const bool two_blocks = shift * 2 + n16 > 8;
     // E2M1 x E2M1, both K-major, UE4M3 scales; N at [17,23) in units of 8, M = 256 at [24,29) in units of 16
     const uint32_t idesc = (1u << 7) | (1u << 10) | (n16 << 18) | (static_cast<uint32_t>(256 >> 4) << 24);
-    const uint32_t tmem_acc = tmem_base + acc * kWpSecond;
+    const uint32_t tmem_acc = tmem_base + (acc == 0 ? 0 : kWpSfColumn - 16 * n16);
     if (!wait_or_abort(&smem->acc_empty[acc], acc_phase ^ 1u, smem, status)) return;
-    const bool wider = n16 > kWpSecond / 16;
-    if (round != 0 && (acc == 0 ? wider : shares) &&
-        !wait_or_abort(&smem->acc_shared[acc ^ 1u], acc == 0 ? acc_phase ^ 1u : acc_phase, smem, status))
-      return;
-    shares = wider;
+    if (before + n16 > kWpSfColumn / 16 && !wait_or_abort(&smem->acc_shared[acc ^ 1u], acc == 0 ? acc_phase ^ 1u : acc_phase, smem, status)) return;
+    before = n16;
 #pragma unroll 1
     for (uint32_t kb = 0; kb < kWpKBlocks; ++kb) {
       if (!landed && !wait_or_abort(&smem->full[stage], phase, smem, status)) return;
@@ -317,13 +314,13 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
   // The plan and the weights may come from before the previous kernel: see W13PairOperands::early_weights.
   if (!p.early_weights) grid_dependency_wait();
 
-  bool wide = false;  // some chunk has more than kWpSecond rows
+  bool wide = false;  // some chunk has more than kWpNarrow rows
   if (warp < 4) {
     // thread = expert: chunks before it
     const int e = threadIdx.x;
     const int row = p.expert_offsets[e], next_row = p.expert_offsets[e + 1];
     const int own = wp_chunks_of(next_row - row);
-    wide = wp_chunk_rows(next_row - row) > kWpSecond;
+    wide = wp_chunk_rows(next_row - row) > kWpNarrow;
     int inclusive = own;
 #pragma unroll
     for (int offset = 1; offset < 32; offset <<= 1) {
@@ -443,70 +440,95 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
     const bool there = __all_sync(0xffffffffu, wait_or_abort(&smem->table, 0, smem, p.status));
     int acc = 0;
     uint32_t acc_phase = 0;
+    uint32_t even[16], odd[16];
     WpItem item;
     for (int round = 0; there && wp_item(smem, round, item); ++round) {
       const int unit = 2 * item.unit_pair + static_cast<int>(rank);
       const int steps = unit < kWpUnits ? (item.valid + 31) >> 5 : 0;  // of 32 tokens, dealt to the two warps of a block
       const float alpha = p.alpha[item.expert];
+      const unsigned long long alphas = two(alpha, alpha);
       const float multiplier = p.next_scale_q[item.expert];
       if (!__all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc], acc_phase, smem, p.status))) break;
       tc_fence_after_sync();
-      const uint32_t tmem_rows = tmem_base + (static_cast<uint32_t>(block * 32) << 16) + static_cast<uint32_t>(acc) * kWpSecond;
+      const uint32_t tmem_rows = tmem_base + (static_cast<uint32_t>(block * 32) << 16) + (acc == 0 ? 0u : kWpSfColumn - static_cast<uint32_t>(item.n));
       uint8_t* const scales = p.next_scales + static_cast<size_t>(smem->scale_rows[item.expert]) * groups;
-      // from the end that the two accumulators share
+      // from the end that the two accumulators share; the next step's accumulators are fetched under a step's arithmetic
       int turn = (part + round) % kWpParts;
-      bool first = true, released = false;
+      bool first = true;
+      const auto load = [&](int turn_of_load) {
+        const int step = acc == 0 ? steps - 1 - turn_of_load : turn_of_load;
+        wp_load_16x32(tmem_rows + 32 * step, even);
+        wp_load_16x32(tmem_rows + (16u << 16) + 32 * step, odd);
+      };
+      if (turn < steps) {
+        load(turn);
+        tmem_load_wait();
+      }
 #pragma unroll 1
-      do {
-        uint32_t even[16], odd[16];
-        const int step = acc == 0 ? steps - 1 - turn : turn;
-        if (turn < steps) {
-          wp_load_16x32(tmem_rows + 32 * step, even);
-          wp_load_16x32(tmem_rows + (16u << 16) + 32 * step, odd);
-          tmem_load_wait();
-        }
-        released = turn + kWpParts >= steps;
-        if (first || released) {
+      for (;;) {
+        const bool last = turn + kWpParts >= steps;
+        if (first || last) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
             if (first) wp_arrive(&smem->acc_shared[acc], is_leader);
-            if (released) wp_arrive(&smem->acc_empty[acc], is_leader);
+            if (last) wp_arrive(&smem->acc_empty[acc], is_leader);
           }
           first = false;
         }
         if (turn >= steps) break;
-        const int token = 32 * step + own_token;
+        const int token = 32 * (acc == 0 ? steps - 1 - turn : turn) + own_token;
         // bf16(alpha * acc), columns 2i and 2i + 1 of token k = 2g + s (8g + 2 (lane % 4) + s of the 32)
         uint32_t up[8], gate[8];
-        int smallest = 0;  // its sign bit: some magnitude lies below the table
-        float v0[8], v1[8];
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          const int r = 2 * k;
+          const unsigned long long u0 = mul2(alphas, two(__uint_as_float(even[r]), __uint_as_float(even[r + 1])));
+          const unsigned long long u1 = mul2(alphas, two(__uint_as_float(odd[r]), __uint_as_float(odd[r + 1])));
+          const unsigned long long g0 = mul2(alphas, two(__uint_as_float(even[r + 2]), __uint_as_float(even[r + 3])));
+          const unsigned long long g1 = mul2(alphas, two(__uint_as_float(odd[r + 2]), __uint_as_float(odd[r + 3])));
+          up[k] = pack_bf16x2(low_of(u0), low_of(u1));
+          up[k + 1] = pack_bf16x2(high_of(u0), high_of(u1));
+          gate[k] = pack_bf16x2(low_of(g0), low_of(g1));
+          gate[k + 1] = pack_bf16x2(high_of(g0), high_of(g1));
+        }
+        if (!last) load(turn + kWpParts);  // under this step's arithmetic; waited for at its end
+        // erf of the magnitudes from the table, two indices to a word
+        constexpr uint32_t kFirst = kErfFirst * 0x10001u, kLast = (kErfFirst + kErfEntries - 1) * 0x10001u;
+        float erf0[8], erf1[8];
+        uint32_t smallest = 0xffffffffu;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const int r = 4 * (k >> 1) + (k & 1);
-          up[k] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(even[r])), __fmul_rn(alpha, __uint_as_float(odd[r])));
-          gate[k] = pack_bf16x2(__fmul_rn(alpha, __uint_as_float(even[r + 2])), __fmul_rn(alpha, __uint_as_float(odd[r + 2])));
-          const int index0 = erf_index(gate[k] & 0x7fffu), index1 = erf_index((gate[k] >> 16) & 0x7fffu);
-          smallest |= index0 | index1;
-          v0[k] = gelu_from_erf(__uint_as_float(gate[k] << 16), smem->tables.erf_of[max(index0, 0)]);
-          v1[k] = gelu_from_erf(__uint_as_float(gate[k] & 0xffff0000u), smem->tables.erf_of[max(index1, 0)]);
+          const uint32_t magnitudes = gate[k] & 0x7fff7fffu;
+          smallest = __vminu2(smallest, magnitudes);
+          const uint32_t offsets = 4u * __vminu2(__vmaxu2(magnitudes, kFirst), kLast) - 4u * kFirst;
+          const char* const table = reinterpret_cast<const char*>(smem->tables.erf_of);
+          erf0[k] = *reinterpret_cast<const float*>(table + (offsets & 0xffffu));
+          erf1[k] = *reinterpret_cast<const float*>(table + (offsets >> 16));
         }
-        if (smallest < 0) {
+        if (__vminu2(smallest, kFirst) != kFirst) {  // one gate in 20000 of unit variance, and the zeros of rows that do not exist
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            if (erf_index(gate[k] & 0x7fffu) < 0) v0[k] = wp_gelu_small(__uint_as_float(gate[k] << 16), smem->tables.erf_table);
-            if (erf_index((gate[k] >> 16) & 0x7fffu) < 0)
-              v1[k] = wp_gelu_small(__uint_as_float(gate[k] & 0xffff0000u), smem->tables.erf_table);
+            const uint32_t low = gate[k] & 0x7fffu, high = (gate[k] >> 16) & 0x7fffu;
+            if (low < kErfFirst) erf0[k] = erf_below_table(__uint_as_float(low << 16));
+            if (high < kErfFirst) erf1[k] = erf_below_table(__uint_as_float(high << 16));
           }
         }
         __syncwarp();
-        float most[8];
+        // gelu_from_erf of the gates times up
+        float v0[8], v1[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          v0[k] = __fmul_rn(v0[k], __uint_as_float(up[k] << 16));
-          v1[k] = __fmul_rn(v1[k], __uint_as_float(up[k] & 0xffff0000u));
-          most[k] = fmaxf(fabsf(v0[k]), fabsf(v1[k]));
+          const float gate0 = __uint_as_float(gate[k] << 16), gate1 = __uint_as_float(gate[k] & 0xffff0000u);
+          const unsigned long long half = mul2(two(0.5f, 0.5f), two(gate0, gate1));
+          const unsigned long long one_plus = add2(two(1.0f, 1.0f), two(copysignf(erf0[k], gate0), copysignf(erf1[k], gate1)));
+          const unsigned long long v = mul2(mul2(half, one_plus), two(__uint_as_float(up[k] << 16), __uint_as_float(up[k] & 0xffff0000u)));
+          v0[k] = low_of(v);
+          v1[k] = high_of(v);
         }
+        float most[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) most[k] = fmaxf(fabsf(v0[k]), fabsf(v1[k]));
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const float received = __shfl_xor_sync(0xffffffffu, a ? most[k] : most[k + 4], 16);
@@ -528,7 +550,13 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           float inverses[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) inverses[k] = __shfl_sync(0xffffffffu, inverse, (lane & 3) | (16 * half + 4 * k));
-          const float *x0 = v0 + 4 * half, *x1 = v1 + 4 * half;
+          float x0[4], x1[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned long long x = mul2(two(v0[4 * half + k], v1[4 * half + k]), two(inverses[k], inverses[k]));
+            x0[k] = low_of(x);
+            x1[k] = high_of(x);
+          }
           asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
               "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
               "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
@@ -536,9 +564,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
               "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
               "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
               : "=r"(words[half])
-              : "f"(__fmul_rn(x0[0], inverses[0])), "f"(__fmul_rn(x1[0], inverses[0])), "f"(__fmul_rn(x0[1], inverses[1])),
-                "f"(__fmul_rn(x1[1], inverses[1])), "f"(__fmul_rn(x0[2], inverses[2])), "f"(__fmul_rn(x1[2], inverses[2])),
-                "f"(__fmul_rn(x0[3], inverses[3])), "f"(__fmul_rn(x1[3], inverses[3])));
+              : "f"(x0[0]), "f"(x1[0]), "f"(x0[1]), "f"(x1[1]), "f"(x0[2]), "f"(x1[2]), "f"(x0[3]), "f"(x1[3]));
         }
         // 8 x 8 bytes over the eight lanes, transposed: bits 2, 1 and 0 of the lane number in turn
         const uint32_t received_a = __shfl_xor_sync(0xffffffffu, a ? words[0] : words[1], 16);
@@ -553,8 +579,10 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
               make_uint2(__byte_perm(first, second, low_word), __byte_perm(first, second, high_word));
           scales[sf_offset(item.local + token, 4 * unit + block, groups)] = static_cast<uint8_t>(scale);
         }
+        if (last) break;
         turn += kWpParts;
-      } while (!released);
+        tmem_load_wait();
+      }
       if (++acc == kWpAccStages) {
         acc = 0;
         acc_phase ^= 1u;

@@ -45,6 +45,30 @@ __device__ __forceinline__ void load_erf_table(float* shared_table) {
   if (threadIdx.x < GV_ERF_TABLE_FLOATS) shared_table[threadIdx.x] = g_erf_table[threadIdx.x >> 3][threadIdx.x & 7];
 }
 
+// Two floats in a register pair: one instruction works on both, each rounded as by itself.
+__device__ __forceinline__ unsigned long long two(float low, float high) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(low), "f"(high));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float low_of(unsigned long long v) { return __uint_as_float(static_cast<uint32_t>(v)); }
+__device__ __forceinline__ float high_of(unsigned long long v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+
 __device__ __forceinline__ float bf16_bits_to_float(uint32_t bits16) {
   return __uint_as_float(bits16 << 16);
 }

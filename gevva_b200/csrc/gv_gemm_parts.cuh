@@ -172,6 +172,15 @@ __device__ __forceinline__ void fill_geglu_tables(GegluTables* tables) {
                                 tables->erf_table);
 }
 
+// gv_erff of a bf16 magnitude below the table over the square root of two: its first interval, whose coefficients are the same for all lanes.
+__device__ __forceinline__ float erf_below_table(float magnitude) {
+  const float u = __fsub_rn(__fmul_rn(magnitude, 0.7071067811865475f), 0.25f);
+  float p = g_erf_table[0][6];
+#pragma unroll
+  for (int i = 5; i >= 0; --i) p = __fmaf_rn(p, u, g_erf_table[0][i]);
+  return p;
+}
+
 // erf-GELU of a bf16 value from erf of its magnitude (gv_gelu_erf's last three operations).
 __device__ __forceinline__ float gelu_from_erf(float value, float erf_of_magnitude) {
   return __fmul_rn(__fmul_rn(0.5f, value), __fadd_rn(1.0f, copysignf(erf_of_magnitude, value)));
