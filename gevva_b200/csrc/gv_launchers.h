@@ -47,6 +47,12 @@ struct RoutePlan {
                            // kernel (gv_stream_schedule.h)
 };
 
+// Weights that the kernel behind a launch begins with, asked into L2 by that launch (two arrays; empty: nothing is asked).
+struct WeightsAhead {
+  const uint8_t* base[2];
+  uint32_t bytes[2];  // multiples of 16
+};
+
 void launch_route(const void* logits_bf16, int ld, const void* expert_scale_bf16, float* weights,
                   int* ids, int tokens, const float* activation_scales,
                   const float* projection_weight_scale, cudaStream_t stream);
@@ -71,7 +77,7 @@ void launch_route_sort_quantize_small(const void* input_bf16, const int* expert_
 // stream's previous kernel is the route sort of this batch.
 void launch_quantize_input(const void* input_bf16, const int* expert_ids, const float* in_scale_q,
                            const RoutePlan& plan, int tokens, uint8_t* packed, uint8_t* scales, bool behind_sort,
-                           cudaStream_t stream);
+                           const WeightsAhead& ahead, cudaStream_t stream);
 
 // bf16 [R, 1408] ([up;gate]) -> codes [R, 352] + swizzled scale bytes.
 void launch_geglu_quantize(const void* fused_bf16, const float* in_scale_q, const RoutePlan& plan,

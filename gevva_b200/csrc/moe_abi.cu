@@ -26,6 +26,13 @@ using namespace gv;
 
 constexpr int kMaxTokens = 131072;
 constexpr int kStreamTokens = 640;  // see moe_streams
+// The quantiser of a call that goes on to the experts asks for the first weights of w13, which all such batches need (nearly every expert has
+// rows, and they are taken in order): HBM has little else to do while the sort and the quantiser run.  16 experts are the first
+// item of every SM and a little more (8 and 80 MB instead of 36 gain less).  Where the experts stream, us of the listed number of layers without / with: 300 tokens
+// 361.8 / 358.9 (four), 400 187.8 / 184.7, 613 191.3 / 189.2, 640 205.1 / 202.3 (two), Zipf(1.1) 500 the same; feed-forward layers of 301 tokens 314.2 / 312.7, 400
+// 330.0 / 326.9 (three), 640 248.9 / 248.1 (two).  By pairs: 700 228.9 / 227.0, 1000 244.8 / 241.9, 1400 280.3 / 277.7 (two), 2048 nothing, and feed-forward layers, whose
+// dense MLP runs between, lose by it (1000 tokens 311 / 319, 2048 442 / 447), as others' that take their rows unreduced would.
+constexpr int kAheadExperts = 16, kAheadTokens = 1536;
 // w2 by CTA pairs that share weights between two row tiles of an expert: from 160 rows an expert on average, where most experts
 // have two tiles.  Two layers in a graph, one CTA a tile and pairs, us: 1536 tokens 262 and 278, 2048 308 and 320, 2304 341 and 332, 2432 347 and
 // 344, 2560 362 and 361, 2688 365 and 361, 3072 383 and 371, 4096 496 and 494.  (Evenly loaded experts; the sides cross between 2048 and 2304.)
@@ -345,6 +352,12 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
   // pairing two row tiles of an expert; they keep the one-CTA-per-tile kernel.
   const bool use_pairs = runner->pairs && tokens > gv::kFusedSortQuantizeMaxTokens;
   const unsigned front = GEVVA_MOE_STAGE_SORT | GEVVA_MOE_STAGE_QUANTIZE;
+  const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
+  const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
+  // Weights on the MMA's M side, by CTA pairs: faster than (2048 tokens on) or as fast as the one-CTA tile kernel
+  // wherever a batch does not stream (figures in grouped_gemm_w13_pair.cu).
+  const bool w13_by_pairs = !use_pairs && sm_count >= 2 && !runner->w13_single &&
+                            (tokens > kStreamTokens || (runner->w13_pair_form && tokens > gv::kFusedSortQuantizeMaxTokens));
   const unsigned layer_body = front | GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU | GEVVA_MOE_STAGE_W2;
   const bool streams = !(stages & GEVVA_MOE_STAGE_UNFUSED) && gv::moe_streams(runner, tokens);
   if ((stages & layer_body) == layer_body && streams && runner->decode_front && gv::stream_layer_fits(tokens, sm_count)) {
@@ -365,16 +378,18 @@ int gv::moe_launch_stages_on(gevva_moe* runner, const void* in, const int* ids, 
       gv::launch_route_sort(ids, routes, s->plan, stream);
     }
     StageRange range(runner->nvtx && (stages & GEVVA_MOE_STAGE_QUANTIZE), "gevva_moe.quantize");
-    if (stages & GEVVA_MOE_STAGE_QUANTIZE)
+    if (stages & GEVVA_MOE_STAGE_QUANTIZE) {
+      gv::WeightsAhead ahead{};
+      if ((stages & gemms) == gemms && (streams || (w13_by_pairs && tokens <= kAheadTokens && (stages & GEVVA_MOE_STAGE_REDUCE)))) {
+        ahead.base[0] = static_cast<const uint8_t*>(runner->weights.w13);
+        ahead.bytes[0] = kAheadExperts * gv::kW13Out * (gv::kHidden / 2);
+        ahead.base[1] = streams ? runner->w13_sf_units : runner->w13_sf_fragments;
+        ahead.bytes[1] = static_cast<uint32_t>(gv::w13_unit_scale_bytes(kAheadExperts));
+      }
       gv::launch_quantize_input(in, ids, runner->weights.in_scale_q1, s->plan, tokens, s->input_codes,
-                                s->input_sf, (stages & GEVVA_MOE_STAGE_SORT) != 0, stream);
+                                s->input_sf, (stages & GEVVA_MOE_STAGE_SORT) != 0, ahead, stream);
+    }
   }
-  const unsigned both = GEVVA_MOE_STAGE_W13 | GEVVA_MOE_STAGE_GEGLU;
-  const unsigned gemms = both | GEVVA_MOE_STAGE_W2;
-  // Weights on the MMA's M side, by CTA pairs: faster than (2048 tokens on) or as fast as the one-CTA tile kernel
-  // wherever a batch does not stream (figures in grouped_gemm_w13_pair.cu).
-  const bool w13_by_pairs = !use_pairs && sm_count >= 2 && !runner->w13_single &&
-                            (tokens > kStreamTokens || (runner->w13_pair_form && tokens > gv::kFusedSortQuantizeMaxTokens));
   if ((stages & gemms) == gemms && streams) {
     StageRange range(runner->nvtx, "gevva_moe.w13+geglu+w2");
     gv::launch_stream_experts(runner->stream_experts, s->plan, sm_count, stream);

@@ -433,11 +433,15 @@ void launch_route_sort(const int* expert_ids, int routes, const RoutePlan& plan,
 // come from the sort.  So the loads and the arithmetic of the CTAs that find room happen during the
 // sort, and what follows it is the stores.
 // ---------------------------------------------------------------------------
+//
+// ahead: while the sort and this kernel run, nothing else wants the memory, so the CTAs ask for a share each of the weights that the
+// experts' kernel begins with (a hint: it changes no result).  A copy is of at most kAheadPiece bytes.
+constexpr uint32_t kAheadPiece = 16384;
 template <bool kEarly>
 __global__ void __launch_bounds__(kQuantizeThreadsPerToken)
 quantize_input_kernel(const __nv_bfloat16* __restrict__ input, const int* __restrict__ expert_ids,
                       const float* __restrict__ in_scale_q, RoutePlan plan,
-                      uint8_t* __restrict__ packed, uint8_t* __restrict__ scales) {
+                      uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, const WeightsAhead ahead) {
   constexpr int groups = kHidden / 16;
   __shared__ float route_multiplier[kTopK];
   __shared__ int route_row[kTopK];  // sorted row, or -1 for a rejected expert id
@@ -448,6 +452,15 @@ quantize_input_kernel(const __nv_bfloat16* __restrict__ input, const int* __rest
   float maximum[2];
   QuantisedBlocks blocks;
   int expert = -1;
+  if (threadIdx.x < 2) {
+    const uint32_t bytes = threadIdx.x ? ahead.bytes[1] : ahead.bytes[0];
+    const uint8_t* const base = threadIdx.x ? ahead.base[1] : ahead.base[0];
+    const uint32_t share = (bytes / gridDim.x + 128u) & ~127u;  // all shares together are more than all bytes
+    for (uint32_t at = blockIdx.x * share; at < bytes && at < (blockIdx.x + 1) * share; at += kAheadPiece) {
+      const uint32_t left = min(bytes, (blockIdx.x + 1) * share) - at;
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + at), "r"(left < kAheadPiece ? left : kAheadPiece) : "memory");
+    }
+  }
   if (!kEarly) grid_dependency_wait();  // the route sort's plan, and the previous user of the output buffers
   load_token_columns(input, token, part, values, maximum);
   if (threadIdx.x < kTopK) {
@@ -595,10 +608,10 @@ void launch_route_sort_quantize_small(const void* input_bf16, const int* expert_
 
 void launch_quantize_input(const void* input_bf16, const int* expert_ids, const float* in_scale_q,
                            const RoutePlan& plan, int tokens, uint8_t* packed, uint8_t* scales, bool behind_sort,
-                           cudaStream_t stream) {
+                           const WeightsAhead& ahead, cudaStream_t stream) {
   const __nv_bfloat16* input = static_cast<const __nv_bfloat16*>(input_bf16);
   launch_chained(behind_sort ? quantize_input_kernel<true> : quantize_input_kernel<false>, dim3(tokens),
-                 dim3(kQuantizeThreadsPerToken), 0, stream, input, expert_ids, in_scale_q, plan, packed, scales);
+                 dim3(kQuantizeThreadsPerToken), 0, stream, input, expert_ids, in_scale_q, plan, packed, scales, ahead);
 }
 
 // ---------------------------------------------------------------------------

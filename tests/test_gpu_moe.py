@@ -701,6 +701,27 @@ def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_devic
     assert results[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens", [297, 640, 641, 1536, 1537])
+def test_weights_asked_ahead_change_no_result(gm, weights, cuda_device, tokens):
+    """From 297 to 1536 tokens the quantiser of a whole call asks for the experts' first weights, shared out over its CTAs; called
+    stage by stage, or above, it does not: the same codes, scale bytes and output."""
+    from gevva_b200 import runtime as rt
+    x = hashgen.activations(tokens, HIDDEN, 91, cuda_device)
+    dev_ids = torch.from_numpy(random_ids(tokens, 29)).to(cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    results = []
+    for split in (False, True):
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens)
+        out = torch.zeros_like(x)
+        for stage in ((rt.STAGE_SORT, rt.STAGE_QUANTIZE, rt.STAGE_ALL & ~(rt.STAGE_SORT | rt.STAGE_QUANTIZE)) if split else (rt.STAGE_ALL,)):
+            runner.launch_stages(stage, tokens, input=x, expert_ids=dev_ids, route_weights=rw, output=out)
+        runner.check()
+        results.append((out, runner.buffer(rt.BUF_INTER_CODES)[: tokens * TOP_K * INTER // 2].clone()))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert results[0][0].float().abs().max() > 0
+
+
 def ids_with_counts(tokens, counts):
     """Expert ids in which expert e has counts[e] tokens, exactly; the other experts share the rest."""
     counts = list(counts) + [0] * (EXPERTS - len(counts))
