@@ -261,19 +261,22 @@ __device__ __forceinline__ bool grid_barrier(int* sync, int ctas, int* status) {
 // Either way every CTA has its own base then (the group geometry is written by all of them with identical values) and
 // scatters its routes.  Cooperative and alone, same box, us a pass: 613 tokens 198.3 -> 191.9 (two layers), 1000 tokens 244.3 -> 237.5, 1500
 // tokens 267.4 -> 262, feed-forward layers of 300 tokens 331 -> 322 (three), 1024 tokens 323.5 -> 313.5 (two), 1500 tokens 383.7 -> 379.2.
-// The line is where it still paid when it was drawn.  Around it, with the kernels of today, two layers called from Python and two feed-forward layers:
-// 1536 tokens 276 -> 270 and 354 -> 347, 1664 281 -> 275 and 372 -> 360, 1792 295 -> 291 and 385 -> 377, 1920 308 -> 305 and 403 -> 404, 2048 328 -> 322 and
-// 427 -> 426 (in graphs half of that and less): up to fifteen chunks would gain, too.
-constexpr int kSortAloneChunks = 12;
+// The line, against twelve chunks and 33 KB of shared memory (25 now: the CTAs of larger batches find room beside the dense MLP's sooner), us a pass: two layers of
+// 1700 tokens 278.1 -> 274.5, 2048 313.6 -> 311.6, one of 2500 178.9 -> 177.3, 3072 207.7 -> 206.0; two feed-forward layers of 1800 tokens 393.0 -> 390.6, 2048
+// 426.8 -> 424.8, one of 3072 273.9 -> 270.8, 4096 (which meets) 355.2 -> 351.2.  A layer of 4096 tokens alone 243.2 -> 246.7: counting has become the longer way.
+constexpr int kSortAloneChunks = 24;
 __global__ void __launch_bounds__(kSortChunk)
 route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chunks, bool alone, RoutePlan plan) {
-  constexpr int kCopies = 16;  // of the counts of other chunks, so that fewer warps meet at a counter
+  constexpr int kCopies = 8;   // of the counts of other chunks, so that fewer warps meet at a counter
+  constexpr int kAtOnce = 16;  // other chunks' histograms
   __shared__ int warp_counts[32 * kExperts];
-  __shared__ int fetched[32 * kExperts];  // alone: [before this chunk, behind it][copy][expert]
+  __shared__ int fetched[kAtOnce * kExperts];  // alone: [before this chunk, behind it][copy][expert]
+  static_assert(2 * kCopies <= kAtOnce, "both uses of `fetched`");
   __shared__ int remapped[kExperts];
   __shared__ int scan_scratch[16];
   const int tid = threadIdx.x;
-  for (int i = tid; i < 32 * kExperts; i += kSortChunk) warp_counts[i] = fetched[i] = 0;
+  for (int i = tid; i < 32 * kExperts; i += kSortChunk) warp_counts[i] = 0;
+  for (int i = tid; i < kAtOnce * kExperts; i += kSortChunk) fetched[i] = 0;
   __syncthreads();
   grid_dependency_wait();  // the ids are written, and the plan's last readers are done
   grid_launch_dependents();  // after the wait: whoever starts now may read what came before this kernel
@@ -330,11 +333,11 @@ route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chun
     if (tid < kExperts) plan.chunk_hist[chunk * kExperts + tid] = total;
     total = 0;
     if (!grid_barrier(plan.sync, chunks, plan.status)) return;
-    // All chunk histograms, 32 chunks at a time: the whole CTA fetches them in one round of loads
+    // All chunk histograms, 16 chunks at a time: the whole CTA fetches them in one round of loads
     // (128 threads walking them chunk by chunk is a chain of trips to L2), then expert `tid` adds
     // its column from shared memory.
-    for (int first = 0; first < chunks; first += 32) {
-      const int count = chunks - first < 32 ? chunks - first : 32;
+    for (int first = 0; first < chunks; first += kAtOnce) {
+      const int count = chunks - first < kAtOnce ? chunks - first : kAtOnce;
       for (int i = tid; i < count * kExperts; i += kSortChunk) fetched[i] = __ldcg(&plan.chunk_hist[first * kExperts + i]);
       __syncthreads();
       if (tid < kExperts) {

@@ -225,6 +225,22 @@ def test_route_sort_at_the_edges_of_its_forms(gm, oracle, big_runner, cuda_devic
         assert (got[key] == want[key]).all(), key
 
 
+@pytest.mark.parametrize("tokens", [2047, 2049, 3071, 3072, 3073, 4095, 4096])
+def test_route_sort_around_its_longest_counts(gm, oracle, big_runner, cuda_device, tokens):
+    """The line lies at 24 chunks, and CTAs that meet read sixteen chunks' counts at a time: both sides of either, with experts that a
+    token names twice and one that takes a route of every token."""
+    from gevva_b200 import runtime as rt
+    ids = random_ids(tokens, 7 + tokens)
+    ids[::5, 6] = ids[::5, 1]
+    ids[:, 3] = 99
+    big_runner.launch_stages(rt.STAGE_SORT, tokens, expert_ids=torch.from_numpy(ids).to(cuda_device))
+    assert big_runner.last_status() == 0
+    got = plan_arrays(gm, big_runner, tokens * TOP_K)
+    want = oracle.sort(ids)
+    for key in ("sorted_experts", "sorted_routes", "inverse", "offsets", "scale_rows"):
+        assert (got[key] == want[key]).all(), key
+
+
 @pytest.mark.parametrize("tokens", [128, 129, 300, 1535, 1536, 1537])
 def test_route_sort_by_owner_at_one_rank(gm, varied_weights, cuda_device, tokens):
     """Expert-parallel ranks sort by the key that a placement table gives each expert: one rank alone, whose table is a permutation
