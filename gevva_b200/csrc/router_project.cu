@@ -32,10 +32,12 @@ namespace {
 // CTAs per cluster = K slices per token tile: 8 for small batches, else 4, 2 or 1, the largest that
 // keeps the launch within one wave of SMs (a tile's pass is a chain of latencies, so waves cost more
 // than depth)
-// Epilogue warps.  64 rows keep eight busy (four -> eight, us alone: 37 tokens 5.9 -> 5.5, 64 6.7 -> 6.4, 613 9.0 -> 8.2, 1024 9.2 -> 8.4,
+// Epilogue warps.  CTAs of 128-row tiles that keep 64 or 128 rows for themselves route them four lanes a row in one pass of sixteen warps
+// (four -> sixteen, us alone: 6000 tokens 15.8 -> 14.6, 8192 16.9 -> 15.7, 12000 25.3 -> 22.0, 16384 28.5 -> 25.2; a layer of 16384 tokens 793 -> 777; with 32 rows,
+// up to 4608 tokens, 12.2 -> 12.5 at 4096).  64 rows keep eight busy (four -> eight, us alone: 37 tokens 5.9 -> 5.5, 64 6.7 -> 6.4, 613 9.0 -> 8.2, 1024 9.2 -> 8.4,
 // 2048 10.0 -> 9.1); with fewer rows eight are 0.1 slower than four.
-template <int kRows> constexpr int kRpEpilogueWarps = kRows == 64 ? 8 : 4;
-template <int kRows> constexpr int kRpThreads = (2 + kRpEpilogueWarps<kRows>) * 32;
+template <int kRows, int kSplit> constexpr int kRpEpilogueWarps = kRows == 64 ? 8 : kRows == 128 && kSplit <= 2 ? 16 : 4;
+template <int kRows, int kSplit> constexpr int kRpThreads = (2 + kRpEpilogueWarps<kRows, kSplit>) * 32;
 // Rows of a tile.  In batches of up to 2048 tokens the launch is a chain of latencies, and the fewer rows a cluster has, the fewer partial sums
 // each CTA has to send, reduce and route.  128 -> 64 rows, us alone: 9.7 -> 6.8 at 128 and 200 tokens, 10.2 -> 7.6 at 512, 10.2 -> 9.3 at 1024, 10.5 -> 9.7
 // at 2048; above, the clusters no longer run all at once (2368 tokens: 11.0 against 17.3).  64 -> 32 rows: 37 tokens 5.5 -> 5.2, 64 6.2 -> 5.4,
@@ -45,14 +47,19 @@ template <int kRows> constexpr int kRpThreads = (2 + kRpEpilogueWarps<kRows>) * 
 // The K split, which decides the order of the sums, depends on the number of 128-row tiles either way.
 constexpr int kSmallTile = 64, kSmallTileTokens = 2048;
 constexpr int tile_rows(int tokens) { return tokens <= 64 ? 16 : tokens <= 400 ? 32 : tokens <= kSmallTileTokens ? kSmallTile : kTileM; }
-template <int kRows> constexpr int kWarpRows = 2 * kRpEpilogueWarps<kRows>;  // rows of a CTA up to which a warp routes a row (two each); above, a quad of lanes does
+template <int kRows, int kSplit> constexpr int kWarpRows = 2 * kRpEpilogueWarps<kRows, kSplit>;  // rows of a CTA up to which a warp routes a row (two each); above, a quad of lanes does
+// 128-row tiles whose clusters of four, or of two, all run at once on 148 SMs (a CTA fills an SM, and a cluster lies within a GPC).  With more, half as many
+// CTAs a tile sum two slices of K each, so that the sums stay the same up to the number of tiles from which K has fewer slices (a second wave of the clusters
+// before, us alone: 4352 tokens 21.3 -> 15.8, 5120 21.8 -> 16.0, 9600 29.9 -> 24.6; a layer of 4700 tokens 283.9 -> 280.3, of 10000 492.5 -> 485.3).
+constexpr int kTilesOfFour = 33, kFourSlicesTiles = 40, kTilesOfTwo = 74, kTwoSlicesTiles = 80;
 constexpr int kRpTileBytes = kTileM * kTileKBytes;  // 16 KiB: 128 rows of one 128-byte K block
 
 // kRows: token rows of a tile.  Below 128, with eight CTAs a tile, the five or six K blocks of each all fit the ring; the MMA, whose
 // M is 128, reads what lies behind the tile (always inside this structure) as its further rows, whose results nobody looks at.
-template <int kRows>
+// kSlices: K slices of a CTA, summed up for themselves.
+template <int kRows, int kSlices>
 struct alignas(1024) RouterSmem {
-  static constexpr int kStages = kRows <= 64 ? 6 : 5;
+  static constexpr int kStages = kRows <= 64 ? 6 : kSlices == 1 ? 5 : 3;
   static constexpr int kTokenBytes = kRows * kTileKBytes;
   uint8_t a[kStages][kTokenBytes];
   uint8_t b[kStages][kRpTileBytes];
@@ -60,10 +67,10 @@ struct alignas(1024) RouterSmem {
   // [source][local row][128 floats]; the 16-byte chunks of a row are permuted
   // (received_chunk_position) so that neither the row-wise stores nor the reduce's reads, where
   // four lanes share a row, meet in a bank.
-  float received[kRows * kExperts];   // [kSplit][kRows / kSplit rows][128 floats]
+  float received[kSlices * kRows * kExperts];   // [kSplit * kSlices][kRows / kSplit rows][128 floats]
   uint64_t full[kStages];
   uint64_t empty[kStages];
-  uint64_t acc_full;
+  uint64_t acc_full[kSlices];
   uint32_t tmem_base;
   volatile int abort;
   __nv_bfloat16 expert_scale[kExperts];
@@ -77,8 +84,9 @@ __device__ __forceinline__ int received_chunk_position(int chunk, int row) {
   return chunk ^ ((row + 2 * (chunk >> 3)) & 7);
 }
 
-template <int kRows> constexpr size_t router_smem_bytes() { return sizeof(RouterSmem<kRows>) + 1024; }
-static_assert(router_smem_bytes<64>() <= 232448 && router_smem_bytes<128>() <= 232448, "shared memory budget of one sm_100 CTA");
+template <int kRows, int kSlices> constexpr size_t router_smem_bytes() { return sizeof(RouterSmem<kRows, kSlices>) + 1024; }
+static_assert(router_smem_bytes<64, 1>() <= 232448 && router_smem_bytes<128, 1>() <= 232448 && router_smem_bytes<128, 2>() <= 232448,
+              "shared memory budget of one sm_100 CTA");
 
 struct RouterParams {
   const float* bias;                   // optional f32 [128], added before the bf16 rounding
@@ -129,11 +137,11 @@ __device__ __forceinline__ void issue_router_k_block(uint32_t tmem_acc, uint32_t
 #undef GV_RP_MMA
 }
 
-template <bool kFp8, int kSplit, int kRows>
-__global__ void __launch_bounds__(kRpThreads<kRows>, 1)
+template <bool kFp8, int kSplit, int kRows, int kSlices>
+__global__ void __launch_bounds__(kRpThreads<kRows, kSplit>, 1)
 route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                      const RouterParams p) {
-  using Smem = RouterSmem<kRows>;
+  using Smem = RouterSmem<kRows, kSlices>;
   constexpr int kRpStages = Smem::kStages;
   extern __shared__ uint8_t smem_raw[];
   Smem* smem = reinterpret_cast<Smem*>(
@@ -143,22 +151,24 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   const uint32_t rank = cluster_cta_rank();
   constexpr int kOwnRows = kRows / kSplit;   // tile rows this CTA reduces and routes
   const int m_tile = static_cast<int>(blockIdx.x) / kSplit;
-  const int kb_begin = static_cast<int>(rank) * p.k_blocks / kSplit;
-  const int kb_end = (static_cast<int>(rank) + 1) * p.k_blocks / kSplit;
+  constexpr int kSources = kSplit * kSlices;
+  const int slice0 = static_cast<int>(rank) * kSlices;
+  const int kb_begin = slice0 * p.k_blocks / kSources;
+  const int kb_end = (slice0 + kSlices) * p.k_blocks / kSources;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kRpStages; ++s) {
       mbar_init(&smem->full[s], 1);
       mbar_init(&smem->empty[s], 1);
     }
-    mbar_init(&smem->acc_full, 1);
+    for (int s = 0; s < kSlices; ++s) mbar_init(&smem->acc_full[s], 1);
     smem->abort = 0;
     fence_barrier_init();
     prefetch_tensor_map(&map_x);
     prefetch_tensor_map(&map_w);
   }
   if (warp == 1) {
-    tmem_alloc(&smem->tmem_base, kExperts);
+    tmem_alloc(&smem->tmem_base, kSlices * kExperts);
     tmem_relinquish();
   }
   // The next kernel of the stream (launched with programmatic serialization) may take its place on
@@ -217,14 +227,21 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const uint32_t a_lo0 = (smem_u32(smem->a[0]) & 0x3ffffu) >> 4;
     const uint32_t b_lo0 = (smem_u32(smem->b[0]) & 0x3ffffu) >> 4;
     const bool leader = elect_one();
+    int slice = 0;
+    bool fresh = true;  // the slice's first K block
     for (int kb = kb_begin; kb < kb_end; ++kb) {
       if (!wait_or_abort(&smem->full[stage], phase, smem, p.status)) break;
       if (leader) {
-        issue_router_k_block<kFp8>(tmem_base, a_lo0 + static_cast<uint32_t>(stage) * (Smem::kTokenBytes >> 4),
+        issue_router_k_block<kFp8>(tmem_base + static_cast<uint32_t>(slice) * kExperts, a_lo0 + static_cast<uint32_t>(stage) * (Smem::kTokenBytes >> 4),
                                    b_lo0 + static_cast<uint32_t>(stage) * (kRpTileBytes >> 4),
-                                   kb != kb_begin ? 1u : 0u);
+                                   fresh ? 0u : 1u);
         tc_commit(&smem->empty[stage]);
-        if (kb + 1 == kb_end) tc_commit(&smem->acc_full);
+      }
+      fresh = false;
+      if (kb + 1 == (slice0 + slice + 1) * p.k_blocks / kSources) {
+        if (leader) tc_commit(&smem->acc_full[slice]);
+        ++slice;
+        fresh = true;
       }
       if (++stage == kRpStages) {
         stage = 0;
@@ -236,7 +253,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     // (the per-expert scale, which part 2 would otherwise look up behind its last comparison)
     if (threadIdx.x - 64 < kExperts) smem->expert_scale[threadIdx.x - 64] = p.expert_scale[threadIdx.x - 64];
     const int quarter = warp & 3;  // the tensor-memory lanes this warp may read
-    constexpr int kParts = 4 / (kRpEpilogueWarps<kRows> / 4);  // the columns of a row are shared by the quarter's warps
+    constexpr int kParts = 4 / (kRpEpilogueWarps<kRows, kSplit> / 4);  // the columns of a row are shared by the quarter's warps
     const int first_part = (warp - 2) / 4 * kParts;
     const int row = quarter * 32 + lane;
     const int owner = row % kSplit;
@@ -245,15 +262,17 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     // tensor-memory loads are warp-wide, so a warp takes part if any of its 32 rows exists
     const bool row_exists = row < kRows && m_tile * kRows + row < p.tokens;
     const bool warp_has_rows = quarter * 32 < kRows && m_tile * kRows + quarter * 32 < p.tokens;
-    if (wait_or_abort(&smem->acc_full, 0, smem, p.status) && warp_has_rows) {
+#pragma unroll 1
+    for (int slice = 0; slice < kSlices; ++slice) {
+      if (!wait_or_abort(&smem->acc_full[slice], 0, smem, p.status) || !warp_has_rows) break;
       tc_fence_after_sync();
       const uint32_t remote_row =
-          cluster_map_shared(smem_u32(smem->received + (rank * kOwnRows + owner_row) * kExperts),
+          cluster_map_shared(smem_u32(smem->received + ((slice0 + slice) * kOwnRows + owner_row) * kExperts),
                              static_cast<uint32_t>(owner));
 #pragma unroll 1
       for (int part = first_part; part < first_part + kParts; ++part) {
         uint32_t r[32];
-        tmem_load_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 32, r);
+        tmem_load_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + slice * kExperts + part * 32, r);
         tmem_load_wait();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -273,19 +292,19 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   cluster_sync_all();
 
   if (warp >= 2 && !smem->abort) {
-    // ---------------- epilogue, part 2: reduce this CTA's rows and route them, 32 at a time ----------------
+    // ---------------- epilogue, part 2: reduce this CTA's rows and route them ----------------
     const int tile_rows = p.tokens - m_tile * kRows;   // may exceed the tile
     // rows kSplit * i + rank < tile_rows
     const int own_rows = tile_rows >= kRows ? kOwnRows : (tile_rows - static_cast<int>(rank) + kSplit - 1) / kSplit;
-    constexpr int kWarps = kRpEpilogueWarps<kRows>;
-    const bool few = kOwnRows <= kWarpRows<kRows> || own_rows <= kWarpRows<kRows>;
+    constexpr int kWarps = kRpEpilogueWarps<kRows, kSplit>;
+    const bool few = kOwnRows <= kWarpRows<kRows, kSplit> || own_rows <= kWarpRows<kRows, kSplit>;
     if (few) {
       // a few rows: one warp per row, four logits a lane (a third of the quads' chain)
       for (int row_local = warp - 2; row_local < own_rows; row_local += kWarps) {
         const int token = m_tile * kRows + row_local * kSplit + static_cast<int>(rank);
         float4 acc = make_float4(0, 0, 0, 0);
 #pragma unroll
-        for (int source = 0; source < kSplit; ++source) {
+        for (int source = 0; source < kSources; ++source) {
           const float4 v = reinterpret_cast<const float4*>(
               smem->received + (source * kOwnRows + row_local) * kExperts)[received_chunk_position(lane, row_local)];
           acc = source == 0 ? v
@@ -304,19 +323,17 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                         p.ids + static_cast<size_t>(token) * kTopK);
       }
     }
-    if constexpr (kOwnRows > kWarpRows<kRows>) if (!few) {
-    static_assert(kOwnRows % 32 == 0 && kWarps == 4, "128-row tiles: whole passes of 32 rows by all epilogue threads");
+    if constexpr (kOwnRows > kWarpRows<kRows, kSplit>) if (!few) {
+    static_assert(kOwnRows % 8 == 0 && kOwnRows <= 8 * kWarps, "128-row tiles: a row for every four lanes, in one pass");
     const int t = threadIdx.x - 64;
     const int part = t & 3;         // columns [32 * part, 32 * part + 32)
-#pragma unroll 1
-    for (int pass = 0; pass < kOwnRows / 32; ++pass) {
-      if (m_tile * kRows + pass * 32 * kSplit >= p.tokens) break;   // no row of this pass exists
-      const int row_local = pass * 32 + (t >> 2);   // tile row kSplit * row_local + rank
+    if (8 * (warp - 2) < kOwnRows && 8 * (warp - 2) < own_rows) {
+      const int row_local = t >> 2;   // tile row kSplit * row_local + rank
       const int token = m_tile * kRows + row_local * kSplit + static_cast<int>(rank);
       const bool valid = token < p.tokens;
       float4 acc[8];
 #pragma unroll
-      for (int source = 0; source < kSplit; ++source) {
+      for (int source = 0; source < kSources; ++source) {
         const float4* source_row =
             reinterpret_cast<const float4*>(smem->received + (source * kOwnRows + row_local) * kExperts);
 #pragma unroll
@@ -368,11 +385,11 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   if (warp == 1) {
     tc_fence_after_sync();
     __syncwarp();
-    tmem_dealloc(tmem_base, kExperts);
+    tmem_dealloc(tmem_base, kSlices * kExperts);
   }
 }
 
-template <bool kFp8, int kSplit, int kRows>
+template <bool kFp8, int kSplit, int kRows, int kSlices = 1>
 cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, const RouterParams& p,
                            cudaStream_t stream) {
   static bool prepared[64] = {};
@@ -380,16 +397,16 @@ cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, c
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return e;
   if (device >= 0 && device < 64 && !prepared[device]) {
-    e = cudaFuncSetAttribute(route_project_kernel<kFp8, kSplit, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(router_smem_bytes<kRows>()));
+    e = cudaFuncSetAttribute(route_project_kernel<kFp8, kSplit, kRows, kSlices>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(router_smem_bytes<kRows, kSlices>()));
     if (e != cudaSuccess) return e;
     prepared[device] = true;
   }
   const int m_tiles = (p.tokens + kRows - 1) / kRows;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(m_tiles * kSplit));
-  config.blockDim = dim3(kRpThreads<kRows>);
-  config.dynamicSmemBytes = router_smem_bytes<kRows>();
+  config.blockDim = dim3(kRpThreads<kRows, kSplit>);
+  config.dynamicSmemBytes = router_smem_bytes<kRows, kSlices>();
   config.stream = stream;
   // Clusters of kSplit CTAs; and the launch may begin while the previous kernel of the stream is
   // still running (the kernel waits at grid_dependency_wait before it reads or writes global memory),
@@ -403,7 +420,7 @@ cudaError_t launch_variant(const CUtensorMap& map_x, const CUtensorMap& map_w, c
   attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = 2;
-  return cudaLaunchKernelEx(&config, route_project_kernel<kFp8, kSplit, kRows>, map_x, map_w, p);
+  return cudaLaunchKernelEx(&config, route_project_kernel<kFp8, kSplit, kRows, kSlices>, map_x, map_w, p);
 }
 
 template <bool kFp8>
@@ -415,8 +432,10 @@ cudaError_t launch_split(const CUtensorMap& map_x, const CUtensorMap& map_w, con
   if (tile == 32) return launch_variant<kFp8, 8, 32>(map_x, map_w, p, stream);
   if (m_tiles <= 4) return launch_variant<kFp8, 8, kSmallTile>(map_x, map_w, p, stream);
   if (tile == kSmallTile) return launch_variant<kFp8, 4, kSmallTile>(map_x, map_w, p, stream);
-  if (m_tiles * 4 <= 160) return launch_variant<kFp8, 4, kTileM>(map_x, map_w, p, stream);
-  if (m_tiles * 2 <= 160) return launch_variant<kFp8, 2, kTileM>(map_x, map_w, p, stream);
+  if (m_tiles <= kTilesOfFour) return launch_variant<kFp8, 4, kTileM>(map_x, map_w, p, stream);
+  if (m_tiles <= kFourSlicesTiles) return launch_variant<kFp8, 2, kTileM, 2>(map_x, map_w, p, stream);
+  if (m_tiles <= kTilesOfTwo) return launch_variant<kFp8, 2, kTileM>(map_x, map_w, p, stream);
+  if (m_tiles <= kTwoSlicesTiles) return launch_variant<kFp8, 1, kTileM, 2>(map_x, map_w, p, stream);
   return launch_variant<kFp8, 1, kTileM>(map_x, map_w, p, stream);
 }
 

@@ -132,6 +132,16 @@ def test_router_tiles_of_16_and_32_rows(cuda_device, rows, fp8):
     test_router_tiles_of_few_rows(cuda_device, rows, 512, fp8)
 
 
+@pytest.mark.parametrize("rows,of", [(2049, 4224), (4223, 4224), (4224, 4225), (4224, 4353), (4224, 5120), (5121, 9472), (9471, 9472),
+                                     (9472, 9473), (9472, 10240), (10241, 10368)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_router_tiles_of_128_rows(cuda_device, rows, of, fp8):
+    """128-row tiles split over four CTAs (up to 33 tiles) or over two that sum two slices each (up to 40), over two (up to 74) or one that sums
+    two slices (up to 80), or by one CTA, which route their rows a warp a row or four lanes a row, whole and ragged at either side of
+    the lines: the rows of a larger batch with the same slices of K, bit by bit."""
+    test_router_tiles_of_few_rows(cuda_device, rows, of, fp8)
+
+
 def test_router_projection_feeds_the_layer(oracle, cuda_device):
     """The fused router in front of the expert runner: the layer step made of C-ABI calls only."""
     import gevva_b200 as gm
