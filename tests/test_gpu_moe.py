@@ -717,6 +717,30 @@ def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_devic
     assert results[0][0].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("tokens,counts", [
+    (2600, [1, 127, 128, 129, 255, 256, 257, 383, 384, 385, 511, 512, 513, 640, 641, 768, 769, 1023, 1024, 1025, 1281]),
+    (2600, [600, 0, 513] * 8), (4096, [256] * EXPERTS), (4096, [2561, 513, 300])])
+def test_w2_shares_weights_between_pairs(gm, weights, cuda_device, tokens, counts):
+    """w2 by CTA pairs takes an expert's pairs of row tiles two by two against the same weights and deals out what does not fill a round of
+    units in thirds: experts of one to eleven tiles, with and without a pair left over, against the kernel that shares
+    weight tiles in another way."""
+    from gevva_b200 import runtime as rt
+    dev_ids = torch.from_numpy(ids_with_counts(tokens, counts)).to(cuda_device)
+    x = hashgen.activations(tokens, HIDDEN, 85, cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    results = []
+    for pairs in (True, False):
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens, pairs=pairs)
+        out = torch.zeros_like(x)
+        for _ in range(2):
+            runner.launch_batch(x, dev_ids, rw, out, tokens)
+        runner.check()
+        results.append((out, runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].clone()))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert results[0][0].float().abs().max() > 0
+
+
 @pytest.mark.parametrize("tokens", [297, 640, 641, 1536, 1537])
 def test_weights_asked_ahead_change_no_result(gm, weights, cuda_device, tokens):
     """From 297 to 1536 tokens the quantiser of a whole call asks for the experts' first weights, shared out over its CTAs; called
