@@ -8,7 +8,7 @@
 // where one CTA fetches 103 (1024 tokens 36.2 -> 42.4).  Eight epilogue warps and stores without a cache hint make no difference.
 // Two pairs of an expert share the weights, too: each weight stage is used by both, one after the other, and an item fetches 42 KB instead of 59.  (Loads and
 // stores share the fabric: 48 KB stored and 64 KB loaded an item and SM take 1.45 us with everything in L2, either alone 1.0; the kernel took 1.6 at 16384
-// tokens.)  And what does not fill a round of units is dealt out in thirds of them.  Alone, us, without both -> with: 2600 tokens 53.0 -> 50.4, 4096 67.3 -> 65.0, 8192
+// tokens.)  And what does not fill a round of units is dealt out in thirds of them.  Alone, us, without both -> with: 2600 tokens 53.0 -> 50.4, 4096 67.3 -> 64.0, 8192
 // 109.6 -> 108.8, 16384 197.5 -> 191.5; without the thirds 53.2, 65.0, 109.8 and 195; 4096 of uneven loads 69.7 -> 68.6 (without thirds 72.4), Zipf(1.1) 77.2 -> 77.3.
 // Everything else is as in that file, whose column order, re-tiled scales and schedule this one shares: items of 192 columns, a unit
 // five of one pair (three there: 2 % more at 16384 tokens) or three of two, a tile's activations fetched once a unit, two accumulators, results stored from registers.  The last tile of an expert
@@ -113,9 +113,9 @@ struct DownPairSchedule {
     const int clusters = static_cast<int>(gridDim.x) >> 1, mine = static_cast<int>(blockIdx.x) >> 1;
     const int index = round * clusters + ((round & 1) ? clusters - 1 - mine : mine);
     ++round;
-    // What does not fill a round is dealt out in thirds of a unit, so that the last clusters end nearer to one another.
+    // What does not fill a round is dealt out in thirds of a unit where that makes the last clusters' way shorter.
     const int units = smem->units[kExperts], whole = units / clusters * clusters;
-    const int over = index - whole, third = over % 3, number = over < 0 ? index : whole + over / 3;
+    const int over = 3 * (units - whole) <= 2 * clusters ? index - whole : -1, third = over % 3, number = over < 0 ? index : whole + over / 3;
     if (number >= units) return false;  // only the last round is incomplete
     int expert = 0;  // the last one with units[expert] <= number
 #pragma unroll
