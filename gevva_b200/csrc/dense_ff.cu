@@ -338,6 +338,54 @@ __device__ __forceinline__ void words(const uint4& v, uint32_t (&out)[4]) {
   out[3] = v.w;
 }
 
+// ff_prepare_kernel for more rows than its CTAs that run at once: a CTA keeps the three weights for row after row and asks for the next one under this one's
+// arithmetic, which is done on pairs.  The same results.  Alone, us, a block a row and this: 640 rows 5.25 and 4.55, 1024 7.5 and 6.0, 2048 12.8
+// and 10.1, 4096 23.5 and 18.3 (two or four CTAs an SM 20.7 and 21.8); feed-forward layers of 2048 tokens 443.1 and 441.9 (two), 3000 276.8 and 275.2, 4096 362.4
+// and 358.3.  With a row a CTA it is the slower one (64 rows 2.03 and 2.14; three layers of 301 tokens 314.6 and 316.4).
+constexpr int kPrepareCtas = 3 * 148;  // three an SM
+
+__global__ void __launch_bounds__(kRowThreads, 3)
+ff_prepare_rows_kernel(const __nv_bfloat16* __restrict__ input, const __nv_bfloat16* __restrict__ dense_weight,
+                  const __nv_bfloat16* __restrict__ expert_weight,
+                  const __nv_bfloat16* __restrict__ router_scale, __nv_bfloat16* __restrict__ dense_out,
+                  __nv_bfloat16* __restrict__ expert_out, __nv_bfloat16* __restrict__ router_out, int rows) {
+  __shared__ float sums[2][kRowWarps];
+  grid_launch_dependents();
+  uint32_t dw[4], ew[4], rs[4];
+  grid_dependency_wait();
+  const uint4* const in = reinterpret_cast<const uint4*>(input) + threadIdx.x;
+  int row = blockIdx.x;
+  uint4 raw = __ldg(in + static_cast<size_t>(row) * (kHidden / 8));
+  words(__ldg(reinterpret_cast<const uint4*>(dense_weight) + threadIdx.x), dw);
+  words(__ldg(reinterpret_cast<const uint4*>(expert_weight) + threadIdx.x), ew);
+  words(__ldg(reinterpret_cast<const uint4*>(router_scale) + threadIdx.x), rs);
+  const float root = gv_rsqrtf(static_cast<float>(kHidden));
+#pragma unroll 1
+  for (int turn = 0; row < rows; turn ^= 1) {
+    uint32_t x[4];
+    words(raw, x);
+    const int next = row + static_cast<int>(gridDim.x);
+    if (next < rows) raw = __ldg(in + static_cast<size_t>(next) * (kHidden / 8));
+    const float warp_sum = warp_sum_squares_of(x);
+    if ((threadIdx.x & 31) == 0) sums[turn][threadIdx.x >> 5] = warp_sum;
+    __syncthreads();  // (the other turn's sums have been read by all: one barrier a row is enough)
+    const float inverse = inverse_rms(fold_warps(sums[turn]));
+    uint32_t d[4], e[4], r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const unsigned long long normalized = mul2(two_of(x[i]), two(inverse, inverse));
+      d[i] = round2(mul2(normalized, two_of(dw[i])));
+      e[i] = round2(mul2(normalized, two_of(ew[i])));
+      r[i] = round2(mul2(two_of(round2(mul2(two_of(round2(normalized)), two_of(rs[i])))), two(root, root)));
+    }
+    const size_t at = static_cast<size_t>(row) * (kHidden / 8) + threadIdx.x;
+    reinterpret_cast<uint4*>(dense_out)[at] = uint4{d[0], d[1], d[2], d[3]};
+    reinterpret_cast<uint4*>(expert_out)[at] = uint4{e[0], e[1], e[2], e[3]};
+    reinterpret_cast<uint4*>(router_out)[at] = uint4{r[0], r[1], r[2], r[3]};
+    row = next;
+  }
+}
+
 __global__ void __launch_bounds__(kRowThreads, 3)
 ff_finalize_kernel(const __nv_bfloat16* __restrict__ dense, const __nv_bfloat16* __restrict__ dense_weight,
                    const __nv_bfloat16* __restrict__ expert_routes, const float* __restrict__ route_weights,
@@ -436,6 +484,13 @@ void launch_ff_prepare(const void* input, const void* dense_weight, const void* 
                        const void* router_scale, void* dense_out, void* expert_out, void* router_out,
                        int rows, cudaStream_t stream) {
   using B = __nv_bfloat16;
+  if (rows > kPrepareCtas) {
+    launch_chained(ff_prepare_rows_kernel, dim3(kPrepareCtas), dim3(kRowThreads), 0, stream, static_cast<const B*>(input),
+                   static_cast<const B*>(dense_weight), static_cast<const B*>(expert_weight),
+                   static_cast<const B*>(router_scale), static_cast<B*>(dense_out), static_cast<B*>(expert_out),
+                   static_cast<B*>(router_out), rows);
+    return;
+  }
   launch_chained(ff_prepare_kernel, dim3(rows), dim3(kRowThreads), 0, stream, static_cast<const B*>(input),
                  static_cast<const B*>(dense_weight), static_cast<const B*>(expert_weight),
                  static_cast<const B*>(router_scale), static_cast<B*>(dense_out), static_cast<B*>(expert_out),

@@ -43,6 +43,12 @@ def test_ff_prepare_bit_exact(dense_oracle, cuda_device, rows):
         assert (bits(g) == w).all(), name
 
 
+@pytest.mark.parametrize("rows", [444, 445, 888, 889, 1500])
+def test_ff_prepare_row_after_row(dense_oracle, cuda_device, rows):
+    """From 445 rows on a CTA takes row after row: one, two and more rows a CTA, whole and ragged."""
+    test_ff_prepare_bit_exact(dense_oracle, cuda_device, rows)
+
+
 def test_pack_fp8_matches_oracle(dense_oracle, cuda_device):
     from gevva_b200 import feedforward as ff
     w = hashgen.expert_weights_chunk(0, 1, 256, HIDDEN, 33, cuda_device)[0]
