@@ -76,13 +76,13 @@ int gv::dense_launch_on(gevva_dense* d, const void* in, void* out_unscaled, int 
   }
   gv::RoutePlan plan = d->plan;
   plan.status = status;
-  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, plan, stream);
   // By CTA pairs where the MLP has all SMs (figures in dense_gemm_pair.cu).  On the few that it gets beside the experts, whose weight
   // stream bounds the layer, the one-CTA kernels are as fast or faster: whole layers in a graph 16 tokens 264.8 and 266.6 us by pairs, 40 tokens
   // 337 and 343, 301 tokens 321 and 322, 640 tokens 363.5 and 366.
   // The pair kernel stores 32 bytes at a time; rows are whole multiples of that, so an output that is aligned to 16 only, as the
   // one-CTA kernel takes it, goes there (same bits; the MLP takes 54.4 us instead of 46.5 then at 2048 tokens, 27.4 instead of 24.6 at 301).
   const bool pairs = sm_count >= 2 && sm_count == d->sm_count;
+  gv::launch_fp8_quantize_rows(in, d->act_fp8, d->act_scales, tokens, pairs, plan, stream);
   const auto project = [&](gv::GemmOperands op) {
     if (pairs && (reinterpret_cast<uintptr_t>(op.out) & 31) == 0) {
       gv::launch_dense_pairs(op, tokens, status, sm_count, stream);

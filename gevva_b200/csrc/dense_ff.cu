@@ -131,13 +131,16 @@ __device__ __forceinline__ uint32_t abs_max_pair(uint32_t a, uint32_t b) {
   return *reinterpret_cast<const uint32_t*>(&m);
 }
 
+// weights_ahead: the kernel behind this asks for its weights without waiting for it, so it may start only once what came before this has
+// completed (the weights may come from there).
 __global__ void __launch_bounds__(kRowThreads)
 fp8_quantize_rows_kernel(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ out,
-                         float* __restrict__ scales, int rows, RoutePlan plan) {
+                         float* __restrict__ scales, int rows, bool weights_ahead, RoutePlan plan) {
   __shared__ float scratch[kRowWarps];
   __shared__ int scan_scratch[16];
-  grid_launch_dependents();
+  if (!weights_ahead) grid_launch_dependents();
   grid_dependency_wait();
+  if (weights_ahead) grid_launch_dependents();
   // the projections are grouped GEMMs with a single "expert" that owns every row: their plan
   if (blockIdx.x == 0 && threadIdx.x < kExperts) publish_groups(threadIdx.x == 0 ? rows : 0, rows, plan, scan_scratch);
   const size_t base = static_cast<size_t>(blockIdx.x) * kHidden;
@@ -162,10 +165,11 @@ constexpr int kLaneVectors = kRowThreads / 32;  // 11 vectors of 8 columns a lan
 
 __global__ void __launch_bounds__(kWarpRows * 32)
 fp8_quantize_warp_rows_kernel(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ out,
-                              float* __restrict__ scales, int rows, RoutePlan plan) {
+                              float* __restrict__ scales, int rows, bool weights_ahead, RoutePlan plan) {
   __shared__ int scan_scratch[16];
-  grid_launch_dependents();
+  if (!weights_ahead) grid_launch_dependents();
   grid_dependency_wait();
+  if (weights_ahead) grid_launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x < kExperts) publish_groups(threadIdx.x == 0 ? rows : 0, rows, plan, scan_scratch);
   const int row = blockIdx.x * kWarpRows + threadIdx.x / 32, lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -497,15 +501,15 @@ void launch_ff_prepare(const void* input, const void* dense_weight, const void* 
                  static_cast<B*>(router_out));
 }
 
-void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows, const RoutePlan& plan,
+void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows, bool weights_ahead, const RoutePlan& plan,
                               cudaStream_t stream) {
   if (rows >= 1024) {  // figures above the kernel
     launch_chained(fp8_quantize_warp_rows_kernel, dim3((rows + kWarpRows - 1) / kWarpRows), dim3(kWarpRows * 32), 0, stream,
-                   static_cast<const __nv_bfloat16*>(input), out, scales, rows, plan);
+                   static_cast<const __nv_bfloat16*>(input), out, scales, rows, weights_ahead, plan);
     return;
   }
   launch_chained(fp8_quantize_rows_kernel, dim3(rows), dim3(kRowThreads), 0, stream,
-                 static_cast<const __nv_bfloat16*>(input), out, scales, rows, plan);
+                 static_cast<const __nv_bfloat16*>(input), out, scales, rows, weights_ahead, plan);
 }
 
 void launch_gelu_quantize_fp8(const void* gate_up, const float* activation_scales, float gate_w_scale,

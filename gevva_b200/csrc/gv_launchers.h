@@ -247,7 +247,7 @@ void launch_ff_prepare(const void* input, const void* dense_weight, const void* 
                        const void* router_scale, void* dense_out, void* expert_out, void* router_out,
                        int rows, cudaStream_t stream);
 // Also writes the plan of the dense projections seen as grouped GEMMs with one group.
-void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows, const RoutePlan& plan,
+void launch_fp8_quantize_rows(const void* input, uint8_t* out, float* scales, int rows, bool weights_ahead, const RoutePlan& plan,
                               cudaStream_t stream);
 void launch_gelu_quantize_fp8(const void* gate_up, const float* activation_scales, float gate_w_scale,
                               float up_w_scale, const float* gelu_table, uint8_t* out, float* scales, int rows,
