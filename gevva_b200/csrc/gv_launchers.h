@@ -186,7 +186,7 @@ void launch_grouped_gemm_pairs(const GemmOperands& op, const RoutePlan& plan, in
 int prepare_grouped_gemm_pairs();
 
 // Fused w13 + GeGLU + requantise run by CTA pairs with the weights on the MMA's M side and up to
-// 208 rows of one expert on its N side (grouped_gemm_w13_pair.cu).
+// 256 rows of one expert on its N side (grouped_gemm_w13_pair.cu).
 constexpr int kW13PairBoxes = 16;
 struct W13PairOperands {
   CUtensorMap map_x[kW13PairBoxes];  // activation codes [row capacity, 1408] bytes through boxes of 8, 16, ... 128 rows x 128 B
