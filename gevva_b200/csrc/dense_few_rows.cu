@@ -240,7 +240,7 @@ dense_few_gate_up_kernel(const __grid_constant__ CUtensorMap map, const FewParam
     uint32_t gates[16], ups[16];
     tmem_load_32x16(tmem_acc + unit * 16, gates);
     tmem_load_32x16(tmem_acc + (kUnits + unit) * 16, ups);
-    tmem_load_wait();
+    tmem_load_wait(gates, ups);
     const int token = lane >> 4, row = lane & 15;
     uint32_t gate_bits = 0, up_bits = 0;
 #pragma unroll
@@ -307,7 +307,7 @@ dense_few_down_kernel(const __grid_constant__ CUtensorMap map, const FewParams p
     for (int chunk = warp / 4; chunk < kRows / 16; chunk += kEpilogueWarps) {
       uint32_t r[16];  // of token `lane`
       tmem_load_32x16(tmem_acc + chunk * 16, r);
-      tmem_load_wait();
+      tmem_load_wait(r);
       if (lane < p.tokens) {
         uint4* out = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(lane) * kHidden + row0 + chunk * 16);
 #pragma unroll

@@ -232,7 +232,7 @@ dense_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         const int part = step >= groups ? 1 : 0, group = step - part * groups;
         if (step < steps) {
           tmem_load_16x64(tmem_rows + (static_cast<uint32_t>(part * 16) << 16) + static_cast<uint32_t>(acc) * kN + 64 * group, r);
-          tmem_load_wait();
+          tmem_load_wait(r);
         }
         if (step + 1 >= steps) {
           tc_fence_before_sync();

@@ -248,11 +248,14 @@ __device__ __forceinline__ uint32_t stream_word_of(int index, bool down, const S
   return stream_word(smem->chunk_expert[chunk], smem->chunk_index[chunk], index - chunk * per_chunk) | (down ? kStItemDown : 0u);
 }
 
-__device__ __forceinline__ void tmem_load_32x8(uint32_t tmem_address, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(tmem_address)
-               : "memory");
+// Nothing unless `wanted`, which is the same in the whole warp; the registers are undefined then.
+__device__ __forceinline__ void tmem_load_32x8(bool wanted, uint32_t tmem_address, uint32_t (&r)[8]) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %9, 0;\n\t"
+      "@p tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(tmem_address), "r"(static_cast<uint32_t>(wanted))
+      : "memory");
 }
 
 // A number of MMAs as a type.
@@ -1085,8 +1088,8 @@ stream_experts_kernel(const __grid_constant__ StreamMaps maps, const __grid_cons
         const uint32_t source = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * kStRows;
 #pragma unroll
         for (int g = 0; g < 4; ++g)
-          if ((side + 2 * g) * 8 < rows) tmem_load_32x8(source + (side + 2 * g) * 8, r[g]);
-        tmem_load_wait();
+          tmem_load_32x8((side + 2 * g) * 8 < rows, source + (side + 2 * g) * 8, r[g]);
+        tmem_load_wait(r);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&smem->acc_empty[acc]);

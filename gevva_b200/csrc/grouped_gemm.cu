@@ -484,7 +484,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       if constexpr (kMode != kGeglu && !kWide) {
         uint32_t r[32];
         tmem_load_32x32(tmem_row + sub * 32, r);
-        tmem_load_wait();
+        tmem_load_wait(r);
         tc_fence_before_sync();
         mbar_arrive(&smem->acc_empty[acc_stage]);  // accumulators are in registers now
         // same decision in all four warps of the quarter
@@ -495,7 +495,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         uint32_t r0[32], r1[32];
         tmem_load_32x32(tmem_row + sub * 32, r0);
         tmem_load_32x32(tmem_row + kStoreColumns + sub * 32, r1);
-        tmem_load_wait();
+        tmem_load_wait(r0, r1);
         tc_fence_before_sync();
         mbar_arrive(&smem->acc_empty[acc_stage]);
         if (quarter * 32 < rows_valid) {
@@ -514,7 +514,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         tmem_load_32x16(tmem_up + 64, gate0);
         tmem_load_32x16(tmem_up + 16, up1);
         tmem_load_32x16(tmem_up + 80, gate1);
-        tmem_load_wait();
+        tmem_load_wait(up0, gate0, up1, gate1);
         tc_fence_before_sync();
         mbar_arrive(&smem->acc_empty[acc_stage]);
         const bool columns_exist = n_tile * 128 + sub * 32 < kInter;  // the last item is half empty

@@ -364,7 +364,7 @@ grouped_down_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           for (int group = 0; group < groups; ++group) {
             uint32_t r[32];
             tmem_load_16x64(tmem_rows + (static_cast<uint32_t>(part * 16) << 16) + static_cast<uint32_t>(acc) * kDnColumns + 64 * group, r);
-            tmem_load_wait();
+            tmem_load_wait(r);
             if (part + 1 == kParts && group + 1 == groups) {
               tc_fence_before_sync();
               __syncwarp();

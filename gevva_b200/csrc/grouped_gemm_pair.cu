@@ -408,7 +408,7 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
         if (m_tile >= 0) {
           tmem_load_32x32(tmem_row + sub * 32, r0);
           tmem_load_32x32(tmem_row + kStoreColumns + sub * 32, r1);
-          tmem_load_wait();
+          tmem_load_wait(r0, r1);
         }
         tc_fence_before_sync();
         release_accumulator(smem, is_leader, lane);
@@ -425,7 +425,7 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
           tmem_load_32x16(tmem_row + 128 + sub * 32, gate0);
           tmem_load_32x16(tmem_row + sub * 32 + 16, up1);
           tmem_load_32x16(tmem_row + 128 + sub * 32 + 16, gate1);
-          tmem_load_wait();
+          tmem_load_wait(up0, gate0, up1, gate1);
         }
         tc_fence_before_sync();
         release_accumulator(smem, is_leader, lane);

@@ -123,14 +123,16 @@ __device__ __forceinline__ void wp_issue_mmas(uint32_t tmem_acc, uint32_t tmem_s
            j == 0 ? accumulate : 1u);
 }
 
-// 16 lanes x 32 columns: register 4g + i holds columns 8g + 2t + (i & 1) of row lane/4 + 8 * (i / 2).
-__device__ __forceinline__ void wp_load_16x32(uint32_t tmem_address, uint32_t (&r)[16]) {
+// 16 lanes x 32 columns: register 4g + i holds columns 8g + 2t + (i & 1) of row lane/4 + 8 * (i / 2).  Nothing unless `wanted`,
+// which is the same in the whole warp; the registers are undefined then.
+__device__ __forceinline__ void wp_load_16x32(bool wanted, uint32_t tmem_address, uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %17, 0;\n\t"
+      "@p tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t}"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(tmem_address)
+      : "r"(tmem_address), "r"(static_cast<uint32_t>(wanted))
       : "memory");
 }
 
@@ -455,15 +457,13 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
       // from the end that the two accumulators share; the next step's accumulators are fetched under a step's arithmetic
       int turn = (part + round) % kWpParts;
       bool first = true;
-      const auto load = [&](int turn_of_load) {
+      const auto load = [&](bool wanted, int turn_of_load) {
         const int step = acc == 0 ? steps - 1 - turn_of_load : turn_of_load;
-        wp_load_16x32(tmem_rows + 32 * step, even);
-        wp_load_16x32(tmem_rows + (16u << 16) + 32 * step, odd);
+        wp_load_16x32(wanted, tmem_rows + 32 * step, even);
+        wp_load_16x32(wanted, tmem_rows + (16u << 16) + 32 * step, odd);
       };
-      if (turn < steps) {
-        load(turn);
-        tmem_load_wait();
-      }
+      load(turn < steps, turn);
+      tmem_load_wait(even, odd);
 #pragma unroll 1
       for (;;) {
         const bool last = turn + kWpParts >= steps;
@@ -492,7 +492,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
           gate[k] = pack_bf16x2(low_of(g0), low_of(g1));
           gate[k + 1] = pack_bf16x2(high_of(g0), high_of(g1));
         }
-        if (!last) load(turn + kWpParts);  // under this step's arithmetic; waited for at its end
+        load(!last, turn + kWpParts);  // under this step's arithmetic; waited for at its end
         // erf of the magnitudes from the table, two indices to a word
         constexpr uint32_t kFirst = kErfFirst * 0x10001u, kLast = (kErfFirst + kErfEntries - 1) * 0x10001u;
         float erf0[8], erf1[8];
@@ -581,7 +581,7 @@ w13_geglu_pair_kernel(const __grid_constant__ WpTokenMaps map_x, const __grid_co
         }
         if (last) break;
         turn += kWpParts;
-        tmem_load_wait();
+        tmem_load_wait(even, odd);
       }
       if (++acc == kWpAccStages) {
         acc = 0;

@@ -487,9 +487,28 @@ __device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-__device__ __forceinline__ void tmem_load_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// A tensor-memory load writes its registers some time after its instruction, and only this wait says that they are there.  So the wait
+// takes them: every use, copy or spill that the compiler makes of a value then lies behind it (a wait without operands is ordered
+// against other volatile instructions only, not against arithmetic).  For the same reason a load that depends on a condition whose
+// wait lies outside of it is predicated instead of branched over, so that no two versions of a register meet between load and wait.
+#define GV_LOADED8(r, i) "+r"((r)[i]), "+r"((r)[i + 1]), "+r"((r)[i + 2]), "+r"((r)[i + 3]), "+r"((r)[i + 4]), "+r"((r)[i + 5]), "+r"((r)[i + 6]), "+r"((r)[i + 7])
+#define GV_LOADED16(r) GV_LOADED8(r, 0), GV_LOADED8(r, 8)
+#define GV_LOADED32(r) GV_LOADED8(r, 0), GV_LOADED8(r, 8), GV_LOADED8(r, 16), GV_LOADED8(r, 24)
+#define GV_LOAD_WAIT(...) asm volatile("tcgen05.wait::ld.sync.aligned;" : __VA_ARGS__ :: "memory")
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&a)[16]) { GV_LOAD_WAIT(GV_LOADED16(a)); }
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&a)[16], uint32_t (&b)[16]) { GV_LOAD_WAIT(GV_LOADED16(a), GV_LOADED16(b)); }
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&a)[16], uint32_t (&b)[16], uint32_t (&c)[16], uint32_t (&d)[16]) {
+  GV_LOAD_WAIT(GV_LOADED16(a), GV_LOADED16(b), GV_LOADED16(c), GV_LOADED16(d));
 }
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&a)[32]) { GV_LOAD_WAIT(GV_LOADED32(a)); }
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&a)[32], uint32_t (&b)[32]) { GV_LOAD_WAIT(GV_LOADED32(a), GV_LOADED32(b)); }
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&r)[4][8]) {
+  GV_LOAD_WAIT(GV_LOADED8(r[0], 0), GV_LOADED8(r[1], 0), GV_LOADED8(r[2], 0), GV_LOADED8(r[3], 0));
+}
+#undef GV_LOAD_WAIT
+#undef GV_LOADED32
+#undef GV_LOADED16
+#undef GV_LOADED8
 
 // Shared-memory matrix descriptor (sm_100 format, version 1).
 //   layout: 0 = no swizzle, 2 = 128-byte swizzle

@@ -273,7 +273,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       for (int part = first_part; part < first_part + kParts; ++part) {
         uint32_t r[32];
         tmem_load_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + slice * kExperts + part * 32, r);
-        tmem_load_wait();
+        tmem_load_wait(r);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int chunk = part * 8 + i;
