@@ -352,10 +352,13 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
   return rank;
 }
 
-// Barrier over every thread of the cluster; writes to (distributed) shared memory made before
+// Barrier over every thread of the cluster, by whole warps; writes to (distributed) shared memory made before
 // the arrive are visible to every thread after its wait.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 
 // Address, in the cluster's shared window, of the byte that `local_address` names in the CTA of

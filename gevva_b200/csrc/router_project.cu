@@ -177,6 +177,9 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  // A CTA's shared memory may be written by its peers once it runs: every thread says so here, and waits for all others where its
+  // warp would store to them (the wait is over by then: it lies behind the K blocks).
+  if (kSplit > 1) cluster_arrive();
   const uint32_t tmem_base = smem->tmem_base;
   // While the previous kernel drains, this CTA's slice of the router matrix is asked into L2 (a hint: the
   // loads themselves come after the wait); a model's other weights have pushed it out since last time.
@@ -262,6 +265,10 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     // tensor-memory loads are warp-wide, so a warp takes part if any of its 32 rows exists
     const bool row_exists = row < kRows && m_tile * kRows + row < p.tokens;
     const bool warp_has_rows = quarter * 32 < kRows && m_tile * kRows + quarter * 32 < p.tokens;
+    if (kSplit > 1) {
+      __syncwarp();
+      cluster_wait();
+    }
 #pragma unroll 1
     for (int slice = 0; slice < kSlices; ++slice) {
       if (!wait_or_abort(&smem->acc_full[slice], 0, smem, p.status) || !warp_has_rows) break;
@@ -286,6 +293,10 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     }
   }
 
+  if (kSplit > 1 && warp < 2) {  // (the epilogue's warps have waited for the cluster's start above)
+    __syncwarp();
+    cluster_wait();
+  }
   // Every thread of every CTA of the cluster arrives here, also after a failed wait.  The barrier
   // orders the posted stores above before the owners' reads below; after it no CTA touches another
   // CTA's shared memory, so a CTA may finish while its peers still work.
