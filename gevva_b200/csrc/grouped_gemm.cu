@@ -466,7 +466,7 @@ grouped_nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const int row0 = p.expert_offsets[expert] + local0;
       const int rows_valid = p.expert_offsets[expert + 1] - row0;  // may exceed 128
       const float alpha = p.alpha[expert];
-      const bool acc_ready = wait_or_abort(&smem->acc_full[acc_stage], acc_phase, smem, p.status);
+      const bool acc_ready = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[acc_stage], acc_phase, smem, p.status));
       if constexpr (kMode != kGeglu) {
         // The four warps of a quarter meet at named barriers while they store, so they must
         // leave together: a warp whose wait failed says so, and all four read the answer behind

@@ -391,7 +391,7 @@ grouped_nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const 
         rows_valid = p.expert_offsets[expert + 1] - row0;  // may exceed 128
         alpha = p.alpha[expert];
       }
-      const bool acc_ready = wait_or_abort(&smem->acc_full, acc_phase, smem, p.status);
+      const bool acc_ready = __all_sync(0xffffffffu, wait_or_abort(&smem->acc_full, acc_phase, smem, p.status));
       acc_phase ^= 1u;
       if constexpr (kMode != kGeglu) {
         if (!acc_ready) smem->quarter_left[quarter] = 1;

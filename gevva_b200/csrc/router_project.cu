@@ -271,7 +271,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     }
 #pragma unroll 1
     for (int slice = 0; slice < kSlices; ++slice) {
-      if (!wait_or_abort(&smem->acc_full[slice], 0, smem, p.status) || !warp_has_rows) break;
+      if (!warp_has_rows || !__all_sync(0xffffffffu, wait_or_abort(&smem->acc_full[slice], 0, smem, p.status))) break;
       tc_fence_after_sync();
       const uint32_t remote_row =
           cluster_map_shared(smem_u32(smem->received + ((slice0 + slice) * kOwnRows + owner_row) * kExperts),

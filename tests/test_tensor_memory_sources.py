@@ -71,3 +71,12 @@ def test_no_branch_between_a_load_and_its_wait(source):
     """A load that is branched over, with its wait behind the branch, would let the compiler merge old and new registers in between."""
     text = code(os.path.join(CSRC, source))
     assert not re.findall(r"\bif\s*(?:constexpr\s*)?\([^;{}]*\)\s*(?:load|tmem_load_\d+x\d+|wp_load_16x32)\(", text)
+
+
+@pytest.mark.parametrize("source", [os.path.basename(p) for p in SOURCES if p.endswith(".cu")])
+def test_warps_agree_before_they_load(source):
+    """The loads are made by whole warps.  A wait that runs out may run out for some of its lanes: the warp votes, and goes on or leaves
+    together."""
+    text = code(os.path.join(CSRC, source))
+    waits = [m.start() for m in re.finditer(r"wait_or_abort\(&smem->acc_full", text)]
+    assert waits and all(text[:at].endswith("__all_sync(0xffffffffu, ") for at in waits)
