@@ -355,6 +355,8 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 // Barrier over every thread of the cluster, by whole warps; writes to (distributed) shared memory made before
 // the arrive are visible to every thread after its wait.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// (orders nothing: says only that this CTA runs)
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
   cluster_arrive();
