@@ -179,7 +179,7 @@ route_project_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   tc_fence_after_sync();
   // A CTA's shared memory may be written by its peers once it runs: every thread says so here, and waits for all others where its
   // warp would store to them (the wait is over by then: it lies behind the K blocks).
-  if (kSplit > 1) cluster_arrive();
+  if (kSplit > 1) cluster_arrive_relaxed();
   const uint32_t tmem_base = smem->tmem_base;
   // While the previous kernel drains, this CTA's slice of the router matrix is asked into L2 (a hint: the
   // loads themselves come after the wait); a model's other weights have pushed it out since last time.
