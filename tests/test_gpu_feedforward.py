@@ -374,6 +374,76 @@ def test_dense_pairs_at_tile_edges(dense_weights, cuda_device, tokens):
     assert guarded[:tokens].float().abs().max() > 0
 
 
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("tokens", [1, 3, 600, 2048])
+def test_weights_written_right_before_the_dense_mlp(dense_weights, cuda_device, tokens, graph):
+    """The dense GEMMs fetch weights before the kernel in front of them has ended.  What kernels in front of the whole call write is there all
+    the same, also where those let their successors start before they have written anything: ff_prepare, whose normalised rows of
+    ones are its norm weight, whose bytes are the MLP's weights here.  The last hundred rows that it writes come behind a w2 on four
+    SMs, which takes a millisecond and lets it start at its own beginning, so a call that did not wait for it would find what was there before.
+    For the MLP by itself and for a layer's, on the same stream and on a second one."""
+    from gevva_b200 import feedforward as ff
+    from gevva_b200.runtime import STAGE_W2
+    from gevva_b200.synthetic import SyntheticStack
+    gate_up, down, gs, us, ds = dense_weights
+    lib = ff._lib()
+    ones = torch.ones((DENSE, HIDDEN), dtype=torch.bfloat16, device=cuda_device)
+    unused = [torch.empty_like(ones) for _ in range(2)]
+    stack = SyntheticStack(1, 2600, cuda_device, seed=11)
+    delay = stack.layers[0].experts
+    stack.forward(hashgen.activations(2600, HIDDEN, 94, cuda_device))  # (a plan and operands for the w2)
+    launch_on = lib["_ZN2gv20moe_launch_stages_onEP9gevva_moePKvPKiPKfPvijP11CUstream_sti"]  # gv::moe_launch_stages_on
+    launch_on.argtypes = [ctypes.c_void_p] * 5 + [ctypes.c_int, ctypes.c_uint, ctypes.c_void_p, ctypes.c_int]
+    generator = torch.Generator(device=cuda_device).manual_seed(tokens)
+    # two rows of bf16 values, both of whose bytes are finite E4M3 numbers: 0.5 to 2 in steps of 1/256 and up, of either sign
+    rows = [(torch.randint(0x3F00, 0x3F7F, (HIDDEN,), generator=generator, device=cuda_device) +
+             0x8000 * torch.randint(0, 2, (HIDDEN,), generator=generator, device=cuda_device)).to(torch.uint16).view(torch.bfloat16)
+            for _ in range(2)]
+
+    def write(weights, row, count=DENSE):
+        stream = torch.cuda.current_stream().cuda_stream
+        for buffer in weights:
+            assert lib.gevva_ff_prepare(ones.data_ptr(), row.data_ptr(), row.data_ptr(), row.data_ptr(), buffer.data_ptr(), unused[0].data_ptr(),
+                                        unused[1].data_ptr(), min(count, buffer.numel() // (2 * HIDDEN)), stream) == 0
+
+    def check(weights, run):
+        want, calls = [], []
+        for row, other in zip(rows, reversed(rows)):
+            write(weights, row)
+            torch.cuda.synchronize()
+            assert all(torch.equal(buffer.view(torch.bfloat16).view(-1, HIDDEN), row.expand(buffer.numel() // (2 * HIDDEN), HIDDEN))
+                       for buffer in weights)
+            want.append(run().clone())
+            torch.cuda.synchronize()
+
+            def call(row=row, other=other):
+                write(weights, row)
+                write(weights[:1], other, 100)
+                assert launch_on(delay._handle, None, None, None, None, 2600, STAGE_W2, torch.cuda.current_stream().cuda_stream, 4) == 0
+                write(weights[:1], row, 100)
+                return run()
+
+            if graph:
+                captured = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(captured):
+                    out = call()
+                calls.append(lambda captured=captured, out=out: (captured.replay(), out)[1])
+            else:
+                calls.append(call)
+        assert want[0].isfinite().all() and not torch.equal(*want)
+        for turn in range(6):
+            assert torch.equal(calls[turn % 2](), want[turn % 2])
+
+    x = hashgen.activations(tokens, HIDDEN, 95, cuda_device)
+    mlp = ff.DenseMlp(gate_up.clone(), down.clone(), gs, us, ds, tokens)
+    check(mlp._keep, lambda: mlp.launch(x)[0])
+    layer = SyntheticStack(1, max(tokens, 64), cuda_device, seed=12).layers[0]
+    aux = torch.cuda.Stream(device=cuda_device)
+    check(layer.dense._keep, lambda: layer.forward(x))
+    check(layer.dense._keep, lambda: layer.forward(x, aux_stream=aux))
+    delay.check()
+
+
 @pytest.mark.parametrize("tokens", [1, 3, 129, 600])
 def test_dense_output_aligned_to_16_bytes(dense_weights, cuda_device, tokens):
     """An output that starts between two 32-byte lines gets the bits of one that does not, and nothing around it."""

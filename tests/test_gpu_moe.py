@@ -210,9 +210,9 @@ def test_route_sort_matches_oracle(gm, oracle, big_runner, cuda_device, tokens, 
 
 
 @pytest.mark.parametrize("tokens", [256, 257, 640, 1151, 1153, 1535, 1536, 1537])
-def test_route_sort_at_the_edges_of_its_forms(gm, oracle, big_runner, cuda_device, tokens):
-    """Up to twelve chunks of 1024 routes every CTA of the one-launch sort counts the other chunks itself, beyond they meet: whole and
-    ragged last chunks on both sides, with experts that a token names twice and one that takes a route of every token."""
+def test_route_sort_at_the_edges_of_its_chunks(gm, oracle, big_runner, cuda_device, tokens):
+    """Every CTA of the one-launch sort counts the chunks of 1024 routes before and behind its own itself: whole and ragged last
+    chunks, with experts that a token names twice and one that takes a route of every token."""
     from gevva_b200 import runtime as rt
     ids = random_ids(tokens, 7 + tokens)
     ids[::5, 6] = ids[::5, 1]
@@ -241,10 +241,11 @@ def test_route_sort_around_its_longest_counts(gm, oracle, big_runner, cuda_devic
         assert (got[key] == want[key]).all(), key
 
 
-@pytest.mark.parametrize("tokens", [128, 129, 300, 1535, 1536, 1537])
+@pytest.mark.parametrize("tokens", [128, 129, 300, 1535, 1536, 1537, 3072, 3073, 4096])
 def test_route_sort_by_owner_at_one_rank(gm, varied_weights, cuda_device, tokens):
     """Expert-parallel ranks sort by the key that a placement table gives each expert: one rank alone, whose table is a permutation
-    of its own experts, has the bits of the plain runner in all three one-launch forms of the sort, twice over."""
+    of its own experts, has the bits of the plain runner in all three one-launch forms of the sort (up to 128 tokens one CTA a token, up to 24
+    chunks CTAs that count for themselves, above CTAs that meet), twice over."""
     import ctypes
     from gevva_b200.expert_parallel import _EpConfig, local_expert_weights
     from gevva_b200.runtime import _Weights
@@ -648,7 +649,7 @@ def test_w2_pairs_at_tile_edges(gm, weights, cuda_device, tokens, edges):
 @pytest.mark.parametrize("tokens,edges", [(641, [1, 7, 8, 9, 127, 128, 129, 255, 256, 257]),
                                           (1000, [15, 16, 17, 33, 191, 192, 193, 208, 209, 385])])
 def test_large_batches_at_tile_and_chunk_edges(gm, weights, cuda_device, tokens, edges):
-    """The w13 and w2 kernels of batches above 640 tokens, whose chunks of up to 208 rows, 128-row tiles, items
+    """The w13 and w2 kernels of batches above 640 tokens, whose chunks of up to 256 rows, 128-row tiles, items
     and units of items end raggedly, against the CTA-pair kernels that share weight tiles: the same w2 operand
     and routed rows, with every stage in one call and each in a call of its own."""
     from gevva_b200 import runtime as rt
@@ -686,7 +687,7 @@ def test_large_batches_at_tile_and_chunk_edges(gm, weights, cuda_device, tokens,
 @pytest.mark.parametrize("tokens,kind", [(129, "random"), (130, "skewed"), (300, "skewed"), (777, "random"),
                                          (4096, "random")])
 def test_weight_major_pair_w13_equals_the_single_cta_w13(gm, weights, cuda_device, tokens, kind, monkeypatch):
-    """The fused w13 stage run by CTA pairs with the weights on the MMA's M side and up to 208 rows of
+    """The fused w13 stage run by CTA pairs with the weights on the MMA's M side and up to 256 rows of
     an expert on its N side (any multiple of 16) writes the same w2 operand codes and scale bytes as
     the one-CTA-per-tile kernel (in its short and, with more than eight rounds of items, its long order),
     and the layer output follows."""
@@ -757,6 +758,38 @@ def test_weights_asked_ahead_change_no_result(gm, weights, cuda_device, tokens):
             runner.launch_stages(stage, tokens, input=x, expert_ids=dev_ids, route_weights=rw, output=out)
         runner.check()
         results.append((out, runner.buffer(rt.BUF_INTER_CODES)[: tokens * TOP_K * INTER // 2].clone()))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert results[0][0].float().abs().max() > 0
+
+
+@pytest.mark.parametrize("tokens,sms", [(700, 148), (1000, 31), (1000, 66), (1000, 148), (2559, 61), (2600, 58), (2600, 100), (2600, 148), (4112, 4)])
+def test_large_batches_on_any_number_of_sms(gm, weights, cuda_device, tokens, sms):
+    """The persistent kernels deal their items out over the SMs that a call has.  What is left of the last round of w2's units goes out in
+    thirds up to two thirds of a round (31 and 148 of 1000 tokens, 58 and 148 of 2600) and in units above (66; 100, one unit too many); w13 works the
+    items of 512 rounds out ahead and the others, of which 257 rows an expert on four SMs make 256, in turn.  The same operands and
+    rows as from the kernels that share weight tiles, on all SMs."""
+    import ctypes
+    from gevva_b200 import runtime as rt
+    launch_on = gm.library()["_ZN2gv20moe_launch_stages_onEP9gevva_moePKvPKiPKfPvijP11CUstream_sti"]  # gv::moe_launch_stages_on
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    launch_on.argtypes = [vp, vp, vp, vp, vp, i32, ctypes.c_uint, vp, i32]
+    dev_ids = torch.from_numpy(ids_with_counts(tokens, [])).to(cuda_device)
+    x = hashgen.activations(tokens, HIDDEN, 93, cuda_device)
+    rw = torch.full((tokens, TOP_K), 0.125, device=cuda_device)
+    results = []
+    for pairs in (True, False):
+        runner = gm.Nvfp4ExpertRunner(weights[0], tokens, pairs=pairs)
+        out = torch.zeros_like(x)
+        for _ in range(2):
+            if pairs:
+                runner.launch_batch(x, dev_ids, rw, out, tokens)
+            else:
+                assert launch_on(runner._handle, x.data_ptr(), dev_ids.data_ptr(), rw.data_ptr(), out.data_ptr(), tokens, rt.STAGE_ALL,
+                                 torch.cuda.current_stream().cuda_stream, sms) == 0
+        runner.check()
+        results.append((out, runner.buffer(rt.BUF_INTER_CODES)[: tokens * TOP_K * INTER // 2].clone(),
+                        runner.buffer(rt.BUF_W2_OUT, torch.bfloat16)[: tokens * TOP_K * HIDDEN].clone()))
     for a, b in zip(*results):
         assert torch.equal(a, b)
     assert results[0][0].float().abs().max() > 0
