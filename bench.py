@@ -37,10 +37,10 @@ NOMINAL_FP4_TFLOPS = 9000.0
 W13_ALGORITHMIC_BYTES = 128 * (1982464 + 247808) + 32768 * (1408 + 176) + 32768 * (352 + 44)
 # RECORDED figures (ncu captures summarised under profiles/, not measured by this run):
 # dram__bytes_read.sum + dram__bytes_write.sum of one fused w13 launch at this workload
-W13_DRAM_TRAFFIC_BYTES_RECORDED = 314354432 + 57057280
+W13_DRAM_TRAFFIC_BYTES_RECORDED = 342250496 + 9220608
 # DRAM bytes of one layer step at 4096 tokens: the two GEMMs as captured, the quantiser
 # (23 MB read + 52 MB written) and the reduce (185 MB read + 23 MB written) by their algorithmic bytes
-LAYER_DRAM_BYTES_RECORDED = (314354432 + 57057280) + (163974912 + 159908864) + 75000000 + 207600000
+LAYER_DRAM_BYTES_RECORDED = W13_DRAM_TRAFFIC_BYTES_RECORDED + (164371456 + 130129664) + 75000000 + 207600000
 WORKLOAD = "prefill_4096_tokens_router_bias_N(0,0.5)"
 INPUT_BATCHES = 4
 
@@ -827,7 +827,7 @@ def run_gpu(args):
                          "frac": achieved / fp4_peak,
                          "traffic": W13_DRAM_TRAFFIC_BYTES_RECORDED,
                          "traffic_source": "recorded: dram__bytes_read+write of one launch, ncu capture of this "
-                                           "workload summarised in profiles/expert_gemms_prefill4096.md",
+                                           "workload summarised in profiles/cta_pair_gemms_and_row_kernels.md",
                          "algorithmic_bytes": W13_ALGORITHMIC_BYTES,
                          "peak_source": f"4 x bf16_tflops of MEASURED_PEAKS.json ({peak_kind}); "
                                         "no FP4 entry exists",

@@ -2,7 +2,7 @@
 //
 // What bounds it.  A 128 x 256 tile of one CTA (grouped_gemm.cu) takes in 48 KB a K block of 128 for 512 tensor-pipe cycles, and an SM
 // takes in 73 bytes a cycle: 660 cycles.  A pair (tcgen05 cta_group::2, M = 256) computes 256 tokens x 256 columns with half of either
-// operand in each CTA, 32 KB: 450 cycles, under the MMAs' 512.  The whole MLP, one CTA a tile -> pairs
+// operand in each CTA, 32 KB: 450 cycles, under the MMAs' 512.  The whole MLP, one CTA a tile -> pairs as they were first
 // (us): 1 token 25.5 -> 22.8, 128 tokens 29.0 -> 24.8, 301 tokens 31.3 -> 25.1, 640 tokens 34.9 -> 30.1, 1024 tokens 38.0 -> 33.6, 2048 tokens 62.8 ->
 // 54.2, 4096 tokens 106 -> 94 (of the last two 23 and 38 were its quantisers; 48 and 81 with those of today).
 // 192 columns an item where that leaves the clusters less to do (the second projection at 2048 tokens: 88 items of 256 are two

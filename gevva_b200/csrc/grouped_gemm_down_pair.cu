@@ -2,10 +2,10 @@
 //
 // What bounds it.  Operands in and rows out share the way between an SM and L2: 100 KB in take 0.72 us an item there, 48 KB out 0.84 to
 // 1.0 us, both 1.4 to 2.1.  One CTA a tile (grouped_gemm_down.cu) fetches 103 KB for 128 rows x 192 columns and takes 2 us; a pair
-// (tcgen05 cta_group::2, M = 256) needs the weights once for two row tiles, each CTA half of them: 66 KB an item and CTA.
-// Alone, one CTA a tile -> this (us): 2048 tokens 46.7 -> 47.5, 3000 tokens 57 -> 53, 4096 tokens 71 -> 68, 8192 tokens 132 -> 118, 16384 tokens
-// 248 -> 203; without its stores 44 at 4096 tokens and 115 at 16384.  Below, most experts have a single tile, whose pair fetches 132 KB
-// where one CTA fetches 103 (1024 tokens 36.2 -> 42.4).  Eight epilogue warps and stores without a cache hint make no difference.
+// (tcgen05 cta_group::2, M = 256) needs the weights once for two row tiles, each CTA half of them: 66 KB an item and CTA.  With few tokens most
+// experts have a single tile, whose pair fetches 132 KB where one CTA fetches 103; where the line lies is said at kDownPairTokens (moe_abi.cu).
+// Without its stores the form before the next paragraph took 44 us of 68 at 4096 tokens, 115 of 203 at 16384.  Eight epilogue warps and stores without a cache
+// hint make no difference.
 // Two pairs of an expert share the weights, too: each weight stage is used by both, one after the other, and an item fetches 42 KB instead of 59.  (Loads and
 // stores share the fabric: 48 KB stored and 64 KB loaded an item and SM take 1.45 us with everything in L2, either alone 1.0; the kernel took 1.6 at 16384
 // tokens.)  And what does not fill a round of units is dealt out in thirds of them.  Alone, us, without both -> with: 2600 tokens 53.0 -> 50.4, 4096 67.3 -> 64.0, 8192

@@ -7,7 +7,9 @@
 // the tokens sit on N, which may be any multiple of 16, a group of 200 rows is one item and not two 128-row tiles.
 // An item is 11 K blocks, each of four MMAs of N / 2 tensor cycles (39 at least) and eight or twelve scale copies.  Issuing those takes one
 // thread some 300 cycles a K block, and beside the epilogue's warps on its scheduler more, so a narrow item costs nearly what one of
-// 170 rows does: chunks are as wide as the MMA allows.  Chunks of 208 rows and a loop of the whole warp -> this (us, alone): 4096 tokens 96.5 -> 88.2,
+// 170 rows does: chunks are as wide as the MMA allows.  (That is not the whole of it: 4096 tokens' 1176 items come to 35 us so, and their operands to 54 us of
+// HBM and 40 of L2 time, but the kernel takes 77 to 85; an item of 256 rows takes some 9300 cycles, 5632 of them the tensor pipe's.  What the
+// issuing thread waits for in the others has not been counted.)  Chunks of 208 rows and a loop of the whole warp -> this (us, alone): 4096 tokens 96.5 -> 88.2,
 // of uneven loads 94.2 -> 87.4, 16384 290 -> 269; a whole layer of 700 tokens 109.5 -> 108.5, 4096 254 -> 245, 16384 795 -> 770.
 // Beside large batches the clock drops to 1.35 GHz under the power limit (this kernel repeated for seconds at 4096 tokens).
 // Alone (us, one-CTA kernel -> the first form of this one; uniform routing): 53.1 -> 53.2 at 1024 tokens, 63.9 -> 58.9 at 2048,
@@ -34,7 +36,7 @@
 // accumulators fetched ahead: 700 tokens 53.2 -> 51.6 us, 4096 88.2 -> 85.2, 16384 269 -> 263; a layer of 700 tokens 108.5 -> 107.4,
 // of 4096 245 -> 240.  (With the accumulator transposed
 // through shared memory by sixteen warps that traffic bounded the kernel, 107 us at 4096 tokens; with this epilogue
-// twelve or sixteen warps are 3 to 8 % slower than eight, and five stages up to 8 % slower than six.)  Every wait is bounded.
+// twelve warps are as fast as eight and sixteen 10 % slower.)  Every wait is bounded.
 #include "gv_common.cuh"
 #include "gv_cta_pair.cuh"
 #include "gv_gemm_parts.cuh"
@@ -182,7 +184,8 @@ __device__ __noinline__ uint32_t wp_pack(const WpSmem* smem, int round) {
          static_cast<uint32_t>((valid + 15) >> 4) << 10 | static_cast<uint32_t>(local >> 6) << 15;
 }
 
-// Behind a wait for `table` but for the first round, whose loads do not wait for it.
+// Behind a wait for `table` but for the first round, whose loads do not wait for it.  (Rounds past the table are those of the largest batches on a
+// few SMs.)
 __device__ __forceinline__ uint32_t wp_word(const WpSmem* smem, int round) {
   return round != 0 && round < kWpTable ? smem->items[round] : wp_pack(smem, round);
 }

@@ -379,15 +379,6 @@ __device__ __forceinline__ void cluster_store_uint4(uint32_t cluster_address, ui
                : "memory");
 }
 
-__device__ __forceinline__ float4 cluster_load_float4(uint32_t cluster_address) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(cluster_address)
-               : "memory");
-  return v;
-}
-
 // ---- tensor memory ---------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(

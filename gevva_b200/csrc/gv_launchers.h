@@ -191,7 +191,8 @@ constexpr int kW13PairBoxes = 16;
 struct W13PairOperands {
   CUtensorMap map_x[kW13PairBoxes];  // activation codes [row capacity, 1408] bytes through boxes of 8, 16, ... 128 rows x 128 B
   CUtensorMap map_w;      // w13 codes in the row order of its MMAs, a unit of 64 columns (up and gate rows) a copy
-  CUtensorMap map_x_sf;   // activation scale regions as [128-row blocks, 44 atoms, 512 B], box 2 blocks x 4 atoms
+  CUtensorMap map_x_sf;   // activation scale regions as [128-row blocks, 44 atoms, 512 B], box of one block x 4 atoms: a
+                          // second copy where a chunk has rows in two blocks
   CUtensorMap map_w_sf;   // unit-tiled weight scales (launch_retile_w13_unit_scales), box of four atoms
   const float* alpha;           // [experts]
   uint8_t* next_codes;          // [row capacity, 352]

@@ -26,16 +26,20 @@ using namespace gv;
 
 constexpr int kMaxTokens = 131072;
 constexpr int kStreamTokens = 640;  // see moe_streams
-// The quantiser of a call that goes on to the experts asks for the first weights of w13, which all such batches need (nearly every expert has
-// rows, and they are taken in order): HBM has little else to do while the sort and the quantiser run.  16 experts are the first
+// The quantiser of a call that goes on to the experts asks for the first weights of w13, which such batches need (nearly every expert has
+// rows, and they are taken in order; where no route goes to those sixteen it costs up to 1.1 us: 400 tokens on the last eight experts 44.5 -> 45.6 a layer, 613 56.8 -> 57.9,
+// 300 to 613 on the last sixty-four as before, 82.4 instead of 85.4 and 87.4 instead of 90.9 on all): HBM has little else to do while the sort and the quantiser run.  16 experts are the first
 // item of every SM and a little more (8 and 80 MB instead of 36 gain less).  Where the experts stream, us of the listed number of layers without / with: 300 tokens
 // 361.8 / 358.9 (four), 400 187.8 / 184.7, 613 191.3 / 189.2, 640 205.1 / 202.3 (two), Zipf(1.1) 500 the same; feed-forward layers of 301 tokens 314.2 / 312.7, 400
 // 330.0 / 326.9 (three), 640 248.9 / 248.1 (two).  By pairs: 700 228.9 / 227.0, 1000 244.8 / 241.9, 1400 280.3 / 277.7 (two), 2048 nothing, and feed-forward layers, whose
 // dense MLP runs between, lose by it (1000 tokens 311 / 319, 2048 442 / 447), as others' that take their rows unreduced would.
 constexpr int kAheadExperts = 16, kAheadTokens = 1536;
 // w2 by CTA pairs that share weights between two row tiles of an expert: from 160 rows an expert on average, where most experts
-// have two tiles.  Two layers in a graph, one CTA a tile and pairs, us: 1536 tokens 262 and 278, 2048 308 and 320, 2304 341 and 332, 2432 347 and
-// 344, 2560 362 and 361, 2688 365 and 361, 3072 383 and 371, 4096 496 and 494.  (Evenly loaded experts; the sides cross between 2048 and 2304.)
+// have two tiles.  One CTA a tile and pairs, us a layer of two in a graph, pauses between (spread 0.3): even loads 2048 tokens 144.8 and 148.0, 2304 158.4 and 156.0,
+// 2560 164.2 and 161.3, 3072 176.0 and 172.0, 4096 221.8 and 214.4, 8192 381.6 and 369.6; router bias of deviation 0.5 2048 147.2 and 152.9, 2560 166.7 and 169.3,
+// 3072 184.1 and 187.4, 3584 202.4 and 203.3, 4096 221.9 and 221.2, 8192 384.7 and 370.5; Zipf(1.1) 2560 175.3 and 182.1, 3072 196.3 and 198.6, 4096 231.3 and
+// 234.3, 5000 270.8 and 269.6, 8192 395.3 and 389.7.  So the sides cross between 2048 and 2304 tokens of even loads and only at some 4000 and 4500 of uneven ones, which lose
+// up to 2 and 4 % in between; the host does not know the routes, and the line lies between.
 constexpr int kDownPairTokens = 2560;
 static_assert(kStreamTokens <= gv::kStreamMaxTokens, "the streaming kernel's chunk list");
 
@@ -327,12 +331,11 @@ int gv::moe_sm_count(const gevva_moe* runner) { return runner->sm_count; }
 int gv::moe_max_tokens(const gevva_moe* runner) { return runner->scratch->max_tokens; }
 
 // Few rows an expert: the layer streams weights, and one launch with the weights on the MMA's M side does both GEMMs.
-// Against the launches of larger batches (w13 by CTA pairs, then w2), us a layer of four distinct ones in a graph, one B200:
-// router logits without bias, 300 tokens 96.7 against 99.7, 400 98.4 / 101.8, 500 101 / 105.5, 640 108.2 / 112.8 (up to 296
-// tokens it also takes in the sort and the quantiser); with a bias of deviation 0.5 96.9 / 99.2, 100.3 / 102.4, 106.1 / 104.9,
-// 114.8 / 112.5; with a Zipf(1.1) bias 83.9 / 84.5, 90.3 / 86.5, 96.4 / 91.2, 110.7 / 103.7: a heavy expert has many 64-row
-// chunks, each with the whole of its weights.  The host does not know the routes.  The line is that of evenly loaded
-// experts, for which the launch pays all the way; strongly skewed batches of 400 to 640 tokens lose 4 to 7 us by it.
+// Against the launches of larger batches (w13 by CTA pairs, then w2), us a layer of four distinct ones in a graph, pauses between, one B200 (spread 0.2):
+// router logits without bias, 300 tokens 86.1 against 94.1, 400 87.3 / 96.3, 500 90.1 / 99.5, 640 95.4 / 104.6 (up to 296
+// tokens it also takes in the sort and the quantiser); with a bias of deviation 0.5 85.4 / 93.9, 88.0 / 96.4, 91.7 / 100.1,
+// 98.4 / 105.5; with a Zipf(1.1) bias 72.9 / 79.5, 78.0 / 84.0, 84.8 / 88.9, 95.7 / 99.6: a heavy expert has many 64-row
+// chunks, each with the whole of its weights.  The launch pays all the way to the line, least for the heaviest experts.
 // (The pair options leave batches of at most 128 tokens alone.)
 bool gv::moe_streams(const gevva_moe* runner, int tokens) {
   const bool pair_options = (runner->pairs || runner->w13_pair_form) && tokens > gv::kFusedSortQuantizeMaxTokens;

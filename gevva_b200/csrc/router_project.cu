@@ -6,15 +6,16 @@
 // route_128_top8_kernel<<<tokens,128>>>).  Here both are one kernel and the logits never
 // reach HBM: tokens sit on MMA-M (16 to 128 per tile), the 128 experts on MMA-N, K = 2816.
 //
-// A tile (of 16, 32 or 64 tokens in batches of up to 2048) has its K range split over a cluster of four CTAs (two, or one, for batches whose tiles
-// would otherwise not fit one wave of SMs; eight for batches of at most 512 tokens), so a
+// A tile (of 16, 32 or 64 tokens in batches of up to 2048) has its K range cut into four slices (two, or one, in batches of many tiles;
+// eight for batches of at most 512 tokens), of which each CTA of the tile's cluster has one, or two where clusters of one CTA a slice
+// would not all run at once: a
 // 4096-token batch runs on 128 SMs and a decode-sized batch streams the router matrix through
 // eight SMs instead of one.  Each
-// CTA accumulates its K slice in tensor memory (tcgen05.mma kind::f16 for bf16 operands,
+// CTA accumulates its slices in tensor memory, each by itself (tcgen05.mma kind::f16 for bf16 operands,
 // kind::f8f6f4 for E4M3).  Tile row r belongs to CTA r % split of the cluster: every CTA stores
-// its fp32 partial sums (128 a row) row by row straight into the owners' shared memory (posted
-// st.shared::cluster stores), and after one cluster barrier each owner sums the partials of its
-// rows (a tile's / split) in rank order (a fixed order: results do not depend on timing), adds the optional
+// its fp32 partial sums (128 a row and slice) row by row straight into the owners' shared memory (posted
+// st.shared::cluster stores, behind a cluster barrier that says that the owners run), and after a second cluster barrier each owner sums the partials of its
+// rows (a tile's / split) in the order of the slices (a fixed order: results do not depend on timing), adds the optional
 // per-expert bias, rounds to bf16 as the GEMM would have stored it, and routes its rows (gv_route.cuh): a warp per
 // token where it has at most two a warp, else four lanes per token.
 //
@@ -29,9 +30,9 @@ namespace gv {
 
 namespace {
 
-// CTAs per cluster = K slices per token tile: 8 for small batches, else 4, 2 or 1, the largest that
+// K slices per token tile = CTAs per cluster x slices of a CTA: 8 for small batches, else 4, 2 or 1, with one slice a CTA where that
 // keeps the launch within one wave of SMs (a tile's pass is a chain of latencies, so waves cost more
-// than depth)
+// than depth), else two.
 // Epilogue warps.  CTAs of 128-row tiles that keep 64 or 128 rows for themselves route them four lanes a row in one pass of sixteen warps
 // (four -> sixteen, us alone: 6000 tokens 15.8 -> 14.6, 8192 16.9 -> 15.7, 12000 25.3 -> 22.0, 16384 28.5 -> 25.2; a layer of 16384 tokens 793 -> 777; with 32 rows,
 // up to 4608 tokens, 12.2 -> 12.5 at 4096).  64 rows keep eight busy (four -> eight, us alone: 37 tokens 5.9 -> 5.5, 64 6.7 -> 6.4, 613 9.0 -> 8.2, 1024 9.2 -> 8.4,

@@ -40,7 +40,7 @@ def test_pair_kernels_use_the_pair_forms_alone(source):
 
 
 CLUSTER_SOURCES = sorted(os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cu")) if "cudaLaunchAttributeClusterDimension" in code(p))
-REMOTE = r"\b(?:cluster_map_shared|cluster_store_uint4|cluster_load_float4|pair_arrive_remote|mbar_arrive_remote|wp_arrive|release_accumulator|pair_tmem_alloc|pair_commit_both|pair_mma)\s*\("
+REMOTE = r"\b(?:cluster_map_shared|cluster_store_uint4|pair_arrive_remote|mbar_arrive_remote|wp_arrive|release_accumulator|pair_tmem_alloc|pair_commit_both|pair_mma)\s*\("
 
 
 def test_cluster_kernels_are_found():
