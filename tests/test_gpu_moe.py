@@ -210,7 +210,7 @@ def test_route_sort_matches_oracle(gm, oracle, big_runner, cuda_device, tokens, 
 
 
 @pytest.mark.parametrize("tokens", [256, 257, 640, 1151, 1153, 1535, 1536, 1537])
-def test_route_sort_at_the_edges_of_its_chunks(gm, oracle, big_runner, cuda_device, tokens):
+def test_route_sort_at_the_edges_of_its_forms(gm, oracle, big_runner, cuda_device, tokens):
     """Every CTA of the one-launch sort counts the chunks of 1024 routes before and behind its own itself: whole and ragged last
     chunks, with experts that a token names twice and one that takes a route of every token."""
     from gevva_b200 import runtime as rt
@@ -241,11 +241,11 @@ def test_route_sort_around_its_longest_counts(gm, oracle, big_runner, cuda_devic
         assert (got[key] == want[key]).all(), key
 
 
-@pytest.mark.parametrize("tokens", [128, 129, 300, 1535, 1536, 1537, 3072, 3073, 4096])
+@pytest.mark.parametrize("tokens", [128, 129, 300, 1535, 1536, 1537])
 def test_route_sort_by_owner_at_one_rank(gm, varied_weights, cuda_device, tokens):
     """Expert-parallel ranks sort by the key that a placement table gives each expert: one rank alone, whose table is a permutation
-    of its own experts, has the bits of the plain runner in all three one-launch forms of the sort (up to 128 tokens one CTA a token, up to 24
-    chunks CTAs that count for themselves, above CTAs that meet), twice over."""
+    of its own experts, has the bits of the plain runner in the one-launch forms of the sort whose CTAs do not meet (one CTA up to 128 tokens, then
+    CTAs that count for themselves), twice over."""
     import ctypes
     from gevva_b200.expert_parallel import _EpConfig, local_expert_weights
     from gevva_b200.runtime import _Weights
@@ -285,6 +285,12 @@ def test_route_sort_by_owner_at_one_rank(gm, varied_weights, cuda_device, tokens
         assert lib.gevva_moe_ep_status(ep, ctypes.byref(rows)) == 0 and rows.value == routes
         assert torch.equal(got, want) and got.float().abs().max() > 0
     lib.gevva_moe_ep_destroy(ep)
+
+
+@pytest.mark.parametrize("tokens", [3072, 3073, 4096])
+def test_route_sort_by_owner_around_its_longest_counts(gm, varied_weights, cuda_device, tokens):
+    """The same at 24 chunks, up to which CTAs count for themselves, and above, where they meet: what a rank sorts at its usual sizes."""
+    test_route_sort_by_owner_at_one_rank(gm, varied_weights, cuda_device, tokens)
 
 
 def test_bad_expert_id_is_reported(gm, big_runner, cuda_device):
