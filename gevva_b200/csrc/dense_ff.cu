@@ -346,7 +346,7 @@ __device__ __forceinline__ void words(const uint4& v, uint32_t (&out)[4]) {
 // arithmetic, which is done on pairs.  The same results.  Alone, us, a block a row and this: 640 rows 5.25 and 4.55, 1024 7.5 and 6.0, 2048 12.8
 // and 10.1, 4096 23.5 and 18.3 (two or four CTAs an SM 20.7 and 21.8); feed-forward layers of 2048 tokens 443.1 and 441.9 (two), 3000 276.8 and 275.2, 4096 362.4
 // and 358.3.  With a row a CTA it is the slower one (64 rows 2.03 and 2.14; three layers of 301 tokens 314.6 and 316.4).
-constexpr int kPrepareCtas = 3 * 148;  // three an SM
+constexpr int kPrepareCtas = 3;  // of an SM
 
 __global__ void __launch_bounds__(kRowThreads, 3)
 ff_prepare_rows_kernel(const __nv_bfloat16* __restrict__ input, const __nv_bfloat16* __restrict__ dense_weight,
@@ -488,8 +488,9 @@ void launch_ff_prepare(const void* input, const void* dense_weight, const void* 
                        const void* router_scale, void* dense_out, void* expert_out, void* router_out,
                        int rows, cudaStream_t stream) {
   using B = __nv_bfloat16;
-  if (rows > kPrepareCtas) {
-    launch_chained(ff_prepare_rows_kernel, dim3(kPrepareCtas), dim3(kRowThreads), 0, stream, static_cast<const B*>(input),
+  const int ctas = kPrepareCtas * current_sm_count();
+  if (ctas > 0 && rows > ctas) {
+    launch_chained(ff_prepare_rows_kernel, dim3(ctas), dim3(kRowThreads), 0, stream, static_cast<const B*>(input),
                    static_cast<const B*>(dense_weight), static_cast<const B*>(expert_weight),
                    static_cast<const B*>(router_scale), static_cast<B*>(dense_out), static_cast<B*>(expert_out),
                    static_cast<B*>(router_out), rows);

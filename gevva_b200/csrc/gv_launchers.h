@@ -20,6 +20,7 @@ int dense_launch_on(gevva_dense* dense, const void* in, void* out_unscaled, int 
                     int sm_count, int* status);
 int moe_sm_count(const gevva_moe* runner);
 int moe_max_tokens(const gevva_moe* runner);
+int current_sm_count();  // of the current device; 0 if the runtime does not say
 // Whether the runner's expert GEMMs of a batch of this size are one launch that streams the weights.
 bool moe_streams(const gevva_moe* runner, int tokens);
 

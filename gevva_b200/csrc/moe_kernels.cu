@@ -368,8 +368,7 @@ route_sort_fused_kernel(const int* __restrict__ expert_ids, int routes, int chun
   }
 }
 
-namespace {
-// SM count of the current device, cached per device ordinal.
+// Cached per device ordinal.
 int current_sm_count() {
   static int cached[64] = {0};
   int device = 0;
@@ -380,7 +379,6 @@ int current_sm_count() {
   }
   return cached[device];
 }
-}  // namespace
 
 void launch_route_sort(const int* expert_ids, int routes, const RoutePlan& plan,
                        cudaStream_t stream) {

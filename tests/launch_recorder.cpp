@@ -17,6 +17,7 @@ std::map<const void*, std::string>& names() {
   return table;
 }
 std::string log_text;
+int current_device = 0, current_sms = 148;
 struct Pending {
   dim3 grid, block;
   size_t shared;
@@ -54,6 +55,12 @@ const char* recorder_take_log() {
   taken.swap(log_text);
   log_text.clear();
   return taken.c_str();
+}
+
+// From now on the current device is this one, of so many SMs.
+void recorder_set_device(int device, int sms) {
+  current_device = device;
+  current_sms = sms;
 }
 
 void** __cudaRegisterFatBinary(void*) {
@@ -115,17 +122,17 @@ cudaError_t cudaGetSymbolAddress(void** pointer, const void* symbol) {
   return cudaSuccess;
 }
 cudaError_t cudaGetDevice(int* device) {
-  *device = 0;
+  *device = current_device;
   return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* value, cudaDeviceAttr attribute, int) {
-  *value = attribute == cudaDevAttrComputeCapabilityMajor ? 10 : attribute == cudaDevAttrMultiProcessorCount ? 148 : 0;
+  *value = attribute == cudaDevAttrComputeCapabilityMajor ? 10 : attribute == cudaDevAttrMultiProcessorCount ? current_sms : 0;
   return cudaSuccess;
 }
 cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp* properties, int) {
   *properties = cudaDeviceProp{};
   properties->major = 10;
-  properties->multiProcessorCount = 148;
+  properties->multiProcessorCount = current_sms;
   return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }

@@ -210,6 +210,19 @@ def test_feed_forward_layer_refuses_before_it_launches(recorder, capacity, dense
     assert recorder.launches() == []
 
 
+@pytest.mark.parametrize("device,sms", [(0, 148), (1, 74)])
+def test_prepare_takes_three_ctas_of_each_sm_that_there_is(recorder, device, sms):
+    """A CTA a row up to as many as run at once on the current device, then so many CTAs that take row after row."""
+    recorder.lib.recorder_set_device(device, sms)
+    try:
+        for rows in (1, 3 * sms, 3 * sms + 1, 4096):
+            assert recorder.lib.gevva_ff_prepare(*[ctypes.c_void_p(ADDRESS)] * 7, rows, ctypes.c_void_p(STREAM)) == 0
+            (launch,) = recorder.launches()
+            assert (launch["kernel"], launch["grid"]) == (("ff_prepare_kernel", rows) if rows <= 3 * sms else ("ff_prepare_rows_kernel", 3 * sms))
+    finally:
+        recorder.lib.recorder_set_device(0, 148)
+
+
 class _Cuda:
     """What forward() checks of a tensor."""
     is_cuda = True
